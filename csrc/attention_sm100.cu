@@ -144,10 +144,12 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t sQ = smem_base, sK = smem_base + 2 * kTile, sV = smem_base + 4 * kTile;   // Q, K, V: two stages each
   const uint32_t bars = smem_base + 6 * kTile;
-  // qf[2] qe[2] kf[2] vf[2] ke[2] ve[2] s[2] p[2] pv oe[2] | tmem slot
+  // qf[2] qe[2] kf[2] vf[2] ke[2] ve[2] s[2] p[2] pv[2] oe[2] | tmem slot
+  // pv has one barrier per S buffer: a softmax warp that runs ahead of its siblings reaches the wait for PV of tile g-1 while
+  // PV of tile g-2 has not even been issued; the parity of a single barrier could not tell the two apart
   const uint32_t bar_qf = bars, bar_qe = bars + 16, bar_kf = bars + 32, bar_vf = bars + 48, bar_ke = bars + 64,
-                 bar_ve = bars + 80, bar_s = bars + 96, bar_p = bars + 112, bar_pv = bars + 128, bar_oe = bars + 136,
-                 tmem_slot = bars + 152;
+                 bar_ve = bars + 80, bar_s = bars + 96, bar_p = bars + 112, bar_pv = bars + 128, bar_oe = bars + 144,
+                 tmem_slot = bars + 160;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nq = (p.S_q + BM - 1) / BM;
   const int n_tiles_kv = (p.S_kv + BN - 1) / BN;
@@ -158,8 +160,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
       mbar_init(bar_qf + 8 * i, 1); mbar_init(bar_qe + 8 * i, 1);
       mbar_init(bar_kf + 8 * i, 1); mbar_init(bar_vf + 8 * i, 1); mbar_init(bar_ke + 8 * i, 1); mbar_init(bar_ve + 8 * i, 1);
       mbar_init(bar_s + 8 * i, 1); mbar_init(bar_p + 8 * i, 128); mbar_init(bar_oe + 8 * i, 128);
+      mbar_init(bar_pv + 8 * i, 1);
     }
-    mbar_init(bar_pv, 1);
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -253,7 +255,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
           mma_ts(tmem_O + ob * HD, tmem_S + st * BN + k * 8, make_smem_desc(v_s + k * 2048, kHalf, 1024), idesc_o,
                  (cur.j | k) ? 1u : 0u);
         tcgen05_commit_e(bar_ve + 8 * st);
-        tcgen05_commit_e(bar_pv);
+        tcgen05_commit_e(bar_pv + 8 * st);
         if (ahead.ok) { issue_s(ahead); advance(ahead); }        // overwrites P of tile g — behind PV_g in pipe order
         advance(cur);
       }
@@ -306,7 +308,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
           const float m_new = fmaxf(m_ref, mx);
           const bool need = (m_new - m_ref) * sl2 > 8.f;
           if (__any_sync(0xffffffffu, need)) {
-            mbar_wait(bar_pv, (uint32_t)((g - 1) & 1));      // PV of the previous tile retired: O is quiescent
+            mbar_wait(bar_pv + 8 * ((g - 1) & 1), (uint32_t)(((g - 1) >> 1) & 1));      // PV of the previous tile retired: O is quiescent
             tcgen05_fence_after();
             const float f = need ? ex2((m_ref - m_new) * sl2) : 1.f;
             if (need) m_ref = m_new;
@@ -351,7 +353,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
         mbar_arrive(bar_p + 8 * st);
       }
       // ---- epilogue: O / l → bf16, LSE (the MMA warp is already working on the next item in the other O buffer)
-      mbar_wait(bar_pv, (uint32_t)((g - 1) & 1));
+      mbar_wait(bar_pv + 8 * ((g - 1) & 1), (uint32_t)(((g - 1) >> 1) & 1));
       tcgen05_fence_after();
       const float inv_l = 1.f / l;
       const bool row_ok = q_idx < p.S_q;
