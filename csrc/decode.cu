@@ -7,6 +7,8 @@
 //                      with 16-byte loads, fp32 accumulation.
 #include <cuda.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -15,106 +17,189 @@ namespace nxd {
 namespace {
 
 constexpr int HD = 128;
-constexpr int kDecThreads = 128;
+constexpr int kDecWarps = 4;
+constexpr int kDecThreads = kDecWarps * 32;
+constexpr int kDecRows = 16;                                 // cache rows of one tile of a warp
+constexpr int kDecStages = 3;
+constexpr int kDecTileBytes = kDecRows * HD * 2;             // 4 KB of K, as much of V
+constexpr int kDecSmem = kDecWarps * kDecStages * 2 * kDecTileBytes;      // 96 KB: two blocks per SM
 
-// 16 lanes share one kv position (8 dims = 16 bytes each); a warp covers 2 positions per step, the CTA 8.
+NXD_DEVICE void cp_async16(uint32_t dst, const void* src, bool live) {    // not live: 16 zero bytes, nothing is read
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+NXD_DEVICE void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> NXD_DEVICE void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+NXD_DEVICE void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+NXD_DEVICE void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {   // rows 8..15 of A are zero
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %5}, {%7, %8}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(0u), "r"(a2), "r"(b0), "r"(b1));
+}
+
+// One block per (key/value head, sequence, stretch of the cache); its G <= 8 query heads share every row that is read.
+// Bound by HBM: 512 bytes per cache row and key/value head.  Each warp walks 16-row tiles of its own through its own ring of
+// cp.async stages (2 x 8 KB in flight per warp, 128 KB per SM, no block barrier in the loop).  Scores come from mma.sync
+// (a 16 x 8 x 16 step holds all heads of the group; exact products, fp32 sums), so a row costs a few instructions per warp
+// instead of a dot product with four shuffles per head; probabilities stay fp32 and meet V in fp32 FMAs, lane = 4 columns.
+// 8 sequences, 8192-row cache (three quarters in use), 32 heads on 8: 39 us = 5.2 TB/s; with dot products on CUDA cores and
+// 8 rows in flight per block it was 148 us.
 template <int G>
-__global__ void __launch_bounds__(kDecThreads) decode_attn_kernel(
+__global__ void __launch_bounds__(kDecThreads, 2) decode_attn_kernel(
     const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kc, const __nv_bfloat16* __restrict__ vc,
-    const long* __restrict__ positions, float* __restrict__ part_o, float* __restrict__ part_ml, int B, int H, int Hkv, int L,
-    long k_sb, long k_ss, long k_sh, long v_sb, long v_ss, long v_sh, long q_sb, long q_sh, float scale_log2, int splits) {
+    const long* __restrict__ positions, float* __restrict__ part_o, float* __restrict__ part_ml,
+    __nv_bfloat16* __restrict__ out, int B, int H, int Hkv, int L,
+    long k_sb, long k_ss, long k_sh, long v_sb, long v_ss, long v_sh, long q_sb, long q_sh, long o_sb, long o_sh,
+    float scale_log2, int splits) {
+  extern __shared__ __align__(128) uint8_t dec_smem[];
   const int kvh = blockIdx.x, b = blockIdx.y, split = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int sub = lane >> 4, l16 = lane & 15;               // position slot within the warp step, 8-dim slice
-  const int n_valid = min((int)positions[b] + 1, L);
+  const long pos = positions[b];
+  const int n_valid = (int)(pos < 0 ? 0 : (pos >= L ? L : pos + 1));
   const int per = (n_valid + splits - 1) / splits;
   const int s0 = split * per, s1 = min(n_valid, s0 + per);
+  const uint32_t ring = (uint32_t)__cvta_generic_to_shared(dec_smem) + warp * (kDecStages * 2 * kDecTileBytes);
+  const __nv_bfloat16* kb = kc + b * k_sb + (long)kvh * k_sh;
+  const __nv_bfloat16* vb = vc + b * v_sb + (long)kvh * v_sh;
 
-  auto load8 = [](const __nv_bfloat16* p, float (&f)[8], float mul) {
-    const uint4 a = *reinterpret_cast<const uint4*>(p);
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&a);
+  // 16 lanes copy one 256-byte row, 16-byte chunk c of row r lands at chunk (c ^ (r & 7)): both ways of reading are conflict-free
+  const int cr = lane >> 4, cc = lane & 15;
+  auto load_tile = [&](int row0, int stage) {
+    const uint32_t dst = ring + stage * (2 * kDecTileBytes);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) { const float2 t = __bfloat1622float2(h[i]); f[2 * i] = t.x * mul; f[2 * i + 1] = t.y * mul; }
-  };
-  float qf[G][8];
-#pragma unroll
-  for (int g = 0; g < G; ++g) load8(q + b * q_sb + (long)(kvh * G + g) * q_sh + l16 * 8, qf[g], scale_log2);
-  float m[G], l[G], o[G][8];
-#pragma unroll
-  for (int g = 0; g < G; ++g) {
-    m[g] = -INFINITY; l[g] = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) o[g][i] = 0.f;
-  }
-  const __nv_bfloat16* kb = kc + b * k_sb + (long)kvh * k_sh + l16 * 8;
-  const __nv_bfloat16* vb = vc + b * v_sb + (long)kvh * v_sh + l16 * 8;
-  for (int sbase = s0 + warp * 2; sbase < s1; sbase += 8) {      // warp-uniform trip count (full-mask shuffles inside)
-    const int s = sbase + sub;
-    const bool live = s < s1;
-    float kf[8], vf[8];
-    if (live) {
-      load8(kb + (long)s * k_ss, kf, 1.f);
-      load8(vb + (long)s * v_ss, vf, 1.f);
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) { kf[i] = 0.f; vf[i] = 0.f; }
+    for (int i = 0; i < kDecRows / 2; ++i) {
+      const int r = i * 2 + cr, s = row0 + r;
+      const bool live = s < s1;
+      const long at = live ? s : s0;                       // a row that exists, read or not
+      const uint32_t off = r * 256 + ((cc ^ (r & 7)) << 4);
+      cp_async16(dst + off, kb + at * k_ss + cc * 8, live);
+      cp_async16(dst + kDecTileBytes + off, vb + at * v_ss + cc * 8, live);
     }
+  };
+  const int first = s0 + warp * kDecRows;
+  const int tiles = first < s1 ? (s1 - first + kDecWarps * kDecRows - 1) / (kDecWarps * kDecRows) : 0;
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      float d = 0.f;
+  for (int st = 0; st < kDecStages - 1; ++st) {
+    if (st < tiles) load_tile(first + st * kDecWarps * kDecRows, st);
+    cp_async_commit();
+  }
+
+  // query fragments: row = head of the group (rows >= G zero), two 32-bit words per 16 columns
+  const int hq = lane >> 2, quad = lane & 3;
+  uint32_t qa[8][2];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) d = fmaf(qf[g][i], kf[i], d);
-      d += __shfl_xor_sync(0xffffffffu, d, 1);
-      d += __shfl_xor_sync(0xffffffffu, d, 2);
-      d += __shfl_xor_sync(0xffffffffu, d, 4);
-      d += __shfl_xor_sync(0xffffffffu, d, 8);            // score·log2e of (position s, head g) in all 16 lanes
-      if (live) {
-        const float mn = fmaxf(m[g], d);
-        const float corr = exp2f(m[g] - mn), p = exp2f(d - mn);
-        m[g] = mn;
-        l[g] = l[g] * corr + p;
+  for (int k = 0; k < 8; ++k) {
+    qa[k][0] = qa[k][1] = 0u;
+    if (hq < G) {
+      const __nv_bfloat16* qp = q + b * q_sb + (long)(kvh * G + hq) * q_sh + k * 16 + quad * 2;
+      qa[k][0] = *reinterpret_cast<const uint32_t*>(qp);
+      qa[k][1] = *reinterpret_cast<const uint32_t*>(qp + 8);
+    }
+  }
+  __shared__ __align__(16) float sm_p[kDecWarps][kDecRows][G];
+  float m = -INFINITY, l = 0.f;                            // of head hq; l of this lane's columns only
+  float o[G][4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) o[g][i] = fmaf(o[g][i], corr, p * vf[i]);
+  for (int g = 0; g < G; ++g)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[g][i] = 0.f;
+
+  for (int t = 0; t < tiles; ++t) {
+    const int row0 = first + t * kDecWarps * kDecRows;
+    cp_async_wait<kDecStages - 2>();
+    __syncwarp();                                          // tile t of all lanes is there; all lanes are done with tile t - 1
+    if (t + kDecStages - 1 < tiles) load_tile(row0 + (kDecStages - 1) * kDecWarps * kDecRows, (t + kDecStages - 1) % kDecStages);
+    cp_async_commit();
+    const uint32_t ks = ring + (t % kDecStages) * (2 * kDecTileBytes), vs = ks + kDecTileBytes;
+    float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      // matrices: rows 0-7 / columns 16k.., rows 0-7 / 16k + 8.., rows 8-15 / 16k.., rows 8-15 / 16k + 8..
+      const int r = ((lane >> 4) << 3) + (lane & 7), c = k * 2 + ((lane >> 3) & 1);
+      uint32_t kf[4];
+      ldmatrix_x4(kf, ks + r * 256 + ((c ^ (r & 7)) << 4));
+      mma_bf16(d[0], qa[k][0], qa[k][1], kf[0], kf[1]);
+      mma_bf16(d[1], qa[k][0], qa[k][1], kf[2], kf[3]);
+    }
+    float sc[4] = {d[0][0] * scale_log2, d[0][1] * scale_log2, d[1][0] * scale_log2, d[1][1] * scale_log2};
+    if (row0 + kDecRows > s1) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (row0 + (i >> 1) * 8 + quad * 2 + (i & 1) >= s1) sc[i] = -INFINITY;
+    }
+    float mx = fmaxf(fmaxf(sc[0], sc[1]), fmaxf(sc[2], sc[3]));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    const bool grew = mx > m;
+    if (__any_sync(0xffffffffu, grew)) {
+      const float mn = fmaxf(m, mx);
+      const float corr = grew ? exp2f(m - mn) : 1.f;       // m = -inf: 0
+      m = mn;
+      l *= corr;
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        const float c = __shfl_sync(0xffffffffu, corr, g * 4);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[g][i] *= c;
+      }
+    }
+    const float ms = m == -INFINITY ? 0.f : m;
+    float p[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { p[i] = exp2f(sc[i] - ms); l += p[i]; }
+    if (hq < G) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sm_p[warp][(i >> 1) * 8 + quad * 2 + (i & 1)][hq] = p[i];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < kDecRows; ++r) {
+      uint2 raw;
+      asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(raw.x), "=r"(raw.y)
+                   : "r"(vs + r * 256 + (((lane >> 1) ^ (r & 7)) << 4) + (lane & 1) * 8));
+      const float2 v01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+      const float2 v23 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        const float pg = sm_p[warp][r][g];
+        o[g][0] = fmaf(pg, v01.x, o[g][0]);
+        o[g][1] = fmaf(pg, v01.y, o[g][1]);
+        o[g][2] = fmaf(pg, v23.x, o[g][2]);
+        o[g][3] = fmaf(pg, v23.y, o[g][3]);
       }
     }
   }
-  // merge the 2 position slots of the warp (lanes l16, l16+16), then the 4 warps through smem
-  __shared__ float sm_o[4][G][HD];
-  __shared__ float sm_m[4][G], sm_l[4][G];
-#pragma unroll
-  for (int g = 0; g < G; ++g) {
-    const float m2 = __shfl_xor_sync(0xffffffffu, m[g], 16), l2 = __shfl_xor_sync(0xffffffffu, l[g], 16);
-    const float mn = fmaxf(m[g], m2);
-    const float c1 = mn == -INFINITY ? 0.f : exp2f(m[g] - mn), c2 = mn == -INFINITY ? 0.f : exp2f(m2 - mn);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float o2 = __shfl_xor_sync(0xffffffffu, o[g][i], 16);
-      o[g][i] = o[g][i] * c1 + o2 * c2;
-    }
-    l[g] = l[g] * c1 + l2 * c2;
-    m[g] = mn;
-    if (sub == 0) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) sm_o[warp][g][l16 * 8 + i] = o[g][i];
-      if (l16 == 0) { sm_m[warp][g] = m[g]; sm_l[warp][g] = l[g]; }
-    }
-  }
+  l += __shfl_xor_sync(0xffffffffu, l, 1);
+  l += __shfl_xor_sync(0xffffffffu, l, 2);
+  // ---- the four warps' sums, through the ring (every copy has landed: tiles that were asked for were waited for)
+  cp_async_wait<0>();
   __syncthreads();
-  // thread t = dim; loop over heads of the group
-  const int d = threadIdx.x;
+  float* sm_o = reinterpret_cast<float*>(dec_smem);        // [warp][G][128]
+  __shared__ float sm_m[kDecWarps][8], sm_l[kDecWarps][8];
+#pragma unroll
+  for (int g = 0; g < G; ++g)
+    *reinterpret_cast<float4*>(sm_o + (warp * G + g) * HD + lane * 4) = make_float4(o[g][0], o[g][1], o[g][2], o[g][3]);
+  if (quad == 0) { sm_m[warp][hq] = m; sm_l[warp][hq] = l; }
+  __syncthreads();
+  const int col = threadIdx.x;
 #pragma unroll
   for (int g = 0; g < G; ++g) {
-    float mn = fmaxf(fmaxf(sm_m[0][g], sm_m[1][g]), fmaxf(sm_m[2][g], sm_m[3][g]));
+    const float mn = fmaxf(fmaxf(sm_m[0][g], sm_m[1][g]), fmaxf(sm_m[2][g], sm_m[3][g]));
     float acc = 0.f, ls = 0.f;
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
+    for (int w = 0; w < kDecWarps; ++w) {
       const float c = mn == -INFINITY ? 0.f : exp2f(sm_m[w][g] - mn);
-      acc += sm_o[w][g][d] * c;
+      acc += sm_o[(w * G + g) * HD + col] * c;
       ls += sm_l[w][g] * c;
     }
-    const long idx = (((long)b * H + kvh * G + g) * splits + split);
-    part_o[idx * HD + d] = acc;
-    if (d == 0) { part_ml[idx * 2] = mn; part_ml[idx * 2 + 1] = ls; }
+    if (out != nullptr) {                                  // the only stretch: nothing to merge
+      out[b * o_sb + (long)(kvh * G + g) * o_sh + col] = __float2bfloat16_rn(ls > 0.f ? acc / ls : 0.f);
+    } else {
+      const long idx = (((long)b * H + kvh * G + g) * splits + split);
+      part_o[idx * HD + col] = acc;
+      if (col == 0) { part_ml[idx * 2] = mn; part_ml[idx * 2 + 1] = ls; }
+    }
   }
 }
 
@@ -247,16 +332,28 @@ void decode_rope_kv(const void* q, const void* k, const void* v, const long* pos
   NXD_CUDA_CHECK(cudaGetLastError());
 }
 
+// Stretches per (sequence, key/value head): about six blocks per SM in all, so that sequences of unequal length fill the GPU to
+// the end (8 x 8192 rows, 8 key/value heads: 39 us; four per SM 41, sixteen 45), and no stretch below 256 rows, where a block's
+// start and the merge outweigh its reading (1 x 2048 rows, 40 heads: 11.2 us with the merge; 128-row stretches 12.1, 64-row 14.7).
+int decode_splits(int pairs, int L) {
+  const int want = (6 * 148 + pairs - 1) / pairs;
+  return std::max(1, std::min(std::min(want, 64), (L + 255) / 256));
+}
+
 void decode_attention(const void* q, const void* k, const void* v, const long* positions, void* out, float* part_o,
                       float* part_ml, int B, int H, int Hkv, int L, const long* ks, const long* vs, long q_sb, long q_sh,
                       long o_sb, long o_sh, float scale, int splits, cudaStream_t st, float* fin_o, float* fin_ml) {
   const int G = H / Hkv;
   dim3 grid(Hkv, B, splits);
   const float sl2 = scale * 1.4426950408889634f;
+  const bool whole = splits == 1 && fin_o == nullptr;
 #define NXD_DEC(Gv)                                                                                                  \
-  decode_attn_kernel<Gv><<<grid, kDecThreads, 0, st>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)k,             \
-      (const __nv_bfloat16*)v, positions, part_o, part_ml, B, H, Hkv, L, ks[0], ks[1], ks[2], vs[0], vs[1], vs[2], q_sb, \
-      q_sh, sl2, splits)
+  do {                                                                                                               \
+    NXD_CUDA_CHECK(cudaFuncSetAttribute(decode_attn_kernel<Gv>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecSmem)); \
+    decode_attn_kernel<Gv><<<grid, kDecThreads, kDecSmem, st>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)k,      \
+        (const __nv_bfloat16*)v, positions, part_o, part_ml, whole ? (__nv_bfloat16*)out : nullptr, B, H, Hkv, L,      \
+        ks[0], ks[1], ks[2], vs[0], vs[1], vs[2], q_sb, q_sh, o_sb, o_sh, sl2, splits);                                \
+  } while (0)
   switch (G) {
     case 1: NXD_DEC(1); break;
     case 2: NXD_DEC(2); break;
@@ -266,7 +363,7 @@ void decode_attention(const void* q, const void* k, const void* v, const long* p
   }
 #undef NXD_DEC
   if (fin_o != nullptr) decode_combine_partial_kernel<<<B * H, HD, 0, st>>>(part_o, part_ml, fin_o, fin_ml, splits);
-  else decode_combine_kernel<<<B * H, HD, 0, st>>>(part_o, part_ml, (__nv_bfloat16*)out, splits, o_sb, o_sh, H);
+  else if (!whole) decode_combine_kernel<<<B * H, HD, 0, st>>>(part_o, part_ml, (__nv_bfloat16*)out, splits, o_sb, o_sh, H);
   NXD_CUDA_CHECK(cudaGetLastError());
 }
 

@@ -141,6 +141,7 @@ void gemv_mx_grouped(const void* x, const void* w, const void* scale, const long
                      cudaStream_t st);
 
 // ---- decode (decode.cu)
+int decode_splits(int pairs, int L);
 void decode_attention(const void* q, const void* k, const void* v, const long* positions, void* out, float* part_o,
                       float* part_ml, int B, int H, int Hkv, int L, const long* ks, const long* vs, long q_sb, long q_sh,
                       long o_sb, long o_sh, float scale, int splits, cudaStream_t st, float* fin_o = nullptr,

@@ -1,0 +1,55 @@
+"""Single-token attention over a cache, at the edges of its tiles (16 rows a warp, 64 a block) and stretches."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _reference(q, k, v, positions):
+    out = torch.zeros(q.shape, device=q.device)
+    group = q.shape[2] // k.shape[2]
+    for b, p in enumerate(positions.tolist()):
+        n = max(0, min(p + 1, k.shape[1]))
+        if n == 0:
+            continue
+        kb, vb = (t[b, :n].float().repeat_interleave(group, 1) for t in (k, v))
+        s = torch.einsum("hd,lhd->hl", q[b, 0].float(), kb) / math.sqrt(128)
+        out[b, 0] = torch.einsum("hl,lhd->hd", torch.softmax(s, -1), vb)
+    return out
+
+
+@pytest.mark.parametrize("group", [1, 2, 4, 8])
+@pytest.mark.parametrize("rows,positions", [(1, [0, 0]), (17, [15, 16]), (130, [63, 64]), (700, [-1, 699]), (2500, [2499, 40]),
+                                            (64, [62, 5000])])
+def test_edges(group, rows, positions):
+    from neuronx_distributed_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(rows + group)
+    kv = torch.randn(2, rows, 2, 2 * 128, generator=g, device="cuda").bfloat16()      # k and v interleaved: strided views
+    k, v = kv[..., :128], kv[..., 128:]
+    q = torch.randn(2, 1, 2 * group, 128, generator=g, device="cuda").bfloat16() * 3
+    pos = torch.tensor(positions, device="cuda")
+    want = _reference(q, k, v, pos)
+    for b, p in enumerate(positions):
+        if 0 <= p + 1 < rows:
+            kv[b, p + 1:] = math.nan                                               # rows behind the position are never used
+    got = ops.attention.decode_attention(q, k, v, pos).float()
+    # one rounding to bfloat16 (2^-9 of the value) over fp32 sums
+    assert (got - want).abs().max() <= 2.0 ** -8 * want.abs().max()
+    assert torch.isfinite(got).all()
+
+
+def test_partial_results_merge_to_the_whole():
+    from neuronx_distributed_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = (torch.randn(2, n, h, 128, generator=g, device="cuda").bfloat16() for n, h in ((1, 8), (600, 2), (600, 2)))
+    pos = torch.tensor([599, 250], device="cuda")
+    whole = ops.attention.decode_attention(q, k, v, pos).float()[:, 0]
+    parts = [ops._ext.ext().decode_attention_partial(q, k[:, a:a + 300], v[:, a:a + 300], pos - a, 128 ** -0.5) for a in (0, 300)]
+    m = torch.maximum(parts[0][1][..., 0], parts[1][1][..., 0])
+    num = sum(o * torch.exp(ml[..., 0] - m)[..., None] for o, ml in parts)
+    den = sum(ml[..., 1] * torch.exp(ml[..., 0] - m) for _, ml in parts)
+    assert (num / den[..., None] - whole).abs().max() <= 2.0 ** -8 * whole.abs().max()
