@@ -407,7 +407,9 @@ static Tensor gemv(const Tensor& x, const Tensor& w, const c10::optional<Tensor>
 }
 
 // ---- grouped (MoE) GEMMs -------------------------------------------------------------------------
-static Tensor grouped_gemm(const Tensor& a, const Tensor& w, const Tensor& block_expert, int64_t block_rows, bool trans_b) {
+static Tensor grouped_gemm(const Tensor& a, const Tensor& w, const Tensor& block_expert, int64_t block_rows, bool trans_b,
+                           const c10::optional<Tensor>& seg) {
+  // seg (int32 block prefix sums [E+1], optional): row blocks from seg[E] on hold no tokens and are left unwritten
   TORCH_CHECK(a.is_cuda() && a.scalar_type() == at::kBFloat16 && a.dim() == 2 && a.is_contiguous());
   TORCH_CHECK(w.scalar_type() == at::kBFloat16 && w.dim() == 3 && w.is_contiguous());
   TORCH_CHECK(block_expert.scalar_type() == at::kInt && block_expert.is_cuda());
@@ -417,7 +419,12 @@ static Tensor grouped_gemm(const Tensor& a, const Tensor& w, const Tensor& block
   TORCH_CHECK(block_expert.numel() * block_rows == M);
   c10::cuda::CUDAGuard guard(a.device());
   Tensor out = at::empty({M, N}, a.options());
-  nxd::grouped_gemm_bf16(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, E, trans_b, block_expert.data_ptr<int>(),
+  const int* used = nullptr;
+  if (seg.has_value()) {
+    TORCH_CHECK(seg->is_cuda() && seg->is_contiguous() && seg->scalar_type() == at::kInt && seg->numel() == E + 1);
+    used = seg->data_ptr<int>() + E;
+  }
+  nxd::grouped_gemm_bf16(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, E, trans_b, block_expert.data_ptr<int>(), used,
                          (int)block_rows, nxd::kBF16, stream());
   return out;
 }
@@ -791,7 +798,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("row_topk_supported", &row_topk_supported);
   m.def("gemv", &gemv, py::arg("x"), py::arg("w"), py::arg("residual") = py::none());
   m.def("gemm_fp8", &gemm_fp8);
-  m.def("grouped_gemm", &grouped_gemm);
+  m.def("grouped_gemm", &grouped_gemm, py::arg("a"), py::arg("w"), py::arg("block_expert"), py::arg("block_rows"), py::arg("trans_b"),
+        py::arg("seg") = c10::nullopt);
   m.def("grouped_wgrad", &grouped_wgrad);
   m.def("flash_attn_fwd", &flash_attn_fwd);
   m.def("flash_attn_bwd", &flash_attn_bwd, py::arg("go"), py::arg("q"), py::arg("k"), py::arg("v"), py::arg("o"), py::arg("lse"),

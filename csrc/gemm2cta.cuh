@@ -69,33 +69,16 @@ NXD_DEVICE void store_chunk(OutT* orow, int col0, int N, const uint32_t (&r)[32]
       }
     }
   } else {
-    if (col0 + 32 <= N) {
+    if (col0 + 32 <= N) {                    // fp32 outputs that accumulate leave through epilogue_tile_tma_f32
       float4* dst = (float4*)(orow + col0);
-      if (accumulate == 2) {                 // split-K partial: vector atomic add (fire-and-forget reduction at L2)
 #pragma unroll
-        for (int v = 0; v < 8; ++v)
-          asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
-                       ::"l"(dst + v), "f"(__uint_as_float(r[4 * v])), "f"(__uint_as_float(r[4 * v + 1])),
-                         "f"(__uint_as_float(r[4 * v + 2])), "f"(__uint_as_float(r[4 * v + 3])) : "memory");
-      } else {
-#pragma unroll
-        for (int v = 0; v < 8; ++v) {
-          float4 o = make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]), __uint_as_float(r[4 * v + 2]),
-                                 __uint_as_float(r[4 * v + 3]));
-          if (accumulate) { const float4 p = dst[v]; o.x += p.x; o.y += p.y; o.z += p.z; o.w += p.w; }
-          dst[v] = o;
-        }
-      }
+      for (int v = 0; v < 8; ++v)
+        dst[v] = make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]), __uint_as_float(r[4 * v + 2]),
+                             __uint_as_float(r[4 * v + 3]));
     } else {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        if (col0 + j < N) {
-          float v = __uint_as_float(r[j]);
-          if (accumulate == 2) { atomicAdd(((float*)orow) + col0 + j, v); continue; }
-          if (accumulate) v += ((float*)orow)[col0 + j];
-          ((float*)orow)[col0 + j] = v;
-        }
-      }
+      for (int j = 0; j < 32; ++j)
+        if (col0 + j < N) ((float*)orow)[col0 + j] = __uint_as_float(r[j]);
     }
   }
 }
@@ -129,14 +112,63 @@ NXD_DEVICE void bulk_wait_n(int n) {       // all but the newest n bulk groups h
   }
 }
 
+NXD_DEVICE void tma_store_3d(const CUtensorMap* map, uint32_t smem_src, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+               ::"l"(map), "r"(smem_src), "r"(c0), "r"(c1), "r"(c2) : "memory");
+}
+NXD_DEVICE void tma_reduce_add_3d(const CUtensorMap* map, uint32_t smem_src, int c0, int c1, int c2) {
+  asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
+               ::"l"(map), "r"(smem_src), "r"(c0), "r"(c1), "r"(c2) : "memory");
+}
+
+// fp32 twin of epilogue_tile_tma below: slabs of 32 columns (128-byte rows again) leave through a 3-D map {columns, rows, matrices},
+// as a plain store or added to memory by the copy engine (`add`: gradient accumulation, split-K partials).  A weight gradient is
+// bound by these writes as much as by its products: with one row-strided 16-byte store per thread and instruction the tensor pipe
+// waited for the epilogue.  7B feed-forward weight gradients over 4096 tokens: 846 + 39 us (stores, zeroing for a split) -> 744.
+NXD_DEVICE void epilogue_tile_tma_f32(uint32_t tmem_acc, uint32_t stage_smem, const CUtensorMap* omap, int row0, int mat, int col0,
+                                      int N, int q, int lane, bool issuer, uint32_t& slab_ctr, bool add, bool zero) {
+  const int row = q * 32 + lane;
+#pragma unroll 1
+  for (int s = 0; s < TILE_N / 32; ++s) {
+    const int c0 = col0 + s * 32;
+    if (c0 >= N) break;
+    const uint32_t buf = stage_smem + (slab_ctr & 1u) * kEpiSlabBytes;
+    uint32_t r[32];
+    tcgen05_ld_32x32(tmem_acc + s * 32, r);
+    if (issuer) bulk_wait_read<1>();
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    tcgen05_wait_ld();
+    if (zero) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) r[j] = 0u;
+    }
+    const uint32_t rbase = buf + (uint32_t)row * 128u;
+    const uint32_t sw = (uint32_t)(row & 7);
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};"
+                   ::"r"(rbase + (((uint32_t)c ^ sw) << 4)), "r"(r[4 * c]), "r"(r[4 * c + 1]), "r"(r[4 * c + 2]), "r"(r[4 * c + 3])
+                   : "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    if (issuer) {
+      if (add) tma_reduce_add_3d(omap, buf, c0, row0, mat);
+      else tma_store_3d(omap, buf, c0, row0, mat);
+      bulk_commit();
+    }
+    ++slab_ctr;
+  }
+}
+
 // Epilogue of one 128x256 accumulator (this CTA's TMEM lanes) to a row-major bf16 matrix through TMA stores.
 // Executed by the 128 epilogue threads (warps 2-5, named barrier 1); thread `issuer` (one of them) owns the bulk groups.
 // Per 64-column slab: wait until the staging buffer's previous store has read it, tcgen05.ld 2x32 columns, pack to bf16,
 // write the thread's 128-byte row in the 128B-swizzle pattern (conflict-free: 8 consecutive rows hit 8 different 16-byte
 // bank groups), fence to the async proxy, TMA-store the slab.  Rows/columns beyond the matrix are clipped by TMA.
 // Returns the number of bulk groups committed (slabs inside the matrix).  `slab_ctr` carries the buffer parity.
+template <bool MATS = false>      // MATS: a 3-D map {columns, rows, matrices}, matrix `mat`; `zero`: the accumulator was never written
 NXD_DEVICE int epilogue_tile_tma(uint32_t tmem_acc, uint32_t stage_smem, const CUtensorMap* omap, int row0, int col0, int N,
-                                 int q, int lane, bool issuer, uint32_t& slab_ctr) {
+                                 int q, int lane, bool issuer, uint32_t& slab_ctr, int mat = 0, bool zero = false) {
   const int row = q * 32 + lane;
   int groups = 0;
 #pragma unroll 1
@@ -150,6 +182,12 @@ NXD_DEVICE int epilogue_tile_tma(uint32_t tmem_acc, uint32_t stage_smem, const C
     tcgen05_ld_32x32(tmem_acc + s * kEpiSlabCols, r0);
     tcgen05_ld_32x32(tmem_acc + s * kEpiSlabCols + 32, r1);
     tcgen05_wait_ld();
+    if constexpr (MATS) {
+      if (zero) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) r0[j] = r1[j] = 0u;
+      }
+    }
     const uint32_t rbase = buf + (uint32_t)row * 128u;
     const uint32_t sw = (uint32_t)(row & 7);
 #pragma unroll
@@ -164,7 +202,11 @@ NXD_DEVICE int epilogue_tile_tma(uint32_t tmem_acc, uint32_t stage_smem, const C
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("bar.sync 1, 128;" ::: "memory");
-    if (issuer) { tma_store_2d(omap, buf, c0, row0); bulk_commit(); }
+    if (issuer) {
+      if constexpr (MATS) tma_store_3d(omap, buf, c0, row0, mat);
+      else tma_store_2d(omap, buf, c0, row0);
+      bulk_commit();
+    }
     ++slab_ctr;
     ++groups;
   }

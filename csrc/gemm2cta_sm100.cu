@@ -20,14 +20,47 @@
 namespace nxd {
 namespace g2 {
 
-template <bool A_KMAJOR, bool B_KMAJOR, typename OutT>
+// Grouped (routed experts) modes.  MODE 3: every `block_rows`-row block of A (a multiple of 256: a pair's tile stays inside one
+// block) meets the weights of one expert, `b_rows` rows further down the stacked B per expert; `used_blocks` (device, may be
+// null) bounds the blocks that hold tokens.  MODE 4 (weight gradients): one output matrix per expert, summed over that
+// expert's row blocks [seg[e], seg[e + 1]); an expert without tokens gets zeros.
+struct Group {
+  const int* block_expert;
+  const int* seg;
+  const int* used_blocks;
+  int block_rows, b_rows, groups;
+};
+
+// one unit of work of a pair: an output tile and its range of k-blocks
+struct Unit { int m_blk, n_blk, mat, kb0, kb1; };
+
+template <int MODE>
+NXD_DEVICE Unit unit_of(int unit, int num_tiles, int tiles_m, int tiles_n, int num_kb, int kb_per, const Group& g) {
+  Unit u;
+  u.mat = 0;
+  if constexpr (MODE == 4) {
+    const int per = tiles_m * tiles_n;
+    u.mat = unit / per;
+    tile_coords(unit - u.mat * per, tiles_m, tiles_n, u.m_blk, u.n_blk);
+    u.kb0 = g.seg[u.mat] * (g.block_rows / BK);
+    u.kb1 = g.seg[u.mat + 1] * (g.block_rows / BK);
+  } else {
+    const int ks = unit / num_tiles;
+    tile_coords(unit - ks * num_tiles, tiles_m, tiles_n, u.m_blk, u.n_blk);
+    u.kb0 = ks * kb_per;
+    u.kb1 = min(num_kb, (ks + 1) * kb_per);
+  }
+  return u;
+}
+
+template <bool A_KMAJOR, bool B_KMAJOR, typename OutT, int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                       const __grid_constant__ CUtensorMap tma_out, OutT* __restrict__ out, int M, int N, int K, int accumulate,
-                      int split_k) {
-  // accumulate: 0 store, 1 read-modify-write, 2 atomic add (split-K: `split_k` CTA pairs share one output tile, each
-  // reduces a K range and adds its fp32 partial with red.global.add.v4 — used for the weight-gradient GEMMs whose output
-  // has too few tiles to fill the 74 CTA pairs while K = tokens is huge)
+                      int split_k, const Group grp) {
+  // accumulate: 0 store, 1 add to what is there.  split_k > 1 (fp32 outputs): that many pairs share one output tile, each sums
+  // a K range and adds its partial — for weight gradients whose output has too few tiles to fill the 74 pairs while
+  // K = tokens is long.  fp32 outputs always leave through TMA (stored or added in memory), bf16 ones unless they accumulate.
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = (uint64_t*)(smem + kBarOffset);
@@ -39,8 +72,10 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t cta = cluster_ctarank();
   const bool leader = cta == 0;
-  const int tiles_m = (M + TILE_M - 1) / TILE_M, tiles_n = (N + TILE_N - 1) / TILE_N;
-  const int num_tiles = tiles_m * tiles_n;
+  int tiles_m = (M + TILE_M - 1) / TILE_M;
+  const int tiles_n = (N + TILE_N - 1) / TILE_N;
+  if constexpr (MODE == 3) { if (grp.used_blocks) tiles_m = min(tiles_m, *grp.used_blocks * (grp.block_rows / TILE_M)); }
+  const int num_tiles = (MODE == 4 ? grp.groups : 1) * tiles_m * tiles_n;
   const int num_kb = (K + BK - 1) / BK;
   const int kb_per = (num_kb + split_k - 1) / split_k;       // k-blocks per split (host guarantees no empty split)
   const int num_units = num_tiles * split_k;
@@ -71,13 +106,12 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     if (lane == 0) {
       int stage = 0; uint32_t phase = 0;
       for (int unit = pair; unit < num_units; unit += num_pairs) {
-        const int tile = unit % num_tiles, ks = unit / num_tiles;
-        int m_blk, n_blk;
-        tile_coords(tile, tiles_m, tiles_n, m_blk, n_blk);
-        const int m0 = m_blk * TILE_M + (int)cta * CTA_M;
-        const int n0 = n_blk * TILE_N + (int)cta * HALF_N;
-        const int kb1 = min(num_kb, (ks + 1) * kb_per);
-        for (int kb = ks * kb_per; kb < kb1; ++kb) {
+        const Unit u = unit_of<MODE>(unit, num_tiles, tiles_m, tiles_n, num_kb, kb_per, grp);
+        const int m0 = u.m_blk * TILE_M + (int)cta * CTA_M;
+        const int n0 = u.n_blk * TILE_N + (int)cta * HALF_N;
+        int b_off = 0;
+        if constexpr (MODE == 3) b_off = grp.block_expert[u.m_blk * TILE_M / grp.block_rows] * grp.b_rows;
+        for (int kb = u.kb0; kb < u.kb1; ++kb) {
           mbar_wait(bar_empty + 8 * stage, phase ^ 1);
           const uint32_t full = bar_full + 8 * stage;          // same offset in the leader's smem
           if (leader) mbar_expect_tx(full, 2 * kStageBytes);
@@ -91,10 +125,10 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
             for (int j = 0; j < CTA_M / 64; ++j) tma_load_2d_2cta(sa + j * 8192, &tma_a, full, m0 + j * 64, k0);
           }
           if constexpr (B_KMAJOR) {
-            tma_load_2d_2cta(sb, &tma_b, full, k0, n0);                          // box {64 k, 128 n}
+            tma_load_2d_2cta(sb, &tma_b, full, k0, b_off + n0);                  // box {64 k, 128 n}
           } else {
 #pragma unroll
-            for (int j = 0; j < HALF_N / 64; ++j) tma_load_2d_2cta(sb + j * 8192, &tma_b, full, n0 + j * 64, k0);
+            for (int j = 0; j < HALF_N / 64; ++j) tma_load_2d_2cta(sb + j * 8192, &tma_b, full, n0 + j * 64, b_off + k0);
           }
           if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
@@ -107,11 +141,11 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       constexpr uint32_t idesc = make_idesc(!A_KMAJOR, !B_KMAJOR, TILE_M, TILE_N);
       int stage = 0; uint32_t phase = 0; int as = 0; uint32_t aphase = 0;
       for (int unit = pair; unit < num_units; unit += num_pairs) {
-        const int ks = unit / num_tiles;
+        const Unit u = unit_of<MODE>(unit, num_tiles, tiles_m, tiles_n, num_kb, kb_per, grp);
         mbar_wait(bar_tempty + 8 * as, aphase ^ 1);
         tcgen05_fence_after();
         const uint32_t tmem_d = tmem_base + as * TILE_N;
-        const int kb0 = ks * kb_per, kb1 = min(num_kb, (ks + 1) * kb_per);
+        const int kb0 = u.kb0, kb1 = u.kb1;
         for (int kb = kb0; kb < kb1; ++kb) {
           mbar_wait(bar_full + 8 * stage, phase);
           tcgen05_fence_after();
@@ -134,31 +168,32 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     // ===== epilogue (both CTAs; own 128 TMEM lanes) =====
     const int q = warp & 3;
     const uint32_t tempty_leader = mapa_shared(bar_tempty, 0);
-    const bool use_tma_store = sizeof(OutT) == 2 && !accumulate;     // fp32 / read-modify-write outputs keep direct stores
     const bool issuer = threadIdx.x == 64;
     uint32_t slab_ctr = 0;
     int as = 0; uint32_t aphase = 0;
     for (int unit = pair; unit < num_units; unit += num_pairs) {
-      const int tile = unit % num_tiles;
-      int m_blk, n_blk;
-      tile_coords(tile, tiles_m, tiles_n, m_blk, n_blk);
+      const Unit u = unit_of<MODE>(unit, num_tiles, tiles_m, tiles_n, num_kb, kb_per, grp);
       mbar_wait(bar_tfull + 8 * as, aphase);
       tcgen05_fence_after();
-      const int n0 = n_blk * TILE_N;
-      if (use_tma_store) {
-        epilogue_tile_tma(tmem_base + ((uint32_t)(q * 32) << 16) + as * TILE_N, smem_base + kEpiOffset, &tma_out,
-                          m_blk * TILE_M + (int)cta * CTA_M, n0, N, q, lane, issuer, slab_ctr);
+      const int n0 = u.n_blk * TILE_N, row0 = u.m_blk * TILE_M + (int)cta * CTA_M;
+      const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + as * TILE_N;
+      const bool empty = MODE == 4 && u.kb0 == u.kb1;
+      if constexpr (sizeof(OutT) == 4) {
+        epilogue_tile_tma_f32(acc, smem_base + kEpiOffset, &tma_out, row0, u.mat, n0, N, q, lane, issuer, slab_ctr,
+                              accumulate || split_k > 1, empty);
+      } else if (!accumulate) {
+        epilogue_tile_tma<MODE == 4>(acc, smem_base + kEpiOffset, &tma_out, row0, n0, N, q, lane, issuer, slab_ctr, u.mat, empty);
       } else {
-        const int row = m_blk * TILE_M + (int)cta * CTA_M + q * 32 + lane;
-        OutT* orow = out + (size_t)row * N;
+        const int row = row0 + q * 32 + lane;
+        OutT* orow = out + ((size_t)u.mat * M + row) * N;
         const bool row_ok = row < M;
 #pragma unroll 1
         for (int c = 0; c < TILE_N / 32; ++c) {
           uint32_t r[32];
-          tcgen05_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + as * TILE_N + c * 32, r);
+          tcgen05_ld_32x32(acc + c * 32, r);
           tcgen05_wait_ld();
           const int col0 = n0 + c * 32;
-          if (row_ok && col0 < N) store_chunk<OutT>(orow, col0, N, r, accumulate);
+          if (row_ok && col0 < N && !empty) store_chunk<OutT>(orow, col0, N, r, accumulate);
         }
       }
       tcgen05_fence_before();
@@ -675,17 +710,27 @@ gemm_bf16_2cta_tp_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
 CUtensorMap make_tmap_bf16(const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_cols, uint32_t box_rows);
 int device_sm_count();
 
-template <bool AK, bool BK_, typename OutT>
+CUtensorMap make_tmap_mats(const void* ptr, bool f32, uint64_t mats, uint64_t rows, uint64_t cols, uint32_t box_cols, uint32_t box_rows);
+
+template <bool AK, bool BK_, typename OutT, int MODE = 0>
 static void launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& to, void* out, int M, int N, int K,
-                    int accumulate, int split_k, int grid, cudaStream_t st) {
-  auto kern = g2::gemm_bf16_2cta_kernel<AK, BK_, OutT>;
+                    int accumulate, int split_k, const g2::Group& grp, int grid, cudaStream_t st) {
+  auto kern = g2::gemm_bf16_2cta_kernel<AK, BK_, OutT, MODE>;
   static bool configured = false;
   if (!configured) {
     NXD_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, g2::kSmem));
     configured = true;
   }
-  kern<<<grid, g2::kThreads, g2::kSmem, st>>>(ta, tb, to, (OutT*)out, M, N, K, accumulate, split_k);
+  kern<<<grid, g2::kThreads, g2::kSmem, st>>>(ta, tb, to, (OutT*)out, M, N, K, accumulate, split_k, grp);
   NXD_CUDA_CHECK(cudaGetLastError());
+}
+
+// Map of an output: fp32 slabs of 32 columns, bf16 slabs of 64; bf16 outputs that accumulate take no map (a dummy).
+static CUtensorMap out_map(const void* out, int out_dt, bool accumulate, bool mats, int groups, int M, int N, const CUtensorMap& dummy) {
+  if (out_dt == kF32) return make_tmap_mats(out, true, groups, M, N, 32, g2::CTA_M);
+  if (accumulate) return dummy;
+  if (N % 8) nxd_throw("CTA-pair GEMM: bf16 output needs N % 8 == 0", __FILE__, __LINE__);
+  return mats ? make_tmap_mats(out, false, groups, M, N, g2::kEpiSlabCols, g2::CTA_M) : make_tmap_bf16(out, M, N, g2::kEpiSlabCols, g2::CTA_M);
 }
 
 void gemm_bf16_2cta(const void* a, const void* b, void* out, int M, int N, int K, bool trans_a, bool trans_b, int out_dt,
@@ -693,46 +738,72 @@ void gemm_bf16_2cta(const void* a, const void* b, void* out, int M, int N, int K
   const bool AK = !trans_a, BK_ = trans_b;
   const CUtensorMap ta = AK ? make_tmap_bf16(a, M, K, g2::BK, g2::CTA_M) : make_tmap_bf16(a, K, M, 64, g2::BK);
   const CUtensorMap tb = BK_ ? make_tmap_bf16(b, N, K, g2::BK, g2::HALF_N) : make_tmap_bf16(b, K, N, 64, g2::BK);
-  // output map for the TMA-store epilogue (bf16, non-accumulating; needs a 16-byte row pitch) — otherwise a dummy
-  const bool tma_out_ok = out_dt == kBF16 && !accumulate && N % 8 == 0;
-  const CUtensorMap to = tma_out_ok ? make_tmap_bf16(out, M, N, g2::kEpiSlabCols, g2::CTA_M) : ta;
-  if (out_dt == kBF16 && !accumulate && !tma_out_ok) nxd_throw("gemm_bf16_2cta: bf16 output needs N % 8 == 0", __FILE__, __LINE__);
+  const CUtensorMap to = out_map(out, out_dt, accumulate, false, 1, M, N, ta);
   const int tiles = ((M + g2::TILE_M - 1) / g2::TILE_M) * ((N + g2::TILE_N - 1) / g2::TILE_N);
   const int pairs = device_sm_count() / 2;
   // Split-K for fp32 outputs (weight gradients): K = tokens is long while the output often has fewer tiles than the
-  // chip has CTA pairs (TP=8: 32-176 tiles on 74 pairs).  Pick the split that minimises waves/split with a small cost per
-  // extra partial (atomic epilogue traffic); every split keeps >= 16 k-blocks so the mainloop still amortises its epilogue.
+  // chip has CTA pairs (TP=8: 32-176 tiles on 74 pairs).  A split is taken where the waves it saves (0.39 us per k-block of a
+  // 256 x 256 tile) cost more than its traffic: zeroing the output first and one more pass over it per further partial, at
+  // 6 bytes/ps; every split keeps >= 16 k-blocks so that the main loop still amortises its epilogue.
   int split = 1;
   const char* split_env = getenv("NXD_GEMM_SPLITK");            // re-read per call: A/B sweeps toggle it at run time
   const bool split_enabled = !(split_env && split_env[0] == '0');
   const int num_kb = (K + g2::BK - 1) / g2::BK;
-  if (out_dt == kF32 && split_enabled && N % 4 == 0) {
-    double best = (double)((tiles + pairs - 1) / pairs);
+  if (out_dt == kF32 && split_enabled) {
+    const double pass_us = (double)M * N * 4 / 6e6;
+    double best = (double)((tiles + pairs - 1) / pairs) * num_kb * 0.39;
     for (int s2 = 2; s2 <= 8; ++s2) {
       if (num_kb / s2 < 16) break;
       const int per = (num_kb + s2 - 1) / s2;
       if (per * (s2 - 1) >= num_kb) continue;                       // would leave an empty split
-      const double cost = (double)((tiles * s2 + pairs - 1) / pairs) / s2 * (1.0 + 0.04 * (s2 - 1));
-      if (cost < best - 1e-9) { best = cost; split = s2; }
+      const double cost = (double)((tiles * s2 + pairs - 1) / pairs) * per * 0.39 + (s2 - 1) * pass_us + (accumulate ? 0. : pass_us);
+      if (cost < best) { best = cost; split = s2; }
     }
   }
-  int acc_mode = accumulate ? 1 : 0;
-  if (split > 1) {
-    if (!accumulate) NXD_CUDA_CHECK(cudaMemsetAsync(out, 0, (size_t)M * N * sizeof(float), st));   // partials add into zeros
-    acc_mode = 2;
-  }
+  if (split > 1 && !accumulate) NXD_CUDA_CHECK(cudaMemsetAsync(out, 0, (size_t)M * N * sizeof(float), st));   // partials add into zeros
   const int units = tiles * split;
   const int grid = 2 * (units < pairs ? units : pairs);
+  const g2::Group none{};
 #define NXD_L2(AKv, BKv)                                                                          \
   do {                                                                                            \
-    if (out_dt == kBF16) launch2<AKv, BKv, __nv_bfloat16>(ta, tb, to, out, M, N, K, acc_mode, split, grid, st); \
-    else launch2<AKv, BKv, float>(ta, tb, to, out, M, N, K, acc_mode, split, grid, st);          \
+    if (out_dt == kBF16) launch2<AKv, BKv, __nv_bfloat16>(ta, tb, to, out, M, N, K, accumulate, split, none, grid, st); \
+    else launch2<AKv, BKv, float>(ta, tb, to, out, M, N, K, accumulate, split, none, grid, st);   \
   } while (0)
   if (AK && BK_) NXD_L2(true, true);
   else if (AK && !BK_) NXD_L2(true, false);
   else if (!AK && !BK_) NXD_L2(false, false);
   else NXD_L2(false, true);
 #undef NXD_L2
+}
+
+// Grouped GEMMs of routed experts whose row blocks are multiples of 256 rows (see grouped_gemm_bf16 / grouped_wgrad_bf16).
+void grouped_gemm_bf16_2cta(const void* a, const void* b, void* out, int M, int N, int K, int E, bool trans_b, const int* block_expert,
+                            const int* used_blocks, int block_rows, int out_dt, cudaStream_t st) {
+  const CUtensorMap ta = make_tmap_bf16(a, M, K, g2::BK, g2::CTA_M);
+  const CUtensorMap tb = trans_b ? make_tmap_bf16(b, (uint64_t)E * N, K, g2::BK, g2::HALF_N) : make_tmap_bf16(b, (uint64_t)E * K, N, 64, g2::BK);
+  const CUtensorMap to = out_map(out, out_dt, false, false, 1, M, N, ta);
+  const g2::Group grp{block_expert, nullptr, used_blocks, block_rows, trans_b ? N : K, E};
+  const int tiles = ((M + g2::TILE_M - 1) / g2::TILE_M) * ((N + g2::TILE_N - 1) / g2::TILE_N), pairs = device_sm_count() / 2;
+  const int grid = 2 * (tiles < pairs ? tiles : pairs);
+  if (trans_b) {
+    if (out_dt == kBF16) launch2<true, true, __nv_bfloat16, 3>(ta, tb, to, out, M, N, K, 0, 1, grp, grid, st);
+    else launch2<true, true, float, 3>(ta, tb, to, out, M, N, K, 0, 1, grp, grid, st);
+  } else {
+    if (out_dt == kBF16) launch2<true, false, __nv_bfloat16, 3>(ta, tb, to, out, M, N, K, 0, 1, grp, grid, st);
+    else launch2<true, false, float, 3>(ta, tb, to, out, M, N, K, 0, 1, grp, grid, st);
+  }
+}
+
+void grouped_wgrad_bf16_2cta(const void* a, const void* b, void* out, int rows_total, int Mo, int No, int E, const int* seg_first_block,
+                             int block_rows, int out_dt, bool accumulate, cudaStream_t st) {
+  const CUtensorMap ta = make_tmap_bf16(a, rows_total, Mo, 64, g2::BK);
+  const CUtensorMap tb = make_tmap_bf16(b, rows_total, No, 64, g2::BK);
+  const CUtensorMap to = out_map(out, out_dt, accumulate, true, E, Mo, No, ta);
+  const g2::Group grp{nullptr, seg_first_block, nullptr, block_rows, 0, E};
+  const int tiles = E * ((Mo + g2::TILE_M - 1) / g2::TILE_M) * ((No + g2::TILE_N - 1) / g2::TILE_N), pairs = device_sm_count() / 2;
+  const int grid = 2 * (tiles < pairs ? tiles : pairs);
+  if (out_dt == kBF16) launch2<false, false, __nv_bfloat16, 4>(ta, tb, to, out, Mo, No, rows_total, accumulate, 1, grp, grid, st);
+  else launch2<false, false, float, 4>(ta, tb, to, out, Mo, No, rows_total, accumulate, 1, grp, grid, st);
 }
 
 

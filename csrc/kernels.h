@@ -99,7 +99,11 @@ void gemm_fp8(const void* a, const void* b, void* out, int M, int N, int K, cons
               cudaStream_t st);
 // ---- grouped (MoE blockwise) GEMMs, gemm_sm100.cu
 void grouped_gemm_bf16(const void* a, const void* b, void* out, int M, int N, int K, int E, bool trans_b,
-                       const int* block_expert, int block_rows, int out_dt, cudaStream_t st);
+                       const int* block_expert, const int* used_blocks, int block_rows, int out_dt, cudaStream_t st);
+void grouped_gemm_bf16_2cta(const void* a, const void* b, void* out, int M, int N, int K, int E, bool trans_b, const int* block_expert,
+                            const int* used_blocks, int block_rows, int out_dt, cudaStream_t st);
+void grouped_wgrad_bf16_2cta(const void* a, const void* b, void* out, int rows_total, int Mo, int No, int E, const int* seg_first_block,
+                             int block_rows, int out_dt, bool accumulate, cudaStream_t st);
 void grouped_wgrad_bf16(const void* a, const void* b, void* out, int rows_total, int Mo, int No, int E,
                         const int* seg_first_block, int block_rows, int out_dt, bool accumulate, cudaStream_t st);
 

@@ -84,7 +84,7 @@ def linear_nt(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
 
 # ---------------------------------------------------------------------------------------------------------------------
 # Grouped (MoE blockwise) GEMM: rows of ``x`` come in ``block_size``-row blocks, block i is multiplied by the weights of
-# expert ``block_to_expert[i]``.  CUDA: MODE 3/4 of ``csrc/gemm_sm100.cu`` (the per-block expert only shifts the TMA
+# expert ``block_to_expert[i]``.  CUDA: MODE 3 / 4 of ``csrc/gemm2cta_sm100.cu`` (the per-block expert only shifts the TMA
 # coordinate of the weight tile — no per-block weight copies, no host sync); CPU / odd shapes: plain loop.
 # Role of the reference's blockwise NKI kernels (modules/moe/blockwise.py:180-468, 1037-1127).
 def _grouped_ok(x: torch.Tensor, w: torch.Tensor, block_size: int) -> bool:
@@ -102,11 +102,11 @@ def _grouped_ref(x, w, b2e, block_size):
 
 class _GroupedMatmul(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, w, b2e, seg_first_block, block_size):
+    def forward(ctx, x, w, b2e, seg_first_block, block_size, skip_unused):
         ctx.save_for_backward(x, w, b2e, seg_first_block)
-        ctx.block_size = block_size
+        ctx.block_size, ctx.skip_unused = block_size, skip_unused
         _ext.count_launch()
-        return _ext.ext().grouped_gemm(x.contiguous(), w.contiguous(), b2e, block_size, False)
+        return _ext.ext().grouped_gemm(x.contiguous(), w.contiguous(), b2e, block_size, False, seg_first_block if skip_unused else None)
 
     @staticmethod
     def backward(ctx, gy):
@@ -115,7 +115,7 @@ class _GroupedMatmul(torch.autograd.Function):
         gx = gw = None
         if ctx.needs_input_grad[0]:
             _ext.count_launch()
-            gx = _ext.ext().grouped_gemm(gy, w.contiguous(), b2e, ctx.block_size, True)       # dy · W[e]ᵀ
+            gx = _ext.ext().grouped_gemm(gy, w.contiguous(), b2e, ctx.block_size, True, seg if ctx.skip_unused else None)       # dy · W[e]ᵀ
         if ctx.needs_input_grad[1]:
             _ext.count_launch()
             mg = getattr(w, "main_grad", None)
@@ -129,12 +129,13 @@ class _GroupedMatmul(torch.autograd.Function):
             else:
                 gw = torch.empty_like(w)
                 _ext.ext().grouped_wgrad(x.contiguous(), gy, gw, seg, ctx.block_size, False)
-        return gx, gw, None, None, None
+        return gx, gw, None, None, None, None
 
 
 def grouped_matmul(x: torch.Tensor, w: torch.Tensor, block_to_expert: torch.Tensor, seg_first_block: torch.Tensor,
-                   block_size: int) -> torch.Tensor:
-    """``y[i·B:(i+1)·B] = x[i·B:(i+1)·B] @ w[block_to_expert[i]]`` with ``x [nb·B, K]``, ``w [E, K, N]``."""
+                   block_size: int, skip_unused: bool = False) -> torch.Tensor:
+    """``y[i·B:(i+1)·B] = x[i·B:(i+1)·B] @ w[block_to_expert[i]]`` with ``x [nb·B, K]``, ``w [E, K, N]``.  With ``skip_unused``
+    the row blocks from ``seg_first_block[E]`` on hold no tokens: their rows of the result are unspecified."""
     if _grouped_ok(x, w, block_size):
-        return _GroupedMatmul.apply(x, w, block_to_expert.int(), seg_first_block.int(), block_size)
+        return _GroupedMatmul.apply(x, w, block_to_expert.int(), seg_first_block.int(), block_size, skip_unused)
     return _grouped_ref(x, w, block_to_expert, block_size)

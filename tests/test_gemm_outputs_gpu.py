@@ -1,0 +1,39 @@
+"""fp32 GEMM outputs at the edges of their tiles: stored, accumulated, and split over the tokens."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("tokens,M,N,accumulate", [(64, 256, 8, False), (136, 264, 40, True), (1000, 520, 264, False), (4096, 512, 1032, True),
+                                                   (4096, 4096, 4096, False)])
+def test_weight_gradients_in_fp32(tokens, M, N, accumulate):
+    from neuronx_distributed_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    dy, x = (torch.randn(tokens, n, generator=g, device="cuda").bfloat16() for n in (M, N))
+    out = torch.randn(M + 1, N, generator=g, device="cuda")
+    guard, want = out[M].clone(), dy.double().t() @ x.double() + (out[:M].double() if accumulate else 0)
+    ops.gemm.matmul(dy, x, True, False, out=out[:M], accumulate=accumulate)
+    # exact products, fp32 sums over `tokens` terms
+    assert (out[:M].double() - want).abs().max() <= 2.0 ** -22 * tokens * dy.float().abs().max() * x.float().abs().max()
+    assert torch.equal(out[M], guard)
+
+
+@pytest.mark.parametrize("M,N,counts", [(64, 128, [1, 0, 3]), (320, 192, [2, 2, 0, 0]), (256, 64, [0, 5])])
+@pytest.mark.parametrize("dtype,accumulate", [(torch.bfloat16, False), (torch.float32, False), (torch.float32, True)])
+def test_grouped_weight_gradients(M, N, counts, dtype, accumulate):
+    from neuronx_distributed_b200 import ops
+
+    g, block = torch.Generator(device="cuda").manual_seed(M), 128
+    seg = torch.cumsum(torch.tensor([0] + counts), 0).int()
+    rows = int(seg[-1]) * block + 256
+    x, dy = (torch.randn(rows, n, generator=g, device="cuda").bfloat16() for n in (M, N))
+    out = torch.randn(len(counts), M, N, generator=g, device="cuda").to(dtype)
+    want = out.double() if accumulate else torch.zeros(out.shape, device="cuda", dtype=torch.double)
+    for e in range(len(counts)):
+        a, b = int(seg[e]) * block, int(seg[e + 1]) * block
+        want[e] += x[a:b].double().t() @ dy[a:b].double()
+    ops._ext.ext().grouped_wgrad(x, dy, out, seg.cuda(), block, accumulate)
+    # fp32 sums as above; one rounding to bfloat16 (2^-9) of the result
+    assert (out.double() - want).abs().max() <= (2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -16) * max(1.0, want.abs().max())
