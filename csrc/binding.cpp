@@ -217,6 +217,58 @@ static py::tuple moe_block_metadata(const Tensor& expert_index, int64_t num_expe
   return py::make_tuple(b2e, tp2id, counts);
 }
 
+// expert_index [T, k] int64 → int32 (expert of each row block [nb], token of each slot [nb*B] (-1 = padding), block prefix sums [E+1],
+// slot of each choice [T*k])
+static py::tuple moe_slots(const Tensor& expert_index, int64_t num_experts, int64_t block_size, int64_t num_blocks) {
+  CHECK_IN(expert_index);
+  TORCH_CHECK(expert_index.dim() == 2 && expert_index.scalar_type() == at::kLong && num_blocks * block_size < (1ll << 31));
+  c10::cuda::CUDAGuard g(expert_index.device());
+  auto o = expert_index.options().dtype(at::kInt);
+  auto b2e = at::empty({num_blocks}, o), token = at::empty({num_blocks * block_size}, o), seg = at::empty({num_experts + 1}, o);
+  auto slot = at::empty({expert_index.numel()}, o);
+  nxd::moe_slots(expert_index.data_ptr<long>(), expert_index.numel(), (int)expert_index.size(1), (int)num_experts, (int)block_size,
+                 (int)num_blocks, b2e.data_ptr<int>(), token.data_ptr<int>(), seg.data_ptr<int>(), slot.data_ptr<int>(), stream());
+  return py::make_tuple(b2e, token, seg, slot);
+}
+#define CHECK_MOE_ROWS(x) TORCH_CHECK((x).is_cuda() && (x).is_contiguous() && (x).scalar_type() == at::kBFloat16 && (x).dim() == 2 && (x).size(1) % 8 == 0 && (uintptr_t)(x).data_ptr() % 16 == 0)
+#define CHECK_MOE_INTS(x) TORCH_CHECK((x).is_cuda() && (x).is_contiguous() && (x).scalar_type() == at::kInt)
+static Tensor moe_gather(const Tensor& x, const Tensor& slot_token, const Tensor& seg, int64_t block_size) {
+  CHECK_MOE_ROWS(x); CHECK_MOE_INTS(slot_token); CHECK_MOE_INTS(seg);
+  c10::cuda::CUDAGuard g(x.device());
+  auto out = at::empty({slot_token.numel(), x.size(1)}, x.options());
+  nxd::moe_gather(x.data_ptr(), slot_token.data_ptr<int>(), seg.data_ptr<int>() + seg.numel() - 1, out.data_ptr(), (int)x.size(1),
+                  (int)block_size, (int)slot_token.numel(), stream());
+  return out;
+}
+static Tensor moe_combine(const Tensor& y, const Tensor& slot_of, const Tensor& expert_index, const c10::optional<Tensor>& w) {
+  CHECK_MOE_ROWS(y); CHECK_MOE_INTS(slot_of);
+  CHECK_IN(expert_index);
+  TORCH_CHECK(expert_index.dim() == 2 && expert_index.scalar_type() == at::kLong && slot_of.numel() == expert_index.numel());
+  const float* wp = nullptr;
+  int E = 0;
+  if (w.has_value()) {
+    TORCH_CHECK(w->is_contiguous() && w->scalar_type() == at::kFloat && w->dim() == 2 && w->size(0) == expert_index.size(0));
+    wp = w->data_ptr<float>(); E = (int)w->size(1);
+  }
+  c10::cuda::CUDAGuard g(y.device());
+  auto out = at::empty({expert_index.size(0), y.size(1)}, y.options());
+  nxd::moe_combine(y.data_ptr(), slot_of.data_ptr<int>(), expert_index.data_ptr<long>(), wp, out.data_ptr(), (int)expert_index.size(0),
+                   (int)y.size(1), E, (int)expert_index.size(1), stream());
+  return out;
+}
+static py::tuple moe_combine_grad(const Tensor& g, const Tensor& y, const Tensor& slot_token, const Tensor& block_expert, const Tensor& seg,
+                                  const Tensor& w, int64_t block_size) {
+  CHECK_MOE_ROWS(g); CHECK_MOE_ROWS(y); CHECK_MOE_INTS(slot_token); CHECK_MOE_INTS(block_expert); CHECK_MOE_INTS(seg);
+  TORCH_CHECK(w.is_contiguous() && w.scalar_type() == at::kFloat && w.dim() == 2 && w.size(0) == g.size(0) && w.size(1) == seg.numel() - 1);
+  TORCH_CHECK(y.size(0) == slot_token.numel() && y.size(1) == g.size(1) && block_expert.numel() * block_size == slot_token.numel());
+  c10::cuda::CUDAGuard guard(g.device());
+  auto dy = at::empty_like(y), dw = at::zeros_like(w);
+  nxd::moe_combine_grad(g.data_ptr(), y.data_ptr(), slot_token.data_ptr<int>(), block_expert.data_ptr<int>(),
+                        seg.data_ptr<int>() + seg.numel() - 1, w.data_ptr<float>(), dy.data_ptr(), dw.data_ptr<float>(), (int)y.size(1),
+                        (int)w.size(1), (int)block_size, (int)slot_token.numel(), stream());
+  return py::make_tuple(dy, dw);
+}
+
 // q [B,1,H,D], k/v [B,1,Hkv,D] (views of the fused QKV GEMV output), cache [B,L,Hkv,D]: rotate q → new tensor, rotate k and
 // copy v straight into the cache row positions[b]
 static Tensor decode_rope_kv(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& positions, const Tensor& cos_t,
@@ -793,6 +845,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   });
   m.def("decode_rope_kv", &decode_rope_kv);
   m.def("moe_block_metadata", &moe_block_metadata);
+  m.def("moe_slots", &moe_slots);
+  m.def("moe_gather", &moe_gather);
+  m.def("moe_combine", &moe_combine);
+  m.def("moe_combine_grad", &moe_combine_grad);
   m.def("row_argmax", &row_argmax);
   m.def("row_topk", &row_topk);
   m.def("row_topk_supported", &row_topk_supported);

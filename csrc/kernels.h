@@ -119,6 +119,13 @@ void row_topk(const void* x, float* vals, long* idxs, int rows, int V, int k, lo
 
 void moe_block_metadata(const void* expert_index, bool idx64, long n, int k, int E, int B, int nb, long* block_to_expert, long* tp2id,
                         long* counts, cudaStream_t st);
+void moe_slots(const long* expert_index, long n, int k, int E, int B, int nb, int* block_expert, int* slot_token, int* seg, int* slot_of,
+               cudaStream_t st);
+void moe_gather(const void* x, const int* slot_token, const int* used_blocks, void* out, int H, int B, int rows, cudaStream_t st);
+void moe_combine(const void* y, const int* slot_of, const long* expert_index, const float* w, void* out, int T, int H, int E, int k,
+                 cudaStream_t st);
+void moe_combine_grad(const void* g, const void* y, const int* slot_token, const int* block_expert, const int* used_blocks, const float* w,
+                      void* dy, float* dw, int H, int E, int B, int rows, cudaStream_t st);
 
 // ---- decode-time MoE block in one cooperative launch (moe_tkg.cu)
 bool moe_block_tkg_supported(int T, int H, int E, int I, int K);

@@ -113,81 +113,3 @@ void row_topk(const void* x, float* vals, long* idxs, int rows, int V, int k, lo
 }
 
 }  // namespace nxd
-
-// =====================================================================================================================
-// MoE block-metadata build (role of the reference's `find_nonzero_indices` / `indexed_flatten` NKI kernels K9,
-// modules/moe/expert_mlps_v2.py:1079-1206): from the routed expert ids [T, k] produce, in ONE launch and without a sort,
-//   tokens_per_expert [E], block_to_expert [nb], token_position_to_id [nb * B]  (-1 = padding)
-// with every expert's tokens in ascending token order (the stable order of the torch.argsort-based path it replaces).
-// One CTA of 1024 threads: smem histogram → per-expert block ranges → chunked stable scatter (warp match + cross-warp prefix).
-namespace nxd {
-namespace {
-
-constexpr int kMoeThreads = 1024;
-constexpr int kMoeMaxExperts = 256;
-
-template <typename IdxT>
-__global__ void __launch_bounds__(kMoeThreads) moe_block_metadata_kernel(const IdxT* __restrict__ expert_index, long n, int k, int E,
-                                                                         int B, int nb, long* __restrict__ block_to_expert,
-                                                                         long* __restrict__ tp2id, long* __restrict__ counts_out) {
-  __shared__ int counts[kMoeMaxExperts];
-  __shared__ int base[kMoeMaxExperts];
-  __shared__ int wc[32][kMoeMaxExperts];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (int e = tid; e < E; e += kMoeThreads) counts[e] = 0;
-  for (long s = tid; s < (long)nb * B; s += kMoeThreads) tp2id[s] = -1;
-  __syncthreads();
-  for (long i = tid; i < n; i += kMoeThreads) {
-    const int e = (int)expert_index[i];
-    if (e >= 0 && e < E) atomicAdd(&counts[e], 1);
-  }
-  __syncthreads();
-  if (tid == 0) {
-    int blk = 0;
-    for (int e = 0; e < E; ++e) {
-      const int nblk = (counts[e] + B - 1) / B;
-      base[e] = blk * B;                               // first slot of expert e
-      for (int b = blk; b < blk + nblk && b < nb; ++b) block_to_expert[b] = e;
-      blk += nblk;
-    }
-    for (int b = blk; b < nb; ++b) block_to_expert[b] = E - 1;        // unused tail blocks (all padding)
-  }
-  for (int e = tid; e < E; e += kMoeThreads) counts_out[e] = counts[e];
-  __syncthreads();
-  for (long chunk = 0; chunk < n; chunk += kMoeThreads) {
-    for (int j = tid; j < 32 * E; j += kMoeThreads) wc[j / E][j % E] = 0;
-    __syncthreads();
-    const long i = chunk + tid;
-    int e = -1;
-    if (i < n) { e = (int)expert_index[i]; if (e < 0 || e >= E) e = -1; }
-    const unsigned mask = __match_any_sync(0xffffffffu, e);
-    const int rank_in_warp = __popc(mask & ((1u << lane) - 1u));
-    if (e >= 0 && rank_in_warp == 0) wc[warp][e] = __popc(mask);
-    __syncthreads();
-    if (e >= 0) {
-      int before = 0;
-      for (int w = 0; w < warp; ++w) before += wc[w][e];
-      const long slot = (long)base[e] + before + rank_in_warp;
-      if (slot < (long)nb * B) tp2id[slot] = i / k;
-    }
-    __syncthreads();
-    for (int ee = tid; ee < E; ee += kMoeThreads) {
-      int tot = 0;
-      for (int w = 0; w < 32; ++w) tot += wc[w][ee];
-      base[ee] += tot;
-    }
-    __syncthreads();
-  }
-}
-
-}  // namespace
-
-void moe_block_metadata(const void* expert_index, bool idx64, long n, int k, int E, int B, int nb, long* block_to_expert, long* tp2id,
-                        long* counts, cudaStream_t st) {
-  if (E > kMoeMaxExperts) nxd_throw("moe_block_metadata: at most 256 experts", __FILE__, __LINE__);
-  if (idx64) moe_block_metadata_kernel<long><<<1, kMoeThreads, 0, st>>>((const long*)expert_index, n, k, E, B, nb, block_to_expert, tp2id, counts);
-  else moe_block_metadata_kernel<int><<<1, kMoeThreads, 0, st>>>((const int*)expert_index, n, k, E, B, nb, block_to_expert, tp2id, counts);
-  NXD_CUDA_CHECK(cudaGetLastError());
-}
-
-}  // namespace nxd

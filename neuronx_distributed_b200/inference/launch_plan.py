@@ -51,7 +51,8 @@ _EXT_RESOURCE_PREFIXES = ("vmm_", "symm_", "tp_gemm", "nvls_", "gemv_allreduce",
 # writing to EVERY tensor argument: conservative — such tensors count as state, are never hoisted or dropped — but safe.
 _EXT_PURE = frozenset({"rmsnorm_fwd", "rmsnorm_bwd", "add_rmsnorm_fwd", "add_rmsnorm_bwd", "swiglu_fwd", "swiglu_bwd", "rope_apply",
                        "ce_stats", "ce_backward", "decode_attention", "decode_attention_partial", "gemv", "gemv_mx",
-                       "gemm_mxfp8", "moe_block_tkg", "moe_block_metadata", "row_argmax", "row_topk", "flash_attn_fwd",
+                       "gemm_mxfp8", "moe_block_tkg", "moe_block_metadata", "moe_slots", "moe_gather", "moe_combine",
+                       "moe_combine_grad", "row_argmax", "row_topk", "flash_attn_fwd",
                        "flash_attn_bwd", "moe_block_tkg_supported", "row_topk_supported", "grouped_gemm"})
 # … and the ones that write exactly these positional arguments (everything else they take is read-only)
 _EXT_WRITES = {"gemm_bf16": (2,), "gemm_bf16_2cta": (2,), "gemm_fp8": (2,), "grouped_wgrad": (2,), "decode_rope_kv": (6, 7),

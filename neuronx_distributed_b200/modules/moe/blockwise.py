@@ -9,7 +9,7 @@ of ``block_size`` and each block is multiplied by exactly one expert's weights:
     token_position_to_id  : flat [num_blocks·B] token id feeding each block slot (−1 = padding)
 
 On CUDA the two projections are grouped tcgen05 GEMMs (``ops.gemm.grouped_matmul`` → MODE 3/4 of
-``csrc/gemm_sm100.cu``): the block's expert only shifts the TMA coordinate of the weight tile, the backward runs the
+``csrc/gemm2cta_sm100.cu``): the block's expert only shifts the TMA coordinate of the weight tile, the backward runs the
 grouped dgrad and a per-expert segmented wgrad, and nothing syncs with the host.  On CPU it is a gathered einsum.
 """
 from __future__ import annotations
@@ -19,6 +19,7 @@ from dataclasses import dataclass
 from typing import Any, Optional, Tuple
 
 import torch
+import torch.nn.functional as F
 
 from .moe_configs import (  # noqa: F401  (re-exported here as in the reference, blockwise.py:83-87)
     ActFnType,
@@ -101,14 +102,45 @@ def blockwise_mlp_from_metadata(hidden: torch.Tensor, expert_affinities_masked: 
     return out
 
 
+def _grouped_swiglu_ok(hidden: torch.Tensor, expert_index: torch.Tensor, experts, num_experts: int) -> bool:
+    """silu-gated experts without clamps or biases on the grouped kernels: what ``_grouped_swiglu`` computes."""
+    from ... import ops
+
+    if not (experts.glu_mlp and experts.glu_type == "glu" and experts.act is F.silu):
+        return False
+    if any(c is not None for c in (experts.gc_hi, experts.gc_lo, experts.uc_hi, experts.uc_lo)):
+        return False
+    up, down = experts.gate_up_proj, experts.down_proj
+    if up.bias is not None or down.bias is not None or up.weight.shape[0] != num_experts:
+        return False
+    return (ops.moe_blocks.usable(hidden, expert_index, num_experts) and up.weight.shape[2] % 16 == 0
+            and ops.gemm._grouped_ok(hidden, up.weight, ops.moe_blocks.BLOCK) and ops.gemm._grouped_ok(hidden, down.weight, ops.moe_blocks.BLOCK))
+
+
+def _grouped_swiglu(hidden: torch.Tensor, expert_affinities: torch.Tensor, expert_index: torch.Tensor, experts, num_experts: int) -> torch.Tensor:
+    """The dropless computation on kernels of its own: rows are copied to expert order once, both projections are grouped GEMMs
+    over blocks of 256 rows (blocks without tokens are skipped), and each token sums its choices in fp32."""
+    from ... import ops
+
+    mb = ops.moe_blocks
+    T, k = expert_index.shape
+    slots = mb.make_slots(expert_index, num_experts, get_num_blocks(T, k, num_experts, mb.BLOCK))
+    x = mb.gather(hidden, slots)
+    h = ops.gemm.grouped_matmul(x, experts.gate_up_proj.weight, slots.block_expert, slots.seg, mb.BLOCK, skip_unused=True)
+    y = ops.gemm.grouped_matmul(ops.act.swiglu(h), experts.down_proj.weight, slots.block_expert, slots.seg, mb.BLOCK, skip_unused=True)
+    return mb.combine(y, expert_affinities.float(), slots)
+
+
 def blockwise_expert_mlp(hidden: torch.Tensor, expert_affinities: torch.Tensor, expert_index: torch.Tensor,
                          experts, block_size: int, normalize: bool = False) -> torch.Tensor:
     """Dropless MoE MLP: ``out[t] = Σ_j aff[t, e_j] · MLP_{e_j}(hidden[t])``."""
     E = expert_affinities.shape[-1]
-    b2e, tp2id, _ = build_block_metadata(expert_index, E, block_size)
     if normalize:
         denom = expert_affinities.gather(1, expert_index).sum(-1, keepdim=True).clamp(min=1e-9)
         expert_affinities = expert_affinities / denom
+    if _grouped_swiglu_ok(hidden, expert_index, experts, E):
+        return _grouped_swiglu(hidden, expert_affinities, expert_index, experts, E)
+    b2e, tp2id, _ = build_block_metadata(expert_index, E, block_size)
     proj = experts.gate_up_proj if experts.glu_mlp else experts.up_proj
     return blockwise_mlp_from_metadata(hidden, expert_affinities, proj.weight, experts.down_proj.weight, tp2id, b2e, block_size,
                                        experts.activation, proj.bias,

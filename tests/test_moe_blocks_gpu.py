@@ -1,0 +1,80 @@
+"""Routed experts on the block kernels against plain PyTorch."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _experts(E, H, I):
+    import torch.distributed as dist
+
+    from neuronx_distributed_b200.modules.moe import ExpertMLPsV2, RoutedExpertsMLPOpsConfig
+    from neuronx_distributed_b200.parallel_layers import parallel_state as ps
+
+    if not dist.is_initialized():
+        dist.init_process_group("gloo", store=dist.HashStore(), rank=0, world_size=1)
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_model_parallel(tensor_model_parallel_size=1)
+    cfg = RoutedExpertsMLPOpsConfig(num_experts=E, top_k=2, hidden_size=H, intermediate_size=I, hidden_act="silu", glu_mlp=True,
+                                    capacity_factor=None, normalize_top_k_affinities=False)
+    return ExpertMLPsV2(cfg, dtype=torch.bfloat16, device="cuda").train()
+
+
+def _reference(x, aff, idx, w1, w2):
+    out = torch.zeros_like(x)
+    for j in range(idx.shape[1]):
+        for e in range(w1.shape[0]):
+            rows = (idx[:, j] == e).nonzero().squeeze(1)
+            gate, up = (x[rows] @ w1[e]).chunk(2, -1)
+            out = out.index_add(0, rows, (torch.nn.functional.silu(gate) * up) @ w2[e] * aff[rows, e].unsqueeze(1))
+    return out
+
+
+@pytest.mark.parametrize("T,E,H,I,choice", [(37, 8, 256, 192, "random"), (512, 4, 128, 64, "one expert"), (1025, 3, 320, 128, "random"),
+                                            (700, 16, 128, 128, "twice"), (3000, 130, 64, 64, "random")])
+def test_experts(T, E, H, I, choice):
+    from neuronx_distributed_b200.modules.moe import blockwise
+
+    m = _experts(E, H, I)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, H, generator=g, device="cuda").bfloat16().requires_grad_()
+    aff = torch.rand(T, E, generator=g, device="cuda").requires_grad_()
+    idx = torch.stack([torch.randperm(E, generator=g, device="cuda")[:2] for _ in range(T)])
+    if choice == "one expert":                              # the others get no tokens: zero weight gradients
+        idx[:] = torch.tensor([1, 2], device="cuda")
+    if choice == "twice":
+        idx[:, 1] = idx[:, 0]
+    w1, w2 = m.mlp_op.gate_up_proj.weight, m.mlp_op.down_proj.weight
+    with torch.no_grad():
+        for w in (w1, w2):
+            w.copy_(torch.randn(w.shape, generator=g, device="cuda") * w.shape[1] ** -0.5)
+    go = torch.randn(T, H, generator=g, device="cuda").bfloat16()
+    assert blockwise._grouped_swiglu_ok(x, idx, m.mlp_op, E)
+    y = blockwise.blockwise_expert_mlp(x, aff, idx, m.mlp_op, 512)
+    got = [y, *torch.autograd.grad(y, (x, aff, w1, w2), go)]
+    ref = [t.detach().double().requires_grad_() for t in (x, aff, w1, w2)]
+    z = _reference(ref[0], ref[1], idx, ref[2], ref[3])
+    want = [z, *torch.autograd.grad(z, ref, go.double())]
+    # inputs of every product are rounded to bfloat16 once (2^-9), two to three in a row on each path
+    for a, b in zip(got, want):
+        assert (a.double() - b).norm() <= 0.012 * b.norm()
+    for e in range(E):
+        if not (idx == e).any():
+            assert not got[3][e].any() and not got[4][e].any()
+
+
+@pytest.mark.parametrize("n,E,block", [(1, 1, 128), (1023, 5, 256), (1025, 256, 128), (70000, 33, 256)])
+def test_slots(n, E, block):
+    from neuronx_distributed_b200 import ops
+    from neuronx_distributed_b200.modules.moe.blockwise import build_block_metadata, get_num_blocks
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    idx = torch.randint(0, E, (n, 1), generator=g, device="cuda")
+    s = ops.moe_blocks.make_slots(idx, E, get_num_blocks(n, 1, E, block), block)
+    b2e, tp2id, counts = build_block_metadata(idx.cpu(), E, block)
+    assert torch.equal(s.token.cpu().long(), tp2id) and torch.equal(s.block_expert.cpu().long(), b2e)
+    assert torch.equal(s.token[s.slot.long()].cpu().long(), torch.arange(n))
+    first = torch.cat([torch.zeros(1, dtype=torch.long), torch.cumsum((counts + block - 1) // block, 0)])
+    assert torch.equal(s.seg.cpu().long(), first)
+    for a, b in zip(build_block_metadata(idx, E, block), (b2e, tp2id, counts)):
+        assert torch.equal(a.cpu(), b)
