@@ -555,6 +555,17 @@ static void gemm_bf16(const Tensor& a, const Tensor& b, Tensor out, bool trans_a
                  nullptr, stream());
 }
 
+// y [M, N] = x [M, K] · w [N, K]ᵀ for 1 <= M <= 256 rows; split: blocks per 128 rows of w (0 = by rule)
+static Tensor gemm_few_rows(const Tensor& x, const Tensor& w, int64_t split) {
+  CHECK_IN(x); CHECK_IN(w);
+  TORCH_CHECK(x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 && x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1));
+  TORCH_CHECK(split == 0 || split == 1 || split == 2 || split == 4 || split == 8);
+  c10::cuda::CUDAGuard g(x.device());
+  Tensor y = at::empty({x.size(0), w.size(0)}, x.options());
+  nxd::gemm_few_rows(x.data_ptr(), w.data_ptr(), nullptr, y.data_ptr(), (int)x.size(0), (int)w.size(0), (int)x.size(1), (int)split, stream());
+  return y;
+}
+
 static void gemm_bf16_2cta(const Tensor& a, const Tensor& b, Tensor out, bool trans_a, bool trans_b, bool accumulate) {
   CHECK_IN(a); CHECK_IN(b); CHECK_IN(out);
   TORCH_CHECK(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16 && a.dim() == 2 && b.dim() == 2);
@@ -854,6 +865,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("row_topk_supported", &row_topk_supported);
   m.def("gemv", &gemv, py::arg("x"), py::arg("w"), py::arg("residual") = py::none());
   m.def("gemm_fp8", &gemm_fp8);
+  m.def("gemm_few_rows", &gemm_few_rows, py::arg("x"), py::arg("w"), py::arg("split") = 0);
   m.def("grouped_gemm", &grouped_gemm, py::arg("a"), py::arg("w"), py::arg("block_expert"), py::arg("block_rows"), py::arg("trans_b"),
         py::arg("seg") = c10::nullopt);
   m.def("grouped_wgrad", &grouped_wgrad);

@@ -95,6 +95,7 @@ void zero1_all_gather(const float* master, const int64_t* peer_bufs, long param_
                       int flag_off, uint32_t epoch, int rank, int world, long shard_numel, uint32_t* done_ctr, int param_dt,
                       cudaStream_t st);
 
+void gemm_few_rows(const void* x, const void* w, const void* residual, void* y, int M, int N, int K, int split, cudaStream_t st);
 void gemm_fp8(const void* a, const void* b, void* out, int M, int N, int K, const float* scale_a, const float* scale_b,
               cudaStream_t st);
 // ---- grouped (MoE blockwise) GEMMs, gemm_sm100.cu

@@ -37,6 +37,13 @@ def _eligible(a: torch.Tensor, b: torch.Tensor, M: int, N: int, K: int) -> bool:
     return M >= 1 and N % 8 == 0 and K % 8 == 0 and M % 8 == 0
 
 
+def _few_rows(M: int, N: int, K: int) -> bool:
+    """Rows for which streaming the weights decides the time (``csrc/gemm_few_sm100.cu``).  Up to 128 always (48 rows of 4096 x 11008:
+    21 us against 69); above, one block fits an SM, and it wins where the wide tiles would leave SMs idle (200 rows: 4096 x 11008
+    28 us against 71, 7168 x 8192 35 against 58) or by its smaller padding (136 rows of 22016 x 4096: 57 against 65; 248: 73 against 68)."""
+    return M <= 176 or (M < 256 and N <= 9472 and K >= 2048)
+
+
 def matmul(a: torch.Tensor, b: torch.Tensor, trans_a: bool = False, trans_b: bool = False,
            out: torch.Tensor | None = None, accumulate: bool = False, out_dtype=None) -> torch.Tensor:
     """``op(a) @ op(b)`` for 2-D tensors. ``accumulate`` adds into ``out`` (fp32 or bf16)."""
@@ -51,6 +58,9 @@ def matmul(a: torch.Tensor, b: torch.Tensor, trans_a: bool = False, trans_b: boo
         _ext.count_launch()
         return _ext.ext().gemv(a, b, None)
     if _eligible(a, b, M, N, K) and out_dtype in (torch.bfloat16, torch.float32):
+        if out is None and not trans_a and trans_b and out_dtype == torch.bfloat16 and _few_rows(M, N, K):
+            _ext.count_launch()
+            return _ext.ext().gemm_few_rows(a, b)
         if out is None:
             out = torch.empty(M, N, dtype=out_dtype, device=a.device)
             accumulate = False
