@@ -2,17 +2,20 @@
 // online softmax with one thread per query row.  Role parity: reference kernels/flash_attn.py:162-212
 // (nki_flash_attn_func → flash_fwd / flash_attn_bwd) and modules/attention call sites.
 //
-// Forward, one CTA per (128-query tile, head, batch), one CTA per SM (TMEM: S double buffer + O = 384 of 512 columns):
-//   warp 0      TMA producer : Q once, then K_j / V_j tiles ([128 kv × 128 d] as two 128B-swizzled [128 × 64] boxes)
-//   warp 1      MMA issuer   : S = Q·K_jᵀ  (A, B K-major, 8 × UMMA 128×128×16)  → TMEM cols [0,128)
-//                              O += P·V_j (A = P read from TMEM, B = V MN-major)  → TMEM cols [128,256)
-//   warps 2-5   softmax      : thread = query row (tcgen05.ld 32x32b: lane ↔ TMEM lane): row max, exp2, row sum, P packed
-//                              to bf16 and written back over S with tcgen05.st.  The O accumulator is only rescaled when
+// Forward, persistent, one CTA per SM walking items of 256 query rows of one (head, batch): two 128-row tiles that share every
+// K / V tile and are half a step out of phase, so that one tile's softmax runs under the other tile's products.
+// TMEM (512 columns): S of tile 0 / 1, O of tile 0 / 1, 128 columns each.
+//   warp 0      TMA producer : Q0, Q1, then K_j / V_j tiles ([128 kv × 128 d] as two 128B-swizzled [128 × 64] boxes), ring of 5
+//   warp 1      MMA issuer   : S = Q·K_jᵀ  (A, B K-major, 8 × UMMA 128×128×16)
+//                              O += P·V_j (A = P read from TMEM, B = V MN-major)
+//   warps 2-5, 6-9  softmax  : thread = query row of tile 0 / 1 (tcgen05.ld 32x32b: lane ↔ TMEM lane): row max, exp2, row sum, P
+//                              packed to bf16 and written back over S with tcgen05.st.  The O accumulator is only rescaled when
 //                              the running max grew by more than 2^8 (lazy rescale), so the common tile does no TMEM
 //                              round trip for O at all.
 // Outputs: O (bf16, arbitrary b/s/h strides) and LSE (fp32 [B, H, S], natural log) for the backward.
 #include <cuda.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <string>
 
@@ -28,11 +31,11 @@ CUtensorMap make_tmap_bf16_strided(const void* ptr, uint64_t rows, uint64_t cols
 namespace fa {
 
 constexpr int BM = 128, BN = 128, HD = 128;
-constexpr int kThreads = 192;
-constexpr int kPolyPairs = 0;      // of every 8 element pairs, how many use ex2_poly in the forward softmax
+constexpr int kThreads = 320;
+constexpr int kRing = 5;                         // K / V tiles in flight or in use
 constexpr uint32_t kTile = BM * HD * 2;          // 32 KB
 constexpr uint32_t kHalf = kTile / 2;            // one [128 × 64] box
-constexpr uint32_t kSmemFwd = 6 * kTile + 1024 /*align*/ + 256 /*barriers*/;
+constexpr uint32_t kSmemFwd = (2 + kRing) * kTile + 1024 /*align*/ + 512 /*barriers*/;
 
 // Warp-uniform issue: the whole MMA warp runs the issue loop in convergent control flow and one elected lane executes each
 // tcgen05 instruction (helpers tcgen05_mma_f16_e / tcgen05_commit_e in sm100_ptx.cuh explain why; mma_ts is the variant whose
@@ -45,6 +48,13 @@ NXD_DEVICE void mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32
       "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
       ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+NXD_DEVICE void tcgen05_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                 "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+               : "r"(taddr)
+               : "memory");
 }
 NXD_DEVICE void tcgen05_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
@@ -60,16 +70,7 @@ NXD_DEVICE void tcgen05_st_32x16p(uint32_t taddr, const uint32_t* r) {   // firs
         "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
-NXD_DEVICE void tcgen05_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]),
-        "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]),
-        "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-      : "memory");
-}
+NXD_DEVICE void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 NXD_DEVICE void tcgen05_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 NXD_DEVICE float ex2(float x) {
   float y;
@@ -98,70 +99,90 @@ struct FwdParams {
   long o_sb, o_ss, o_sh;      // output strides in elements
   float scale, scale_log2;
   int causal;
+  int group_bh;               // (batch, head) pairs whose K / V stay in L2 together
+  int split;                  // both streams on one query tile (see fwd_item)
   float* lse;                 // [B, H, S_q]
 };
 
-// exp2 on the FMA pipe (Cody–Waite split + degree-3 minimax on [-0.5, 0.5], rel. error ≈ 1e-4 — far below bf16's 4e-3):
-// the MUFU unit does 4 lanes/clk/SMSP, so a 128-wide row costs 1024 MUFU cycles per warp; moving ~30 % of the elements
-// here balances MUFU time against issue slots.
-NXD_DEVICE float ex2_poly(float x) {
-  x = fmaxf(x, -125.f);
-  const float t = x + 12582912.f;                   // 1.5·2^23: the integer part lands in the low mantissa bits
-  const float f = x - (t - 12582912.f);             // f ∈ [-0.5, 0.5]
-  float pz = fmaf(f, 0.0550087f, 0.2422104f);      // minimax fit of 2^f, max rel. error 1.0e-4
-  pz = fmaf(pz, f, 0.6932829f);
-  pz = fmaf(pz, f, 1.0f);
-  return __int_as_float(__float_as_int(pz) + (__float_as_int(t) << 23));
-}
+// Work items.  Two streams (t = 0, 1; a softmax warpgroup, an S and an O buffer each) share a block:
+//   pair  : query tiles 2 qt, 2 qt + 1 of one (batch, head); both streams walk the same K / V tiles (causal: the second needs one
+//           more; behind an odd number of tiles there is no second).
+//   split : few tiles for many SMs (every block gets one item): both streams work on the SAME query tile, stream t takes the K / V
+//           tiles of its parity and the partial results are merged at the end, which halves the serial chain.
+// Items come heaviest first within groups of heads whose K / V stay in L2 together, and a block that is done takes the next one
+// from the hardware's queue of blocks that have not started (cluster launch control): no counter in memory to clear.  All heads
+// heaviest first made every block stream another head and re-read K / V from HBM for every tile; a fixed assignment left blocks idle for a fifth
+// of the time (2 x 4096 tokens, 32 heads: 440 of 555 thousand cycles active).
+struct FwdItem { int qt, head, b, n, n0, n1; };
 
-// Persistent forward: one CTA per SM walks (q-tile, head, batch) work items in round-robin order.
-// TMEM: S double buffer [0,256) (P_j is written over S_j in place), O double buffer [256,512).  Tensor-pipe order is
-// S_0 S_1 PV_0 S_2 PV_1 S_3 … across item boundaries: the QKᵀ of the next tiles (including the first tiles of the NEXT work
-// item, whose Q sits in the second Q buffer) and the PV of the previous tile run while the softmax warps work on the current
-// tile, and the epilogue of item i (O_i → HBM) overlaps the first QKᵀ/PV of item i+1 (second O buffer).  The one-time costs
-// (TMEM allocation, barrier init, descriptor prefetch, first TMA round trip) are paid once per SM instead of once per tile.
-struct FwdItem { int qt, head, b, n_kv; };
-
-// Work order = (batch·head) major, q-tile minor — the order the hardware block scheduler would use, so the CTAs running at any
-// moment work on the same few heads and K/V stay in L2 (sorting all items heaviest-first instead made every CTA stream a
-// different head and re-read K/V from HBM for every q tile: 4.4 GB instead of 0.27 GB per call, measured 15 % slower).  The q
-// tile is rotated by the head index so that a CTA's round-robin slice (stride = grid size) mixes heavy and light causal tiles.
-NXD_DEVICE FwdItem fwd_item(int idx, int nq, int n_tiles_kv, const FwdParams& p) {
-  FwdItem it;
-  const int bh = idx / nq, j = idx % nq;
-  it.qt = nq - 1 - (j + bh) % nq;
+NXD_DEVICE FwdItem fwd_item(int idx, const FwdParams& p) {
+  FwdItem it{};
+  if (idx < 0) return it;                          // n = 0: no item
+  const int nq = (p.S_q + BM - 1) / BM, np = p.split ? nq : (nq + 1) / 2, bhs = p.H * p.B;
+  const int grp = idx / (np * p.group_bh), rem = idx - grp * np * p.group_bh;
+  const int gs = min(p.group_bh, bhs - grp * p.group_bh);
+  const int bh = grp * p.group_bh + rem % gs, at = np - 1 - rem / gs;
   it.head = bh % p.H;
   it.b = bh / p.H;
-  it.n_kv = p.causal ? min(it.qt + 1, n_tiles_kv) : n_tiles_kv;
+  const int n_tiles_kv = (p.S_kv + BN - 1) / BN;
+  if (p.split) {
+    it.qt = at;
+    it.n = p.causal ? min(at + 1, n_tiles_kv) : n_tiles_kv;
+    it.n0 = (it.n + 1) / 2;
+    it.n1 = it.n / 2;
+  } else {
+    it.qt = 2 * at;
+    it.n0 = p.causal ? min(it.qt + 1, n_tiles_kv) : n_tiles_kv;
+    it.n1 = it.qt + 1 >= nq ? 0 : p.causal ? min(it.qt + 2, n_tiles_kv) : n_tiles_kv;
+    it.n = max(it.n0, it.n1);
+  }
   return it;
 }
-NXD_DEVICE int fwd_item_index(int k) { return k * (int)gridDim.x + (int)blockIdx.x; }
 
+// The block asks for the index of a block that has not started; the 16-byte answer completes `bar`.
+NXD_DEVICE void clc_request(uint32_t answer, uint32_t bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(answer), "r"(bar) : "memory");
+}
+NXD_DEVICE int clc_answer(uint32_t answer) {       // block index, or -1: none left
+  uint32_t got, x;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t"
+      "ld.shared.b128 h, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "mov.u32 %1, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t}"
+      : "=&r"(got), "=&r"(x)
+      : "r"(answer)
+      : "memory");
+  return got ? (int)x : -1;
+}
+
+// Bound by the exponentials (MUFU: 1024 cycles per 128 x 128 tile and softmax warp, two warps per scheduler), the products (1024
+// cycles per tile) and the chain between them.  Tensor order is S0 S1 | PV0_j S0_{j+1} | PV1_j S1_{j+1} | …, across item
+// boundaries, with one S buffer per stream: S_{j+1} follows PV_j in pipe order, so a softmax warp that sees S_{j+1} knows that
+// PV_j is done.  P is handed over in two halves: the first half's products run under the second half's exponentials.
 __global__ void __launch_bounds__(kThreads, 1)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
               const __grid_constant__ CUtensorMap tv, __nv_bfloat16* __restrict__ out, const FwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t sQ = smem_base, sK = smem_base + 2 * kTile, sV = smem_base + 4 * kTile;   // Q, K, V: two stages each
-  const uint32_t bars = smem_base + 6 * kTile;
-  // qf[2] qe[2] kf[2] vf[2] ke[2] ve[2] s[2] p[2] pv[2] oe[2] | tmem slot
-  // pv has one barrier per S buffer: a softmax warp that runs ahead of its siblings reaches the wait for PV of tile g-1 while
-  // PV of tile g-2 has not even been issued; the parity of a single barrier could not tell the two apart
-  const uint32_t bar_qf = bars, bar_qe = bars + 16, bar_kf = bars + 32, bar_vf = bars + 48, bar_ke = bars + 64,
-                 bar_ve = bars + 80, bar_s = bars + 96, bar_p = bars + 112, bar_pv = bars + 128, bar_oe = bars + 144,
-                 tmem_slot = bars + 160;
+  const uint32_t sQ = smem_base, sKV = smem_base + 2 * kTile;
+  const uint32_t bars = smem_base + (2 + kRing) * kTile;
+  // per stream: qf[2] qe[2] s[2] pa[2] pb[2] of[2] oe[2] | next item: full[2] empty[2] answer[2] | ring: kvf[5] kve[5] | tmem slot
+  const uint32_t bar_qf = bars, bar_qe = bars + 16, bar_s = bars + 32, bar_pa = bars + 48, bar_pb = bars + 64, bar_of = bars + 80,
+                 bar_oe = bars + 96, bar_nf = bars + 112, bar_ne = bars + 128, answers = bars + 144, bar_kvf = bars + 176,
+                 bar_kve = bars + 176 + 8 * kRing, tmem_slot = bars + 176 + 16 * kRing;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nq = (p.S_q + BM - 1) / BM;
-  const int n_tiles_kv = (p.S_kv + BN - 1) / BN;
-  const int n_items = nq * p.H * p.B;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
-      mbar_init(bar_qf + 8 * i, 1); mbar_init(bar_qe + 8 * i, 1);
-      mbar_init(bar_kf + 8 * i, 1); mbar_init(bar_vf + 8 * i, 1); mbar_init(bar_ke + 8 * i, 1); mbar_init(bar_ve + 8 * i, 1);
-      mbar_init(bar_s + 8 * i, 1); mbar_init(bar_p + 8 * i, 128); mbar_init(bar_oe + 8 * i, 128);
-      mbar_init(bar_pv + 8 * i, 1);
+      mbar_init(bar_qf + 8 * i, 1); mbar_init(bar_qe + 8 * i, 1); mbar_init(bar_s + 8 * i, 1);
+      mbar_init(bar_pa + 8 * i, 128); mbar_init(bar_pb + 8 * i, 128);
+      mbar_init(bar_of + 8 * i, 1); mbar_init(bar_oe + 8 * i, 128);
+      mbar_init(bar_nf + 8 * i, 1); mbar_init(bar_ne + 8 * i, 10);       // readers: producer, MMA warp, 8 softmax warps
     }
+    for (int i = 0; i < kRing; ++i) { mbar_init(bar_kvf + 8 * i, 1); mbar_init(bar_kve + 8 * i, 1); }
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -174,127 +195,166 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
   const uint32_t tmem_S = tmem_base, tmem_O = tmem_base + 256;
+  // item number il of this block (-1: none), for a whole warp or for the producer's lane alone
+  auto item_index = [&](int il, bool whole_warp) {
+    if (il == 0) return (int)blockIdx.x;
+    if (p.split) return -1;                        // one item per block
+    const int st = (il - 1) & 1;
+    mbar_wait(bar_nf + 8 * st, (uint32_t)(((il - 1) >> 1) & 1));
+    const int idx = clc_answer(answers + 16 * st);
+    fence_async_smem();                            // this read before the next answer is written there
+    if (whole_warp) __syncwarp();
+    if (!whole_warp || lane == 0) mbar_arrive(bar_ne + 8 * st);
+    return idx;
+  };
 
   if (warp == 0) {
     if (lane == 0) {
       prefetch_tmap(&tq); prefetch_tmap(&tk); prefetch_tmap(&tv);
-      int g = 0;
+      int slot = 0; uint32_t ph = 0;
+      int items[2] = {0, 0};
+      auto load_kv = [&](const CUtensorMap* map, int c, int r) {
+        mbar_wait(bar_kve + 8 * slot, ph ^ 1);
+        mbar_expect_tx(bar_kvf + 8 * slot, kTile);
+        tma_load_2d(sKV + slot * kTile, map, bar_kvf + 8 * slot, c, r);
+        tma_load_2d(sKV + slot * kTile + kHalf, map, bar_kvf + 8 * slot, c + 64, r);
+        if (++slot == kRing) { slot = 0; ph ^= 1; }
+      };
       for (int il = 0;; ++il) {
-        const int idx = fwd_item_index(il);
-        if (idx >= n_items) break;
-        const FwdItem it = fwd_item(idx, nq, n_tiles_kv, p);
+        const int idx = item_index(il, false);
+        if (idx < 0) break;
+        const FwdItem it = fwd_item(idx, p);
         const int kvh = it.head / (p.H / p.Hkv);
-        const int qb = il & 1;
-        mbar_wait(bar_qe + 8 * qb, (uint32_t)(((il >> 1) & 1) ^ 1));
         const int qc = it.b * p.q.col_b + it.head * p.q.col_h, qr = it.b * p.q.row_b + it.head * p.q.row_h + it.qt * BM;
-        mbar_expect_tx(bar_qf + 8 * qb, kTile);
-        tma_load_2d(sQ + qb * kTile, &tq, bar_qf + 8 * qb, qc, qr);
-        tma_load_2d(sQ + qb * kTile + kHalf, &tq, bar_qf + 8 * qb, qc + 64, qr);
         const int kc = it.b * p.k.col_b + kvh * p.k.col_h, kr = it.b * p.k.row_b + kvh * p.k.row_h;
         const int vc = it.b * p.v.col_b + kvh * p.v.col_h, vr = it.b * p.v.row_b + kvh * p.v.row_h;
-        for (int j = 0; j < it.n_kv; ++j, ++g) {
-          const int st = g & 1;
-          const uint32_t ph = (uint32_t)((g >> 1) & 1);
-          mbar_wait(bar_ke + 8 * st, ph ^ 1);
-          mbar_expect_tx(bar_kf + 8 * st, kTile);
-          tma_load_2d(sK + st * kTile, &tk, bar_kf + 8 * st, kc, kr + j * BN);
-          tma_load_2d(sK + st * kTile + kHalf, &tk, bar_kf + 8 * st, kc + 64, kr + j * BN);
-          mbar_wait(bar_ve + 8 * st, ph ^ 1);
-          mbar_expect_tx(bar_vf + 8 * st, kTile);
-          tma_load_2d(sV + st * kTile, &tv, bar_vf + 8 * st, vc, vr + j * BN);
-          tma_load_2d(sV + st * kTile + kHalf, &tv, bar_vf + 8 * st, vc + 64, vr + j * BN);
+        for (int t = 0; t < 2; ++t) {
+          if (t == 0 ? it.n0 > 0 : (it.n1 > 0 && !p.split)) {
+            mbar_wait(bar_qe + 8 * t, (uint32_t)((items[t] & 1) ^ 1));
+            ++items[t];
+            mbar_expect_tx(bar_qf + 8 * t, kTile);
+            tma_load_2d(sQ + t * kTile, &tq, bar_qf + 8 * t, qc, qr + t * BM);
+            tma_load_2d(sQ + t * kTile + kHalf, &tq, bar_qf + 8 * t, qc + 64, qr + t * BM);
+          }
+          if (t == 0 && it.n > 0) load_kv(&tk, kc, kr);
+        }
+        for (int j = 0; j < it.n; ++j) {
+          if (j > 0) load_kv(&tk, kc, kr + j * BN);
+          load_kv(&tv, vc, vr + j * BN);
+        }
+        // asked for when the last tile is on its way (two steps before the end): asked at the item's start, the blocks would share
+        // out the queue before they know which of them are done first (1 x 2048 tokens, 32 heads: 59 us)
+        if (!p.split) {
+          mbar_wait(bar_ne + 8 * (il & 1), (uint32_t)(((il >> 1) & 1) ^ 1));
+          mbar_expect_tx(bar_nf + 8 * (il & 1), 16);
+          clc_request(answers + 16 * (il & 1), bar_nf + 8 * (il & 1));
         }
       }
     }
     __syncwarp();
   } else if (warp == 1) {
-    {   // all 32 lanes run this loop; the helpers elect one lane per tcgen05 instruction
-      constexpr uint32_t idesc_s = make_idesc(false, false, BM, BN);
-      constexpr uint32_t idesc_o = make_idesc(false, true, BM, HD);
-      // cursor over the flattened (item, kv-tile) sequence of this CTA
-      struct Cur { int il, j, n_kv, g; bool ok; };
-      auto start = [&](int il, int g) {
-        Cur c{il, 0, 0, g, false};
-        const int idx = fwd_item_index(il);
-        if (idx < n_items) { c.n_kv = fwd_item(idx, nq, n_tiles_kv, p).n_kv; c.ok = true; }
-        return c;
-      };
-      auto advance = [&](Cur& c) {
-        ++c.g;
-        if (++c.j == c.n_kv) c = start(c.il + 1, c.g);
-      };
-      auto issue_s = [&](const Cur& c) {
-        const int st = c.g & 1, qb = c.il & 1;
-        if (c.j == 0) mbar_wait(bar_qf + 8 * qb, (uint32_t)((c.il >> 1) & 1));
-        mbar_wait(bar_kf + 8 * st, (uint32_t)((c.g >> 1) & 1));
-        tcgen05_fence_after();
-        const uint32_t q_s = sQ + qb * kTile, k_s = sK + st * kTile;
+    // all 32 lanes run this loop; the helpers elect one lane per tcgen05 instruction
+    constexpr uint32_t idesc_s = make_idesc(false, false, BM, BN);
+    constexpr uint32_t idesc_o = make_idesc(false, true, BM, HD);
+    int steps[2] = {0, 0}, q_items[2] = {0, 0}, o_items[2] = {0, 0};
+    // stream t, K tile number `pos` of the ring; `last_k`: no other stream uses it after this; `first` / `last` of the item
+    auto issue_s = [&](int t, int pos, bool first, bool last, bool last_k) {
+      const int slot = pos % kRing, tq_ = p.split ? 0 : t;
+      if (first) { mbar_wait(bar_qf + 8 * tq_, (uint32_t)(q_items[t] & 1)); ++q_items[t]; }
+      mbar_wait(bar_kvf + 8 * slot, (uint32_t)((pos / kRing) & 1));
+      tcgen05_fence_after();
+      const uint32_t q_s = sQ + tq_ * kTile, k_s = sKV + slot * kTile;
 #pragma unroll
-        for (int kb = 0; kb < 2; ++kb)
+      for (int kb = 0; kb < 2; ++kb)
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            tcgen05_mma_f16_e(tmem_S + st * BN, make_smem_desc(q_s + kb * kHalf + kk * 32, 16, 1024),
-                   make_smem_desc(k_s + kb * kHalf + kk * 32, 16, 1024), idesc_s, (kb | kk) ? 1u : 0u);
-        tcgen05_commit_e(bar_ke + 8 * st);
-        tcgen05_commit_e(bar_s + 8 * st);
-        if (c.j == c.n_kv - 1) tcgen05_commit_e(bar_qe + 8 * qb);       // last QKᵀ of the item: its Q buffer is free
-      };
-      Cur ahead = start(0, 0), cur = ahead;
-      if (ahead.ok) { issue_s(ahead); advance(ahead); }
-      if (ahead.ok) { issue_s(ahead); advance(ahead); }
-      while (cur.ok) {
-        const int st = cur.g & 1, ob = cur.il & 1;
-        const uint32_t ph = (uint32_t)((cur.g >> 1) & 1);
-        mbar_wait(bar_p + 8 * st, ph);
-        mbar_wait(bar_vf + 8 * st, ph);
-        if (cur.j == 0) mbar_wait(bar_oe + 8 * ob, (uint32_t)(((cur.il >> 1) & 1) ^ 1));   // epilogue of item il-2 left O[ob]
-        tcgen05_fence_after();
-        const uint32_t v_s = sV + st * kTile;
+        for (int kk = 0; kk < 4; ++kk)
+          tcgen05_mma_f16_e(tmem_S + t * BN, make_smem_desc(q_s + kb * kHalf + kk * 32, 16, 1024),
+                 make_smem_desc(k_s + kb * kHalf + kk * 32, 16, 1024), idesc_s, (kb | kk) ? 1u : 0u);
+      tcgen05_commit_e(bar_s + 8 * t);
+      if (last_k) tcgen05_commit_e(bar_kve + 8 * slot);
+      if (last && !p.split) tcgen05_commit_e(bar_qe + 8 * t);
+    };
+    auto get = [&](int il) { return fwd_item(item_index(il, true), p); };
+    // ring position of step j of stream t (its K; V is the next), counted from the item's first
+    auto at = [&](int t, int j) { return p.split ? 2 * (2 * j + t) : 2 * j; };
+    FwdItem it = get(0);
+    int pos0 = 0;                                  // ring position of the item's first K tile
+    for (int t = 0; t < 2; ++t) {
+      const int nt = t ? it.n1 : it.n0;
+      if (nt > 0) issue_s(t, at(t, 0), true, nt == 1, p.split || t == 1 || it.n1 == 0);
+    }
+    for (int il = 0; it.n > 0; ++il) {
+      FwdItem nx{};
+      const int pos1 = pos0 + 2 * it.n, steps_n = max(it.n0, it.n1);
+      for (int j = 0; j < steps_n; ++j) {
+        if (j == steps_n - 1) nx = get(il + 1);
 #pragma unroll
-        for (int k = 0; k < BN / 16; ++k)
-          mma_ts(tmem_O + ob * HD, tmem_S + st * BN + k * 8, make_smem_desc(v_s + k * 2048, kHalf, 1024), idesc_o,
-                 (cur.j | k) ? 1u : 0u);
-        tcgen05_commit_e(bar_ve + 8 * st);
-        tcgen05_commit_e(bar_pv + 8 * st);
-        if (ahead.ok) { issue_s(ahead); advance(ahead); }        // overwrites P of tile g — behind PV_g in pipe order
-        advance(cur);
+        for (int t = 0; t < 2; ++t) {
+          const int nt = t ? it.n1 : it.n0;
+          if (j < nt) {
+            const int pos = pos0 + at(t, j) + 1, slot = pos % kRing;
+            const uint32_t ph = (uint32_t)(steps[t] & 1);
+            ++steps[t];
+            mbar_wait(bar_kvf + 8 * slot, (uint32_t)((pos / kRing) & 1));
+            if (j == 0) { mbar_wait(bar_oe + 8 * t, (uint32_t)((o_items[t] & 1) ^ 1)); ++o_items[t]; }   // the item before left O
+            const uint32_t v_s = sKV + slot * kTile;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              mbar_wait((h ? bar_pb : bar_pa) + 8 * t, ph);
+              tcgen05_fence_after();
+#pragma unroll
+              for (int k = h * 4; k < h * 4 + 4; ++k)
+                mma_ts(tmem_O + t * HD, tmem_S + t * BN + k * 8, make_smem_desc(v_s + k * 2048, kHalf, 1024), idesc_o, (j | k) ? 1u : 0u);
+            }
+            if (p.split || t == 1 || j >= it.n1) tcgen05_commit_e(bar_kve + 8 * slot);
+            if (j == nt - 1) tcgen05_commit_e(bar_of + 8 * t);
+          }
+          if (j < steps_n - 1) {                   // S over P of this step: behind its PV in pipe order
+            if (j + 1 < nt) issue_s(t, pos0 + at(t, j + 1), false, j + 2 == nt, p.split || t == 1 || j + 1 >= it.n1);
+          } else {                                 // first S of the next item (this stream's last PV has been issued)
+            const int nn = t ? nx.n1 : nx.n0;
+            if (nn > 0) issue_s(t, pos1 + at(t, 0), true, nn == 1, p.split || t == 1 || nx.n1 == 0);
+          }
+        }
       }
+      it = nx;
+      pos0 = pos1;
     }
     __syncwarp();
   } else {
+    const int t = warp >= 6;                       // stream of this warpgroup
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+    const uint32_t tS = tmem_S + t * BN + lane_base, tO = tmem_O + t * HD + lane_base;
+    const uint32_t my_s = bar_s + 8 * t, my_pa = bar_pa + 8 * t, my_pb = bar_pb + 8 * t, my_of = bar_of + 8 * t, my_oe = bar_oe + 8 * t;
     const float sl2 = p.scale_log2;
-    int g = 0;
+    int g = 0, items = 0;
     for (int il = 0;; ++il) {
-      const int idx = fwd_item_index(il);
-      if (idx >= n_items) break;
-      const FwdItem it = fwd_item(idx, nq, n_tiles_kv, p);
-      const int qt = it.qt, ob = il & 1;
-      const int q_idx = qt * BM + row;
-      const uint32_t tO = tmem_O + ob * HD + lane_base;
+      const int idx = item_index(il, true);
+      if (idx < 0) break;
+      const FwdItem it = fwd_item(idx, p);
+      const int nt = t ? it.n1 : it.n0;
+      if (nt == 0) continue;
+      const int q0 = (it.qt + (p.split ? 0 : t)) * BM, q_idx = q0 + row;
       float m_ref = -INFINITY, l = 0.f;
-      for (int j = 0; j < it.n_kv; ++j, ++g) {
-        const int st = g & 1;
-        const uint32_t tS = tmem_S + st * BN + lane_base;
-        mbar_wait(bar_s + 8 * st, (uint32_t)((g >> 1) & 1));
+      for (int j = 0; j < nt; ++j, ++g) {
+        mbar_wait(my_s, (uint32_t)(g & 1));
         tcgen05_fence_after();
-        const int kv0 = j * BN;
-        const bool masked = (p.causal && kv0 + BN - 1 > qt * BM) || (kv0 + BN > p.S_kv);
+        const int kv0 = (p.split ? 2 * j + t : j) * BN;
+        const bool masked = (p.causal && kv0 + BN - 1 > q0) || (kv0 + BN > p.S_kv);
         // ---- the whole S row (128 fp32) comes into registers with four back-to-back TMEM loads and one wait
         uint32_t sr[4][32];
 #pragma unroll
         for (int c = 0; c < 4; ++c) tcgen05_ld_32x32(tS + c * 32, sr[c]);
         tcgen05_wait_ld();
         if (masked) {      // diagonal / ragged tile: −inf in place, the exp below turns it into an exact 0
+          const int lim = min(p.S_kv - 1, p.causal ? q_idx : 0x7fffffff) - kv0;      // last visible column of the tile
 #pragma unroll
           for (int c = 0; c < 4; ++c)
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const int kv = kv0 + c * 32 + i;
-              if (!(kv < p.S_kv && (!p.causal || kv <= q_idx))) sr[c][i] = 0xff800000u;
-            }
+            for (int i = 0; i < 32; ++i)
+              if (c * 32 + i > lim) sr[c][i] = 0xff800000u;
         }
         float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -307,20 +367,18 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
         } else {
           const float m_new = fmaxf(m_ref, mx);
           const bool need = (m_new - m_ref) * sl2 > 8.f;
-          if (__any_sync(0xffffffffu, need)) {
-            mbar_wait(bar_pv + 8 * ((g - 1) & 1), (uint32_t)(((g - 1) >> 1) & 1));      // PV of the previous tile retired: O is quiescent
-            tcgen05_fence_after();
+          if (__any_sync(0xffffffffu, need)) {           // PV of the step before is done (this S came after it): O is quiescent
             const float f = need ? ex2((m_ref - m_new) * sl2) : 1.f;
             if (need) m_ref = m_new;
             l *= f;
 #pragma unroll 1
-            for (int c = 0; c < 4; ++c) {
-              uint32_t r[32];
-              tcgen05_ld_32x32(tO + c * 32, r);
+            for (int c = 0; c < 8; ++c) {
+              uint32_t r[16];
+              tcgen05_ld_32x16(tO + c * 16, r);
               tcgen05_wait_ld();
 #pragma unroll
-              for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * f);
-              tcgen05_st_32x32(tO + c * 32, r);
+              for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * f);
+              tcgen05_st_32x16(tO + c * 16, r);
             }
           }
         }
@@ -334,50 +392,84 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
           for (int i = 0; i < 32; i += 2) {
             float x0, x1;
             unpack2(fma2(pack2u(sr[c][i], sr[c][i + 1]), sl2_2, nmb_2), x0, x1);
-            // kPolyPairs of every 8 pairs take the FMA-pipe exp2; 0 = all on MUFU (a lone warp per SMSP is issue-bound, not
-            // MUFU-bound, once the polynomial's 8 extra instructions are counted — measured, see profiles/)
-            const bool poly = ((i >> 1) & 7) < kPolyPairs;
-            const float p0 = poly ? ex2_poly(x0) : ex2(x0);
-            const float p1 = poly ? ex2_poly(x1) : ex2(x1);
+            const float p0 = ex2(x0), p1 = ex2(x1);
             l2acc[c] = add2(l2acc[c], pack2(p0, p1));
             sr[c][i >> 1] = pack_bf16(p0, p1);
           }
           tcgen05_st_32x16p(tS + c * 16, sr[c]);
+          if (c & 1) {
+            tcgen05_wait_st();
+            tcgen05_fence_before();
+            mbar_arrive(c == 1 ? my_pa : my_pb);
+          }
         }
         float l4[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) { float a, bq; unpack2(l2acc[c], a, bq); l4[c] = a + bq; }
         l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
-        tcgen05_wait_st();
-        tcgen05_fence_before();
-        mbar_arrive(bar_p + 8 * st);
       }
-      // ---- epilogue: O / l → bf16, LSE (the MMA warp is already working on the next item in the other O buffer)
-      mbar_wait(bar_pv + 8 * ((g - 1) & 1), (uint32_t)(((g - 1) >> 1) & 1));
+      // ---- epilogue: O comes into registers at once, so that the next item's first product may overwrite it while this one is
+      //      scaled and stored
+      mbar_wait(my_of, (uint32_t)(items & 1));
+      ++items;
       tcgen05_fence_after();
+      uint32_t r[4][32];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tcgen05_ld_32x32(tO + c * 32, r[c]);
+      tcgen05_wait_ld();
+      tcgen05_fence_before();
+      mbar_arrive(my_oe);
+      if (p.split && it.n1 > 0) {
+        // stream 1's sums to stream 0 through the Q buffers (every product with Q is done: stream 1's last PV was issued after
+        // the last S of both) and, for maximum and row sum, a ring slot nobody fills any more (a split block has one item)
+        const uint32_t so = sQ + row * 16, sml = sKV + row * 8;
+        if (t == 1) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int v4 = 0; v4 < 8; ++v4)
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(so + (c * 8 + v4) * 2048), "r"(r[c][v4 * 4]), "r"(r[c][v4 * 4 + 1]),
+                           "r"(r[c][v4 * 4 + 2]), "r"(r[c][v4 * 4 + 3]) : "memory");
+        }
+        // the ring: stream 0's last V must have been read before a slot is overwritten
+        if (t == 1) { mbar_wait(bar_of, 0); asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(sml), "f"(m_ref), "f"(l) : "memory"); }
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (t == 1) continue;
+        float m1, l1;
+        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(m1), "=f"(l1) : "r"(sml) : "memory");
+        const float m = fmaxf(m_ref, m1);
+        const float f0 = ex2((m_ref - m) * sl2), f1 = m1 == -INFINITY ? 0.f : ex2((m1 - m) * sl2);
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int v4 = 0; v4 < 8; ++v4) {
+            float4 o1;
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(o1.x), "=f"(o1.y), "=f"(o1.z), "=f"(o1.w)
+                         : "r"(so + (c * 8 + v4) * 2048) : "memory");
+            const float w[4] = {o1.x, o1.y, o1.z, o1.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              r[c][v4 * 4 + i] = __float_as_uint(fmaf(__uint_as_float(r[c][v4 * 4 + i]), f0, w[i] * f1));
+          }
+        l = l * f0 + l1 * f1;
+        m_ref = m;
+      }
       const float inv_l = 1.f / l;
-      const bool row_ok = q_idx < p.S_q;
-      __nv_bfloat16* orow = out + (long)it.b * p.o_sb + (long)q_idx * p.o_ss + (long)it.head * p.o_sh;
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t r[32];
-        tcgen05_ld_32x32(tO + c * 32, r);
-        tcgen05_wait_ld();
-        if (row_ok) {
+      if (q_idx < p.S_q) {
+        __nv_bfloat16* orow = out + (long)it.b * p.o_sb + (long)q_idx * p.o_ss + (long)it.head * p.o_sh;
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
 #pragma unroll
           for (int v4 = 0; v4 < 4; ++v4) {
             uint4 o;
-            o.x = pack_bf16(__uint_as_float(r[v4 * 8 + 0]) * inv_l, __uint_as_float(r[v4 * 8 + 1]) * inv_l);
-            o.y = pack_bf16(__uint_as_float(r[v4 * 8 + 2]) * inv_l, __uint_as_float(r[v4 * 8 + 3]) * inv_l);
-            o.z = pack_bf16(__uint_as_float(r[v4 * 8 + 4]) * inv_l, __uint_as_float(r[v4 * 8 + 5]) * inv_l);
-            o.w = pack_bf16(__uint_as_float(r[v4 * 8 + 6]) * inv_l, __uint_as_float(r[v4 * 8 + 7]) * inv_l);
+            o.x = pack_bf16(__uint_as_float(r[c][v4 * 8 + 0]) * inv_l, __uint_as_float(r[c][v4 * 8 + 1]) * inv_l);
+            o.y = pack_bf16(__uint_as_float(r[c][v4 * 8 + 2]) * inv_l, __uint_as_float(r[c][v4 * 8 + 3]) * inv_l);
+            o.z = pack_bf16(__uint_as_float(r[c][v4 * 8 + 4]) * inv_l, __uint_as_float(r[c][v4 * 8 + 5]) * inv_l);
+            o.w = pack_bf16(__uint_as_float(r[c][v4 * 8 + 6]) * inv_l, __uint_as_float(r[c][v4 * 8 + 7]) * inv_l);
             *reinterpret_cast<uint4*>(orow + c * 32 + v4 * 8) = o;
           }
-        }
+        p.lse[((long)it.b * p.H + it.head) * p.S_q + q_idx] = m_ref * p.scale + __logf(l);
       }
-      if (row_ok) p.lse[((long)it.b * p.H + it.head) * p.S_q + q_idx] = m_ref * p.scale + __logf(l);
-      tcgen05_fence_before();
-      mbar_arrive(bar_oe + 8 * ob);
     }
   }
   tcgen05_fence_before();
@@ -430,7 +522,6 @@ NXD_DEVICE void bulk_reduce_add_f32(void* gdst, uint32_t smem_src, uint32_t byte
 NXD_DEVICE void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 NXD_DEVICE void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 NXD_DEVICE void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-NXD_DEVICE void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 NXD_DEVICE void named_bar(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 
 // Softmax-side math of one backward tile, split in two phases so the exp work (needs only Sᵀ, which the tensor pipe delivered a
@@ -878,10 +969,15 @@ void flash_attn_fwd(const void* q, const void* k, const void* v, void* out, floa
     NXD_CUDA_CHECK(cudaFuncSetAttribute(fa_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemFwd));
     configured = true;
   }
-  const int n_items = ((S_q + BM - 1) / BM) * H * B;
+  const long kv_bytes = (long)S_kv * HD * 4 * Hkv / H;            // K and V of one query head (its share of the group's)
+  p.group_bh = (int)std::min<long>((long)H * B, std::max<long>(1, (48l << 20) / std::max<long>(1, kv_bytes)));
   static int sms = 0;
   if (!sms) { int dev; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
-  fa_fwd_kernel<<<n_items < sms ? n_items : sms, kThreads, kSmemFwd, st>>>(tq, tk, tv, (__nv_bfloat16*)out, p);
+  const int nq = (S_q + BM - 1) / BM;
+  p.split = (long)nq * H * B <= sms;
+  const long items = (long)(p.split ? nq : (nq + 1) / 2) * H * B;
+  if (items == 0) return;
+  fa_fwd_kernel<<<(unsigned)items, kThreads, kSmemFwd, st>>>(tq, tk, tv, (__nv_bfloat16*)out, p);
   NXD_CUDA_CHECK(cudaGetLastError());
 }
 
