@@ -38,11 +38,11 @@ static std::vector<Tensor> rmsnorm_bwd(const Tensor& g, const Tensor& x, const T
   c10::cuda::CUDAGuard guard(x.device());
   const int rows = (int)x.size(0), H = (int)x.size(1);
   auto dx = at::empty_like(x);
-  auto dw = at::zeros({H}, x.options().dtype(at::kFloat));
+  auto dw = rows > 0 ? at::empty({H}, x.options()) : at::zeros({H}, x.options());      // fp32 sums, the weight's type
   if (rows > 0) {
-    auto partial = at::empty({nxd::rmsnorm_bwd_num_partials(rows), H}, x.options().dtype(at::kFloat));
+    auto partial = at::empty({nxd::rmsnorm_bwd_num_partials(rows, H, dt_code(x)), H}, x.options().dtype(at::kFloat));
     nxd::rmsnorm_bwd(g.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr<float>(), dx.data_ptr(),
-                     partial.data_ptr<float>(), dw.data_ptr<float>(), rows, H, dt_code(x), stream());
+                     partial.data_ptr<float>(), dw.data_ptr(), rows, H, dt_code(x), stream());
   }
   return {dx, dw};
 }
@@ -66,11 +66,11 @@ static std::vector<Tensor> add_rmsnorm_bwd(const Tensor& gy, const Tensor& gh, c
   c10::cuda::CUDAGuard guard(h.device());
   const int rows = (int)h.size(0), H = (int)h.size(1);
   auto dh = at::empty_like(h);
-  auto dw = at::zeros({H}, h.options().dtype(at::kFloat));
+  auto dw = rows > 0 ? at::empty({H}, h.options()) : at::zeros({H}, h.options());
   if (rows > 0) {
-    auto partial = at::empty({nxd::rmsnorm_bwd_num_partials(rows), H}, h.options().dtype(at::kFloat));
+    auto partial = at::empty({nxd::rmsnorm_bwd_num_partials(rows, H, dt_code(h)), H}, h.options().dtype(at::kFloat));
     nxd::add_rmsnorm_bwd(gy.data_ptr(), gh.data_ptr(), h.data_ptr(), w.data_ptr(), rstd.data_ptr<float>(), dh.data_ptr(),
-                         partial.data_ptr<float>(), dw.data_ptr<float>(), rows, H, dt_code(h), stream());
+                         partial.data_ptr<float>(), dw.data_ptr(), rows, H, dt_code(h), stream());
   }
   return {dh, dw};
 }

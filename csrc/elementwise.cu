@@ -1,5 +1,5 @@
 // Hand-written sm_100a elementwise / normalisation / loss kernels.
-//   rmsnorm fwd+bwd   (reference call site: modules/rms_norm.py:10-33)
+//   rmsnorm fwd       (reference call site: modules/rms_norm.py:10-33; backward: fused_norm.cu)
 //   swiglu  fwd+bwd   (examples/training/llama/modeling_llama_nxd.py:208-219)
 //   rope apply        (overrides/transformer_overrides.py:20-32)
 //   vocab-parallel cross-entropy stats + backward (parallel_layers/loss_functions.py:12-129)
@@ -59,84 +59,6 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const T* __restrict__ 
     for (int j = 0; j < N; ++j) po.set(j, p.f(j) * rstd * pw.f(j));
     po.store(yr + v * N);
   }
-}
-
-// =====================================================================================
-// RMSNorm backward. Persistent CTAs stride over rows; each thread owns fixed columns so the
-// dW partial lives in registers across rows.  partial_dw: [gridDim.x, H] fp32.
-//   dx = rstd * (g*w - xhat * mean_H(g*w*xhat)),  dw = sum_rows g*xhat
-// =====================================================================================
-template <typename T, int MAXV>
-__global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const T* __restrict__ g, const T* __restrict__ x,
-                                                          const T* __restrict__ w, const float* __restrict__ rstd,
-                                                          T* __restrict__ dx, float* __restrict__ partial_dw, int rows,
-                                                          int H) {
-  using P = Pack16<T>;
-  constexpr int N = P::N;
-  __shared__ float red[32];
-  const int nvec = H / N;
-  float dw[MAXV][N];
-  P pw[MAXV];
-#pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
-    const int v = threadIdx.x + i * blockDim.x;
-#pragma unroll
-    for (int j = 0; j < N; ++j) dw[i][j] = 0.f;
-    if (v < nvec) pw[i].load_nc(w + v * N);
-  }
-  for (int row = blockIdx.x; row < rows; row += gridDim.x) {
-    const T* xr = x + (size_t)row * H;
-    const T* gr = g + (size_t)row * H;
-    T* dxr = dx + (size_t)row * H;
-    const float rs = rstd[row];
-    P px[MAXV], pg[MAXV];
-    float dot = 0.f;
-#pragma unroll
-    for (int i = 0; i < MAXV; ++i) {
-      const int v = threadIdx.x + i * blockDim.x;
-      if (v < nvec) {
-        px[i].load(xr + v * N);
-        pg[i].load(gr + v * N);
-#pragma unroll
-        for (int j = 0; j < N; ++j) {
-          const float xh = px[i].f(j) * rs, gg = pg[i].f(j);
-          dot += gg * pw[i].f(j) * xh;
-          dw[i][j] += gg * xh;
-        }
-      }
-    }
-    dot = block_sum(dot, red) / (float)H;
-#pragma unroll
-    for (int i = 0; i < MAXV; ++i) {
-      const int v = threadIdx.x + i * blockDim.x;
-      if (v < nvec) {
-        P po;
-#pragma unroll
-        for (int j = 0; j < N; ++j) {
-          const float xh = px[i].f(j) * rs;
-          po.set(j, rs * (pg[i].f(j) * pw[i].f(j) - xh * dot));
-        }
-        po.store(dxr + v * N);
-      }
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
-    const int v = threadIdx.x + i * blockDim.x;
-    if (v < nvec) {
-      float* o = partial_dw + (size_t)blockIdx.x * H + v * N;
-#pragma unroll
-      for (int j = 0; j < N; ++j) o[j] = dw[i][j];
-    }
-  }
-}
-
-__global__ void reduce_partials_kernel(const float* __restrict__ partial, float* __restrict__ out, int nparts, int H) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= H) return;
-  float s = 0.f;
-  for (int p = 0; p < nparts; ++p) s += partial[(size_t)p * H + c];
-  out[c] = s;
 }
 
 // =====================================================================================
@@ -331,21 +253,6 @@ void rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int rows, i
     const int th = pick_threads<T>(H);
     rmsnorm_fwd_kernel<T, 4><<<rows, th, 0, st>>>((const T*)x, (const T*)w, (T*)y, rstd, H, eps);
   });
-  NXD_CUDA_CHECK(cudaGetLastError());
-}
-
-int rmsnorm_bwd_num_partials(int rows) { return min(rows, num_sms() * 4); }
-
-void rmsnorm_bwd(const void* g, const void* x, const void* w, const float* rstd, void* dx, float* partial, float* dw,
-                 int rows, int H, int dt, cudaStream_t st) {
-  const int grid = rmsnorm_bwd_num_partials(rows);
-  DISPATCH_DTYPE(dt, {
-    const int nvec = H / Pack16<T>::N;
-    if (H % Pack16<T>::N || nvec > 256 * 4) nxd_throw("rmsnorm_bwd: unsupported H", __FILE__, __LINE__);
-    const int th = pick_threads<T>(H);
-    rmsnorm_bwd_kernel<T, 4><<<grid, th, 0, st>>>((const T*)g, (const T*)x, (const T*)w, rstd, (T*)dx, partial, rows, H);
-  });
-  reduce_partials_kernel<<<(H + 255) / 256, 256, 0, st>>>(partial, dw, grid, H);
   NXD_CUDA_CHECK(cudaGetLastError());
 }
 
