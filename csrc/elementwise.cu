@@ -156,31 +156,46 @@ __global__ void __launch_bounds__(256) rope_kernel(const T* __restrict__ x, T* _
 // =====================================================================================
 template <typename T>
 __global__ void __launch_bounds__(256) ce_stats_kernel(const T* __restrict__ logits, const int64_t* __restrict__ target,
-                                                       float* __restrict__ stats, int V, int vocab_start) {
+                                                       float* __restrict__ stats, int V, int vocab_start, int vec) {
   using P = Pack16<T>;
   constexpr int N = P::N;
   __shared__ float red[32];
   const int row = blockIdx.x;
   const T* xr = logits + (size_t)row * V;
   float m = -INFINITY, s = 0.f, sx = 0.f;
-  const int nvec = V / N;
-  for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
-    P p; p.load(xr + v * N);
-    float lm = p.f(0);
+  const int nvec = vec ? V / N : 0;                 // rows of another alignment: element by element
+  // four packets in flight and one rescaling of the sum for all of them
+  constexpr int U = 4;
+  for (int v0 = threadIdx.x; v0 < nvec; v0 += U * blockDim.x) {
+    P p[U];
+    float lm = m;
 #pragma unroll
-    for (int j = 1; j < N; ++j) lm = fmaxf(lm, p.f(j));
-    const float nm = fmaxf(m, lm);
+    for (int u = 0; u < U; ++u)
+      if (v0 + u * (int)blockDim.x < nvec) p[u].load(xr + (size_t)(v0 + u * blockDim.x) * N);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (v0 + u * (int)blockDim.x < nvec) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) lm = fmaxf(lm, p[u].f(j));
+      }
+    if (lm == -INFINITY) { sx += lm; continue; }    // nothing but masked columns so far
     float acc = 0.f;
 #pragma unroll
-    for (int j = 0; j < N; ++j) { const float f = p.f(j); acc += __expf(f - nm); sx += f; }
-    s = s * __expf(m - nm) + acc;
-    m = nm;
+    for (int u = 0; u < U; ++u)
+      if (v0 + u * (int)blockDim.x < nvec) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) { const float f = p[u].f(j); acc += __expf(f - lm); sx += f; }
+      }
+    s = s * __expf(m - lm) + acc;
+    m = lm;
   }
   for (int c = nvec * N + threadIdx.x; c < V; c += blockDim.x) {  // ragged tail
     const float f = to_f32<T>(xr[c]);
     const float nm = fmaxf(m, f);
+    sx += f;
+    if (nm == -INFINITY && f == f) continue;
     s = s * __expf(m - nm) + __expf(f - nm);
-    m = nm; sx += f;
+    m = nm;
   }
   const float gm = block_max(m, red);
   const float contrib = (m == -INFINITY) ? 0.f : s * __expf(m - gm);
@@ -198,25 +213,28 @@ template <typename T>
 __global__ void __launch_bounds__(256) ce_bwd_kernel(const T* __restrict__ logits, const int64_t* __restrict__ target,
                                                      const float* __restrict__ lse, const float* __restrict__ gout,
                                                      T* __restrict__ grad, int V, int vocab_start, float smoothing,
-                                                     float inv_vocab) {
+                                                     float inv_vocab, int vec) {
   using P = Pack16<T>;
   constexpr int N = P::N;
-  const int row = blockIdx.x;
+  const int row = gridDim.x - 1 - blockIdx.x;       // the rows that the statistics read last are the ones still in L2
   const T* xr = logits + (size_t)row * V;
   T* gr = grad + (size_t)row * V;
   const float l = lse[row], g = gout[row];
   const long local = (long)target[row] - vocab_start;
   const float sm_term = smoothing * inv_vocab;
-  const int nvec = V / N;
+  const int nvec = vec ? V / N : 0;
+#pragma unroll 4
   for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
-    P p, o; p.load(xr + v * N);
+    P p, o;
+    *reinterpret_cast<uint4*>(p.v) = __ldcs(reinterpret_cast<const uint4*>(xr + v * N));
+    const int at = (int)(local - (long)v * N);      // of the target within this packet, if in 0..N-1
 #pragma unroll
     for (int j = 0; j < N; ++j) {
       float d = __expf(p.f(j) - l) - sm_term;
-      if ((long)(v * N + j) == local) d -= (1.f - smoothing);
+      if (j == at) d -= (1.f - smoothing);
       o.set(j, d * g);
     }
-    o.store(gr + v * N);
+    __stcs(reinterpret_cast<uint4*>(gr + v * N), *reinterpret_cast<const uint4*>(o.v));
   }
   for (int c = nvec * N + threadIdx.x; c < V; c += blockDim.x) {
     float d = __expf(to_f32<T>(xr[c]) - l) - sm_term;
@@ -317,12 +335,8 @@ void rope_apply(const void* x, void* out, const float* cos_t, const float* sin_t
 void ce_stats(const void* logits, const int64_t* target, float* stats, int rows, int V, int vocab_start, int dt,
               cudaStream_t st) {
   DISPATCH_DTYPE(dt, {
-    if (((uintptr_t)logits % 16) || (V % Pack16<T>::N)) {
-      // rows would be misaligned for 16-byte loads → scalar path through the tail loop
-      ce_stats_kernel<T><<<rows, 256, 0, st>>>((const T*)logits, target, stats, V, vocab_start);
-    } else {
-      ce_stats_kernel<T><<<rows, 256, 0, st>>>((const T*)logits, target, stats, V, vocab_start);
-    }
+    const int vec = (uintptr_t)logits % 16 == 0 && V % Pack16<T>::N == 0;
+    ce_stats_kernel<T><<<rows, 256, 0, st>>>((const T*)logits, target, stats, V, vocab_start, vec);
   });
   NXD_CUDA_CHECK(cudaGetLastError());
 }
@@ -330,8 +344,9 @@ void ce_stats(const void* logits, const int64_t* target, float* stats, int rows,
 void ce_backward(const void* logits, const int64_t* target, const float* lse, const float* gout, void* grad, int rows,
                  int V, int vocab_start, float smoothing, int vocab, int dt, cudaStream_t st) {
   DISPATCH_DTYPE(dt, {
+    const int vec = ((uintptr_t)logits | (uintptr_t)grad) % 16 == 0 && V % Pack16<T>::N == 0;
     ce_bwd_kernel<T><<<rows, 256, 0, st>>>((const T*)logits, target, lse, gout, (T*)grad, V, vocab_start, smoothing,
-                                           1.f / (float)vocab);
+                                           1.f / (float)vocab, vec);
   });
   NXD_CUDA_CHECK(cudaGetLastError());
 }

@@ -1,0 +1,79 @@
+// Gradient of an embedding table, added into the fp32 gradient buffer that the optimizer gave the weight:
+//   main_grad[id] += sum of gy[t] over all t with ids[t] == id       (fp32, ascending t: the same sum on every run)
+// One block per token; the block of an id's first occurrence sums them all, the others leave.  It replaces a dense bf16 table (filled, scattered
+// into, converted and copied: 0.6 ms at 32000 x 4096 for 2048 tokens whose rows are 17 MB).
+#include "common.cuh"
+#include "kernels.h"
+
+namespace nxd {
+namespace {
+
+constexpr int kThreads = 256;
+constexpr int kVec = 4;          // packets of 8 columns per thread and sweep: 8192 columns
+
+__global__ void __launch_bounds__(kThreads) embedding_grad_kernel(const long* __restrict__ ids, const __nv_bfloat16* __restrict__ gy,
+                                                                  float* __restrict__ main_grad, int T, int H, long V) {
+  __shared__ int list[kThreads];
+  __shared__ int warp_count[kThreads / 32];
+  const int t0 = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const long id = ids[t0];
+  if (id < 0 || id >= V) return;
+  int seen = 0;
+#pragma unroll 4
+  for (int u = tid; u < t0; u += kThreads) seen |= ids[u] == id;
+  if (__syncthreads_or(seen)) return;
+  const int nvec = H / 8;
+  for (int v0 = 0; v0 < nvec; v0 += kVec * kThreads) {
+    float acc[kVec][8];
+#pragma unroll
+    for (int i = 0; i < kVec; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    for (int base = t0; base < T; base += kThreads) {
+      const int u = base + tid;
+      const bool hit = u < T && ids[u] == id;
+      const unsigned m = __ballot_sync(0xffffffffu, hit);
+      if (lane == 0) warp_count[warp] = __popc(m);
+      __syncthreads();
+      int before = 0, n = 0;
+#pragma unroll
+      for (int w = 0; w < kThreads / 32; ++w) { if (w < warp) before += warp_count[w]; n += warp_count[w]; }
+      if (hit) list[before + __popc(m & ((1u << lane) - 1u))] = u;
+      __syncthreads();
+      for (int k = 0; k < n; ++k) {
+        const __nv_bfloat16* row = gy + (size_t)list[k] * H;
+#pragma unroll
+        for (int i = 0; i < kVec; ++i) {
+          const int v = v0 + i * kThreads + tid;
+          if (v < nvec) {
+            Pack16<__nv_bfloat16> p;
+            p.load_nc(row + v * 8);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[i][j] += p.f(j);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kVec; ++i) {
+      const int v = v0 + i * kThreads + tid;
+      if (v < nvec) {
+        float4* o = reinterpret_cast<float4*>(main_grad + (size_t)id * H + v * 8);
+        float4 a = o[0], b = o[1];
+        a.x += acc[i][0]; a.y += acc[i][1]; a.z += acc[i][2]; a.w += acc[i][3];
+        b.x += acc[i][4]; b.y += acc[i][5]; b.z += acc[i][6]; b.w += acc[i][7];
+        o[0] = a; o[1] = b;
+      }
+    }
+  }
+}
+
+}  // namespace
+
+void embedding_grad(const long* ids, const void* gy, float* main_grad, int T, int H, long V, cudaStream_t st) {
+  if (T == 0) return;
+  embedding_grad_kernel<<<T, kThreads, 0, st>>>(ids, (const __nv_bfloat16*)gy, main_grad, T, H, V);
+  NXD_CUDA_CHECK(cudaGetLastError());
+}
+
+}  // namespace nxd

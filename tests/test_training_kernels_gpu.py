@@ -1,0 +1,72 @@
+"""Kernels of the training step at the edges of their chunks: optimizer tables, embedding gradients, vocabulary loss."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("sizes", [[1, 3, 0, 8191], [8192, 8193, 5], [7] * 60 + [40000], [3000000]])
+@pytest.mark.parametrize("gdtype", [torch.float32, torch.bfloat16])
+def test_optimizer_tables(sizes, gdtype):
+    from neuronx_distributed_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(len(sizes))
+    p, m, v = ([torch.rand(n, generator=g, device="cuda") for n in sizes] for _ in range(3))
+    gr = [torch.randn(n, generator=g, device="cuda").to(gdtype) for n in sizes]
+    low = [t.bfloat16() for t in p]
+    want = []
+    scale, lr, b1, b2, eps, wd, step = 0.5, 1e-2, 0.9, 0.99, 1e-6, 0.1, 3
+    for a, b, c, d in zip(p, gr, m, v):
+        gg, a, c, d = (t.double() for t in (b, a, c, d))
+        gg = gg * scale
+        c, d = b1 * c + (1 - b1) * gg, b2 * d + (1 - b2) * gg * gg
+        a = a - lr * math.sqrt(1 - b2 ** step) / (1 - b1 ** step) * c / (d.sqrt() + eps)
+        want.append((a * (1 - lr * wd), c, d))
+    total = sum(float((t.double() ** 2).sum()) for t in gr)
+    # fp32 sums in chunks of 8192 elements and one atomic per block
+    assert abs(float(ops.optim.multi_tensor_sq_norm(gr)) - total) <= 2.0 ** -19 * max(total, 1e-9)
+    ops.optim.fused_adamw_(p, gr, m, v, lr, b1, b2, eps, wd, step, torch.tensor(scale, device="cuda"), low)
+    for i, w in enumerate(want):
+        for a, b in zip((p[i], m[i], v[i]), w):
+            if a.numel():
+                assert ((a.double() - b).abs() <= 2.0 ** -18 * (1 + b.abs())).all()
+        assert torch.equal(low[i], p[i].bfloat16())
+    before = [t.clone() for t in gr]
+    ops.optim.multi_tensor_scale_(gr, 0.25)
+    assert all(torch.equal(a, b * 0.25) for a, b in zip(gr, before))
+
+
+@pytest.mark.parametrize("T,V,H", [(1, 5, 8), (700, 3, 264), (300, 5000, 8200), (257, 1, 4096)])
+@pytest.mark.parametrize("fresh", [True, False])
+def test_embedding_gradient(T, V, H, fresh):
+    from neuronx_distributed_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(T)
+    ids = torch.randint(0, V, (T,), generator=g, device="cuda")
+    gy = torch.randn(T, H, generator=g, device="cuda").bfloat16()
+    mg = torch.randn(V, H, generator=g, device="cuda")
+    want = (torch.zeros_like(mg) if fresh else mg).double().index_add(0, ids, gy.double())
+    ops._ext.ext().embedding_grad(ids, gy, mg, fresh)
+    assert (mg.double() - want).abs().max() <= 2.0 ** -23 * T * 8          # fp32 sums of at most T terms of size 4
+
+
+@pytest.mark.parametrize("V", [8, 257, 2040, 32000, 50257])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_vocabulary_loss(V, dtype):
+    from neuronx_distributed_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(V)
+    x = (3 * torch.randn(37, V, generator=g, device="cuda")).to(dtype)
+    x[1, :V // 2] = -math.inf                                              # masked columns, whole packets of them first
+    tgt = torch.randint(V // 2, V, (37,), generator=g, device="cuda")
+    stats = ops.cross_entropy.ce_stats(x, tgt, 0)
+    lse = stats[:, 0] + torch.log(stats[:, 1])
+    want = torch.logsumexp(x.double(), -1)
+    assert (lse.double() - want).abs().max() < 2e-5
+    assert torch.equal(stats[:, 2], x.gather(1, tgt[:, None])[:, 0].float())
+    gout = torch.rand(37, generator=g, device="cuda")
+    got = ops.cross_entropy.ce_backward(x, tgt, lse, gout, 0, 0.0, V)
+    ref = (torch.softmax(x.double(), -1) - torch.nn.functional.one_hot(tgt, V)) * gout[:, None].double()
+    assert (got.double() - ref).abs().max() <= (2.0 ** -8 if dtype == torch.bfloat16 else 2e-5)
