@@ -164,31 +164,30 @@ __global__ void __launch_bounds__(256) ce_stats_kernel(const T* __restrict__ log
   const T* xr = logits + (size_t)row * V;
   float m = -INFINITY, s = 0.f, sx = 0.f;
   const int nvec = vec ? V / N : 0;                 // rows of another alignment: element by element
-  // four packets in flight and one rescaling of the sum for all of them
-  constexpr int U = 4;
-  for (int v0 = threadIdx.x; v0 < nvec; v0 += U * blockDim.x) {
-    P p[U];
+  auto take = [&](const P& p) {
     float lm = m;
 #pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (v0 + u * (int)blockDim.x < nvec) p[u].load(xr + (size_t)(v0 + u * blockDim.x) * N);
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (v0 + u * (int)blockDim.x < nvec) {
-#pragma unroll
-        for (int j = 0; j < N; ++j) lm = fmaxf(lm, p[u].f(j));
-      }
-    if (lm == -INFINITY) { sx += lm; continue; }    // nothing but masked columns so far
+    for (int j = 0; j < N; ++j) lm = fmaxf(lm, p.f(j));
     float acc = 0.f;
+    if (lm != -INFINITY) {                          // else nothing but masked columns so far
 #pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (v0 + u * (int)blockDim.x < nvec) {
+      for (int j = 0; j < N; ++j) acc += __expf(p.f(j) - lm);
+      s = s * __expf(m - lm) + acc;
+    }
 #pragma unroll
-        for (int j = 0; j < N; ++j) { const float f = p[u].f(j); acc += __expf(f - lm); sx += f; }
-      }
-    s = s * __expf(m - lm) + acc;
+    for (int j = 0; j < N; ++j) sx += p.f(j);
     m = lm;
+  };
+  int v = threadIdx.x;
+  constexpr int U = 4;                              // packets in flight per thread
+  for (; v + (U - 1) * (int)blockDim.x < nvec; v += U * blockDim.x) {
+    P p[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) p[u].load(xr + (size_t)(v + u * blockDim.x) * N);
+#pragma unroll
+    for (int u = 0; u < U; ++u) take(p[u]);
   }
+  for (; v < nvec; v += blockDim.x) { P p; p.load(xr + (size_t)v * N); take(p); }
   for (int c = nvec * N + threadIdx.x; c < V; c += blockDim.x) {  // ragged tail
     const float f = to_f32<T>(xr[c]);
     const float nm = fmaxf(m, f);

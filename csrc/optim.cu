@@ -16,8 +16,8 @@ constexpr long kChunk = 8192;   // elements of a chunk
 constexpr int kBlocksPerSm = 6;
 
 // Up to 48 tensors of a launch, cut into chunks; blocks stride over all chunks, so that the launch ends evenly whatever the sizes
-// (640 blocks of 65536 elements per launch were 4.3 per SM, five on some: a 0.67 G element step took sixteen such launches, 3.70 ms;
-// one launch of this form 3.2).
+// (640 blocks of 65536 elements per launch were 4.3 per SM, five on some).  Squared norm of 0.67 G fp32 elements: 492 -> 397 us (6.7
+// TB/s); AdamW 3.70 ms in one launch as in sixteen: its nine streams run at 5.4 TB/s either way.
 template <int DEPTH> struct ChunkTable {
   void* ptr[DEPTH][kMaxTensors];
   long numel[kMaxTensors];

@@ -76,7 +76,7 @@ class _FlashAttn(torch.autograd.Function):
     def backward(ctx, go):
         q, k, v, o, lse = ctx.saved_tensors
         e = _ext.ext()
-        _ext.count_launch(4)   # memset + prep + main + dq convert
+        _ext.count_launch(3)   # prep + main + dq convert
         dq, dk, dv = e.flash_attn_bwd(_tma_view(go), q, k, v, o, lse, bool(ctx.causal), float(ctx.scale), True)
         return dq, dk, dv, None, None
 
@@ -97,7 +97,7 @@ class _FlashAttnLse(torch.autograd.Function):
     @staticmethod
     def backward(ctx, go, g_lse):
         q, k, v, o, lse = ctx.saved_tensors
-        _ext.count_launch(4)
+        _ext.count_launch(3)
         go = torch.zeros_like(o) if go is None else go
         dlse = None if g_lse is None else g_lse.float().contiguous()
         dq, dk, dv = _ext.ext().flash_attn_bwd(_tma_view(go.to(o.dtype)), q, k, v, o, lse, bool(ctx.causal), float(ctx.scale), False, dlse)
