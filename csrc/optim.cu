@@ -6,18 +6,21 @@
 //                          (utils/adamw_fp32_optim_params.py:91-155)
 #include <algorithm>
 
+#include <cuda.h>
+
 #include "common.cuh"
 #include "kernels.h"
+#include "sm100_ptx.cuh"
 
 namespace nxd {
 
 constexpr int kMaxTensors = 48;
-constexpr long kChunk = 8192;   // elements of a chunk
+constexpr long kChunk = 4096;   // elements of a chunk
 constexpr int kBlocksPerSm = 6;
 
 // Up to 48 tensors of a launch, cut into chunks; blocks stride over all chunks, so that the launch ends evenly whatever the sizes
-// (640 blocks of 65536 elements per launch were 4.3 per SM, five on some).  Squared norm of 0.67 G fp32 elements: 492 -> 397 us (6.7
-// TB/s); AdamW 3.70 ms in one launch as in sixteen: its nine streams run at 5.4 TB/s either way.
+// (640 blocks of 65536 elements per launch were 4.3 per SM, five on some).  Squared norm of 0.67 G fp32 elements: 492 -> 397 us
+// (6.7 TB/s).
 template <int DEPTH> struct ChunkTable {
   void* ptr[DEPTH][kMaxTensors];
   long numel[kMaxTensors];
@@ -82,89 +85,151 @@ __global__ void __launch_bounds__(256) scale_kernel(const __grid_constant__ Chun
   });
 }
 
-// Bound by HBM: 16 + 14 bytes per element with fp32 gradients and a bf16 copy.  State is read and written once: streaming accesses.
-template <typename G, typename L, bool HAS_LOW>
-__global__ void __launch_bounds__(256, kBlocksPerSm) adamw_kernel(const __grid_constant__ ChunkTable<5> tab, float step_size, float beta1, float beta2,
-                                                                  float eps, float decay_pre, float decay_post, float vscale,
-                                                                  const float* __restrict__ grad_scale) {
-  // One update rule covers both AdamW forms:
-  //   p = (p * decay_pre - step_size * m / (sqrt(v * vscale) + eps)) * decay_post
-  // torch form : step_size = lr/bc1, vscale = 1/bc2, decay_pre = 1 - lr*wd, decay_post = 1
-  // HF form    : step_size = lr*sqrt(bc2)/bc1, vscale = 1, decay_pre = 1, decay_post = 1 - lr*wd
-  //              (reference utils/adamw_fp32_optim_params.py:130-155: eps added before bias correction, decay applied last)
-  const float gs = grad_scale ? *grad_scale : 1.f;
-  auto update = [&](float g, float& m, float& v, float p) {
-    const float gr = g * gs;
+// One update rule covers both AdamW forms:
+//   p = (p * decay_pre - step_size * m / (sqrt(v * vscale) + eps)) * decay_post
+// torch form : step_size = lr/bc1, vscale = 1/bc2, decay_pre = 1 - lr*wd, decay_post = 1
+// HF form    : step_size = lr*sqrt(bc2)/bc1, vscale = 1, decay_pre = 1, decay_post = 1 - lr*wd
+//              (reference utils/adamw_fp32_optim_params.py:130-155: eps added before bias correction, decay applied last)
+struct AdamRule {
+  float step_size, beta1, beta2, eps, decay_pre, decay_post, vscale;
+  NXD_DEVICE float operator()(float gr, float& m, float& v, float p) const {
     m = beta1 * m + (1.f - beta1) * gr;
     v = beta2 * v + (1.f - beta2) * gr * gr;
     return (p * decay_pre - step_size * m / (sqrtf(v * vscale) + eps)) * decay_post;
+  }
+};
+
+constexpr int kAdamThreads = 512;
+constexpr int kAdamStages = 3;
+constexpr int kAdamStage = 5 * (int)kChunk * 4 - (int)kChunk * 2;       // p, g, m, v and a 16-bit copy: 72 KB
+constexpr int kAdamSmem = kAdamStages * kAdamStage + 64;
+
+// Bound by HBM: 16 + 14 bytes per element with fp32 gradients and a bf16 copy, in nine streams.  Whole chunks travel as bulk copies
+// of 16 KB through a ring in shared memory, updated in place there: a stream's bytes reach a DRAM page together.  0.67 G elements:
+// 3.09 ms (6.5 TB/s); with 16-byte accesses per thread 3.70 (5.4), however the blocks were cut.  Chunks that are short or unaligned
+// are updated in global memory.
+template <typename G, typename L, bool HAS_LOW>
+__global__ void __launch_bounds__(kAdamThreads, 1) adamw_kernel(const __grid_constant__ ChunkTable<5> tab, const AdamRule rule,
+                                                                const float* __restrict__ grad_scale) {
+  extern __shared__ __align__(128) uint8_t adam_smem[];
+  const uint32_t base = smem_u32(adam_smem), bars = base + kAdamStages * kAdamStage;
+  const float gs = grad_scale ? *grad_scale : 1.f;
+  const long total = tab.first[tab.tensors];
+  const int tid = threadIdx.x;
+  if (tid == 0) {
+    for (int i = 0; i < kAdamStages; ++i) mbar_init(bars + 8 * i, 1);
+    fence_barrier_init();
+  }
+  __syncthreads();
+  struct Chunk { float *p, *m, *v; const G* g; L* low; int n; bool bulk; };
+  int t_at = 0;                                    // chunks are visited in ascending order
+  auto find = [&](long c, int& t) {
+    while (tab.first[t + 1] <= c) ++t;
+    const long off = (c - tab.first[t]) * kChunk;
+    Chunk k;
+    k.p = (float*)tab.ptr[0][t] + off; k.g = (const G*)tab.ptr[1][t] + off;
+    k.m = (float*)tab.ptr[2][t] + off; k.v = (float*)tab.ptr[3][t] + off;
+    k.low = HAS_LOW ? (L*)tab.ptr[4][t] + off : nullptr;
+    k.n = (int)min(tab.numel[t] - off, kChunk);
+    k.bulk = k.n == kChunk && (((uintptr_t)k.p | (uintptr_t)k.g | (uintptr_t)k.m | (uintptr_t)k.v | (uintptr_t)k.low) % 16) == 0;
+    return k;
   };
-  each_chunk(tab, [&](int t, long base, long n) {
-    float* p = (float*)tab.ptr[0][t] + base;
-    const G* g = (const G*)tab.ptr[1][t] + base;
-    float* m = (float*)tab.ptr[2][t] + base;
-    float* v = (float*)tab.ptr[3][t] + base;
-    L* low = HAS_LOW ? (L*)tab.ptr[4][t] + base : nullptr;
-    // 4 elements / thread / iteration: fp32 state moves as 16-byte packets
-    const bool aligned = ((uintptr_t)p % 16 == 0) && ((uintptr_t)m % 16 == 0) && ((uintptr_t)v % 16 == 0) &&
-                         ((uintptr_t)g % (4 * sizeof(G)) == 0) && (!HAS_LOW || (uintptr_t)low % (4 * sizeof(L)) == 0);
-    long i0 = 0;
-    if (aligned) {
-      const long nv = n / 4;
-#pragma unroll 2
-      for (long q = threadIdx.x; q < nv; q += 256) {
-        float4 pp = __ldcs(reinterpret_cast<float4*>(p + q * 4));
-        float4 mm = __ldcs(reinterpret_cast<float4*>(m + q * 4));
-        float4 vv = __ldcs(reinterpret_cast<float4*>(v + q * 4));
+  constexpr uint32_t F = (uint32_t)kChunk * 4, GB = (uint32_t)kChunk * sizeof(G), LB = (uint32_t)kChunk * sizeof(L);
+  static_assert(4 * kChunk * 4 + kChunk * 2 == kAdamStage && sizeof(L) <= 4, "stage layout");
+  // an fp32 copy equals p and is stored from there
+  auto load = [&](const Chunk& k, int st) {        // thread 0
+    const uint32_t s = base + st * kAdamStage, bar = bars + 8 * st;
+    mbar_expect_tx(bar, 3 * F + GB);
+    auto copy = [&](uint32_t dst, const void* src, uint32_t bytes) {
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                   ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+    };
+    copy(s, k.p, F); copy(s + F, k.m, F); copy(s + 2 * F, k.v, F); copy(s + 3 * F, k.g, GB);
+  };
+  auto store = [&](void* dst, uint32_t src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
+  };
+  int t_load = 0;
+  long next = blockIdx.x;                          // next chunk to ask for (thread 0)
+  auto load_next = [&](int st) {
+    if (next < total) {
+      const Chunk k = find(next, t_load);
+      if (k.bulk) load(k, st);
+    }
+    next += gridDim.x;
+  };
+  if (tid == 0) { load_next(0); load_next(1); }
+  uint32_t phases = 0;                             // parity of each stage's barrier
+  int st = 0;
+  for (long c = blockIdx.x; c < total; c += gridDim.x) {
+    const Chunk k = find(c, t_at);
+    if (k.bulk) {
+      mbar_wait(bars + 8 * st, (phases >> st) & 1u);
+      phases ^= 1u << st;
+      uint8_t* s = adam_smem + st * kAdamStage;
+      float4* sp = reinterpret_cast<float4*>(s);
+      float4* sm = reinterpret_cast<float4*>(s + F);
+      float4* sv = reinterpret_cast<float4*>(s + 2 * F);
+#pragma unroll
+      for (int q = tid; q < (int)kChunk / 4; q += kAdamThreads) {
+        float4 pp = sp[q], mm = sm[q], vv = sv[q];
         float gg[4];
         if constexpr (sizeof(G) == 4) {
-          const float4 t4 = __ldcs(reinterpret_cast<const float4*>(g + q * 4));
+          const float4 t4 = reinterpret_cast<const float4*>(s + 3 * F)[q];
           gg[0] = t4.x; gg[1] = t4.y; gg[2] = t4.z; gg[3] = t4.w;
         } else {
-          const uint2 raw = __ldcs(reinterpret_cast<const uint2*>(g + q * 4));
+          const uint2 raw = reinterpret_cast<const uint2*>(s + 3 * F)[q];
           const G* h = reinterpret_cast<const G*>(&raw);
 #pragma unroll
           for (int j = 0; j < 4; ++j) gg[j] = to_f32<G>(h[j]);
         }
         float* pa = &pp.x; float* ma = &mm.x; float* va = &vv.x;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) pa[j] = update(gg[j], ma[j], va[j], pa[j]);
-        __stcs(reinterpret_cast<float4*>(p + q * 4), pp);
-        __stcs(reinterpret_cast<float4*>(m + q * 4), mm);
-        __stcs(reinterpret_cast<float4*>(v + q * 4), vv);
-        if constexpr (HAS_LOW) {
-          if constexpr (sizeof(L) == 4) {
-            *reinterpret_cast<float4*>(low + q * 4) = pp;
-          } else {
-            uint2 raw; L* h = reinterpret_cast<L*>(&raw);
+        for (int j = 0; j < 4; ++j) pa[j] = rule(gg[j] * gs, ma[j], va[j], pa[j]);
+        sp[q] = pp; sm[q] = mm; sv[q] = vv;
+        if constexpr (HAS_LOW && sizeof(L) == 2) {
+          uint2 raw; L* h = reinterpret_cast<L*>(&raw);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) h[j] = from_f32<L>(pa[j]);
-            *reinterpret_cast<uint2*>(low + q * 4) = raw;
-          }
+          for (int j = 0; j < 4; ++j) h[j] = from_f32<L>(pa[j]);
+          reinterpret_cast<uint2*>(s + 4 * F)[q] = raw;
         }
       }
-      i0 = nv * 4;
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    } else {
+      for (int i = tid; i < k.n; i += kAdamThreads) {
+        float mi = k.m[i], vi = k.v[i];
+        const float pi = rule(to_f32<G>(k.g[i]) * gs, mi, vi, k.p[i]);
+        k.m[i] = mi; k.v[i] = vi; k.p[i] = pi;
+        if constexpr (HAS_LOW) k.low[i] = from_f32<L>(pi);
+      }
     }
-    for (long i = i0 + threadIdx.x; i < n; i += 256) {
-      float mi = m[i], vi = v[i];
-      const float pi = update(to_f32<G>(g[i]), mi, vi, p[i]);
-      m[i] = mi; v[i] = vi; p[i] = pi;
-      if constexpr (HAS_LOW) low[i] = from_f32<L>(pi);
+    __syncthreads();
+    if (tid == 0) {
+      if (k.bulk) {
+        const uint32_t s = base + st * kAdamStage;
+        store(k.p, s, F); store(k.m, s + F, F); store(k.v, s + 2 * F, F);
+        if constexpr (HAS_LOW) store(k.low, sizeof(L) == 2 ? s + 4 * F : s, LB);
+      }
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");      // the stage before has left: it takes the chunk after the next
+      load_next((st + 2) % kAdamStages);
     }
-  });
+    st = (st + 1) % kAdamStages;
+  }
+  if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
 int device_sm_count();
 
 // launches once per 48 tensors
 template <int DEPTH, typename Launch>
-static void run_tables(const std::vector<TensorRef>* lists, Launch&& launch) {
+static void run_tables(const std::vector<TensorRef>* lists, int blocks_per_sm, Launch&& launch) {
   ChunkTable<DEPTH> tab;
   tab.tensors = 0;
   tab.first[0] = 0;
   auto flush = [&]() {
     const long chunks = tab.first[tab.tensors];
-    if (chunks > 0) launch(tab, (int)std::min<long>(chunks, (long)device_sm_count() * kBlocksPerSm));
+    if (chunks > 0) launch(tab, (int)std::min<long>(chunks, (long)device_sm_count() * blocks_per_sm));
     tab.tensors = 0;
   };
   for (size_t t = 0; t < lists[0].size(); ++t) {
@@ -181,7 +246,7 @@ static void run_tables(const std::vector<TensorRef>* lists, Launch&& launch) {
 
 void multi_tensor_sq_norm(const std::vector<TensorRef>& ts, int dt, float* out, cudaStream_t st) {
   const std::vector<TensorRef> lists[1] = {ts};
-  run_tables<1>(lists, [&](const ChunkTable<1>& tab, int nb) {
+  run_tables<1>(lists, kBlocksPerSm, [&](const ChunkTable<1>& tab, int nb) {
     switch (dt) {
       case kF32: sq_norm_kernel<float><<<nb, 256, 0, st>>>(tab, out); break;
       case kBF16: sq_norm_kernel<__nv_bfloat16><<<nb, 256, 0, st>>>(tab, out); break;
@@ -194,7 +259,7 @@ void multi_tensor_sq_norm(const std::vector<TensorRef>& ts, int dt, float* out, 
 
 void multi_tensor_scale(const std::vector<TensorRef>& ts, int dt, const float* scale, cudaStream_t st) {
   const std::vector<TensorRef> lists[1] = {ts};
-  run_tables<1>(lists, [&](const ChunkTable<1>& tab, int nb) {
+  run_tables<1>(lists, kBlocksPerSm, [&](const ChunkTable<1>& tab, int nb) {
     switch (dt) {
       case kF32: scale_kernel<float><<<nb, 256, 0, st>>>(tab, scale); break;
       case kBF16: scale_kernel<__nv_bfloat16><<<nb, 256, 0, st>>>(tab, scale); break;
@@ -211,12 +276,14 @@ void fused_adamw(const std::vector<TensorRef>& p, const std::vector<TensorRef>& 
                  int hf_form, cudaStream_t st) {
   const std::vector<TensorRef> lists[5] = {p, g, m, v, lowp};
   const bool has_low = !lowp.empty();
-  const float step_size = hf_form ? lr * sqrtf(bc2) / bc1 : lr / bc1;
-  const float vscale = hf_form ? 1.f : 1.f / bc2;
-  const float decay_pre = hf_form ? 1.f : 1.f - lr * wd;
-  const float decay_post = hf_form ? 1.f - lr * wd : 1.f;
-  run_tables<5>(lists, [&](const ChunkTable<5>& tab, int nb) {
-#define LAUNCH(G, L, HL) adamw_kernel<G, L, HL><<<nb, 256, 0, st>>>(tab, step_size, beta1, beta2, eps, decay_pre, decay_post, vscale, grad_scale)
+  AdamRule rule{hf_form ? lr * sqrtf(bc2) / bc1 : lr / bc1, beta1, beta2, eps, hf_form ? 1.f : 1.f - lr * wd, hf_form ? 1.f - lr * wd : 1.f,
+                hf_form ? 1.f : 1.f / bc2};
+  run_tables<5>(lists, 1, [&](const ChunkTable<5>& tab, int nb) {
+#define LAUNCH(G, L, HL)                                                                                                     \
+  do {                                                                                                                       \
+    NXD_CUDA_CHECK(cudaFuncSetAttribute(adamw_kernel<G, L, HL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAdamSmem));    \
+    adamw_kernel<G, L, HL><<<nb, kAdamThreads, kAdamSmem, st>>>(tab, rule, grad_scale);                                      \
+  } while (0)
     if (gdt == kF32) {
       if (!has_low) LAUNCH(float, float, false);
       else if (ldt == kBF16) LAUNCH(float, __nv_bfloat16, true);
