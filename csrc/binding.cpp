@@ -585,7 +585,11 @@ static void gemm_bf16_2cta(const Tensor& a, const Tensor& b, Tensor out, bool tr
   const int N = (int)(trans_b ? b.size(0) : b.size(1));
   TORCH_CHECK((trans_b ? b.size(1) : b.size(0)) == K && out.size(0) == M && out.size(1) == N, "gemm shape mismatch");
   c10::cuda::CUDAGuard g(a.device());
-  nxd::gemm_bf16_2cta(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, trans_a, trans_b, dt_code(out), accumulate, stream());
+  const size_t bytes = nxd::gemm_2cta_workspace(M, N, K, dt_code(out), accumulate);
+  Tensor ws;
+  if (bytes) ws = at::empty({(int64_t)(bytes / 4)}, a.options().dtype(at::kFloat));
+  nxd::gemm_bf16_2cta(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, trans_a, trans_b, dt_code(out), accumulate,
+                      bytes ? ws.data_ptr<float>() : nullptr, stream());
 }
 
 // all-gather(A shards along rows) → GEMM.  `a_shard` [M/world, K]; gathered A lives in the symmetric payload at

@@ -9,6 +9,7 @@
 //   warps 2-5 epilogue   (both)
 #include <cuda.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <string>
 
@@ -31,13 +32,30 @@ struct Group {
   int block_rows, b_rows, groups;
 };
 
-// one unit of work of a pair: an output tile and its range of k-blocks
-struct Unit { int m_blk, n_blk, mat, kb0, kb1; };
+// The tiles of the last, partial round of pairs (`tiles` of them, at most half as many as pairs) are split along K over `splits`
+// pairs each, `kb_per` k-blocks apiece; their fp32 partials go to a workspace [tiles * splits][256][256] that gemm_tail_kernel
+// sums.  80 tiles on 74 pairs took two tiles' time for 1.08 of work.
+struct Tail { int tiles, splits, kb_per; };
+
+// one unit of work of a pair: an output tile and its range of k-blocks; `part`: a split of a tail tile, number `mat`
+struct Unit { int m_blk, n_blk, mat, kb0, kb1; bool part; };
 
 template <int MODE>
-NXD_DEVICE Unit unit_of(int unit, int num_tiles, int tiles_m, int tiles_n, int num_kb, int kb_per, const Group& g) {
+NXD_DEVICE Unit unit_of(int unit, int num_tiles, int tiles_m, int tiles_n, int num_kb, int kb_per, const Group& g, const Tail& tail) {
   Unit u;
   u.mat = 0;
+  u.part = false;
+  if constexpr (MODE == 0) {
+    const int x = unit - (num_tiles - tail.tiles);
+    if (tail.tiles > 0 && x >= 0) {                        // never together with split_k
+      u.part = true;
+      u.mat = x;
+      tile_coords(num_tiles - tail.tiles + x / tail.splits, tiles_m, tiles_n, u.m_blk, u.n_blk);
+      u.kb0 = x % tail.splits * tail.kb_per;
+      u.kb1 = min(num_kb, u.kb0 + tail.kb_per);
+      return u;
+    }
+  }
   if constexpr (MODE == 4) {
     const int per = tiles_m * tiles_n;
     u.mat = unit / per;
@@ -56,8 +74,8 @@ NXD_DEVICE Unit unit_of(int unit, int num_tiles, int tiles_m, int tiles_n, int n
 template <bool A_KMAJOR, bool B_KMAJOR, typename OutT, int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                      const __grid_constant__ CUtensorMap tma_out, OutT* __restrict__ out, int M, int N, int K, int accumulate,
-                      int split_k, const Group grp) {
+                      const __grid_constant__ CUtensorMap tma_out, const __grid_constant__ CUtensorMap tma_part, OutT* __restrict__ out,
+                      int M, int N, int K, int accumulate, int split_k, const Group grp, const Tail tail) {
   // accumulate: 0 store, 1 add to what is there.  split_k > 1 (fp32 outputs): that many pairs share one output tile, each sums
   // a K range and adds its partial — for weight gradients whose output has too few tiles to fill the 74 pairs while
   // K = tokens is long.  fp32 outputs always leave through TMA (stored or added in memory), bf16 ones unless they accumulate.
@@ -78,7 +96,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   const int num_tiles = (MODE == 4 ? grp.groups : 1) * tiles_m * tiles_n;
   const int num_kb = (K + BK - 1) / BK;
   const int kb_per = (num_kb + split_k - 1) / split_k;       // k-blocks per split (host guarantees no empty split)
-  const int num_units = num_tiles * split_k;
+  const int num_units = num_tiles * split_k + tail.tiles * (tail.splits - 1);
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
 
   if (warp == 0 && lane == 0) {
@@ -106,7 +124,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     if (lane == 0) {
       int stage = 0; uint32_t phase = 0;
       for (int unit = pair; unit < num_units; unit += num_pairs) {
-        const Unit u = unit_of<MODE>(unit, num_tiles, tiles_m, tiles_n, num_kb, kb_per, grp);
+        const Unit u = unit_of<MODE>(unit, num_tiles, tiles_m, tiles_n, num_kb, kb_per, grp, tail);
         const int m0 = u.m_blk * TILE_M + (int)cta * CTA_M;
         const int n0 = u.n_blk * TILE_N + (int)cta * HALF_N;
         int b_off = 0;
@@ -141,7 +159,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       constexpr uint32_t idesc = make_idesc(!A_KMAJOR, !B_KMAJOR, TILE_M, TILE_N);
       int stage = 0; uint32_t phase = 0; int as = 0; uint32_t aphase = 0;
       for (int unit = pair; unit < num_units; unit += num_pairs) {
-        const Unit u = unit_of<MODE>(unit, num_tiles, tiles_m, tiles_n, num_kb, kb_per, grp);
+        const Unit u = unit_of<MODE>(unit, num_tiles, tiles_m, tiles_n, num_kb, kb_per, grp, tail);
         mbar_wait(bar_tempty + 8 * as, aphase ^ 1);
         tcgen05_fence_after();
         const uint32_t tmem_d = tmem_base + as * TILE_N;
@@ -172,13 +190,16 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     uint32_t slab_ctr = 0;
     int as = 0; uint32_t aphase = 0;
     for (int unit = pair; unit < num_units; unit += num_pairs) {
-      const Unit u = unit_of<MODE>(unit, num_tiles, tiles_m, tiles_n, num_kb, kb_per, grp);
+      const Unit u = unit_of<MODE>(unit, num_tiles, tiles_m, tiles_n, num_kb, kb_per, grp, tail);
       mbar_wait(bar_tfull + 8 * as, aphase);
       tcgen05_fence_after();
       const int n0 = u.n_blk * TILE_N, row0 = u.m_blk * TILE_M + (int)cta * CTA_M;
       const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + as * TILE_N;
       const bool empty = MODE == 4 && u.kb0 == u.kb1;
-      if constexpr (sizeof(OutT) == 4) {
+      if (MODE == 0 && u.part) {
+        epilogue_tile_tma_f32(acc, smem_base + kEpiOffset, &tma_part, (int)cta * CTA_M, u.mat, 0, TILE_N, q, lane, issuer, slab_ctr,
+                              false, false);
+      } else if constexpr (sizeof(OutT) == 4) {
         epilogue_tile_tma_f32(acc, smem_base + kEpiOffset, &tma_out, row0, u.mat, n0, N, q, lane, issuer, slab_ctr,
                               accumulate || split_k > 1, empty);
       } else if (!accumulate) {
@@ -206,6 +227,34 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   tcgen05_fence_before();
   cluster_sync_all();               // peer must be done with our smem/TMEM before teardown
   if (warp == 1) { __syncwarp(); tcgen05_dealloc_2cta(tmem_base, kTmemCols); }
+}
+
+// out tile (+)= sum of its splits' partials, in order: one thread per 8 columns of a row
+template <typename OutT>
+__global__ void __launch_bounds__(256) gemm_tail_kernel(const float* __restrict__ part, OutT* __restrict__ out, int M, int N, int first,
+                                                        int tiles_m, int tiles_n, int splits, int accumulate) {
+  const int t = blockIdx.y, row = blockIdx.x * 8 + (threadIdx.x >> 5), col = (threadIdx.x & 31) * 8;
+  int m_blk, n_blk;
+  tile_coords(first + t, tiles_m, tiles_n, m_blk, n_blk);
+  const int gr = m_blk * TILE_M + row, gc = n_blk * TILE_N + col;
+  if (gr >= M || gc >= N) return;                          // N is a multiple of 8
+  const float* src = part + ((size_t)t * splits * TILE_M + row) * TILE_N + col;
+  float a[8] = {};
+#pragma unroll 4
+  for (int s = 0; s < splits; ++s) {
+    const float4 x = *reinterpret_cast<const float4*>(src + (size_t)s * TILE_M * TILE_N);
+    const float4 y = *reinterpret_cast<const float4*>(src + (size_t)s * TILE_M * TILE_N + 4);
+    a[0] += x.x; a[1] += x.y; a[2] += x.z; a[3] += x.w; a[4] += y.x; a[5] += y.y; a[6] += y.z; a[7] += y.w;
+  }
+  OutT* dst = out + (size_t)gr * N + gc;
+#pragma unroll
+  for (int v = 0; v < 8; v += Pack16<OutT>::N) {
+    Pack16<OutT> o;
+    if (accumulate) o.load(dst + v);
+#pragma unroll
+    for (int j = 0; j < Pack16<OutT>::N; ++j) o.set(j, accumulate ? a[v + j] + o.f(j) : a[v + j]);
+    o.store(dst + v);
+  }
 }
 
 
@@ -713,15 +762,15 @@ int device_sm_count();
 CUtensorMap make_tmap_mats(const void* ptr, bool f32, uint64_t mats, uint64_t rows, uint64_t cols, uint32_t box_cols, uint32_t box_rows);
 
 template <bool AK, bool BK_, typename OutT, int MODE = 0>
-static void launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& to, void* out, int M, int N, int K,
-                    int accumulate, int split_k, const g2::Group& grp, int grid, cudaStream_t st) {
+static void launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& to, const CUtensorMap& tp, void* out, int M, int N, int K,
+                    int accumulate, int split_k, const g2::Group& grp, const g2::Tail& tail, int grid, cudaStream_t st) {
   auto kern = g2::gemm_bf16_2cta_kernel<AK, BK_, OutT, MODE>;
   static bool configured = false;
   if (!configured) {
     NXD_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, g2::kSmem));
     configured = true;
   }
-  kern<<<grid, g2::kThreads, g2::kSmem, st>>>(ta, tb, to, (OutT*)out, M, N, K, accumulate, split_k, grp);
+  kern<<<grid, g2::kThreads, g2::kSmem, st>>>(ta, tb, to, tp, (OutT*)out, M, N, K, accumulate, split_k, grp, tail);
   NXD_CUDA_CHECK(cudaGetLastError());
 }
 
@@ -733,47 +782,86 @@ static CUtensorMap out_map(const void* out, int out_dt, bool accumulate, bool ma
   return mats ? make_tmap_mats(out, false, groups, M, N, g2::kEpiSlabCols, g2::CTA_M) : make_tmap_bf16(out, M, N, g2::kEpiSlabCols, g2::CTA_M);
 }
 
-void gemm_bf16_2cta(const void* a, const void* b, void* out, int M, int N, int K, bool trans_a, bool trans_b, int out_dt,
-                    bool accumulate, cudaStream_t st) {
-  const bool AK = !trans_a, BK_ = trans_b;
-  const CUtensorMap ta = AK ? make_tmap_bf16(a, M, K, g2::BK, g2::CTA_M) : make_tmap_bf16(a, K, M, 64, g2::BK);
-  const CUtensorMap tb = BK_ ? make_tmap_bf16(b, N, K, g2::BK, g2::HALF_N) : make_tmap_bf16(b, K, N, 64, g2::BK);
-  const CUtensorMap to = out_map(out, out_dt, accumulate, false, 1, M, N, ta);
-  const int tiles = ((M + g2::TILE_M - 1) / g2::TILE_M) * ((N + g2::TILE_N - 1) / g2::TILE_N);
-  const int pairs = device_sm_count() / 2;
+// How a product is shared out: split-K of every tile (fp32 outputs), or of the last round's tiles alone, or neither.  Time of a
+// 256 x 256 tile: 0.39 us per k-block; a pass over fp32 memory: 6 bytes/ps.
+struct GemmPlan { int tiles, split; g2::Tail tail; };
+static GemmPlan gemm_plan(int M, int N, int K, int out_dt, bool accumulate) {
+  const int pairs = device_sm_count() / 2, num_kb = (K + g2::BK - 1) / g2::BK;
+  GemmPlan p;
+  p.tiles = ((M + g2::TILE_M - 1) / g2::TILE_M) * ((N + g2::TILE_N - 1) / g2::TILE_N);
+  p.split = 1;
+  p.tail = g2::Tail{0, 1, num_kb};
+  const double kb_us = 0.39;
+  double best = (double)((p.tiles + pairs - 1) / pairs) * num_kb * kb_us;
+  // The tail: s pairs per tile, at least 4 k-blocks each; worth it where it saves more than the launch that sums (3 us) and its traffic.
+  // 1000 x 5120 x 13824 (80 tiles): 104 us, 143 with a second round of six tiles; cut into narrower columns instead, its pieces waited
+  // for their loads as long as a whole tile.  1000 x 27648 x 5120 from [K, N] weights: 203, 281 before.
+  const int last = p.tiles % pairs;
+  int s = last > 0 ? std::min(16, std::min(pairs / last, num_kb / 4)) : 1;
+  if (s > 1) {
+    const int per = (num_kb + s - 1) / s;
+    s = (num_kb + per - 1) / per;                          // no empty split
+    const double cost = (p.tiles / pairs) * num_kb * kb_us + per * kb_us + 3.0 + 2.0 * last * s * 0.262144 / 6.0;
+    if (s > 1 && cost < best) { best = cost; p.tail = g2::Tail{last, s, per}; }
+  }
   // Split-K for fp32 outputs (weight gradients): K = tokens is long while the output often has fewer tiles than the
-  // chip has CTA pairs (TP=8: 32-176 tiles on 74 pairs).  A split is taken where the waves it saves (0.39 us per k-block of a
-  // 256 x 256 tile) cost more than its traffic: zeroing the output first and one more pass over it per further partial, at
-  // 6 bytes/ps; every split keeps >= 16 k-blocks so that the main loop still amortises its epilogue.
-  int split = 1;
+  // chip has CTA pairs (TP=8: 32-176 tiles on 74 pairs).  A split is taken where the waves it saves cost more than its traffic:
+  // zeroing the output first and one more pass over it per further partial; every split keeps >= 16 k-blocks so that the main
+  // loop still amortises its epilogue.
   const char* split_env = getenv("NXD_GEMM_SPLITK");            // re-read per call: A/B sweeps toggle it at run time
-  const bool split_enabled = !(split_env && split_env[0] == '0');
-  const int num_kb = (K + g2::BK - 1) / g2::BK;
-  if (out_dt == kF32 && split_enabled) {
+  if (out_dt == kF32 && !(split_env && split_env[0] == '0')) {
     const double pass_us = (double)M * N * 4 / 6e6;
-    double best = (double)((tiles + pairs - 1) / pairs) * num_kb * 0.39;
     for (int s2 = 2; s2 <= 8; ++s2) {
       if (num_kb / s2 < 16) break;
       const int per = (num_kb + s2 - 1) / s2;
       if (per * (s2 - 1) >= num_kb) continue;                       // would leave an empty split
-      const double cost = (double)((tiles * s2 + pairs - 1) / pairs) * per * 0.39 + (s2 - 1) * pass_us + (accumulate ? 0. : pass_us);
-      if (cost < best) { best = cost; split = s2; }
+      const double cost = (double)((p.tiles * s2 + pairs - 1) / pairs) * per * kb_us + (s2 - 1) * pass_us + (accumulate ? 0. : pass_us);
+      if (cost < best) { best = cost; p.split = s2; p.tail = g2::Tail{0, 1, num_kb}; }
     }
   }
+  return p;
+}
+
+// bytes of fp32 workspace that gemm_bf16_2cta takes for these sizes (0: none)
+size_t gemm_2cta_workspace(int M, int N, int K, int out_dt, bool accumulate) {
+  const GemmPlan p = gemm_plan(M, N, K, out_dt, accumulate);
+  return (size_t)p.tail.tiles * p.tail.splits * g2::TILE_M * g2::TILE_N * sizeof(float);
+}
+
+// `workspace`: gemm_2cta_workspace bytes, 16-byte aligned, or null: then no tail is split
+void gemm_bf16_2cta(const void* a, const void* b, void* out, int M, int N, int K, bool trans_a, bool trans_b, int out_dt,
+                    bool accumulate, float* workspace, cudaStream_t st) {
+  const bool AK = !trans_a, BK_ = trans_b;
+  const CUtensorMap ta = AK ? make_tmap_bf16(a, M, K, g2::BK, g2::CTA_M) : make_tmap_bf16(a, K, M, 64, g2::BK);
+  const CUtensorMap tb = BK_ ? make_tmap_bf16(b, N, K, g2::BK, g2::HALF_N) : make_tmap_bf16(b, K, N, 64, g2::BK);
+  const CUtensorMap to = out_map(out, out_dt, accumulate, false, 1, M, N, ta);
+  GemmPlan p = gemm_plan(M, N, K, out_dt, accumulate);
+  if (!workspace) p.tail = g2::Tail{0, 1, 1};
+  const int pairs = device_sm_count() / 2, split = p.split;
   if (split > 1 && !accumulate) NXD_CUDA_CHECK(cudaMemsetAsync(out, 0, (size_t)M * N * sizeof(float), st));   // partials add into zeros
-  const int units = tiles * split;
+  const CUtensorMap tp = p.tail.tiles ? make_tmap_mats(workspace, true, (uint64_t)p.tail.tiles * p.tail.splits, g2::TILE_M, g2::TILE_N, 32, g2::CTA_M) : ta;
+  const int units = p.tiles * split + p.tail.tiles * (p.tail.splits - 1);
   const int grid = 2 * (units < pairs ? units : pairs);
   const g2::Group none{};
 #define NXD_L2(AKv, BKv)                                                                          \
   do {                                                                                            \
-    if (out_dt == kBF16) launch2<AKv, BKv, __nv_bfloat16>(ta, tb, to, out, M, N, K, accumulate, split, none, grid, st); \
-    else launch2<AKv, BKv, float>(ta, tb, to, out, M, N, K, accumulate, split, none, grid, st);   \
+    if (out_dt == kBF16) launch2<AKv, BKv, __nv_bfloat16>(ta, tb, to, tp, out, M, N, K, accumulate, split, none, p.tail, grid, st); \
+    else launch2<AKv, BKv, float>(ta, tb, to, tp, out, M, N, K, accumulate, split, none, p.tail, grid, st); \
   } while (0)
   if (AK && BK_) NXD_L2(true, true);
   else if (AK && !BK_) NXD_L2(true, false);
   else if (!AK && !BK_) NXD_L2(false, false);
   else NXD_L2(false, true);
 #undef NXD_L2
+  if (p.tail.tiles) {
+    const int tiles_m = (M + g2::TILE_M - 1) / g2::TILE_M, tiles_n = (N + g2::TILE_N - 1) / g2::TILE_N;
+    const dim3 tg(g2::TILE_M / 8, p.tail.tiles);
+    if (out_dt == kBF16)
+      g2::gemm_tail_kernel<__nv_bfloat16><<<tg, 256, 0, st>>>(workspace, (__nv_bfloat16*)out, M, N, p.tiles - p.tail.tiles, tiles_m, tiles_n, p.tail.splits, accumulate);
+    else
+      g2::gemm_tail_kernel<float><<<tg, 256, 0, st>>>(workspace, (float*)out, M, N, p.tiles - p.tail.tiles, tiles_m, tiles_n, p.tail.splits, accumulate);
+    NXD_CUDA_CHECK(cudaGetLastError());
+  }
 }
 
 // Grouped GEMMs of routed experts whose row blocks are multiples of 256 rows (see grouped_gemm_bf16 / grouped_wgrad_bf16).
@@ -786,11 +874,11 @@ void grouped_gemm_bf16_2cta(const void* a, const void* b, void* out, int M, int 
   const int tiles = ((M + g2::TILE_M - 1) / g2::TILE_M) * ((N + g2::TILE_N - 1) / g2::TILE_N), pairs = device_sm_count() / 2;
   const int grid = 2 * (tiles < pairs ? tiles : pairs);
   if (trans_b) {
-    if (out_dt == kBF16) launch2<true, true, __nv_bfloat16, 3>(ta, tb, to, out, M, N, K, 0, 1, grp, grid, st);
-    else launch2<true, true, float, 3>(ta, tb, to, out, M, N, K, 0, 1, grp, grid, st);
+    if (out_dt == kBF16) launch2<true, true, __nv_bfloat16, 3>(ta, tb, to, to, out, M, N, K, 0, 1, grp, g2::Tail{0, 1, 1}, grid, st);
+    else launch2<true, true, float, 3>(ta, tb, to, to, out, M, N, K, 0, 1, grp, g2::Tail{0, 1, 1}, grid, st);
   } else {
-    if (out_dt == kBF16) launch2<true, false, __nv_bfloat16, 3>(ta, tb, to, out, M, N, K, 0, 1, grp, grid, st);
-    else launch2<true, false, float, 3>(ta, tb, to, out, M, N, K, 0, 1, grp, grid, st);
+    if (out_dt == kBF16) launch2<true, false, __nv_bfloat16, 3>(ta, tb, to, to, out, M, N, K, 0, 1, grp, g2::Tail{0, 1, 1}, grid, st);
+    else launch2<true, false, float, 3>(ta, tb, to, to, out, M, N, K, 0, 1, grp, g2::Tail{0, 1, 1}, grid, st);
   }
 }
 
@@ -802,8 +890,8 @@ void grouped_wgrad_bf16_2cta(const void* a, const void* b, void* out, int rows_t
   const g2::Group grp{nullptr, seg_first_block, nullptr, block_rows, 0, E};
   const int tiles = E * ((Mo + g2::TILE_M - 1) / g2::TILE_M) * ((No + g2::TILE_N - 1) / g2::TILE_N), pairs = device_sm_count() / 2;
   const int grid = 2 * (tiles < pairs ? tiles : pairs);
-  if (out_dt == kBF16) launch2<false, false, __nv_bfloat16, 4>(ta, tb, to, out, Mo, No, rows_total, accumulate, 1, grp, grid, st);
-  else launch2<false, false, float, 4>(ta, tb, to, out, Mo, No, rows_total, accumulate, 1, grp, grid, st);
+  if (out_dt == kBF16) launch2<false, false, __nv_bfloat16, 4>(ta, tb, to, to, out, Mo, No, rows_total, accumulate, 1, grp, g2::Tail{0, 1, 1}, grid, st);
+  else launch2<false, false, float, 4>(ta, tb, to, to, out, Mo, No, rows_total, accumulate, 1, grp, g2::Tail{0, 1, 1}, grid, st);
 }
 
 

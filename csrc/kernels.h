@@ -53,8 +53,9 @@ void gemm_bf16(const void* a, const void* b, void* out, int M, int N, int K, boo
                bool accumulate, const GemmComm& comm, const void* a_local_shard, cudaStream_t st);
 bool gemm_self_check_supported();
 // CTA-pair (cta_group::2) variant, plain GEMM only
+size_t gemm_2cta_workspace(int M, int N, int K, int out_dt, bool accumulate);
 void gemm_bf16_2cta(const void* a, const void* b, void* out, int M, int N, int K, bool trans_a, bool trans_b, int out_dt,
-                    bool accumulate, cudaStream_t st);
+                    bool accumulate, float* workspace, cudaStream_t st);
 
 void gemm_bf16_2cta_tp(int mode, const void* a, const void* b, void* out_or_partial, void* rs_out, const void* a_local,
                        int M, int N, int K, bool trans_b, int rank, int world, const int64_t* peer_bufs,

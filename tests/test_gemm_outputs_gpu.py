@@ -37,3 +37,26 @@ def test_grouped_weight_gradients(M, N, counts, dtype, accumulate):
     ops._ext.ext().grouped_wgrad(x, dy, out, seg.cuda(), block, accumulate)
     # fp32 sums as above; one rounding to bfloat16 (2^-9) of the result
     assert (out.double() - want).abs().max() <= (2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -16) * max(1.0, want.abs().max())
+
+
+# a last round of few tiles is split along K and summed by a second kernel: ragged rows and columns, both output types
+@pytest.mark.parametrize("M,N,K", [(1000, 5120, 1032), (264, 2056, 4096), (300, 264, 640), (5000, 4104, 520)])
+@pytest.mark.parametrize("dtype,accumulate", [(torch.bfloat16, False), (torch.bfloat16, True), (torch.float32, False), (torch.float32, True)])
+@pytest.mark.parametrize("trans", [(False, True), (False, False), (True, False)])
+def test_split_tail(M, N, K, dtype, accumulate, trans):
+    from neuronx_distributed_b200 import ops
+
+    if trans[0] and M % 8:
+        M += 8 - M % 8
+    g = torch.Generator(device="cuda").manual_seed(K)
+    a = torch.randn(*((K, M) if trans[0] else (M, K)), generator=g, device="cuda").bfloat16()
+    b = torch.randn(*((N, K) if trans[1] else (K, N)), generator=g, device="cuda").bfloat16()
+    out = torch.randn(M + 1, N, generator=g, device="cuda").to(dtype)
+    guard = out[M].clone()
+    want = (a.double().t() if trans[0] else a.double()) @ (b.double().t() if trans[1] else b.double())
+    if accumulate:
+        want = want + out[:M].double()
+    ops._ext.ext().gemm_bf16_2cta(a, b, out[:M], trans[0], trans[1], accumulate)
+    # fp32 sums over K terms; one rounding to bfloat16
+    assert (out[:M].double() - want).abs().max() <= (2.0 ** -8 if dtype is torch.bfloat16 else 0) * want.abs().max() + 2.0 ** -20 * K
+    assert torch.equal(out[M], guard)
