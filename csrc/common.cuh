@@ -27,6 +27,22 @@ inline void nxd_throw(const std::string& msg, const char* file, int line) {
 
 namespace nxd {
 
+// Programmatic dependent launch: a kernel that was launched with launch_dependent starts while the one before it in the stream still
+// runs, and must pass pdl_wait before it touches anything that kernel wrote; pdl_trigger in the earlier one lets it start.
+NXD_DEVICE void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+NXD_DEVICE void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... KArgs, typename... Args>
+inline void launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  NXD_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...));
+}
+
 // ---------------------------------------------------------------- type helpers
 template <typename T> struct Vec8;  // 8 elements of a 16-bit type = 16 bytes
 template <> struct Vec8<__nv_bfloat16> { uint4 raw; };

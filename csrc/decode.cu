@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(kDecThreads, 2) decode_attn_kernel(
   extern __shared__ __align__(128) uint8_t dec_smem[];
   const int kvh = blockIdx.x, b = blockIdx.y, split = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_trigger();                                           // the merge's blocks may take their places; they wait for this grid
   const long pos = positions[b];
   const int n_valid = (int)(pos < 0 ? 0 : (pos >= L ? L : pos + 1));
   const int per = (n_valid + splits - 1) / splits;
@@ -207,6 +208,7 @@ __global__ void __launch_bounds__(HD) decode_combine_kernel(const float* __restr
                                                             __nv_bfloat16* __restrict__ out, int splits, long o_sb, long o_sh,
                                                             int H) {
   const int bh = blockIdx.x, d = threadIdx.x;
+  pdl_wait();
   float mn = -INFINITY;
   for (int s = 0; s < splits; ++s) mn = fmaxf(mn, part_ml[((long)bh * splits + s) * 2]);
   float acc = 0.f, ls = 0.f;
@@ -226,6 +228,7 @@ __global__ void __launch_bounds__(HD) decode_combine_kernel(const float* __restr
 __global__ void __launch_bounds__(HD) decode_combine_partial_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                                                     float* __restrict__ fin_o, float* __restrict__ fin_ml, int splits) {
   const int bh = blockIdx.x, d = threadIdx.x;
+  pdl_wait();
   float mn = -INFINITY;
   for (int s = 0; s < splits; ++s) mn = fmaxf(mn, part_ml[((long)bh * splits + s) * 2]);
   float acc = 0.f, ls = 0.f;
@@ -362,8 +365,8 @@ void decode_attention(const void* q, const void* k, const void* v, const long* p
     default: nxd_throw("decode_attention: unsupported GQA group size", __FILE__, __LINE__);
   }
 #undef NXD_DEC
-  if (fin_o != nullptr) decode_combine_partial_kernel<<<B * H, HD, 0, st>>>(part_o, part_ml, fin_o, fin_ml, splits);
-  else if (!whole) decode_combine_kernel<<<B * H, HD, 0, st>>>(part_o, part_ml, (__nv_bfloat16*)out, splits, o_sb, o_sh, H);
+  if (fin_o != nullptr) launch_dependent(decode_combine_partial_kernel, B * H, HD, 0, st, part_o, part_ml, fin_o, fin_ml, splits);
+  else if (!whole) launch_dependent(decode_combine_kernel, B * H, HD, 0, st, part_o, part_ml, (__nv_bfloat16*)out, splits, o_sb, o_sh, H);
   NXD_CUDA_CHECK(cudaGetLastError());
 }
 

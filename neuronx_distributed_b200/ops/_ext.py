@@ -61,14 +61,35 @@ def load_error() -> Optional[BaseException]:
     return _LOAD_ERROR
 
 
+_ENVIRON = getattr(os.environ, "_data", None)      # POSIX: the dict behind os.environ (bytes to bytes)
+
+
+def env(name: str, default: str = "") -> str:
+    """``os.environ.get`` for switches that are read on every call: a look into the dict behind it (a missing key costs
+    ``os.environ`` an encoded copy of the name and an exception, about 1 us, a hundred times in a training step)."""
+    if _ENVIRON is None:
+        return os.environ.get(name, default)
+    key = _ENV_KEYS.get(name)
+    if key is None:
+        key = _ENV_KEYS[name] = os.environ.encodekey(name)
+    v = _ENVIRON.get(key)
+    return default if v is None else os.environ.decodevalue(v)
+
+
+_ENV_KEYS: dict = {}
+
+
 def use_cuda(*tensors: torch.Tensor) -> bool:
     """True when the hand-written kernels must handle these tensors.
 
     CPU tensors → False (reference math).  CUDA tensors → True if the extension loaded; if
     it did not, raise loudly unless the eager fallback is explicitly allowed."""
-    if not tensors or not all(isinstance(t, torch.Tensor) and t.is_cuda for t in tensors):
+    if not tensors:
         return False
-    if os.environ.get("NXD_FORCE_EAGER", "0") == "1":
+    for t in tensors:
+        if not (isinstance(t, torch.Tensor) and t.is_cuda):
+            return False
+    if env("NXD_FORCE_EAGER") == "1":
         return False
     if _load() is not None:
         return True

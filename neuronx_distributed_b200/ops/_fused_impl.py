@@ -473,19 +473,19 @@ def _row_sp_forward_op(x: torch.Tensor, weight: torch.Tensor, group) -> torch.Te
 def select(x: torch.Tensor, weight: torch.Tensor, in_mode: str, out_mode: str, seq_dim: int, group):
     """Return a fused implementation for this call or ``None`` (the caller then runs NCCL collectives + the plain GEMM).
     Every reason for ``None`` on a CUDA tensor is logged once, so nobody sits on the unfused path without knowing."""
-    if os.environ.get("NXD_DISABLE_FUSED_TP", "0") == "1":
-        return None
-    if not x.is_cuda:
-        return None
-    world = dist.get_world_size(group)
-    if world == 1:
-        return None
     if in_mode == "gather" and out_mode == "none":
         kind = "Column+SP"
     elif in_mode == "none" and out_mode == "scatter":
         kind = "Row+SP"
     else:
         return None           # non-SP modes have their own path (all-reduce), not a fallback of this one
+    if _ext.env("NXD_DISABLE_FUSED_TP") == "1":
+        return None
+    if not x.is_cuda:
+        return None
+    world = dist.get_world_size(group)
+    if world == 1:
+        return None
 
     def no(reason: str):
         _log_once(f"{kind}:{reason}", f"fused {kind} TP linear not used ({reason}): falling back to NCCL collective + plain GEMM")

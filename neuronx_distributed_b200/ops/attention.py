@@ -28,7 +28,7 @@ def _sdpa(q, k, v, causal: bool, scale: Optional[float]):
 
 
 def _own_kernel_ok(q, k, v) -> bool:
-    if os.environ.get("NXD_DISABLE_OWN_ATTENTION", "0") == "1":
+    if _ext.env("NXD_DISABLE_OWN_ATTENTION") == "1":
         return False
     if not (q.is_cuda and q.dtype == torch.bfloat16 and k.dtype == torch.bfloat16 and v.dtype == torch.bfloat16
             and q.shape[-1] == 128 and q.dim() == 4):

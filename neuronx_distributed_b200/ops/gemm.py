@@ -21,11 +21,11 @@ _USE_2CTA = os.environ.get("NXD_GEMM_2CTA", "1") == "1"   # CTA-pair kernel (cta
 
 
 def fused_wgrad_enabled() -> bool:
-    return os.environ.get("NXD_DISABLE_FUSED_WGRAD", "0") != "1" and os.environ.get("NXD_DISABLE_TCGEN05_GEMM", "0") != "1"
+    return _ext.env("NXD_DISABLE_FUSED_WGRAD") != "1" and _ext.env("NXD_DISABLE_TCGEN05_GEMM") != "1"
 
 
 def _eligible(a: torch.Tensor, b: torch.Tensor, M: int, N: int, K: int) -> bool:
-    if os.environ.get("NXD_DISABLE_TCGEN05_GEMM", "0") == "1":
+    if _ext.env("NXD_DISABLE_TCGEN05_GEMM") == "1":
         return False
     if not (a.is_cuda and b.is_cuda and a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16):
         return False
@@ -53,7 +53,7 @@ def matmul(a: torch.Tensor, b: torch.Tensor, trans_a: bool = False, trans_b: boo
     out_dtype = out_dtype or (out.dtype if out is not None else a.dtype)
     if (M <= 8 and not trans_a and trans_b and out is None and out_dtype == torch.bfloat16 and a.is_cuda
             and a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and K % 8 == 0 and a.is_contiguous() and b.is_contiguous()
-            and _ext.ext() is not None and hasattr(_ext.ext(), "gemv") and os.environ.get("NXD_DISABLE_TCGEN05_GEMM", "0") != "1"):
+            and _ext.ext() is not None and hasattr(_ext.ext(), "gemv") and _ext.env("NXD_DISABLE_TCGEN05_GEMM") != "1"):
         # decode-time GEMV: a bandwidth problem (every weight byte read once), not a tensor-core one — csrc/decode.cu
         _ext.count_launch()
         return _ext.ext().gemv(a, b, None)
@@ -70,7 +70,7 @@ def matmul(a: torch.Tensor, b: torch.Tensor, trans_a: bool = False, trans_b: boo
         else:
             _ext.ext().gemm_bf16(a, b, out, bool(trans_a), bool(trans_b), bool(accumulate))
         return out
-    if a.is_cuda and a.dtype == torch.bfloat16 and not os.environ.get("NXD_DISABLE_TCGEN05_GEMM") \
+    if a.is_cuda and a.dtype == torch.bfloat16 and not _ext.env("NXD_DISABLE_TCGEN05_GEMM") \
             and (not a.is_contiguous() or not b.is_contiguous()):
         # make operands dense once and retry the tensor-core kernel
         return matmul(a.contiguous(), b.contiguous(), trans_a, trans_b, out, accumulate, out_dtype)
@@ -101,7 +101,7 @@ def _grouped_ok(x: torch.Tensor, w: torch.Tensor, block_size: int) -> bool:
     e = _ext.ext()
     return (x.is_cuda and e is not None and hasattr(e, "grouped_gemm") and x.dtype == torch.bfloat16
             and w.dtype == torch.bfloat16 and block_size % 128 == 0 and w.shape[1] % 64 == 0 and w.shape[2] % 64 == 0
-            and os.environ.get("NXD_DISABLE_GROUPED_GEMM", "0") != "1")
+            and _ext.env("NXD_DISABLE_GROUPED_GEMM") != "1")
 
 
 def _grouped_ref(x, w, b2e, block_size):
