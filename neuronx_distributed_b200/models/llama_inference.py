@@ -13,6 +13,7 @@ from torch import nn
 from .. import ops
 from ..inference.kv_cache import KVCacheManager
 from ..utils.sampling import Sampler
+from ..modules.rms_norm import RMSNorm
 from .llama import LlamaConfig, LlamaForCausalLM
 
 
@@ -59,16 +60,18 @@ class LlamaForInference(nn.Module):
 
     # ------------------------------------------------------------------ shared pieces
     def _attn_block(self, layer_idx: int, layer, x: torch.Tensor, positions: Optional[torch.Tensor], prefill: bool,
-                    kv_len: Optional[int], tree=None) -> torch.Tensor:
+                    kv_len: Optional[int], tree=None, normed: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """``x`` plus the attention block's output; with ``normed`` (the block's input norm of ``x``) the output alone."""
         att = layer.self_attn
-        h = layer.input_layernorm(x)
+        h = layer.input_layernorm(x) if normed is None else normed
         q, k, v = att.qkv_proj(h)                          # [S, B, h*D]
         S, B = q.shape[0], q.shape[1]
         D = att.head_dim
         q = q.reshape(S, B, att.num_heads_local, D).transpose(0, 1)
         k = k.reshape(S, B, att.num_kv_heads_local, D).transpose(0, 1)
-        v = v.reshape(S, B, att.num_kv_heads_local, D).transpose(0, 1).contiguous()
+        v = v.reshape(S, B, att.num_kv_heads_local, D).transpose(0, 1)      # a view: caches and kernels take its strides
         if self.flash_decoding and not prefill:
+            v = v.contiguous()
             assert S == 1 and tree is None, "flash decoding serves plain token generation (no speculation window)"
             from ..modules.attention.flash_decode import flash_decode_attention, write_decode_sharded
 
@@ -114,7 +117,7 @@ class LlamaForInference(nn.Module):
             kc, vc = self.kv.get(layer_idx, kv_len)
             o = _decode_attention(q, kc, vc, positions)
         o = o.transpose(0, 1).reshape(S, B, att.num_heads_local * D)
-        return _row_linear_plus_residual(att.o_proj, o, x)
+        return _row_linear_plus_residual(att.o_proj, o, x) if normed is None else att.o_proj(o)
 
     def _tkg_block(self, layer_idx: int, layer):
         """Decode-time fused view of a MoE layer (shares its router / experts / norm; owns no parameters).  Kept outside the
@@ -132,6 +135,20 @@ class LlamaForInference(nn.Module):
     def _body(self, input_ids: torch.Tensor, positions: Optional[torch.Tensor], prefill: bool, kv_len: Optional[int], tree=None):
         core = self._core
         x = core.embed_tokens(input_ids).transpose(0, 1).contiguous()               # [S, B, H]
+        if prefill and _plain_norms(core):
+            # residual sums inside the norms that follow them: one pass over the rows instead of two
+            d = None
+            for i, layer in enumerate(core.layers):
+                n1, n2 = layer.input_layernorm, layer.post_attention_layernorm
+                if d is None:
+                    h = n1(x)
+                else:
+                    h, x = ops.norm.add_rms_norm(d, x, n1.weight, n1.variance_epsilon)
+                a = self._attn_block(i, layer, x, positions, prefill, kv_len, tree, normed=h)
+                h, x = ops.norm.add_rms_norm(a, x, n2.weight, n2.variance_epsilon)
+                y = layer.mlp(h)
+                d = y[0] if isinstance(y, tuple) else y                             # MoE blocks also return router logits
+            return ops.norm.add_rms_norm(d, x, core.norm.weight, core.norm.variance_epsilon)[0]
         for i, layer in enumerate(core.layers):
             x = self._attn_block(i, layer, x, positions, prefill, kv_len, tree)
             mlp = layer.mlp
@@ -198,6 +215,12 @@ class LlamaForInference(nn.Module):
             out.append(tok)
             pos = pos + 1
         return torch.stack(out, dim=1)
+
+
+def _plain_norms(core) -> bool:
+    """Every norm of the decoder is an RMSNorm without hooks (hooks see the module's own call), and there is a layer."""
+    norms = [n for layer in core.layers for n in (layer.input_layernorm, layer.post_attention_layernorm)] + [core.norm]
+    return len(norms) > 1 and all(type(n) is RMSNorm and not n._forward_hooks and not n._forward_pre_hooks for n in norms)
 
 
 def _row_linear_plus_residual(lin, inp: torch.Tensor, residual: torch.Tensor) -> torch.Tensor:

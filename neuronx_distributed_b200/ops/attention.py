@@ -8,7 +8,6 @@ Layout: q ``[B, S, Hq, D]``, k/v ``[B, S, Hkv, D]`` → out ``[B, S, Hq, D]``.
 from __future__ import annotations
 
 import math
-import os
 from typing import Optional
 
 import torch
