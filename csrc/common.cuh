@@ -34,12 +34,15 @@ NXD_DEVICE void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"
 
 template <typename... KArgs, typename... Args>
 inline void launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+  // a captured launch is an ordinary one: gaps inside a graph are short, and its instantiation took 30 ms longer with such edges
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  NXD_CUDA_CHECK(cudaStreamIsCapturing(st, &capture));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr; cfg.numAttrs = 1;
+  cfg.attrs = &attr; cfg.numAttrs = capture == cudaStreamCaptureStatusNone ? 1 : 0;
   NXD_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...));
 }
 
