@@ -106,6 +106,42 @@ static Tensor rope_apply(const Tensor& x, const Tensor& cos_t, const Tensor& sin
   return out;
 }
 
+// fused [S, B, (H + 2 K) D] → rotated q [B, S, H, D], k [B, S, K, D]
+static std::vector<Tensor> rope_qkv_fwd(const Tensor& x, const Tensor& cos_t, const Tensor& sin_t, int64_t H, int64_t K) {
+  CHECK_IN(x); CHECK_IN(cos_t); CHECK_IN(sin_t);
+  TORCH_CHECK(x.dim() == 3 && x.size(2) % (H + 2 * K) == 0 && (uintptr_t)x.data_ptr() % 16 == 0);
+  const int64_t D = x.size(2) / (H + 2 * K);
+  TORCH_CHECK((D / 2 * x.element_size()) % 16 == 0 && cos_t.scalar_type() == at::kFloat && sin_t.scalar_type() == at::kFloat &&
+              cos_t.size(0) >= x.size(0) && cos_t.size(1) == D / 2 && sin_t.sizes() == cos_t.sizes());
+  c10::cuda::CUDAGuard g(x.device());
+  auto q = at::empty({x.size(1), x.size(0), H, D}, x.options()), k = at::empty({x.size(1), x.size(0), K, D}, x.options());
+  nxd::rope_qkv_fwd(x.data_ptr(), q.data_ptr(), k.data_ptr(), cos_t.data_ptr<float>(), sin_t.data_ptr<float>(), (int)x.size(0),
+                    (int)x.size(1), (int)H, (int)K, (int)D, dt_code(x), stream());
+  return {q, k};
+}
+// gradients [B, S, h, D] (any batch / position / head strides that keep 16-byte packets) → fused [S, B, (H + 2 K) D]
+static Tensor rope_qkv_bwd(const Tensor& gq, const Tensor& gk, const Tensor& gv, const Tensor& cos_t, const Tensor& sin_t) {
+  CHECK_IN(cos_t); CHECK_IN(sin_t);
+  const int64_t B = gq.size(0), S = gq.size(1), H = gq.size(2), D = gq.size(3), K = gk.size(2);
+  long strides[3][3];
+  const Tensor* ts[3] = {&gq, &gk, &gv};
+  for (int i = 0; i < 3; ++i) {
+    const Tensor& t = *ts[i];
+    TORCH_CHECK(t.is_cuda() && t.dim() == 4 && t.stride(3) == 1 && t.size(0) == B && t.size(1) == S && t.size(3) == D &&
+                t.size(2) == (i ? K : H) && t.scalar_type() == gq.scalar_type() && (uintptr_t)t.data_ptr() % 16 == 0);
+    for (int d = 0; d < 3; ++d) {
+      strides[i][d] = t.stride(d);
+      TORCH_CHECK(t.size(d) == 1 || (t.stride(d) * t.element_size()) % 16 == 0);
+    }
+  }
+  TORCH_CHECK((D / 2 * gq.element_size()) % 16 == 0 && cos_t.size(0) >= S && cos_t.size(1) == D / 2 && sin_t.sizes() == cos_t.sizes());
+  c10::cuda::CUDAGuard g(gq.device());
+  auto out = at::empty({S, B, (H + 2 * K) * D}, gq.options());
+  nxd::rope_qkv_bwd(gq.data_ptr(), gk.data_ptr(), gv.data_ptr(), strides, out.data_ptr(), cos_t.data_ptr<float>(), sin_t.data_ptr<float>(),
+                    (int)S, (int)B, (int)H, (int)K, (int)D, dt_code(gq), stream());
+  return out;
+}
+
 static Tensor ce_stats(const Tensor& logits, const Tensor& target, int64_t vocab_start) {
   CHECK_IN(logits); CHECK_IN(target);
   TORCH_CHECK(target.scalar_type() == at::kLong && logits.dim() == 2 && target.numel() == logits.size(0));
@@ -848,6 +884,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("swiglu_fwd", &swiglu_fwd);
   m.def("swiglu_bwd", &swiglu_bwd);
   m.def("rope_apply", &rope_apply);
+  m.def("rope_qkv_fwd", &rope_qkv_fwd);
+  m.def("rope_qkv_bwd", &rope_qkv_bwd);
   m.def("ce_stats", &ce_stats);
   m.def("ce_backward", &ce_backward);
   m.def("multi_tensor_sq_norm", &multi_tensor_sq_norm);

@@ -22,6 +22,10 @@ void swiglu_fwd(const void* gu, void* out, long rows, int I, int dt, cudaStream_
 void swiglu_bwd(const void* go, const void* gu, void* dgu, long rows, int I, int dt, cudaStream_t st);
 void rope_apply(const void* x, void* out, const float* cos_t, const float* sin_t, int B, int S, int Hh, int D, long sb,
                 long ss, long sh, float sign, int dt, cudaStream_t st);
+void rope_qkv_fwd(const void* x, void* q, void* k, const float* cos_t, const float* sin_t, int S, int B, int H, int K, int D, int dt,
+                  cudaStream_t st);
+void rope_qkv_bwd(const void* gq, const void* gk, const void* gv, const long (*strides)[3], void* out, const float* cos_t, const float* sin_t,
+                  int S, int B, int H, int K, int D, int dt, cudaStream_t st);
 void ce_stats(const void* logits, const int64_t* target, float* stats, int rows, int V, int vocab_start, int dt,
               cudaStream_t st);
 void ce_backward(const void* logits, const int64_t* target, const float* lse, const float* gout, void* grad, int rows,

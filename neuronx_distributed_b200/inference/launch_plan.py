@@ -50,6 +50,7 @@ _EXT_RESOURCE_PREFIXES = ("vmm_", "symm_", "tp_gemm", "nvls_", "gemv_allreduce",
 # ``grouped_gemm`` with an ``out`` argument, ``decode_rope_kv`` appending to the cache, optimizer kernels …) is treated as
 # writing to EVERY tensor argument: conservative — such tensors count as state, are never hoisted or dropped — but safe.
 _EXT_PURE = frozenset({"rmsnorm_fwd", "rmsnorm_bwd", "add_rmsnorm_fwd", "add_rmsnorm_bwd", "swiglu_fwd", "swiglu_bwd", "rope_apply",
+                       "rope_qkv_fwd", "rope_qkv_bwd",
                        "ce_stats", "ce_backward", "decode_attention", "decode_attention_partial", "gemv", "gemm_few_rows", "gemv_mx",
                        "gemm_mxfp8", "moe_block_tkg", "moe_block_metadata", "moe_slots", "moe_gather", "moe_combine",
                        "moe_combine_grad", "row_argmax", "row_topk", "flash_attn_fwd",

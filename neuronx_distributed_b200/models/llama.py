@@ -136,12 +136,16 @@ class LlamaAttention(nn.Module):
         if clip is not None:                      # DBRX: clamp the projections (HF DbrxAttention clip_qkv)
             q, k, v = q.clamp(-clip, clip), k.clamp(-clip, clip), v.clamp(-clip, clip)
         S, B = q.shape[0], q.shape[1]
-        # [S,B,h,D] → [B,S,h,D] views (free when B == 1)
-        q = q.reshape(S, B, self.num_heads_local, self.head_dim).transpose(0, 1)
-        k = k.reshape(S, B, self.num_kv_heads_local, self.head_dim).transpose(0, 1)
-        v = v.reshape(S, B, self.num_kv_heads_local, self.head_dim).transpose(0, 1)
-        q = ops.rope.apply_rotary(q, cos, sin)
-        k = ops.rope.apply_rotary(k, cos, sin)
+        fused = ops.rope.fused_qkv(q, k, v, cos, sin, self.num_heads_local, self.num_kv_heads_local, self.head_dim)
+        if fused is not None:
+            q, k, v = ops.rope.rotary_qkv(fused, cos, sin, self.num_heads_local, self.num_kv_heads_local)
+        else:
+            # [S,B,h,D] → [B,S,h,D] views (free when B == 1)
+            q = q.reshape(S, B, self.num_heads_local, self.head_dim).transpose(0, 1)
+            k = k.reshape(S, B, self.num_kv_heads_local, self.head_dim).transpose(0, 1)
+            v = v.reshape(S, B, self.num_kv_heads_local, self.head_dim).transpose(0, 1)
+            q = ops.rope.apply_rotary(q, cos, sin)
+            k = ops.rope.apply_rotary(k, cos, sin)
         if self.cfg.context_parallel and ps.get_context_model_parallel_size() > 1:
             from ..modules.attention.ring import pull_attention, ring_attention
 

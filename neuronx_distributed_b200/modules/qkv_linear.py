@@ -204,6 +204,8 @@ class GQAQKVColumnParallelLinear(BaseParallelLayer):
         if self.kv_size_multiplier > 1:
             k = _KVGradSum.apply(k, self.kv_group, self.reduce_dtype)
             v = _KVGradSum.apply(v, self.kv_group, self.reduce_dtype)
+        elif not self.gather_output and isinstance(out, torch.Tensor) and out.is_cuda:
+            q._qkv_sections = (out, k, v)     # a rotation may read the three sections where they lie
         if self.gather_output:
             q = mappings.gather_from_tensor_model_parallel_region(q, self.tensor_parallel_group)
             k = mappings.gather_from_tensor_model_parallel_region(k, self.tensor_parallel_group)

@@ -47,6 +47,56 @@ def apply_rotary(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch
     return _Rope.apply(x, cos, sin)
 
 
+class _RopeQKV(torch.autograd.Function):
+    """Rotated q and k and the view v of a fused projection output; backward fills ONE fused gradient (no concatenation)."""
+
+    @staticmethod
+    def forward(ctx, qkv, cos, sin, heads, kv_heads):
+        cos, sin = cos.contiguous().float(), sin.contiguous().float()
+        ctx.save_for_backward(cos, sin)
+        _ext.count_launch()
+        q, k = _ext.ext().rope_qkv_fwd(qkv, cos, sin, int(heads), int(kv_heads))
+        D = q.shape[-1]
+        v = qkv[..., (heads + kv_heads) * D:].unflatten(-1, (kv_heads, D))
+        return q, k, v.transpose(0, 1)
+
+    @staticmethod
+    def backward(ctx, gq, gk, gv):
+        cos, sin = ctx.saved_tensors
+        _ext.count_launch()
+        return _ext.ext().rope_qkv_bwd(_packets(gq), _packets(gk), _packets(gv), cos, sin), None, None, None, None
+
+
+def _packets(t: torch.Tensor) -> torch.Tensor:
+    per = 16 // t.element_size()
+    ok = t.stride(3) == 1 and t.data_ptr() % 16 == 0 and all(t.shape[d] == 1 or t.stride(d) % per == 0 for d in range(3))
+    return t if ok else t.contiguous()
+
+
+def fused_qkv(q, k, v, cos, sin, heads: int, kv_heads: int, head_dim: int):
+    """The projection output ``[S, B, (heads + 2 kv_heads) head_dim]`` whose sections ``q``, ``k`` and ``v`` still are, when
+    :func:`rotary_qkv` takes it (whole 16-byte packets in each half of a head); None when one of the three was replaced or
+    watched on the way (an adapter, a hook of the projection), or the sizes are for the separate rotations."""
+    sections = getattr(q, "_qkv_sections", None)
+    if not isinstance(sections, tuple) or sections[1] is not k or sections[2] is not v:
+        return None
+    qkv = sections[0]
+    if any(t._backward_hooks or t.retains_grad for t in (q, k, v)):
+        return None
+    if (qkv.dim() != 3 or qkv.dtype not in (torch.bfloat16, torch.float16, torch.float32) or head_dim % 2
+            or qkv.shape[-1] != (heads + 2 * kv_heads) * head_dim or (head_dim // 2 * qkv.element_size()) % 16
+            or not qkv.is_contiguous() or qkv.data_ptr() % 16 or cos.dim() != 2 or cos.shape != sin.shape
+            or cos.shape[0] < qkv.shape[0] or cos.shape[1] != head_dim // 2 or not _ext.use_cuda(qkv, cos, sin)):
+        return None
+    return qkv
+
+
+def rotary_qkv(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, heads: int, kv_heads: int):
+    """``qkv [S, B, (heads + 2 kv_heads) D]`` → rotated ``q [B, S, heads, D]``, ``k`` and the view ``v [B, S, kv_heads, D]``:
+    :func:`apply_rotary` of the first two sections, each direction one launch (``csrc/elementwise.cu`` rope_qkv)."""
+    return _RopeQKV.apply(qkv, cos, sin, heads, kv_heads)
+
+
 def rope_tables(seq_len: int, dim: int, base: float = 10000.0, device=None, offset: int = 0,
                 scaling: float = 1.0):
     inv = 1.0 / (base ** (torch.arange(0, dim, 2, dtype=torch.float32, device=device) / dim))
