@@ -16,6 +16,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <string>
 
@@ -478,8 +479,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
 }
 
 // ====================================================================================================================
-// Backward.  One CTA per (128-row KV tile, kv head, batch); it keeps K/V resident in smem and dK/dV resident in TMEM and
-// walks the 64-row query tiles (× the GQA group) that can see this KV tile.  Everything is computed transposed so that the
+// Backward.  One CTA per (128-row KV tile, kv head or a part of its query heads, batch); it keeps K/V resident in smem and dK/dV
+// resident in TMEM and walks the 64-row query tiles (× the query heads of its part) that can see this KV tile.  Everything is computed transposed so that the
 // softmax threads own a *kv* row and P/dS land directly in the operand layouts the next GEMMs need:
 //   Sᵀ  = K·Qᵀ        (A = K  K-major, B = Q  K-major)            → TMEM [128 kv × 64 q]
 //   dPᵀ = V·dOᵀ       (A = V  K-major, B = dO K-major)            → TMEM [128 kv × 64 q]
@@ -504,7 +505,9 @@ struct BwdParams {
   long dk_sb, dk_ss, dk_sh, dv_sb, dv_ss, dv_sh;
   float scale, scale_log2;
   int causal;
-  int group_bh;                // (batch, KV head) pairs whose Q / dO / dQ stay in L2 together
+  int group_bh;                // (batch, KV head, part) triples whose Q / dO / dQ stay in L2 together
+  int parts;                   // blocks that share the query heads of one KV head (divides the group)
+  float* kv_part;              // parts > 1: fp32 dK and dV of each part, [2][B, Hkv, parts][S_kv, 128]
   const float* stats;          // [2][B*H*S_pad (+pad)] : −lse·log2e , −δ·scale
   long stats_stride;
   float* dq_acc;               // [B, H, S_pad, 128] fp32
@@ -611,16 +614,18 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Blocks start heaviest first (causal: the first K/V tiles see the most query tiles) within groups of heads that share L2: head by
   // head, the last heads' heavy tiles started when most SMs had nothing left (1 x 2048 x 32 heads: 142 us, now 119).
-  int n, kvh, b;
+  int n, kvh, b, vh;                                       // vh: the part's index among all parts of all KV heads
+  const int heads_v = p.Hkv * p.parts;
   {
-    const int tiles = (p.S_kv + BN - 1) / BN, bhs = p.B * p.Hkv;
+    const int tiles = (p.S_kv + BN - 1) / BN, bhs = p.B * heads_v;
     const int grp = (int)blockIdx.x / (tiles * p.group_bh), rem = (int)blockIdx.x - grp * tiles * p.group_bh;
     const int gs = min(p.group_bh, bhs - grp * p.group_bh), bh = grp * p.group_bh + rem % gs;
     n = rem / gs;
-    kvh = bh % p.Hkv;
-    b = bh / p.Hkv;
+    vh = bh % heads_v;
+    kvh = vh / p.parts;
+    b = bh / heads_v;
   }
-  const int group = p.H / p.Hkv;
+  const int group = p.H / heads_v;                         // query heads of this block: vh * group ...
   const int nq = (p.S_q + BQ - 1) / BQ;
   const int t0 = p.causal ? (n * BN) / BQ : 0;
   const int per_head = nq - t0;
@@ -661,7 +666,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
       for (int it = 0; it < n_iter; ++it) {
         const int qs = it % kQStages;
         const uint32_t ph = (uint32_t)((it / kQStages) & 1);
-        const int head = kvh * group + it / per_head, t = t0 + it % per_head;
+        const int head = vh * group + it / per_head, t = t0 + it % per_head;
         mbar_wait(bar_qe + 8 * qs, ph ^ 1);
         const uint32_t full = bar_qf + 8 * qs;
         mbar_expect_tx(full, 2 * kQTile + 512);
@@ -818,7 +823,12 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
 #pragma unroll
           for (int i = 0; i < 32; ++i) r[i] = 0;
         }
-        if (row_ok) {
+        if (row_ok && p.parts > 1) {
+          float* part = p.kv_part + ((((long)which * p.B + b) * heads_v + vh) * p.S_kv + kv) * HD + c * 32;
+#pragma unroll
+          for (int v4 = 0; v4 < 8; ++v4)
+            *reinterpret_cast<uint4*>(part + v4 * 4) = make_uint4(r[v4 * 4], r[v4 * 4 + 1], r[v4 * 4 + 2], r[v4 * 4 + 3]);
+        } else if (row_ok) {
 #pragma unroll
           for (int v4 = 0; v4 < 4; ++v4) {
             uint4 o;
@@ -839,7 +849,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
     const int tid = threadIdx.x - 192;
     for (int it = 0; it < n_iter; ++it) {
       const int st = it & 1;
-      const int head = kvh * group + it / per_head, t = t0 + it % per_head;
+      const int head = vh * group + it / per_head, t = t0 + it % per_head;
       mbar_wait(bar_dq, (uint32_t)(it & 1));
       tcgen05_fence_after();
       float* gdst = p.dq_acc + (((long)b * p.H + head) * p.S_pad + (long)t * BQ) * HD;
@@ -959,6 +969,28 @@ __global__ void fa_bwd_dq_out_kernel(const float* __restrict__ acc, __nv_bfloat1
   *reinterpret_cast<uint4*>(dq + b * sb + s * ss + h * sh + c * 8) = o;
 }
 
+// dK and dV of a KV head out of the fp32 sums of its parts, added in their order; 8 elements per thread.
+__global__ void fa_bwd_kv_out_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, int B,
+                                     int S, int Hkv, int parts, long k_sb, long k_ss, long k_sh, long v_sb, long v_ss, long v_sh) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x, n = (long)B * Hkv * S * 16;        // over 2 * B*Hkv*S*16
+  if (i >= 2 * n) return;
+  const bool is_v = i >= n;
+  const int c = (int)(i & 15);
+  const long r = (is_v ? i - n : i) >> 4;
+  const int s = (int)(r % S), h = (int)((r / S) % Hkv), b = (int)(r / ((long)S * Hkv));
+  const float* src = part + (((((long)is_v * B + b) * Hkv + h) * parts) * S + s) * HD + c * 8;
+  float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+  for (int j = 0; j < parts; ++j) {
+    const float4 a = reinterpret_cast<const float4*>(src + (long)j * S * HD)[0], e = reinterpret_cast<const float4*>(src + (long)j * S * HD)[1];
+    x.x += a.x; x.y += a.y; x.z += a.z; x.w += a.w;
+    y.x += e.x; y.y += e.y; y.z += e.z; y.w += e.w;
+  }
+  uint4 o;
+  o.x = pack_bf16(x.x, x.y); o.y = pack_bf16(x.z, x.w); o.z = pack_bf16(y.x, y.y); o.w = pack_bf16(y.z, y.w);
+  __nv_bfloat16* dst = is_v ? dv + b * v_sb + s * v_ss + h * v_sh : dk + b * k_sb + s * k_ss + h * k_sh;
+  *reinterpret_cast<uint4*>(dst + c * 8) = o;
+}
+
 // ---- host side -----------------------------------------------------------------------------------------------------
 // A [B, S, H, 128] bf16 view with strides (sb, ss, sh, 1) becomes a 2-D TMA tensor whose rows are `ss` apart; batch and
 // head offsets fold into the row coordinate when they are multiples of ss, else into the column coordinate.
@@ -1012,11 +1044,39 @@ void flash_attn_fwd(const void* q, const void* k, const void* v, void* out, floa
   NXD_CUDA_CHECK(cudaGetLastError());
 }
 
+int device_sm_count();
+
+// Blocks per KV head.  Unit: one 64-row query tile, about 1.8 us.  A launch lasts as long as its heaviest block, or as the sum of all over
+// the SMs and, since causal blocks differ, a quarter of the heaviest at the end; equal blocks come in whole rounds.  Every part costs
+// three tiles of start and end, and 256 KB of fp32 sums written and read (0.03 over the chip).  Taken where the estimate falls by a
+// twentieth.  The sums are at most twice the fp32 dQ buffer.  Whole backward, caches flushed, one block per KV head and by this rule:
+//   1 x 2048 tokens, 32 heads on 8: 214 and 154 us;  64 on 8: 407 and 290;  1 x 4096, 32 on 2: 1402 and 439;  64 on 8: 1058 and 837;
+//   1 x 512, 32 on 8: 70 and 48;  16 on 1: 192 and 44.  Left whole: 1 x 4096, 32 on 8 (415; two parts 433), 2 x 2048 (255; 294).
+int flash_attn_bwd_parts(int B, int S_q, int S_kv, int H, int Hkv, bool causal) {
+  using namespace fa;
+  const int group = H / Hkv, sms = device_sm_count();
+  const long nq = (S_q + BQ - 1) / BQ, tiles = (S_kv + BN - 1) / BN;
+  if (S_q <= 0 || S_kv <= 0 || H % Hkv) return 1;
+  long steps = 0;                                                 // query tiles of one head, over its K/V tiles
+  for (long n = 0; n < tiles; ++n) steps += nq - (causal ? n * (BN / BQ) : 0);
+  int best = 1;
+  double best_t = 0;
+  for (int parts = 1; parts <= group; ++parts) {
+    if (group % parts) continue;
+    const double blocks = (double)tiles * Hkv * B * parts, heavy = (double)nq * (group / parts) + 3;
+    const double all = ((double)steps * H * B + 3 * blocks) / sms;
+    const double waves = causal ? 0 : heavy * std::ceil(blocks / sms);            // equal blocks: whole rounds
+    const double t = std::max({heavy, all + (causal ? heavy / 4 : 0), waves}) + (parts > 1 ? 2 + 0.03 * blocks : 0);
+    if (parts == 1 || t < best_t * (best == 1 ? 0.95 : 1.0)) { best = parts; best_t = t; }
+  }
+  return best;
+}
+
 void flash_attn_bwd(const void* go, const void* q, const void* k, const void* v, const void* o, const float* lse,
                     const float* dlse, void* dq,
-                    void* dk, void* dv, float* stats, float* dq_acc, int B, int S_q, int S_kv, int H, int Hkv, int S_pad,
-                    const long* gs, const long* qs, const long* ks, const long* vs, const long* os, const long* dqs,
-                    const long* dks, const long* dvs, float scale, bool causal, cudaStream_t st) {
+                    void* dk, void* dv, float* stats, float* dq_acc, float* kv_part, int parts, int B, int S_q, int S_kv, int H,
+                    int Hkv, int S_pad, const long* gs, const long* qs, const long* ks, const long* vs, const long* os,
+                    const long* dqs, const long* dks, const long* dvs, float scale, bool causal, cudaStream_t st) {
   using namespace fa;
   if (causal && S_q != S_kv) nxd_throw("attention: causal needs S_q == S_kv", __FILE__, __LINE__);
   BwdParams p;
@@ -1031,6 +1091,7 @@ void flash_attn_bwd(const void* go, const void* q, const void* k, const void* v,
   p.causal = causal ? 1 : 0;
   p.stats = stats; p.stats_stride = (long)B * H * S_pad + 64;
   p.dq_acc = dq_acc;
+  p.parts = parts; p.kv_part = kv_part;
   { const char* e = getenv("NXD_FA_DEBUG"); p.debug = e ? atoi(e) : 0; }
   // NXD_FA_DETERMINISTIC=1: ordered dQ accumulation (see fa_bwd_kernel<true>); the turnstile counters live in a per-device
   // buffer that only grows (debug mode: allocation is synchronous, not meant for graph capture)
@@ -1063,15 +1124,20 @@ void flash_attn_bwd(const void* go, const void* q, const void* k, const void* v,
     NXD_CUDA_CHECK(cudaFuncSetAttribute(fa_bwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBwd));
     configured = true;
   }
-  const long head_bytes = (long)S_q * HD * 8 * (H / Hkv);         // Q, dO and fp32 dQ of one KV head's group
-  p.group_bh = (int)std::min<long>((long)Hkv * B, std::max<long>(1, (64l << 20) / std::max<long>(1, head_bytes)));
-  const unsigned grid = (unsigned)((S_kv + BN - 1) / BN * (long)Hkv * B);
+  const long head_bytes = (long)S_q * HD * 8 * (H / Hkv / parts); // Q, dO and fp32 dQ of one block's query heads
+  p.group_bh = (int)std::min<long>((long)Hkv * parts * B, std::max<long>(1, (64l << 20) / std::max<long>(1, head_bytes)));
+  const unsigned grid = (unsigned)((S_kv + BN - 1) / BN * (long)Hkv * parts * B);
   if (det) fa_bwd_kernel<true><<<grid, kThreadsBwd, kSmemBwd, st>>>(tq, tk, tv, tg, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, p);
   else fa_bwd_kernel<false><<<grid, kThreadsBwd, kSmemBwd, st>>>(tq, tk, tv, tg, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, p);
   {
     const long n = (long)B * H * S_q * 16;
     fa_bwd_dq_out_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dq, B, S_q, H, S_pad, dqs[0],
                                                                      dqs[1], dqs[2]);
+  }
+  if (parts > 1) {
+    const long n = 2l * B * Hkv * S_kv * 16;
+    fa_bwd_kv_out_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(kv_part, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, B, S_kv, Hkv, parts,
+                                                                     dks[0], dks[1], dks[2], dvs[0], dvs[1], dvs[2]);
   }
   NXD_CUDA_CHECK(cudaGetLastError());
 }

@@ -175,10 +175,12 @@ void flash_attn_fwd(const void* q, const void* k, const void* v, void* out, floa
                     int Hkv, const long* qs, const long* ks, const long* vs, const long* os, float scale, bool causal,
                     cudaStream_t st);
 
+// parts (a divisor of H / Hkv; flash_attn_bwd_parts is the rule): blocks per KV head; kv_part: 2 * B * Hkv * parts * S_kv * 128 floats
+int flash_attn_bwd_parts(int B, int S_q, int S_kv, int H, int Hkv, bool causal);
 void flash_attn_bwd(const void* go, const void* q, const void* k, const void* v, const void* o, const float* lse,
                     const float* dlse, void* dq,
-                    void* dk, void* dv, float* stats, float* dq_acc, int B, int S_q, int S_kv, int H, int Hkv, int S_pad,
-                    const long* gs, const long* qs, const long* ks, const long* vs, const long* os, const long* dqs,
-                    const long* dks, const long* dvs, float scale, bool causal, cudaStream_t st);
+                    void* dk, void* dv, float* stats, float* dq_acc, float* kv_part, int parts, int B, int S_q, int S_kv, int H,
+                    int Hkv, int S_pad, const long* gs, const long* qs, const long* ks, const long* vs, const long* os,
+                    const long* dqs, const long* dks, const long* dvs, float scale, bool causal, cudaStream_t st);
 
 }  // namespace nxd
