@@ -1,6 +1,6 @@
 """RMSNorm with fp32 statistics and a sequence-parallel-tagged weight
 (reference ``modules/rms_norm.py:10-72``).  Forward/backward run the sm_100a kernels in
-``csrc/elementwise.cu`` via :func:`ops.norm.rms_norm`."""
+``csrc/elementwise.cu`` (forward) and ``csrc/fused_norm.cu`` (backward) via :func:`ops.norm.rms_norm`."""
 from __future__ import annotations
 
 import numbers

@@ -1,4 +1,4 @@
-"""RMSNorm forward/backward (kernels: ``csrc/elementwise.cu`` rmsnorm_fwd / rmsnorm_bwd).
+"""RMSNorm forward (``csrc/elementwise.cu`` rmsnorm_fwd) and backward (``csrc/fused_norm.cu`` norm_bwd).
 
 fp32 statistics regardless of I/O dtype (reference ``modules/rms_norm.py:10-33``).  The backward
 kernel emits dX and per-CTA partial dW rows that a tiny second kernel reduces.
