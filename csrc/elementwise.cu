@@ -230,18 +230,17 @@ __global__ void __launch_bounds__(256) ce_stats_kernel(const T* __restrict__ log
   const T* xr = logits + (size_t)row * V;
   float m = -INFINITY, s = 0.f, sx = 0.f;
   const int nvec = vec ? V / N : 0;                 // rows of another alignment: element by element
+  // fmaxf passes NaN by, so behind nothing but masked columns and NaN the maximum is still -inf: the terms are then taken against 0,
+  // where a masked column adds 0 and NaN adds NaN, and the sum is NaN in the end wherever one stood
   auto take = [&](const P& p) {
     float lm = m;
 #pragma unroll
     for (int j = 0; j < N; ++j) lm = fmaxf(lm, p.f(j));
+    const float ref = lm == -INFINITY ? 0.f : lm;
     float acc = 0.f;
-    if (lm != -INFINITY) {                          // else nothing but masked columns so far
 #pragma unroll
-      for (int j = 0; j < N; ++j) acc += __expf(p.f(j) - lm);
-      s = s * __expf(m - lm) + acc;
-    }
-#pragma unroll
-    for (int j = 0; j < N; ++j) sx += p.f(j);
+    for (int j = 0; j < N; ++j) { const float f = p.f(j); acc += __expf(f - ref); sx += f; }
+    s = s * __expf(m - ref) + acc;
     m = lm;
   };
   int v = threadIdx.x;
@@ -256,14 +255,12 @@ __global__ void __launch_bounds__(256) ce_stats_kernel(const T* __restrict__ log
   for (; v < nvec; v += blockDim.x) { P p; p.load(xr + (size_t)v * N); take(p); }
   for (int c = nvec * N + threadIdx.x; c < V; c += blockDim.x) {  // ragged tail
     const float f = to_f32<T>(xr[c]);
-    const float nm = fmaxf(m, f);
-    sx += f;
-    if (nm == -INFINITY && f == f) continue;
-    s = s * __expf(m - nm) + __expf(f - nm);
-    m = nm;
+    const float nm = fmaxf(m, f), ref = nm == -INFINITY ? 0.f : nm;
+    s = s * __expf(m - ref) + __expf(f - ref);
+    m = nm; sx += f;
   }
   const float gm = block_max(m, red);
-  const float contrib = (m == -INFINITY) ? 0.f : s * __expf(m - gm);
+  const float contrib = s * __expf(m - (gm == -INFINITY ? 0.f : gm));      // m = -inf: 0, or NaN
   const float gs = block_sum(contrib, red);
   const float gsx = block_sum(sx, red);
   if (threadIdx.x == 0) {

@@ -7,6 +7,17 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
+def _groups():
+    import torch.distributed as dist
+
+    from neuronx_distributed_b200.parallel_layers import parallel_state as ps
+
+    if not dist.is_initialized():
+        dist.init_process_group("gloo", store=dist.HashStore(), rank=0, world_size=1)
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_model_parallel(tensor_model_parallel_size=1)
+
+
 @pytest.mark.parametrize("sizes", [[1, 3, 0, 8191], [8192, 8193, 5], [7] * 60 + [40000], [3000000]])
 @pytest.mark.parametrize("gdtype", [torch.float32, torch.bfloat16])
 def test_optimizer_tables(sizes, gdtype):
@@ -70,3 +81,31 @@ def test_vocabulary_loss(V, dtype):
     got = ops.cross_entropy.ce_backward(x, tgt, lse, gout, 0, 0.0, V)
     ref = (torch.softmax(x.double(), -1) - torch.nn.functional.one_hot(tgt, V)) * gout[:, None].double()
     assert (got.double() - ref).abs().max() <= (2.0 ** -8 if dtype == torch.bfloat16 else 2e-5)
+
+
+# NaN ends in the loss wherever it stands: alone in a packet, beside masked columns, behind them, in rows of one packet
+@pytest.mark.parametrize("V", [8, 40, 2048, 4096, 5003])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_vocabulary_loss_of_nan(V, dtype):
+    from neuronx_distributed_b200 import ops
+    from neuronx_distributed_b200.parallel_layers.loss_functions import parallel_cross_entropy
+
+    _groups()
+    g = torch.Generator(device="cuda").manual_seed(V)
+    x = torch.randn(7, V, generator=g, device="cuda").to(dtype)
+    x[0, :8] = math.nan
+    x[1, :8] = -math.inf
+    x[1, 5] = math.nan
+    x[2, :V // 2] = -math.inf
+    x[2, V // 2] = math.nan
+    x[3, V - 1] = math.nan
+    x[4] = math.nan
+    x[5, :V // 2] = -math.inf                               # masked, no NaN
+    tgt = torch.full((7,), V - 2, device="cuda")
+    stats = ops.cross_entropy.ce_stats(x, tgt, 0)
+    want = [True] * 5 + [False] * 2
+    assert stats[:, 1].isnan().tolist() == want
+    loss = parallel_cross_entropy(x.unsqueeze(1), tgt.unsqueeze(1)).flatten()
+    assert loss.isnan().tolist() == want
+    ref = torch.nn.functional.cross_entropy(x[5:].double(), tgt[5:], reduction="none")
+    assert (loss[5:].double() - ref).abs().max() < 2e-5
