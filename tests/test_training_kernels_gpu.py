@@ -109,3 +109,16 @@ def test_vocabulary_loss_of_nan(V, dtype):
     assert loss.isnan().tolist() == want
     ref = torch.nn.functional.cross_entropy(x[5:].double(), tgt[5:], reduction="none")
     assert (loss[5:].double() - ref).abs().max() < 2e-5
+
+
+def test_vocabulary_loss_of_foreign_targets():
+    """Targets that are no column of this shard, however far away, subtract nothing."""
+    from neuronx_distributed_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(6, 4096, generator=g, device="cuda")
+    tgt = torch.tensor([-1, -100, 4096, 2 ** 32 + 3, -2 ** 63, 2 ** 63 - 1], device="cuda")
+    stats = ops.cross_entropy.ce_stats(x, tgt, 0)
+    assert not stats[:, 2].any()
+    got = ops.cross_entropy.ce_backward(x, tgt, torch.logsumexp(x, -1), torch.ones(6, device="cuda"), 0, 0.0, 4096)
+    assert (got.double() - torch.softmax(x.double(), -1)).abs().max() <= 2e-5
