@@ -896,6 +896,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("multi_tensor_scale", &multi_tensor_scale);
   m.def("fused_adamw", &fused_adamw);
   m.def("gemm_bf16", &gemm_bf16);
+  m.def("gemm_2cta_workspace", [](int64_t M, int64_t N, int64_t K, bool f32_out, bool accumulate) {      // bytes; 0: no split tail
+    return (int64_t)nxd::gemm_2cta_workspace((int)M, (int)N, (int)K, f32_out ? nxd::kF32 : nxd::kBF16, accumulate);
+  });
   m.def("gemm_bf16_2cta", &gemm_bf16_2cta);
   m.def("oneshot_allreduce", &oneshot_allreduce);
   m.def("decode_attention", &decode_attention);

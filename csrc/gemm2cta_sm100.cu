@@ -796,7 +796,8 @@ static GemmPlan gemm_plan(int M, int N, int K, int out_dt, bool accumulate) {
   // The tail: s pairs per tile, at least 4 k-blocks each; worth it where it saves more than the launch that sums (3 us) and its traffic.
   // 1000 x 5120 x 13824 (80 tiles): 104 us, 143 with a second round of six tiles; cut into narrower columns instead, its pieces waited
   // for their loads as long as a whole tile.  1000 x 27648 x 5120 from [K, N] weights: 203, 281 before.
-  const int last = p.tiles % pairs;
+  // Rows of other lengths have no tail: gemm_tail_kernel writes whole groups of 8 columns.
+  const int last = N % 8 == 0 ? p.tiles % pairs : 0;
   int s = last > 0 ? std::min(16, std::min(pairs / last, num_kb / 4)) : 1;
   if (s > 1) {
     const int per = (num_kb + s - 1) / s;

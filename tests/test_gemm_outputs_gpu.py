@@ -60,3 +60,20 @@ def test_split_tail(M, N, K, dtype, accumulate, trans):
     # fp32 sums over K terms; one rounding to bfloat16
     assert (out[:M].double() - want).abs().max() <= (2.0 ** -8 if dtype is torch.bfloat16 else 0) * want.abs().max() + 2.0 ** -20 * K
     assert torch.equal(out[M], guard)
+
+
+# the kernel that sums a split tail writes whole groups of 8 columns: products of other widths are not split
+@pytest.mark.parametrize("N", [4, 5116])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_no_tail_for_other_widths(N, accumulate):
+    from neuronx_distributed_b200 import ops
+
+    e, M, K = ops._ext.ext(), 1000, 1992
+    assert e.gemm_2cta_workspace(M, 5112, K, True, accumulate) > 0 and e.gemm_2cta_workspace(M, N, K, True, accumulate) == 0
+    g = torch.Generator(device="cuda").manual_seed(N)
+    a, b = (torch.randn(n, K, generator=g, device="cuda").bfloat16() for n in (M, N))
+    out = torch.randn(M + 1, N, generator=g, device="cuda")
+    guard, want = out[M].clone(), a.double() @ b.double().t() + (out[:M].double() if accumulate else 0)
+    e.gemm_bf16_2cta(a, b, out[:M], False, True, accumulate)
+    assert (out[:M].double() - want).abs().max() <= 2.0 ** -20 * K      # fp32 sums over K terms
+    assert torch.equal(out[M], guard)
