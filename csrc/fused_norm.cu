@@ -45,6 +45,19 @@ __global__ void __launch_bounds__(256) add_rmsnorm_fwd_kernel(const T* __restric
       cache[i].store(h + base + v * N);
     }
   }
+  // rows wider than the registers hold (1024 packets): the second pass reads the stored sum again
+  for (int v = threadIdx.x + MAXV * blockDim.x; v < nvec; v += blockDim.x) {
+    P px, pr;
+    px.load(x + base + v * N);
+    pr.load(r + base + v * N);
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      px.set(j, px.f(j) + pr.f(j));
+      const float f = px.f(j);
+      ss += f * f;
+    }
+    px.store(h + base + v * N);
+  }
   ss = block_sum(ss, red);
   const float rstd = rsqrtf(ss / (float)H + eps);
   if (threadIdx.x == 0) rstd_out[row] = rstd;
@@ -58,6 +71,14 @@ __global__ void __launch_bounds__(256) add_rmsnorm_fwd_kernel(const T* __restric
       for (int j = 0; j < N; ++j) po.set(j, cache[i].f(j) * rstd * pw.f(j));
       po.store(y + base + v * N);
     }
+  }
+  for (int v = threadIdx.x + MAXV * blockDim.x; v < nvec; v += blockDim.x) {
+    P p, pw, po;
+    p.load(h + base + v * N);
+    pw.load_nc(w + v * N);
+#pragma unroll
+    for (int j = 0; j < N; ++j) po.set(j, p.f(j) * rstd * pw.f(j));
+    po.store(y + base + v * N);
   }
 }
 
@@ -194,8 +215,7 @@ template <typename T> static int fn_pick_threads(int H) {
 void add_rmsnorm_fwd(const void* x, const void* r, const void* w, void* h, void* y, float* rstd, int rows, int H,
                      float eps, int dt, cudaStream_t st) {
   FN_DISPATCH_DTYPE(dt, {
-    const int nvec = H / Pack16<T>::N;
-    if (H % Pack16<T>::N || nvec > 256 * 4) nxd_throw("add_rmsnorm: unsupported H", __FILE__, __LINE__);
+    if (H % Pack16<T>::N) nxd_throw("add_rmsnorm: H must be a multiple of the 16-byte vector width", __FILE__, __LINE__);
     const int th = fn_pick_threads<T>(H);
     add_rmsnorm_fwd_kernel<T, 4><<<rows, th, 0, st>>>((const T*)x, (const T*)r, (const T*)w, (T*)h, (T*)y, rstd, H, eps);
   });

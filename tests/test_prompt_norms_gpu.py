@@ -1,0 +1,65 @@
+"""Prompts of served models: residual sums inside the norms against the separate sums."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _served(hidden, heads, dtype, layers=2, batch=1, seq=32):
+    import torch.distributed as dist
+
+    from neuronx_distributed_b200.models.llama import LlamaConfig
+    from neuronx_distributed_b200.models.llama_inference import LlamaForInference
+    from neuronx_distributed_b200.parallel_layers import parallel_state as ps
+
+    if not dist.is_initialized():
+        dist.init_process_group("gloo", store=dist.HashStore(), rank=0, world_size=1)
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_model_parallel(tensor_model_parallel_size=1)
+    torch.manual_seed(0)
+    cfg = LlamaConfig(vocab_size=64, hidden_size=hidden, intermediate_size=256, num_hidden_layers=layers, num_attention_heads=heads,
+                      num_key_value_heads=1, max_position_embeddings=seq, dtype=dtype, device=torch.device("cuda"))
+    m = LlamaForInference(cfg, batch_size=batch, max_seq_len=seq, on_device_sampling=False).eval()
+    with torch.no_grad():
+        for p in m.lm.parameters():
+            if p.dim() == 2:
+                p.copy_(torch.randn_like(p) * p.shape[1] ** -0.5)
+    return m
+
+
+def _prompt(model, ids):
+    logits = model.context_encoding(ids, torch.full((ids.shape[0],), ids.shape[1] - 1, device="cuda"))
+    n = ids.shape[1]
+    return [logits] + [c[:, :n].clone() for c in [*model.kv.k, *model.kv.v]]
+
+
+def _separate_sums(model, ids):
+    """The same prompt with a hook on a norm: hooks see the module's own call, so the sums are made outside the norms."""
+    handle = model._core.norm.register_forward_hook(lambda *a: None)
+    try:
+        return _prompt(model, ids)
+    finally:
+        handle.remove()
+
+
+@pytest.mark.parametrize("H", [8, 1024, 2056, 4100, 8192, 8200, 16384, 20488])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_sum_and_norm_of_any_width(H, dtype):
+    from neuronx_distributed_b200 import ops
+
+    if H % (16 // dtype.itemsize):
+        pytest.skip("the norm takes whole 16-byte packets")
+    g = torch.Generator(device="cuda").manual_seed(H)
+    x, r, w = (torch.randn(*s, generator=g, device="cuda").to(dtype) for s in ((5, H), (5, H), (H,)))
+    with torch.no_grad():
+        y, h = ops.norm.add_rms_norm(x, r, w, 1e-5)
+        assert torch.equal(h, x + r) and torch.equal(y, ops.norm.rms_norm(x + r, w, 1e-5))
+
+
+# widths whose norms do not fit the registers of a block: 1024 packets of 16 bytes
+@pytest.mark.parametrize("hidden,heads,dtype", [(8320, 65, torch.bfloat16), (4224, 33, torch.float32)])
+def test_prompt_of_wide_model(hidden, heads, dtype):
+    m = _served(hidden, heads, dtype, layers=1)
+    ids = torch.randint(0, 64, (1, 20), device="cuda")
+    for a, b in zip(_prompt(m, ids), _separate_sums(m, ids)):
+        assert torch.equal(a, b)
