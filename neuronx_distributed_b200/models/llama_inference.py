@@ -135,8 +135,9 @@ class LlamaForInference(nn.Module):
     def _body(self, input_ids: torch.Tensor, positions: Optional[torch.Tensor], prefill: bool, kv_len: Optional[int], tree=None):
         core = self._core
         x = core.embed_tokens(input_ids).transpose(0, 1).contiguous()               # [S, B, H]
-        if prefill and _plain_norms(core):
-            # residual sums inside the norms that follow them: one pass over the rows instead of two
+        if prefill and x.shape[0] * x.shape[1] > 8 and _plain_norms(core):
+            # residual sums inside the norms that follow them: one pass over the rows instead of two.  Up to 8 rows the sum rides in
+            # the output projection's GEMV (+ all-reduce) instead, in fp32 and rounded once (_row_linear_plus_residual)
             d = None
             for i, layer in enumerate(core.layers):
                 n1, n2 = layer.input_layernorm, layer.post_attention_layernorm

@@ -63,3 +63,12 @@ def test_prompt_of_wide_model(hidden, heads, dtype):
     ids = torch.randint(0, 64, (1, 20), device="cuda")
     for a, b in zip(_prompt(m, ids), _separate_sums(m, ids)):
         assert torch.equal(a, b)
+
+
+# up to eight rows the output projection adds the residual to its fp32 sum and rounds once, as token generation does
+@pytest.mark.parametrize("batch,seq", [(1, 1), (2, 3), (1, 8), (4, 2), (1, 9), (2, 12)])
+def test_short_prompts_round_once(batch, seq):
+    m = _served(512, 4, torch.bfloat16, batch=batch)
+    ids = torch.randint(0, 64, (batch, seq), device="cuda")
+    for a, b in zip(_prompt(m, ids), _separate_sums(m, ids)):
+        assert torch.equal(a, b)
