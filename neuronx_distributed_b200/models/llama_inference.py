@@ -9,6 +9,7 @@ from typing import Optional
 
 import torch
 from torch import nn
+from torch.nn.modules.module import _global_forward_hooks, _global_forward_pre_hooks
 
 from .. import ops
 from ..inference.kv_cache import KVCacheManager
@@ -219,9 +220,13 @@ class LlamaForInference(nn.Module):
 
 
 def _plain_norms(core) -> bool:
-    """Every norm of the decoder is an RMSNorm without hooks (hooks see the module's own call), and there is a layer."""
+    """Every norm of the decoder is an RMSNorm whose own call nobody watches (no hook on it or on all modules, no forward of its own),
+    and there is a layer."""
+    if _global_forward_hooks or _global_forward_pre_hooks:
+        return False
     norms = [n for layer in core.layers for n in (layer.input_layernorm, layer.post_attention_layernorm)] + [core.norm]
-    return len(norms) > 1 and all(type(n) is RMSNorm and not n._forward_hooks and not n._forward_pre_hooks for n in norms)
+    return len(norms) > 1 and all(type(n) is RMSNorm and not n._forward_hooks and not n._forward_pre_hooks and "forward" not in n.__dict__
+                                  for n in norms)
 
 
 def _row_linear_plus_residual(lin, inp: torch.Tensor, residual: torch.Tensor) -> torch.Tensor:

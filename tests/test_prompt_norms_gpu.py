@@ -72,3 +72,25 @@ def test_short_prompts_round_once(batch, seq):
     ids = torch.randint(0, 64, (batch, seq), device="cuda")
     for a, b in zip(_prompt(m, ids), _separate_sums(m, ids)):
         assert torch.equal(a, b)
+
+
+def test_watched_norms_are_called():
+    """A hook on all modules and a forward of one module's own see every norm of a prompt."""
+    from neuronx_distributed_b200.modules.rms_norm import RMSNorm
+
+    m = _served(256, 2, torch.bfloat16)
+    ids = torch.randint(0, 64, (1, 16), device="cuda")
+    seen = []
+    for register in (torch.nn.modules.module.register_module_forward_hook, torch.nn.modules.module.register_module_forward_pre_hook):
+        seen.clear()
+        handle = register(lambda mod, *a: seen.append(mod) if isinstance(mod, RMSNorm) else None)
+        try:
+            _prompt(m, ids)
+        finally:
+            handle.remove()
+        assert len(seen) == 2 * 2 + 1
+    n = m._core.layers[1].input_layernorm
+    seen.clear()
+    n.forward = lambda x: (seen.append(n), type(n).forward(n, x))[1]
+    _prompt(m, ids)
+    assert len(seen) == 1
