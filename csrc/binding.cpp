@@ -253,16 +253,15 @@ static py::tuple moe_block_metadata(const Tensor& expert_index, int64_t num_expe
   return py::make_tuple(b2e, tp2id, counts);
 }
 
-// main_grad [V, H] fp32 += rows of gy [T, H] bf16 at ids [T] int64 (with zero_first: = )
-static void embedding_grad(const Tensor& ids, const Tensor& gy, Tensor main_grad, bool zero_first) {
-  CHECK_IN(ids); CHECK_IN(gy); CHECK_IN(main_grad);
-  TORCH_CHECK(ids.scalar_type() == at::kLong && gy.scalar_type() == at::kBFloat16 && main_grad.scalar_type() == at::kFloat &&
-              gy.dim() == 2 && main_grad.dim() == 2 && gy.size(0) == ids.numel() && gy.size(1) == main_grad.size(1) && gy.size(1) % 8 == 0);
-  TORCH_CHECK(((uintptr_t)gy.data_ptr() | (uintptr_t)main_grad.data_ptr()) % 16 == 0);
+// out [V, H] bf16 or fp32 += rows of gy [T, H] bf16 at ids [T] int64 (with zero_first: = )
+static void embedding_grad(const Tensor& ids, const Tensor& gy, Tensor out, bool zero_first) {
+  CHECK_IN(ids); CHECK_IN(gy); CHECK_IN(out);
+  TORCH_CHECK(ids.scalar_type() == at::kLong && gy.scalar_type() == at::kBFloat16 && (out.scalar_type() == at::kFloat || out.scalar_type() == at::kBFloat16) &&
+              gy.dim() == 2 && out.dim() == 2 && gy.size(0) == ids.numel() && gy.size(1) == out.size(1) && gy.size(1) % 8 == 0);
+  TORCH_CHECK(((uintptr_t)gy.data_ptr() | (uintptr_t)out.data_ptr()) % 16 == 0);
   c10::cuda::CUDAGuard g(gy.device());
-  if (zero_first) main_grad.zero_();
-  nxd::embedding_grad(ids.data_ptr<long>(), gy.data_ptr(), main_grad.data_ptr<float>(), (int)ids.numel(), (int)gy.size(1), main_grad.size(0),
-                      stream());
+  if (zero_first) out.zero_();
+  nxd::embedding_grad(ids.data_ptr<long>(), gy.data_ptr(), out.data_ptr(), dt_code(out), (int)ids.numel(), (int)gy.size(1), out.size(0), stream());
 }
 
 // expert_index [T, k] int64 → int32 (expert of each row block [nb], token of each slot [nb*B] (-1 = padding), block prefix sums [E+1],

@@ -1,7 +1,6 @@
-// Gradient of an embedding table, added into the fp32 gradient buffer that the optimizer gave the weight:
-//   main_grad[id] += sum of gy[t] over all t with ids[t] == id       (fp32, ascending t: the same sum on every run)
-// One block per token; the block of an id's first occurrence sums them all, the others leave.  It replaces a dense bf16 table (filled, scattered
-// into, converted and copied): 2048 tokens, 32000 x 4096: 0.56 ms before, 24 us and 79 to zero the buffer now.
+// Gradient of an embedding table:
+//   out[id] += sum of gy[t] over all t with ids[t] == id       (fp32, ascending t: the same sum on every run)
+// One block per token; the block of an id's first occurrence sums them all, the others leave.
 #include "common.cuh"
 #include "kernels.h"
 
@@ -11,8 +10,9 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kVec = 4;          // packets of 8 columns per thread and sweep: 8192 columns
 
+template <typename T_>
 __global__ void __launch_bounds__(kThreads) embedding_grad_kernel(const long* __restrict__ ids, const __nv_bfloat16* __restrict__ gy,
-                                                                  float* __restrict__ main_grad, int T, int H, long V) {
+                                                                  T_* __restrict__ out, int T, int H, long V) {
   __shared__ int list[kThreads];
   __shared__ int warp_count[kThreads / 32];
   const int t0 = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -58,11 +58,14 @@ __global__ void __launch_bounds__(kThreads) embedding_grad_kernel(const long* __
     for (int i = 0; i < kVec; ++i) {
       const int v = v0 + i * kThreads + tid;
       if (v < nvec) {
-        float4* o = reinterpret_cast<float4*>(main_grad + (size_t)id * H + v * 8);
-        float4 a = o[0], b = o[1];
-        a.x += acc[i][0]; a.y += acc[i][1]; a.z += acc[i][2]; a.w += acc[i][3];
-        b.x += acc[i][4]; b.y += acc[i][5]; b.z += acc[i][6]; b.w += acc[i][7];
-        o[0] = a; o[1] = b;
+#pragma unroll
+        for (int c = 0; c < 8; c += Pack16<T_>::N) {
+          Pack16<T_> o;
+          o.load(out + (size_t)id * H + v * 8 + c);
+#pragma unroll
+          for (int j = 0; j < Pack16<T_>::N; ++j) o.set(j, o.f(j) + acc[i][c + j]);
+          o.store(out + (size_t)id * H + v * 8 + c);
+        }
       }
     }
   }
@@ -70,9 +73,10 @@ __global__ void __launch_bounds__(kThreads) embedding_grad_kernel(const long* __
 
 }  // namespace
 
-void embedding_grad(const long* ids, const void* gy, float* main_grad, int T, int H, long V, cudaStream_t st) {
+void embedding_grad(const long* ids, const void* gy, void* out, int out_dt, int T, int H, long V, cudaStream_t st) {
   if (T == 0) return;
-  embedding_grad_kernel<<<T, kThreads, 0, st>>>(ids, (const __nv_bfloat16*)gy, main_grad, T, H, V);
+  if (out_dt == kBF16) embedding_grad_kernel<<<T, kThreads, 0, st>>>(ids, (const __nv_bfloat16*)gy, (__nv_bfloat16*)out, T, H, V);
+  else embedding_grad_kernel<<<T, kThreads, 0, st>>>(ids, (const __nv_bfloat16*)gy, (float*)out, T, H, V);
   NXD_CUDA_CHECK(cudaGetLastError());
 }
 

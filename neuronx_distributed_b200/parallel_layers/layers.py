@@ -240,44 +240,40 @@ class _EmbeddingRS(torch.autograd.Function):
         return None, gw.to(ctx.dtype), None, None
 
 
-class _EmbeddingIntoMainGrad(torch.autograd.Function):
-    """Lookup whose backward pass adds the rows' gradients straight into the weight's fp32 ``main_grad`` (the embedding's
-    counterpart of :func:`wgrad`): no dense gradient table in the weight's type, no conversion, and repeated tokens are summed
-    in fp32 in token order (``csrc/embedding_grad.cu``)."""
+class _TableLookup(torch.autograd.Function):
+    """``F.embedding`` whose gradient is summed by ``csrc/embedding_grad.cu``: repeated tokens in fp32 and in a fixed order.  The
+    gradient is handed to autograd as ``F.embedding`` hands its own, so hooks see it, several lookups add up before the weight's
+    gradient is final, and ``torch.autograd.grad`` returns it.  Like there, only the ids are kept."""
 
     @staticmethod
     def forward(ctx, ids, weight):
-        ctx.save_for_backward(ids, weight)
+        ctx.save_for_backward(ids)
+        ctx.rows = weight.shape[0]
         return F.embedding(ids, weight)
 
     @staticmethod
     def backward(ctx, gy):
         from .. import ops
 
-        ids, weight = ctx.saved_tensors
-        if not _embedding_main_grad_ok(ids, weight) or gy.dtype != torch.bfloat16:
-            return None, torch.ops.aten.embedding_dense_backward(gy, ids, weight.shape[0], -1, False)
+        ids, = ctx.saved_tensors
+        if torch.is_grad_enabled() or gy.dtype != torch.bfloat16:       # create_graph: the gradient is differentiated again
+            return None, torch.ops.aten.embedding_dense_backward(gy, ids, ctx.rows, -1, False)
         g2 = gy.reshape(-1, gy.shape[-1]).contiguous()
         if g2.data_ptr() % 16:
             g2 = g2.clone()
         ops._ext.count_launch()
-        ops._ext.ext().embedding_grad(ids.reshape(-1).contiguous(), g2, weight.main_grad, bool(getattr(weight, "main_grad_fresh", False)))
-        weight.main_grad_fresh = False
-        cb = getattr(weight, "_nxd_grad_ready", None)
-        if cb is not None:
-            cb(weight)
-        return None, None
+        out = torch.empty(ctx.rows, g2.shape[1], dtype=g2.dtype, device=g2.device)
+        ops._ext.ext().embedding_grad(ids.reshape(-1).contiguous(), g2, out, True)
+        return None, out
 
 
-def _embedding_main_grad_ok(ids, weight) -> bool:
+def _own_table_gradient_ok(ids, weight) -> bool:
     """Beyond 32768 tokens the search for equal ids (every token reads the ids before it) would outgrow the sums."""
     from .. import ops
 
-    mg = getattr(weight, "main_grad", None)
-    return (mg is not None and isinstance(ids, torch.Tensor) and ids.is_cuda and ids.dtype == torch.int64 and ids.numel() <= 32768
-            and weight.dtype == torch.bfloat16 and mg.dtype == torch.float32 and mg.is_contiguous() and mg.shape == weight.shape
-            and mg.data_ptr() % 16 == 0 and weight.shape[1] % 8 == 0 and ops.gemm.fused_wgrad_enabled()
-            and ops._ext.ext() is not None and hasattr(ops._ext.ext(), "embedding_grad"))
+    return (isinstance(ids, torch.Tensor) and ids.is_cuda and ids.dtype == torch.int64 and 0 < ids.numel() <= 32768
+            and weight.dtype == torch.bfloat16 and weight.shape[1] % 8 == 0 and ops._ext.use_cuda(weight)
+            and hasattr(ops._ext.ext(), "embedding_grad") and not torch._C._are_functorch_transforms_active())
 
 
 _EMBEDDING_RS = os.environ.get("NXD_EMBEDDING_RS", "0") == "1"     # opt-in until the kernels have run on hardware
@@ -365,8 +361,8 @@ class ParallelEmbedding(BaseParallelLayer):
         if (self.padding_idx is None and self.max_norm is None and not self.scale_grad_by_freq and not self.sparse
                 and self.weight.requires_grad and torch.is_grad_enabled() and getattr(self.weight, "main_grad", None) is not None):
             ids = ids.long()
-            if _embedding_main_grad_ok(ids, self.weight):
-                return _EmbeddingIntoMainGrad.apply(ids, self.weight)
+            if _own_table_gradient_ok(ids, self.weight):
+                return _TableLookup.apply(ids, self.weight)
         return F.embedding(
             ids.long(), self.weight, self.padding_idx, self.max_norm, self.norm_type, self.scale_grad_by_freq, self.sparse
         )
