@@ -261,7 +261,9 @@ static void embedding_grad(const Tensor& ids, const Tensor& gy, Tensor out, bool
   TORCH_CHECK(((uintptr_t)gy.data_ptr() | (uintptr_t)out.data_ptr()) % 16 == 0);
   c10::cuda::CUDAGuard g(gy.device());
   if (zero_first) out.zero_();
-  nxd::embedding_grad(ids.data_ptr<long>(), gy.data_ptr(), out.data_ptr(), dt_code(out), (int)ids.numel(), (int)gy.size(1), out.size(0), stream());
+  const int T = (int)ids.numel(), H = (int)gy.size(1);
+  auto ws = at::empty({(int64_t)nxd::embedding_grad_workspace(T, H)}, gy.options().dtype(at::kFloat));
+  nxd::embedding_grad(ids.data_ptr<long>(), gy.data_ptr(), out.data_ptr(), dt_code(out), ws.data_ptr<float>(), T, H, out.size(0), stream());
 }
 
 // expert_index [T, k] int64 → int32 (expert of each row block [nb], token of each slot [nb*B] (-1 = padding), block prefix sums [E+1],

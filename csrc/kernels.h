@@ -123,7 +123,8 @@ bool row_topk_supported(int V, int k);
 void row_topk(const void* x, float* vals, long* idxs, int rows, int V, int k, long row_stride, long index_offset, int dt,
               cudaStream_t st);
 
-void embedding_grad(const long* ids, const void* gy, void* out, int out_dt, int T, int H, long V, cudaStream_t st);
+size_t embedding_grad_workspace(int T, int H);      // floats, 16-byte aligned
+void embedding_grad(const long* ids, const void* gy, void* out, int out_dt, float* workspace, int T, int H, long V, cudaStream_t st);
 
 void moe_block_metadata(const void* expert_index, bool idx64, long n, int k, int E, int B, int nb, long* block_to_expert, long* tp2id,
                         long* counts, cudaStream_t st);

@@ -241,7 +241,7 @@ class _EmbeddingRS(torch.autograd.Function):
 
 
 class _TableLookup(torch.autograd.Function):
-    """``F.embedding`` whose gradient is summed by ``csrc/embedding_grad.cu``: repeated tokens in fp32 and in a fixed order.  The
+    """``F.embedding`` whose gradient is summed by ``csrc/embedding_grad.cu``: repeated tokens in fp32, in a fixed order.  The
     gradient is handed to autograd as ``F.embedding`` hands its own, so hooks see it, several lookups add up before the weight's
     gradient is final, and ``torch.autograd.grad`` returns it.  Like there, only the ids are kept."""
 
@@ -261,14 +261,14 @@ class _TableLookup(torch.autograd.Function):
         g2 = gy.reshape(-1, gy.shape[-1]).contiguous()
         if g2.data_ptr() % 16:
             g2 = g2.clone()
-        ops._ext.count_launch()
+        ops._ext.count_launch(3)
         out = torch.empty(ctx.rows, g2.shape[1], dtype=g2.dtype, device=g2.device)
         ops._ext.ext().embedding_grad(ids.reshape(-1).contiguous(), g2, out, True)
         return None, out
 
 
 def _own_table_gradient_ok(ids, weight) -> bool:
-    """Beyond 32768 tokens the search for equal ids (every token reads the ids before it) would outgrow the sums."""
+    """Beyond 32768 tokens putting them in order (every id is compared with every other) would outgrow the sums."""
     from .. import ops
 
     return (isinstance(ids, torch.Tensor) and ids.is_cuda and ids.dtype == torch.int64 and 0 < ids.numel() <= 32768

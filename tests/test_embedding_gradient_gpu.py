@@ -80,3 +80,31 @@ def test_hooks_and_direct_gradients():
     emb.collect_output = False                              # then a function transform goes through
     out = torch.vmap(lambda i: emb(i))(ids.view(3, 11))
     assert torch.equal(out, emb(ids).view(3, 11, 64))
+
+
+# ids of one stretch of 64 tokens, of several, and of one more or fewer; on a vocabulary shard the tokens of other ranks all look up row 0
+@pytest.mark.parametrize("T,V,H,repeat", [(64, 9, 8, 1.0), (65, 9, 2056, 1.0), (129, 2, 264, 0.5), (640, 3, 64, 0.0), (1025, 70, 128, 0.0),
+                                          (4096, 500, 1024, 7 / 8), (4099, 500, 1032, 1.0), (32768, 100, 256, 7 / 8)])
+def test_repeated_tokens(T, V, H, repeat):
+    emb, _ = _table(V, H)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    ids = torch.randint(0, V, (T,), generator=g, device="cuda")
+    ids[torch.rand(T, generator=g, device="cuda") < repeat] = 1
+    gy = torch.randn(T, H, generator=g, device="cuda").bfloat16()
+    got, = torch.autograd.grad(emb(ids), emb.weight, gy)
+    want = _sums(ids, gy, V)
+    # fp32 sums of at most T values of size 4 (in stretches: their error grows with the square root), one rounding to bfloat16
+    assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -23 * 8 * T).all()
+    again, = torch.autograd.grad(emb(ids), emb.weight, gy)
+    assert torch.equal(got, again)
+
+
+def test_tokens_outside_the_table_add_nothing():
+    from neuronx_distributed_b200 import ops
+
+    ids = torch.tensor([-1] * 70 + [3] * 3 + [5, 2 ** 40, 6] + [2] * 70, device="cuda")
+    gy = torch.randn(len(ids), 64, device="cuda").bfloat16()
+    out = torch.ones(6, 64, device="cuda")
+    ops._ext.ext().embedding_grad(ids, gy, out, False)
+    ok = (ids >= 0) & (ids < 6)
+    _close(out, 1 + _sums(ids[ok], gy[ok], 6), 70)
