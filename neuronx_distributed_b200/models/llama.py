@@ -17,6 +17,7 @@ from typing import Optional, Tuple
 import torch
 import torch.fx
 from torch import nn
+from torch.nn.modules.module import _global_forward_hooks
 from torch.utils.checkpoint import checkpoint
 
 from ..utils.profiling import nvtx_range
@@ -103,6 +104,13 @@ class LlamaMLP(nn.Module):
         return self.down_proj(ops.act.swiglu(self.gate_up_proj(x)))
 
 
+def _unwatched(proj: nn.Module) -> bool:
+    """Nobody but its caller sees what the projection returns (no hook on it or on all modules, no wrapper, no forward of its own), so
+    its three sections need not stay in the autograd graph one by one: whoever keeps one can ask for its gradient."""
+    return (type(proj) is GQAQKVColumnParallelLinear and not proj._forward_hooks and not _global_forward_hooks
+            and "forward" not in proj.__dict__)
+
+
 class LlamaAttention(nn.Module):
     def __init__(self, cfg: LlamaConfig):
         super().__init__()
@@ -136,7 +144,8 @@ class LlamaAttention(nn.Module):
         if clip is not None:                      # DBRX: clamp the projections (HF DbrxAttention clip_qkv)
             q, k, v = q.clamp(-clip, clip), k.clamp(-clip, clip), v.clamp(-clip, clip)
         S, B = q.shape[0], q.shape[1]
-        fused = ops.rope.fused_qkv(q, k, v, cos, sin, self.num_heads_local, self.num_kv_heads_local, self.head_dim)
+        fused = (ops.rope.fused_qkv(q, k, v, cos, sin, self.num_heads_local, self.num_kv_heads_local, self.head_dim)
+                 if _unwatched(self.qkv_proj) else None)
         if fused is not None:
             q, k, v = ops.rope.rotary_qkv(fused, cos, sin, self.num_heads_local, self.num_kv_heads_local)
         else:

@@ -75,8 +75,9 @@ def _packets(t: torch.Tensor) -> torch.Tensor:
 
 def fused_qkv(q, k, v, cos, sin, heads: int, kv_heads: int, head_dim: int):
     """The projection output ``[S, B, (heads + 2 kv_heads) head_dim]`` whose sections ``q``, ``k`` and ``v`` still are, when
-    :func:`rotary_qkv` takes it (whole 16-byte packets in each half of a head); None when one of the three was replaced or
-    watched on the way (an adapter, a hook of the projection), or the sizes are for the separate rotations."""
+    :func:`rotary_qkv` takes it (whole 16-byte packets in each half of a head); None when one of the three was replaced on the way
+    (an adapter) or carries a hook, or the sizes are for the separate rotations.  The sections leave the autograd graph: the caller
+    makes sure that nobody else holds one."""
     sections = getattr(q, "_qkv_sections", None)
     if not isinstance(sections, tuple) or sections[1] is not k or sections[2] is not v:
         return None
