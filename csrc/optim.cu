@@ -104,10 +104,67 @@ constexpr int kAdamStages = 3;
 constexpr int kAdamStage = 5 * (int)kChunk * 4 - (int)kChunk * 2;       // p, g, m, v and a 16-bit copy: 72 KB
 constexpr int kAdamSmem = kAdamStages * kAdamStage + 64;
 
-// Bound by HBM: 16 + 14 bytes per element with fp32 gradients and a bf16 copy, in nine streams.  Whole chunks travel as bulk copies
-// of 16 KB through a ring in shared memory, updated in place there: a stream's bytes reach a DRAM page together.  0.67 G elements:
-// 3.09 ms (6.5 TB/s); with 16-byte accesses per thread 3.70 (5.4), however the blocks were cut.  Chunks that are short or unaligned
-// are updated in global memory.
+// One chunk in global memory: four elements per access where fp32 arrays are 16-byte aligned and 16-bit ones 8-byte, else one.
+template <typename G, typename L, bool HAS_LOW>
+NXD_DEVICE void adam_in_place(float* p, const G* g, float* m, float* v, L* low, int n, const AdamRule& rule, float gs) {
+  int i0 = 0;
+  if ((((uintptr_t)p | (uintptr_t)m | (uintptr_t)v) % 16) == 0 && (uintptr_t)g % (4 * sizeof(G)) == 0 && (!HAS_LOW || (uintptr_t)low % (4 * sizeof(L)) == 0)) {
+    i0 = n / 4 * 4;
+#pragma unroll 2
+    for (int i = threadIdx.x * 4; i < i0; i += blockDim.x * 4) {
+      float4 pp = *reinterpret_cast<const float4*>(p + i), mm = *reinterpret_cast<const float4*>(m + i), vv = *reinterpret_cast<const float4*>(v + i);
+      float gg[4];
+      if constexpr (sizeof(G) == 4) {
+        const float4 t4 = *reinterpret_cast<const float4*>(g + i);
+        gg[0] = t4.x; gg[1] = t4.y; gg[2] = t4.z; gg[3] = t4.w;
+      } else {
+        const uint2 raw = *reinterpret_cast<const uint2*>(g + i);
+        const G* h = reinterpret_cast<const G*>(&raw);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) gg[j] = to_f32<G>(h[j]);
+      }
+      float* pa = &pp.x; float* ma = &mm.x; float* va = &vv.x;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) pa[j] = rule(gg[j] * gs, ma[j], va[j], pa[j]);
+      *reinterpret_cast<float4*>(p + i) = pp;
+      *reinterpret_cast<float4*>(m + i) = mm;
+      *reinterpret_cast<float4*>(v + i) = vv;
+      if constexpr (HAS_LOW) {
+        if constexpr (sizeof(L) == 4) {
+          *reinterpret_cast<float4*>(low + i) = pp;
+        } else {
+          uint2 raw; L* h = reinterpret_cast<L*>(&raw);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) h[j] = from_f32<L>(pa[j]);
+          *reinterpret_cast<uint2*>(low + i) = raw;
+        }
+      }
+    }
+  }
+  for (int i = i0 + threadIdx.x; i < n; i += blockDim.x) {
+    float mi = m[i], vi = v[i];
+    const float pi = rule(to_f32<G>(g[i]) * gs, mi, vi, p[i]);
+    m[i] = mi; v[i] = vi; p[i] = pi;
+    if constexpr (HAS_LOW) low[i] = from_f32<L>(pi);
+  }
+}
+
+// Tensors that the bulk copies of adamw_kernel cannot take (an array that is not 16-byte aligned: slices).  64 tensors of 1 M elements,
+// 16-bit arrays 8-byte aligned / all arrays off by one element: 337 us (5.6 TB/s) and 435; element by element on the bulk kernel 730 and 804.
+template <typename G, typename L, bool HAS_LOW>
+__global__ void __launch_bounds__(256) adamw_direct_kernel(const __grid_constant__ ChunkTable<5> tab, const AdamRule rule,
+                                                           const float* __restrict__ grad_scale) {
+  const float gs = grad_scale ? *grad_scale : 1.f;
+  each_chunk(tab, [&](int t, long base, long n) {
+    adam_in_place<G, L, HAS_LOW>((float*)tab.ptr[0][t] + base, (const G*)tab.ptr[1][t] + base, (float*)tab.ptr[2][t] + base,
+                                 (float*)tab.ptr[3][t] + base, HAS_LOW ? (L*)tab.ptr[4][t] + base : nullptr, (int)n, rule, gs);
+  });
+}
+
+// Bound by HBM: 16 + 14 bytes per element with fp32 gradients and a bf16 copy: four streams in, four out.  Whole chunks travel as bulk
+// copies of 16 KB through a ring in shared memory, updated in place there: a stream's bytes reach a DRAM page together.  0.67 G
+// elements: 3.09 ms (6.5 TB/s); with 16-byte accesses per thread 3.70 (5.4), however the blocks were cut.  Chunks that are shorter
+// (the ends of tensors) are updated in global memory.
 template <typename G, typename L, bool HAS_LOW>
 __global__ void __launch_bounds__(kAdamThreads, 1) adamw_kernel(const __grid_constant__ ChunkTable<5> tab, const AdamRule rule,
                                                                 const float* __restrict__ grad_scale) {
@@ -131,7 +188,7 @@ __global__ void __launch_bounds__(kAdamThreads, 1) adamw_kernel(const __grid_con
     k.m = (float*)tab.ptr[2][t] + off; k.v = (float*)tab.ptr[3][t] + off;
     k.low = HAS_LOW ? (L*)tab.ptr[4][t] + off : nullptr;
     k.n = (int)min(tab.numel[t] - off, kChunk);
-    k.bulk = k.n == kChunk && (((uintptr_t)k.p | (uintptr_t)k.g | (uintptr_t)k.m | (uintptr_t)k.v | (uintptr_t)k.low) % 16) == 0;
+    k.bulk = k.n == kChunk;                        // the arrays are 16-byte aligned
     return k;
   };
   constexpr uint32_t F = (uint32_t)kChunk * 4, GB = (uint32_t)kChunk * sizeof(G), LB = (uint32_t)kChunk * sizeof(L);
@@ -196,12 +253,7 @@ __global__ void __launch_bounds__(kAdamThreads, 1) adamw_kernel(const __grid_con
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     } else {
-      for (int i = tid; i < k.n; i += kAdamThreads) {
-        float mi = k.m[i], vi = k.v[i];
-        const float pi = rule(to_f32<G>(k.g[i]) * gs, mi, vi, k.p[i]);
-        k.m[i] = mi; k.v[i] = vi; k.p[i] = pi;
-        if constexpr (HAS_LOW) k.low[i] = from_f32<L>(pi);
-      }
+      adam_in_place<G, L, HAS_LOW>(k.p, k.g, k.m, k.v, k.low, k.n, rule, gs);
     }
     __syncthreads();
     if (tid == 0) {
@@ -274,13 +326,20 @@ void fused_adamw(const std::vector<TensorRef>& p, const std::vector<TensorRef>& 
                  const std::vector<TensorRef>& v, const std::vector<TensorRef>& lowp, int gdt, int ldt, float lr,
                  float beta1, float beta2, float eps, float wd, float bc1, float bc2, const float* grad_scale,
                  int hf_form, cudaStream_t st) {
-  const std::vector<TensorRef> lists[5] = {p, g, m, v, lowp};
+  const std::vector<TensorRef>* lists[5] = {&p, &g, &m, &v, &lowp};
   const bool has_low = !lowp.empty();
   AdamRule rule{hf_form ? lr * sqrtf(bc2) / bc1 : lr / bc1, beta1, beta2, eps, hf_form ? 1.f : 1.f - lr * wd, hf_form ? 1.f - lr * wd : 1.f,
                 hf_form ? 1.f : 1.f / bc2};
-  run_tables<5>(lists, 1, [&](const ChunkTable<5>& tab, int nb) {
+  std::vector<TensorRef> parts[2][5];              // 16-byte aligned throughout, others
+  for (size_t t = 0; t < p.size(); ++t) {
+    uintptr_t bits = 0;
+    for (const auto* l : lists) if (!l->empty()) bits |= (uintptr_t)(*l)[t].ptr;
+    for (int d = 0; d < 5; ++d) if (!lists[d]->empty()) parts[bits % 16 != 0][d].push_back((*lists[d])[t]);
+  }
+  for (int direct = 0; direct < 2; ++direct) run_tables<5>(parts[direct], direct ? kBlocksPerSm : 1, [&](const ChunkTable<5>& tab, int nb) {
 #define LAUNCH(G, L, HL)                                                                                                     \
   do {                                                                                                                       \
+    if (direct) { adamw_direct_kernel<G, L, HL><<<nb, 256, 0, st>>>(tab, rule, grad_scale); break; }                         \
     NXD_CUDA_CHECK(cudaFuncSetAttribute(adamw_kernel<G, L, HL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAdamSmem));    \
     adamw_kernel<G, L, HL><<<nb, kAdamThreads, kAdamSmem, st>>>(tab, rule, grad_scale);                                      \
   } while (0)

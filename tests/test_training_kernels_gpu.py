@@ -122,3 +122,38 @@ def test_vocabulary_loss_of_foreign_targets():
     assert not stats[:, 2].any()
     got = ops.cross_entropy.ce_backward(x, tgt, torch.logsumexp(x, -1), torch.ones(6, device="cuda"), 0, 0.0, 4096)
     assert (got.double() - torch.softmax(x.double(), -1)).abs().max() <= 2e-5
+
+
+# chunks are 4096 elements; slices: fp32 arrays at `offset` elements, 16-bit ones at 2 or 4 more or fewer
+@pytest.mark.parametrize("sizes", [[4095], [4096, 4097, 8192], [3] * 50 + [12289]])
+@pytest.mark.parametrize("offset", [(0, 0), (0, 4), (4, 4), (4, 2), (1, 1)])
+@pytest.mark.parametrize("gdtype,ldtype", [(torch.bfloat16, torch.bfloat16), (torch.float32, torch.bfloat16), (torch.float16, torch.float32),
+                                           (torch.float32, None)])
+def test_optimizer_slices(sizes, offset, gdtype, ldtype):
+    from neuronx_distributed_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(len(sizes))
+    whole = []
+
+    def arrays(dtype, at):
+        whole.append([torch.rand(n + 16, generator=g, device="cuda").to(dtype) for n in sizes])
+        return [t[at:at + n] for t, n in zip(whole[-1], sizes)]
+
+    p, m, v = (arrays(torch.float32, offset[0]) for _ in range(3))
+    gr = arrays(gdtype, offset[1])
+    low = arrays(ldtype, offset[1]) if ldtype is not None else None
+    outside = [[t.clone() for t in w] for w in whole]
+    want = []
+    scale, lr, b1, b2, eps, wd, step = 0.5, 1e-2, 0.9, 0.99, 1e-6, 0.1, 3
+    for a, gg, c, d in zip(p, gr, m, v):
+        a, c, d, gg = a.double(), c.double(), d.double(), gg.double() * scale
+        c, d = b1 * c + (1 - b1) * gg, b2 * d + (1 - b2) * gg * gg
+        want.append(((a - lr * math.sqrt(1 - b2 ** step) / (1 - b1 ** step) * c / (d.sqrt() + eps)) * (1 - lr * wd), c, d))
+    ops.optim.fused_adamw_(p, gr, m, v, lr, b1, b2, eps, wd, step, torch.tensor(scale, device="cuda"), low)
+    for i, w in enumerate(want):
+        for a, b in zip((p[i], m[i], v[i]), w):             # a few fp32 roundings
+            assert ((a.double() - b).abs() <= 2.0 ** -18 * (1 + b.abs())).all()
+        assert low is None or torch.equal(low[i], p[i].to(ldtype))
+    for w, o, at in zip(whole, outside, [offset[0]] * 3 + [offset[1]] * 2):
+        for a, b, n in zip(w, o, sizes):
+            assert torch.equal(a[:at], b[:at]) and torch.equal(a[at + n:], b[at + n:])
