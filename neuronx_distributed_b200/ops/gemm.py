@@ -58,6 +58,9 @@ def matmul(a: torch.Tensor, b: torch.Tensor, trans_a: bool = False, trans_b: boo
         _ext.count_launch()
         return _ext.ext().gemv(a, b, None)
     if _eligible(a, b, M, N, K) and out_dtype in (torch.bfloat16, torch.float32):
+        if out is not None and out.data_ptr() % 16:          # outputs leave through TMA or 16-byte stores: by way of a buffer
+            res = matmul(a, b, trans_a, trans_b, out_dtype=torch.float32)
+            return out.add_(res) if accumulate else out.copy_(res)
         if out is None and not trans_a and trans_b and out_dtype == torch.bfloat16 and _few_rows(M, N, K):
             _ext.count_launch()
             return _ext.ext().gemm_few_rows(a, b)

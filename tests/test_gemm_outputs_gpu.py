@@ -77,3 +77,21 @@ def test_no_tail_for_other_widths(N, accumulate):
     e.gemm_bf16_2cta(a, b, out[:M], False, True, accumulate)
     assert (out[:M].double() - want).abs().max() <= 2.0 ** -20 * K      # fp32 sums over K terms
     assert torch.equal(out[M], guard)
+
+
+def test_output_views_of_any_alignment():
+    """TMA wants 16-byte aligned outputs; views that are not get their result by way of a buffer, added to them in fp32."""
+    from neuronx_distributed_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(5)
+    for dtype in (torch.float32, torch.bfloat16):
+        for N in (16, 264):
+            a, b = (torch.randn(n, 72, generator=g, device="cuda").bfloat16() for n in (320, N))
+            flat = torch.zeros(320 * N + 2, device="cuda", dtype=dtype)
+            for accumulate in (False, True):
+                out = flat[1:-1].view(320, N)
+                assert ops.gemm.matmul(a, b, trans_b=True, out=out, accumulate=accumulate) is out
+            want = 2 * (a.double() @ b.double().t())
+            # fp32 sums over 72 terms; stored and added to, each with one rounding to bfloat16 (2^-9)
+            assert (out.double() - want).abs().max() <= (2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -18) * want.abs().max()
+            assert flat[0] == 0 and flat[-1] == 0
