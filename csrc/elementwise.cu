@@ -282,15 +282,15 @@ __global__ void __launch_bounds__(256) ce_bwd_kernel(const T* __restrict__ logit
   const T* xr = logits + (size_t)row * V;
   T* gr = grad + (size_t)row * V;
   const float l = lse[row], g = gout[row];
-  const long local = (long)target[row] - vocab_start;
-  const int mine = local >= 0 && local < V ? (int)local : -1;      // the target's column here, if any
+  long local = (long)target[row] - vocab_start;
+  if (local < 0 || local >= V) local = -1;          // no column of this shard
   const float sm_term = smoothing * inv_vocab;
   const int nvec = vec ? V / N : 0;
 #pragma unroll 4
   for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
     P p, o;
     *reinterpret_cast<uint4*>(p.v) = __ldcs(reinterpret_cast<const uint4*>(xr + v * N));
-    const int at = mine - v * N;                    // of the target within this packet, if in 0..N-1
+    const int at = (int)(local - (long)v * N);      // of the target within this packet, if in 0..N-1
 #pragma unroll
     for (int j = 0; j < N; ++j) {
       float d = __expf(p.f(j) - l) - sm_term;
@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(256) ce_bwd_kernel(const T* __restrict__ logit
   }
   for (int c = nvec * N + threadIdx.x; c < V; c += blockDim.x) {
     float d = __expf(to_f32<T>(xr[c]) - l) - sm_term;
-    if (c == mine) d -= (1.f - smoothing);
+    if ((long)c == local) d -= (1.f - smoothing);
     gr[c] = from_f32<T>(d * g);
   }
 }
