@@ -178,6 +178,14 @@ static void multi_tensor_sq_norm(const std::vector<Tensor>& ts, Tensor out) {
   c10::cuda::CUDAGuard g(ts[0].device());
   nxd::multi_tensor_sq_norm(refs(ts), dt_code(ts[0]), out.data_ptr<float>(), stream());
 }
+// buffer (fp32) = grad (bf16 / fp16), or += it
+static void grad_to_buffer(const Tensor& grad, Tensor buffer, bool add) {
+  CHECK_IN(grad); CHECK_IN(buffer);
+  TORCH_CHECK(buffer.scalar_type() == at::kFloat && (grad.scalar_type() == at::kBFloat16 || grad.scalar_type() == at::kHalf) &&
+              grad.numel() == buffer.numel() && ((uintptr_t)grad.data_ptr() | (uintptr_t)buffer.data_ptr()) % 16 == 0);
+  c10::cuda::CUDAGuard g(grad.device());
+  nxd::grad_to_buffer(grad.data_ptr(), dt_code(grad), buffer.data_ptr<float>(), grad.numel(), add, stream());
+}
 static void multi_tensor_scale(const std::vector<Tensor>& ts, const Tensor& scale) {
   if (ts.empty()) return;
   c10::cuda::CUDAGuard g(ts[0].device());
@@ -260,7 +268,7 @@ static void embedding_grad(const Tensor& ids, const Tensor& gy, Tensor out, bool
               gy.dim() == 2 && out.dim() == 2 && gy.size(0) == ids.numel() && gy.size(1) == out.size(1) && gy.size(1) % 8 == 0);
   TORCH_CHECK(((uintptr_t)gy.data_ptr() | (uintptr_t)out.data_ptr()) % 16 == 0);
   c10::cuda::CUDAGuard g(gy.device());
-  if (zero_first) out.zero_();
+  if (zero_first) C10_CUDA_CHECK(cudaMemsetAsync(out.data_ptr(), 0, out.nbytes(), stream()));
   const int T = (int)ids.numel(), H = (int)gy.size(1);
   auto ws = at::empty({(int64_t)nxd::embedding_grad_workspace(T, H)}, gy.options().dtype(at::kFloat));
   nxd::embedding_grad(ids.data_ptr<long>(), gy.data_ptr(), out.data_ptr(), dt_code(out), ws.data_ptr<float>(), T, H, out.size(0), stream());
@@ -894,6 +902,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("ce_stats", &ce_stats);
   m.def("ce_backward", &ce_backward);
   m.def("multi_tensor_sq_norm", &multi_tensor_sq_norm);
+  m.def("grad_to_buffer", &grad_to_buffer);
   m.def("multi_tensor_scale", &multi_tensor_scale);
   m.def("fused_adamw", &fused_adamw);
   m.def("gemm_bf16", &gemm_bf16);

@@ -34,6 +34,7 @@ void ce_backward(const void* logits, const int64_t* target, const float* lse, co
 // ---- optim.cu
 struct TensorRef { void* ptr; long numel; };
 void multi_tensor_sq_norm(const std::vector<TensorRef>& ts, int dt, float* out, cudaStream_t st);
+void grad_to_buffer(const void* grad, int dt, float* buffer, long n, bool add, cudaStream_t st);
 void multi_tensor_scale(const std::vector<TensorRef>& ts, int dt, const float* scale, cudaStream_t st);
 // p,m,v fp32; g dtype gdt; optional low-precision copy lowp (dtype ldt, may be empty)
 void fused_adamw(const std::vector<TensorRef>& p, const std::vector<TensorRef>& g, const std::vector<TensorRef>& m,

@@ -85,6 +85,32 @@ __global__ void __launch_bounds__(256) scale_kernel(const __grid_constant__ Chun
   });
 }
 
+// buffer = gradient, or += it, in fp32: a 16-bit gradient that autograd delivers into the optimizer's buffer.  Bound by HBM: four
+// elements per access, so that a warp's stores are whole lines, and eight accesses in flight per thread.  32000 x 4096 bf16: 137 us (5.7 TB/s), added 204; as copy_ 351.
+template <typename G, bool ADD>
+__global__ void __launch_bounds__(256) grad_to_buffer_kernel(const G* __restrict__ g, float* __restrict__ buf, long n) {
+  constexpr int U = 8;
+  const long quads = n / 4, step = (long)gridDim.x * 256;
+  const uint2* g4 = reinterpret_cast<const uint2*>(g);
+  float4* b4 = reinterpret_cast<float4*>(buf);
+  auto put = [&](const uint2& raw, long v) {
+    const G* x = reinterpret_cast<const G*>(&raw);
+    float4 y = make_float4(to_f32<G>(x[0]), to_f32<G>(x[1]), to_f32<G>(x[2]), to_f32<G>(x[3]));
+    if (ADD) { const float4 b = b4[v]; y.x += b.x; y.y += b.y; y.z += b.z; y.w += b.w; }
+    b4[v] = y;
+  };
+  long v = (long)blockIdx.x * 256 + threadIdx.x;
+  for (; v + (U - 1) * step < quads; v += U * step) {
+    uint2 x[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) x[u] = __ldg(g4 + v + u * step);
+#pragma unroll
+    for (int u = 0; u < U; ++u) put(x[u], v + u * step);
+  }
+  for (; v < quads; v += step) put(__ldg(g4 + v), v);
+  for (long i = quads * 4 + (long)blockIdx.x * 256 + threadIdx.x; i < n; i += step) buf[i] = ADD ? buf[i] + to_f32<G>(g[i]) : to_f32<G>(g[i]);
+}
+
 // One update rule covers both AdamW forms:
 //   p = (p * decay_pre - step_size * m / (sqrt(v * vscale) + eps)) * decay_post
 // torch form : step_size = lr/bc1, vscale = 1/bc2, decay_pre = 1 - lr*wd, decay_post = 1
@@ -319,6 +345,21 @@ void multi_tensor_scale(const std::vector<TensorRef>& ts, int dt, const float* s
       default: nxd_throw("bad dtype", __FILE__, __LINE__);
     }
   });
+  NXD_CUDA_CHECK(cudaGetLastError());
+}
+
+void grad_to_buffer(const void* grad, int dt, float* buffer, long n, bool add, cudaStream_t st) {
+  if (n == 0) return;
+  const int grid = (int)std::min<long>((n / 4 + 255) / 256 + 1, (long)device_sm_count() * 8);
+#define NXD_G2B(G)                                                                                        \
+  do {                                                                                                    \
+    if (add) grad_to_buffer_kernel<G, true><<<grid, 256, 0, st>>>((const G*)grad, buffer, n);             \
+    else grad_to_buffer_kernel<G, false><<<grid, 256, 0, st>>>((const G*)grad, buffer, n);                \
+  } while (0)
+  if (dt == kBF16) NXD_G2B(__nv_bfloat16);
+  else if (dt == kF16) NXD_G2B(__half);
+  else nxd_throw("grad_to_buffer: 16-bit gradients", __FILE__, __LINE__);
+#undef NXD_G2B
   NXD_CUDA_CHECK(cudaGetLastError());
 }
 

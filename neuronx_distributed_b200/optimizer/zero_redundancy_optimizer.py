@@ -294,11 +294,9 @@ class Zero1Optimizer(torch.optim.Optimizer):
         def hook(param):
             if param.grad is None:
                 return
-            if getattr(param, "main_grad_fresh", False):   # first contribution since zero_grad: overwrite
-                param.main_grad.copy_(param.grad)
-                param.main_grad_fresh = False
-            else:
-                param.main_grad.add_(param.grad)
+            # first contribution since zero_grad: overwrite
+            ops.optim.grad_to_buffer_(param.main_grad, param.grad, not getattr(param, "main_grad_fresh", False))
+            param.main_grad_fresh = False
             param.grad = None
             cb = getattr(param, "_nxd_grad_ready", None)
             if cb is not None:

@@ -157,3 +157,23 @@ def test_optimizer_slices(sizes, offset, gdtype, ldtype):
     for w, o, at in zip(whole, outside, [offset[0]] * 3 + [offset[1]] * 2):
         for a, b, n in zip(w, o, sizes):
             assert torch.equal(a[:at], b[:at]) and torch.equal(a[at + n:], b[at + n:])
+
+
+@pytest.mark.parametrize("n", [(1 << 20) - 1, 1 << 20, (1 << 20) + 13, 5 * 1000 * 1003])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("offset", [0, 1, 8])
+def test_gradients_into_the_buffer(n, dtype, offset):
+    from neuronx_distributed_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    grad = torch.randn(n + offset, generator=g, device="cuda").to(dtype)[offset:]
+    whole = torch.randn(n + 32, generator=g, device="cuda")
+    buf, outside = whole[16:16 + n], whole.clone()
+    want = buf + grad                                       # one fp32 sum per element
+    ops.optim.grad_to_buffer_(buf, grad, True)
+    assert torch.equal(buf, want)
+    ops.optim.grad_to_buffer_(buf, grad, False)
+    assert torch.equal(buf, grad.float())
+    assert torch.equal(whole[:16], outside[:16]) and torch.equal(whole[16 + n:], outside[16 + n:])
+    with pytest.raises(RuntimeError):
+        ops.optim.grad_to_buffer_(buf, grad[:n - 1], False)
