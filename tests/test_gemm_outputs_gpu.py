@@ -39,15 +39,19 @@ def test_grouped_weight_gradients(M, N, counts, dtype, accumulate):
     assert (out.double() - want).abs().max() <= (2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -16) * max(1.0, want.abs().max())
 
 
-# a last round of few tiles is split along K and summed by a second kernel: ragged rows and columns, both output types
-@pytest.mark.parametrize("M,N,K", [(1000, 5120, 1032), (264, 2056, 4096), (300, 264, 640), (5000, 4104, 520)])
+# a last round of few tiles is split along K and summed by a second kernel: ragged rows, columns and k-blocks, both output types; behind
+# full rounds of 74 tiles (80 and 160 tiles) and alone; `tail`: the output types for which the plan splits it
+@pytest.mark.parametrize("M,N,K,tail", [(1000, 5112, 1992, "bf16 fp32"), (1000, 5112, 4104, "bf16 fp32"), (2040, 5112, 4104, "bf16 fp32"),
+                                        (264, 2056, 4096, "bf16"), (520, 1032, 1992, "bf16"), (1000, 5120, 1032, ""), (300, 264, 640, ""),
+                                        (5000, 4104, 520, "")])
 @pytest.mark.parametrize("dtype,accumulate", [(torch.bfloat16, False), (torch.bfloat16, True), (torch.float32, False), (torch.float32, True)])
 @pytest.mark.parametrize("trans", [(False, True), (False, False), (True, False)])
-def test_split_tail(M, N, K, dtype, accumulate, trans):
+def test_split_tail(M, N, K, tail, dtype, accumulate, trans):
     from neuronx_distributed_b200 import ops
 
     if trans[0] and M % 8:
         M += 8 - M % 8
+    assert (ops._ext.ext().gemm_2cta_workspace(M, N, K, dtype is torch.float32, accumulate) > 0) == (("fp32" if dtype is torch.float32 else "bf16") in tail)
     g = torch.Generator(device="cuda").manual_seed(K)
     a = torch.randn(*((K, M) if trans[0] else (M, K)), generator=g, device="cuda").bfloat16()
     b = torch.randn(*((N, K) if trans[1] else (K, N)), generator=g, device="cuda").bfloat16()
