@@ -942,6 +942,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("seg") = c10::nullopt);
   m.def("grouped_wgrad", &grouped_wgrad);
   m.def("flash_attn_fwd", &flash_attn_fwd);
+  m.def("flash_attn_bwd_parts", &nxd::flash_attn_bwd_parts);
   m.def("flash_attn_bwd", &flash_attn_bwd, py::arg("go"), py::arg("q"), py::arg("k"), py::arg("v"), py::arg("o"), py::arg("lse"),
         py::arg("causal"), py::arg("scale"), py::arg("sbhd_out"), py::arg("dlse") = py::none(), py::arg("parts") = 0);
   m.def("ag_gemm_bf16", &ag_gemm_bf16);

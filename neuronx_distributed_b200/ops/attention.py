@@ -56,6 +56,12 @@ def _tma_view(t: torch.Tensor) -> torch.Tensor:
     return t
 
 
+def _bwd_launches(q, k, causal: bool) -> int:
+    """Preparation, main kernel, dQ, and the sums of dK and dV where blocks share a group of query heads."""
+    (B, S, H, _), (Skv, Hkv) = q.shape, k.shape[1:3]
+    return 3 if H == Hkv else 3 + (_ext.ext().flash_attn_bwd_parts(B, S, Skv, H, Hkv, causal) > 1)
+
+
 class _FlashAttn(torch.autograd.Function):
     """tcgen05 flash attention (``csrc/attention_sm100.cu``): forward saves (q, k, v, o, lse); backward is the transposed
     five-GEMM kernel.  Outputs/gradients are laid out ``[S,B,H,D]`` in memory (returned as ``[B,S,H,D]`` views) so the
@@ -75,7 +81,7 @@ class _FlashAttn(torch.autograd.Function):
     def backward(ctx, go):
         q, k, v, o, lse = ctx.saved_tensors
         e = _ext.ext()
-        _ext.count_launch(3)   # prep + main + dq convert
+        _ext.count_launch(_bwd_launches(q, k, bool(ctx.causal)))
         dq, dk, dv = e.flash_attn_bwd(_tma_view(go), q, k, v, o, lse, bool(ctx.causal), float(ctx.scale), True)
         return dq, dk, dv, None, None
 
@@ -96,7 +102,7 @@ class _FlashAttnLse(torch.autograd.Function):
     @staticmethod
     def backward(ctx, go, g_lse):
         q, k, v, o, lse = ctx.saved_tensors
-        _ext.count_launch(3)
+        _ext.count_launch(_bwd_launches(q, k, bool(ctx.causal)))
         go = torch.zeros_like(o) if go is None else go
         dlse = None if g_lse is None else g_lse.float().contiguous()
         dq, dk, dv = _ext.ext().flash_attn_bwd(_tma_view(go.to(o.dtype)), q, k, v, o, lse, bool(ctx.causal), float(ctx.scale), False, dlse)
