@@ -4,8 +4,6 @@
 //   rope apply        (overrides/transformer_overrides.py:20-32)
 //   vocab-parallel cross-entropy stats + backward (parallel_layers/loss_functions.py:12-129)
 // All are HBM-bound: 16-byte vector accesses, one pass over the data, fp32 math.
-#include <type_traits>
-
 #include "common.cuh"
 #include "kernels.h"
 

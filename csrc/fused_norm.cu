@@ -7,7 +7,7 @@
 //
 // Unfused this is an add kernel (read x, r; write h) plus the norm (read h; write y) = 5 row passes forward and, backward,
 // the norm backward (read gy, h; write d) plus an add (read d, gh; write dh) = 6; fused: 4 and 4.
-// The norm math is the one of elementwise.cu (rmsnorm_fwd_kernel / rmsnorm_bwd_kernel); h is rounded to the storage dtype
+// The forward math is that of rmsnorm_fwd_kernel (elementwise.cu), the backward kernel serves both norms; h is rounded to the storage dtype
 // BEFORE the statistics so that y is exactly rmsnorm(h_stored), i.e. bit-compatible with the unfused sequence.
 #include <algorithm>
 

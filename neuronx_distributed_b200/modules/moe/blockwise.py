@@ -45,7 +45,7 @@ def build_block_metadata(expert_index: torch.Tensor, num_experts: int, block_siz
 
         e = ops._ext.ext()
         if e is not None and hasattr(e, "moe_block_metadata"):
-            # one launch, no sort (csrc/select.cu moe_block_metadata_kernel — role of the reference's index-build NKI kernels)
+            # one launch, no sort (csrc/moe_blocks.cu moe_slots_kernel — role of the reference's index-build NKI kernels)
             ops._ext.count_launch()
             return e.moe_block_metadata(expert_index.contiguous(), int(num_experts), int(block_size), int(nb))
     flat_e = expert_index.reshape(-1)
@@ -133,7 +133,8 @@ def _grouped_swiglu(hidden: torch.Tensor, expert_affinities: torch.Tensor, exper
 
 def blockwise_expert_mlp(hidden: torch.Tensor, expert_affinities: torch.Tensor, expert_index: torch.Tensor,
                          experts, block_size: int, normalize: bool = False) -> torch.Tensor:
-    """Dropless MoE MLP: ``out[t] = Σ_j aff[t, e_j] · MLP_{e_j}(hidden[t])``."""
+    """Dropless MoE MLP: ``out[t] = Σ_j aff[t, e_j] · MLP_{e_j}(hidden[t])``.  ``block_size`` is the layout of the general path; silu-gated
+    experts on the grouped kernels take blocks of 256 rows whatever it says (their CTA-pair tile; blocks without tokens are skipped)."""
     E = expert_affinities.shape[-1]
     if normalize:
         denom = expert_affinities.gather(1, expert_index).sum(-1, keepdim=True).clamp(min=1e-9)

@@ -36,7 +36,7 @@ def test_optimizer_tables(sizes, gdtype):
         a = a - lr * math.sqrt(1 - b2 ** step) / (1 - b1 ** step) * c / (d.sqrt() + eps)
         want.append((a * (1 - lr * wd), c, d))
     total = sum(float((t.double() ** 2).sum()) for t in gr)
-    # fp32 sums in chunks of 8192 elements and one atomic per block
+    # fp32 sums in chunks of 4096 elements and one atomic per block
     assert abs(float(ops.optim.multi_tensor_sq_norm(gr)) - total) <= 2.0 ** -19 * max(total, 1e-9)
     ops.optim.fused_adamw_(p, gr, m, v, lr, b1, b2, eps, wd, step, torch.tensor(scale, device="cuda"), low)
     for i, w in enumerate(want):
