@@ -5,7 +5,7 @@
     torchrun --nproc-per-node N tools/nvls_bench.py --stage perf      # NVLS vs cudaIpc-push vs NCCL+GEMM on the Llama-2-7B shapes
     torchrun --nproc-per-node N tools/nvls_bench.py --stage sweep     # comm-CTA sweep of the NVLS kernels
 
-Every record is one JSON line on rank 0 and is appended to gpurun_out/nvls_bench_tpN.jsonl.  Timing: CUDA events on the
+Every record is one JSON line on rank 0 and is appended to output/nvls_bench_tpN.jsonl.  Timing: CUDA events on the
 launching stream, 5 warm-ups, median of 20, max over ranks; the collectives' inputs are rewritten between iterations
 by the kernels themselves (payload double-buffered), GEMM operands are far larger than they can stay hot against the
 traffic of the neighbouring ops (and the fused path's gain is overlap, which an L2-resident operand does not create).
@@ -307,8 +307,8 @@ def main():
 
     ps.initialize_model_parallel(tensor_model_parallel_size=WORLD)
     g = ps.get_tensor_model_parallel_group()
-    os.makedirs("gpurun_out", exist_ok=True)
-    OUT = f"gpurun_out/nvls_bench_tp{WORLD}.jsonl"
+    os.makedirs("output", exist_ok=True)
+    OUT = f"output/nvls_bench_tp{WORLD}.jsonl"
     try:
         if args.stage == "probe":
             stage_probe(g)

@@ -1,6 +1,6 @@
 """Micro-benchmark of the fused TP kernels vs the NCCL + GEMM baseline on the Llama-2-7B shapes.
 
-torchrun --nproc-per-node N tools/tp_bench.py        → gpurun_out/tp_bench_tpN.json
+torchrun --nproc-per-node N tools/tp_bench.py        → output/tp_bench_tpN.json
 Reports per op: fused µs, baseline µs (NCCL collective + own tcgen05 GEMM, and + cuBLAS), and the roofline
 max(FLOPs / measured-GEMM-peak, NVLink-bytes / 770 GB/s) with the achieved fraction."""
 import json
@@ -103,8 +103,8 @@ def main():
              "nccl_reduce_scatter_fp32_us": timeit(lambda: comm.reduce_scatter(y.float(), 0, g))}
     if rank == 0:
         print(json.dumps(extra), flush=True)
-        os.makedirs("gpurun_out", exist_ok=True)
-        json.dump({"ops": res, "collectives": extra}, open(f"gpurun_out/tp_bench_tp{world}.json", "w"), indent=1)
+        os.makedirs("output", exist_ok=True)
+        json.dump({"ops": res, "collectives": extra}, open(f"output/tp_bench_tp{world}.json", "w"), indent=1)
     dist.barrier()
     ps.destroy_model_parallel()
     dist.destroy_process_group()
