@@ -103,9 +103,12 @@ def blockwise_mlp_from_metadata(hidden: torch.Tensor, expert_affinities_masked: 
 
 
 def _grouped_swiglu_ok(hidden: torch.Tensor, expert_index: torch.Tensor, experts, num_experts: int) -> bool:
-    """silu-gated experts without clamps or biases on the grouped kernels: what ``_grouped_swiglu`` computes."""
+    """silu-gated experts without clamps, biases or an activation of their own on the grouped kernels: what ``_grouped_swiglu`` computes."""
     from ... import ops
+    from .experts import Experts
 
+    if getattr(type(experts), "activation", None) is not Experts.activation or "activation" in vars(experts):
+        return False
     if not (experts.glu_mlp and experts.glu_type == "glu" and experts.act is F.silu):
         return False
     if any(c is not None for c in (experts.gc_hi, experts.gc_lo, experts.uc_hi, experts.uc_lo)):

@@ -78,3 +78,24 @@ def test_slots(n, E, block):
     assert torch.equal(s.seg.cpu().long(), first)
     for a, b in zip(build_block_metadata(idx, E, block), (b2e, tp2id, counts)):
         assert torch.equal(a.cpu(), b)
+
+
+def test_experts_with_an_activation_of_their_own():
+    from neuronx_distributed_b200.modules.moe import blockwise
+
+    m = _experts(4, 128, 64)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(200, 128, generator=g, device="cuda").bfloat16()
+    aff, idx = torch.rand(200, 4, generator=g, device="cuda"), torch.randint(0, 4, (200, 1), generator=g, device="cuda")
+    op = m.mlp_op
+    want = blockwise.blockwise_expert_mlp(x, aff, idx, op, 128)
+    plain = type(op)
+    op.activation = lambda h: 2 * plain.activation(op, h)                 # on the object
+    assert not blockwise._grouped_swiglu_ok(x, idx, op, 4)
+    got = [blockwise.blockwise_expert_mlp(x, aff, idx, op, 128)]
+    del op.activation
+    op.__class__ = type("Doubled", (plain,), {"activation": lambda self, h: 2 * plain.activation(self, h)})      # of its class
+    assert not blockwise._grouped_swiglu_ok(x, idx, op, 4)
+    got.append(blockwise.blockwise_expert_mlp(x, aff, idx, op, 128))
+    for y in got:                                           # roundings to bfloat16 on the way, as in test_experts
+        assert (y.double() - 2 * want.double()).norm() <= 0.012 * 2 * want.double().norm()
