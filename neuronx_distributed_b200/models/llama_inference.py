@@ -136,7 +136,8 @@ class LlamaForInference(nn.Module):
     def _body(self, input_ids: torch.Tensor, positions: Optional[torch.Tensor], prefill: bool, kv_len: Optional[int], tree=None):
         core = self._core
         x = core.embed_tokens(input_ids).transpose(0, 1).contiguous()               # [S, B, H]
-        if prefill and x.shape[0] * x.shape[1] > 8 and _plain_norms(core):
+        if (prefill and x.shape[0] * x.shape[1] > 8 and type(self)._attn_block is LlamaForInference._attn_block
+                and "_attn_block" not in self.__dict__ and _plain_norms(core)):
             # residual sums inside the norms that follow them: one pass over the rows instead of two.  Up to 8 rows the sum rides in
             # the output projection's GEMV (+ all-reduce) instead, in fp32 and rounded once (_row_linear_plus_residual)
             d = None

@@ -94,3 +94,19 @@ def test_watched_norms_are_called():
     n.forward = lambda x: (seen.append(n), type(n).forward(n, x))[1]
     _prompt(m, ids)
     assert len(seen) == 1
+
+
+def test_attention_block_of_a_subclass():
+    """A class with an attention block of its own gets the stream and gives it back with the block's output added."""
+    m = _served(256, 2, torch.bfloat16)
+    ids = torch.randint(0, 64, (1, 16), device="cuda")
+    want, plain, calls = _prompt(m, ids), type(m), []
+
+    def block(self, i, layer, x, positions, prefill, kv_len, tree=None):
+        calls.append(i)
+        return plain._attn_block(self, i, layer, x, positions, prefill, kv_len, tree)
+
+    m.__class__ = type("Own", (plain,), {"_attn_block": block})
+    for a, b in zip(_prompt(m, ids), want):
+        assert torch.equal(a, b)
+    assert calls == [0, 1]
