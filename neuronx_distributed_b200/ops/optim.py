@@ -60,7 +60,7 @@ def grad_to_buffer_(buffer: torch.Tensor, grad: torch.Tensor, add: bool) -> None
     """``buffer = grad`` or ``buffer += grad``: a gradient that autograd delivers into the optimizer's gradient buffer.  Large 16-bit
     gradients of fp32 buffers (a token table) have a kernel; below a million elements a plain copy takes no longer."""
     if (grad.numel() >= 1 << 20 and buffer.is_cuda and grad.is_cuda and buffer.dtype == torch.float32
-            and grad.dtype in (torch.bfloat16, torch.float16) and buffer.shape == grad.shape and buffer.is_contiguous()
+            and grad.dtype in (torch.bfloat16, torch.float16) and buffer.shape == grad.shape and buffer.device == grad.device and buffer.is_contiguous()
             and grad.is_contiguous() and (buffer.data_ptr() | grad.data_ptr()) % 16 == 0 and _ext.use_cuda(buffer, grad)):
         _ext.count_launch()
         _ext.ext().grad_to_buffer(grad, buffer, bool(add))
