@@ -19,6 +19,7 @@
 
 #ifdef __cplusplus
 #include <stdexcept>
+#include <atomic>
 #include <string>
 inline void nxd_throw(const std::string& msg, const char* file, int line) {
   throw std::runtime_error(msg + " (" + file + ":" + std::to_string(line) + ")");
@@ -26,6 +27,19 @@ inline void nxd_throw(const std::string& msg, const char* file, int line) {
 #endif
 
 namespace nxd {
+
+// Lets `kernel` take `bytes` of dynamic shared memory, once per device and place of use (the call itself takes about 1 us).
+#define NXD_ALLOW_SMEM(kernel, bytes)                                                                                      \
+  do {                                                                                                                     \
+    static std::atomic<unsigned long long> allowed_{0};                                                                    \
+    int dev_;                                                                                                              \
+    NXD_CUDA_CHECK(cudaGetDevice(&dev_));                                                                                  \
+    const unsigned long long bit_ = dev_ < 64 ? 1ull << dev_ : 0ull;                                                       \
+    if (!(allowed_.load(std::memory_order_acquire) & bit_)) {                                                              \
+      NXD_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));                    \
+      allowed_.fetch_or(bit_, std::memory_order_release);                                                                  \
+    }                                                                                                                      \
+  } while (0)
 
 // Programmatic dependent launch: a kernel that was launched with launch_dependent starts while the one before it in the stream still
 // runs, and must pass pdl_wait before it touches anything that kernel wrote; pdl_trigger in the earlier one lets it start.

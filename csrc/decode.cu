@@ -352,7 +352,7 @@ void decode_attention(const void* q, const void* k, const void* v, const long* p
   const bool whole = splits == 1 && fin_o == nullptr;
 #define NXD_DEC(Gv)                                                                                                  \
   do {                                                                                                               \
-    NXD_CUDA_CHECK(cudaFuncSetAttribute(decode_attn_kernel<Gv>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecSmem)); \
+    NXD_ALLOW_SMEM(decode_attn_kernel<Gv>, kDecSmem);                                                                  \
     decode_attn_kernel<Gv><<<grid, kDecThreads, kDecSmem, st>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)k,      \
         (const __nv_bfloat16*)v, positions, part_o, part_ml, whole ? (__nv_bfloat16*)out : nullptr, B, H, Hkv, L,      \
         ks[0], ks[1], ks[2], vs[0], vs[1], vs[2], q_sb, q_sh, o_sb, o_sh, sl2, splits);                                \

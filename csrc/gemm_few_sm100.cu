@@ -168,7 +168,7 @@ void gemm_few_rows(const void* x, const void* w, const void* residual, void* y, 
   int cols = 32;
   while (cols < TN) cols *= 2;
   const CUtensorMap tw = make_tmap_bf16(w, N, K, BK, kSlab), tx = make_tmap_bf16(x, M, K, BK, TN);
-  NXD_CUDA_CHECK(cudaFuncSetAttribute(gemm_few_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+  NXD_ALLOW_SMEM(gemm_few_kernel, 226 * 1024);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(slabs * split); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute attr{};

@@ -28,10 +28,22 @@ template <int DEPTH> struct ChunkTable {
   int tensors;
 };
 
+// tensor of chunk c
+template <int DEPTH>
+NXD_DEVICE int tensor_of(const ChunkTable<DEPTH>& tab, long c) {
+  int lo = 0, hi = tab.tensors - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi) / 2;
+    if (tab.first[mid + 1] <= c) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
+
 // calls f(tensor, first element, elements) for every chunk of this block
 template <int DEPTH, typename F>
 NXD_DEVICE void each_chunk(const ChunkTable<DEPTH>& tab, F&& f) {
-  int t = 0;
+  int t = tensor_of(tab, blockIdx.x);
   for (long c = blockIdx.x; c < tab.first[tab.tensors]; c += gridDim.x) {
     while (tab.first[t + 1] <= c) ++t;
     const long base = (c - tab.first[t]) * kChunk;
@@ -205,7 +217,7 @@ __global__ void __launch_bounds__(kAdamThreads, 1) adamw_kernel(const __grid_con
   }
   __syncthreads();
   struct Chunk { float *p, *m, *v; const G* g; L* low; int n; bool bulk; };
-  int t_at = 0;                                    // chunks are visited in ascending order
+  int t_at = tensor_of(tab, blockIdx.x), t_load = t_at;      // chunks are visited in ascending order
   auto find = [&](long c, int& t) {
     while (tab.first[t + 1] <= c) ++t;
     const long off = (c - tab.first[t]) * kChunk;
@@ -232,7 +244,6 @@ __global__ void __launch_bounds__(kAdamThreads, 1) adamw_kernel(const __grid_con
   auto store = [&](void* dst, uint32_t src, uint32_t bytes) {
     asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
   };
-  int t_load = 0;
   long next = blockIdx.x;                          // next chunk to ask for (thread 0)
   auto load_next = [&](int st) {
     if (next < total) {
@@ -372,6 +383,7 @@ void fused_adamw(const std::vector<TensorRef>& p, const std::vector<TensorRef>& 
   AdamRule rule{hf_form ? lr * sqrtf(bc2) / bc1 : lr / bc1, beta1, beta2, eps, hf_form ? 1.f : 1.f - lr * wd, hf_form ? 1.f - lr * wd : 1.f,
                 hf_form ? 1.f : 1.f / bc2};
   std::vector<TensorRef> parts[2][5];              // 16-byte aligned throughout, others
+  for (int d = 0; d < 5; ++d) parts[0][d].reserve(lists[d]->size());
   for (size_t t = 0; t < p.size(); ++t) {
     uintptr_t bits = 0;
     for (const auto* l : lists) if (!l->empty()) bits |= (uintptr_t)(*l)[t].ptr;
@@ -381,7 +393,7 @@ void fused_adamw(const std::vector<TensorRef>& p, const std::vector<TensorRef>& 
 #define LAUNCH(G, L, HL)                                                                                                     \
   do {                                                                                                                       \
     if (direct) { adamw_direct_kernel<G, L, HL><<<nb, 256, 0, st>>>(tab, rule, grad_scale); break; }                         \
-    NXD_CUDA_CHECK(cudaFuncSetAttribute(adamw_kernel<G, L, HL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAdamSmem));    \
+    NXD_ALLOW_SMEM((adamw_kernel<G, L, HL>), kAdamSmem);                                                                     \
     adamw_kernel<G, L, HL><<<nb, kAdamThreads, kAdamSmem, st>>>(tab, rule, grad_scale);                                      \
   } while (0)
     if (gdt == kF32) {
