@@ -793,7 +793,8 @@ static GemmPlan gemm_plan(int M, int N, int K, int out_dt, bool accumulate) {
   p.tail = g2::Tail{0, 1, num_kb};
   const double kb_us = 0.39;
   double best = (double)((p.tiles + pairs - 1) / pairs) * num_kb * kb_us;
-  // The tail: s pairs per tile, at least 4 k-blocks each; worth it where it saves more than the launch that sums (3 us) and its traffic.
+  // The tail: s pairs per tile, at least 4 k-blocks each; worth it where it saves more than the launch that sums (4 us) and its traffic
+  // (256 x 1024 x 1024 stays whole: 14.3 us, 17.4 with a tail).
   // 1000 x 5120 x 13824 (80 tiles): 104 us, 143 with a second round of six tiles; cut into narrower columns instead, its pieces waited
   // for their loads as long as a whole tile.  1000 x 27648 x 5120 from [K, N] weights: 203, 281 before.
   // Rows of other lengths have no tail: gemm_tail_kernel writes whole groups of 8 columns.
@@ -802,7 +803,7 @@ static GemmPlan gemm_plan(int M, int N, int K, int out_dt, bool accumulate) {
   if (s > 1) {
     const int per = (num_kb + s - 1) / s;
     s = (num_kb + per - 1) / per;                          // no empty split
-    const double cost = (p.tiles / pairs) * num_kb * kb_us + per * kb_us + 3.0 + 2.0 * last * s * 0.262144 / 6.0;
+    const double cost = (p.tiles / pairs) * num_kb * kb_us + per * kb_us + 4.0 + 2.0 * last * s * 0.262144 / 6.0;
     if (s > 1 && cost < best) { best = cost; p.tail = g2::Tail{last, s, per}; }
   }
   // Split-K for fp32 outputs (weight gradients): K = tokens is long while the output often has fewer tiles than the

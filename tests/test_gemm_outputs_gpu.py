@@ -41,8 +41,8 @@ def test_grouped_weight_gradients(M, N, counts, dtype, accumulate):
 
 # a last round of few tiles is split along K and summed by a second kernel: ragged rows, columns and k-blocks, both output types; behind
 # full rounds of 74 tiles (80 and 160 tiles) and alone; `tail`: the output types for which the plan splits it
-@pytest.mark.parametrize("M,N,K,tail", [(1000, 5112, 1992, "bf16 fp32"), (1000, 5112, 4104, "bf16 fp32"), (2040, 5112, 4104, "bf16 fp32"),
-                                        (264, 2056, 4096, "bf16"), (520, 1032, 1992, "bf16"), (1000, 5120, 1032, ""), (300, 264, 640, ""),
+@pytest.mark.parametrize("M,N,K,tail", [(1000, 5112, 2504, "bf16 fp32"), (1000, 5112, 4104, "bf16 fp32"), (2040, 5112, 4104, "bf16 fp32"),
+                                        (264, 2056, 4096, "bf16"), (520, 1032, 2504, "bf16"), (256, 1024, 1024, ""), (1000, 5120, 1032, ""), (300, 264, 640, ""),
                                         (5000, 4104, 520, "")])
 @pytest.mark.parametrize("dtype,accumulate", [(torch.bfloat16, False), (torch.bfloat16, True), (torch.float32, False), (torch.float32, True)])
 @pytest.mark.parametrize("trans", [(False, True), (False, False), (True, False)])
@@ -72,7 +72,7 @@ def test_split_tail(M, N, K, tail, dtype, accumulate, trans):
 def test_no_tail_for_other_widths(N, accumulate):
     from neuronx_distributed_b200 import ops
 
-    e, M, K = ops._ext.ext(), 1000, 1992
+    e, M, K = ops._ext.ext(), 1000, 2504
     assert e.gemm_2cta_workspace(M, 5112, K, True, accumulate) > 0 and e.gemm_2cta_workspace(M, N, K, True, accumulate) == 0
     g = torch.Generator(device="cuda").manual_seed(N)
     a, b = (torch.randn(n, K, generator=g, device="cuda").bfloat16() for n in (M, N))
