@@ -1018,6 +1018,7 @@ void flash_attn_fwd(const void* q, const void* k, const void* v, void* out, floa
                     cudaStream_t st) {
   using namespace fa;
   if (causal && S_q != S_kv) nxd_throw("attention: causal needs S_q == S_kv", __FILE__, __LINE__);
+  if (S_kv <= 0 && (long)S_q * H * B > 0) nxd_throw("attention: no keys", __FILE__, __LINE__);      // the kernel's items have a K / V tile
   FwdParams p;
   p.S_q = S_q; p.S_kv = S_kv; p.H = H; p.Hkv = Hkv; p.B = B;
   const CUtensorMap tq = view_tmap(View{q, B, S_q, H, qs[0], qs[1], qs[2]}, p.q);

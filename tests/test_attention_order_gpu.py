@@ -60,3 +60,12 @@ def test_all_keys_visible(sq, skv, heads):
     p = torch.softmax(q.float().transpose(1, 2) @ k.float().transpose(1, 2).transpose(-1, -2) / math.sqrt(128), -1)
     want = (p @ v.float().transpose(1, 2)).transpose(1, 2)
     assert ((got - want).norm(dim=-1) <= 0.02 * want.norm(dim=-1) + 1e-3).all()
+
+
+@pytest.mark.parametrize("batch", [1, 2])
+def test_no_keys_is_an_error(batch):
+    from neuronx_distributed_b200 import ops
+
+    q, k = (torch.randn(batch, n, 8, 128, device="cuda").bfloat16() for n in (40, 0))
+    with pytest.raises(RuntimeError):
+        ops.attention.flash_attention(q, k, k, causal=False)
