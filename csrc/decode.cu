@@ -338,8 +338,9 @@ void decode_rope_kv(const void* q, const void* k, const void* v, const long* pos
 // Stretches per (sequence, key/value head): about six blocks per SM in all, so that sequences of unequal length fill the GPU to
 // the end (8 x 8192 rows, 8 key/value heads: 39 us; four per SM 41, sixteen 45), and no stretch below 256 rows, where a block's
 // start and the merge outweigh its reading (1 x 2048 rows, 40 heads: 11.2 us with the merge; 128-row stretches 12.1, 64-row 14.7).
+int device_sm_count();
 int decode_splits(int pairs, int L) {
-  const int want = (6 * 148 + pairs - 1) / pairs;
+  const int want = (6 * device_sm_count() + pairs - 1) / pairs;
   return std::max(1, std::min(std::min(want, 64), (L + 255) / 256));
 }
 

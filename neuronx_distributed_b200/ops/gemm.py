@@ -41,8 +41,9 @@ def _few_rows(M: int, N: int, K: int) -> bool:
     """Rows for which streaming the weights decides the time (``csrc/gemm_few_sm100.cu``).  Up to 64 always (48 rows of 4096 x 11008:
     21 us against 69) and up to 128 unless the columns are so many that the wide tiles fill the GPU many times over (128 rows: 57344 x 8192
     168 against 171, 128256 x 4096 206 against 194).  Above, one block fits an SM, and it wins on long rows where the wide tiles would leave
-    SMs idle (200 rows: 4096 x 11008 28 us against 71, 7168 x 8192 35 against 58) or by its smaller padding (136 rows of 22016 x 4096: 57
-    against 65; 248: 73 against 68); on short rows it loses (176 rows: 32000 x 512 29 against 26, 8192 x 1024 20 against 18)."""
+    SMs idle (200 rows: 4096 x 11008 28 us against 71, 7168 x 8192 35 against 58; 9472 columns are 74 slabs of 128, one for each pair of
+    SMs) or by its smaller padding (136 rows of 22016 x 4096: 57 against 65; 248: 73 against 68); on short rows it loses (176 rows:
+    32000 x 512 29 against 26, 8192 x 1024 20 against 18)."""
     if M <= 128:
         return M <= 64 or N <= 65536
     return K >= 2048 and (N <= 9472 or (M <= 176 and N <= 65536)) and M < 256
