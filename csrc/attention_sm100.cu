@@ -1055,9 +1055,9 @@ int device_sm_count();
 //   1 x 512, 32 on 8: 70 and 48;  16 on 1: 192 and 44.  Left whole: 1 x 4096, 32 on 8 (415; two parts 433), 2 x 2048 (255; 294).
 int flash_attn_bwd_parts(int B, int S_q, int S_kv, int H, int Hkv, bool causal) {
   using namespace fa;
-  const int group = H / Hkv, sms = device_sm_count();
+  if (S_q <= 0 || S_kv <= 0 || H < 1 || Hkv < 1 || H % Hkv) return 1;
+  const int group = H / Hkv, sms = std::max(1, device_sm_count());
   const long nq = (S_q + BQ - 1) / BQ, tiles = (S_kv + BN - 1) / BN;
-  if (S_q <= 0 || S_kv <= 0 || H % Hkv) return 1;
   long steps = 0;                                                 // query tiles of one head, over its K/V tiles
   for (long n = 0; n < tiles; ++n) steps += nq - (causal ? n * (BN / BQ) : 0);
   int best = 1;

@@ -786,7 +786,7 @@ static CUtensorMap out_map(const void* out, int out_dt, bool accumulate, bool ma
 // 256 x 256 tile: 0.39 us per k-block; a pass over fp32 memory: 6 bytes/ps.
 struct GemmPlan { int tiles, split; g2::Tail tail; };
 static GemmPlan gemm_plan(int M, int N, int K, int out_dt, bool accumulate) {
-  const int pairs = device_sm_count() / 2, num_kb = (K + g2::BK - 1) / g2::BK;
+  const int pairs = std::max(1, device_sm_count() / 2), num_kb = (K + g2::BK - 1) / g2::BK;      // (no device: one, for the asking)
   GemmPlan p;
   p.tiles = ((M + g2::TILE_M - 1) / g2::TILE_M) * ((N + g2::TILE_N - 1) / g2::TILE_N);
   p.split = 1;
