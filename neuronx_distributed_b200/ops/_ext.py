@@ -61,13 +61,14 @@ def load_error() -> Optional[BaseException]:
     return _LOAD_ERROR
 
 
+_OS_ENVIRON = os.environ
 _ENVIRON = getattr(os.environ, "_data", None)      # POSIX: the dict behind os.environ (bytes to bytes)
 
 
 def env(name: str, default: str = "") -> str:
     """``os.environ.get`` for switches that are read on every call: a look into the dict behind it (a missing key costs
     ``os.environ`` an encoded copy of the name and an exception, about 1 us, a hundred times in a training step)."""
-    if _ENVIRON is None:
+    if _ENVIRON is None or os.environ is not _OS_ENVIRON:      # another mapping has been put in its place
         return os.environ.get(name, default)
     key = _ENV_KEYS.get(name)
     if key is None:
