@@ -13,6 +13,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "sm100_ptx.cuh"
 
 namespace nxd {
 
@@ -85,89 +86,106 @@ __global__ void __launch_bounds__(256) add_rmsnorm_fwd_kernel(const T* __restric
 }
 
 // Backward of both norms (RES: with the gradient arriving on the residual path).  Persistent blocks stride over rows; each thread
-// owns fixed columns, so its part of dW lives in registers across rows.  Bound by HBM if enough bytes are in flight: the rows of
-// the next step (up to three 16-byte packets per thread) are loaded before this step's sum is reduced, and the sum costs one
-// barrier (two alternating sets of partials).  8192 x 4096, bf16, with the residual path: 58 us (41 for its bytes), 95 with loads
-// behind two barriers per row; the sum of the parts 3.5 us.
-template <typename T, int VPT, bool RES>
-__global__ void __launch_bounds__(512, VPT == 1 ? 2 : 1) norm_bwd_kernel(const T* __restrict__ gy, const T* __restrict__ gh,
-                                                                         const T* __restrict__ h, const T* __restrict__ w,
-                                                                         const float* __restrict__ rstd, T* __restrict__ dh,
-                                                                         float* __restrict__ partial_dw, int rows, int H) {
+// owns one or two packets of columns, so its part of dW lives in registers across rows.  Bound by HBM if enough bytes are in flight: whole
+// rows come into two stages of shared memory by bulk copies (a row's h, gy and gh are one stage; three or four stages are no faster), and
+// the row's sum costs one barrier, behind which the stage is asked for again.  With the loads of the next row in registers instead, the
+// blocks per SM were half as many.  Both kernels, bf16 with the residual path, before and now: 8192 x 4096 61.7 and 51.1 us (41 for its
+// bytes at the copy rate), 16384 x 4096 111 and 90, 16384 x 1024 45 and 32, 16384 x 8192 171 and 159, 64 x 4096 8.3 and 6.3.
+template <typename T, bool RES, int VPT, int MAXT>
+__global__ void __launch_bounds__(MAXT, MAXT == 1024 ? 1 : VPT == 1 ? 3 : 2) norm_bwd_kernel(const T* __restrict__ gy, const T* __restrict__ gh,
+                                                                        const T* __restrict__ h, const T* __restrict__ w,
+                                                                        const float* __restrict__ rstd, T* __restrict__ dh,
+                                                                        float* __restrict__ partial_dw, int rows, int H) {
   using P = Pack16<T>;
   constexpr int N = P::N;
-  __shared__ float red[2][16];
-  const int nvec = H / N, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  extern __shared__ __align__(128) uint8_t ring_raw[];
+  __shared__ __align__(16) float red[2][32];
+  __shared__ __align__(8) uint64_t full_bar[2];
+  const uint32_t ring = smem_u32(ring_raw), full = smem_u32(full_bar);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const uint32_t row_bytes = (uint32_t)H * sizeof(T), stage_bytes = (RES ? 3 : 2) * row_bytes;
   const float inv_h = 1.f / (float)H;
-  struct Row { P h[VPT], g[VPT], r[VPT]; float rs; };
+  auto fetch = [&](unsigned row, int st) {                      // one thread
+    const uint32_t dst = ring + st * stage_bytes, bar = full + 8 * st;
+    const size_t base = (size_t)row * H;
+    mbar_expect_tx(bar, stage_bytes);
+    bulk_load(dst, h + base, row_bytes, bar);
+    bulk_load(dst + row_bytes, gy + base, row_bytes, bar);
+    if constexpr (RES) bulk_load(dst + 2 * row_bytes, gh + base, row_bytes, bar);
+  };
+  if (threadIdx.x == 0) {
+    mbar_init(full, 1);
+    mbar_init(full + 8, 1);
+    fence_barrier_init();
+    fetch(blockIdx.x, 0);                                  // the grid has no more blocks than rows
+    if (blockIdx.x + gridDim.x < (unsigned)rows) fetch(blockIdx.x + gridDim.x, 1);
+  }
+  if (threadIdx.x < 32) red[0][threadIdx.x] = red[1][threadIdx.x] = 0.f;
   float dw[VPT][N];
   P pw[VPT];
-  bool live[VPT];
+  auto at = [&](int i) { return (int)(threadIdx.x + i * blockDim.x) * N; };      // column of this thread's packet i
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
-    const int v = threadIdx.x + i * blockDim.x;
-    live[i] = v < nvec;
 #pragma unroll
     for (int j = 0; j < N; ++j) dw[i][j] = 0.f;
-    if (live[i]) pw[i].load_nc(w + v * N);
+    if (at(i) < H) pw[i].load_nc(w + at(i));
   }
-  auto load = [&](Row& x, int row) {
-    const size_t base = (size_t)row * H;
-    x.rs = rstd[row];
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int v = threadIdx.x + i * blockDim.x;
-      if (live[i]) {
-        x.h[i].load(h + base + v * N);
-        x.g[i].load(gy + base + v * N);
-        if constexpr (RES) x.r[i].load(gh + base + v * N);
-      }
-    }
-  };
-  Row cur, nxt;
-  if ((int)blockIdx.x < rows) load(cur, blockIdx.x);
-  int buf = 0;
-  for (int row = blockIdx.x; row < rows; row += gridDim.x) {
-    if (row + (int)gridDim.x < rows) load(nxt, row + gridDim.x);
-    const float rs = cur.rs;
+  float rs = rstd[blockIdx.x];
+  __syncthreads();
+  pdl_trigger();                                           // the sum of the parts may take its place; it waits for this grid
+  int st = 0;
+  uint32_t ph = 0;
+  for (unsigned row = blockIdx.x; row < (unsigned)rows; row += gridDim.x) {
+    const float rs_next = row + gridDim.x < (unsigned)rows ? rstd[row + gridDim.x] : 0.f;
+    mbar_wait(full + 8 * st, ph);
+    P xh[VPT], xg[VPT], xr[VPT];
     float dot = 0.f;
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-      if (live[i]) {
+      if (at(i) < H) {
+        const T* src = reinterpret_cast<const T*>(ring_raw + st * stage_bytes) + at(i);
+        xh[i].load(src);
+        xg[i].load(src + H);
+        if constexpr (RES) xr[i].load(src + 2 * H);
 #pragma unroll
         for (int j = 0; j < N; ++j) {
-          const float hh = cur.h[i].f(j) * rs, gg = cur.g[i].f(j);
+          const float hh = xh[i].f(j) * rs, gg = xg[i].f(j);
           dot += gg * pw[i].f(j) * hh;
           dw[i][j] += gg * hh;
         }
       }
     }
     dot = warp_sum(dot);
-    if (lane == 0) red[buf][warp] = dot;
+    if (lane == 0) red[st][warp] = dot;
     __syncthreads();
-    dot = warp_sum(lane < nw ? red[buf][lane] : 0.f) * inv_h;
-    buf ^= 1;
+    if (threadIdx.x == 0 && row + 2 * gridDim.x < (unsigned)rows) fetch(row + 2 * gridDim.x, st);
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    #pragma unroll
+    for (int i = 0; i < MAXT / 32; i += 4) {                      // a broadcast read of all warps' sums: shorter than five more shuffles
+      const float4 t = *reinterpret_cast<const float4*>(&red[st][i]);
+      sum.x += t.x; sum.y += t.y; sum.z += t.z; sum.w += t.w;
+    }
+    dot = ((sum.x + sum.y) + (sum.z + sum.w)) * inv_h;
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-      const int v = threadIdx.x + i * blockDim.x;
-      if (live[i]) {
+      if (at(i) < H) {
         P po;
 #pragma unroll
         for (int j = 0; j < N; ++j) {
-          const float hh = cur.h[i].f(j) * rs;
-          const float d = rs * (cur.g[i].f(j) * pw[i].f(j) - hh * dot);
-          po.set(j, RES ? cur.r[i].f(j) + d : d);
+            const float d = rs * (xg[i].f(j) * pw[i].f(j) - (xh[i].f(j) * rs) * dot);
+          po.set(j, RES ? xr[i].f(j) + d : d);
         }
-        po.store(dh + (size_t)row * H + v * N);
+        po.store(dh + (size_t)row * H + at(i));
       }
     }
-    cur = nxt;
+    rs = rs_next;
+    st ^= 1;
+    if (st == 0) ph ^= 1;
   }
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
-    const int v = threadIdx.x + i * blockDim.x;
-    if (live[i]) {
-      float* o = partial_dw + (size_t)blockIdx.x * H + v * N;
+    if (at(i) < H) {
+      float* o = partial_dw + (size_t)blockIdx.x * H + at(i);
 #pragma unroll
       for (int j = 0; j < N; j += 4) *reinterpret_cast<float4*>(o + j) = make_float4(dw[i][j], dw[i][j + 1], dw[i][j + 2], dw[i][j + 3]);
     }
@@ -179,6 +197,7 @@ __global__ void __launch_bounds__(512, VPT == 1 ? 2 : 1) norm_bwd_kernel(const T
 template <typename T>
 static __global__ void __launch_bounds__(256) norm_bwd_reduce_kernel(const float* __restrict__ partial, T* __restrict__ out, int nparts, int H) {
   __shared__ float4 part[32][8];
+  pdl_wait();
   const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3, c = blockIdx.x * 32 + tx * 4;
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
   if (c < H) {
@@ -227,18 +246,30 @@ void add_rmsnorm_fwd(const void* x, const void* r, const void* w, void* h, void*
 
 int device_sm_count();
 
-// Threads of a block: one packet each up to 512, then two; two to four blocks per SM (one where a thread owns two packets).
+// Threads of a block: one packet each, but two each between 512 and 768 packets, so that two blocks fit an SM.  Blocks per SM: as
+// registers allow, but no fewer than four rows per block (each block ends in a part of dW that another kernel reads; 1024 x 4096 in
+// blocks of two to three rows 14.4 us, of seven 12.4).
 static void norm_bwd_shape(int rows, int H, int dt, int& threads, int& vpt, int& grid) {
-  const int nvec = H / (dt == kF32 ? 4 : 8);
-  threads = std::min(512, (nvec + 31) / 32 * 32);
-  vpt = (nvec + threads - 1) / threads;
-  const int per_sm = vpt > 1 ? 1 : threads > 256 ? 2 : 4;
-  grid = std::min(rows, device_sm_count() * per_sm);
+  const int size = dt == kF32 ? 4 : 2, nvec = H / (16 / size);
+  vpt = nvec > 512 && nvec <= 768 ? 2 : 1;
+  threads = std::max(32, ((nvec + vpt - 1) / vpt + 31) / 32 * 32);
+  const int sms = device_sm_count(), most = std::min(8, (threads > 512 || vpt > 1 ? 1024 : 1536) / threads);
+  grid = std::min(rows, sms * std::max(1, std::min(most, rows / (4 * sms))));
 }
 int rmsnorm_bwd_num_partials(int rows, int H, int dt) {
   int th, vpt, grid;
   norm_bwd_shape(rows, H, dt, th, vpt, grid);
   return grid;
+}
+
+template <typename T, bool RES, int VPT, int MAXT>
+static void norm_bwd_launch(const void* gy, const void* gh, const void* h, const void* w, const float* rstd, void* dh, float* partial, int rows,
+                            int H, int threads, int grid, cudaStream_t st) {
+  constexpr int kMost = 6 * 1024 * 16;                     // two stages of three rows of 1024 packets
+  NXD_ALLOW_SMEM((norm_bwd_kernel<T, RES, VPT, MAXT>), kMost);
+  norm_bwd_kernel<T, RES, VPT, MAXT><<<grid, threads, (size_t)(RES ? 6 : 4) * H * sizeof(T), st>>>(
+      (const T*)gy, (const T*)gh, (const T*)h, (const T*)w, rstd, (T*)dh, partial, rows, H);
+  NXD_CUDA_CHECK(cudaGetLastError());
 }
 
 template <bool RES>
@@ -249,11 +280,11 @@ static void norm_bwd(const void* gy, const void* gh, const void* h, const void* 
   FN_DISPATCH_DTYPE(dt, {
     const int nvec = H / Pack16<T>::N;
     if (H % Pack16<T>::N || nvec > 256 * 4) nxd_throw("rmsnorm_bwd: unsupported H", __FILE__, __LINE__);
-    if (vpt == 1) norm_bwd_kernel<T, 1, RES><<<grid, th, 0, st>>>((const T*)gy, (const T*)gh, (const T*)h, (const T*)w, rstd, (T*)dh, partial, rows, H);
-    else norm_bwd_kernel<T, 2, RES><<<grid, th, 0, st>>>((const T*)gy, (const T*)gh, (const T*)h, (const T*)w, rstd, (T*)dh, partial, rows, H);
-    norm_bwd_reduce_kernel<T><<<(H + 31) / 32, 256, 0, st>>>(partial, (T*)dw, grid, H);
+    if (vpt == 2) norm_bwd_launch<T, RES, 2, 512>(gy, gh, h, w, rstd, dh, partial, rows, H, th, grid, st);
+    else if (th <= 512) norm_bwd_launch<T, RES, 1, 512>(gy, gh, h, w, rstd, dh, partial, rows, H, th, grid, st);
+    else norm_bwd_launch<T, RES, 1, 1024>(gy, gh, h, w, rstd, dh, partial, rows, H, th, grid, st);
+    launch_dependent(norm_bwd_reduce_kernel<T>, (H + 31) / 32, 256, 0, st, (const float*)partial, (T*)dw, grid, H);
   });
-  NXD_CUDA_CHECK(cudaGetLastError());
 }
 
 void add_rmsnorm_bwd(const void* gy, const void* gh, const void* h, const void* w, const float* rstd, void* dh,

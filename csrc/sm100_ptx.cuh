@@ -60,6 +60,11 @@ NXD_DEVICE void tma_load_2d(uint32_t smem_dst, const CUtensorMap* map, uint32_t 
       ::"r"(smem_dst), "l"(map), "r"(bar), "r"(c0), "r"(c1)
       : "memory");
 }
+// untiled copy of `bytes` (both addresses and the size multiples of 16) that completes `bar`
+NXD_DEVICE void bulk_load(uint32_t smem_dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(smem_dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
 NXD_DEVICE void prefetch_tmap(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
