@@ -152,6 +152,17 @@ static Tensor ce_stats(const Tensor& logits, const Tensor& target, int64_t vocab
                   (int)logits.size(1), (int)vocab_start, dt_code(logits), stream());
   return stats;
 }
+// loss and log-normaliser of rows that hold the whole vocabulary
+static std::vector<Tensor> ce_loss(const Tensor& logits, const Tensor& target) {
+  CHECK_IN(logits); CHECK_IN(target);
+  TORCH_CHECK(target.scalar_type() == at::kLong && logits.dim() == 2 && target.numel() == logits.size(0));
+  c10::cuda::CUDAGuard g(logits.device());
+  auto loss = at::empty({logits.size(0)}, logits.options().dtype(at::kFloat)), lse = at::empty_like(loss);
+  if (logits.size(0))
+    nxd::ce_loss(logits.data_ptr(), target.data_ptr<int64_t>(), lse.data_ptr<float>(), loss.data_ptr<float>(),
+                 (int)logits.size(0), (int)logits.size(1), dt_code(logits), stream());
+  return {loss, lse};
+}
 static Tensor ce_backward(const Tensor& logits, const Tensor& target, const Tensor& lse, const Tensor& gout,
                           int64_t vocab_start, double smoothing, int64_t vocab) {
   CHECK_IN(logits); CHECK_IN(target); CHECK_IN(lse); CHECK_IN(gout);
@@ -900,6 +911,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("rope_qkv_fwd", &rope_qkv_fwd);
   m.def("rope_qkv_bwd", &rope_qkv_bwd);
   m.def("ce_stats", &ce_stats);
+  m.def("ce_loss", &ce_loss);
   m.def("ce_backward", &ce_backward);
   m.def("multi_tensor_sq_norm", &multi_tensor_sq_norm);
   m.def("grad_to_buffer", &grad_to_buffer);

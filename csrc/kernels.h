@@ -28,6 +28,7 @@ void rope_qkv_bwd(const void* gq, const void* gk, const void* gv, const long (*s
                   int S, int B, int H, int K, int D, int dt, cudaStream_t st);
 void ce_stats(const void* logits, const int64_t* target, float* stats, int rows, int V, int vocab_start, int dt,
               cudaStream_t st);
+void ce_loss(const void* logits, const int64_t* target, float* lse, float* loss, int rows, int V, int dt, cudaStream_t st);
 void ce_backward(const void* logits, const int64_t* target, const float* lse, const float* gout, void* grad, int rows,
                  int V, int vocab_start, float smoothing, int vocab, int dt, cudaStream_t st);
 

@@ -51,7 +51,7 @@ _EXT_RESOURCE_PREFIXES = ("vmm_", "symm_", "tp_gemm", "nvls_", "gemv_allreduce",
 # writing to EVERY tensor argument: conservative — such tensors count as state, are never hoisted or dropped — but safe.
 _EXT_PURE = frozenset({"rmsnorm_fwd", "rmsnorm_bwd", "add_rmsnorm_fwd", "add_rmsnorm_bwd", "swiglu_fwd", "swiglu_bwd", "rope_apply",
                        "rope_qkv_fwd", "rope_qkv_bwd",
-                       "ce_stats", "ce_backward", "decode_attention", "decode_attention_partial", "gemv", "gemm_few_rows", "gemv_mx",
+                       "ce_stats", "ce_loss", "ce_backward", "decode_attention", "decode_attention_partial", "gemv", "gemm_few_rows", "gemv_mx",
                        "gemm_mxfp8", "moe_block_tkg", "moe_block_metadata", "moe_slots", "moe_gather", "moe_combine",
                        "moe_combine_grad", "row_argmax", "row_topk", "flash_attn_fwd",
                        "flash_attn_bwd", "flash_attn_bwd_parts", "moe_block_tkg_supported", "row_topk_supported", "grouped_gemm"})

@@ -26,6 +26,16 @@ def ce_stats(logits2d: torch.Tensor, target: torch.Tensor, vocab_start: int) -> 
     return torch.stack([mx, se, tl, x.sum(-1)], dim=1)
 
 
+def ce_loss(logits2d: torch.Tensor, target: torch.Tensor):
+    """``(loss, lse)`` per row, fp32, of rows that hold the whole vocabulary: what ``ce_stats`` gives, finished in the same pass."""
+    if _ext.use_cuda(logits2d) and logits2d.dtype in (torch.bfloat16, torch.float32, torch.float16):
+        _ext.count_launch()
+        return _ext.ext().ce_loss(logits2d.contiguous(), target.contiguous().long())
+    stats = ce_stats(logits2d, target, 0)
+    lse = stats[:, 0] + torch.log(stats[:, 1])
+    return lse - stats[:, 2], lse
+
+
 def ce_backward(logits2d, target, lse, gout, vocab_start: int, smoothing: float, vocab: int) -> torch.Tensor:
     if _ext.use_cuda(logits2d) and logits2d.dtype in (torch.bfloat16, torch.float32, torch.float16):
         _ext.count_launch()

@@ -45,6 +45,12 @@ class _ParallelCrossEntropy(torch.autograd.Function):
         start, _ = EmbeddingUtility.range_from_per_partition_vocab_size(vp, r, n)
         logits2d = vocab_parallel_logits.reshape(-1, vp)
         tgt = target.reshape(-1)
+        vocab = vp * n
+        ctx.label_smoothing, ctx.vocab, ctx.start, ctx.shape = label_smoothing, vocab, start, vocab_parallel_logits.shape
+        if n == 1 and not label_smoothing > 0:
+            loss, lse = ops.cross_entropy.ce_loss(logits2d, tgt)
+            ctx.save_for_backward(logits2d, tgt, lse)
+            return loss.view(target.shape)
         # stats: [T, 4] = (max, sumexp, target_logit, sum_logits)
         stats = ops.cross_entropy.ce_stats(logits2d, tgt, start)
         if n > 1:
@@ -57,15 +63,12 @@ class _ParallelCrossEntropy(torch.autograd.Function):
             gmax, sumexp, pred, sum_logits = stats[:, 0], stats[:, 1], stats[:, 2], stats[:, 3]
         lse = gmax + torch.log(sumexp)  # log normaliser per row
         loss = lse - pred
-        vocab = vp * n
         if label_smoothing > 0:
             assert 1.0 > label_smoothing > 0.0
             smoothing = label_smoothing * vocab / (vocab - 1)
             mean_log_probs = sum_logits / vocab - lse
             loss = (1.0 - smoothing) * loss - smoothing * mean_log_probs
-        ctx.label_smoothing, ctx.vocab, ctx.start = label_smoothing, vocab, start
         ctx.save_for_backward(logits2d, tgt, lse)
-        ctx.shape = vocab_parallel_logits.shape
         return loss.view(target.shape)
 
     @staticmethod
