@@ -4,6 +4,7 @@
 #include <pybind11/stl.h>
 #include <torch/extension.h>
 
+#include "bindings.h"
 #include "kernels.h"
 #include "symm.h"
 
@@ -21,7 +22,7 @@ static int dt_code(const Tensor& t) {
 static cudaStream_t stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 #define CHECK_IN(t) TORCH_CHECK((t).is_cuda() && (t).is_contiguous(), #t " must be a contiguous CUDA tensor")
 
-static std::vector<Tensor> rmsnorm_fwd(const Tensor& x, const Tensor& w, double eps) {
+std::vector<Tensor> rmsnorm_fwd(const Tensor& x, const Tensor& w, double eps) {
   CHECK_IN(x); CHECK_IN(w);
   TORCH_CHECK(x.dim() == 2 && w.numel() == x.size(1) && w.scalar_type() == x.scalar_type());
   c10::cuda::CUDAGuard g(x.device());
@@ -33,7 +34,7 @@ static std::vector<Tensor> rmsnorm_fwd(const Tensor& x, const Tensor& w, double 
   return {y, rstd};
 }
 
-static std::vector<Tensor> rmsnorm_bwd(const Tensor& g, const Tensor& x, const Tensor& w, const Tensor& rstd) {
+std::vector<Tensor> rmsnorm_bwd(const Tensor& g, const Tensor& x, const Tensor& w, const Tensor& rstd) {
   CHECK_IN(g); CHECK_IN(x); CHECK_IN(w); CHECK_IN(rstd);
   c10::cuda::CUDAGuard guard(x.device());
   const int rows = (int)x.size(0), H = (int)x.size(1);
@@ -47,7 +48,7 @@ static std::vector<Tensor> rmsnorm_bwd(const Tensor& g, const Tensor& x, const T
   return {dx, dw};
 }
 
-static std::vector<Tensor> add_rmsnorm_fwd(const Tensor& x, const Tensor& r, const Tensor& w, double eps) {
+std::vector<Tensor> add_rmsnorm_fwd(const Tensor& x, const Tensor& r, const Tensor& w, double eps) {
   CHECK_IN(x); CHECK_IN(r); CHECK_IN(w);
   TORCH_CHECK(x.dim() == 2 && r.sizes() == x.sizes() && w.numel() == x.size(1) && w.scalar_type() == x.scalar_type() &&
               r.scalar_type() == x.scalar_type());
@@ -61,7 +62,7 @@ static std::vector<Tensor> add_rmsnorm_fwd(const Tensor& x, const Tensor& r, con
   return {y, h, rstd};
 }
 
-static std::vector<Tensor> add_rmsnorm_bwd(const Tensor& gy, const Tensor& gh, const Tensor& h, const Tensor& w, const Tensor& rstd) {
+std::vector<Tensor> add_rmsnorm_bwd(const Tensor& gy, const Tensor& gh, const Tensor& h, const Tensor& w, const Tensor& rstd) {
   CHECK_IN(gy); CHECK_IN(gh); CHECK_IN(h); CHECK_IN(w); CHECK_IN(rstd);
   c10::cuda::CUDAGuard guard(h.device());
   const int rows = (int)h.size(0), H = (int)h.size(1);
@@ -75,7 +76,7 @@ static std::vector<Tensor> add_rmsnorm_bwd(const Tensor& gy, const Tensor& gh, c
   return {dh, dw};
 }
 
-static Tensor swiglu_fwd(const Tensor& gu) {
+Tensor swiglu_fwd(const Tensor& gu) {
   CHECK_IN(gu);
   c10::cuda::CUDAGuard g(gu.device());
   const int I = (int)gu.size(1) / 2;
@@ -83,7 +84,7 @@ static Tensor swiglu_fwd(const Tensor& gu) {
   if (gu.numel()) nxd::swiglu_fwd(gu.data_ptr(), out.data_ptr(), gu.size(0), I, dt_code(gu), stream());
   return out;
 }
-static Tensor swiglu_bwd(const Tensor& go, const Tensor& gu) {
+Tensor swiglu_bwd(const Tensor& go, const Tensor& gu) {
   CHECK_IN(go); CHECK_IN(gu);
   c10::cuda::CUDAGuard g(gu.device());
   auto d = at::empty_like(gu);
@@ -107,7 +108,7 @@ static Tensor rope_apply(const Tensor& x, const Tensor& cos_t, const Tensor& sin
 }
 
 // fused [S, B, (H + 2 K) D] → rotated q [B, S, H, D], k [B, S, K, D]
-static std::vector<Tensor> rope_qkv_fwd(const Tensor& x, const Tensor& cos_t, const Tensor& sin_t, int64_t H, int64_t K) {
+std::vector<Tensor> rope_qkv_fwd(const Tensor& x, const Tensor& cos_t, const Tensor& sin_t, int64_t H, int64_t K) {
   CHECK_IN(x); CHECK_IN(cos_t); CHECK_IN(sin_t);
   TORCH_CHECK(x.dim() == 3 && x.size(2) % (H + 2 * K) == 0 && (uintptr_t)x.data_ptr() % 16 == 0);
   const int64_t D = x.size(2) / (H + 2 * K);
@@ -120,7 +121,7 @@ static std::vector<Tensor> rope_qkv_fwd(const Tensor& x, const Tensor& cos_t, co
   return {q, k};
 }
 // gradients [B, S, h, D] (any batch / position / head strides that keep 16-byte packets) → fused [S, B, (H + 2 K) D]
-static Tensor rope_qkv_bwd(const Tensor& gq, const Tensor& gk, const Tensor& gv, const Tensor& cos_t, const Tensor& sin_t) {
+Tensor rope_qkv_bwd(const Tensor& gq, const Tensor& gk, const Tensor& gv, const Tensor& cos_t, const Tensor& sin_t) {
   CHECK_IN(cos_t); CHECK_IN(sin_t);
   const int64_t B = gq.size(0), S = gq.size(1), H = gq.size(2), D = gq.size(3), K = gk.size(2);
   long strides[3][3];
@@ -153,7 +154,7 @@ static Tensor ce_stats(const Tensor& logits, const Tensor& target, int64_t vocab
   return stats;
 }
 // loss and log-normaliser of rows that hold the whole vocabulary
-static std::vector<Tensor> ce_loss(const Tensor& logits, const Tensor& target) {
+std::vector<Tensor> ce_loss(const Tensor& logits, const Tensor& target) {
   CHECK_IN(logits); CHECK_IN(target);
   TORCH_CHECK(target.scalar_type() == at::kLong && logits.dim() == 2 && target.numel() == logits.size(0));
   c10::cuda::CUDAGuard g(logits.device());
@@ -163,7 +164,7 @@ static std::vector<Tensor> ce_loss(const Tensor& logits, const Tensor& target) {
                  (int)logits.size(0), (int)logits.size(1), dt_code(logits), stream());
   return {loss, lse};
 }
-static Tensor ce_backward(const Tensor& logits, const Tensor& target, const Tensor& lse, const Tensor& gout,
+Tensor ce_backward(const Tensor& logits, const Tensor& target, const Tensor& lse, const Tensor& gout,
                           int64_t vocab_start, double smoothing, int64_t vocab) {
   CHECK_IN(logits); CHECK_IN(target); CHECK_IN(lse); CHECK_IN(gout);
   c10::cuda::CUDAGuard g(logits.device());
@@ -512,7 +513,7 @@ static Tensor gemv_mx_grouped(const Tensor& x, const Tensor& w, const Tensor& sc
   nxd::gemv_mx_grouped(x.data_ptr(), w.data_ptr(), scale.data_ptr(), expert.data_ptr<long>(), y.data_ptr(), S, N, K, E, (int)fmt, stream());
   return y;
 }
-static Tensor gemv(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& residual) {
+Tensor gemv(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& residual) {
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 && x.dim() == 2 && w.dim() == 2);
   TORCH_CHECK(x.is_contiguous() && w.is_contiguous() && x.size(1) == w.size(1) && x.size(0) >= 1 && x.size(0) <= 8 && x.size(1) % 8 == 0);
   c10::cuda::CUDAGuard guard(x.device());
@@ -567,7 +568,7 @@ static void check_qkv(const Tensor& t, const char* name) {
               name, ": expected a bf16 CUDA [B,S,H,128] view with contiguous head_dim");
 }
 // returns (out [B,S,H,D] view — memory laid out [S,B,H,D] when sbhd_out —, lse [B,H,S] fp32)
-static std::vector<Tensor> flash_attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, bool causal, double scale,
+std::vector<Tensor> flash_attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, bool causal, double scale,
                                           bool sbhd_out) {
   check_qkv(q, "q"); check_qkv(k, "k"); check_qkv(v, "v");
   const int B = q.size(0), S = q.size(1), H = q.size(2), Skv = k.size(1), Hkv = k.size(2);
@@ -582,7 +583,7 @@ static std::vector<Tensor> flash_attn_fwd(const Tensor& q, const Tensor& k, cons
   return {out, lse};
 }
 
-static std::vector<Tensor> flash_attn_bwd(const Tensor& go, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o,
+std::vector<Tensor> flash_attn_bwd(const Tensor& go, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o,
                                           const Tensor& lse, bool causal, double scale, bool sbhd_out,
                                           const c10::optional<Tensor>& dlse, int64_t parts) {
   check_qkv(q, "q"); check_qkv(k, "k"); check_qkv(v, "v"); check_qkv(go, "grad_out"); check_qkv(o, "out");
@@ -615,7 +616,7 @@ static std::vector<Tensor> flash_attn_bwd(const Tensor& go, const Tensor& q, con
 }
 
 // ---- GEMM ---------------------------------------------------------------------------------------
-static void gemm_bf16(const Tensor& a, const Tensor& b, Tensor out, bool trans_a, bool trans_b, bool accumulate) {
+void gemm_bf16(const Tensor& a, const Tensor& b, Tensor out, bool trans_a, bool trans_b, bool accumulate) {
   CHECK_IN(a); CHECK_IN(b); CHECK_IN(out);
   TORCH_CHECK(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16 && a.dim() == 2 && b.dim() == 2);
   const int M = (int)(trans_a ? a.size(1) : a.size(0)), K = (int)(trans_a ? a.size(0) : a.size(1));
@@ -628,7 +629,7 @@ static void gemm_bf16(const Tensor& a, const Tensor& b, Tensor out, bool trans_a
 }
 
 // y [M, N] = x [M, K] · w [N, K]ᵀ for 1 <= M <= 256 rows; split: blocks per 128 rows of w (0 = by rule)
-static Tensor gemm_few_rows(const Tensor& x, const Tensor& w, int64_t split) {
+Tensor gemm_few_rows(const Tensor& x, const Tensor& w, int64_t split) {
   CHECK_IN(x); CHECK_IN(w);
   TORCH_CHECK(x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 && x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1));
   TORCH_CHECK(split == 0 || split == 1 || split == 2 || split == 4 || split == 8);
@@ -638,7 +639,7 @@ static Tensor gemm_few_rows(const Tensor& x, const Tensor& w, int64_t split) {
   return y;
 }
 
-static void gemm_bf16_2cta(const Tensor& a, const Tensor& b, Tensor out, bool trans_a, bool trans_b, bool accumulate) {
+void gemm_bf16_2cta(const Tensor& a, const Tensor& b, Tensor out, bool trans_a, bool trans_b, bool accumulate) {
   CHECK_IN(a); CHECK_IN(b); CHECK_IN(out);
   TORCH_CHECK(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16 && a.dim() == 2 && b.dim() == 2);
   const int M = (int)(trans_a ? a.size(1) : a.size(0)), K = (int)(trans_a ? a.size(0) : a.size(1));
@@ -901,6 +902,7 @@ static Tensor nvls_reduce_scatter(const Tensor& x, const Tensor& peer_bases, int
 }
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  bind_native_autograd(m);
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
   m.def("rmsnorm_bwd", &rmsnorm_bwd);
   m.def("add_rmsnorm_fwd", &add_rmsnorm_fwd);

@@ -16,6 +16,7 @@ from pathlib import Path
 from typing import Optional
 
 import torch
+from torch.autograd import forward_ad
 
 PKG_DIR = Path(__file__).resolve().parent.parent
 BUILD_DIR = PKG_DIR / "_build"
@@ -102,6 +103,23 @@ def use_cuda(*tensors: torch.Tensor) -> bool:
     )
 
 
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+
+
+def native(*tensors: torch.Tensor):
+    """The autograd nodes of ``csrc/native_autograd.cpp`` where they may stand in for the Functions in Python: plain CUDA tensors, calls
+    that nobody records or traces, no functorch transform, no forward-mode AD; else ``None``."""
+    if _PLAN_PROXY is not None:
+        return None
+    for t in tensors:
+        if type(t) not in _PLAIN or not t.is_cuda:
+            return None
+    if (_load() is None or env("NXD_FORCE_EAGER") == "1" or torch._C._are_functorch_transforms_active()
+            or torch._C._get_tracing_state() is not None or forward_ad._current_level >= 0):
+        return None
+    return _C.native
+
+
 # launch accounting — bench.py reports how many of OUR kernels ran in the timed region
 _LAUNCHES = 0
 
@@ -112,9 +130,9 @@ def count_launch(n: int = 1) -> None:
 
 
 def launches() -> int:
-    return _LAUNCHES
+    return _LAUNCHES + (_C.native.launches() if _C is not None else 0)
 
 
 def reset_launches() -> None:
     global _LAUNCHES
-    _LAUNCHES = 0
+    _LAUNCHES = -(_C.native.launches() if _C is not None else 0)

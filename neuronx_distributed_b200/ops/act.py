@@ -46,6 +46,9 @@ class _SwiGLU(torch.autograd.Function):
 
 def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     """``gate_up[..., :I]`` is gate, ``gate_up[..., I:]`` is up."""
+    n = _ext.native(gate_up)
+    if n is not None and gate_up.shape[-1] % 16 == 0 and gate_up.dtype in (torch.bfloat16, torch.float32, torch.float16):
+        return n.swiglu(gate_up)
     return _SwiGLU.apply(gate_up)
 
 

@@ -120,6 +120,9 @@ def flash_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: b
                     scale: Optional[float] = None) -> torch.Tensor:
     scale = scale if scale is not None else 1.0 / math.sqrt(q.shape[-1])
     if _own_kernel_ok(q, k, v) and (not causal or q.shape[1] == k.shape[1]):
+        n = _ext.native(q, k, v)
+        if n is not None:
+            return n.flash_attention(q, k, v, bool(causal), float(scale))
         return _FlashAttn.apply(q, k, v, causal, scale)
     return _sdpa(q, k, v, causal, scale)
 

@@ -10,6 +10,9 @@ import torch
 from . import _ext
 
 
+_KERNEL_DTYPES = (torch.bfloat16, torch.float32, torch.float16)
+
+
 def _rms_ref(x, w, eps):
     xf = x.float()
     rstd = torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + eps)
@@ -49,6 +52,9 @@ class _RMSNorm(torch.autograd.Function):
 
 
 def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6) -> torch.Tensor:
+    n = _ext.native(x, weight)
+    if n is not None and x.dtype in _KERNEL_DTYPES:
+        return n.rms_norm(x, weight, eps)
     return _RMSNorm.apply(x, weight, eps)
 
 
@@ -91,4 +97,7 @@ class _AddRMSNorm(torch.autograd.Function):
 
 def add_rms_norm(x: torch.Tensor, residual: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6):
     """Returns ``(rmsnorm(x + residual) * weight, x + residual)``."""
+    n = _ext.native(x, residual, weight)
+    if n is not None and x.dtype in _KERNEL_DTYPES and residual.dtype == x.dtype:
+        return n.add_rms_norm(x, residual, weight, eps)
     return _AddRMSNorm.apply(x, residual, weight, eps)

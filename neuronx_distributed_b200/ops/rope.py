@@ -95,6 +95,9 @@ def fused_qkv(q, k, v, cos, sin, heads: int, kv_heads: int, head_dim: int):
 def rotary_qkv(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, heads: int, kv_heads: int):
     """``qkv [S, B, (heads + 2 kv_heads) D]`` → rotated ``q [B, S, heads, D]``, ``k`` and the view ``v [B, S, kv_heads, D]``:
     :func:`apply_rotary` of the first two sections, each direction one launch (``csrc/elementwise.cu`` rope_qkv)."""
+    n = _ext.native(qkv, cos, sin)
+    if n is not None:
+        return n.rope_qkv(qkv, cos, sin, heads, kv_heads)
     return _RopeQKV.apply(qkv, cos, sin, heads, kv_heads)
 
 

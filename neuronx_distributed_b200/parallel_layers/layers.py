@@ -588,6 +588,24 @@ class _TPLinear(torch.autograd.Function):
         return gx, gw, gbias, None, None, None, None, None, None, None
 
 
+_NATIVE_WGRAD = None
+
+
+def _native_linear(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Tensor]:
+    """``x @ Wᵀ`` of one rank as a node without Python in it, or None where the kernels do not take its products as they are."""
+    from .. import ops
+
+    global _NATIVE_WGRAD
+    n = ops._ext.native(x, weight)
+    if n is None or not ops.gemm._USE_2CTA or ops._ext.env("NXD_DISABLE_TCGEN05_GEMM") == "1":
+        return None
+    if _NATIVE_WGRAD is not n:
+        n.set_weight_gradient(lambda *a: wgrad(*a), lambda: ops.gemm.fused_wgrad_enabled())
+        _NATIVE_WGRAD = n
+    N, K = weight.shape if weight.dim() == 2 else (0, 0)
+    return n.linear(x, weight, K > 0 and ops.gemm._few_rows(x.numel() // K, N, K))
+
+
 def tp_linear(
     x: torch.Tensor,
     weight: torch.Tensor,
@@ -605,7 +623,12 @@ def tp_linear(
     input-gradient GEMM only (weight gradient sees them unscaled) — the GQA KV-replication correction."""
     assert dgrad_col_scale is None or out_mode == "none"
     group = group if group is not None else ps.get_tensor_model_parallel_group()
-    if autocast or torch.is_autocast_enabled():
+    cast = autocast or torch.is_autocast_enabled()
+    if not cast and bias is None and dgrad_col_scale is None and save_for_backward and _group_size(group) == 1:
+        y = _native_linear(x, weight)
+        if y is not None:
+            return y
+    if cast:
         dt = torch.get_autocast_dtype("cuda" if x.is_cuda else "cpu") if torch.is_autocast_enabled() else x.dtype
         x = x.to(dt)
         weight = weight.to(dt)

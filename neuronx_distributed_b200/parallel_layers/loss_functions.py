@@ -88,6 +88,14 @@ class _ParallelCrossEntropy(torch.autograd.Function):
 
 def parallel_cross_entropy(vocab_parallel_logits, target, label_smoothing: float = 0.0, process_group=None):
     """Per-token cross-entropy for logits sharded along the vocab (last) dim across TP."""
+    from ..ops import _ext
+
+    if not label_smoothing > 0 and isinstance(vocab_parallel_logits, torch.Tensor) and vocab_parallel_logits.is_cuda:
+        n = _ext.native(vocab_parallel_logits, target)
+        if n is not None and vocab_parallel_logits.dtype in (torch.bfloat16, torch.float32, torch.float16):
+            group = process_group if process_group is not None else ps.get_tensor_model_parallel_group()
+            if dist.get_world_size(group) == 1:
+                return n.cross_entropy(vocab_parallel_logits, target)
     return _ParallelCrossEntropy.apply(vocab_parallel_logits, target, label_smoothing, process_group)
 
 

@@ -9,6 +9,17 @@ import torch
 from torch import nn
 
 
+def _set_training(module: nn.Module) -> None:
+    """``module.train()``, without its walk that sets every flag again (3 us a module) where all are set already."""
+    stack = [module]
+    while stack:
+        m = stack.pop()
+        if not m.training or type(m).train is not nn.Module.train or "train" in m.__dict__:
+            module.train()
+            return
+        stack.extend(c for c in m._modules.values() if c is not None)
+
+
 class NxDModel(nn.Module):
     def __init__(self, module: nn.Module, nxd_config: dict):
         super().__init__()
@@ -30,7 +41,7 @@ class NxDModel(nn.Module):
     def run_train(self, *args, **kwargs):
         if self.pp_enabled:
             return self.module.run_train(*args, **kwargs)
-        self.module.train()
+        _set_training(self.module)
         out = self.module(*args, **kwargs)
         loss = out[0] if isinstance(out, (tuple, list)) else (out.loss if hasattr(out, "loss") else out)
         loss.backward()
