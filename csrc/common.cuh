@@ -43,20 +43,22 @@ namespace nxd {
 
 // Programmatic dependent launch: a kernel that was launched with launch_dependent starts while the one before it in the stream still
 // runs, and must pass pdl_wait before it touches anything that kernel wrote; pdl_trigger in the earlier one lets it start.
+// Every kernel launched so waits before it reads or writes anything of others and before it returns, so that its end is its predecessors' end
+// too.  Pointers to what a predecessor wrote are not __restrict__ there: a load through the read-only path must not move above the wait.
 NXD_DEVICE void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 NXD_DEVICE void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// memory that is read later to L2 (address and size multiples of 16): no read as far as order goes, so it may stand above pdl_wait
+NXD_DEVICE void prefetch_l2(const void* p, uint32_t bytes) { asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory"); }
+
 template <typename... KArgs, typename... Args>
 inline void launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
-  // a captured launch is an ordinary one: gaps inside a graph are short, and its instantiation took 30 ms longer with such edges
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  NXD_CUDA_CHECK(cudaStreamIsCapturing(st, &capture));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr; cfg.numAttrs = capture == cudaStreamCaptureStatusNone ? 1 : 0;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
   NXD_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...));
 }
 

@@ -47,15 +47,16 @@ NXD_DEVICE void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a2, uint32_t b0, u
 // 8 rows in flight per block it was 148 us.
 template <int G>
 __global__ void __launch_bounds__(kDecThreads, 2) decode_attn_kernel(
-    const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kc, const __nv_bfloat16* __restrict__ vc,
-    const long* __restrict__ positions, float* __restrict__ part_o, float* __restrict__ part_ml,
-    __nv_bfloat16* __restrict__ out, int B, int H, int Hkv, int L,
+    const __nv_bfloat16* q, const __nv_bfloat16* kc, const __nv_bfloat16* vc,
+    const long* positions, float* part_o, float* part_ml,
+    __nv_bfloat16* out, int B, int H, int Hkv, int L,
     long k_sb, long k_ss, long k_sh, long v_sb, long v_ss, long v_sh, long q_sb, long q_sh, long o_sb, long o_sh,
     float scale_log2, int splits) {
   extern __shared__ __align__(128) uint8_t dec_smem[];
   const int kvh = blockIdx.x, b = blockIdx.y, split = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   pdl_trigger();                                           // the merge's blocks may take their places; they wait for this grid
+  pdl_wait();
   const long pos = positions[b];
   const int n_valid = (int)(pos < 0 ? 0 : (pos >= L ? L : pos + 1));
   const int per = (n_valid + splits - 1) / splits;
@@ -204,10 +205,11 @@ __global__ void __launch_bounds__(kDecThreads, 2) decode_attn_kernel(
   }
 }
 
-__global__ void __launch_bounds__(HD) decode_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                                            __nv_bfloat16* __restrict__ out, int splits, long o_sb, long o_sh,
+__global__ void __launch_bounds__(HD) decode_combine_kernel(const float* part_o, const float* part_ml,
+                                                            __nv_bfloat16* out, int splits, long o_sb, long o_sh,
                                                             int H) {
   const int bh = blockIdx.x, d = threadIdx.x;
+  pdl_trigger();
   pdl_wait();
   float mn = -INFINITY;
   for (int s = 0; s < splits; ++s) mn = fmaxf(mn, part_ml[((long)bh * splits + s) * 2]);
@@ -225,8 +227,8 @@ __global__ void __launch_bounds__(HD) decode_combine_kernel(const float* __restr
 // Same merge over the splits, but the result stays un-normalised: o (relative to the row maximum), the maximum (natural-log
 // units) and the row sum — what a rank contributes to distributed flash-decoding, where the final normalisation happens after
 // the cross-rank log-sum-exp merge (modules/attention/flash_decode.py).
-__global__ void __launch_bounds__(HD) decode_combine_partial_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                                                    float* __restrict__ fin_o, float* __restrict__ fin_ml, int splits) {
+__global__ void __launch_bounds__(HD) decode_combine_partial_kernel(const float* part_o, const float* part_ml,
+                                                                    float* fin_o, float* fin_ml, int splits) {
   const int bh = blockIdx.x, d = threadIdx.x;
   pdl_wait();
   float mn = -INFINITY;
@@ -242,13 +244,18 @@ __global__ void __launch_bounds__(HD) decode_combine_partial_kernel(const float*
   if (d == 0) { fin_ml[bh * 2] = mn * 0.6931471805599453f; fin_ml[bh * 2 + 1] = ls; }
 }
 
+// While the kernel before it still runs (a norm, a rotation, the merge of an attention), the first bytes of its weights come to L2:
+// 13B, one token, us: 324 with ordinary launches, 310.5 with dependent ones, 307.4 / 309.5 / 333 with 2 / 4 / 10 KB of a row ahead.
+constexpr int kGemvAhead = 2048;
+
 // y[m, n] = Σ_k x[m, k] · W[n, k]; one warp per output column n (8 columns per 256-thread CTA), M ≤ 8 rows of x kept hot in L1.
 template <int M>
-__global__ void __launch_bounds__(256) gemv_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-                                                   const __nv_bfloat16* __restrict__ residual, __nv_bfloat16* __restrict__ y,
+__global__ void __launch_bounds__(256) gemv_kernel(const __nv_bfloat16* x, const __nv_bfloat16* w, const __nv_bfloat16* residual, __nv_bfloat16* y,
                                                    int N, int K) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = blockIdx.x * 8 + warp;
+  if (lane == 0 && n < N) prefetch_l2(w + (long)n * K, (uint32_t)min(K * 2, kGemvAhead));
+  pdl_wait();
   if (n >= N) return;
   float acc[M];
 #pragma unroll
@@ -256,7 +263,7 @@ __global__ void __launch_bounds__(256) gemv_kernel(const __nv_bfloat16* __restri
   const __nv_bfloat16* wr = w + (long)n * K;
 #pragma unroll 4
   for (int k = lane * 8; k < K; k += 256) {
-    const uint4 wv = __ldg(reinterpret_cast<const uint4*>(wr + k));       // weights stream through once
+    const uint4 wv = *reinterpret_cast<const uint4*>(wr + k);       // weights stream through once
     const __nv_bfloat162* w2 = reinterpret_cast<const __nv_bfloat162*>(&wv);
     float wf[8];
 #pragma unroll
@@ -273,6 +280,7 @@ __global__ void __launch_bounds__(256) gemv_kernel(const __nv_bfloat16* __restri
       }
     }
   }
+  pdl_trigger();       // not before: blocks that start beside this kernel's fill the SMs unevenly and stay there (8192 wide: 179 us -> 232 a token)
 #pragma unroll
   for (int m = 0; m < M; ++m) {
     const float v = warp_sum(acc[m]);
@@ -287,15 +295,17 @@ __global__ void __launch_bounds__(256) gemv_kernel(const __nv_bfloat16* __restri
 // Decode-time RoPE + KV-cache append in ONE launch (was ~25 tiny elementwise / index_put kernels per layer in the token-
 // generation graph): q [B,H,D] rotated into q_out, k rotated and v copied into the cache row positions[b].  One warp per head
 // row; cos/sin rows gathered by position.  HF rotate-half convention (csrc/elementwise.cu rope_kernel).
-__global__ void __launch_bounds__(128) decode_rope_kv_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
-                                                            const __nv_bfloat16* __restrict__ v, const long* __restrict__ positions,
-                                                            const float* __restrict__ cos_t, const float* __restrict__ sin_t,
-                                                            __nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ kc,
-                                                            __nv_bfloat16* __restrict__ vc, int B, int H, int Hkv, int D, int L,
+__global__ void __launch_bounds__(128) decode_rope_kv_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k,
+                                                            const __nv_bfloat16* v, const long* positions,
+                                                            const float* cos_t, const float* sin_t,
+                                                            __nv_bfloat16* q_out, __nv_bfloat16* kc,
+                                                            __nv_bfloat16* vc, int B, int H, int Hkv, int D, int L,
                                                             long q_sb, long q_sh, long k_sb, long k_sh, long v_sb, long v_sh,
                                                             long c_sb, long c_ss, long c_sh) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int rows = B * (H + 2 * Hkv);
+  pdl_trigger();
+  pdl_wait();
   if (warp >= rows) return;
   const int b = warp / (H + 2 * Hkv), r = warp % (H + 2 * Hkv);
   long pos = positions[b];
@@ -329,10 +339,9 @@ void decode_rope_kv(const void* q, const void* k, const void* v, const long* pos
                     long v_sb, long v_sh, long c_sb, long c_ss, long c_sh, cudaStream_t st) {
   const int rows = B * (H + 2 * Hkv);
   const int grid = (rows * 32 + 127) / 128;
-  decode_rope_kv_kernel<<<grid, 128, 0, st>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, positions,
-                                              cos_t, sin_t, (__nv_bfloat16*)q_out, (__nv_bfloat16*)kc, (__nv_bfloat16*)vc, B, H, Hkv, D, L,
-                                              q_sb, q_sh, k_sb, k_sh, v_sb, v_sh, c_sb, c_ss, c_sh);
-  NXD_CUDA_CHECK(cudaGetLastError());
+  launch_dependent(decode_rope_kv_kernel, grid, 128, 0, st, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, positions,
+                   cos_t, sin_t, (__nv_bfloat16*)q_out, (__nv_bfloat16*)kc, (__nv_bfloat16*)vc, B, H, Hkv, D, L,
+                   q_sb, q_sh, k_sb, k_sh, v_sb, v_sh, c_sb, c_ss, c_sh);
 }
 
 // Stretches per (sequence, key/value head): about six blocks per SM in all, so that sequences of unequal length fill the GPU to
@@ -354,7 +363,7 @@ void decode_attention(const void* q, const void* k, const void* v, const long* p
 #define NXD_DEC(Gv)                                                                                                  \
   do {                                                                                                               \
     NXD_ALLOW_SMEM(decode_attn_kernel<Gv>, kDecSmem);                                                                  \
-    decode_attn_kernel<Gv><<<grid, kDecThreads, kDecSmem, st>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)k,      \
+    launch_dependent(decode_attn_kernel<Gv>, grid, kDecThreads, kDecSmem, st, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k,      \
         (const __nv_bfloat16*)v, positions, part_o, part_ml, whole ? (__nv_bfloat16*)out : nullptr, B, H, Hkv, L,      \
         ks[0], ks[1], ks[2], vs[0], vs[1], vs[2], q_sb, q_sh, o_sb, o_sh, sl2, splits);                                \
   } while (0)
@@ -383,8 +392,8 @@ void gemv_bf16(const void* x, const void* w, const void* residual, void* y, int 
     return gemm_few_rows(x, w, residual, y, M, N, K, 0, st);
   const int grid = (N + 7) / 8;
 #define NXD_GEMV(Mv)                                                                                                \
-  gemv_kernel<Mv><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const __nv_bfloat16*)residual, \
-                                        (__nv_bfloat16*)y, N, K)
+  launch_dependent(gemv_kernel<Mv>, grid, 256, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const __nv_bfloat16*)residual, \
+                   (__nv_bfloat16*)y, N, K)
   switch (M) {
     case 1: NXD_GEMV(1); break;
     case 2: NXD_GEMV(2); break;

@@ -15,12 +15,14 @@ namespace nxd {
 // RMSNorm forward: one CTA per row, row cached in registers (up to MAXV 16-byte packets/thread)
 // =====================================================================================
 template <typename T, int MAXV>
-__global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w,
-                                                          T* __restrict__ y, float* __restrict__ rstd_out, int H,
+__global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const T* x, const T* w,
+                                                          T* y, float* __restrict__ rstd_out, int H,
                                                           float eps) {
   using P = Pack16<T>;
   constexpr int N = P::N;
   __shared__ float red[32];
+  pdl_trigger();
+  pdl_wait();
   const int row = blockIdx.x;
   const T* xr = x + (size_t)row * H;
   T* yr = y + (size_t)row * H;
@@ -49,14 +51,14 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const T* __restrict__ 
   for (int i = 0; i < MAXV; ++i) {
     const int v = threadIdx.x + i * blockDim.x;
     if (v < nvec) {
-      P pw, po; pw.load_nc(w + v * N);
+      P pw, po; pw.load(w + v * N);
 #pragma unroll
       for (int j = 0; j < N; ++j) po.set(j, cache[i].f(j) * rstd * pw.f(j));
       po.store(yr + v * N);
     }
   }
   for (int v = threadIdx.x + MAXV * blockDim.x; v < nvec; v += blockDim.x) {
-    P p, pw, po; p.load(xr + v * N); pw.load_nc(w + v * N);
+    P p, pw, po; p.load(xr + v * N); pw.load(w + v * N);
 #pragma unroll
     for (int j = 0; j < N; ++j) po.set(j, p.f(j) * rstd * pw.f(j));
     po.store(yr + v * N);
@@ -67,9 +69,11 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const T* __restrict__ 
 // SwiGLU: out[t, i] = silu(gu[t, i]) * gu[t, I + i]
 // =====================================================================================
 template <typename T>
-__global__ void __launch_bounds__(256) swiglu_fwd_kernel(const T* __restrict__ gu, T* __restrict__ out, size_t rows, int I) {
+__global__ void __launch_bounds__(256) swiglu_fwd_kernel(const T* gu, T* out, size_t rows, int I) {
   using P = Pack16<T>;
   constexpr int N = P::N;
+  pdl_trigger();
+  pdl_wait();
   const int vec_per_row = I / N;
   const size_t total = rows * (size_t)vec_per_row;
   for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x) {
@@ -416,7 +420,7 @@ void rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int rows, i
   DISPATCH_DTYPE(dt, {
     if (H % Pack16<T>::N) nxd_throw("rmsnorm: H must be a multiple of the 16-byte vector width", __FILE__, __LINE__);
     const int th = pick_threads<T>(H);
-    rmsnorm_fwd_kernel<T, 4><<<rows, th, 0, st>>>((const T*)x, (const T*)w, (T*)y, rstd, H, eps);
+    launch_dependent(rmsnorm_fwd_kernel<T, 4>, rows, th, 0, st, (const T*)x, (const T*)w, (T*)y, rstd, H, eps);
   });
   NXD_CUDA_CHECK(cudaGetLastError());
 }
@@ -425,7 +429,7 @@ void swiglu_fwd(const void* gu, void* out, long rows, int I, int dt, cudaStream_
   DISPATCH_DTYPE(dt, {
     const size_t total = (size_t)rows * (I / Pack16<T>::N);
     const int grid = (int)min((size_t)num_sms() * 16, (total + 255) / 256);
-    swiglu_fwd_kernel<T><<<max(grid, 1), 256, 0, st>>>((const T*)gu, (T*)out, (size_t)rows, I);
+    launch_dependent(swiglu_fwd_kernel<T>, max(grid, 1), 256, 0, st, (const T*)gu, (T*)out, (size_t)rows, I);
   });
   NXD_CUDA_CHECK(cudaGetLastError());
 }

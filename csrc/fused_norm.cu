@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(MAXT, MAXT == 1024 ? 1 : VPT == 1 ? 3 : 2) nor
 // Sum of the blocks' parts of dW, written in the weight's type: 32 columns per block, 32 parts in flight at a time (one thread per
 // column that walked all parts took 27 us for 592 parts of 4096 columns).
 template <typename T>
-static __global__ void __launch_bounds__(256) norm_bwd_reduce_kernel(const float* __restrict__ partial, T* __restrict__ out, int nparts, int H) {
+static __global__ void __launch_bounds__(256) norm_bwd_reduce_kernel(const float* partial, T* out, int nparts, int H) {
   __shared__ float4 part[32][8];
   pdl_wait();
   const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3, c = blockIdx.x * 32 + tx * 4;
