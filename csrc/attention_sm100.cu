@@ -500,7 +500,6 @@ struct BwdParams {
   const float* stats;          // [2][B*H*S_pad (+pad)] : −lse·log2e , −δ·scale
   long stats_stride;
   float* dq_acc;               // [B, H, S_pad, 128] fp32
-  int debug;                   // NXD_FA_DEBUG bits (perf triage only): 1 no bulk reduce, 2 no dQ staging, 4 no softmax math
   unsigned* turnstile;         // DET only: [B, H, ceil(S_q / BQ)] contributions already added to each dQ tile
 };
 
@@ -601,6 +600,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
   const uint32_t bar_kv = bars, bar_qf = bars + 8, bar_qe = bars + 32, bar_s = bars + 56, bar_dp = bars + 72,
                  bar_p = bars + 80, bar_dq = bars + 88, bar_dqr = bars + 96, bar_acc = bars + 104, tmem_slot = bars + 128;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_trigger();                                           // fa_bwd_dq_out_kernel's blocks wait on the SMs that run out of this kernel's
   // Blocks start heaviest first (causal: the first K/V tiles see the most query tiles) within groups of heads that share L2: head by
   // head, the last heads' heavy tiles started when most SMs had nothing left (1 x 2048 x 32 heads: 142 us, now 119).
   int n, kvh, b, vh;                                       // vh: the part's index among all parts of all KV heads
@@ -652,6 +652,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
       tma_load_2d(sK + kHalf, &tk, bar_kv, kc + 64, kr);
       tma_load_2d(sV, &tv, bar_kv, vc, vr);
       tma_load_2d(sV + kHalf, &tv, bar_kv, vc + 64, vr);
+      pdl_wait();                                          // the statistics come from the kernel before; q, k, v and dO do not
       for (int it = 0; it < n_iter; ++it) {
         const int qs = it % kQStages;
         const uint32_t ph = (uint32_t)((it / kQStages) & 1);
@@ -772,10 +773,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
       tcgen05_ld_32x32(tmem_dP + lane_base, dpv[0]);
       tcgen05_ld_32x32(tmem_dP + lane_base + 32, dpv[1]);
       tcgen05_wait_ld();
-      if (!(p.debug & 4)) {
-        if (masked) bwd_ds_math<true>(dpv, pf, stats_s, sc);
-        else bwd_ds_math<false>(dpv, pf, stats_s, sc);
-      }
+      if (masked) bwd_ds_math<true>(dpv, pf, stats_s, sc);
+      else bwd_ds_math<false>(dpv, pf, stats_s, sc);
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         // dSᵀ row → smem, 128B-swizzled: 16-byte chunk c of row r lives at chunk (c ^ (r & 7))
@@ -836,6 +835,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
     const int d = quarter * 32 + lane;
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     const int tid = threadIdx.x - 192;
+    if (tid == 0) pdl_wait();                              // which zeroes what is added to here
     for (int it = 0; it < n_iter; ++it) {
       const int st = it & 1;
       const int head = vh * group + it / per_head, t = t0 + it % per_head;
@@ -848,7 +848,6 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
       tcgen05_wait_ld();
       tcgen05_fence_before();
       mbar_arrive(bar_dqr);                     // the MMA warp may overwrite dQᵀ with the next tile right away
-      if (p.debug & 2) continue;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         if (tid == 0) bulk_wait_read0();        // previous bulk reduce has finished reading the staging tile
@@ -858,7 +857,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
           asm volatile("st.shared.b32 [%0], %1;" ::"r"(sdQ + c * 512 + d * 4), "r"(r[h][c]) : "memory");
         fence_async_smem();
         named_bar(1, 128);
-        if (tid == 0 && !(p.debug & 1)) {
+        if (tid == 0) {
           if constexpr (DET) {
             if (h == 0) {                           // my turn: the n earlier K/V tiles of this column have been added
               const unsigned* turn = p.turnstile + ((long)b * p.H + head) * nq + t;
@@ -896,56 +895,49 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
 }
 
 // −δ·scale and −lse·log2e per (b, h, s), and zeros for the row's dQ accumulator (rows up to S_pad).  16 lanes per row, 16 bytes per
-// lane, four rows of a half warp in flight; heads fastest, as o and dO lie in memory.  1 x 2048 x 32 heads: 15 us; with 8-byte loads,
-// one row per warp and a memset of its own, 25.
+// lane; heads fastest, as o and dO lie in memory.  The main kernel's blocks take their places and load K and V beside this one, and the
+// conversion of dQ starts on the SMs that run out of it: whole backward, 1 x 2048 x 32 heads, 146 us with launches one after the other,
+// 140 so, 136 with one row per half warp instead of four in flight; 1 x 1000 x 32: 61 and 53; 1 x 70 x 32: 21.6 and 14.5.
 __global__ void __launch_bounds__(256) fa_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ go,
                                    const float* __restrict__ lse, const float* __restrict__ dlse, float* __restrict__ stats,
                                    float* __restrict__ dq_acc, long stats_stride, int B, int S,
                                    int H, int S_pad, long o_sb, long o_ss, long o_sh, long g_sb, long g_ss, long g_sh,
                                    float scale) {
-  constexpr int R = 4;
+  pdl_trigger();
   const int lane = threadIdx.x & 15, bh = B * H;
-  const long rows = (long)S_pad * bh, r0 = (long)blockIdx.x * (16 * R) + (threadIdx.x >> 4);
-  Pack16<__nv_bfloat16> ov[R], gv[R];
-  int s[R], h[R], b[R];
+  const long r = (long)blockIdx.x * 16 + (threadIdx.x >> 4);
+  const int s = r < (long)S_pad * bh ? (int)(r / bh) : S_pad, in = (int)(r % bh), h = in % H, b = in / H;
+  Pack16<__nv_bfloat16> ov, gv;
+  if (s < S) {
+    ov.load_nc(o + b * o_sb + s * o_ss + h * o_sh + lane * 8);
+    gv.load_nc(go + b * g_sb + s * g_ss + h * g_sh + lane * 8);
+  }
+  if (s < S_pad) {
+    float4* z = reinterpret_cast<float4*>(dq_acc + (((long)b * H + h) * S_pad + s) * HD) + lane;
+    z[0] = z[16] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  float acc = 0.f;
+  if (s < S) {
 #pragma unroll
-  for (int i = 0; i < R; ++i) {
-    const long r = r0 + 16 * i;
-    s[i] = r < rows ? (int)(r / bh) : S_pad;
-    const int in = (int)(r % bh);
-    h[i] = in % H; b[i] = in / H;
-    if (s[i] < S) {
-      ov[i].load_nc(o + b[i] * o_sb + s[i] * o_ss + h[i] * o_sh + lane * 8);
-      gv[i].load_nc(go + b[i] * g_sb + s[i] * g_ss + h[i] * g_sh + lane * 8);
-    }
+    for (int j = 0; j < 8; ++j) acc += ov.f(j) * gv.f(j);
   }
 #pragma unroll
-  for (int i = 0; i < R; ++i) {
-    if (s[i] < S_pad) {
-      float4* z = reinterpret_cast<float4*>(dq_acc + (((long)b[i] * H + h[i]) * S_pad + s[i]) * HD) + lane;
-      z[0] = z[16] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    float acc = 0.f;
-    if (s[i] < S) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc += ov[i].f(j) * gv[i].f(j);
-    }
-#pragma unroll
-    for (int m = 8; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
-    if (lane == 0 && s[i] < S) {
-      const long row = (long)b[i] * H + h[i], idx = row * S_pad + s[i];
-      stats[idx] = -lse[row * S + s[i]] * 1.4426950408889634f;
-      // a gradient flowing into LSE itself (ring attention merges blocks through their LSEs) adds g_lse·P to dS, i.e. it
-      // simply shifts δ: dS = P∘(dP − (δ − g_lse))
-      const float g_lse = dlse ? dlse[row * S + s[i]] : 0.f;
-      stats[stats_stride + idx] = -(acc - g_lse) * scale;
-    }
+  for (int m = 8; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
+  if (lane == 0 && s < S) {
+    const long row = (long)b * H + h, idx = row * S_pad + s;
+    stats[idx] = -lse[row * S + s] * 1.4426950408889634f;
+    // a gradient flowing into LSE itself (ring attention merges blocks through their LSEs) adds g_lse·P to dS, i.e. it
+    // simply shifts δ: dS = P∘(dP − (δ − g_lse))
+    const float g_lse = dlse ? dlse[row * S + s] : 0.f;
+    stats[stats_stride + idx] = -(acc - g_lse) * scale;
   }
 }
 
 // fp32 dQ accumulator [B,H,S_pad,128] → bf16 dq with arbitrary (b, s, h) strides; 8 elements per thread.
-__global__ void fa_bwd_dq_out_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, int B, int S, int H,
+__global__ void fa_bwd_dq_out_kernel(const float* acc, __nv_bfloat16* dq, int B, int S, int H,
                                      int S_pad, long sb, long ss, long sh) {
+  pdl_trigger();
+  pdl_wait();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;        // over B*H*S*16
   if (i >= (long)B * H * S * 16) return;
   const int c = (int)(i & 15);
@@ -959,8 +951,9 @@ __global__ void fa_bwd_dq_out_kernel(const float* __restrict__ acc, __nv_bfloat1
 }
 
 // dK and dV of a KV head out of the fp32 sums of its parts, added in their order; 8 elements per thread.
-__global__ void fa_bwd_kv_out_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, int B,
+__global__ void fa_bwd_kv_out_kernel(const float* part, __nv_bfloat16* dk, __nv_bfloat16* dv, int B,
                                      int S, int Hkv, int parts, long k_sb, long k_ss, long k_sh, long v_sb, long v_ss, long v_sh) {
+  pdl_wait();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x, n = (long)B * Hkv * S * 16;        // over 2 * B*Hkv*S*16
   if (i >= 2 * n) return;
   const bool is_v = i >= n;
@@ -1082,7 +1075,6 @@ void flash_attn_bwd(const void* go, const void* q, const void* k, const void* v,
   p.stats = stats; p.stats_stride = (long)B * H * S_pad + 64;
   p.dq_acc = dq_acc;
   p.parts = parts; p.kv_part = kv_part;
-  { const char* e = getenv("NXD_FA_DEBUG"); p.debug = e ? atoi(e) : 0; }
   // NXD_FA_DETERMINISTIC=1: ordered dQ accumulation (see fa_bwd_kernel<true>); the turnstile counters live in a per-device
   // buffer that only grows (debug mode: allocation is synchronous, not meant for graph capture)
   bool det = false;
@@ -1104,7 +1096,7 @@ void flash_attn_bwd(const void* go, const void* q, const void* k, const void* v,
   }
   {
     const long rows = (long)B * H * S_pad;
-    fa_bwd_prep_kernel<<<(unsigned)((rows + 63) / 64), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)go, lse, dlse, stats,
+    fa_bwd_prep_kernel<<<(unsigned)((rows + 15) / 16), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)go, lse, dlse, stats,
                                                                      dq_acc, p.stats_stride, B, S_q, H, S_pad, os[0], os[1], os[2], gs[0],
                                                                      gs[1], gs[2], scale);
   }
@@ -1117,19 +1109,19 @@ void flash_attn_bwd(const void* go, const void* q, const void* k, const void* v,
   const long head_bytes = (long)S_q * HD * 8 * (H / Hkv / parts); // Q, dO and fp32 dQ of one block's query heads
   p.group_bh = (int)std::min<long>((long)Hkv * parts * B, std::max<long>(1, (64l << 20) / std::max<long>(1, head_bytes)));
   const unsigned grid = (unsigned)((S_kv + BN - 1) / BN * (long)Hkv * parts * B);
-  if (det) fa_bwd_kernel<true><<<grid, kThreadsBwd, kSmemBwd, st>>>(tq, tk, tv, tg, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, p);
-  else fa_bwd_kernel<false><<<grid, kThreadsBwd, kSmemBwd, st>>>(tq, tk, tv, tg, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, p);
+  NXD_CUDA_CHECK(cudaGetLastError());
+  launch_dependent(det ? fa_bwd_kernel<true> : fa_bwd_kernel<false>, grid, kThreadsBwd, kSmemBwd, st, tq, tk, tv, tg, (__nv_bfloat16*)dk,
+                   (__nv_bfloat16*)dv, p);
   {
     const long n = (long)B * H * S_q * 16;
-    fa_bwd_dq_out_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dq, B, S_q, H, S_pad, dqs[0],
-                                                                     dqs[1], dqs[2]);
+    launch_dependent(fa_bwd_dq_out_kernel, (unsigned)((n + 255) / 256), 256, 0, st, (const float*)dq_acc, (__nv_bfloat16*)dq, B, S_q, H, S_pad, dqs[0],
+                     dqs[1], dqs[2]);
   }
   if (parts > 1) {
     const long n = 2l * B * Hkv * S_kv * 16;
-    fa_bwd_kv_out_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(kv_part, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, B, S_kv, Hkv, parts,
-                                                                     dks[0], dks[1], dks[2], dvs[0], dvs[1], dvs[2]);
+    launch_dependent(fa_bwd_kv_out_kernel, (unsigned)((n + 255) / 256), 256, 0, st, (const float*)kv_part, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, B,
+                     S_kv, Hkv, parts, dks[0], dks[1], dks[2], dvs[0], dvs[1], dvs[2]);
   }
-  NXD_CUDA_CHECK(cudaGetLastError());
 }
 
 }  // namespace nxd
