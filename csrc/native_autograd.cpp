@@ -165,7 +165,7 @@ PyObject* g_fused_wgrad_enabled = nullptr;                 // ops.gemm.fused_wgr
 
 void product(const Tensor& a, const Tensor& b, const Tensor& out, bool ta, bool tb, bool acc) {
   count();
-  if (out.size(0) >= 256) gemm_bf16_2cta(a, b, out, ta, tb, acc);
+  if (out.size(0) > 128 || out.size(1) <= 16384) gemm_bf16_2cta(a, b, out, ta, tb, acc);      // ops/gemm.py _pairs
   else gemm_bf16(a, b, out, ta, tb, acc);
 }
 

@@ -49,6 +49,13 @@ def _few_rows(M: int, N: int, K: int) -> bool:
     return K >= 2048 and (N <= 9472 or (M <= 176 and N <= 65536)) and M < 256
 
 
+def _pairs(M: int, N: int) -> bool:
+    """Products for the CTA-pair kernel; the other one, tiles of 128 rows on single CTAs without a split of K, wins where at most 128 rows
+    meet so many columns that its tiles fill the GPU (64 rows: 32000 x 4096 47 us against 56; but 128 rows of 4096 x 22016 129 against 43, of
+    1024 x 5632 35 against 17, of 8192 x 7168 51 against 34).  The same line stands in ``csrc/native_autograd.cpp``."""
+    return M > 128 or N <= 16384
+
+
 def matmul(a: torch.Tensor, b: torch.Tensor, trans_a: bool = False, trans_b: bool = False,
            out: torch.Tensor | None = None, accumulate: bool = False, out_dtype=None) -> torch.Tensor:
     """``op(a) @ op(b)`` for 2-D tensors. ``accumulate`` adds into ``out`` (fp32 or bf16)."""
@@ -73,7 +80,7 @@ def matmul(a: torch.Tensor, b: torch.Tensor, trans_a: bool = False, trans_b: boo
             out = torch.empty(M, N, dtype=out_dtype, device=a.device)
             accumulate = False
         _ext.count_launch()
-        if _USE_2CTA and M >= 256 and hasattr(_ext.ext(), "gemm_bf16_2cta"):
+        if _USE_2CTA and _pairs(M, N) and hasattr(_ext.ext(), "gemm_bf16_2cta"):
             _ext.ext().gemm_bf16_2cta(a, b, out, bool(trans_a), bool(trans_b), bool(accumulate))
         else:
             _ext.ext().gemm_bf16(a, b, out, bool(trans_a), bool(trans_b), bool(accumulate))
