@@ -92,8 +92,10 @@ __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const T* gu, T* out, si
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) swiglu_bwd_kernel(const T* __restrict__ go, const T* __restrict__ gu,
-                                                         T* __restrict__ dgu, size_t rows, int I) {
+__global__ void __launch_bounds__(256) swiglu_bwd_kernel(const T* go, const T* gu,
+                                                         T* dgu, size_t rows, int I) {
+  pdl_trigger();
+  pdl_wait();
   using P = Pack16<T>;
   constexpr int N = P::N;
   const int vec_per_row = I / N;
@@ -136,9 +138,11 @@ __device__ __forceinline__ void rotate(const Pack16<T>& p1, const Pack16<T>& p2,
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) rope_kernel(const T* __restrict__ x, T* __restrict__ out,
-                                                   const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+__global__ void __launch_bounds__(256) rope_kernel(const T* x, T* out,
+                                                   const float* cos_t, const float* sin_t,
                                                    int B, int S, int Hh, int D, long sb, long ss, long sh, float sign) {
+  pdl_trigger();
+  pdl_wait();
   using P = Pack16<T>;
   constexpr int N = P::N;
   const int half = D / 2;
@@ -168,9 +172,11 @@ __global__ void __launch_bounds__(256) rope_kernel(const T* __restrict__ x, T* _
 // thread.  With the caches flushed, 2048 tokens x (32 + 2 x 32) heads of 128 take 18.5 us forward and 29.6 back (10.3 and 15.4 at the
 // copy rate); two rotations each way and a concatenation took 23.6 and 37.9.  4 x 1024 x (32 + 2 x 8): 20.5 and 30.9, were 25.6 and 138.
 template <typename T>
-__global__ void __launch_bounds__(256) rope_qkv_fwd_kernel(const T* __restrict__ x, T* __restrict__ q, T* __restrict__ k,
-                                                           const float* __restrict__ cos_t, const float* __restrict__ sin_t, int B, int H,
+__global__ void __launch_bounds__(256) rope_qkv_fwd_kernel(const T* x, T* q, T* k,
+                                                           const float* cos_t, const float* sin_t, int B, int H,
                                                            int K, int D, float sign) {
+  pdl_trigger();
+  pdl_wait();
   using P = Pack16<T>;
   constexpr int N = P::N;
   const int half = D / 2, per = half / N, s = blockIdx.x / B, S = gridDim.x / B;
@@ -180,8 +186,8 @@ __global__ void __launch_bounds__(256) rope_qkv_fwd_kernel(const T* __restrict__
     const int h = i / per, c = (i - h * per) * N;
     T* dst = h < H ? q + (to * H + h) * D : k + (to * K + h - H) * D;
     P p1, p2, o1, o2;
-    p1.load_nc(row + (size_t)h * D + c);
-    p2.load_nc(row + (size_t)h * D + half + c);
+    p1.load(row + (size_t)h * D + c);
+    p2.load(row + (size_t)h * D + half + c);
     const float* cr = cos_t + (size_t)s * half + c;
     const float* sr = sin_t + (size_t)s * half + c;
     rotate(p1, p2, cr, sr, sign, o1, o2);
@@ -193,9 +199,11 @@ __global__ void __launch_bounds__(256) rope_qkv_fwd_kernel(const T* __restrict__
 // A gradient [B, S, heads, D] and its strides over batch, position and head.
 struct RopeGrad { const void* p; long sb, ss, sh; };
 template <typename T>
-__global__ void __launch_bounds__(256) rope_qkv_bwd_kernel(const RopeGrad gq, const RopeGrad gk, const RopeGrad gv, T* __restrict__ out,
-                                                           const float* __restrict__ cos_t, const float* __restrict__ sin_t, int B, int H,
+__global__ void __launch_bounds__(256) rope_qkv_bwd_kernel(const RopeGrad gq, const RopeGrad gk, const RopeGrad gv, T* out,
+                                                           const float* cos_t, const float* sin_t, int B, int H,
                                                            int K, int D, float sign) {
+  pdl_trigger();
+  pdl_wait();
   using P = Pack16<T>;
   constexpr int N = P::N;
   const int half = D / 2, per = half / N, s = blockIdx.x / B, b = blockIdx.x - s * B;
@@ -206,8 +214,8 @@ __global__ void __launch_bounds__(256) rope_qkv_bwd_kernel(const RopeGrad gq, co
     const int hh = h < H ? h : h < H + K ? h - H : h - H - K;
     const T* src = (const T*)g.p + b * g.sb + s * g.ss + hh * g.sh;
     P p1, p2, o1, o2;
-    p1.load_nc(src + c);
-    p2.load_nc(src + half + c);
+    p1.load(src + c);
+    p2.load(src + half + c);
     if (h < H + K) {
       const float* cr = cos_t + (size_t)s * half + c;
       const float* sr = sin_t + (size_t)s * half + c;
@@ -303,8 +311,10 @@ template <typename T, int U> NXD_DEVICE float packets_max(const Pack16<T> (&p)[U
 // thirds of the time).  4096 x 32000, bf16: 44 us (40 at the copy rate), ce_stats_kernel 49 and three launches of 1.9 to 3.1 behind it;
 // a ring of bulk copies under persistent blocks took 49 too.
 template <typename T, int THREADS>
-__global__ void __launch_bounds__(THREADS, 2048 / THREADS) ce_loss_kernel(const T* __restrict__ logits, const int64_t* __restrict__ target,
-                                                                           float* __restrict__ lse, float* __restrict__ loss, int V, int vec) {
+__global__ void __launch_bounds__(THREADS, 2048 / THREADS) ce_loss_kernel(const T* logits, const int64_t* target,
+                                                                           float* lse, float* loss, int V, int vec) {
+  pdl_trigger();
+  pdl_wait();
   using P = Pack16<T>;
   constexpr int N = P::N, U = 4;                // packets in flight per thread
   __shared__ float red[32];
@@ -360,10 +370,12 @@ __global__ void __launch_bounds__(THREADS, 2048 / THREADS) ce_loss_kernel(const 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) ce_bwd_kernel(const T* __restrict__ logits, const int64_t* __restrict__ target,
-                                                     const float* __restrict__ lse, const float* __restrict__ gout,
-                                                     T* __restrict__ grad, int V, int vocab_start, float smoothing,
+__global__ void __launch_bounds__(256) ce_bwd_kernel(const T* logits, const int64_t* target,
+                                                     const float* lse, const float* gout,
+                                                     T* grad, int V, int vocab_start, float smoothing,
                                                      float inv_vocab, int vec) {
+  pdl_trigger();
+  pdl_wait();
   using P = Pack16<T>;
   constexpr int N = P::N;
   const int row = gridDim.x - 1 - blockIdx.x;       // the rows that the statistics read last are the ones still in L2
@@ -438,7 +450,7 @@ void swiglu_bwd(const void* go, const void* gu, void* dgu, long rows, int I, int
   DISPATCH_DTYPE(dt, {
     const size_t total = (size_t)rows * (I / Pack16<T>::N);
     const int grid = (int)min((size_t)num_sms() * 16, (total + 255) / 256);
-    swiglu_bwd_kernel<T><<<max(grid, 1), 256, 0, st>>>((const T*)go, (const T*)gu, (T*)dgu, (size_t)rows, I);
+    launch_dependent(swiglu_bwd_kernel<T>, max(grid, 1), 256, 0, st, (const T*)go, (const T*)gu, (T*)dgu, (size_t)rows, I);
   });
   NXD_CUDA_CHECK(cudaGetLastError());
 }
@@ -478,7 +490,7 @@ void rope_apply(const void* x, void* out, const float* cos_t, const float* sin_t
     }
     const size_t total = (size_t)B * S * Hh * ((D / 2) / Pack16<T>::N);
     const int grid = (int)min((size_t)num_sms() * 16, (total + 255) / 256);
-    rope_kernel<T><<<max(grid, 1), 256, 0, st>>>((const T*)x, (T*)out, cos_t, sin_t, B, S, Hh, D, sb, ss, sh, sign);
+    launch_dependent(rope_kernel<T>, max(grid, 1), 256, 0, st, (const T*)x, (T*)out, cos_t, sin_t, B, S, Hh, D, sb, ss, sh, sign);
   });
   NXD_CUDA_CHECK(cudaGetLastError());
 }
@@ -487,7 +499,7 @@ void rope_qkv_fwd(const void* x, void* q, void* k, const float* cos_t, const flo
                   cudaStream_t st) {
   if (S * B == 0) return;
   DISPATCH_DTYPE(dt, {
-    rope_qkv_fwd_kernel<T><<<S * B, 256, 0, st>>>((const T*)x, (T*)q, (T*)k, cos_t, sin_t, B, H, K, D, 1.0f);
+    launch_dependent(rope_qkv_fwd_kernel<T>, S * B, 256, 0, st, (const T*)x, (T*)q, (T*)k, cos_t, sin_t, B, H, K, D, 1.0f);
   });
   NXD_CUDA_CHECK(cudaGetLastError());
 }
@@ -498,7 +510,7 @@ void rope_qkv_bwd(const void* gq, const void* gk, const void* gv, const long (*s
   const RopeGrad g[3] = {{gq, strides[0][0], strides[0][1], strides[0][2]}, {gk, strides[1][0], strides[1][1], strides[1][2]},
                          {gv, strides[2][0], strides[2][1], strides[2][2]}};
   DISPATCH_DTYPE(dt, {
-    rope_qkv_bwd_kernel<T><<<S * B, 256, 0, st>>>(g[0], g[1], g[2], (T*)out, cos_t, sin_t, B, H, K, D, -1.0f);
+    launch_dependent(rope_qkv_bwd_kernel<T>, S * B, 256, 0, st, g[0], g[1], g[2], (T*)out, cos_t, sin_t, B, H, K, D, -1.0f);
   });
   NXD_CUDA_CHECK(cudaGetLastError());
 }
@@ -517,7 +529,7 @@ void ce_stats(const void* logits, const int64_t* target, float* stats, int rows,
 void ce_loss(const void* logits, const int64_t* target, float* lse, float* loss, int rows, int V, int dt, cudaStream_t st) {
   DISPATCH_DTYPE(dt, {
     const int vec = (uintptr_t)logits % 16 == 0 && V % Pack16<T>::N == 0;
-    auto go = [&](auto kernel, int threads) { kernel<<<rows, threads, 0, st>>>((const T*)logits, target, lse, loss, V, vec); };
+    auto go = [&](auto kernel, int threads) { launch_dependent(kernel, rows, threads, 0, st, (const T*)logits, target, lse, loss, V, vec); };
     if ((long)V * sizeof(T) >= 128 << 10 || rows <= 2 * num_sms()) go(ce_loss_kernel<T, 512>, 512);
     else go(ce_loss_kernel<T, 256>, 256);
   });
@@ -528,7 +540,7 @@ void ce_backward(const void* logits, const int64_t* target, const float* lse, co
                  int V, int vocab_start, float smoothing, int vocab, int dt, cudaStream_t st) {
   DISPATCH_DTYPE(dt, {
     const int vec = ((uintptr_t)logits | (uintptr_t)grad) % 16 == 0 && V % Pack16<T>::N == 0;
-    ce_bwd_kernel<T><<<rows, 256, 0, st>>>((const T*)logits, target, lse, gout, (T*)grad, V, vocab_start, smoothing,
+    launch_dependent(ce_bwd_kernel<T>, rows, 256, 0, st, (const T*)logits, target, lse, gout, (T*)grad, V, vocab_start, smoothing,
                                            1.f / (float)vocab, vec);
   });
   NXD_CUDA_CHECK(cudaGetLastError());

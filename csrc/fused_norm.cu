@@ -20,10 +20,8 @@ namespace nxd {
 // WIDE: rows of more than 256 * MAXV packets; a kernel of its own, since its second loops cost the others registers (bf16: 66 instead
 // of 48; 8192 x 5120: 74 us instead of 57).
 template <typename T, int MAXV, bool WIDE>
-__global__ void __launch_bounds__(256) add_rmsnorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ r,
-                                                              const T* __restrict__ w, T* __restrict__ h,
-                                                              T* __restrict__ y, float* __restrict__ rstd_out, int H,
-                                                              float eps) {
+NXD_DEVICE void add_rmsnorm_rows(const T* __restrict__ x, const T* __restrict__ r, const T* __restrict__ w, T* __restrict__ h,
+                                 T* __restrict__ y, float* __restrict__ rstd_out, int H, float eps) {
   using P = Pack16<T>;
   constexpr int N = P::N;
   __shared__ float red[32];
@@ -69,7 +67,7 @@ __global__ void __launch_bounds__(256) add_rmsnorm_fwd_kernel(const T* __restric
     const int v = threadIdx.x + i * blockDim.x;
     if (v < nvec) {
       P pw, po;
-      pw.load_nc(w + v * N);
+      pw.load(w + v * N);
 #pragma unroll
       for (int j = 0; j < N; ++j) po.set(j, cache[i].f(j) * rstd * pw.f(j));
       po.store(y + base + v * N);
@@ -78,11 +76,18 @@ __global__ void __launch_bounds__(256) add_rmsnorm_fwd_kernel(const T* __restric
   for (int v = threadIdx.x + MAXV * blockDim.x; WIDE && v < nvec; v += blockDim.x) {
     P p, pw, po;
     p.load(h + base + v * N);
-    pw.load_nc(w + v * N);
+    pw.load(w + v * N);
 #pragma unroll
     for (int j = 0; j < N; ++j) po.set(j, p.f(j) * rstd * pw.f(j));
     po.store(y + base + v * N);
   }
+}
+
+template <typename T, int MAXV, bool WIDE>
+__global__ void __launch_bounds__(256) add_rmsnorm_fwd_kernel(const T* x, const T* r, const T* w, T* h, T* y, float* rstd_out, int H, float eps) {
+  pdl_trigger();
+  pdl_wait();
+  add_rmsnorm_rows<T, MAXV, WIDE>(x, r, w, h, y, rstd_out, H, eps);
 }
 
 // Backward of both norms (RES: with the gradient arriving on the residual path).  Persistent blocks stride over rows; each thread
@@ -92,10 +97,12 @@ __global__ void __launch_bounds__(256) add_rmsnorm_fwd_kernel(const T* __restric
 // blocks per SM were half as many.  Both kernels, bf16 with the residual path, before and now: 8192 x 4096 61.7 and 51.1 us (41 for its
 // bytes at the copy rate), 16384 x 4096 111 and 90, 16384 x 1024 45 and 32, 16384 x 8192 171 and 159, 64 x 4096 8.3 and 6.3.
 template <typename T, bool RES, int VPT, int MAXT>
-__global__ void __launch_bounds__(MAXT, MAXT == 1024 ? 1 : VPT == 1 ? 3 : 2) norm_bwd_kernel(const T* __restrict__ gy, const T* __restrict__ gh,
-                                                                        const T* __restrict__ h, const T* __restrict__ w,
-                                                                        const float* __restrict__ rstd, T* __restrict__ dh,
-                                                                        float* __restrict__ partial_dw, int rows, int H) {
+__global__ void __launch_bounds__(MAXT, MAXT == 1024 ? 1 : VPT == 1 ? 3 : 2) norm_bwd_kernel(const T* gy, const T* gh,
+                                                                        const T* h, const T* w,
+                                                                        const float* rstd, T* dh,
+                                                                        float* partial_dw, int rows, int H) {
+  pdl_trigger();                                           // the sum of the parts may take its place; it waits for this grid
+  pdl_wait();
   using P = Pack16<T>;
   constexpr int N = P::N;
   extern __shared__ __align__(128) uint8_t ring_raw[];
@@ -128,11 +135,10 @@ __global__ void __launch_bounds__(MAXT, MAXT == 1024 ? 1 : VPT == 1 ? 3 : 2) nor
   for (int i = 0; i < VPT; ++i) {
 #pragma unroll
     for (int j = 0; j < N; ++j) dw[i][j] = 0.f;
-    if (at(i) < H) pw[i].load_nc(w + at(i));
+    if (at(i) < H) pw[i].load(w + at(i));
   }
   float rs = rstd[blockIdx.x];
   __syncthreads();
-  pdl_trigger();                                           // the sum of the parts may take its place; it waits for this grid
   int st = 0;
   uint32_t ph = 0;
   for (unsigned row = blockIdx.x; row < (unsigned)rows; row += gridDim.x) {
@@ -239,7 +245,7 @@ void add_rmsnorm_fwd(const void* x, const void* r, const void* w, void* h, void*
     if (H % Pack16<T>::N) nxd_throw("add_rmsnorm: H must be a multiple of the 16-byte vector width", __FILE__, __LINE__);
     const int th = fn_pick_threads<T>(H);
     auto kernel = H / Pack16<T>::N <= 256 * 4 ? add_rmsnorm_fwd_kernel<T, 4, false> : add_rmsnorm_fwd_kernel<T, 4, true>;
-    kernel<<<rows, th, 0, st>>>((const T*)x, (const T*)r, (const T*)w, (T*)h, (T*)y, rstd, H, eps);
+    launch_dependent(kernel, rows, th, 0, st, (const T*)x, (const T*)r, (const T*)w, (T*)h, (T*)y, rstd, H, eps);
   });
   NXD_CUDA_CHECK(cudaGetLastError());
 }
@@ -267,9 +273,8 @@ static void norm_bwd_launch(const void* gy, const void* gh, const void* h, const
                             int H, int threads, int grid, cudaStream_t st) {
   constexpr int kMost = 6 * 1024 * 16;                     // two stages of three rows of 1024 packets
   NXD_ALLOW_SMEM((norm_bwd_kernel<T, RES, VPT, MAXT>), kMost);
-  norm_bwd_kernel<T, RES, VPT, MAXT><<<grid, threads, (size_t)(RES ? 6 : 4) * H * sizeof(T), st>>>(
-      (const T*)gy, (const T*)gh, (const T*)h, (const T*)w, rstd, (T*)dh, partial, rows, H);
-  NXD_CUDA_CHECK(cudaGetLastError());
+  launch_dependent(norm_bwd_kernel<T, RES, VPT, MAXT>, grid, threads, (size_t)(RES ? 6 : 4) * H * sizeof(T), st,
+                   (const T*)gy, (const T*)gh, (const T*)h, (const T*)w, rstd, (T*)dh, partial, rows, H);
 }
 
 template <bool RES>

@@ -74,8 +74,9 @@ NXD_DEVICE Unit unit_of(int unit, int num_tiles, int tiles_m, int tiles_n, int n
 template <bool A_KMAJOR, bool B_KMAJOR, typename OutT, int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                      const __grid_constant__ CUtensorMap tma_out, const __grid_constant__ CUtensorMap tma_part, OutT* __restrict__ out,
+                      const __grid_constant__ CUtensorMap tma_out, const __grid_constant__ CUtensorMap tma_part, OutT* out,
                       int M, int N, int K, int accumulate, int split_k, const Group grp, const Tail tail) {
+  if constexpr (MODE == 0) pdl_trigger();
   // accumulate: 0 store, 1 add to what is there.  split_k > 1 (fp32 outputs): that many pairs share one output tile, each sums
   // a K range and adds its partial — for weight gradients whose output has too few tiles to fill the 74 pairs while
   // K = tokens is long.  fp32 outputs always leave through TMA (stored or added in memory), bf16 ones unless they accumulate.
@@ -118,6 +119,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   cluster_sync_all();               // barriers of both CTAs are initialised before any remote arrive
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if constexpr (MODE == 0) pdl_wait();                       // all before this has run beside the end of the kernel before
 
   if (warp == 0) {
     // ===== TMA producer (both CTAs) =====
@@ -231,8 +233,10 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
 
 // out tile (+)= sum of its splits' partials, in order: one thread per 8 columns of a row
 template <typename OutT>
-__global__ void __launch_bounds__(256) gemm_tail_kernel(const float* __restrict__ part, OutT* __restrict__ out, int M, int N, int first,
+__global__ void __launch_bounds__(256) gemm_tail_kernel(const float* part, OutT* out, int M, int N, int first,
                                                         int tiles_m, int tiles_n, int splits, int accumulate) {
+  pdl_trigger();
+  pdl_wait();
   const int t = blockIdx.y, row = blockIdx.x * 8 + (threadIdx.x >> 5), col = (threadIdx.x & 31) * 8;
   int m_blk, n_blk;
   tile_coords(first + t, tiles_m, tiles_n, m_blk, n_blk);
@@ -770,8 +774,14 @@ static void launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensor
     NXD_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, g2::kSmem));
     configured = true;
   }
-  kern<<<grid, g2::kThreads, g2::kSmem, st>>>(ta, tb, to, tp, (OutT*)out, M, N, K, accumulate, split_k, grp, tail);
-  NXD_CUDA_CHECK(cudaGetLastError());
+  // A dependent: barriers, TMEM and maps of the next product are set up beside the end of this one (1 x 1000 tokens of 13B: 1152 us, 1130 with
+  // products, their tails, norms, SwiGLU and rotation so).  Not the grouped ones: they read the blocks' experts first and gain nothing.
+  if (MODE == 0) {
+    launch_dependent(kern, grid, g2::kThreads, g2::kSmem, st, ta, tb, to, tp, (OutT*)out, M, N, K, accumulate, split_k, grp, tail);
+  } else {
+    kern<<<grid, g2::kThreads, g2::kSmem, st>>>(ta, tb, to, tp, (OutT*)out, M, N, K, accumulate, split_k, grp, tail);
+    NXD_CUDA_CHECK(cudaGetLastError());
+  }
 }
 
 // Map of an output: fp32 slabs of 32 columns, bf16 slabs of 64; bf16 outputs that accumulate take no map (a dummy).
@@ -859,9 +869,9 @@ void gemm_bf16_2cta(const void* a, const void* b, void* out, int M, int N, int K
     const int tiles_m = (M + g2::TILE_M - 1) / g2::TILE_M, tiles_n = (N + g2::TILE_N - 1) / g2::TILE_N;
     const dim3 tg(g2::TILE_M / 8, p.tail.tiles);
     if (out_dt == kBF16)
-      g2::gemm_tail_kernel<__nv_bfloat16><<<tg, 256, 0, st>>>(workspace, (__nv_bfloat16*)out, M, N, p.tiles - p.tail.tiles, tiles_m, tiles_n, p.tail.splits, accumulate);
+      launch_dependent(g2::gemm_tail_kernel<__nv_bfloat16>, tg, 256, 0, st, (const float*)workspace, (__nv_bfloat16*)out, M, N, p.tiles - p.tail.tiles, tiles_m, tiles_n, p.tail.splits, accumulate);
     else
-      g2::gemm_tail_kernel<float><<<tg, 256, 0, st>>>(workspace, (float*)out, M, N, p.tiles - p.tail.tiles, tiles_m, tiles_n, p.tail.splits, accumulate);
+      launch_dependent(g2::gemm_tail_kernel<float>, tg, 256, 0, st, (const float*)workspace, (float*)out, M, N, p.tiles - p.tail.tiles, tiles_m, tiles_n, p.tail.splits, accumulate);
     NXD_CUDA_CHECK(cudaGetLastError());
   }
 }
