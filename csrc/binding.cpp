@@ -143,6 +143,34 @@ Tensor rope_qkv_bwd(const Tensor& gq, const Tensor& gk, const Tensor& gv, const 
   return out;
 }
 
+// q [B, S, H, D], k / v [B, S, K, D] (strided views in 16-byte packets) → rotated q; k rotated and v copied into rows 0..S-1 of the caches
+static Tensor prefill_rope_kv(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cos_t, const Tensor& sin_t, Tensor kc, Tensor vc) {
+  CHECK_IN(cos_t); CHECK_IN(sin_t);
+  TORCH_CHECK(q.dim() == 4 && k.dim() == 4 && kc.dim() == 4 && v.sizes() == k.sizes() && vc.sizes() == kc.sizes() && vc.strides() == kc.strides());
+  const int64_t B = q.size(0), S = q.size(1), H = q.size(2), D = q.size(3), K = k.size(2);
+  long strides[3][3], cs[3];
+  const Tensor* ts[3] = {&q, &k, &v};
+  for (int i = 0; i < 3; ++i) {
+    const Tensor& t = *ts[i];
+    TORCH_CHECK(t.is_cuda() && t.stride(3) == 1 && t.size(0) == B && t.size(1) == S && t.size(3) == D && t.scalar_type() == q.scalar_type() &&
+                (uintptr_t)t.data_ptr() % 16 == 0);
+    for (int d = 0; d < 3; ++d) {
+      strides[i][d] = t.stride(d);
+      TORCH_CHECK(t.size(d) == 1 || (t.stride(d) * t.element_size()) % 16 == 0);
+    }
+  }
+  TORCH_CHECK(kc.is_cuda() && kc.scalar_type() == q.scalar_type() && vc.scalar_type() == q.scalar_type() && kc.stride(3) == 1 && kc.size(0) >= B &&
+              kc.size(1) >= S && kc.size(2) == K && kc.size(3) == D && ((uintptr_t)kc.data_ptr() | (uintptr_t)vc.data_ptr()) % 16 == 0);
+  for (int d = 0; d < 3; ++d) { cs[d] = kc.stride(d); TORCH_CHECK((cs[d] * kc.element_size()) % 16 == 0); }
+  TORCH_CHECK((D / 2 * q.element_size()) % 16 == 0 && D % 2 == 0 && cos_t.scalar_type() == at::kFloat && sin_t.scalar_type() == at::kFloat &&
+              cos_t.dim() == 2 && cos_t.size(0) >= S && cos_t.size(1) == D / 2 && sin_t.sizes() == cos_t.sizes());
+  c10::cuda::CUDAGuard g(q.device());
+  auto out = at::empty({B, S, H, D}, q.options());
+  nxd::prefill_rope_kv(q.data_ptr(), k.data_ptr(), v.data_ptr(), strides, out.data_ptr(), kc.data_ptr(), vc.data_ptr(), cs, cos_t.data_ptr<float>(),
+                       sin_t.data_ptr<float>(), (int)B, (int)S, (int)H, (int)K, (int)D, dt_code(q), stream());
+  return out;
+}
+
 static Tensor ce_stats(const Tensor& logits, const Tensor& target, int64_t vocab_start) {
   CHECK_IN(logits); CHECK_IN(target);
   TORCH_CHECK(target.scalar_type() == at::kLong && logits.dim() == 2 && target.numel() == logits.size(0));
@@ -912,6 +940,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("rope_apply", &rope_apply);
   m.def("rope_qkv_fwd", &rope_qkv_fwd);
   m.def("rope_qkv_bwd", &rope_qkv_bwd);
+  m.def("prefill_rope_kv", &prefill_rope_kv);
   m.def("ce_stats", &ce_stats);
   m.def("ce_loss", &ce_loss);
   m.def("ce_backward", &ce_backward);

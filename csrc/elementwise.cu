@@ -228,6 +228,36 @@ __global__ void __launch_bounds__(256) rope_qkv_bwd_kernel(const RopeGrad gq, co
   }
 }
 
+// Prompts of served models: q rotated into a tensor of its own, k rotated and v copied into rows 0..S-1 of the caches, which the attention
+// then reads.  One block per token row, as above.  1000 tokens, 40 + 2 x 40 heads of 128: two rotations and two copies took 12 and 16 us.
+template <typename T>
+__global__ void __launch_bounds__(256) prefill_rope_kv_kernel(const RopeGrad gq, const RopeGrad gk, const RopeGrad gv, T* q_out, T* kc, T* vc,
+                                                              long c_sb, long c_ss, long c_sh, const float* cos_t, const float* sin_t, int B,
+                                                              int S, int H, int K, int D) {
+  using P = Pack16<T>;
+  constexpr int N = P::N;
+  pdl_trigger();
+  pdl_wait();
+  const int half = D / 2, per = half / N, s = blockIdx.x / B, b = blockIdx.x - s * B;
+  for (int i = threadIdx.x; i < (H + 2 * K) * per; i += 256) {
+    const int h = i / per, c = (i - h * per) * N;
+    const RopeGrad& g = h < H ? gq : h < H + K ? gk : gv;
+    const int hh = h < H ? h : h < H + K ? h - H : h - H - K;
+    const T* src = (const T*)g.p + b * g.sb + s * g.ss + hh * g.sh;
+    T* dst = h < H ? q_out + (((size_t)b * S + s) * H + hh) * D : (h < H + K ? kc : vc) + b * c_sb + s * c_ss + hh * c_sh;
+    P p1, p2, o1, o2;
+    p1.load(src + c);
+    p2.load(src + half + c);
+    if (h < H + K) {
+      rotate(p1, p2, cos_t + (size_t)s * half + c, sin_t + (size_t)s * half + c, 1.f, o1, o2);
+    } else {
+      o1 = p1; o2 = p2;
+    }
+    o1.store(dst + c);
+    o2.store(dst + half + c);
+  }
+}
+
 // =====================================================================================
 // Cross-entropy statistics: per row (max, sum exp(x-max), target logit if owned, sum x).
 // One CTA per row; online softmax per thread then block merge.
@@ -513,6 +543,18 @@ void rope_qkv_bwd(const void* gq, const void* gk, const void* gv, const long (*s
     launch_dependent(rope_qkv_bwd_kernel<T>, S * B, 256, 0, st, g[0], g[1], g[2], (T*)out, cos_t, sin_t, B, H, K, D, -1.0f);
   });
   NXD_CUDA_CHECK(cudaGetLastError());
+}
+
+// strides of q, k, v: batch, position, head; caches [B, L, K, D] with one set of strides
+void prefill_rope_kv(const void* q, const void* k, const void* v, const long (*strides)[3], void* q_out, void* kc, void* vc, const long* cs,
+                     const float* cos_t, const float* sin_t, int B, int S, int H, int K, int D, int dt, cudaStream_t st) {
+  if (S * B == 0) return;
+  const RopeGrad g[3] = {{q, strides[0][0], strides[0][1], strides[0][2]}, {k, strides[1][0], strides[1][1], strides[1][2]},
+                         {v, strides[2][0], strides[2][1], strides[2][2]}};
+  DISPATCH_DTYPE(dt, {
+    launch_dependent(prefill_rope_kv_kernel<T>, S * B, 256, 0, st, g[0], g[1], g[2], (T*)q_out, (T*)kc, (T*)vc, cs[0], cs[1], cs[2], cos_t, sin_t,
+                     B, S, H, K, D);
+  });
 }
 
 void ce_stats(const void* logits, const int64_t* target, float* stats, int rows, int V, int vocab_start, int dt,

@@ -26,6 +26,8 @@ void rope_qkv_fwd(const void* x, void* q, void* k, const float* cos_t, const flo
                   cudaStream_t st);
 void rope_qkv_bwd(const void* gq, const void* gk, const void* gv, const long (*strides)[3], void* out, const float* cos_t, const float* sin_t,
                   int S, int B, int H, int K, int D, int dt, cudaStream_t st);
+void prefill_rope_kv(const void* q, const void* k, const void* v, const long (*strides)[3], void* q_out, void* kc, void* vc, const long* cs,
+                     const float* cos_t, const float* sin_t, int B, int S, int H, int K, int D, int dt, cudaStream_t st);
 void ce_stats(const void* logits, const int64_t* target, float* stats, int rows, int V, int vocab_start, int dt,
               cudaStream_t st);
 void ce_loss(const void* logits, const int64_t* target, float* lse, float* loss, int rows, int V, int dt, cudaStream_t st);

@@ -94,12 +94,19 @@ class LlamaForInference(nn.Module):
             kc, vc = self.kv.get(layer_idx, kv_len)
             o = _window_attention(q, kc, vc, positions, None if tree is None else tree[0])
         elif prefill:
-            cos, sin = self.rope_cos[:S], self.rope_sin[:S]
-            q, k = ops.rope.apply_rotary(q, cos, sin), ops.rope.apply_rotary(k, cos, sin)
-            if self.flash_decoding:
-                self.kv.write_prefill_sharded(layer_idx, k, v, self.kv_rank)
+            kc, vc = self.kv.k[layer_idx], self.kv.v[layer_idx]
+            if self._prefill_in_cache(q, k, v, kc, vc):
+                # one launch: rotation of q and k and the cache's rows (csrc/elementwise.cu); the attention reads k and v there
+                ops._ext.count_launch()
+                q = ops._ext.ext().prefill_rope_kv(q, k, v, self.rope_cos, self.rope_sin, kc, vc)
+                k, v = kc[:B, :S], vc[:B, :S]
             else:
-                self.kv.write_prefill(layer_idx, k, v)
+                cos, sin = self.rope_cos[:S], self.rope_sin[:S]
+                q, k = ops.rope.apply_rotary(q, cos, sin), ops.rope.apply_rotary(k, cos, sin)
+                if self.flash_decoding:
+                    self.kv.write_prefill_sharded(layer_idx, k, v, self.kv_rank)
+                else:
+                    self.kv.write_prefill(layer_idx, k, v)
             o = ops.attention.flash_attention(q, k, v, causal=True)
         elif (q.is_cuda and q.dtype == torch.bfloat16 and self.kv.kv_quant is None and self.kv.seq_shards == 1
               and ops._ext.ext() is not None and hasattr(ops._ext.ext(), "decode_rope_kv")):
@@ -119,6 +126,22 @@ class LlamaForInference(nn.Module):
             o = _decode_attention(q, kc, vc, positions)
         o = o.transpose(0, 1).reshape(S, B, att.num_heads_local * D)
         return _row_linear_plus_residual(att.o_proj, o, x) if normed is None else att.o_proj(o)
+
+    def _prefill_in_cache(self, q, k, v, kc, vc) -> bool:
+        """The caches hold rows in the projection's own type that the one-launch rotation can write (whole 16-byte packets), nobody records
+        the calls, and no gradient is asked for."""
+        if (self.flash_decoding or type(self.kv) is not KVCacheManager or "write_prefill" in self.kv.__dict__ or self.kv.kv_quant is not None
+                or self.kv.seq_shards != 1 or torch.is_grad_enabled() or ops._ext.native(q, k, v, kc, vc, self.rope_cos, self.rope_sin) is None):
+            return False
+        per, S = 16 // q.element_size(), q.shape[1]
+        if (q.dtype not in (torch.bfloat16, torch.float16, torch.float32) or not q.dtype == k.dtype == v.dtype == kc.dtype == vc.dtype
+                or q.shape[-1] % (2 * per) or q.numel() == 0 or S > kc.shape[1] or q.shape[0] > kc.shape[0] or S > self.rope_cos.shape[0]
+                or k.shape[2:] != kc.shape[2:] or vc.shape != kc.shape or self.rope_cos.shape[1] * 2 != q.shape[-1]
+                or self.rope_cos.dtype != torch.float32 or self.rope_sin.dtype != torch.float32
+                or not (self.rope_cos.is_contiguous() and self.rope_sin.is_contiguous() and kc.is_contiguous() and vc.is_contiguous())
+                or kc.data_ptr() % 16 or vc.data_ptr() % 16):
+            return False
+        return all(t.stride(3) == 1 and t.data_ptr() % 16 == 0 and all(t.shape[d] == 1 or t.stride(d) % per == 0 for d in range(3)) for t in (q, k, v))
 
     def _tkg_block(self, layer_idx: int, layer):
         """Decode-time fused view of a MoE layer (shares its router / experts / norm; owns no parameters).  Kept outside the

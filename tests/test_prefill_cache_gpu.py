@@ -1,0 +1,55 @@
+"""Rotation of a prompt straight into the caches against the separate rotations and copies: the same bits, nothing written beyond the prompt."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("B,S,H,K,D", [(1, 1, 1, 1, 16), (1, 1000, 40, 40, 128), (2, 37, 8, 1, 128), (3, 64, 5, 5, 64)])
+def test_rows_in_the_caches(B, S, H, K, D, dtype):
+    from neuronx_distributed_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(S)
+    qkv = torch.randn(S, B, (H + 2 * K) * D, generator=g, device="cuda").to(dtype)
+    q, k, v = (t.unflatten(-1, (-1, D)).transpose(0, 1) for t in qkv.split([H * D, K * D, K * D], -1))
+    cos, sin = ops.rope.rope_tables(S + 5, D, device="cuda")
+    kc, vc = (torch.full((B + 1, S + 3, K, D), 7.0, device="cuda", dtype=dtype) for _ in range(2))
+    got = ops._ext.ext().prefill_rope_kv(q, k, v, cos, sin, kc, vc)
+    assert torch.equal(got, ops.rope.apply_rotary(q, cos[:S], sin[:S]))
+    assert torch.equal(kc[:B, :S], ops.rope.apply_rotary(k, cos[:S], sin[:S])) and torch.equal(vc[:B, :S], v)
+    for c in (kc, vc):
+        assert (c[B] == 7).all() and (c[:, S:] == 7).all()
+
+
+@pytest.mark.parametrize("batch,seq", [(1, 9), (2, 37), (1, 128)])
+def test_prompt_is_the_same(batch, seq, monkeypatch):
+    import torch.distributed as dist
+
+    from neuronx_distributed_b200.models.llama import LlamaConfig
+    from neuronx_distributed_b200.models.llama_inference import LlamaForInference
+    from neuronx_distributed_b200.parallel_layers import parallel_state as ps
+
+    if not dist.is_initialized():
+        dist.init_process_group("nccl", store=dist.HashStore(), rank=0, world_size=1, device_id=torch.device("cuda", 0))
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_model_parallel(tensor_model_parallel_size=1)
+    torch.manual_seed(0)
+    cfg = LlamaConfig(vocab_size=512, hidden_size=512, intermediate_size=1024, num_hidden_layers=2, num_attention_heads=4, num_key_value_heads=2,
+                      max_position_embeddings=128, dtype=torch.bfloat16, device=torch.device("cuda", 0))
+    model = LlamaForInference(cfg, batch_size=batch, max_seq_len=128, on_device_sampling=False).eval()
+    ids = torch.randint(0, 512, (batch, seq), device="cuda")
+    out = []
+    for own in (True, False):
+        model.kv.reset()
+        taken = []
+        if own:
+            inner = LlamaForInference._prefill_in_cache
+            monkeypatch.setattr(LlamaForInference, "_prefill_in_cache", lambda *a: taken.append(inner(*a)) or taken[-1])
+        else:
+            monkeypatch.setattr(LlamaForInference, "_prefill_in_cache", lambda *a: False)
+        logits = model.context_encoding(ids)
+        assert not own or taken == [True, True]
+        out.append([logits.clone(), *(t.clone() for t in model.kv.k + model.kv.v)])
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
