@@ -26,8 +26,7 @@
 
 namespace nxd {
 
-CUtensorMap make_tmap_bf16_strided(const void* ptr, uint64_t rows, uint64_t cols, uint64_t row_stride_elems,
-                                   uint32_t box_cols, uint32_t box_rows);
+CUtensorMap make_tmap_bf16_heads(const void* ptr, const uint64_t (&dims)[4], const uint64_t (&strides)[3], uint32_t box_cols, uint32_t box_rows);
 
 namespace fa {
 
@@ -80,8 +79,9 @@ NXD_DEVICE uint32_t pack_bf16(float lo, float hi) {
   return r;
 }
 
-// TMA coordinates of element (b, head, s, 0): c0 = b*col_b + head*col_h, c1 = b*row_b + head*row_h + s.
-struct Coord { int col_b, col_h, row_b, row_h; };
+// TMA coordinates of element (b, head, s, 0) in a map of dimensions (d, s, head, b): (0, s, head * h, b * b).  h, b: 1, or 0 where the view has one
+// head or sequence, or repeats one (stride 0).
+struct Coord { int h, b; };
 
 struct FwdParams {
   int S_q, S_kv, H, Hkv, B;
@@ -203,11 +203,11 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
       prefetch_tmap(&tq); prefetch_tmap(&tk); prefetch_tmap(&tv);
       int slot = 0; uint32_t ph = 0;
       int items[2] = {0, 0};
-      auto load_kv = [&](const CUtensorMap* map, int c, int r) {
+      auto load_kv = [&](const CUtensorMap* map, int r, int h, int b) {
         mbar_wait(bar_kve + 8 * slot, ph ^ 1);
         mbar_expect_tx(bar_kvf + 8 * slot, kTile);
-        tma_load_2d(sKV + slot * kTile, map, bar_kvf + 8 * slot, c, r);
-        tma_load_2d(sKV + slot * kTile + kHalf, map, bar_kvf + 8 * slot, c + 64, r);
+        tma_load_4d(sKV + slot * kTile, map, bar_kvf + 8 * slot, 0, r, h, b);
+        tma_load_4d(sKV + slot * kTile + kHalf, map, bar_kvf + 8 * slot, 64, r, h, b);
         if (++slot == kRing) { slot = 0; ph ^= 1; }
       };
       for (int il = 0;; ++il) {
@@ -215,22 +215,21 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
         if (idx < 0) break;
         const FwdItem it = fwd_item(idx, p);
         const int kvh = it.head / (p.H / p.Hkv);
-        const int qc = it.b * p.q.col_b + it.head * p.q.col_h, qr = it.b * p.q.row_b + it.head * p.q.row_h + it.qt * BM;
-        const int kc = it.b * p.k.col_b + kvh * p.k.col_h, kr = it.b * p.k.row_b + kvh * p.k.row_h;
-        const int vc = it.b * p.v.col_b + kvh * p.v.col_h, vr = it.b * p.v.row_b + kvh * p.v.row_h;
+        const int qh = it.head * p.q.h, qb = it.b * p.q.b, qr = it.qt * BM;
+        const int kh = kvh * p.k.h, kb = it.b * p.k.b, vh = kvh * p.v.h, vb = it.b * p.v.b;
         for (int t = 0; t < 2; ++t) {
           if (t == 0 ? it.n0 > 0 : (it.n1 > 0 && !p.split)) {
             mbar_wait(bar_qe + 8 * t, (uint32_t)((items[t] & 1) ^ 1));
             ++items[t];
             mbar_expect_tx(bar_qf + 8 * t, kTile);
-            tma_load_2d(sQ + t * kTile, &tq, bar_qf + 8 * t, qc, qr + t * BM);
-            tma_load_2d(sQ + t * kTile + kHalf, &tq, bar_qf + 8 * t, qc + 64, qr + t * BM);
+            tma_load_4d(sQ + t * kTile, &tq, bar_qf + 8 * t, 0, qr + t * BM, qh, qb);
+            tma_load_4d(sQ + t * kTile + kHalf, &tq, bar_qf + 8 * t, 64, qr + t * BM, qh, qb);
           }
-          if (t == 0 && it.n > 0) load_kv(&tk, kc, kr);
+          if (t == 0 && it.n > 0) load_kv(&tk, 0, kh, kb);
         }
         for (int j = 0; j < it.n; ++j) {
-          if (j > 0) load_kv(&tk, kc, kr + j * BN);
-          load_kv(&tv, vc, vr + j * BN);
+          if (j > 0) load_kv(&tk, j * BN, kh, kb);
+          load_kv(&tv, j * BN, vh, vb);
         }
         // asked for when the last tile is on its way (two steps before the end): asked at the item's start, the blocks would share
         // out the queue before they know which of them are done first (1 x 2048 tokens, 32 heads: 59 us)
@@ -645,13 +644,12 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
   if (warp == 0) {
     if (lane == 0 && n_iter > 0) {
       prefetch_tmap(&tq); prefetch_tmap(&tk); prefetch_tmap(&tv); prefetch_tmap(&tg);
-      const int kc = b * p.k.col_b + kvh * p.k.col_h, kr = b * p.k.row_b + kvh * p.k.row_h + kv0;
-      const int vc = b * p.v.col_b + kvh * p.v.col_h, vr = b * p.v.row_b + kvh * p.v.row_h + kv0;
+      const int kh = kvh * p.k.h, kb = b * p.k.b, v_h = kvh * p.v.h, vb = b * p.v.b;
       mbar_expect_tx(bar_kv, 2 * kTile);
-      tma_load_2d(sK, &tk, bar_kv, kc, kr);
-      tma_load_2d(sK + kHalf, &tk, bar_kv, kc + 64, kr);
-      tma_load_2d(sV, &tv, bar_kv, vc, vr);
-      tma_load_2d(sV + kHalf, &tv, bar_kv, vc + 64, vr);
+      tma_load_4d(sK, &tk, bar_kv, 0, kv0, kh, kb);
+      tma_load_4d(sK + kHalf, &tk, bar_kv, 64, kv0, kh, kb);
+      tma_load_4d(sV, &tv, bar_kv, 0, kv0, v_h, vb);
+      tma_load_4d(sV + kHalf, &tv, bar_kv, 64, kv0, v_h, vb);
       pdl_wait();                                          // the statistics come from the kernel before; q, k, v and dO do not
       for (int it = 0; it < n_iter; ++it) {
         const int qs = it % kQStages;
@@ -660,12 +658,11 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
         mbar_wait(bar_qe + 8 * qs, ph ^ 1);
         const uint32_t full = bar_qf + 8 * qs;
         mbar_expect_tx(full, 2 * kQTile + 512);
-        const int qc = b * p.q.col_b + head * p.q.col_h, qr = b * p.q.row_b + head * p.q.row_h + t * BQ;
-        const int gc = b * p.g.col_b + head * p.g.col_h, gr = b * p.g.row_b + head * p.g.row_h + t * BQ;
-        tma_load_2d(sQ + qs * kQTile, &tq, full, qc, qr);
-        tma_load_2d(sQ + qs * kQTile + kQTile / 2, &tq, full, qc + 64, qr);
-        tma_load_2d(sdO + qs * kQTile, &tg, full, gc, gr);
-        tma_load_2d(sdO + qs * kQTile + kQTile / 2, &tg, full, gc + 64, gr);
+        const int qh = head * p.q.h, qb = b * p.q.b, gh = head * p.g.h, gb = b * p.g.b;
+        tma_load_4d(sQ + qs * kQTile, &tq, full, 0, t * BQ, qh, qb);
+        tma_load_4d(sQ + qs * kQTile + kQTile / 2, &tq, full, 64, t * BQ, qh, qb);
+        tma_load_4d(sdO + qs * kQTile, &tg, full, 0, t * BQ, gh, gb);
+        tma_load_4d(sdO + qs * kQTile + kQTile / 2, &tg, full, 64, t * BQ, gh, gb);
         const float* st = p.stats + ((long)b * p.H + head) * p.S_pad + t * BQ;
         bulk_load_1d(sStats + qs * 512, st, 256, full);
         bulk_load_1d(sStats + qs * 512 + 256, st + p.stats_stride, 256, full);
@@ -974,23 +971,21 @@ __global__ void fa_bwd_kv_out_kernel(const float* part, __nv_bfloat16* dk, __nv_
 }
 
 // ---- host side -----------------------------------------------------------------------------------------------------
-// A [B, S, H, 128] bf16 view with strides (sb, ss, sh, 1) becomes a 2-D TMA tensor whose rows are `ss` apart; batch and
-// head offsets fold into the row coordinate when they are multiples of ss, else into the column coordinate.
+// A [B, S, H, 128] bf16 view with strides (sb, ss, sh, 1) as a map of four dimensions, so that rows behind the S-th of a (batch, head) read
+// as zeros: masked keys have probability 0, and 0 x NaN of whatever lies there (another sequence, a cache's old rows) would be NaN.
 struct View { const void* ptr; int B, S, H; long sb, ss, sh; };
 
 static CUtensorMap view_tmap(const View& v, Coord& c, uint32_t box_rows = 128) {
-  long rows = v.S, cols = HD;
-  c = Coord{0, 0, 0, 0};
-  auto fold = [&](long stride, int n, int& col_mul, int& row_mul) {
-    if (n == 1) return;
-    if (stride >= v.ss && stride % v.ss == 0) { row_mul = (int)(stride / v.ss); rows += (long)(n - 1) * row_mul; }
-    else { col_mul = (int)stride; cols += (long)(n - 1) * stride; }
-  };
-  fold(v.sb, v.B, c.col_b, c.row_b);
-  fold(v.sh, v.H, c.col_h, c.row_h);
-  if (cols > v.ss && rows > 1) nxd_throw("attention: unsupported q/k/v strides", __FILE__, __LINE__);
-  if ((v.ss * 2) % 16 || ((uintptr_t)v.ptr % 16)) nxd_throw("attention: q/k/v must be 16-byte aligned", __FILE__, __LINE__);
-  return make_tmap_bf16_strided(v.ptr, (uint64_t)rows, (uint64_t)cols, (uint64_t)v.ss, 64, box_rows);
+  // strides as the callers prepare them (ops/attention.py _tma_view): heads and sequences whole rows apart, or beside one another within a row
+  long cols = HD;
+  for (const auto& [stride, n] : {std::pair<long, int>{v.sb, v.B}, {v.sh, v.H}})
+    if (n > 1 && !(v.ss > 0 && stride >= v.ss && stride % v.ss == 0)) cols += (n - 1) * stride;
+  if (cols > v.ss && v.S > 1) nxd_throw("attention: unsupported q/k/v strides", __FILE__, __LINE__);
+  c = Coord{v.H > 1 && v.sh != 0, v.B > 1 && v.sb != 0};
+  const long ss = v.S > 1 ? v.ss : HD, sh = c.h ? v.sh : HD, sb = c.b ? v.sb : HD;        // of dimensions of one: any
+  if ((ss | sh | sb) % 8 || ((uintptr_t)v.ptr % 16)) nxd_throw("attention: q/k/v must be 16-byte aligned", __FILE__, __LINE__);
+  return make_tmap_bf16_heads(v.ptr, {(uint64_t)HD, (uint64_t)v.S, (uint64_t)(c.h ? v.H : 1), (uint64_t)(c.b ? v.B : 1)},
+                              {(uint64_t)ss, (uint64_t)sh, (uint64_t)sb}, 64, box_rows);
 }
 
 }  // namespace fa

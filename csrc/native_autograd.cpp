@@ -100,8 +100,8 @@ struct RopeQKV : Function<RopeQKV> {
 };
 
 // ------------------------------------------------------------------------------------------------------------ attention
-// The kernels read q / k / v through 2-D maps built from (b, s, h) strides: head_dim contiguous, batch and head offsets that fold into
-// rows or columns of the map; anything else is copied once (ops/attention.py _tma_view).
+// What the kernels' maps take as it is: head_dim contiguous, sequences and heads whole rows apart or beside one another within a row; anything
+// else is copied once (ops/attention.py _tma_view).
 Tensor map_view(const Tensor& t) {
   if (t.stride(3) != 1 || !aligned(t)) return t.contiguous();
   const int64_t ss = t.stride(1);

@@ -37,9 +37,9 @@ def _own_kernel_ok(q, k, v) -> bool:
 
 
 def _tma_view(t: torch.Tensor) -> torch.Tensor:
-    """The kernels read q/k/v through 2-D TMA maps built from (b, s, h) strides: head_dim must be contiguous and the batch /
-    head offsets must fold into rows or columns of that map (true for [B,S,H,D], [S,B,H,D], [B,H,S,D] memory and for slices
-    of a fused projection output); anything else is copied once."""
+    """The kernels read q/k/v through TMA maps built from (b, s, h) strides (csrc/attention_sm100.cu view_tmap): head_dim must be contiguous,
+    sequences and heads whole rows apart or beside one another within a row (true for [B,S,H,D], [S,B,H,D], [B,H,S,D] memory, for
+    slices of a fused projection output and of a cache); anything else is copied once."""
     if t.stride(3) != 1 or t.data_ptr() % 16:
         return t.contiguous()
     ss = t.stride(1)

@@ -53,3 +53,63 @@ def test_prompt_is_the_same(batch, seq, monkeypatch):
         out.append([logits.clone(), *(t.clone() for t in model.kv.k + model.kv.v)])
     for a, b in zip(*out):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("seq,longest", [(37, 128), (200, 256), (130, 130)])
+def test_old_rows_of_the_caches_are_never_used(seq, longest):
+    import torch.distributed as dist
+
+    from neuronx_distributed_b200.models.llama import LlamaConfig
+    from neuronx_distributed_b200.models.llama_inference import LlamaForInference
+    from neuronx_distributed_b200.parallel_layers import parallel_state as ps
+
+    if not dist.is_initialized():
+        dist.init_process_group("nccl", store=dist.HashStore(), rank=0, world_size=1, device_id=torch.device("cuda", 0))
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_model_parallel(tensor_model_parallel_size=1)
+    torch.manual_seed(0)
+    cfg = LlamaConfig(vocab_size=512, hidden_size=512, intermediate_size=1024, num_hidden_layers=2, num_attention_heads=4, num_key_value_heads=2,
+                      max_position_embeddings=longest, dtype=torch.bfloat16, device=torch.device("cuda", 0))
+    model = LlamaForInference(cfg, batch_size=2, max_seq_len=longest, on_device_sampling=False).eval()
+    ids = torch.randint(0, 512, (2, seq), device="cuda")
+    out = []
+    for left_there in (0.0, float("nan"), float("inf")):
+        for t in model.kv.k + model.kv.v:
+            t.fill_(left_there)
+        logits = model.context_encoding(ids)
+        out.append([logits.clone(), *(t[:, :seq].clone() for t in model.kv.k + model.kv.v)])
+    for other in out[1:]:
+        for a, b in zip(out[0], other):
+            assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("seq", [1, 37, 130, 200, 256])
+@pytest.mark.parametrize("order", ["bshd", "sbhd", "bhsd", "cache"])
+def test_a_sequence_does_not_see_its_neighbours(order, seq):
+    """Rows behind a sequence's last belong to others: NaN there (keys, values, queries, gradients) stays there, forward and backward."""
+    from neuronx_distributed_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(seq)
+
+    def make(heads):
+        shape = {"bshd": (2, seq, heads, 128), "sbhd": (seq, 2, heads, 128), "bhsd": (2, heads, seq, 128), "cache": (2, seq + 20, heads, 128)}[order]
+        t = torch.randn(shape, generator=g, device="cuda").bfloat16()
+        return {"bshd": t, "sbhd": t.transpose(0, 1), "bhsd": t.transpose(1, 2), "cache": t[:, :seq]}[order], t
+
+    (q, qm), (k, km), (v, vm), (go, gm) = make(4), make(2), make(2), make(4)
+    f = ops._ext.ext()
+
+    def both():
+        o, lse = f.flash_attn_fwd(q, k, v, True, 128 ** -0.5, True)
+        return [o, *f.flash_attn_bwd(go, q, k, v, o, lse, True, 128 ** -0.5, True, None, 1)]
+
+    want = [t[0].clone() for t in both()]
+    keep = [t[0].clone() for t in (q, k, v, go)]
+    for t, m, x in zip((q, k, v, go), (qm, km, vm, gm), keep):
+        m.fill_(float("nan"))
+        t[0] = x
+    for i, (a, b) in enumerate(zip(both(), want)):
+        if i == 1:                                         # dQ: sums over K/V tiles arrive in any order: fp32, then one rounding to bf16
+            assert (a[0].double() - b.double()).abs().max() <= 2.0 ** -7 * b.double().abs().max()
+        else:
+            assert torch.equal(a[0], b)
