@@ -163,9 +163,11 @@ struct CrossEntropy : Function<CrossEntropy> {
 PyObject* g_wgrad = nullptr;                               // layers.wgrad
 PyObject* g_fused_wgrad_enabled = nullptr;                 // ops.gemm.fused_wgrad_enabled
 
+bool pairs(int64_t M, int64_t N) { return M > 128 || N <= 16384; }      // ops/gemm.py _pairs
+
 void product(const Tensor& a, const Tensor& b, const Tensor& out, bool ta, bool tb, bool acc) {
   count();
-  if (out.size(0) > 128 || out.size(1) <= 16384) gemm_bf16_2cta(a, b, out, ta, tb, acc);      // ops/gemm.py _pairs
+  if (pairs(out.size(0), out.size(1))) gemm_bf16_2cta(a, b, out, ta, tb, acc);
   else gemm_bf16(a, b, out, ta, tb, acc);
 }
 
@@ -263,6 +265,7 @@ void bind_native_autograd(py::module_& m) {
   });
   n.def("cross_entropy", [](const Tensor& logits, const Tensor& target) { return CrossEntropy::apply(logits, target); });
   n.def("linear", &linear);
+  n.def("pairs", &pairs);
   n.def("launches", [] { return g_launches.load(); });
   n.def("set_weight_gradient", [](py::object wgrad, py::object enabled) {      // kept for the life of the process
     g_wgrad = wgrad.release().ptr();
