@@ -17,7 +17,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <cstdlib>
 #include <string>
 
 #include "common.cuh"
@@ -990,6 +989,8 @@ static CUtensorMap view_tmap(const View& v, Coord& c, uint32_t box_rows = 128) {
 
 }  // namespace fa
 
+int device_sm_count();
+
 void flash_attn_fwd(const void* q, const void* k, const void* v, void* out, float* lse, int B, int S_q, int S_kv, int H,
                     int Hkv, const long* qs, const long* ks, const long* vs, const long* os, float scale, bool causal,
                     cudaStream_t st) {
@@ -1005,15 +1006,10 @@ void flash_attn_fwd(const void* q, const void* k, const void* v, void* out, floa
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   p.causal = causal ? 1 : 0;
   p.lse = lse;
-  static bool configured = false;
-  if (!configured) {
-    NXD_CUDA_CHECK(cudaFuncSetAttribute(fa_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemFwd));
-    configured = true;
-  }
+  NXD_ALLOW_SMEM(fa_fwd_kernel, kSmemFwd);
   const long kv_bytes = (long)S_kv * HD * 4 * Hkv / H;            // K and V of one query head (its share of the group's)
   p.group_bh = (int)std::min<long>((long)H * B, std::max<long>(1, (48l << 20) / std::max<long>(1, kv_bytes)));
-  static int sms = 0;
-  if (!sms) { int dev; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
+  const int sms = device_sm_count();
   const int nq = (S_q + BM - 1) / BM;
   p.split = (long)nq * H * B <= sms;
   const long items = (long)(p.split ? nq : (nq + 1) / 2) * H * B;
@@ -1022,8 +1018,6 @@ void flash_attn_fwd(const void* q, const void* k, const void* v, void* out, floa
   fa_fwd_kernel<<<(unsigned)items, kThreads, kSmemFwd, st>>>(tq, tk, tv, (__nv_bfloat16*)out, p);
   NXD_CUDA_CHECK(cudaGetLastError());
 }
-
-int device_sm_count();
 
 // Blocks per KV head.  Unit: one 64-row query tile, about 1.8 us.  A launch lasts as long as its heaviest block, or as the sum of all over
 // the SMs and, since causal blocks differ, a quarter of the heaviest at the end; equal blocks come in whole rounds.  Every part costs
@@ -1051,9 +1045,12 @@ int flash_attn_bwd_parts(int B, int S_q, int S_kv, int H, int Hkv, bool causal) 
   return best;
 }
 
+int flash_attn_bwd_query_tiles(int S_q) { return (S_q + fa::BQ - 1) / fa::BQ; }
+
+// `turnstile`: null, or one counter per (batch, head, query tile) for dQ in a fixed order (fa_bwd_kernel<true>)
 void flash_attn_bwd(const void* go, const void* q, const void* k, const void* v, const void* o, const float* lse,
                     const float* dlse, void* dq,
-                    void* dk, void* dv, float* stats, float* dq_acc, float* kv_part, int parts, int B, int S_q, int S_kv, int H,
+                    void* dk, void* dv, float* stats, float* dq_acc, float* kv_part, unsigned* turnstile, int parts, int B, int S_q, int S_kv, int H,
                     int Hkv, int S_pad, const long* gs, const long* qs, const long* ks, const long* vs, const long* os,
                     const long* dqs, const long* dks, const long* dvs, float scale, bool causal, cudaStream_t st) {
   using namespace fa;
@@ -1071,25 +1068,9 @@ void flash_attn_bwd(const void* go, const void* q, const void* k, const void* v,
   p.stats = stats; p.stats_stride = (long)B * H * S_pad + 64;
   p.dq_acc = dq_acc;
   p.parts = parts; p.kv_part = kv_part;
-  // NXD_FA_DETERMINISTIC=1: ordered dQ accumulation (see fa_bwd_kernel<true>); the turnstile counters live in a per-device
-  // buffer that only grows (debug mode: allocation is synchronous, not meant for graph capture)
-  bool det = false;
-  { const char* e = getenv("NXD_FA_DETERMINISTIC"); det = e && atoi(e) != 0; }
-  p.turnstile = nullptr;
-  if (det) {
-    static unsigned* turn[64] = {nullptr};
-    static size_t cap[64] = {0};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const size_t need = (size_t)B * H * ((S_q + BQ - 1) / BQ) * sizeof(unsigned);
-    if (cap[dev & 63] < need) {
-      if (turn[dev & 63]) { NXD_CUDA_CHECK(cudaDeviceSynchronize()); cudaFree(turn[dev & 63]); }
-      NXD_CUDA_CHECK(cudaMalloc(&turn[dev & 63], need));
-      cap[dev & 63] = need;
-    }
-    p.turnstile = turn[dev & 63];
-    NXD_CUDA_CHECK(cudaMemsetAsync(p.turnstile, 0, need, st));
-  }
+  const bool det = turnstile != nullptr;
+  p.turnstile = turnstile;
+  if (det) NXD_CUDA_CHECK(cudaMemsetAsync(turnstile, 0, (size_t)B * H * flash_attn_bwd_query_tiles(S_q) * sizeof(unsigned), st));
   {
     const long rows = (long)B * H * S_pad;
     // an ordinary launch: the main kernel reads q, k, v and dO before it waits for this one, so they have to be there when this one starts
@@ -1097,12 +1078,8 @@ void flash_attn_bwd(const void* go, const void* q, const void* k, const void* v,
                                                                      dq_acc, p.stats_stride, B, S_q, H, S_pad, os[0], os[1], os[2], gs[0],
                                                                      gs[1], gs[2], scale);
   }
-  static bool configured = false;
-  if (!configured) {
-    NXD_CUDA_CHECK(cudaFuncSetAttribute(fa_bwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBwd));
-    NXD_CUDA_CHECK(cudaFuncSetAttribute(fa_bwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBwd));
-    configured = true;
-  }
+  NXD_ALLOW_SMEM(fa_bwd_kernel<false>, kSmemBwd);
+  NXD_ALLOW_SMEM(fa_bwd_kernel<true>, kSmemBwd);
   const long head_bytes = (long)S_q * HD * 8 * (H / Hkv / parts); // Q, dO and fp32 dQ of one block's query heads
   p.group_bh = (int)std::min<long>((long)Hkv * parts * B, std::max<long>(1, (64l << 20) / std::max<long>(1, head_bytes)));
   const unsigned grid = (unsigned)((S_kv + BN - 1) / BN * (long)Hkv * parts * B);

@@ -19,6 +19,13 @@ static int dt_code(const Tensor& t) {
     default: TORCH_CHECK(false, "unsupported dtype ", t.scalar_type());
   }
 }
+// A switch of the environment.  Threads that write os.environ hold the interpreter's lock and autograd's threads come here without it; getenv
+// beside setenv is not safe.
+static std::string env_switch(const char* name) {
+  py::gil_scoped_acquire lock;
+  const char* e = getenv(name);
+  return e ? e : "";
+}
 static cudaStream_t stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 #define CHECK_IN(t) TORCH_CHECK((t).is_cuda() && (t).is_contiguous(), #t " must be a contiguous CUDA tensor")
 
@@ -629,6 +636,8 @@ std::vector<Tensor> flash_attn_bwd(const Tensor& go, const Tensor& q, const Tens
   TORCH_CHECK(parts >= 1 && H % (Hkv * parts) == 0);
   Tensor kv_part;
   if (parts > 1) kv_part = at::empty({2, B, Hkv * parts, Skv, 128}, q.options().dtype(at::kFloat));
+  Tensor turnstile;                                        // dQ in a fixed order: bit-reproducible, slower
+  if (atoi(env_switch("NXD_FA_DETERMINISTIC").c_str()) != 0) turnstile = at::empty({B, H, nxd::flash_attn_bwd_query_tiles(S)}, q.options().dtype(at::kInt));
   auto st3 = [](const Tensor& t, long* out) { out[0] = t.stride(0); out[1] = t.stride(1); out[2] = t.stride(2); };
   long gs[3], qs[3], ks[3], vs[3], os[3], dqs[3], dks[3], dvs[3];
   st3(go, gs); st3(q, qs); st3(k, ks); st3(v, vs); st3(o, os); st3(dq, dqs); st3(dk, dks); st3(dv, dvs);
@@ -639,7 +648,8 @@ std::vector<Tensor> flash_attn_bwd(const Tensor& go, const Tensor& q, const Tens
   }
   nxd::flash_attn_bwd(go.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(), dlse_p,
                       dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), stats.data_ptr<float>(), dq_acc.data_ptr<float>(),
-                      parts > 1 ? kv_part.data_ptr<float>() : nullptr, (int)parts, B, S, Skv, H, Hkv, S_pad, gs, qs, ks, vs, os, dqs, dks, dvs, (float)scale, causal, stream());
+                      parts > 1 ? kv_part.data_ptr<float>() : nullptr, turnstile.defined() ? (unsigned*)turnstile.data_ptr() : nullptr, (int)parts,
+                      B, S, Skv, H, Hkv, S_pad, gs, qs, ks, vs, os, dqs, dks, dvs, (float)scale, causal, stream());
   return {dq, dk, dv};
 }
 
@@ -667,6 +677,9 @@ Tensor gemm_few_rows(const Tensor& x, const Tensor& w, int64_t split) {
   return y;
 }
 
+// NXD_GEMM_SPLITK=0: no sums in any order; read per call, sweeps toggle it at run time
+static bool gemm_split_k() { return env_switch("NXD_GEMM_SPLITK").substr(0, 1) != "0"; }
+
 void gemm_bf16_2cta(const Tensor& a, const Tensor& b, Tensor out, bool trans_a, bool trans_b, bool accumulate) {
   CHECK_IN(a); CHECK_IN(b); CHECK_IN(out);
   TORCH_CHECK(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16 && a.dim() == 2 && b.dim() == 2);
@@ -674,10 +687,11 @@ void gemm_bf16_2cta(const Tensor& a, const Tensor& b, Tensor out, bool trans_a, 
   const int N = (int)(trans_b ? b.size(0) : b.size(1));
   TORCH_CHECK((trans_b ? b.size(1) : b.size(0)) == K && out.size(0) == M && out.size(1) == N, "gemm shape mismatch");
   c10::cuda::CUDAGuard g(a.device());
-  const size_t bytes = nxd::gemm_2cta_workspace(M, N, K, dt_code(out), accumulate);
+  const bool split_k = gemm_split_k();
+  const size_t bytes = nxd::gemm_2cta_workspace(M, N, K, dt_code(out), accumulate, split_k);
   Tensor ws;
   if (bytes) ws = at::empty({(int64_t)(bytes / 4)}, a.options().dtype(at::kFloat));
-  nxd::gemm_bf16_2cta(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, trans_a, trans_b, dt_code(out), accumulate,
+  nxd::gemm_bf16_2cta(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, trans_a, trans_b, dt_code(out), accumulate, split_k,
                       bytes ? ws.data_ptr<float>() : nullptr, stream());
 }
 
@@ -950,7 +964,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("fused_adamw", &fused_adamw);
   m.def("gemm_bf16", &gemm_bf16);
   m.def("gemm_2cta_workspace", [](int64_t M, int64_t N, int64_t K, bool f32_out, bool accumulate) {      // bytes; 0: no split tail
-    return (int64_t)nxd::gemm_2cta_workspace((int)M, (int)N, (int)K, f32_out ? nxd::kF32 : nxd::kBF16, accumulate);
+    return (int64_t)nxd::gemm_2cta_workspace((int)M, (int)N, (int)K, f32_out ? nxd::kF32 : nxd::kBF16, accumulate, gemm_split_k());
   });
   m.def("gemm_bf16_2cta", &gemm_bf16_2cta);
   m.def("oneshot_allreduce", &oneshot_allreduce);

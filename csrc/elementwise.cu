@@ -464,11 +464,8 @@ template <typename T> static int pick_threads(int H) {
     default: nxd_throw("unsupported dtype", __FILE__, __LINE__);        \
   }
 
-static int num_sms() {
-  static int n = 0;
-  if (!n) { int dev; cudaGetDevice(&dev); cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev); }
-  return n;
-}
+int device_sm_count();
+static int num_sms() { return device_sm_count(); }
 
 void rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int rows, int H, float eps, int dt, cudaStream_t st) {
   DISPATCH_DTYPE(dt, {

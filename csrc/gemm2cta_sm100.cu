@@ -769,11 +769,7 @@ template <bool AK, bool BK_, typename OutT, int MODE = 0>
 static void launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& to, const CUtensorMap& tp, void* out, int M, int N, int K,
                     int accumulate, int split_k, const g2::Group& grp, const g2::Tail& tail, int grid, cudaStream_t st) {
   auto kern = g2::gemm_bf16_2cta_kernel<AK, BK_, OutT, MODE>;
-  static bool configured = false;
-  if (!configured) {
-    NXD_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, g2::kSmem));
-    configured = true;
-  }
+  NXD_ALLOW_SMEM(kern, g2::kSmem);
   // A dependent: barriers, TMEM and maps of the next product are set up beside the end of this one (1 x 1000 tokens of 13B: 1152 us, 1130 with
   // products, their tails, norms, SwiGLU and rotation so).  Not the grouped ones: they read the blocks' experts first and gain nothing.
   if (MODE == 0) {
@@ -795,7 +791,7 @@ static CUtensorMap out_map(const void* out, int out_dt, bool accumulate, bool ma
 // How a product is shared out: split-K of every tile (fp32 outputs), or of the last round's tiles alone, or neither.  Time of a
 // 256 x 256 tile: 0.39 us per k-block; a pass over fp32 memory: 6 bytes/ps.
 struct GemmPlan { int tiles, split; g2::Tail tail; };
-static GemmPlan gemm_plan(int M, int N, int K, int out_dt, bool accumulate) {
+static GemmPlan gemm_plan(int M, int N, int K, int out_dt, bool accumulate, bool split_k) {
   const int pairs = std::max(1, device_sm_count() / 2), num_kb = (K + g2::BK - 1) / g2::BK;      // (no device: one, for the asking)
   GemmPlan p;
   p.tiles = ((M + g2::TILE_M - 1) / g2::TILE_M) * ((N + g2::TILE_N - 1) / g2::TILE_N);
@@ -822,8 +818,7 @@ static GemmPlan gemm_plan(int M, int N, int K, int out_dt, bool accumulate) {
   // loop still amortises its epilogue.  Its partials are added in any order.  Outputs of fewer rows than a tile never take it: their few
   // tiles are a tail, whose partials are summed in order, so that the same inputs give the same bits (128 x 4096 over 8192 tokens: 21.4 us
   // stored, 22.0 added to what is there; 20.4 and 16.4 with partials added in any order, 55 and 60 without a split).
-  const char* split_env = getenv("NXD_GEMM_SPLITK");            // re-read per call: A/B sweeps toggle it at run time
-  if (out_dt == kF32 && M >= g2::TILE_M && !(split_env && split_env[0] == '0')) {
+  if (out_dt == kF32 && M >= g2::TILE_M && split_k) {
     const double pass_us = (double)M * N * 4 / 6e6;
     for (int s2 = 2; s2 <= 8; ++s2) {
       if (num_kb / s2 < 16) break;
@@ -837,19 +832,19 @@ static GemmPlan gemm_plan(int M, int N, int K, int out_dt, bool accumulate) {
 }
 
 // bytes of fp32 workspace that gemm_bf16_2cta takes for these sizes (0: none)
-size_t gemm_2cta_workspace(int M, int N, int K, int out_dt, bool accumulate) {
-  const GemmPlan p = gemm_plan(M, N, K, out_dt, accumulate);
+size_t gemm_2cta_workspace(int M, int N, int K, int out_dt, bool accumulate, bool split_k) {
+  const GemmPlan p = gemm_plan(M, N, K, out_dt, accumulate, split_k);
   return (size_t)p.tail.tiles * p.tail.splits * g2::TILE_M * g2::TILE_N * sizeof(float);
 }
 
-// `workspace`: gemm_2cta_workspace bytes, 16-byte aligned, or null: then no tail is split
+// `split_k`: fp32 outputs may be sums in any order; `workspace`: gemm_2cta_workspace bytes, 16-byte aligned, or null: then no tail is split
 void gemm_bf16_2cta(const void* a, const void* b, void* out, int M, int N, int K, bool trans_a, bool trans_b, int out_dt,
-                    bool accumulate, float* workspace, cudaStream_t st) {
+                    bool accumulate, bool split_k, float* workspace, cudaStream_t st) {
   const bool AK = !trans_a, BK_ = trans_b;
   const CUtensorMap ta = AK ? make_tmap_bf16(a, M, K, g2::BK, g2::CTA_M) : make_tmap_bf16(a, K, M, 64, g2::BK);
   const CUtensorMap tb = BK_ ? make_tmap_bf16(b, N, K, g2::BK, g2::HALF_N) : make_tmap_bf16(b, K, N, 64, g2::BK);
   const CUtensorMap to = out_map(out, out_dt, accumulate, false, 1, M, N, ta);
-  GemmPlan p = gemm_plan(M, N, K, out_dt, accumulate);
+  GemmPlan p = gemm_plan(M, N, K, out_dt, accumulate, split_k);
   if (!workspace) p.tail = g2::Tail{0, 1, 1};
   const int pairs = device_sm_count() / 2, split = p.split;
   if (split > 1 && !accumulate) NXD_CUDA_CHECK(cudaMemsetAsync(out, 0, (size_t)M * N * sizeof(float), st));   // partials add into zeros
@@ -913,11 +908,7 @@ template <bool AK, bool BK_, int MODE>
 static void launch_tp(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tal, void* out, int M, int N, int K,
                       const g2::TpComm& c, int grid, cudaStream_t st) {
   auto kern = g2::gemm_bf16_2cta_tp_kernel<AK, BK_, MODE>;
-  static bool configured = false;
-  if (!configured) {
-    NXD_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, g2::kSmem));
-    configured = true;
-  }
+  NXD_ALLOW_SMEM(kern, g2::kSmem);
   kern<<<grid, g2::kThreads, g2::kSmem, st>>>(ta, tb, tal, (__nv_bfloat16*)out, M, N, K, c);
   NXD_CUDA_CHECK(cudaGetLastError());
 }

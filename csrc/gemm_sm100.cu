@@ -401,14 +401,13 @@ typedef CUresult (*PFN_encodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_
                                     CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 static PFN_encodeTiled get_encode() {
-  static PFN_encodeTiled fn = nullptr;
-  if (!fn) {
+  static const PFN_encodeTiled fn = [] {                   // a throw is no result: the next call asks again
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q;
     NXD_CUDA_CHECK(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q));
     if (!p || q != cudaDriverEntryPointSuccess) nxd_throw("cuTensorMapEncodeTiled not available", __FILE__, __LINE__);
-    fn = (PFN_encodeTiled)p;
-  }
+    return (PFN_encodeTiled)p;
+  }();
   return fn;
 }
 
@@ -454,8 +453,13 @@ static CUtensorMap make_tmap_u8(const void* ptr, uint64_t rows, uint64_t cols, u
 }
 
 static int sm_count() {
-  static int n = 0;
-  if (!n) { int dev; cudaGetDevice(&dev); cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev); }
+  static std::atomic<int> count{0};                        // 0: not known yet, or no device
+  int n = count.load(std::memory_order_relaxed);
+  if (!n) {
+    int dev;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
+      count.store(n, std::memory_order_relaxed);
+  }
   return n;
 }
 
@@ -534,11 +538,7 @@ template <bool AK, bool BK, int MODE, typename OutT>
 static void launch(const CUtensorMap& ta, const CUtensorMap& tb, void* out, int M, int N, int K, bool accumulate,
                    const CommDev& c, int grid, cudaStream_t st) {
   auto kern = gemm_bf16_kernel<AK, BK, MODE, OutT>;
-  static bool configured = false;
-  if (!configured) {
-    NXD_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-    configured = true;
-  }
+  NXD_ALLOW_SMEM(kern, kSmemBytes);
   kern<<<grid, kThreads, kSmemBytes, st>>>(ta, tb, (OutT*)out, M, N, K, accumulate ? 1 : 0, c);
   NXD_CUDA_CHECK(cudaGetLastError());
 }
@@ -626,11 +626,7 @@ void gemm_fp8(const void* a, const void* b, void* out, int M, int N, int K, cons
   const int tiles = ((M + BLOCK_M - 1) / BLOCK_M) * ((N + BLOCK_N - 1) / BLOCK_N);
   const int grid = tiles < sm_count() ? tiles : sm_count();
   auto kern = gemm_bf16_kernel<true, true, 0, __nv_bfloat16, true>;
-  static bool configured = false;
-  if (!configured) {
-    NXD_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-    configured = true;
-  }
+  NXD_ALLOW_SMEM(kern, kSmemBytes);
   kern<<<grid, kThreads, kSmemBytes, st>>>(ta, tb, (__nv_bfloat16*)out, M, N, K, 0, c);
   NXD_CUDA_CHECK(cudaGetLastError());
 }

@@ -61,9 +61,9 @@ void gemm_bf16(const void* a, const void* b, void* out, int M, int N, int K, boo
                bool accumulate, const GemmComm& comm, const void* a_local_shard, cudaStream_t st);
 bool gemm_self_check_supported();
 // CTA-pair (cta_group::2) variant, plain GEMM only
-size_t gemm_2cta_workspace(int M, int N, int K, int out_dt, bool accumulate);
+size_t gemm_2cta_workspace(int M, int N, int K, int out_dt, bool accumulate, bool split_k);
 void gemm_bf16_2cta(const void* a, const void* b, void* out, int M, int N, int K, bool trans_a, bool trans_b, int out_dt,
-                    bool accumulate, float* workspace, cudaStream_t st);
+                    bool accumulate, bool split_k, float* workspace, cudaStream_t st);
 
 void gemm_bf16_2cta_tp(int mode, const void* a, const void* b, void* out_or_partial, void* rs_out, const void* a_local,
                        int M, int N, int K, bool trans_b, int rank, int world, const int64_t* peer_bufs,
@@ -182,9 +182,10 @@ void flash_attn_fwd(const void* q, const void* k, const void* v, void* out, floa
 
 // parts (a divisor of H / Hkv; flash_attn_bwd_parts is the rule): blocks per KV head; kv_part: 2 * B * Hkv * parts * S_kv * 128 floats
 int flash_attn_bwd_parts(int B, int S_q, int S_kv, int H, int Hkv, bool causal);
+int flash_attn_bwd_query_tiles(int S_q);
 void flash_attn_bwd(const void* go, const void* q, const void* k, const void* v, const void* o, const float* lse,
                     const float* dlse, void* dq,
-                    void* dk, void* dv, float* stats, float* dq_acc, float* kv_part, int parts, int B, int S_q, int S_kv, int H,
+                    void* dk, void* dv, float* stats, float* dq_acc, float* kv_part, unsigned* turnstile, int parts, int B, int S_q, int S_kv, int H,
                     int Hkv, int S_pad, const long* gs, const long* qs, const long* ks, const long* vs, const long* os,
                     const long* dqs, const long* dks, const long* dvs, float scale, bool causal, cudaStream_t st);
 
