@@ -598,7 +598,6 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
   const uint32_t bar_kv = bars, bar_qf = bars + 8, bar_qe = bars + 32, bar_s = bars + 56, bar_dp = bars + 72,
                  bar_p = bars + 80, bar_dq = bars + 88, bar_dqr = bars + 96, bar_acc = bars + 104, tmem_slot = bars + 128;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  pdl_trigger();                                           // fa_bwd_dq_out_kernel's blocks wait on the SMs that run out of this kernel's
   // Blocks start heaviest first (causal: the first K/V tiles see the most query tiles) within groups of heads that share L2: head by
   // head, the last heads' heavy tiles started when most SMs had nothing left (1 x 2048 x 32 heads: 142 us, now 119).
   int n, kvh, b, vh;                                       // vh: the part's index among all parts of all KV heads
@@ -634,6 +633,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
+  pdl_trigger();                                           // fa_bwd_dq_out_kernel's blocks wait on the SMs that run out of this kernel's
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
   // TMEM columns: dK [0,128) | dV [128,256) | Sᵀ/Pᵀ double buffer [256,384) | dPᵀ [384,448) | dQᵀ [448,512)

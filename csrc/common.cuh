@@ -42,7 +42,9 @@ namespace nxd {
   } while (0)
 
 // Programmatic dependent launch: a kernel that was launched with launch_dependent starts while the one before it in the stream still
-// runs, and must pass pdl_wait before it touches anything that kernel wrote; pdl_trigger in the earlier one lets it start.
+// runs, and must pass pdl_wait before it touches anything that kernel wrote; pdl_trigger in the earlier one lets it start.  A kernel that
+// allocates tensor memory triggers behind the allocation: blocks of a later kernel that hold tensor memory and wait could otherwise keep one of its
+// blocks on the same SM from ever getting its own.
 // Every kernel launched so waits before it reads or writes anything of others and before it returns, so that its end is its predecessors' end
 // too.  Pointers to what a predecessor wrote are not __restrict__ there: a load through the read-only path must not move above the wait.
 NXD_DEVICE void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

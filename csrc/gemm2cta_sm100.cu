@@ -76,7 +76,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                       const __grid_constant__ CUtensorMap tma_out, const __grid_constant__ CUtensorMap tma_part, OutT* out,
                       int M, int N, int K, int accumulate, int split_k, const Group grp, const Tail tail) {
-  if constexpr (MODE == 0) pdl_trigger();
   // accumulate: 0 store, 1 add to what is there.  split_k > 1 (fp32 outputs): that many pairs share one output tile, each sums
   // a K range and adds its partial — for weight gradients whose output has too few tiles to fill the 74 pairs while
   // K = tokens is long.  fp32 outputs always leave through TMA (stored or added in memory), bf16 ones unless they accumulate.
@@ -119,7 +118,10 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   cluster_sync_all();               // barriers of both CTAs are initialised before any remote arrive
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if constexpr (MODE == 0) pdl_wait();                       // all before this has run beside the end of the kernel before
+  if constexpr (MODE == 0) {
+    pdl_trigger();                                           // behind the allocation (launch_dependent)
+    pdl_wait();                                              // all before this has run beside the end of the kernel before
+  }
 
   if (warp == 0) {
     // ===== TMA producer (both CTAs) =====

@@ -63,7 +63,6 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant
   const int num_kb = (K + BK - 1) / BK, per = (num_kb + split - 1) / split;
   const int kb0 = rank * per, kb1 = min(num_kb, kb0 + per);       // the host leaves no rank without a k-block
 
-  pdl_trigger();
   if (threadIdx.x == 0) {
     prefetch_tmap(&tma_w); prefetch_tmap(&tma_x);
     for (int kb = kb0; kb < min(kb1, kb0 + kAhead); ++kb) prefetch_l2_tile(&tma_w, kb * BK, n0);
@@ -77,6 +76,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant
   tcgen05_fence_after();
   uint32_t tmem;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot));
+  pdl_trigger();                                           // behind the allocation (launch_dependent)
   pdl_wait();
 
   if (warp == 0) {
