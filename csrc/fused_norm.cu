@@ -252,14 +252,17 @@ void add_rmsnorm_fwd(const void* x, const void* r, const void* w, void* h, void*
 
 int device_sm_count();
 
-// Threads of a block: one packet each, but two each between 512 and 768 packets, so that two blocks fit an SM.  Blocks per SM: as
-// registers allow, but no fewer than four rows per block (each block ends in a part of dW that another kernel reads; 1024 x 4096 in
-// blocks of two to three rows 14.4 us, of seven 12.4).
+// Blocks per SM: as registers allow, but a further one only while each block keeps at least four rows (each ends in a part of dW that another
+// kernel reads; 1024 x 4096 in blocks of two to three rows 14.4 us, of seven 12.4).  Threads of a block: one packet each, but two
+// each between 512 and 768 packets where the rows are enough for two blocks per SM, which then fit (16384 x 6144, without the residual
+// path: 104 us, 116 in one block per SM with a packet each).  With fewer rows a packet each is faster: 1024 x 6144 12.3 us, 13.4 with two,
+// x 5120 11.2 and 12.5, x 4608 10.3 and 12.3 (with the residual path; caches flushed: 19.5 and 21.5, 19.5 and 21.5, 17.4 and 21.5).
 static void norm_bwd_shape(int rows, int H, int dt, int& threads, int& vpt, int& grid) {
   const int size = dt == kF32 ? 4 : 2, nvec = H / (16 / size);
-  vpt = nvec > 512 && nvec <= 768 ? 2 : 1;
+  const int sms = device_sm_count();
+  vpt = nvec > 512 && nvec <= 768 && rows >= 8 * sms ? 2 : 1;
   threads = std::max(32, ((nvec + vpt - 1) / vpt + 31) / 32 * 32);
-  const int sms = device_sm_count(), most = std::min(8, (threads > 512 || vpt > 1 ? 1024 : 1536) / threads);
+  const int most = std::min(8, (threads > 512 || vpt > 1 ? 1024 : 1536) / threads);
   grid = std::min(rows, sms * std::max(1, std::min(most, rows / (4 * sms))));
 }
 int rmsnorm_bwd_num_partials(int rows, int H, int dt) {
