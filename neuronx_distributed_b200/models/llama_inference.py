@@ -94,9 +94,9 @@ class LlamaForInference(nn.Module):
             kc, vc = self.kv.get(layer_idx, kv_len)
             o = _window_attention(q, kc, vc, positions, None if tree is None else tree[0])
         elif prefill:
-            kc, vc = self.kv.k[layer_idx], self.kv.v[layer_idx]
-            if self._prefill_in_cache(q, k, v, kc, vc):
+            if self._prefill_in_cache(q, k, v, layer_idx):
                 # one launch: rotation of q and k and the cache's rows (csrc/elementwise.cu); the attention reads k and v there
+                kc, vc = self.kv.k[layer_idx], self.kv.v[layer_idx]
                 ops._ext.count_launch()
                 q = ops._ext.ext().prefill_rope_kv(q, k, v, self.rope_cos, self.rope_sin, kc, vc)
                 k, v = kc[:B, :S], vc[:B, :S]
@@ -127,11 +127,14 @@ class LlamaForInference(nn.Module):
         o = o.transpose(0, 1).reshape(S, B, att.num_heads_local * D)
         return _row_linear_plus_residual(att.o_proj, o, x) if normed is None else att.o_proj(o)
 
-    def _prefill_in_cache(self, q, k, v, kc, vc) -> bool:
+    def _prefill_in_cache(self, q, k, v, layer_idx: int) -> bool:
         """The caches hold rows in the projection's own type that the one-launch rotation can write (whole 16-byte packets), nobody records
         the calls, and no gradient is asked for."""
         if (self.flash_decoding or type(self.kv) is not KVCacheManager or "write_prefill" in self.kv.__dict__ or self.kv.kv_quant is not None
-                or self.kv.seq_shards != 1 or torch.is_grad_enabled() or ops._ext.native(q, k, v, kc, vc, self.rope_cos, self.rope_sin) is None):
+                or self.kv.seq_shards != 1 or torch.is_grad_enabled()):
+            return False
+        kc, vc = self.kv.k[layer_idx], self.kv.v[layer_idx]                  # a manager of another kind may keep its rows elsewhere
+        if ops._ext.native(q, k, v, kc, vc, self.rope_cos, self.rope_sin) is None:
             return False
         per, S = 16 // q.element_size(), q.shape[1]
         if (q.dtype not in (torch.bfloat16, torch.float16, torch.float32) or not q.dtype == k.dtype == v.dtype == kc.dtype == vc.dtype
