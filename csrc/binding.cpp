@@ -687,7 +687,7 @@ void gemm_bf16_2cta(const Tensor& a, const Tensor& b, Tensor out, bool trans_a, 
   const int N = (int)(trans_b ? b.size(0) : b.size(1));
   TORCH_CHECK((trans_b ? b.size(1) : b.size(0)) == K && out.size(0) == M && out.size(1) == N, "gemm shape mismatch");
   c10::cuda::CUDAGuard g(a.device());
-  const bool split_k = gemm_split_k();
+  const bool split_k = out.scalar_type() == at::kFloat && gemm_split_k();      // others have no such sums
   const size_t bytes = nxd::gemm_2cta_workspace(M, N, K, dt_code(out), accumulate, split_k);
   Tensor ws;
   if (bytes) ws = at::empty({(int64_t)(bytes / 4)}, a.options().dtype(at::kFloat));
