@@ -649,7 +649,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
       tma_load_4d(sK + kHalf, &tk, bar_kv, 64, kv0, kh, kb);
       tma_load_4d(sV, &tv, bar_kv, 0, kv0, v_h, vb);
       tma_load_4d(sV + kHalf, &tv, bar_kv, 64, kv0, v_h, vb);
-      pdl_wait();                                          // the statistics come from the kernel before; q, k, v and dO do not
+      pdl_wait();                                          // the statistics come from the kernel before; K and V do not
       for (int it = 0; it < n_iter; ++it) {
         const int qs = it % kQStages;
         const uint32_t ph = (uint32_t)((it / kQStages) & 1);
@@ -1073,7 +1073,7 @@ void flash_attn_bwd(const void* go, const void* q, const void* k, const void* v,
   if (det) NXD_CUDA_CHECK(cudaMemsetAsync(turnstile, 0, (size_t)B * H * flash_attn_bwd_query_tiles(S_q) * sizeof(unsigned), st));
   {
     const long rows = (long)B * H * S_pad;
-    // an ordinary launch: the main kernel reads q, k, v and dO before it waits for this one, so they have to be there when this one starts
+    // an ordinary launch: the main kernel loads K and V before it waits for this one, so they have to be there when this one starts
     fa_bwd_prep_kernel<<<(unsigned)((rows + 15) / 16), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)go, lse, dlse, stats,
                                                                      dq_acc, p.stats_stride, B, S_q, H, S_pad, os[0], os[1], os[2], gs[0],
                                                                      gs[1], gs[2], scale);

@@ -56,7 +56,7 @@ _EXT_PURE = frozenset({"rmsnorm_fwd", "rmsnorm_bwd", "add_rmsnorm_fwd", "add_rms
                        "moe_combine_grad", "row_argmax", "row_topk", "flash_attn_fwd",
                        "flash_attn_bwd", "flash_attn_bwd_parts", "moe_block_tkg_supported", "row_topk_supported", "grouped_gemm"})
 # … and the ones that write exactly these positional arguments (everything else they take is read-only)
-_EXT_WRITES = {"gemm_bf16": (2,), "gemm_bf16_2cta": (2,), "gemm_fp8": (2,), "grouped_wgrad": (2,), "decode_rope_kv": (6, 7), "prefill_rope_kv": (5, 6),
+_EXT_WRITES = {"gemm_bf16": (2,), "gemm_bf16_2cta": (2,), "gemm_fp8": (2,), "grouped_wgrad": (2,), "decode_rope_kv": (6, 7),
                "multi_tensor_sq_norm": (1,), "embedding_grad": (2,), "grad_to_buffer": (1,)}
 
 
