@@ -113,3 +113,39 @@ def test_a_sequence_does_not_see_its_neighbours(order, seq):
             assert (a[0].double() - b.double()).abs().max() <= 2.0 ** -7 * b.double().abs().max()
         else:
             assert torch.equal(a[0], b)
+
+
+@pytest.mark.parametrize("seq", [1, 130])
+@pytest.mark.parametrize("form", ["heads repeated", "sequences repeated", "one sequence of a batch", "one head of many", "slices of a projection", "every other row"])
+def test_views_as_their_copies(form, seq):
+    """Strides of 0, of dimensions of one and within a row: the maps give what a dense copy gives, forward and backward."""
+    from neuronx_distributed_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(seq)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+
+    def make(h):
+        if form == "heads repeated":
+            return rnd(2, seq, 1, 128).expand(2, seq, h, 128)
+        if form == "sequences repeated":
+            return rnd(1, seq, h, 128).expand(2, seq, h, 128)
+        if form == "one sequence of a batch":
+            return rnd(3, seq + 5, h, 128)[1:2, 2:seq + 2]
+        if form == "one head of many":
+            return rnd(2, seq, 3 * h, 128)[:, :, 2:3]
+        if form == "slices of a projection":
+            return rnd(seq, 2, (h + 3) * 128)[..., 256:256 + h * 128].unflatten(-1, (h, 128)).transpose(0, 1)
+        return rnd(2, 2 * seq, h, 128)[:, ::2]
+
+    q, k, v, go = make(4), make(2), make(2), make(4)
+    f = ops._ext.ext()
+    res = []
+    for dense in (False, True):
+        a, b, c, d = (t.contiguous() if dense else t for t in (q, k, v, go))
+        o, lse = f.flash_attn_fwd(a, b, c, True, 128 ** -0.5, True)
+        res.append([o, lse, *f.flash_attn_bwd(d, a, b, c, o, lse, True, 128 ** -0.5, True, None, 1)])
+    for i, (a, b) in enumerate(zip(*res)):
+        if i == 2:                                         # dQ: sums over K/V tiles arrive in any order: fp32, then one rounding to bf16
+            assert (a.double() - b.double()).abs().max() <= 2.0 ** -7 * b.double().abs().max()
+        else:
+            assert torch.equal(a, b)
