@@ -36,17 +36,34 @@ constexpr uint32_t kTile = BM * HD * 2;          // 32 KB
 constexpr uint32_t kHalf = kTile / 2;            // one [128 × 64] box
 constexpr uint32_t kSmemFwd = (2 + kRing) * kTile + 1024 /*align*/ + 512 /*barriers*/;
 
-// Warp-uniform issue: the whole MMA warp runs the issue loop in convergent control flow and one elected lane executes each
-// tcgen05 instruction (helpers tcgen05_mma_f16_e / tcgen05_commit_e in sm100_ptx.cuh explain why; mma_ts is the variant whose
-// A operand is read from TMEM — P of the forward, Pᵀ of the backward).
-NXD_DEVICE void mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "elect.sync _|q, 0xffffffff;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
+// Warp-uniform issue: the whole MMA warp runs the issue loop in convergent control flow and one elected lane executes the tcgen05
+// instructions (sm100_ptx.cuh explains why).  One election serves the products of a whole tile and the barrier they complete; descriptors
+// advance by constants.  With an election, a predicate and a new descriptor for each product the issuing warp was what a backward step
+// waited for: 32 products of 32 to 64 cycles took it 2200 cycles.
+#define NXD_FA_MMA "@q tcgen05.mma.cta_group::1.kind::f16 "
+#define NXD_FA_BEGIN                                                                                                     \
+  "{\n\t.reg .pred p, q, t;\n\t.reg .b64 a, b;\n\t.reg .b32 c;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t" \
+  "setp.eq.b32 t, 0, 0;\n\t"
+#define NXD_FA_COMMIT(bar) "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [" bar "];\n\t"
+#define NXD_FA_SS(ia, ib) "add.s64 a, %1, " ia ";\n\tadd.s64 b, %2, " ib ";\n\t" NXD_FA_MMA "[%0], a, b, %3, t;\n\t"
+#define NXD_FA_TS(ia, ib) "add.u32 c, %1, " ia ";\n\tadd.s64 b, %2, " ib ";\n\t" NXD_FA_MMA "[%0], [c], b, %3, t;\n\t"
+// Eight products over 128 elements of K, both operands in shared memory; product i reads (i / 4) * 4 and (i % 4) * 1 steps (of 16 bytes) on.
+template <int A4, int A1, int B4, int B1>
+NXD_DEVICE void mma_ss8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate, uint32_t bar) {
+  asm volatile(NXD_FA_BEGIN NXD_FA_MMA "[%0], %1, %2, %3, p;\n\t"
+               NXD_FA_SS("%6", "%13") NXD_FA_SS("%7", "%14") NXD_FA_SS("%8", "%15") NXD_FA_SS("%9", "%16") NXD_FA_SS("%10", "%17")
+               NXD_FA_SS("%11", "%18") NXD_FA_SS("%12", "%19") NXD_FA_COMMIT("%5") "}"
+               ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(bar),
+                 "n"(A1), "n"(2 * A1), "n"(3 * A1), "n"(A4), "n"(A4 + A1), "n"(A4 + 2 * A1), "n"(A4 + 3 * A1),
+                 "n"(B1), "n"(2 * B1), "n"(3 * B1), "n"(B4), "n"(B4 + B1), "n"(B4 + 2 * B1), "n"(B4 + 3 * B1)
+               : "memory");
+}
+// Four products over 64 elements of K, A in TMEM (P of the forward, Pᵀ and dSᵀ of the backward); the last two read A from A2 columns on.
+template <int A2, int B1>
+NXD_DEVICE void mma_ts4(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(NXD_FA_BEGIN NXD_FA_MMA "[%0], [%1], %2, %3, p;\n\t" NXD_FA_TS("8", "%5") NXD_FA_TS("%8", "%6") NXD_FA_TS("%9", "%7") "}"
+               ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate), "n"(B1), "n"(2 * B1), "n"(3 * B1), "n"(A2), "n"(A2 + 8)
+               : "memory");
 }
 NXD_DEVICE void tcgen05_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -71,7 +88,15 @@ NXD_DEVICE void tcgen05_st_32x16p(uint32_t taddr, const uint32_t* r) {   // firs
 }
 NXD_DEVICE void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 NXD_DEVICE void tcgen05_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+NXD_DEVICE void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+NXD_DEVICE void bulk_wait_read1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
+NXD_DEVICE void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 NXD_DEVICE uint64_t pack2u(uint32_t a, uint32_t b) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b)); return r; }
+NXD_DEVICE float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 NXD_DEVICE uint32_t pack_bf16(float lo, float hi) {
   uint32_t r;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
@@ -252,13 +277,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
       mbar_wait(bar_kvf + 8 * slot, (uint32_t)((pos / kRing) & 1));
       tcgen05_fence_after();
       const uint32_t q_s = sQ + tq_ * kTile, k_s = sKV + slot * kTile;
-#pragma unroll
-      for (int kb = 0; kb < 2; ++kb)
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-          tcgen05_mma_f16_e(tmem_S + t * BN, make_smem_desc(q_s + kb * kHalf + kk * 32, 16, 1024),
-                 make_smem_desc(k_s + kb * kHalf + kk * 32, 16, 1024), idesc_s, (kb | kk) ? 1u : 0u);
-      tcgen05_commit_e(bar_s + 8 * t);
+      mma_ss8<kHalf / 16, 2, kHalf / 16, 2>(tmem_S + t * BN, make_smem_desc(q_s, 16, 1024), make_smem_desc(k_s, 16, 1024), idesc_s, 0u, bar_s + 8 * t);
       if (last_k) tcgen05_commit_e(bar_kve + 8 * slot);
       if (last && !p.split) tcgen05_commit_e(bar_qe + 8 * t);
     };
@@ -290,9 +309,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
             for (int h = 0; h < 2; ++h) {
               mbar_wait((h ? bar_pb : bar_pa) + 8 * t, ph);
               tcgen05_fence_after();
-#pragma unroll
-              for (int k = h * 4; k < h * 4 + 4; ++k)
-                mma_ts(tmem_O + t * HD, tmem_S + t * BN + k * 8, make_smem_desc(v_s + k * 2048, kHalf, 1024), idesc_o, (j | k) ? 1u : 0u);
+              mma_ts4<16, 128>(tmem_O + t * HD, tmem_S + t * BN + h * 32, make_smem_desc(v_s + h * 8192, kHalf, 1024), idesc_o, (j | h) ? 1u : 0u);
             }
             if (p.split || t == 1 || j >= it.n1) tcgen05_commit_e(bar_kve + 8 * slot);
             if (j == nt - 1) tcgen05_commit_e(bar_of + 8 * t);
@@ -346,9 +363,9 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
         }
         float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
+        for (int i = 0; i < 32; i += 2)
 #pragma unroll
-          for (int c = 0; c < 4; ++c) mx4[c] = fmaxf(mx4[c], __uint_as_float(sr[c][i]));
+          for (int c = 0; c < 4; ++c) mx4[c] = max3(mx4[c], __uint_as_float(sr[c][i]), __uint_as_float(sr[c][i + 1]));
         const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
         if (j == 0) {
           m_ref = mx;
@@ -473,16 +490,20 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
 //   dPᵀ = V·dOᵀ       (A = V  K-major, B = dO K-major)            → TMEM [128 kv × 64 q]
 //   Pᵀ = exp2(Sᵀ·c − lse₂[q]) ;  dSᵀ = Pᵀ ∘ (dPᵀ·scale − δ[q]·scale)   (thread = kv row; lse₂/δ broadcast from smem)
 //   dV += Pᵀ·dO       (A = Pᵀ from TMEM (in place over Sᵀ), B = dO MN-major)
-//   dK += dSᵀ·Q       (A = dSᵀ smem K-major,               B = Q  MN-major)
+//   dK += dSᵀ·Q       (A = dSᵀ from TMEM (over dPᵀ),       B = Q  MN-major)
 //   dQᵀ = Kᵀ·dSᵀ      (A = K MN-major, B = dSᵀ MN-major)          → TMEM [128 d × 64 q], drained by a second warpgroup
 //                      into smem and added to the fp32 dQ accumulator with one bulk async reduce (no per-element atomics).
-// warp 0 TMA, warp 1 MMA issue, warps 2-5 softmax/dS (+ dK/dV epilogue), warps 6-9 dQ drain.
+// warp 0 TMA, warp 1 MMA issue, warps 2-5 and 6-9 softmax/dS of the first and last 32 query columns (+ dK / dV epilogue), warps 10-13 dQ drain.
+// A step of one query tile takes about 1850 cycles: its products 1660 (1280 of mathematics; operands of 64 columns are read from shared memory
+// faster than they are used), the softmax chain of a step about as long.  One softmax warpgroup (64 exponentials a thread) made it 2070, and
+// one 16 KB stage for the sums of dQ, which the drain waited for, 2250.  Start and end of a block are 10 thousand cycles more, two thirds of
+// them the stores of dK and dV at 32 bytes a cycle and SM beside the last sums of dQ.  Main kernel, 1 x 2048 tokens, 32 heads: 116 us then, 88 now.
 constexpr int BQ = 64;
-constexpr int kThreadsBwd = 320;
+constexpr int kThreadsBwd = 448;
 constexpr int kQStages = 3;
 constexpr uint32_t kQTile = BQ * HD * 2;                        // 16 KB
 constexpr uint32_t kOffK = 0, kOffV = kTile, kOffQ = 2 * kTile, kOffdO = kOffQ + kQStages * kQTile,
-                   kOffdS = kOffdO + kQStages * kQTile, kOffdQ = kOffdS + 2 * kQTile, kOffStats = kOffdQ + 16384,
+                   kOffdS = kOffdO + kQStages * kQTile, kOffdQ = kOffdS + 2 * kQTile, kOffStats = kOffdQ + 2 * 16384,
                    kOffBars = kOffStats + kQStages * 512;
 constexpr uint32_t kSmemBwd = kOffBars + 256 + 1024;
 
@@ -509,9 +530,6 @@ NXD_DEVICE void bulk_reduce_add_f32(void* gdst, uint32_t smem_src, uint32_t byte
   asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;"
                ::"l"(gdst), "r"(smem_src), "r"(bytes) : "memory");
 }
-NXD_DEVICE void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-NXD_DEVICE void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-NXD_DEVICE void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 NXD_DEVICE void named_bar(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 
 // Softmax-side math of one backward tile, split in two phases so the exp work (needs only Sᵀ, which the tensor pipe delivered a
@@ -521,62 +539,52 @@ NXD_DEVICE void named_bar(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"
 // The stats rows hold −lse·log2e and −δ·scale so both affine steps are single packed FMAs; MASKED is a template parameter so
 // the common tile has no per-element branches or selects.
 template <bool MASKED>
-NXD_DEVICE void bwd_p_math(uint32_t (&sv)[2][32], float (&pf)[2][32], uint32_t stats_s, float sl2, int kv, int q0, int S_q,
-                           int S_kv, int causal) {
+NXD_DEVICE void bwd_p_math(uint32_t (&sv)[32], float (&pf)[32], uint32_t stats_s, float sl2, int kv, int q0, int S_q, int S_kv, int causal) {
   const uint64_t sl2_2 = pack2(sl2, sl2);
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
+  for (int i = 0; i < 32; i += 4) {
+    float4 l2;
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(l2.x), "=f"(l2.y), "=f"(l2.z), "=f"(l2.w) : "r"(stats_s + i * 4));
+    const uint64_t nl2[2] = {pack2(l2.x, l2.y), pack2(l2.z, l2.w)};
 #pragma unroll
-    for (int i = 0; i < 32; i += 4) {
-      float4 l2;
-      asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(l2.x), "=f"(l2.y), "=f"(l2.z), "=f"(l2.w)
-                   : "r"(stats_s + (h * 32 + i) * 4));
-      const uint64_t nl2[2] = {pack2(l2.x, l2.y), pack2(l2.z, l2.w)};
-#pragma unroll
-      for (int e2 = 0; e2 < 2; ++e2) {
-        float x0, x1;
-        unpack2(fma2(pack2u(sv[h][i + 2 * e2], sv[h][i + 2 * e2 + 1]), sl2_2, nl2[e2]), x0, x1);
-        float p0 = ex2(x0), p1 = ex2(x1);
-        if constexpr (MASKED) {
-          const int q = q0 + h * 32 + i + 2 * e2;
-          p0 = (kv < S_kv && q < S_q && (!causal || kv <= q)) ? p0 : 0.f;          // selects; also kills NaN padding
-          p1 = (kv < S_kv && q + 1 < S_q && (!causal || kv <= q + 1)) ? p1 : 0.f;
-        }
-        pf[h][i + 2 * e2] = p0;
-        pf[h][i + 2 * e2 + 1] = p1;
+    for (int e2 = 0; e2 < 2; ++e2) {
+      float x0, x1;
+      unpack2(fma2(pack2u(sv[i + 2 * e2], sv[i + 2 * e2 + 1]), sl2_2, nl2[e2]), x0, x1);
+      float p0 = ex2(x0), p1 = ex2(x1);
+      if constexpr (MASKED) {
+        const int q = q0 + i + 2 * e2;
+        p0 = (kv < S_kv && q < S_q && (!causal || kv <= q)) ? p0 : 0.f;          // selects; also kills NaN padding
+        p1 = (kv < S_kv && q + 1 < S_q && (!causal || kv <= q + 1)) ? p1 : 0.f;
       }
-      sv[h][i >> 1] = pack_bf16(pf[h][i], pf[h][i + 1]);
-      sv[h][(i >> 1) + 1] = pack_bf16(pf[h][i + 2], pf[h][i + 3]);
+      pf[i + 2 * e2] = p0;
+      pf[i + 2 * e2 + 1] = p1;
     }
+    sv[i >> 1] = pack_bf16(pf[i], pf[i + 1]);
+    sv[(i >> 1) + 1] = pack_bf16(pf[i + 2], pf[i + 3]);
   }
 }
 
 template <bool MASKED>
-NXD_DEVICE void bwd_ds_math(uint32_t (&dpv)[2][32], const float (&pf)[2][32], uint32_t stats_s, float sc) {
+NXD_DEVICE void bwd_ds_math(uint32_t (&dpv)[32], const float (&pf)[32], uint32_t stats_s, float sc) {
   const uint64_t sc_2 = pack2(sc, sc);
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
+  for (int i = 0; i < 32; i += 4) {
+    float4 dl;
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(dl.x), "=f"(dl.y), "=f"(dl.z), "=f"(dl.w) : "r"(stats_s + 256 + i * 4));
+    const uint64_t ndl[2] = {pack2(dl.x, dl.y), pack2(dl.z, dl.w)};
+    float dsv[4];
 #pragma unroll
-    for (int i = 0; i < 32; i += 4) {
-      float4 dl;
-      asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(dl.x), "=f"(dl.y), "=f"(dl.z), "=f"(dl.w)
-                   : "r"(stats_s + 256 + (h * 32 + i) * 4));
-      const uint64_t ndl[2] = {pack2(dl.x, dl.y), pack2(dl.z, dl.w)};
-      float dsv[4];
-#pragma unroll
-      for (int e2 = 0; e2 < 2; ++e2) {
-        float d0, d1;
-        unpack2(mul2(pack2(pf[h][i + 2 * e2], pf[h][i + 2 * e2 + 1]),
-                     fma2(pack2u(dpv[h][i + 2 * e2], dpv[h][i + 2 * e2 + 1]), sc_2, ndl[e2])), d0, d1);
-        if constexpr (MASKED) {          // P is already exactly 0 where masked, but 0·NaN (padding garbage) must not leak
-          d0 = pf[h][i + 2 * e2] == 0.f ? 0.f : d0;
-          d1 = pf[h][i + 2 * e2 + 1] == 0.f ? 0.f : d1;
-        }
-        dsv[2 * e2] = d0; dsv[2 * e2 + 1] = d1;
+    for (int e2 = 0; e2 < 2; ++e2) {
+      float d0, d1;
+      unpack2(mul2(pack2(pf[i + 2 * e2], pf[i + 2 * e2 + 1]), fma2(pack2u(dpv[i + 2 * e2], dpv[i + 2 * e2 + 1]), sc_2, ndl[e2])), d0, d1);
+      if constexpr (MASKED) {            // P is already exactly 0 where masked, but 0·NaN (padding garbage) must not leak
+        d0 = pf[i + 2 * e2] == 0.f ? 0.f : d0;
+        d1 = pf[i + 2 * e2 + 1] == 0.f ? 0.f : d1;
       }
-      dpv[h][i >> 1] = pack_bf16(dsv[0], dsv[1]);
-      dpv[h][(i >> 1) + 1] = pack_bf16(dsv[2], dsv[3]);
+      dsv[2 * e2] = d0; dsv[2 * e2 + 1] = d1;
     }
+    dpv[i >> 1] = pack_bf16(dsv[0], dsv[1]);
+    dpv[(i >> 1) + 1] = pack_bf16(dsv[2], dsv[3]);
   }
 }
 
@@ -594,8 +602,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t sK = base + kOffK, sV = base + kOffV, sQ = base + kOffQ, sdO = base + kOffdO, sdS = base + kOffdS,
                  sdQ = base + kOffdQ, sStats = base + kOffStats, bars = base + kOffBars;
-  // barriers: kv | qf[3] | qe[3] | s[2] | dp | p | dq | dqr | acc | tmem slot
-  const uint32_t bar_kv = bars, bar_qf = bars + 8, bar_qe = bars + 32, bar_s = bars + 56, bar_dp = bars + 72,
+  // barriers: k | qf[3] | qe[3] | s[2] | dp | p | dq | dqr | acc | v | tmem slot
+  const uint32_t bar_k = bars, bar_v = bars + 112, bar_qf = bars + 8, bar_qe = bars + 32, bar_s = bars + 56, bar_dp = bars + 72,
                  bar_p = bars + 80, bar_dq = bars + 88, bar_dqr = bars + 96, bar_acc = bars + 104, tmem_slot = bars + 128;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Blocks start heaviest first (causal: the first K/V tiles see the most query tiles) within groups of heads that share L2: head by
@@ -619,12 +627,28 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
   const int kv0 = n * BN;
 
   if (threadIdx.x == 0) {
-    mbar_init(bar_kv, 1);
+    mbar_init(bar_k, 1); mbar_init(bar_v, 1);
     for (int i = 0; i < kQStages; ++i) { mbar_init(bar_qf + 8 * i, 1); mbar_init(bar_qe + 8 * i, 1); }
     mbar_init(bar_s, 1); mbar_init(bar_s + 8, 1);
-    mbar_init(bar_dp, 1); mbar_init(bar_p, 128); mbar_init(bar_dq, 1); mbar_init(bar_dqr, 128);
+    mbar_init(bar_dp, 1); mbar_init(bar_p, 256); mbar_init(bar_dq, 1); mbar_init(bar_dqr, 128);
     mbar_init(bar_acc, 1);
     fence_barrier_init();
+    // K, V and the first tile of Q and dO are on their way while the tensor memory is allocated; what the kernel before this one writes (the
+    // statistics) is not among them
+    if (n_iter > 0) {
+      const int kh = kvh * p.k.h, kb = b * p.k.b, v_h = kvh * p.v.h, vb = b * p.v.b, head = vh * group;
+      mbar_expect_tx(bar_k, kTile);
+      tma_load_4d(sK, &tk, bar_k, 0, kv0, kh, kb);
+      tma_load_4d(sK + kHalf, &tk, bar_k, 64, kv0, kh, kb);
+      mbar_expect_tx(bar_qf, 2 * kQTile + 512);
+      tma_load_4d(sQ, &tq, bar_qf, 0, t0 * BQ, head * p.q.h, b * p.q.b);
+      tma_load_4d(sQ + kQTile / 2, &tq, bar_qf, 64, t0 * BQ, head * p.q.h, b * p.q.b);
+      mbar_expect_tx(bar_v, kTile);
+      tma_load_4d(sV, &tv, bar_v, 0, kv0, v_h, vb);
+      tma_load_4d(sV + kHalf, &tv, bar_v, 64, kv0, v_h, vb);
+      tma_load_4d(sdO, &tg, bar_qf, 0, t0 * BQ, head * p.g.h, b * p.g.b);
+      tma_load_4d(sdO + kQTile / 2, &tg, bar_qf, 64, t0 * BQ, head * p.g.h, b * p.g.b);
+    }
   }
   if (warp == 1) {
     tcgen05_alloc(tmem_slot, 512);
@@ -642,26 +666,21 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
 
   if (warp == 0) {
     if (lane == 0 && n_iter > 0) {
-      prefetch_tmap(&tq); prefetch_tmap(&tk); prefetch_tmap(&tv); prefetch_tmap(&tg);
-      const int kh = kvh * p.k.h, kb = b * p.k.b, v_h = kvh * p.v.h, vb = b * p.v.b;
-      mbar_expect_tx(bar_kv, 2 * kTile);
-      tma_load_4d(sK, &tk, bar_kv, 0, kv0, kh, kb);
-      tma_load_4d(sK + kHalf, &tk, bar_kv, 64, kv0, kh, kb);
-      tma_load_4d(sV, &tv, bar_kv, 0, kv0, v_h, vb);
-      tma_load_4d(sV + kHalf, &tv, bar_kv, 64, kv0, v_h, vb);
-      pdl_wait();                                          // the statistics come from the kernel before; K and V do not
+      pdl_wait();                                          // the statistics come from the kernel before
       for (int it = 0; it < n_iter; ++it) {
         const int qs = it % kQStages;
         const uint32_t ph = (uint32_t)((it / kQStages) & 1);
         const int head = vh * group + it / per_head, t = t0 + it % per_head;
-        mbar_wait(bar_qe + 8 * qs, ph ^ 1);
         const uint32_t full = bar_qf + 8 * qs;
-        mbar_expect_tx(full, 2 * kQTile + 512);
-        const int qh = head * p.q.h, qb = b * p.q.b, gh = head * p.g.h, gb = b * p.g.b;
-        tma_load_4d(sQ + qs * kQTile, &tq, full, 0, t * BQ, qh, qb);
-        tma_load_4d(sQ + qs * kQTile + kQTile / 2, &tq, full, 64, t * BQ, qh, qb);
-        tma_load_4d(sdO + qs * kQTile, &tg, full, 0, t * BQ, gh, gb);
-        tma_load_4d(sdO + qs * kQTile + kQTile / 2, &tg, full, 64, t * BQ, gh, gb);
+        if (it > 0) {
+          mbar_wait(bar_qe + 8 * qs, ph ^ 1);
+          mbar_expect_tx(full, 2 * kQTile + 512);
+          const int qh = head * p.q.h, qb = b * p.q.b, gh = head * p.g.h, gb = b * p.g.b;
+          tma_load_4d(sQ + qs * kQTile, &tq, full, 0, t * BQ, qh, qb);
+          tma_load_4d(sQ + qs * kQTile + kQTile / 2, &tq, full, 64, t * BQ, qh, qb);
+          tma_load_4d(sdO + qs * kQTile, &tg, full, 0, t * BQ, gh, gb);
+          tma_load_4d(sdO + qs * kQTile + kQTile / 2, &tg, full, 64, t * BQ, gh, gb);
+        }
         const float* st = p.stats + ((long)b * p.H + head) * p.S_pad + t * BQ;
         bulk_load_1d(sStats + qs * 512, st, 256, full);
         bulk_load_1d(sStats + qs * 512 + 256, st + p.stats_stride, 256, full);
@@ -673,164 +692,153 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
       constexpr uint32_t idesc_s = make_idesc(false, false, 128, BQ);      // Sᵀ, dPᵀ
       constexpr uint32_t idesc_acc = make_idesc(false, true, 128, HD);     // dK, dV
       constexpr uint32_t idesc_dq = make_idesc(true, true, 128, BQ);       // dQᵀ
-      mbar_wait(bar_kv, 0);
+      mbar_wait(bar_k, 0);
       // Issue order per iteration `it` (everything on the tensor pipe retires in this order):
-      //   … Sᵀ_{it+1} already issued …  | wait softmax(it) | dPᵀ_{it+1} | dK_it dV_it | dQᵀ_it | Sᵀ_{it+2}
+      //   … Sᵀ_{it+1} already issued …  | wait softmax(it) | dK_it | dPᵀ_{it+1} | dV_it | dQᵀ_it | Sᵀ_{it+2}
       // so while the softmax warps work on tile it+1 the pipe runs dK/dV/dQ of tile it and Sᵀ of tile it+2.
       auto issue_st = [&](int it) {
         const int qs = it % kQStages, st = it & 1;
         mbar_wait(bar_qf + 8 * qs, (uint32_t)((it / kQStages) & 1));
         tcgen05_fence_after();
         const uint32_t q_s = sQ + qs * kQTile;
-#pragma unroll
-        for (int kb = 0; kb < 2; ++kb)
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            tcgen05_mma_f16_e(tmem_ST + st * BQ, make_smem_desc(sK + kb * kHalf + kk * 32, 16, 1024),
-                            make_smem_desc(q_s + kb * (kQTile / 2) + kk * 32, 16, 1024), idesc_s, (kb | kk) ? 1u : 0u);
-        tcgen05_commit_e(bar_s + 8 * st);
+        mma_ss8<kHalf / 16, 2, kQTile / 32, 2>(tmem_ST + st * BQ, make_smem_desc(sK, 16, 1024), make_smem_desc(q_s, 16, 1024), idesc_s, 0u, bar_s + 8 * st);
       };
       auto issue_dp = [&](int it) {
         const int qs = it % kQStages;
         mbar_wait(bar_qf + 8 * qs, (uint32_t)((it / kQStages) & 1));
         tcgen05_fence_after();
         const uint32_t g_s = sdO + qs * kQTile;
-#pragma unroll
-        for (int kb = 0; kb < 2; ++kb)
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            tcgen05_mma_f16_e(tmem_dP, make_smem_desc(sV + kb * kHalf + kk * 32, 16, 1024),
-                            make_smem_desc(g_s + kb * (kQTile / 2) + kk * 32, 16, 1024), idesc_s, (kb | kk) ? 1u : 0u);
-        tcgen05_commit_e(bar_dp);
+        mma_ss8<kHalf / 16, 2, kQTile / 32, 2>(tmem_dP, make_smem_desc(sV, 16, 1024), make_smem_desc(g_s, 16, 1024), idesc_s, 0u, bar_dp);
       };
       issue_st(0);
+      mbar_wait(bar_v, 0);
       issue_dp(0);
       if (n_iter > 1) issue_st(1);
       for (int it = 0; it < n_iter; ++it) {
         const int qs = it % kQStages, st = it & 1;
-        mbar_wait(bar_p, (uint32_t)(it & 1));             // Pᵀ_it in TMEM, dSᵀ_it in smem, dPᵀ region consumed
+        mbar_wait(bar_p, (uint32_t)(it & 1));             // Pᵀ_it over Sᵀ_it, dSᵀ_it over dPᵀ_it in TMEM and in smem
         tcgen05_fence_after();
-        if (it + 1 < n_iter) issue_dp(it + 1);
         const uint32_t q_s = sQ + qs * kQTile, g_s = sdO + qs * kQTile, ds_s = sdS + st * kQTile;
-#pragma unroll
-        for (int kk = 0; kk < BQ / 16; ++kk)
-          tcgen05_mma_f16_e(tmem_dK, make_smem_desc(ds_s + kk * 32, 16, 1024), make_smem_desc(q_s + kk * 2048, kQTile / 2, 1024),
-                          idesc_acc, (it | kk) ? 1u : 0u);
-#pragma unroll
-        for (int kk = 0; kk < BQ / 16; ++kk)
-          mma_ts(tmem_dV, tmem_ST + st * BQ + kk * 8, make_smem_desc(g_s + kk * 2048, kQTile / 2, 1024), idesc_acc,
-                         (it | kk) ? 1u : 0u);
+        mma_ts4<32, 128>(tmem_dK, tmem_dP, make_smem_desc(q_s, kQTile / 2, 1024), idesc_acc, it ? 1u : 0u);
+        if (it + 1 < n_iter) issue_dp(it + 1);            // over dSᵀ_it: behind dK_it in pipe order
+        mma_ts4<32, 128>(tmem_dV, tmem_ST + st * BQ, make_smem_desc(g_s, kQTile / 2, 1024), idesc_acc, it ? 1u : 0u);
         tcgen05_commit_e(bar_qe + 8 * qs);
         if (it >= 1) {
           mbar_wait(bar_dqr, (uint32_t)((it - 1) & 1));   // dQᵀ_{it-1} has been read out of TMEM
           tcgen05_fence_after();
         }
-#pragma unroll
-        for (int kk = 0; kk < BN / 16; ++kk)
-          tcgen05_mma_f16_e(tmem_dQ, make_smem_desc(sK + kk * 2048, kHalf, 1024), make_smem_desc(ds_s + kk * 2048, kHalf, 1024),
-                          idesc_dq, kk ? 1u : 0u);
-        tcgen05_commit_e(bar_dq);
+        mma_ss8<512, 128, 512, 128>(tmem_dQ, make_smem_desc(sK, kHalf, 1024), make_smem_desc(ds_s, kHalf, 1024), idesc_dq, 0u, bar_dq);
         if (it + 2 < n_iter) issue_st(it + 2);            // overwrites Pᵀ_it — after dV_it in pipe order
       }
       tcgen05_commit_e(bar_acc);
     }
     __syncwarp();
-  } else if (warp < 6) {
-    // ===== softmax / dS warps: thread = kv row =====
-    const int quarter = warp & 3;
+  } else if (warp < 10) {
+    // ===== softmax / dS warps: thread = kv row, 32 of the tile's query columns =====
+    const int quarter = warp & 3, wg = (warp - 2) >> 2;
     const int row = quarter * 32 + lane;
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     const int kv = kv0 + row;
     const float sl2 = p.scale_log2, sc = p.scale;
+    int qs = 0, t = t0;
+    uint32_t ph = 0;
     for (int it = 0; it < n_iter; ++it) {
-      const int qs = it % kQStages, st = it & 1;
-      const int t = t0 + it % per_head;
+      const int st = it & 1;
       const int q0 = t * BQ;
-      mbar_wait(bar_qf + 8 * qs, (uint32_t)((it / kQStages) & 1));     // stats (TMA-written) visible to this thread
+      const uint32_t tS = tmem_ST + st * BQ + wg * 32 + lane_base, tdP = tmem_dP + wg * 32 + lane_base;
+      mbar_wait(bar_qf + 8 * qs, ph);                                  // stats (TMA-written) visible to this thread
       mbar_wait(bar_s + 8 * st, (uint32_t)((it >> 1) & 1));
       tcgen05_fence_after();
       const bool masked = (p.causal && q0 < kv0 + BN - 1) || (q0 + BQ > p.S_q) || (kv0 + BN > p.S_kv);
-      const uint32_t stats_s = sStats + qs * 512;
+      const uint32_t stats_s = sStats + qs * 512 + wg * 128;
       const uint32_t ds_row = sdS + st * kQTile + row * 128;
-      // ---- phase 1 (needs only Sᵀ): Pᵀ, written back over Sᵀ in TMEM
-      uint32_t sv[2][32];
-      float pf[2][32];
-      tcgen05_ld_32x32(tmem_ST + st * BQ + lane_base, sv[0]);
-      tcgen05_ld_32x32(tmem_ST + st * BQ + lane_base + 32, sv[1]);
+      // ---- phase 1 (needs only Sᵀ): Pᵀ, written back over Sᵀ in TMEM (each half over its own columns)
+      uint32_t sv[32];
+      float pf[32];
+      tcgen05_ld_32x32(tS, sv);
       tcgen05_wait_ld();
-      if (masked) bwd_p_math<true>(sv, pf, stats_s, sl2, kv, q0, p.S_q, p.S_kv, p.causal);
-      else bwd_p_math<false>(sv, pf, stats_s, sl2, kv, q0, p.S_q, p.S_kv, p.causal);
-      tcgen05_st_32x16p(tmem_ST + st * BQ + lane_base, sv[0]);
-      tcgen05_st_32x16p(tmem_ST + st * BQ + lane_base + 16, sv[1]);
-      // ---- phase 2 (dPᵀ of this tile was issued while phase 1 ran): dSᵀ → smem
+      if (masked) bwd_p_math<true>(sv, pf, stats_s, sl2, kv, q0 + wg * 32, p.S_q, p.S_kv, p.causal);
+      else bwd_p_math<false>(sv, pf, stats_s, sl2, kv, q0 + wg * 32, p.S_q, p.S_kv, p.causal);
+      tcgen05_st_32x16p(tS, sv);
+      // ---- phase 2 (dPᵀ of this tile was issued while phase 1 ran): dSᵀ → TMEM and smem
       mbar_wait(bar_dp, (uint32_t)(it & 1));
       tcgen05_fence_after();
-      uint32_t dpv[2][32];
-      tcgen05_ld_32x32(tmem_dP + lane_base, dpv[0]);
-      tcgen05_ld_32x32(tmem_dP + lane_base + 32, dpv[1]);
+      uint32_t dpv[32];
+      tcgen05_ld_32x32(tdP, dpv);
       tcgen05_wait_ld();
       if (masked) bwd_ds_math<true>(dpv, pf, stats_s, sc);
       else bwd_ds_math<false>(dpv, pf, stats_s, sc);
+      tcgen05_st_32x16p(tdP, dpv);
+      // dSᵀ row → smem, 128B-swizzled: 16-byte chunk c of row r lives at chunk (c ^ (r & 7))
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        // dSᵀ row → smem, 128B-swizzled: 16-byte chunk c of row r lives at chunk (c ^ (r & 7))
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const uint32_t chunk = (uint32_t)(h * 4 + c) ^ (uint32_t)(row & 7);
-          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(ds_row + chunk * 16), "r"(dpv[h][c * 4]),
-                       "r"(dpv[h][c * 4 + 1]), "r"(dpv[h][c * 4 + 2]), "r"(dpv[h][c * 4 + 3]) : "memory");
-        }
+      for (int c = 0; c < 4; ++c) {
+        const uint32_t chunk = (uint32_t)(wg * 4 + c) ^ (uint32_t)(row & 7);
+        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(ds_row + chunk * 16), "r"(dpv[c * 4]),
+                     "r"(dpv[c * 4 + 1]), "r"(dpv[c * 4 + 2]), "r"(dpv[c * 4 + 3]) : "memory");
       }
       tcgen05_wait_st();
       fence_async_smem();
       tcgen05_fence_before();
       mbar_arrive(bar_p);
+      if (++qs == kQStages) { qs = 0; ph ^= 1; }
+      if (++t == nq) t = t0;
     }
-    // ---- epilogue: dK, dV
+    // ---- epilogue: dK by the first warpgroup, dV by the second, through the shared memory of K .. dO, which nothing reads any more (bar_acc:
+    //      every product is done), so that a store writes whole rows.  In small loops: unrolled, most of its time went into fetching
+    //      instructions that run once a block.
     if (n_iter > 0) {
       mbar_wait(bar_acc, 0);
       tcgen05_fence_after();
     }
-    const bool row_ok = kv < p.S_kv;
-    __nv_bfloat16* dk_row = dk + (long)b * p.dk_sb + (long)kv * p.dk_ss + (long)kvh * p.dk_sh;
-    __nv_bfloat16* dv_row = dv + (long)b * p.dv_sb + (long)kv * p.dv_ss + (long)kvh * p.dv_sh;
+    // 16-byte chunk c of the warp's row i stands at chunk c ^ (i & 7); rows of 256 bytes of bf16 (a store: two rows) or 512 of fp32 (one)
+    const bool f32 = p.parts > 1;
+    const uint32_t acc = (wg ? tmem_dV : tmem_dK) + lane_base, pitch = f32 ? 512 : 256;
+    const uint32_t stage = sK + wg * 2 * kTile + quarter * 32 * pitch, mine = stage + lane * pitch;
+    const int r0 = kv0 + quarter * 32;
 #pragma unroll 1
-    for (int which = 0; which < 2; ++which) {
-      __nv_bfloat16* orow = which ? dv_row : dk_row;
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t r[32];
-        if (n_iter > 0) {
-          tcgen05_ld_32x32((which ? tmem_dV : tmem_dK) + lane_base + c * 32, r);
-          tcgen05_wait_ld();
-        } else {
+    for (int c = 0; c < 4; ++c) {                          // 32 columns
+      uint32_t r[32];
+      if (n_iter > 0) {
+        tcgen05_ld_32x32(acc + c * 32, r);
+        tcgen05_wait_ld();
+      } else {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) r[i] = 0;
-        }
-        if (row_ok && p.parts > 1) {
-          float* part = p.kv_part + ((((long)which * p.B + b) * heads_v + vh) * p.S_kv + kv) * HD + c * 32;
+        for (int i = 0; i < 32; ++i) r[i] = 0;
+      }
+      if (f32) {
 #pragma unroll
-          for (int v4 = 0; v4 < 8; ++v4)
-            *reinterpret_cast<uint4*>(part + v4 * 4) = make_uint4(r[v4 * 4], r[v4 * 4 + 1], r[v4 * 4 + 2], r[v4 * 4 + 3]);
-        } else if (row_ok) {
+        for (int v4 = 0; v4 < 8; ++v4)
+          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(mine + (((c * 8 + v4) ^ (lane & 7)) * 16)), "r"(r[v4 * 4]), "r"(r[v4 * 4 + 1]),
+                       "r"(r[v4 * 4 + 2]), "r"(r[v4 * 4 + 3]) : "memory");
+      } else {
 #pragma unroll
-          for (int v4 = 0; v4 < 4; ++v4) {
-            uint4 o;
-            o.x = pack_bf16(__uint_as_float(r[v4 * 8 + 0]), __uint_as_float(r[v4 * 8 + 1]));
-            o.y = pack_bf16(__uint_as_float(r[v4 * 8 + 2]), __uint_as_float(r[v4 * 8 + 3]));
-            o.z = pack_bf16(__uint_as_float(r[v4 * 8 + 4]), __uint_as_float(r[v4 * 8 + 5]));
-            o.w = pack_bf16(__uint_as_float(r[v4 * 8 + 6]), __uint_as_float(r[v4 * 8 + 7]));
-            *reinterpret_cast<uint4*>(orow + c * 32 + v4 * 8) = o;
-          }
+        for (int v4 = 0; v4 < 4; ++v4) {
+          uint32_t o[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) o[i] = pack_bf16(__uint_as_float(r[v4 * 8 + 2 * i]), __uint_as_float(r[v4 * 8 + 2 * i + 1]));
+          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(mine + (((c * 4 + v4) ^ (lane & 7)) * 16)), "r"(o[0]), "r"(o[1]), "r"(o[2]),
+                       "r"(o[3]) : "memory");
         }
       }
+    }
+    __syncwarp();
+    const int chunks = f32 ? 32 : 16, c = lane & (chunks - 1), step = 32 / chunks;
+    const long row_bytes = f32 ? HD * 4 : (wg ? p.dv_ss : p.dk_ss) * 2;
+    char* dst = f32 ? (char*)(p.kv_part + ((((long)wg * p.B + b) * heads_v + vh) * p.S_kv + r0) * HD)
+                    : (char*)((wg ? dv + (long)b * p.dv_sb + (long)kvh * p.dv_sh : dk + (long)b * p.dk_sb + (long)kvh * p.dk_sh) + (long)r0 * (row_bytes / 2));
+#pragma unroll 4
+    for (int i = lane / chunks; i < 32; i += step) {
+      uint4 o;
+      asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(o.x), "=r"(o.y), "=r"(o.z), "=r"(o.w)
+                   : "r"(stage + i * pitch + ((c ^ (i & 7)) * 16)) : "memory");
+      if (r0 + i < p.S_kv) *reinterpret_cast<uint4*>(dst + i * row_bytes + c * 16) = o;
     }
   } else {
     // ===== dQ drain warps: thread = head-dim index d (TMEM lane), columns = q =====
     const int quarter = warp & 3;
     const int d = quarter * 32 + lane;
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-    const int tid = threadIdx.x - 192;
+    const int tid = threadIdx.x - 320;
     if (tid == 0) pdl_wait();                              // which zeroes what is added to here
     for (int it = 0; it < n_iter; ++it) {
       const int st = it & 1;
@@ -846,11 +854,11 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
       mbar_arrive(bar_dqr);                     // the MMA warp may overwrite dQᵀ with the next tile right away
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        if (tid == 0) bulk_wait_read0();        // previous bulk reduce has finished reading the staging tile
+        if (tid == 0) bulk_wait_read1();        // the bulk reduce before the last has finished reading its half of the stage
         named_bar(1, 128);
 #pragma unroll
         for (int c = 0; c < 32; ++c)
-          asm volatile("st.shared.b32 [%0], %1;" ::"r"(sdQ + c * 512 + d * 4), "r"(r[h][c]) : "memory");
+          asm volatile("st.shared.b32 [%0], %1;" ::"r"(sdQ + h * 16384 + c * 512 + d * 4), "r"(r[h][c]) : "memory");
         fence_async_smem();
         named_bar(1, 128);
         if (tid == 0) {
@@ -870,7 +878,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
               } while (seen < (unsigned)n);
             }
           }
-          bulk_reduce_add_f32(gdst + (long)h * 32 * HD, sdQ, 16384);
+          bulk_reduce_add_f32(gdst + (long)h * 32 * HD, sdQ + h * 16384, 16384);
           bulk_commit();
           if constexpr (DET) {
             if (h == 1) {                           // both halves of the tile are in memory before the next CTA may add
@@ -1019,12 +1027,12 @@ void flash_attn_fwd(const void* q, const void* k, const void* v, void* out, floa
   NXD_CUDA_CHECK(cudaGetLastError());
 }
 
-// Blocks per KV head.  Unit: one 64-row query tile, about 1.8 us.  A launch lasts as long as its heaviest block, or as the sum of all over
-// the SMs and, since causal blocks differ, a quarter of the heaviest at the end; equal blocks come in whole rounds.  Every part costs
-// three tiles of start and end, and 256 KB of fp32 sums written and read (0.03 over the chip).  Taken where the estimate falls by a
-// twentieth.  The sums are at most twice the fp32 dQ buffer.  Whole backward, caches flushed, one block per KV head and by this rule:
-//   1 x 2048 tokens, 32 heads on 8: 214 and 154 us;  64 on 8: 407 and 290;  1 x 4096, 32 on 2: 1402 and 439;  64 on 8: 1058 and 837;
-//   1 x 512, 32 on 8: 70 and 48;  16 on 1: 192 and 44.  Left whole: 1 x 4096, 32 on 8 (415; two parts 433), 2 x 2048 (255; 294).
+// Blocks per KV head.  Unit: one 64-row query tile, about 1 us.  A launch lasts as long as its heaviest block, or as the sum of all over
+// the SMs and, since causal blocks differ, a quarter of the heaviest at the end; equal blocks come in whole rounds.  Every block costs
+// six tiles of start and end, every part 256 KB of fp32 sums written and read (0.03 over the chip).  Taken where the estimate falls by a
+// twentieth.  The sums are at most twice the fp32 dQ buffer.  Whole backward, caches warm, one block per KV head and by this rule:
+//   1 x 2048 tokens, 32 heads on 8: 162 and 113 us;  64 on 8: 310 and 206;  1 x 4096, 32 on 2: 1058 and 351;  64 on 8: 873 and 704;
+//   1 x 512, 32 on 8: 57 and 35;  16 on 1: 178 and 33.  Left whole: 1 x 4096, 32 on 8 (342; two parts 357), 2 x 2048 (202; 242).
 int flash_attn_bwd_parts(int B, int S_q, int S_kv, int H, int Hkv, bool causal) {
   using namespace fa;
   if (S_q <= 0 || S_kv <= 0 || H < 1 || Hkv < 1 || H % Hkv) return 1;
@@ -1036,10 +1044,10 @@ int flash_attn_bwd_parts(int B, int S_q, int S_kv, int H, int Hkv, bool causal) 
   double best_t = 0;
   for (int parts = 1; parts <= group; ++parts) {
     if (group % parts) continue;
-    const double blocks = (double)tiles * Hkv * B * parts, heavy = (double)nq * (group / parts) + 3;
-    const double all = ((double)steps * H * B + 3 * blocks) / sms;
+    const double blocks = (double)tiles * Hkv * B * parts, heavy = (double)nq * (group / parts) + 6;
+    const double all = ((double)steps * H * B + 6 * blocks) / sms;
     const double waves = causal ? 0 : heavy * std::ceil(blocks / sms);            // equal blocks: whole rounds
-    const double t = std::max({heavy, all + (causal ? heavy / 4 : 0), waves}) + (parts > 1 ? 2 + 0.03 * blocks : 0);
+    const double t = std::max({heavy, all + (causal ? heavy / 4 : 0), waves}) + (parts > 1 ? 0.03 * blocks : 0);
     if (parts == 1 || t < best_t * (best == 1 ? 0.95 : 1.0)) { best = parts; best_t = t; }
   }
   return best;

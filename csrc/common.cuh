@@ -46,8 +46,8 @@ namespace nxd {
 // allocates tensor memory triggers behind the allocation: blocks of a later kernel that hold tensor memory and wait could otherwise keep one of its
 // blocks on the same SM from ever getting its own.
 // Every kernel launched so waits, in at least one thread and before it returns, so that its end is its predecessors' end too; threads read or
-// write what others use only behind that wait.  One exception: fa_bwd_kernel (attention_sm100.cu) loads K and V above it, so the launch in
-// front of it has to be an ordinary one that K and V are older than; its other threads follow its two waiting ones through barriers.  Pointers to what a predecessor wrote are not __restrict__ there: a load through the read-only path must not move above the wait.
+// write what others use only behind that wait.  One exception: fa_bwd_kernel (attention_sm100.cu) loads K, V, Q and dO above it, so the launch in
+// front of it has to be an ordinary one that they are older than; its other threads follow its two waiting ones through barriers.  Pointers to what a predecessor wrote are not __restrict__ there: a load through the read-only path must not move above the wait.
 NXD_DEVICE void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 NXD_DEVICE void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
