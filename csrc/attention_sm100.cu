@@ -5,13 +5,14 @@
 // Forward, persistent, one CTA per SM walking items of 256 query rows of one (head, batch): two 128-row tiles that share every
 // K / V tile and are half a step out of phase, so that one tile's softmax runs under the other tile's products.
 // TMEM (512 columns): S of tile 0 / 1, O of tile 0 / 1, 128 columns each.
-//   warp 0      TMA producer : Q0, Q1, then K_j / V_j tiles ([128 kv × 128 d] as two 128B-swizzled [128 × 64] boxes), ring of 5
-//   warp 1      MMA issuer   : S = Q·K_jᵀ  (A, B K-major, 8 × UMMA 128×128×16)
-//                              O += P·V_j (A = P read from TMEM, B = V MN-major)
-//   warps 2-5, 6-9  softmax  : thread = query row of tile 0 / 1 (tcgen05.ld 32x32b: lane ↔ TMEM lane): row max, exp2, row sum, P
+//   warps 0-3, 4-7  softmax  : thread = query row of tile 0 / 1 (tcgen05.ld 32x32b: lane ↔ TMEM lane): row max, exp2, row sum, P
 //                              packed to bf16 and written back over S with tcgen05.st.  The O accumulator is only rescaled when
 //                              the running max grew by more than 2^8 (lazy rescale), so the common tile does no TMEM
 //                              round trip for O at all.
+//   warps 8-11  output       : O of a finished tile out of TMEM, divided by the row sums, to memory, while the softmax goes on to the next item
+//   warp 12     TMA producer : Q0, Q1, then K_j / V_j tiles ([128 kv × 128 d] as two 128B-swizzled [128 × 64] boxes), ring of 4
+//   warp 13     MMA issuer   : S = Q·K_jᵀ  (A, B K-major, 8 × UMMA 128×128×16)
+//                              O += P·V_j (A = P read from TMEM, B = V MN-major)
 // Outputs: O (bf16, arbitrary b/s/h strides) and LSE (fp32 [B, H, S], natural log) for the backward.
 #include <cuda.h>
 
@@ -30,11 +31,12 @@ CUtensorMap make_tmap_bf16_heads(const void* ptr, const uint64_t (&dims)[4], con
 namespace fa {
 
 constexpr int BM = 128, BN = 128, HD = 128;
-constexpr int kThreads = 320;
-constexpr int kRing = 5;                         // K / V tiles in flight or in use
+constexpr int kThreads = 512;
+constexpr int kRing = 4;                         // K / V tiles in flight or in use
 constexpr uint32_t kTile = BM * HD * 2;          // 32 KB
 constexpr uint32_t kHalf = kTile / 2;            // one [128 × 64] box
-constexpr uint32_t kSmemFwd = (2 + kRing) * kTile + 1024 /*align*/ + 512 /*barriers*/;
+constexpr uint32_t kStage = 32 * 64 * 2;         // an output warp's 32 rows x 64 columns on their way to memory
+constexpr uint32_t kSmemFwd = (2 + kRing) * kTile + 4 * kStage + 2048 /*row sums*/ + 1024 /*align*/ + 512 /*barriers*/;
 
 // Warp-uniform issue: the whole MMA warp runs the issue loop in convergent control flow and one elected lane executes the tcgen05
 // instructions (sm100_ptx.cuh explains why).  One election serves the products of a whole tile and the barrier they complete; descriptors
@@ -95,6 +97,11 @@ NXD_DEVICE uint64_t pack2u(uint32_t a, uint32_t b) { uint64_t r; asm("mov.b64 %0
 NXD_DEVICE float max3(float a, float b, float c) {
   float r;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+NXD_DEVICE float max3_nan(float a, float b, float c) {       // NaN where one is
+  float r;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
 }
 NXD_DEVICE uint32_t pack_bf16(float lo, float hi) {
@@ -172,34 +179,83 @@ NXD_DEVICE int clc_answer(uint32_t answer) {       // block index, or -1: none l
   return got ? (int)x : -1;
 }
 
-// Bound by the exponentials (MUFU: 1024 cycles per 128 x 128 tile and softmax warp, two warps per scheduler), the products (1024
-// cycles per tile) and the chain between them.  Tensor order is S0 S1 | PV0_j S0_{j+1} | PV1_j S1_{j+1} | …, across item
-// boundaries, with one S buffer per stream: S_{j+1} follows PV_j in pipe order, so a softmax warp that sees S_{j+1} knows that
-// PV_j is done.  P is handed over in two halves: the first half's products run under the second half's exponentials.
+// P = 2^(s * scale - max) of 32 columns, packed to bf16 in their first half; `sum` grows by it.  MAX: the maximum of the whole row beside it, NaN
+// where there is one.
+template <bool MAX>
+NXD_DEVICE void fwd_exps(uint32_t (&r)[4][32], int c, uint64_t scale, uint64_t shift, uint64_t& sum, float& mx) {
+  float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+  for (int i = 0; i < 32; i += 2) {
+    if constexpr (MAX) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) m4[k] = max3_nan(m4[k], __uint_as_float(r[k][i]), __uint_as_float(r[k][i + 1]));
+    }
+    const uint64_t x = fma2(pack2u(r[c][i], r[c][i + 1]), scale, shift);
+    float p0, p1;
+    unpack2(x, p0, p1);
+    p0 = ex2(p0);
+    p1 = ex2(p1);
+    sum = add2(sum, pack2(p0, p1));
+    r[c][i >> 1] = pack_bf16(p0, p1);
+  }
+  if constexpr (MAX) mx = max3_nan(m4[0], m4[1], max3_nan(m4[2], m4[3], m4[3]));
+}
+// columns behind `lim` to −inf: 0 after the exponential
+NXD_DEVICE void fwd_mask(uint32_t (&r)[32], int lim) {
+#pragma unroll
+  for (int i = 0; i < 32; ++i)
+    if (i > lim) r[i] = 0xff800000u;
+}
+
+// Bound by the tensor pipe and what feeds it: a tile's two products are 1024 cycles of mathematics and as many of operands and TMA writes in
+// shared memory, and take about 1450.  Beside them go the exponentials (128 a row: 1024 cycles per tile and softmax warp, two warps per
+// scheduler).  Tensor order is S0 S1 | PV0_j S0_{j+1} | PV1_j S1_{j+1} | …, across item boundaries, with one S buffer per stream: S_{j+1}
+// follows PV_j in pipe order, so a softmax warp that sees S_{j+1} knows that PV_j is done.  Behind an item's first tile the exponentials begin with
+// the maximum of the tiles before; the tile's own comes out beside the first quarter of them, which is done again where it lies more than 2^8
+// above (maximum first: 1 x 8192, 32 heads, 457 us, so 449).  A warpgroup of its own for O: 1 x 1531, 64 heads on 8, 55.5 -> 49.3 us, 1 x 2048, 32
+// heads 45.1 -> 41.1 with it and the next item's first product behind a stream's own last one.  Left out, none of them faster: P handed
+// over in two or three parts, a quarter of the exponentials by polynomial.
 __global__ void __launch_bounds__(kThreads, 1)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
               const __grid_constant__ CUtensorMap tv, __nv_bfloat16* __restrict__ out, const FwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t sQ = smem_base, sKV = smem_base + 2 * kTile;
-  const uint32_t bars = smem_base + (2 + kRing) * kTile;
-  // per stream: qf[2] qe[2] s[2] pa[2] pb[2] of[2] oe[2] | next item: full[2] empty[2] answer[2] | ring: kvf[5] kve[5] | tmem slot
-  const uint32_t bar_qf = bars, bar_qe = bars + 16, bar_s = bars + 32, bar_pa = bars + 48, bar_pb = bars + 64, bar_of = bars + 80,
-                 bar_oe = bars + 96, bar_nf = bars + 112, bar_ne = bars + 128, answers = bars + 144, bar_kvf = bars + 176,
-                 bar_kve = bars + 176 + 8 * kRing, tmem_slot = bars + 176 + 16 * kRing;
+  const uint32_t sQ = smem_base, sKV = smem_base + 2 * kTile, sO = sKV + kRing * kTile, sStat = sO + 4 * kStage;
+  const uint32_t bars = sStat + 2048;
+  // per stream: qf[2] qe[2] s[2] p[2] of[2] oe[2] lf[2] le[2] | next item: full[2] empty[2] answer[2] | ring: kvf[] kve[] | tmem slot
+  const uint32_t bar_qf = bars, bar_qe = bars + 16, bar_s = bars + 32, bar_p = bars + 48, bar_of = bars + 64,
+                 bar_oe = bars + 80, bar_lf = bars + 96, bar_le = bars + 112, bar_nf = bars + 128, bar_ne = bars + 144, answers = bars + 160,
+                 bar_kvf = bars + 192, bar_kve = bar_kvf + 8 * kRing, tmem_slot = bar_kve + 8 * kRing;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  if (threadIdx.x == 0) {
+  auto load_q = [&](const FwdItem& it, int t) {
+    const int qr = (it.qt + t) * BM, qh = it.head * p.q.h, qb = it.b * p.q.b;
+    mbar_expect_tx(bar_qf + 8 * t, kTile);
+    tma_load_4d(sQ + t * kTile, &tq, bar_qf + 8 * t, 0, qr, qh, qb);
+    tma_load_4d(sQ + t * kTile + kHalf, &tq, bar_qf + 8 * t, 64, qr, qh, qb);
+  };
+  auto load_kv = [&](const CUtensorMap* map, int slot, int r, int h, int b) {
+    mbar_expect_tx(bar_kvf + 8 * slot, kTile);
+    tma_load_4d(sKV + slot * kTile, map, bar_kvf + 8 * slot, 0, r, h, b);
+    tma_load_4d(sKV + slot * kTile + kHalf, map, bar_kvf + 8 * slot, 64, r, h, b);
+  };
+  if (warp == 12 && lane == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(bar_qf + 8 * i, 1); mbar_init(bar_qe + 8 * i, 1); mbar_init(bar_s + 8 * i, 1);
-      mbar_init(bar_pa + 8 * i, 128); mbar_init(bar_pb + 8 * i, 128);
-      mbar_init(bar_of + 8 * i, 1); mbar_init(bar_oe + 8 * i, 128);
-      mbar_init(bar_nf + 8 * i, 1); mbar_init(bar_ne + 8 * i, 10);       // readers: producer, MMA warp, 8 softmax warps
+      mbar_init(bar_p + 8 * i, 128); mbar_init(bar_of + 8 * i, 1); mbar_init(bar_oe + 8 * i, 128);
+      mbar_init(bar_lf + 8 * i, 128); mbar_init(bar_le + 8 * i, 128);
+      mbar_init(bar_nf + 8 * i, 1); mbar_init(bar_ne + 8 * i, 14);       // readers: softmax, output, producer and MMA warps
     }
     for (int i = 0; i < kRing; ++i) { mbar_init(bar_kvf + 8 * i, 1); mbar_init(bar_kve + 8 * i, 1); }
     fence_barrier_init();
+    // the first item's Q and first K are on their way while the tensor memory is allocated
+    const FwdItem it = fwd_item(blockIdx.x, p);
+    const int kvh = it.head / (p.H / p.Hkv);
+    load_q(it, 0);
+    load_kv(&tk, 0, 0, kvh * p.k.h, it.b * p.k.b);
+    if (it.n1 > 0 && !p.split) load_q(it, 1);
   }
-  if (warp == 1) {
+  if (warp == 13) {
     tcgen05_alloc(tmem_slot, 512);
     tcgen05_relinquish();
   }
@@ -222,16 +278,17 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
     return idx;
   };
 
-  if (warp == 0) {
-    if (lane == 0) {
-      prefetch_tmap(&tq); prefetch_tmap(&tk); prefetch_tmap(&tv);
+  // registers: 128 a thread at launch, 2 x 168 + 88 + 88 = 4 x 128 from here on (nothing spills; 184, 80, 64 did: 1 x 600 tokens 22.7 us, so 20.7)
+  if (warp >= 12) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+    if (warp == 12 && lane == 0) {
       int slot = 0; uint32_t ph = 0;
-      int items[2] = {0, 0};
-      auto load_kv = [&](const CUtensorMap* map, int r, int h, int b) {
-        mbar_wait(bar_kve + 8 * slot, ph ^ 1);
-        mbar_expect_tx(bar_kvf + 8 * slot, kTile);
-        tma_load_4d(sKV + slot * kTile, map, bar_kvf + 8 * slot, 0, r, h, b);
-        tma_load_4d(sKV + slot * kTile + kHalf, map, bar_kvf + 8 * slot, 64, r, h, b);
+      uint32_t q_items[2] = {0, 0};
+      auto next = [&](const CUtensorMap* map, int r, int h, int b, bool loaded) {
+        if (!loaded) {
+          mbar_wait(bar_kve + 8 * slot, ph ^ 1);
+          load_kv(map, slot, r, h, b);
+        }
         if (++slot == kRing) { slot = 0; ph ^= 1; }
       };
       for (int il = 0;; ++il) {
@@ -239,21 +296,21 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
         if (idx < 0) break;
         const FwdItem it = fwd_item(idx, p);
         const int kvh = it.head / (p.H / p.Hkv);
-        const int qh = it.head * p.q.h, qb = it.b * p.q.b, qr = it.qt * BM;
         const int kh = kvh * p.k.h, kb = it.b * p.k.b, vh = kvh * p.v.h, vb = it.b * p.v.b;
+#pragma unroll
         for (int t = 0; t < 2; ++t) {
-          if (t == 0 ? it.n0 > 0 : (it.n1 > 0 && !p.split)) {
-            mbar_wait(bar_qe + 8 * t, (uint32_t)((items[t] & 1) ^ 1));
-            ++items[t];
-            mbar_expect_tx(bar_qf + 8 * t, kTile);
-            tma_load_4d(sQ + t * kTile, &tq, bar_qf + 8 * t, 0, qr + t * BM, qh, qb);
-            tma_load_4d(sQ + t * kTile + kHalf, &tq, bar_qf + 8 * t, 64, qr + t * BM, qh, qb);
+          if (t == 0 || (it.n1 > 0 && !p.split)) {
+            if (il > 0) {
+              mbar_wait(bar_qe + 8 * t, (q_items[t] & 1) ^ 1);
+              load_q(it, t);
+            }
+            ++q_items[t];
           }
-          if (t == 0 && it.n > 0) load_kv(&tk, 0, kh, kb);
+          if (t == 0) next(&tk, 0, kh, kb, il == 0);
         }
         for (int j = 0; j < it.n; ++j) {
-          if (j > 0) load_kv(&tk, j * BN, kh, kb);
-          load_kv(&tv, j * BN, vh, vb);
+          if (j > 0) next(&tk, j * BN, kh, kb, false);
+          next(&tv, j * BN, vh, vb, false);
         }
         // asked for when the last tile is on its way (two steps before the end): asked at the item's start, the blocks would share
         // out the queue before they know which of them are done first (1 x 2048 tokens, 32 heads: 59 us)
@@ -263,77 +320,153 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
           clc_request(answers + 16 * (il & 1), bar_nf + 8 * (il & 1));
         }
       }
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    // all 32 lanes run this loop; the helpers elect one lane per tcgen05 instruction
-    constexpr uint32_t idesc_s = make_idesc(false, false, BM, BN);
-    constexpr uint32_t idesc_o = make_idesc(false, true, BM, HD);
-    int steps[2] = {0, 0}, q_items[2] = {0, 0}, o_items[2] = {0, 0};
-    // stream t, K tile number `pos` of the ring; `last_k`: no other stream uses it after this; `first` / `last` of the item
-    auto issue_s = [&](int t, int pos, bool first, bool last, bool last_k) {
-      const int slot = pos % kRing, tq_ = p.split ? 0 : t;
-      if (first) { mbar_wait(bar_qf + 8 * tq_, (uint32_t)(q_items[t] & 1)); ++q_items[t]; }
-      mbar_wait(bar_kvf + 8 * slot, (uint32_t)((pos / kRing) & 1));
-      tcgen05_fence_after();
-      const uint32_t q_s = sQ + tq_ * kTile, k_s = sKV + slot * kTile;
-      mma_ss8<kHalf / 16, 2, kHalf / 16, 2>(tmem_S + t * BN, make_smem_desc(q_s, 16, 1024), make_smem_desc(k_s, 16, 1024), idesc_s, 0u, bar_s + 8 * t);
-      if (last_k) tcgen05_commit_e(bar_kve + 8 * slot);
-      if (last && !p.split) tcgen05_commit_e(bar_qe + 8 * t);
-    };
-    auto get = [&](int il) { return fwd_item(item_index(il, true), p); };
-    // ring position of step j of stream t (its K; V is the next), counted from the item's first
-    auto at = [&](int t, int j) { return p.split ? 2 * (2 * j + t) : 2 * j; };
-    FwdItem it = get(0);
-    int pos0 = 0;                                  // ring position of the item's first K tile
-    for (int t = 0; t < 2; ++t) {
-      const int nt = t ? it.n1 : it.n0;
-      if (nt > 0) issue_s(t, at(t, 0), true, nt == 1, p.split || t == 1 || it.n1 == 0);
-    }
-    for (int il = 0; it.n > 0; ++il) {
-      FwdItem nx{};
-      const int pos1 = pos0 + 2 * it.n, steps_n = max(it.n0, it.n1);
-      for (int j = 0; j < steps_n; ++j) {
-        if (j == steps_n - 1) nx = get(il + 1);
+    } else if (warp == 13) {
+      // all 32 lanes run this loop; the helpers elect one lane
+      constexpr uint32_t idesc_s = make_idesc(false, false, BM, BN);
+      constexpr uint32_t idesc_o = make_idesc(false, true, BM, HD);
+      uint32_t steps = 0, q_items = 0, o_items = 0;                  // bit t: parity of stream t's count
+      // stream t, K tile number `pos` of the ring; `last_k`: no other stream uses it after this; `first` / `last` of the item
+      auto issue_s = [&](int t, int pos, bool first, bool last, bool last_k) {
+        const int slot = pos % kRing, tq_ = p.split ? 0 : t;
+        if (first) { mbar_wait(bar_qf + 8 * tq_, (q_items >> t) & 1); q_items ^= 1u << t; }
+        mbar_wait(bar_kvf + 8 * slot, (uint32_t)((pos / kRing) & 1));
+        tcgen05_fence_after();
+        mma_ss8<kHalf / 16, 2, kHalf / 16, 2>(tmem_S + t * BN, make_smem_desc(sQ + tq_ * kTile, 16, 1024), make_smem_desc(sKV + slot * kTile, 16, 1024),
+                                              idesc_s, 0u, bar_s + 8 * t);
+        if (last_k) tcgen05_commit_e(bar_kve + 8 * slot);
+        if (last && !p.split) tcgen05_commit_e(bar_qe + 8 * t);
+      };
+      auto get = [&](int il) { return fwd_item(item_index(il, true), p); };
+      // ring position of step j of stream t (its K; V is the next), counted from the item's first
+      auto at = [&](int t, int j) { return p.split ? 2 * (2 * j + t) : 2 * j; };
+      FwdItem it = get(0);
+      int pos0 = 0;                                // ring position of the item's first K tile
+      for (int t = 0; t < 2; ++t) {
+        const int nt = t ? it.n1 : it.n0;
+        if (nt > 0) issue_s(t, at(t, 0), true, nt == 1, p.split || t == 1 || it.n1 == 0);
+      }
+      for (int il = 0; it.n > 0; ++il) {
+        FwdItem nx{};
+        const int pos1 = pos0 + 2 * it.n, steps_n = max(it.n0, it.n1);
+        bool asked = false;
+        for (int j = 0; j < steps_n; ++j) {
 #pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          const int nt = t ? it.n1 : it.n0;
-          if (j < nt) {
-            const int pos = pos0 + at(t, j) + 1, slot = pos % kRing;
-            const uint32_t ph = (uint32_t)(steps[t] & 1);
-            ++steps[t];
-            mbar_wait(bar_kvf + 8 * slot, (uint32_t)((pos / kRing) & 1));
-            if (j == 0) { mbar_wait(bar_oe + 8 * t, (uint32_t)((o_items[t] & 1) ^ 1)); ++o_items[t]; }   // the item before left O
-            const uint32_t v_s = sKV + slot * kTile;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              mbar_wait((h ? bar_pb : bar_pa) + 8 * t, ph);
+          for (int t = 0; t < 2; ++t) {
+            const int nt = t ? it.n1 : it.n0;
+            if (j < nt) {
+              const int pos = pos0 + at(t, j) + 1, slot = pos % kRing;
+              const uint32_t ph = (steps >> t) & 1;
+              steps ^= 1u << t;
+              mbar_wait(bar_kvf + 8 * slot, (uint32_t)((pos / kRing) & 1));
+              if (j == 0) { mbar_wait(bar_oe + 8 * t, ((o_items >> t) & 1) ^ 1); o_items ^= 1u << t; }   // the item before left O
+              const uint32_t v_s = sKV + slot * kTile;
+              mbar_wait(bar_p + 8 * t, ph);
               tcgen05_fence_after();
-              mma_ts4<16, 128>(tmem_O + t * HD, tmem_S + t * BN + h * 32, make_smem_desc(v_s + h * 8192, kHalf, 1024), idesc_o, (j | h) ? 1u : 0u);
+#pragma unroll
+              for (int h = 0; h < 2; ++h)
+                mma_ts4<16, 128>(tmem_O + t * HD, tmem_S + t * BN + h * 32, make_smem_desc(v_s + h * 8192, kHalf, 1024), idesc_o, (j | h) ? 1u : 0u);
+              if (p.split || t == 1 || j >= it.n1) tcgen05_commit_e(bar_kve + 8 * slot);
+              if (j == nt - 1) tcgen05_commit_e(bar_of + 8 * t);
             }
-            if (p.split || t == 1 || j >= it.n1) tcgen05_commit_e(bar_kve + 8 * slot);
-            if (j == nt - 1) tcgen05_commit_e(bar_of + 8 * t);
-          }
-          if (j < steps_n - 1) {                   // S over P of this step: behind its PV in pipe order
-            if (j + 1 < nt) issue_s(t, pos0 + at(t, j + 1), false, j + 2 == nt, p.split || t == 1 || j + 1 >= it.n1);
-          } else {                                 // first S of the next item (this stream's last PV has been issued)
-            const int nn = t ? nx.n1 : nx.n0;
-            if (nn > 0) issue_s(t, pos1 + at(t, 0), true, nn == 1, p.split || t == 1 || nx.n1 == 0);
+            if (j + 1 < nt) {                      // S over P of this step: behind its PV in pipe order
+              issue_s(t, pos0 + at(t, j + 1), false, j + 2 == nt, p.split || t == 1 || j + 1 >= it.n1);
+            } else if (j == (nt ? nt : steps_n) - 1) {                  // first S of the next item: this stream's last PV has been issued
+              if (!asked) { nx = get(il + 1); asked = true; }
+              const int nn = t ? nx.n1 : nx.n0;
+              if (nn > 0) issue_s(t, pos1 + at(t, 0), true, nn == 1, p.split || t == 1 || nx.n1 == 0);
+            }
           }
         }
+        it = nx;
+        pos0 = pos1;
       }
-      it = nx;
-      pos0 = pos1;
     }
     __syncwarp();
+  } else if (warp >= 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+    const int quarter = warp & 3, row = quarter * 32 + lane;
+    const uint32_t tO = tmem_O + ((uint32_t)(quarter * 32) << 16), stage = sO + quarter * kStage;
+    uint32_t ph = 0;                               // bit t: parity of stream t's items
+    for (int il = 0;; ++il) {
+      const int idx = item_index(il, true);
+      if (idx < 0) break;
+      const FwdItem it = fwd_item(idx, p);
+      const bool merge = p.split && it.n1 > 0;     // both streams' sums belong to one query tile
+#pragma unroll 1
+      for (int t = 0; t < (p.split ? 1 : 2); ++t) {
+        if ((t ? it.n1 : it.n0) == 0) continue;
+        mbar_wait(bar_of + 8 * t, (ph >> t) & 1);
+        mbar_wait(bar_lf + 8 * t, (ph >> t) & 1);
+        float m, l, f0 = 1.f, f1 = 0.f;
+        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(m), "=f"(l) : "r"(sStat + t * 1024 + row * 8) : "memory");
+        if (merge) {
+          mbar_wait(bar_of + 8, 0);
+          mbar_wait(bar_lf + 8, 0);
+          float m1, l1;
+          asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(m1), "=f"(l1) : "r"(sStat + 1024 + row * 8) : "memory");
+          const float mm = fmaxf(m, m1);
+          f0 = ex2((m - mm) * p.scale_log2);
+          f1 = m1 == -INFINITY ? 0.f : ex2((m1 - mm) * p.scale_log2);
+          l = l * f0 + l1 * f1;
+          m = mm;
+        }
+        ph ^= 1u << t;
+        mbar_arrive(bar_le + 8 * t);
+        tcgen05_fence_after();
+        const float inv_l = 1.f / l;
+        const int r0 = (it.qt + t) * BM + quarter * 32;
+        // The rows leave through the warp's stage, 64 columns at a time, so that a store writes four runs of 128 bytes; stored as they come
+        // out of TMEM they were 32 runs of 16 bytes an instruction.
+        __nv_bfloat16* orow = out + (long)it.b * p.o_sb + (long)(r0 + (lane >> 3)) * p.o_ss + (long)it.head * p.o_sh + (lane & 7) * 8;
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+          __syncwarp();                            // what was in the stage has been read
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {            // 16 columns
+            uint32_t r[16];
+            tcgen05_ld_32x16(tO + t * HD + h * 64 + c * 16, r);
+            if (merge) {
+              uint32_t r1[16];
+              tcgen05_ld_32x16(tO + HD + h * 64 + c * 16, r1);
+              tcgen05_wait_ld();
+#pragma unroll
+              for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(fmaf(__uint_as_float(r[i]), f0, __uint_as_float(r1[i]) * f1));
+            } else {
+              tcgen05_wait_ld();
+            }
+#pragma unroll
+            for (int v4 = 0; v4 < 2; ++v4) {
+              uint32_t o[4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i) o[i] = pack_bf16(__uint_as_float(r[v4 * 8 + 2 * i]) * inv_l, __uint_as_float(r[v4 * 8 + 2 * i + 1]) * inv_l);
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage + lane * 128 + (((c * 2 + v4) ^ (lane & 7)) * 16)), "r"(o[0]),
+                           "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
+            }
+          }
+          if (h == 1) { tcgen05_fence_before(); mbar_arrive(bar_oe + 8 * t); }      // the next item's first product may overwrite O
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {            // rows 4 i + lane / 8
+            const int rr = 4 * i + (lane >> 3);
+            uint4 o;
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(o.x), "=r"(o.y), "=r"(o.z), "=r"(o.w)
+                         : "r"(stage + rr * 128 + (((lane & 7) ^ (rr & 7)) * 16)) : "memory");
+            if (r0 + rr < p.S_q) *reinterpret_cast<uint4*>(orow + (long)(4 * i) * p.o_ss + h * 64) = o;
+          }
+        }
+        if (r0 + lane < p.S_q) p.lse[((long)it.b * p.H + it.head) * p.S_q + r0 + lane] = m * p.scale + __logf(l);
+      }
+    }
   } else {
-    const int t = warp >= 6;                       // stream of this warpgroup
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
+    const int t = warp >= 4;                       // stream of this warpgroup
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     const uint32_t tS = tmem_S + t * BN + lane_base, tO = tmem_O + t * HD + lane_base;
-    const uint32_t my_s = bar_s + 8 * t, my_pa = bar_pa + 8 * t, my_pb = bar_pb + 8 * t, my_of = bar_of + 8 * t, my_oe = bar_oe + 8 * t;
+    const uint32_t my_s = bar_s + 8 * t, my_p = bar_p + 8 * t;
     const float sl2 = p.scale_log2;
+    const uint64_t sl2_2 = pack2(sl2, sl2);
     int g = 0, items = 0;
     for (int il = 0;; ++il) {
       const int idx = item_index(il, true);
@@ -348,34 +481,37 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
         tcgen05_fence_after();
         const int kv0 = (p.split ? 2 * j + t : j) * BN;
         const bool masked = (p.causal && kv0 + BN - 1 > q0) || (kv0 + BN > p.S_kv);
+        // last visible column of this row, and of the warp's first: most quarters of a tile need no look at single columns
+        const int kv_last = p.S_kv - 1 - kv0, lim = p.causal ? min(kv_last, q_idx - kv0) : kv_last;
+        const int lim_lo = p.causal ? min(kv_last, q0 + quarter * 32 - kv0) : kv_last;
         // ---- the whole S row (128 fp32) comes into registers with four back-to-back TMEM loads and one wait
         uint32_t sr[4][32];
 #pragma unroll
         for (int c = 0; c < 4; ++c) tcgen05_ld_32x32(tS + c * 32, sr[c]);
         tcgen05_wait_ld();
-        if (masked) {      // diagonal / ragged tile: −inf in place, the exp below turns it into an exact 0
-          const int lim = min(p.S_kv - 1, p.causal ? q_idx : 0x7fffffff) - kv0;      // last visible column of the tile
+        if (masked) {
 #pragma unroll
           for (int c = 0; c < 4; ++c)
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (c * 32 + i > lim) sr[c][i] = 0xff800000u;
+            if (lim_lo < c * 32 + 31) fwd_mask(sr[c], lim - c * 32);
         }
-        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-        for (int i = 0; i < 32; i += 2)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) mx4[c] = max3(mx4[c], __uint_as_float(sr[c][i]), __uint_as_float(sr[c][i + 1]));
-        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
         if (j == 0) {
-          m_ref = mx;
-        } else {
-          const float m_new = fmaxf(m_ref, mx);
-          const bool need = (m_new - m_ref) * sl2 > 8.f;
-          if (__any_sync(0xffffffffu, need)) {           // PV of the step before is done (this S came after it): O is quiescent
-            const float f = need ? ex2((m_ref - m_new) * sl2) : 1.f;
-            if (need) m_ref = m_new;
-            l *= f;
+          float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+          for (int i = 0; i < 32; i += 2)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) m4[c] = max3(m4[c], __uint_as_float(sr[c][i]), __uint_as_float(sr[c][i + 1]));
+          m_ref = fmaxf(max3(m4[0], m4[1], m4[2]), m4[3]);
+        }
+        uint64_t shift = pack2(-m_ref * sl2, -m_ref * sl2), sum[4] = {0ull, 0ull, 0ull, 0ull};
+        float mx, none;
+        fwd_exps<true>(sr, 0, sl2_2, shift, sum[0], mx);
+        const bool need = (mx - m_ref) * sl2 > 8.f;
+        if (__any_sync(0xffffffffu, need)) {
+          const float f = need ? ex2((m_ref - mx) * sl2) : 1.f;
+          if (need) m_ref = mx;
+          l *= f;
+          shift = pack2(-m_ref * sl2, -m_ref * sl2);
+          if (j > 0) {                             // PV of the step before is done (this S came after it): O is quiescent
 #pragma unroll 1
             for (int c = 0; c < 8; ++c) {
               uint32_t r[16];
@@ -386,100 +522,37 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
               tcgen05_st_32x16(tO + c * 16, r);
             }
           }
+          tcgen05_ld_32x32(tS, sr[0]);
+          tcgen05_wait_ld();
+          if (masked) fwd_mask(sr[0], lim);
+          sum[0] = 0ull;
+          fwd_exps<false>(sr, 0, sl2_2, shift, sum[0], none);
         }
-        // ---- P = exp2(s·scale·log2e − m_ref·scale·log2e), packed to bf16 in place and written over the S columns
-        const float mb = m_ref * sl2;
-        const uint64_t sl2_2 = pack2(sl2, sl2), nmb_2 = pack2(-mb, -mb);
-        uint64_t l2acc[4] = {0ull, 0ull, 0ull, 0ull};
+        if (!(mx < INFINITY)) l = __int_as_float(0x7fffffff);        // NaN or +inf among the scores: a row of NaN
+        tcgen05_st_32x16p(tS, sr[0]);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            float x0, x1;
-            unpack2(fma2(pack2u(sr[c][i], sr[c][i + 1]), sl2_2, nmb_2), x0, x1);
-            const float p0 = ex2(x0), p1 = ex2(x1);
-            l2acc[c] = add2(l2acc[c], pack2(p0, p1));
-            sr[c][i >> 1] = pack_bf16(p0, p1);
-          }
+        for (int c = 1; c < 4; ++c) {
+          fwd_exps<false>(sr, c, sl2_2, shift, sum[c], none);
           tcgen05_st_32x16p(tS + c * 16, sr[c]);
-          if (c & 1) {
-            tcgen05_wait_st();
-            tcgen05_fence_before();
-            mbar_arrive(c == 1 ? my_pa : my_pb);
-          }
         }
+        tcgen05_wait_st();
+        tcgen05_fence_before();
+        mbar_arrive(my_p);
         float l4[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) { float a, bq; unpack2(l2acc[c], a, bq); l4[c] = a + bq; }
+        for (int c = 0; c < 4; ++c) { float a, b; unpack2(sum[c], a, b); l4[c] = a + b; }
         l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
       }
-      // ---- epilogue: O comes into registers at once, so that the next item's first product may overwrite it while this one is
-      //      scaled and stored
-      mbar_wait(my_of, (uint32_t)(items & 1));
+      // ---- maximum and row sum to the output warps
+      mbar_wait(bar_le + 8 * t, (uint32_t)((items & 1) ^ 1));
       ++items;
-      tcgen05_fence_after();
-      uint32_t r[4][32];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) tcgen05_ld_32x32(tO + c * 32, r[c]);
-      tcgen05_wait_ld();
-      tcgen05_fence_before();
-      mbar_arrive(my_oe);
-      if (p.split && it.n1 > 0) {
-        // stream 1's sums to stream 0 through the Q buffers (every product with Q is done: stream 1's last PV was issued after
-        // the last S of both) and, for maximum and row sum, a ring slot nobody fills any more (a split block has one item)
-        const uint32_t so = sQ + row * 16, sml = sKV + row * 8;
-        if (t == 1) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
-#pragma unroll
-            for (int v4 = 0; v4 < 8; ++v4)
-              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(so + (c * 8 + v4) * 2048), "r"(r[c][v4 * 4]), "r"(r[c][v4 * 4 + 1]),
-                           "r"(r[c][v4 * 4 + 2]), "r"(r[c][v4 * 4 + 3]) : "memory");
-        }
-        // the ring: stream 0's last V must have been read before a slot is overwritten
-        if (t == 1) { mbar_wait(bar_of, 0); asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(sml), "f"(m_ref), "f"(l) : "memory"); }
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (t == 1) continue;
-        float m1, l1;
-        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(m1), "=f"(l1) : "r"(sml) : "memory");
-        const float m = fmaxf(m_ref, m1);
-        const float f0 = ex2((m_ref - m) * sl2), f1 = m1 == -INFINITY ? 0.f : ex2((m1 - m) * sl2);
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-          for (int v4 = 0; v4 < 8; ++v4) {
-            float4 o1;
-            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(o1.x), "=f"(o1.y), "=f"(o1.z), "=f"(o1.w)
-                         : "r"(so + (c * 8 + v4) * 2048) : "memory");
-            const float w[4] = {o1.x, o1.y, o1.z, o1.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              r[c][v4 * 4 + i] = __float_as_uint(fmaf(__uint_as_float(r[c][v4 * 4 + i]), f0, w[i] * f1));
-          }
-        l = l * f0 + l1 * f1;
-        m_ref = m;
-      }
-      const float inv_l = 1.f / l;
-      if (q_idx < p.S_q) {
-        __nv_bfloat16* orow = out + (long)it.b * p.o_sb + (long)q_idx * p.o_ss + (long)it.head * p.o_sh;
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-          for (int v4 = 0; v4 < 4; ++v4) {
-            uint4 o;
-            o.x = pack_bf16(__uint_as_float(r[c][v4 * 8 + 0]) * inv_l, __uint_as_float(r[c][v4 * 8 + 1]) * inv_l);
-            o.y = pack_bf16(__uint_as_float(r[c][v4 * 8 + 2]) * inv_l, __uint_as_float(r[c][v4 * 8 + 3]) * inv_l);
-            o.z = pack_bf16(__uint_as_float(r[c][v4 * 8 + 4]) * inv_l, __uint_as_float(r[c][v4 * 8 + 5]) * inv_l);
-            o.w = pack_bf16(__uint_as_float(r[c][v4 * 8 + 6]) * inv_l, __uint_as_float(r[c][v4 * 8 + 7]) * inv_l);
-            *reinterpret_cast<uint4*>(orow + c * 32 + v4 * 8) = o;
-          }
-        p.lse[((long)it.b * p.H + it.head) * p.S_q + q_idx] = m_ref * p.scale + __logf(l);
-      }
+      asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(sStat + t * 1024 + row * 8), "f"(m_ref), "f"(l) : "memory");
+      mbar_arrive(bar_lf + 8 * t);
     }
   }
   tcgen05_fence_before();
   __syncthreads();
-  if (warp == 1) tcgen05_dealloc(tmem_base, 512);
+  if (warp == 13) tcgen05_dealloc(tmem_base, 512);
 }
 
 // ====================================================================================================================

@@ -55,3 +55,22 @@ def test_heads(B, S, H, K):
 def test_flat_and_steep_probabilities(scale):
     """Rows whose maximum hardly moves, and rows whose maximum jumps from tile to tile by more than the accumulator's spare range."""
     _check(1, 700, 700, 4, 4, True, scale)
+
+
+def test_scores_that_are_no_numbers():
+    """NaN and infinite keys or queries make NaN rows where they are seen, and only there."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = (torch.randn(1, 450, 2, 128, generator=g, device="cuda").bfloat16() for _ in range(3))
+    want = ops.attention.flash_attention(q, k, v, causal=True)
+    for value in (math.nan, math.inf):
+        for row in (0, 130, 300, 449):
+            k2, q2 = k.clone(), q.clone()
+            k2[0, row, 1, 5] = value
+            o = ops.attention.flash_attention(q, k2, v, causal=True)
+            assert torch.equal(o[:, :, 0], want[:, :, 0]) and torch.equal(o[:, :row, 1], want[:, :row, 1])
+            seen = q[0, row:, 1, 5] > 0 if value == math.inf else torch.ones(450 - row, dtype=torch.bool, device="cuda")
+            assert o[0, row:, 1][seen].isnan().all()                   # q . k is NaN or +inf; where it is -inf the key has no weight
+            q2[0, row, 1, 5] = math.nan
+            o = ops.attention.flash_attention(q2, k, v, causal=True)
+            rest = torch.arange(450, device="cuda") != row
+            assert o[0, row, 1].isnan().all() and torch.equal(o[:, rest], want[:, rest])
