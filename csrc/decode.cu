@@ -20,9 +20,8 @@ constexpr int HD = 128;
 constexpr int kDecWarps = 4;
 constexpr int kDecThreads = kDecWarps * 32;
 constexpr int kDecRows = 16;                                 // cache rows of one tile of a warp
-constexpr int kDecStages = 3;
 constexpr int kDecTileBytes = kDecRows * HD * 2;             // 4 KB of K, as much of V
-constexpr int kDecSmem = kDecWarps * kDecStages * 2 * kDecTileBytes;      // 96 KB: two blocks per SM
+constexpr int dec_smem_bytes(int stages) { return kDecWarps * stages * 2 * kDecTileBytes; }      // 64 KB: three blocks per SM; 96: two
 
 NXD_DEVICE void cp_async16(uint32_t dst, const void* src, bool live) {    // not live: 16 zero bytes, nothing is read
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
@@ -40,13 +39,15 @@ NXD_DEVICE void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a2, uint32_t b0, u
 
 // One block per (key/value head, sequence, stretch of the cache); its G <= 8 query heads share every row that is read.
 // Bound by HBM: 512 bytes per cache row and key/value head.  Each warp walks 16-row tiles of its own through its own ring of
-// cp.async stages (2 x 8 KB in flight per warp, 128 KB per SM, no block barrier in the loop).  Scores come from mma.sync
+// cp.async stages (no block barrier in the loop): two stages and three blocks per SM, so that starts and ends of blocks lie under the others' copies,
+// or, where a launch has no more than that, three stages (decode_attention).  Scores come from mma.sync
 // (a 16 x 8 x 16 step holds all heads of the group; exact products, fp32 sums), so a row costs a few instructions per warp
 // instead of a dot product with four shuffles per head; probabilities stay fp32 and meet V in fp32 FMAs, lane = 4 columns.
-// 8 sequences, 8192-row cache (three quarters in use), 32 heads on 8: 39 us = 5.2 TB/s; with dot products on CUDA cores and
-// 8 rows in flight per block it was 148 us.
-template <int G>
-__global__ void __launch_bounds__(kDecThreads, 2) decode_attn_kernel(
+// With the merge, us, three stages and two: 8 sequences, 8192-row caches (three quarters in use), 32 heads on 8: 44.6 and 42.5; 16, 4096, 64 on 8:
+// 55.6 and 50.6; 1, 8192, 64 on 8 (256 blocks): 14.3 and 16.7; 3, 300, 40 (240 blocks): 6.8 and 7.3; 1, 2048, 40 (320 blocks): 11.2 and 9.3 out of
+// L2, but a 13B model's token, whose caches come from memory, 304 and 317.
+template <int G, int kDecStages>
+__global__ void __launch_bounds__(kDecThreads, kDecStages == 2 ? 3 : 2) decode_attn_kernel(
     const __nv_bfloat16* q, const __nv_bfloat16* kc, const __nv_bfloat16* vc,
     const long* positions, float* part_o, float* part_ml,
     __nv_bfloat16* out, int B, int H, int Hkv, int L,
@@ -205,23 +206,37 @@ __global__ void __launch_bounds__(kDecThreads, 2) decode_attn_kernel(
   }
 }
 
+// Merge of a head's stretches (at most 64): the sum of o relative to the row's maximum `mn`, and the row sum `ls`; thread = column.  The first
+// sixteen stretches are asked for before their weights are known, and every warp gets all weights with one read per lane; walked one after the
+// other, twice, they took 2 to 3 us more (8 x 8192 rows, 32 heads on 8, both kernels: 40.6 -> 38.9 us; 1 x 2048, 40 heads: 9.4 -> 8.7).
+NXD_DEVICE float merge_stretches(const float* part_o, const float* part_ml, int bh, int splits, float& mn, float& ls) {
+  const float2* ml = reinterpret_cast<const float2*>(part_ml) + (long)bh * splits;
+  const float* po = part_o + (long)bh * splits * HD + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  float v[16];
+#pragma unroll
+  for (int s = 0; s < 16; ++s) v[s] = s < splits ? po[(long)s * HD] : 0.f;
+  const float2 a0 = lane < splits ? ml[lane] : make_float2(-INFINITY, 0.f), a1 = lane + 32 < splits ? ml[lane + 32] : make_float2(-INFINITY, 0.f);
+  mn = warp_max(fmaxf(a0.x, a1.x));
+  const float c0 = mn == -INFINITY ? 0.f : exp2f(a0.x - mn), c1 = mn == -INFINITY ? 0.f : exp2f(a1.x - mn);
+  ls = warp_sum(a0.y * c0 + a1.y * c1);
+  float acc = 0.f;
+#pragma unroll
+  for (int s = 0; s < 16; ++s) acc += v[s] * __shfl_sync(0xffffffffu, c0, s);
+#pragma unroll 8
+  for (int s = 16; s < splits; ++s) acc += po[(long)s * HD] * __shfl_sync(0xffffffffu, s < 32 ? c0 : c1, s & 31);
+  return acc;
+}
+
 __global__ void __launch_bounds__(HD) decode_combine_kernel(const float* part_o, const float* part_ml,
                                                             __nv_bfloat16* out, int splits, long o_sb, long o_sh,
                                                             int H) {
-  const int bh = blockIdx.x, d = threadIdx.x;
   pdl_trigger();
   pdl_wait();
-  float mn = -INFINITY;
-  for (int s = 0; s < splits; ++s) mn = fmaxf(mn, part_ml[((long)bh * splits + s) * 2]);
-  float acc = 0.f, ls = 0.f;
-  for (int s = 0; s < splits; ++s) {
-    const long idx = (long)bh * splits + s;
-    const float c = mn == -INFINITY ? 0.f : exp2f(part_ml[idx * 2] - mn);
-    acc += part_o[idx * HD + d] * c;
-    ls += part_ml[idx * 2 + 1] * c;
-  }
-  const int b = bh / H, h = bh % H;
-  out[b * o_sb + h * o_sh + d] = __float2bfloat16_rn(ls > 0.f ? acc / ls : 0.f);
+  float mn, ls;
+  const float acc = merge_stretches(part_o, part_ml, blockIdx.x, splits, mn, ls);
+  const int b = blockIdx.x / H, h = blockIdx.x % H;
+  out[b * o_sb + h * o_sh + threadIdx.x] = __float2bfloat16_rn(ls > 0.f ? acc / ls : 0.f);
 }
 
 // Same merge over the splits, but the result stays un-normalised: o (relative to the row maximum), the maximum (natural-log
@@ -229,19 +244,11 @@ __global__ void __launch_bounds__(HD) decode_combine_kernel(const float* part_o,
 // the cross-rank log-sum-exp merge (modules/attention/flash_decode.py).
 __global__ void __launch_bounds__(HD) decode_combine_partial_kernel(const float* part_o, const float* part_ml,
                                                                     float* fin_o, float* fin_ml, int splits) {
-  const int bh = blockIdx.x, d = threadIdx.x;
   pdl_wait();
-  float mn = -INFINITY;
-  for (int s = 0; s < splits; ++s) mn = fmaxf(mn, part_ml[((long)bh * splits + s) * 2]);
-  float acc = 0.f, ls = 0.f;
-  for (int s = 0; s < splits; ++s) {
-    const long idx = (long)bh * splits + s;
-    const float c = mn == -INFINITY ? 0.f : exp2f(part_ml[idx * 2] - mn);
-    acc += part_o[idx * HD + d] * c;
-    ls += part_ml[idx * 2 + 1] * c;
-  }
-  fin_o[(long)bh * HD + d] = acc;
-  if (d == 0) { fin_ml[bh * 2] = mn * 0.6931471805599453f; fin_ml[bh * 2 + 1] = ls; }
+  float mn, ls;
+  const float acc = merge_stretches(part_o, part_ml, blockIdx.x, splits, mn, ls);
+  fin_o[(long)blockIdx.x * HD + threadIdx.x] = acc;
+  if (threadIdx.x == 0) { fin_ml[blockIdx.x * 2] = mn * 0.6931471805599453f; fin_ml[blockIdx.x * 2 + 1] = ls; }
 }
 
 // While the kernel before it still runs (a norm, a rotation, the merge of an attention), the first bytes of its weights come to L2:
@@ -345,8 +352,8 @@ void decode_rope_kv(const void* q, const void* k, const void* v, const long* pos
 }
 
 // Stretches per (sequence, key/value head): about six blocks per SM in all, so that sequences of unequal length fill the GPU to
-// the end (8 x 8192 rows, 8 key/value heads: 39 us; four per SM 41, sixteen 45), and no stretch below 256 rows, where a block's
-// start and the merge outweigh its reading (1 x 2048 rows, 40 heads: 11.2 us with the merge; 128-row stretches 12.1, 64-row 14.7).
+// the end (8 x 8192 rows, 8 key/value heads, with the merge: 41.0 us; three per SM 43.6, nine 42.3), and no stretch below 256 rows, where a block's
+// start and the merge outweigh its reading (1 x 2048 rows, 40 heads, 128-row stretches a tenth slower, 64-row a third).  At most 64 (the merge).
 int device_sm_count();
 int decode_splits(int pairs, int L) {
   const int want = (6 * device_sm_count() + pairs - 1) / pairs;
@@ -360,13 +367,16 @@ void decode_attention(const void* q, const void* k, const void* v, const long* p
   dim3 grid(Hkv, B, splits);
   const float sl2 = scale * 1.4426950408889634f;
   const bool whole = splits == 1 && fin_o == nullptr;
-#define NXD_DEC(Gv)                                                                                                  \
+  // Launches that three blocks per SM take at once are a few round trips to memory long, and need them deeper rather than more of them at a time
+  const bool few = (long)Hkv * B * splits <= 3l * device_sm_count();
+#define NXD_DEC_STAGES(Gv, Sv)                                                                                       \
   do {                                                                                                               \
-    NXD_ALLOW_SMEM(decode_attn_kernel<Gv>, kDecSmem);                                                                  \
-    launch_dependent(decode_attn_kernel<Gv>, grid, kDecThreads, kDecSmem, st, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k,      \
+    NXD_ALLOW_SMEM((decode_attn_kernel<Gv, Sv>), dec_smem_bytes(Sv));                                                  \
+    launch_dependent(decode_attn_kernel<Gv, Sv>, grid, kDecThreads, dec_smem_bytes(Sv), st, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k, \
         (const __nv_bfloat16*)v, positions, part_o, part_ml, whole ? (__nv_bfloat16*)out : nullptr, B, H, Hkv, L,      \
         ks[0], ks[1], ks[2], vs[0], vs[1], vs[2], q_sb, q_sh, o_sb, o_sh, sl2, splits);                                \
   } while (0)
+#define NXD_DEC(Gv) do { if (few) NXD_DEC_STAGES(Gv, 3); else NXD_DEC_STAGES(Gv, 2); } while (0)
   switch (G) {
     case 1: NXD_DEC(1); break;
     case 2: NXD_DEC(2); break;
@@ -375,6 +385,7 @@ void decode_attention(const void* q, const void* k, const void* v, const long* p
     default: nxd_throw("decode_attention: unsupported GQA group size", __FILE__, __LINE__);
   }
 #undef NXD_DEC
+#undef NXD_DEC_STAGES
   if (fin_o != nullptr) launch_dependent(decode_combine_partial_kernel, B * H, HD, 0, st, part_o, part_ml, fin_o, fin_ml, splits);
   else if (!whole) launch_dependent(decode_combine_kernel, B * H, HD, 0, st, part_o, part_ml, (__nv_bfloat16*)out, splits, o_sb, o_sh, H);
   NXD_CUDA_CHECK(cudaGetLastError());

@@ -53,3 +53,18 @@ def test_partial_results_merge_to_the_whole():
     num = sum(o * torch.exp(ml[..., 0] - m)[..., None] for o, ml in parts)
     den = sum(ml[..., 1] * torch.exp(ml[..., 0] - m) for _, ml in parts)
     assert (num / den[..., None] - whole).abs().max() <= 2.0 ** -8 * whole.abs().max()
+
+
+@pytest.mark.parametrize("batch,kv_heads,group,rows", [(1, 1, 4, 4096), (1, 1, 8, 4097), (1, 1, 1, 8193), (1, 1, 2, 20000), (1, 40, 1, 2048), (4, 8, 4, 7000),
+                                                      (16, 8, 8, 4096), (3, 37, 2, 511)])
+def test_numbers_of_stretches(batch, kv_heads, group, rows):
+    """Merges of 2 to 64 stretches (16 of them at once), launches of more and of fewer than two blocks per SM."""
+    from neuronx_distributed_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    k, v = (torch.randn(batch, rows, kv_heads, 128, generator=g, device="cuda").bfloat16() for _ in range(2))
+    q = torch.randn(batch, 1, kv_heads * group, 128, generator=g, device="cuda").bfloat16() * 2
+    pos = torch.randint(rows // 2, rows, (batch,), generator=g, device="cuda")
+    want = _reference(q, k, v, pos)
+    got = ops.attention.decode_attention(q, k, v, pos).float()
+    assert (got - want).abs().max() <= 2.0 ** -8 * want.abs().max()
