@@ -25,6 +25,7 @@ namespace g2 {
 // block) meets the weights of one expert, `b_rows` rows further down the stacked B per expert; `used_blocks` (device, may be
 // null) bounds the blocks that hold tokens.  MODE 4 (weight gradients): one output matrix per expert, summed over that
 // expert's row blocks [seg[e], seg[e + 1]); an expert without tokens gets zeros.
+constexpr int kExpertRows = 4;       // row tiles that go through the columns together: about one expert's (with 16, two per cent slower)
 struct Group {
   const int* block_expert;
   const int* seg;
@@ -50,7 +51,7 @@ NXD_DEVICE Unit unit_of(int unit, int num_tiles, int tiles_m, int tiles_n, int n
     if (tail.tiles > 0 && x >= 0) {                        // never together with split_k
       u.part = true;
       u.mat = x;
-      tile_coords(num_tiles - tail.tiles + x / tail.splits, tiles_m, tiles_n, u.m_blk, u.n_blk);
+      tile_coords(num_tiles - tail.tiles + x / tail.splits, tiles_m, tiles_n, raster_rows(tiles_m), u.m_blk, u.n_blk);
       u.kb0 = x % tail.splits * tail.kb_per;
       u.kb1 = min(num_kb, u.kb0 + tail.kb_per);
       return u;
@@ -59,12 +60,12 @@ NXD_DEVICE Unit unit_of(int unit, int num_tiles, int tiles_m, int tiles_n, int n
   if constexpr (MODE == 4) {
     const int per = tiles_m * tiles_n;
     u.mat = unit / per;
-    tile_coords(unit - u.mat * per, tiles_m, tiles_n, u.m_blk, u.n_blk);
+    tile_coords(unit - u.mat * per, tiles_m, tiles_n, kExpertRows, u.m_blk, u.n_blk);
     u.kb0 = g.seg[u.mat] * (g.block_rows / BK);
     u.kb1 = g.seg[u.mat + 1] * (g.block_rows / BK);
   } else {
     const int ks = unit / num_tiles;
-    tile_coords(unit - ks * num_tiles, tiles_m, tiles_n, u.m_blk, u.n_blk);
+    tile_coords(unit - ks * num_tiles, tiles_m, tiles_n, MODE == 0 ? raster_rows(tiles_m) : kExpertRows, u.m_blk, u.n_blk);
     u.kb0 = ks * kb_per;
     u.kb1 = min(num_kb, (ks + 1) * kb_per);
   }
@@ -241,7 +242,7 @@ __global__ void __launch_bounds__(256) gemm_tail_kernel(const float* part, OutT*
   pdl_wait();
   const int t = blockIdx.y, row = blockIdx.x * 8 + (threadIdx.x >> 5), col = (threadIdx.x & 31) * 8;
   int m_blk, n_blk;
-  tile_coords(first + t, tiles_m, tiles_n, m_blk, n_blk);
+  tile_coords(first + t, tiles_m, tiles_n, raster_rows(tiles_m), m_blk, n_blk);
   const int gr = m_blk * TILE_M + row, gc = n_blk * TILE_N + col;
   if (gr >= M || gc >= N) return;                          // N is a multiple of 8
   const float* src = part + ((size_t)t * splits * TILE_M + row) * TILE_N + col;
