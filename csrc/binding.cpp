@@ -360,6 +360,29 @@ static Tensor moe_combine(const Tensor& y, const Tensor& slot_of, const Tensor& 
                    (int)y.size(1), E, (int)expert_index.size(1), stream());
   return out;
 }
+// Chosen affinities divided by their sum, and the gradient of the affinities out of that of the quotients
+static void check_affinities(const Tensor& aff, const Tensor& expert_index) {
+  TORCH_CHECK(aff.is_cuda() && aff.is_contiguous() && aff.scalar_type() == at::kFloat && aff.dim() == 2);
+  TORCH_CHECK(expert_index.is_cuda() && expert_index.is_contiguous() && expert_index.scalar_type() == at::kLong && expert_index.dim() == 2 &&
+              expert_index.size(0) == aff.size(0));
+}
+static Tensor moe_normalize(const Tensor& aff, const Tensor& expert_index) {
+  check_affinities(aff, expert_index);
+  c10::cuda::CUDAGuard g(aff.device());
+  auto out = at::empty_like(aff);
+  nxd::moe_normalize(aff.data_ptr<float>(), expert_index.data_ptr<long>(), nullptr, out.data_ptr<float>(), (int)aff.size(0), (int)aff.size(1),
+                     (int)expert_index.size(1), stream());
+  return out;
+}
+static Tensor moe_normalize_grad(const Tensor& gw, const Tensor& aff, const Tensor& expert_index) {
+  check_affinities(aff, expert_index);
+  TORCH_CHECK(gw.is_cuda() && gw.is_contiguous() && gw.scalar_type() == at::kFloat && gw.sizes() == aff.sizes());
+  c10::cuda::CUDAGuard g(aff.device());
+  auto out = at::empty_like(aff);
+  nxd::moe_normalize(aff.data_ptr<float>(), expert_index.data_ptr<long>(), gw.data_ptr<float>(), out.data_ptr<float>(), (int)aff.size(0),
+                     (int)aff.size(1), (int)expert_index.size(1), stream());
+  return out;
+}
 static py::tuple moe_combine_grad(const Tensor& g, const Tensor& y, const Tensor& slot_token, const Tensor& block_expert, const Tensor& seg,
                                   const Tensor& w, int64_t block_size) {
   CHECK_MOE_ROWS(g); CHECK_MOE_ROWS(y); CHECK_MOE_INTS(slot_token); CHECK_MOE_INTS(block_expert); CHECK_MOE_INTS(seg);
@@ -584,17 +607,20 @@ static Tensor grouped_gemm(const Tensor& a, const Tensor& w, const Tensor& block
                          (int)block_rows, nxd::kBF16, stream());
   return out;
 }
-// dW[e] = x[rows of e]ᵀ · dy[rows of e]  → out [E, Mo, No] (bf16 or fp32), optionally accumulated
+// dW[e] = x[rows of e]ᵀ · dy[rows of e]  → out [E, Mo, No] (bf16 or fp32), optionally accumulated.  slot_token (int32 [rows], optional): -1
+// for the rows behind an expert's last one, which are zero in x and dy
 static void grouped_wgrad(const Tensor& x, const Tensor& dy, Tensor out, const Tensor& seg_first_block, int64_t block_rows,
-                          bool accumulate) {
+                          bool accumulate, const c10::optional<Tensor>& slot_token) {
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.is_contiguous() && dy.scalar_type() == at::kBFloat16 &&
               dy.is_contiguous() && out.is_contiguous() && out.dim() == 3);
   TORCH_CHECK(seg_first_block.scalar_type() == at::kInt && seg_first_block.numel() == out.size(0) + 1);
   TORCH_CHECK(x.size(0) == dy.size(0) && out.size(1) == x.size(1) && out.size(2) == dy.size(1));
   TORCH_CHECK(x.size(1) % 8 == 0 && dy.size(1) % 8 == 0);
   c10::cuda::CUDAGuard guard(x.device());
+  if (slot_token.has_value())
+    TORCH_CHECK(slot_token->is_cuda() && slot_token->is_contiguous() && slot_token->scalar_type() == at::kInt && slot_token->numel() == x.size(0));
   nxd::grouped_wgrad_bf16(x.data_ptr(), dy.data_ptr(), out.data_ptr(), x.size(0), x.size(1), dy.size(1), out.size(0),
-                          seg_first_block.data_ptr<int>(), (int)block_rows, dt_code(out), accumulate, stream());
+                          seg_first_block.data_ptr<int>(), slot_token.has_value() ? slot_token->data_ptr<int>() : nullptr, (int)block_rows, dt_code(out), accumulate, stream());
 }
 
 // ---- attention ----------------------------------------------------------------------------------
@@ -989,6 +1015,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_gather", &moe_gather);
   m.def("moe_combine", &moe_combine);
   m.def("moe_combine_grad", &moe_combine_grad);
+  m.def("moe_normalize", &moe_normalize);
+  m.def("moe_normalize_grad", &moe_normalize_grad);
   m.def("row_argmax", &row_argmax);
   m.def("row_topk", &row_topk);
   m.def("row_topk_supported", &row_topk_supported);
@@ -997,7 +1025,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_few_rows", &gemm_few_rows, py::arg("x"), py::arg("w"), py::arg("split") = 0);
   m.def("grouped_gemm", &grouped_gemm, py::arg("a"), py::arg("w"), py::arg("block_expert"), py::arg("block_rows"), py::arg("trans_b"),
         py::arg("seg") = c10::nullopt);
-  m.def("grouped_wgrad", &grouped_wgrad);
+  m.def("grouped_wgrad", &grouped_wgrad, py::arg("x"), py::arg("dy"), py::arg("out"), py::arg("seg_first_block"), py::arg("block_rows"),
+        py::arg("accumulate"), py::arg("slot_token") = py::none());
   m.def("flash_attn_fwd", &flash_attn_fwd);
   m.def("flash_attn_bwd_parts", &nxd::flash_attn_bwd_parts);
   m.def("flash_attn_bwd", &flash_attn_bwd, py::arg("go"), py::arg("q"), py::arg("k"), py::arg("v"), py::arg("o"), py::arg("lse"),

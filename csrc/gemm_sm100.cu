@@ -609,10 +609,11 @@ void grouped_gemm_bf16(const void* a, const void* b, void* out, int M, int N, in
 }
 
 // out[e] [Mo, No] (+)= A[rows of e, Mo]ᵀ · B[rows of e, No]; expert e owns row blocks [seg_first_block[e], seg_first_block[e+1]).
+// `slot_token` (may be null): token of each row, -1 where an expert's last block is padded with zeros.
 void grouped_wgrad_bf16(const void* a, const void* b, void* out, int rows_total, int Mo, int No, int E,
-                        const int* seg_first_block, int block_rows, int out_dt, bool accumulate, cudaStream_t st) {
+                        const int* seg_first_block, const int* slot_token, int block_rows, int out_dt, bool accumulate, cudaStream_t st) {
   if (block_rows % BLOCK_K) nxd_throw("grouped wgrad: block size must be a multiple of 64", __FILE__, __LINE__);
-  grouped_wgrad_bf16_2cta(a, b, out, rows_total, Mo, No, E, seg_first_block, block_rows, out_dt, accumulate, st);
+  grouped_wgrad_bf16_2cta(a, b, out, rows_total, Mo, No, E, seg_first_block, slot_token, block_rows, out_dt, accumulate, st);
 }
 
 // out[M,N] (bf16) = (a_e4m3[M,K] · b_e4m3[N,K]ᵀ) ∘ scale_a[M] ⊗ scale_b[N]   (quantised inference linear)

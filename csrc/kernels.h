@@ -113,9 +113,9 @@ void grouped_gemm_bf16(const void* a, const void* b, void* out, int M, int N, in
 void grouped_gemm_bf16_2cta(const void* a, const void* b, void* out, int M, int N, int K, int E, bool trans_b, const int* block_expert,
                             const int* used_blocks, int block_rows, int out_dt, cudaStream_t st);
 void grouped_wgrad_bf16_2cta(const void* a, const void* b, void* out, int rows_total, int Mo, int No, int E, const int* seg_first_block,
-                             int block_rows, int out_dt, bool accumulate, cudaStream_t st);
+                             const int* slot_token, int block_rows, int out_dt, bool accumulate, cudaStream_t st);
 void grouped_wgrad_bf16(const void* a, const void* b, void* out, int rows_total, int Mo, int No, int E,
-                        const int* seg_first_block, int block_rows, int out_dt, bool accumulate, cudaStream_t st);
+                        const int* seg_first_block, const int* slot_token, int block_rows, int out_dt, bool accumulate, cudaStream_t st);
 
 // ---- one-shot all-reduce over peer memory (allreduce.cu)
 void oneshot_allreduce(const void* x, void* out, const int64_t* peer_bufs, const int64_t* peer_flags, long slot_bytes,
@@ -137,6 +137,8 @@ void moe_slots(const long* expert_index, long n, int k, int E, int B, int nb, in
 void moe_gather(const void* x, const int* slot_token, const int* used_blocks, void* out, int H, int B, int rows, cudaStream_t st);
 void moe_combine(const void* y, const int* slot_of, const long* expert_index, const float* w, void* out, int T, int H, int E, int k,
                  cudaStream_t st);
+// gw null: out = chosen affinities (others 0) divided by their row's sum; else out = gradient of aff where gw is that of the quotients
+void moe_normalize(const float* aff, const long* expert_index, const float* gw, float* out, int T, int E, int k, cudaStream_t st);
 void moe_combine_grad(const void* g, const void* y, const int* slot_token, const int* block_expert, const int* used_blocks, const float* w,
                       void* dy, float* dw, int H, int E, int B, int rows, cudaStream_t st);
 

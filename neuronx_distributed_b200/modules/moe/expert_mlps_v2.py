@@ -170,10 +170,15 @@ class ExpertMLPsV2(ProcessGroupSafeDeepcopy, nn.Module):
 
     def _topk_affinities(self, aff: torch.Tensor, idx: torch.Tensor, padding_mask=None) -> torch.Tensor:
         """[T, E] affinities keeping only the chosen experts (optionally re-normalised over them)."""
-        mask = torch.zeros_like(aff).scatter_(1, idx, 1.0)
-        a = aff * mask
-        if self.cfg.normalize_top_k_affinities:
-            a = a / a.sum(-1, keepdim=True).clamp(min=1e-9)
+        from ... import ops
+
+        if self.cfg.normalize_top_k_affinities and ops.moe_blocks.normalize_ok(aff, idx):
+            a = ops.moe_blocks.normalize(aff, idx)
+        else:
+            mask = torch.zeros_like(aff).scatter_(1, idx, 1.0)
+            a = aff * mask
+            if self.cfg.normalize_top_k_affinities:
+                a = a / a.sum(-1, keepdim=True).clamp(min=1e-9)
         if padding_mask is not None:
             a = a * padding_mask.reshape(-1, 1).to(a.dtype)
         return a

@@ -11,6 +11,7 @@ any transposition copies:
 from __future__ import annotations
 
 import os
+from typing import Optional
 
 import torch
 
@@ -127,15 +128,16 @@ def _grouped_ref(x, w, b2e, block_size):
 
 class _GroupedMatmul(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, w, b2e, seg_first_block, block_size, skip_unused):
-        ctx.save_for_backward(x, w, b2e, seg_first_block)
+    def forward(ctx, x, w, b2e, seg_first_block, block_size, skip_unused, slot_token):
+        ctx.save_for_backward(x, w, b2e, seg_first_block, slot_token)
         ctx.block_size, ctx.skip_unused = block_size, skip_unused
         _ext.count_launch()
         return _ext.ext().grouped_gemm(x.contiguous(), w.contiguous(), b2e, block_size, False, seg_first_block if skip_unused else None)
 
     @staticmethod
     def backward(ctx, gy):
-        x, w, b2e, seg = ctx.saved_tensors
+        x, w, b2e, seg, slot_token = ctx.saved_tensors
+        extra = () if slot_token is None else (slot_token,)
         gy = gy.contiguous()
         gx = gw = None
         if ctx.needs_input_grad[0]:
@@ -146,21 +148,22 @@ class _GroupedMatmul(torch.autograd.Function):
             mg = getattr(w, "main_grad", None)
             if mg is not None and fused_wgrad_enabled() and mg.dtype == torch.float32 and mg.is_contiguous():
                 fresh = getattr(w, "main_grad_fresh", False)
-                _ext.ext().grouped_wgrad(x.contiguous(), gy, mg.view_as(w), seg, ctx.block_size, not fresh)
+                _ext.ext().grouped_wgrad(x.contiguous(), gy, mg.view_as(w), seg, ctx.block_size, not fresh, *extra)
                 w.main_grad_fresh = False
                 cb = getattr(w, "_nxd_grad_ready", None)
                 if cb is not None:
                     cb(w)
             else:
                 gw = torch.empty_like(w)
-                _ext.ext().grouped_wgrad(x.contiguous(), gy, gw, seg, ctx.block_size, False)
-        return gx, gw, None, None, None, None
+                _ext.ext().grouped_wgrad(x.contiguous(), gy, gw, seg, ctx.block_size, False, *extra)
+        return gx, gw, None, None, None, None, None
 
 
 def grouped_matmul(x: torch.Tensor, w: torch.Tensor, block_to_expert: torch.Tensor, seg_first_block: torch.Tensor,
-                   block_size: int, skip_unused: bool = False) -> torch.Tensor:
+                   block_size: int, skip_unused: bool = False, slot_token: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``y[i·B:(i+1)·B] = x[i·B:(i+1)·B] @ w[block_to_expert[i]]`` with ``x [nb·B, K]``, ``w [E, K, N]``.  With ``skip_unused``
-    the row blocks from ``seg_first_block[E]`` on hold no tokens: their rows of the result are unspecified."""
+    the row blocks from ``seg_first_block[E]`` on hold no tokens: their rows of the result are unspecified.  ``slot_token`` (int32 [nb·B], the
+    token of each row): rows of -1 behind an expert's tokens are zero in ``x`` and in the gradient of ``y``, and the weight gradient skips them."""
     if _grouped_ok(x, w, block_size):
-        return _GroupedMatmul.apply(x, w, block_to_expert.int(), seg_first_block.int(), block_size, skip_unused)
+        return _GroupedMatmul.apply(x, w, block_to_expert.int(), seg_first_block.int(), block_size, skip_unused, slot_token)
     return _grouped_ref(x, w, block_to_expert, block_size)

@@ -73,6 +73,32 @@ class _Combine(torch.autograd.Function):
         return dy, dw, None
 
 
+class _Normalize(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, aff, idx):
+        aff = aff.contiguous()
+        ctx.save_for_backward(aff, idx)
+        _ext.count_launch()
+        return _ext.ext().moe_normalize(aff, idx)
+
+    @staticmethod
+    def backward(ctx, g):
+        aff, idx = ctx.saved_tensors
+        _ext.count_launch()
+        return _ext.ext().moe_normalize_grad(g.contiguous(), aff, idx), None
+
+
+def normalize_ok(aff: torch.Tensor, expert_index: torch.Tensor) -> bool:
+    """fp32 ``[T, E]`` on the device with int64 choices, in a call that nobody records, traces or transforms."""
+    return (aff.dtype == torch.float32 and aff.dim() == 2 and aff.shape[1] <= 256 and expert_index.dtype == torch.int64 and expert_index.dim() == 2
+            and expert_index.device == aff.device and expert_index.shape[0] == aff.shape[0] and _ext.native(aff, expert_index) is not None)
+
+
+def normalize(aff: torch.Tensor, expert_index: torch.Tensor) -> torch.Tensor:
+    """Affinities ``[T, E]`` of the chosen experts divided by their sum (at least 1e-9); the others zero."""
+    return _Normalize.apply(aff, expert_index.contiguous())
+
+
 def gather(x: torch.Tensor, slots: Slots) -> torch.Tensor:
     """``x [T, H]`` → rows in slot order ``[nb * block, H]``; padding rows are zero, rows behind the last used block unspecified."""
     return _Gather.apply(x, slots)

@@ -99,3 +99,55 @@ def test_experts_with_an_activation_of_their_own():
     got.append(blockwise.blockwise_expert_mlp(x, aff, idx, op, 128))
     for y in got:                                           # roundings to bfloat16 on the way, as in test_experts
         assert (y.double() - 2 * want.double()).norm() <= 0.012 * 2 * want.double().norm()
+
+
+@pytest.mark.parametrize("T,E,k,scale", [(1, 1, 1, 1.0), (5, 8, 2, 1.0), (700, 33, 4, 1.0), (129, 256, 8, 1.0), (9, 256, 40, 1.0), (64, 16, 2, 1e-11)])
+def test_normalized_affinities(T, E, k, scale):
+    """Against the chain of plain operations in 64 bits; an expert chosen twice counts once, sums below 1e-9 count as 1e-9."""
+    from neuronx_distributed_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(T + E)
+    aff = (torch.rand(T, E, generator=g, device="cuda") * scale).requires_grad_()
+    idx = torch.randint(0, E, (T, k), generator=g, device="cuda")
+    go = torch.randn(T, E, generator=g, device="cuda")
+    assert ops.moe_blocks.normalize_ok(aff, idx)
+    w = ops.moe_blocks.normalize(aff, idx)
+    got = [w, *torch.autograd.grad(w, aff, go)]
+    a = aff.detach().double().requires_grad_()
+    m = a * torch.zeros_like(a).scatter_(1, idx, 1.0)
+    z = m / m.sum(-1, keepdim=True).clamp(min=1e-9)
+    # sums of up to 256 products in 32 bits, then two quotients: 1e-5 of w, and of what the gradient (go - sum of go * w) / sum subtracts: with
+    # one expert it is zero, a difference of two numbers of the size of go / sum
+    size = (go.double().abs().amax(-1) / m.detach().sum(-1).clamp(min=1e-9)).max()
+    for x, y, bound in zip(got, [z, *torch.autograd.grad(z, a, go.double())], (1.0, size)):
+        assert (x.double() - y).abs().max() <= 1e-5 * bound
+
+
+def test_normalized_affinities_that_are_no_numbers():
+    from neuronx_distributed_b200 import ops
+
+    aff = torch.rand(4, 8, device="cuda")
+    aff[0, 3], aff[1, 2], aff[2, 5] = float("nan"), float("inf"), float("nan")
+    idx = torch.tensor([[3, 1], [2, 0], [0, 1], [6, 7]], device="cuda")
+    mask = torch.zeros_like(aff).scatter_(1, idx, 1.0)
+    want = aff * mask
+    want = want / want.sum(-1, keepdim=True).clamp(min=1e-9)
+    torch.testing.assert_close(ops.moe_blocks.normalize(aff, idx), want, equal_nan=True, rtol=1e-6, atol=0)
+
+
+@pytest.mark.parametrize("counts", [[0, 1, 63, 64, 65], [255, 0, 256, 257, 128], [0, 0, 0, 0, 7], [320, 129, 191, 192, 193]])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_weight_gradients_without_padding(counts, accumulate):
+    """Rows behind an expert's tokens are zero, so that leaving their k-blocks out changes no bit."""
+    from neuronx_distributed_b200 import ops
+
+    E, H, I, block = len(counts), 320, 192, 256
+    idx = torch.cat([torch.full((n,), e) for e, n in enumerate(counts)])[:, None].cuda()
+    nb = sum((n + block - 1) // block for n in counts) + 1
+    s = ops.moe_blocks.make_slots(idx, E, nb, block)
+    g = torch.Generator(device="cuda").manual_seed(sum(counts))
+    x, dy = (torch.randn(nb * block, n, generator=g, device="cuda").bfloat16() * (s.token >= 0)[:, None] for n in (H, I))
+    out = [torch.full((E, H, I), 0.5 if accumulate else float("nan"), device="cuda") for _ in range(2)]
+    ops._ext.ext().grouped_wgrad(x, dy, out[0], s.seg, block, accumulate)
+    ops._ext.ext().grouped_wgrad(x, dy, out[1], s.seg, block, accumulate, s.token)
+    assert torch.equal(out[0], out[1]) and torch.isfinite(out[1]).all()
