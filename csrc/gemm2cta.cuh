@@ -83,6 +83,24 @@ NXD_DEVICE void store_chunk(OutT* orow, int col0, int N, const uint32_t (&r)[32]
   }
 }
 
+// The four products of a k-block and the commit that frees its stage in both CTAs, from a warp that is together: one election, descriptors that
+// advance by constants (steps of 16 bytes).  One lane on its own took about 130 cycles a product, as long as one of 256 columns lasts and
+// twice as long as one of 128.
+template <int STEP_A, int STEP_B>
+NXD_DEVICE void mma4_commit_2cta(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred p, q, t;\n\t.reg .b64 a, b;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "add.s64 a, %1, %6;\n\tadd.s64 b, %2, %9;\n\t@q tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, t;\n\t"
+      "add.s64 a, %1, %7;\n\tadd.s64 b, %2, %10;\n\t@q tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, t;\n\t"
+      "add.s64 a, %1, %8;\n\tadd.s64 b, %2, %11;\n\t@q tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, t;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%5], %12;\n\t}"
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(bar), "n"(STEP_A), "n"(2 * STEP_A), "n"(3 * STEP_A), "n"(STEP_B), "n"(2 * STEP_B),
+        "n"(3 * STEP_B), "h"((uint16_t)3)
+      : "memory");
+}
+
 // Row tiles that go through the columns together.  What the 74 tiles in flight share is read from memory once for each such pass over the columns:
 // all row tiles at once where they are few, so that a large B is read once, near-square rounds (8 x 9 tiles) else.  Training products run under
 // the power cap, where bytes cost time: feed-forward block of 7B, 4096 tokens, both ways, 2731 us with four rows, 2670 so.
@@ -128,11 +146,12 @@ NXD_DEVICE void tma_reduce_add_3d(const CUtensorMap* map, uint32_t smem_src, int
 // as a plain store or added to memory by the copy engine (`add`: gradient accumulation, split-K partials).  A weight gradient is
 // bound by these writes as much as by its products: with one row-strided 16-byte store per thread and instruction the tensor pipe
 // waited for the epilogue.  7B feed-forward weight gradients over 4096 tokens: 846 + 39 us (stores, zeroing for a split) -> 744.
+template <int TN = TILE_N>          // columns of the tile
 NXD_DEVICE void epilogue_tile_tma_f32(uint32_t tmem_acc, uint32_t stage_smem, const CUtensorMap* omap, int row0, int mat, int col0,
                                       int N, int q, int lane, bool issuer, uint32_t& slab_ctr, bool add, bool zero) {
   const int row = q * 32 + lane;
 #pragma unroll 1
-  for (int s = 0; s < TILE_N / 32; ++s) {
+  for (int s = 0; s < TN / 32; ++s) {
     const int c0 = col0 + s * 32;
     if (c0 >= N) break;
     const uint32_t buf = stage_smem + (slab_ctr & 1u) * kEpiSlabBytes;
@@ -169,13 +188,13 @@ NXD_DEVICE void epilogue_tile_tma_f32(uint32_t tmem_acc, uint32_t stage_smem, co
 // write the thread's 128-byte row in the 128B-swizzle pattern (conflict-free: 8 consecutive rows hit 8 different 16-byte
 // bank groups), fence to the async proxy, TMA-store the slab.  Rows/columns beyond the matrix are clipped by TMA.
 // Returns the number of bulk groups committed (slabs inside the matrix).  `slab_ctr` carries the buffer parity.
-template <bool MATS = false>      // MATS: a 3-D map {columns, rows, matrices}, matrix `mat`; `zero`: the accumulator was never written
+template <bool MATS = false, int TN = TILE_N>      // MATS: a 3-D map {columns, rows, matrices}, matrix `mat`; `zero`: the accumulator was never written
 NXD_DEVICE int epilogue_tile_tma(uint32_t tmem_acc, uint32_t stage_smem, const CUtensorMap* omap, int row0, int col0, int N,
                                  int q, int lane, bool issuer, uint32_t& slab_ctr, int mat = 0, bool zero = false) {
   const int row = q * 32 + lane;
   int groups = 0;
 #pragma unroll 1
-  for (int s = 0; s < TILE_N / kEpiSlabCols; ++s) {
+  for (int s = 0; s < TN / kEpiSlabCols; ++s) {
     const int c0 = col0 + s * kEpiSlabCols;
     if (c0 >= N) break;
     const uint32_t buf = stage_smem + (slab_ctr & 1u) * kEpiSlabBytes;

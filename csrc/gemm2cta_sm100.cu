@@ -36,8 +36,8 @@ struct Group {
   const int* slot_token;
 };
 
-// The tiles of the last, partial round of pairs (`tiles` of them, at most half as many as pairs) are split along K over `splits`
-// pairs each, `kb_per` k-blocks apiece; their fp32 partials go to a workspace [tiles * splits][256][256] that gemm_tail_kernel
+// The tiles of the last, partial round of pairs (`tiles` of them) are split along K over `splits`
+// pairs each, `kb_per` k-blocks apiece; their fp32 partials go to a workspace [tiles * splits][256][columns of a tile] that gemm_tail_kernel
 // sums.  80 tiles on 74 pairs took two tiles' time for 1.08 of work.
 struct Tail { int tiles, splits, kb_per; };
 
@@ -81,7 +81,15 @@ NXD_DEVICE Unit unit_of(int unit, int num_tiles, int tiles_m, int tiles_n, int n
   return u;
 }
 
-template <bool A_KMAJOR, bool B_KMAJOR, typename OutT, int MODE>
+// Stages, shared memory and accumulators for tiles of TN columns: 256, or 128 where an output has too few of those to fill the chip.
+template <int TN>
+struct Shape {
+  static constexpr int kHalfN = TN / 2, kBytesB = kHalfN * BK * 2, kBytes = kABytes + kBytesB, kRing = TN == 256 ? kStages : 8;
+  static constexpr int kEpi = kRing * kBytes, kBars = kEpi + kEpiBufs * kEpiSlabBytes, kShared = kBars + 1024 + 256;
+  static_assert(kShared <= 232448, "exceeds the 227 KB of dynamic shared memory per CTA");
+};
+
+template <bool A_KMAJOR, bool B_KMAJOR, typename OutT, int MODE, int TN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                       const __grid_constant__ CUtensorMap tma_out, const __grid_constant__ CUtensorMap tma_part, OutT* out,
@@ -89,19 +97,20 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   // accumulate: 0 store, 1 add to what is there.  split_k > 1 (fp32 outputs): that many pairs share one output tile, each sums
   // a K range and adds its partial — for weight gradients whose output has too few tiles to fill the 74 pairs while
   // K = tokens is long.  fp32 outputs always leave through TMA (stored or added in memory), bf16 ones unless they accumulate.
+  using S = Shape<TN>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint64_t* bars = (uint64_t*)(smem + kBarOffset);
-  uint32_t* tmem_slot = (uint32_t*)(bars + 2 * kStages + 2 * kAcc);
-  const uint32_t bar_full = smem_u32(bars), bar_empty = smem_u32(bars + kStages);
-  const uint32_t bar_tfull = smem_u32(bars + 2 * kStages), bar_tempty = smem_u32(bars + 2 * kStages + kAcc);
+  uint64_t* bars = (uint64_t*)(smem + S::kBars);
+  uint32_t* tmem_slot = (uint32_t*)(bars + 2 * S::kRing + 2 * kAcc);
+  const uint32_t bar_full = smem_u32(bars), bar_empty = smem_u32(bars + S::kRing);
+  const uint32_t bar_tfull = smem_u32(bars + 2 * S::kRing), bar_tempty = smem_u32(bars + 2 * S::kRing + kAcc);
   const uint32_t smem_base = smem_u32(smem);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t cta = cluster_ctarank();
   const bool leader = cta == 0;
   int tiles_m = (M + TILE_M - 1) / TILE_M;
-  const int tiles_n = (N + TILE_N - 1) / TILE_N;
+  const int tiles_n = (N + TN - 1) / TN;
   if constexpr (MODE == 3) { if (grp.used_blocks) tiles_m = min(tiles_m, *grp.used_blocks * (grp.block_rows / TILE_M)); }
   const int num_tiles = (MODE == 4 ? grp.groups : 1) * tiles_m * tiles_n;
   const int num_kb = (K + BK - 1) / BK;
@@ -112,7 +121,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   if (warp == 0 && lane == 0) {
     prefetch_tmap(&tma_a);
     prefetch_tmap(&tma_b);
-    for (int i = 0; i < kStages; ++i) {
+    for (int i = 0; i < S::kRing; ++i) {
       mbar_init(bar_full + 8 * i, 2);     // leader: own arrive.expect_tx + peer's remote arrive
       mbar_init(bar_empty + 8 * i, 1);    // one multicast tcgen05.commit
     }
@@ -123,7 +132,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     fence_barrier_init();
   }
   __syncwarp();
-  if (warp == 1) { tcgen05_alloc_2cta(smem_u32(tmem_slot), kTmemCols); tcgen05_relinquish_2cta(); }
+  if (warp == 1) { tcgen05_alloc_2cta(smem_u32(tmem_slot), kAcc * TN); tcgen05_relinquish_2cta(); }
   tcgen05_fence_before();
   cluster_sync_all();               // barriers of both CTAs are initialised before any remote arrive
   tcgen05_fence_after();
@@ -140,15 +149,15 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       for (int unit = pair; unit < num_units; unit += num_pairs) {
         const Unit u = unit_of<MODE>(unit, num_tiles, tiles_m, tiles_n, num_kb, kb_per, grp, tail);
         const int m0 = u.m_blk * TILE_M + (int)cta * CTA_M;
-        const int n0 = u.n_blk * TILE_N + (int)cta * HALF_N;
+        const int n0 = u.n_blk * TN + (int)cta * S::kHalfN;
         int b_off = 0;
         if constexpr (MODE == 3) b_off = grp.block_expert[u.m_blk * TILE_M / grp.block_rows] * grp.b_rows;
         for (int kb = u.kb0; kb < u.kb1; ++kb) {
           mbar_wait(bar_empty + 8 * stage, phase ^ 1);
           const uint32_t full = bar_full + 8 * stage;          // same offset in the leader's smem
-          if (leader) mbar_expect_tx(full, 2 * kStageBytes);
+          if (leader) mbar_expect_tx(full, 2 * S::kBytes);
           else mbar_arrive_cluster(mapa_shared(full, 0));
-          const uint32_t sa = smem_base + stage * kStageBytes, sb = sa + kABytes;
+          const uint32_t sa = smem_base + stage * S::kBytes, sb = sa + kABytes;
           const int k0 = kb * BK;
           if constexpr (A_KMAJOR) {
             tma_load_2d_2cta(sa, &tma_a, full, k0, m0);                          // box {64 k, 128 m}
@@ -160,38 +169,33 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
             tma_load_2d_2cta(sb, &tma_b, full, k0, b_off + n0);                  // box {64 k, 128 n}
           } else {
 #pragma unroll
-            for (int j = 0; j < HALF_N / 64; ++j) tma_load_2d_2cta(sb + j * 8192, &tma_b, full, n0 + j * 64, b_off + k0);
+            for (int j = 0; j < S::kHalfN / 64; ++j) tma_load_2d_2cta(sb + j * 8192, &tma_b, full, n0 + j * 64, b_off + k0);
           }
-          if (++stage == kStages) { stage = 0; phase ^= 1; }
+          if (++stage == S::kRing) { stage = 0; phase ^= 1; }
         }
       }
     }
     __syncwarp();
   } else if (warp == 1) {
     // ===== MMA issuer (leader CTA only) =====
-    if (leader && lane == 0) {
-      constexpr uint32_t idesc = make_idesc(!A_KMAJOR, !B_KMAJOR, TILE_M, TILE_N);
+    if (leader) {                                          // all lanes; the helpers elect one
+      constexpr uint32_t idesc = make_idesc(!A_KMAJOR, !B_KMAJOR, TILE_M, TN);
       int stage = 0; uint32_t phase = 0; int as = 0; uint32_t aphase = 0;
       for (int unit = pair; unit < num_units; unit += num_pairs) {
         const Unit u = unit_of<MODE>(unit, num_tiles, tiles_m, tiles_n, num_kb, kb_per, grp, tail);
         mbar_wait(bar_tempty + 8 * as, aphase ^ 1);
         tcgen05_fence_after();
-        const uint32_t tmem_d = tmem_base + as * TILE_N;
-        const int kb0 = u.kb0, kb1 = u.kb1;
-        for (int kb = kb0; kb < kb1; ++kb) {
+        const uint32_t tmem_d = tmem_base + as * TN;
+        for (int kb = u.kb0; kb < u.kb1; ++kb) {
           mbar_wait(bar_full + 8 * stage, phase);
           tcgen05_fence_after();
-          const uint32_t sa = smem_base + stage * kStageBytes, sb = sa + kABytes;
-#pragma unroll
-          for (int k = 0; k < BK / UK; ++k) {
-            const uint64_t da = A_KMAJOR ? make_smem_desc(sa + k * 32, 16, 1024) : make_smem_desc(sa + k * 2048, 8192, 1024);
-            const uint64_t db = B_KMAJOR ? make_smem_desc(sb + k * 32, 16, 1024) : make_smem_desc(sb + k * 2048, 8192, 1024);
-            tcgen05_mma_f16_2cta(tmem_d, da, db, idesc, ((kb - kb0) | k) != 0 ? 1u : 0u);
-          }
-          tcgen05_commit_2cta(bar_empty + 8 * stage, 0b11);    // frees the stage in BOTH CTAs
-          if (++stage == kStages) { stage = 0; phase ^= 1; }
+          const uint32_t sa = smem_base + stage * S::kBytes, sb = sa + kABytes;
+          mma4_commit_2cta<A_KMAJOR ? 2 : 128, B_KMAJOR ? 2 : 128>(tmem_d, A_KMAJOR ? make_smem_desc(sa, 16, 1024) : make_smem_desc(sa, 8192, 1024),
+                                                                   B_KMAJOR ? make_smem_desc(sb, 16, 1024) : make_smem_desc(sb, 8192, 1024), idesc,
+                                                                   kb != u.kb0 ? 1u : 0u, bar_empty + 8 * stage);
+          if (++stage == S::kRing) { stage = 0; phase ^= 1; }
         }
-        tcgen05_commit_2cta(bar_tfull + 8 * as, 0b11);         // accumulators ready in both CTAs
+        tcgen05_commit_2cta_e(bar_tfull + 8 * as, 0b11);       // accumulators ready in both CTAs
         if (++as == kAcc) { as = 0; aphase ^= 1; }
       }
     }
@@ -207,23 +211,23 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       const Unit u = unit_of<MODE>(unit, num_tiles, tiles_m, tiles_n, num_kb, kb_per, grp, tail);
       mbar_wait(bar_tfull + 8 * as, aphase);
       tcgen05_fence_after();
-      const int n0 = u.n_blk * TILE_N, row0 = u.m_blk * TILE_M + (int)cta * CTA_M;
-      const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + as * TILE_N;
+      const int n0 = u.n_blk * TN, row0 = u.m_blk * TILE_M + (int)cta * CTA_M;
+      const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + as * TN;
       const bool empty = MODE == 4 && u.kb0 == u.kb1;
       if (MODE == 0 && u.part) {
-        epilogue_tile_tma_f32(acc, smem_base + kEpiOffset, &tma_part, (int)cta * CTA_M, u.mat, 0, TILE_N, q, lane, issuer, slab_ctr,
+        epilogue_tile_tma_f32<TN>(acc, smem_base + S::kEpi, &tma_part, (int)cta * CTA_M, u.mat, 0, TN, q, lane, issuer, slab_ctr,
                               false, false);
       } else if constexpr (sizeof(OutT) == 4) {
-        epilogue_tile_tma_f32(acc, smem_base + kEpiOffset, &tma_out, row0, u.mat, n0, N, q, lane, issuer, slab_ctr,
+        epilogue_tile_tma_f32<TN>(acc, smem_base + S::kEpi, &tma_out, row0, u.mat, n0, N, q, lane, issuer, slab_ctr,
                               accumulate || split_k > 1, empty);
       } else if (!accumulate) {
-        epilogue_tile_tma<MODE == 4>(acc, smem_base + kEpiOffset, &tma_out, row0, n0, N, q, lane, issuer, slab_ctr, u.mat, empty);
+        epilogue_tile_tma<MODE == 4, TN>(acc, smem_base + S::kEpi, &tma_out, row0, n0, N, q, lane, issuer, slab_ctr, u.mat, empty);
       } else {
         const int row = row0 + q * 32 + lane;
         OutT* orow = out + ((size_t)u.mat * M + row) * N;
         const bool row_ok = row < M;
 #pragma unroll 1
-        for (int c = 0; c < TILE_N / 32; ++c) {
+        for (int c = 0; c < TN / 32; ++c) {
           uint32_t r[32];
           tcgen05_ld_32x32(acc + c * 32, r);
           tcgen05_wait_ld();
@@ -240,26 +244,27 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
 
   tcgen05_fence_before();
   cluster_sync_all();               // peer must be done with our smem/TMEM before teardown
-  if (warp == 1) { __syncwarp(); tcgen05_dealloc_2cta(tmem_base, kTmemCols); }
+  if (warp == 1) { __syncwarp(); tcgen05_dealloc_2cta(tmem_base, kAcc * TN); }
 }
 
 // out tile (+)= sum of its splits' partials, in order: one thread per 8 columns of a row
-template <typename OutT>
+template <typename OutT, int TN>
 __global__ void __launch_bounds__(256) gemm_tail_kernel(const float* part, OutT* out, int M, int N, int first,
                                                         int tiles_m, int tiles_n, int splits, int accumulate) {
   pdl_trigger();
   pdl_wait();
-  const int t = blockIdx.y, row = blockIdx.x * 8 + (threadIdx.x >> 5), col = (threadIdx.x & 31) * 8;
+  constexpr int kPer = TN / 8;                             // threads of a row
+  const int t = blockIdx.y, row = blockIdx.x * (256 / kPer) + threadIdx.x / kPer, col = threadIdx.x % kPer * 8;
   int m_blk, n_blk;
   tile_coords(first + t, tiles_m, tiles_n, raster_rows(tiles_m), m_blk, n_blk);
-  const int gr = m_blk * TILE_M + row, gc = n_blk * TILE_N + col;
+  const int gr = m_blk * TILE_M + row, gc = n_blk * TN + col;
   if (gr >= M || gc >= N) return;                          // N is a multiple of 8
-  const float* src = part + ((size_t)t * splits * TILE_M + row) * TILE_N + col;
+  const float* src = part + ((size_t)t * splits * TILE_M + row) * TN + col;
   float a[8] = {};
 #pragma unroll 4
   for (int s = 0; s < splits; ++s) {
-    const float4 x = *reinterpret_cast<const float4*>(src + (size_t)s * TILE_M * TILE_N);
-    const float4 y = *reinterpret_cast<const float4*>(src + (size_t)s * TILE_M * TILE_N + 4);
+    const float4 x = *reinterpret_cast<const float4*>(src + (size_t)s * TILE_M * TN);
+    const float4 y = *reinterpret_cast<const float4*>(src + (size_t)s * TILE_M * TN + 4);
     a[0] += x.x; a[1] += x.y; a[2] += x.z; a[3] += x.w; a[4] += y.x; a[5] += y.y; a[6] += y.z; a[7] += y.w;
   }
   OutT* dst = out + (size_t)gr * N + gc;
@@ -777,17 +782,18 @@ int device_sm_count();
 
 CUtensorMap make_tmap_mats(const void* ptr, bool f32, uint64_t mats, uint64_t rows, uint64_t cols, uint32_t box_cols, uint32_t box_rows);
 
-template <bool AK, bool BK_, typename OutT, int MODE = 0>
+template <bool AK, bool BK_, typename OutT, int MODE = 0, int TN = g2::TILE_N>
 static void launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& to, const CUtensorMap& tp, void* out, int M, int N, int K,
                     int accumulate, int split_k, const g2::Group& grp, const g2::Tail& tail, int grid, cudaStream_t st) {
-  auto kern = g2::gemm_bf16_2cta_kernel<AK, BK_, OutT, MODE>;
-  NXD_ALLOW_SMEM(kern, g2::kSmem);
+  auto kern = g2::gemm_bf16_2cta_kernel<AK, BK_, OutT, MODE, TN>;
+  constexpr int smem = g2::Shape<TN>::kShared;
+  NXD_ALLOW_SMEM(kern, smem);
   // A dependent: barriers, TMEM and maps of the next product are set up beside the end of this one (1 x 1000 tokens of 13B: 1152 us, 1130 with
   // products, their tails, norms, SwiGLU and rotation so).  Not the grouped ones: they read the blocks' experts first and gain nothing.
   if (MODE == 0) {
-    launch_dependent(kern, grid, g2::kThreads, g2::kSmem, st, ta, tb, to, tp, (OutT*)out, M, N, K, accumulate, split_k, grp, tail);
+    launch_dependent(kern, grid, g2::kThreads, smem, st, ta, tb, to, tp, (OutT*)out, M, N, K, accumulate, split_k, grp, tail);
   } else {
-    kern<<<grid, g2::kThreads, g2::kSmem, st>>>(ta, tb, to, tp, (OutT*)out, M, N, K, accumulate, split_k, grp, tail);
+    kern<<<grid, g2::kThreads, smem, st>>>(ta, tb, to, tp, (OutT*)out, M, N, K, accumulate, split_k, grp, tail);
     NXD_CUDA_CHECK(cudaGetLastError());
   }
 }
@@ -800,44 +806,57 @@ static CUtensorMap out_map(const void* out, int out_dt, bool accumulate, bool ma
   return mats ? make_tmap_mats(out, false, groups, M, N, g2::kEpiSlabCols, g2::CTA_M) : make_tmap_bf16(out, M, N, g2::kEpiSlabCols, g2::CTA_M);
 }
 
-// How a product is shared out: split-K of every tile (fp32 outputs), or of the last round's tiles alone, or neither.  Time of a
-// 256 x 256 tile: 0.39 us per k-block; a pass over fp32 memory: 6 bytes/ps.
-struct GemmPlan { int tiles, split; g2::Tail tail; };
+// How a product is shared out: tiles of 256 or 128 columns; split-K of every tile (fp32 outputs), or of the last round's tiles alone, or neither.
+// A k-block of a 256 x 256 tile takes 0.31 us and one of 256 x 128 0.23 (their operands, 32 and 24 KB a CTA, come at about 105 GB/s an SM), a
+// launch 5; a pass over fp32 memory: 6 bytes/ps.
+struct GemmPlan { int tiles, split, width; g2::Tail tail; };      // width: columns of a tile
 static GemmPlan gemm_plan(int M, int N, int K, int out_dt, bool accumulate, bool split_k) {
   const int pairs = std::max(1, device_sm_count() / 2), num_kb = (K + g2::BK - 1) / g2::BK;      // (no device: one, for the asking)
+  const int tiles_m = (M + g2::TILE_M - 1) / g2::TILE_M;
   GemmPlan p;
-  p.tiles = ((M + g2::TILE_M - 1) / g2::TILE_M) * ((N + g2::TILE_N - 1) / g2::TILE_N);
-  p.split = 1;
-  p.tail = g2::Tail{0, 1, num_kb};
-  const double kb_us = 0.39;
-  double best = (double)((p.tiles + pairs - 1) / pairs) * num_kb * kb_us;
-  // The tail: s pairs per tile, at least 4 k-blocks each; worth it where it saves more than the launch that sums (4 us) and its traffic
-  // (256 x 1024 x 1024 stays whole: 14.3 us, 17.4 with a tail).
-  // 1000 x 5120 x 13824 (80 tiles): 104 us, 143 with a second round of six tiles; cut into narrower columns instead, its pieces waited
-  // for their loads as long as a whole tile.  1000 x 27648 x 5120 from [K, N] weights: 203, 281 before.
-  // Rows of other lengths have no tail: gemm_tail_kernel writes whole groups of 8 columns.
-  const int last = N % 8 == 0 ? p.tiles % pairs : 0;
-  int s = last > 0 ? std::min(16, std::min(pairs / last, num_kb / 4)) : 1;
-  if (s > 1) {
-    const int per = (num_kb + s - 1) / s;
-    s = (num_kb + per - 1) / per;                          // no empty split
-    const double cost = (p.tiles / pairs) * num_kb * kb_us + per * kb_us + 4.0 + 2.0 * last * s * 0.262144 / 6.0;
-    if (s > 1 && cost < best) { best = cost; p.tail = g2::Tail{last, s, per}; }
+  double best = 1e30;
+  for (int width = 256; width >= 128; width /= 2) {
+    const double kb_us = width == 256 ? 0.31 : 0.2325;
+    const int tiles = tiles_m * ((N + width - 1) / width);
+    // The tail: the tiles of the last, partial round in s parts each, which may be several rounds themselves; worth it where it saves more than
+    // the launch that sums (2 us) and its traffic.  Chosen so and before (256 columns, s pairs a tile in one round), us: 512 x 5120 x 13824 in 3
+    // parts 64 and 74; 704 x 4096 x 11008 in 3 parts 56 and 62; 304 x 4096 x 4096 in 128 columns 19.6 and 21.2, 304 x 1024 x 2816 in 128 columns
+    // and 4 parts 10.6 and 15.8, 1000 x 1024 x 1024 in 128 columns 8.2 and 10.0; 1000 x 5120 x 13824 (80 tiles) 101 in 5 parts, 147 without.  66
+    // such products of 200 to 1504 rows: none slower than before by more than its noise but one (200 x 4096 x 11008, 37 and 34), a twelfth of a per
+    // cent from the best of all these choices in the mean.
+    // Rows of other lengths have no tail: gemm_tail_kernel writes whole groups of 8 columns.
+    const int last = N % 8 == 0 ? tiles % pairs : 0;
+    for (int s = 1; s <= (last > 0 ? 16 : 1); ++s) {
+      const int per = (num_kb + s - 1) / s;
+      if (s > 1 && (num_kb / s < 4 || per * (s - 1) >= num_kb)) continue;      // short parts, or an empty one
+      const int rounds = (last * s + pairs - 1) / pairs;
+      double cost = ((tiles / pairs) * num_kb + rounds * per) * kb_us + (s > 1 ? 2.0 + 2.0 * last * s * width * 0.001024 / 7.0 : 0.);
+      if (s > 1) cost /= 0.97;                             // a tie stays whole
+      if (cost < best) {
+        best = cost;
+        p.tiles = tiles; p.split = 1; p.width = width;
+        p.tail = s > 1 ? g2::Tail{last, s, per} : g2::Tail{0, 1, num_kb};
+      }
+    }
   }
   // Split-K for fp32 outputs (weight gradients): K = tokens is long while the output often has fewer tiles than the
   // chip has CTA pairs (TP=8: 32-176 tiles on 74 pairs).  A split is taken where the waves it saves cost more than its traffic:
   // zeroing the output first and one more pass over it per further partial; every split keeps >= 16 k-blocks so that the main
   // loop still amortises its epilogue.  Its partials are added in any order.  Outputs of fewer rows than a tile never take it: their few
-  // tiles are a tail, whose partials are summed in order, so that the same inputs give the same bits (128 x 4096 over 8192 tokens: 21.4 us
-  // stored, 22.0 added to what is there; 20.4 and 16.4 with partials added in any order, 55 and 60 without a split).
+  // tiles are a tail, whose partials are summed in order, so that the same inputs give the same bits.
   if (out_dt == kF32 && M >= g2::TILE_M && split_k) {
+    const int tiles = tiles_m * ((N + g2::TILE_N - 1) / g2::TILE_N);
     const double pass_us = (double)M * N * 4 / 6e6;
     for (int s2 = 2; s2 <= 8; ++s2) {
       if (num_kb / s2 < 16) break;
       const int per = (num_kb + s2 - 1) / s2;
       if (per * (s2 - 1) >= num_kb) continue;                       // would leave an empty split
-      const double cost = (double)((p.tiles * s2 + pairs - 1) / pairs) * per * kb_us + (s2 - 1) * pass_us + (accumulate ? 0. : pass_us);
-      if (cost < best) { best = cost; p.split = s2; p.tail = g2::Tail{0, 1, num_kb}; }
+      const double cost = (double)((tiles * s2 + pairs - 1) / pairs) * per * 0.31 + (s2 - 1) * pass_us + (accumulate ? 0. : pass_us);
+      if (cost < best) {
+        best = cost;
+        p.tiles = tiles; p.split = s2; p.width = g2::TILE_N;
+        p.tail = g2::Tail{0, 1, num_kb};
+      }
     }
   }
   return p;
@@ -846,7 +865,7 @@ static GemmPlan gemm_plan(int M, int N, int K, int out_dt, bool accumulate, bool
 // bytes of fp32 workspace that gemm_bf16_2cta takes for these sizes (0: none)
 size_t gemm_2cta_workspace(int M, int N, int K, int out_dt, bool accumulate, bool split_k) {
   const GemmPlan p = gemm_plan(M, N, K, out_dt, accumulate, split_k);
-  return (size_t)p.tail.tiles * p.tail.splits * g2::TILE_M * g2::TILE_N * sizeof(float);
+  return (size_t)p.tail.tiles * p.tail.splits * g2::TILE_M * p.width * sizeof(float);
 }
 
 // `split_k`: fp32 outputs may be sums in any order; `workspace`: gemm_2cta_workspace bytes, 16-byte aligned, or null: then no tail is split
@@ -854,33 +873,36 @@ void gemm_bf16_2cta(const void* a, const void* b, void* out, int M, int N, int K
                     bool accumulate, bool split_k, float* workspace, cudaStream_t st) {
   const bool AK = !trans_a, BK_ = trans_b;
   const CUtensorMap ta = AK ? make_tmap_bf16(a, M, K, g2::BK, g2::CTA_M) : make_tmap_bf16(a, K, M, 64, g2::BK);
-  const CUtensorMap tb = BK_ ? make_tmap_bf16(b, N, K, g2::BK, g2::HALF_N) : make_tmap_bf16(b, K, N, 64, g2::BK);
-  const CUtensorMap to = out_map(out, out_dt, accumulate, false, 1, M, N, ta);
   GemmPlan p = gemm_plan(M, N, K, out_dt, accumulate, split_k);
+  const CUtensorMap tb = BK_ ? make_tmap_bf16(b, N, K, g2::BK, p.width / 2) : make_tmap_bf16(b, K, N, 64, g2::BK);
+  const CUtensorMap to = out_map(out, out_dt, accumulate, false, 1, M, N, ta);
   if (!workspace) p.tail = g2::Tail{0, 1, 1};
   const int pairs = device_sm_count() / 2, split = p.split;
   if (split > 1 && !accumulate) NXD_CUDA_CHECK(cudaMemsetAsync(out, 0, (size_t)M * N * sizeof(float), st));   // partials add into zeros
-  const CUtensorMap tp = p.tail.tiles ? make_tmap_mats(workspace, true, (uint64_t)p.tail.tiles * p.tail.splits, g2::TILE_M, g2::TILE_N, 32, g2::CTA_M) : ta;
+  const CUtensorMap tp = p.tail.tiles ? make_tmap_mats(workspace, true, (uint64_t)p.tail.tiles * p.tail.splits, g2::TILE_M, p.width, 32, g2::CTA_M) : ta;
   const int units = p.tiles * split + p.tail.tiles * (p.tail.splits - 1);
   const int grid = 2 * (units < pairs ? units : pairs);
   const g2::Group none{};
-#define NXD_L2(AKv, BKv)                                                                          \
-  do {                                                                                            \
-    if (out_dt == kBF16) launch2<AKv, BKv, __nv_bfloat16>(ta, tb, to, tp, out, M, N, K, accumulate, split, none, p.tail, grid, st); \
-    else launch2<AKv, BKv, float>(ta, tb, to, tp, out, M, N, K, accumulate, split, none, p.tail, grid, st); \
+#define NXD_L2W(AKv, BKv, OutT, W) launch2<AKv, BKv, OutT, 0, W>(ta, tb, to, tp, out, M, N, K, accumulate, split, none, p.tail, grid, st)
+#define NXD_L2(AKv, BKv)                                                                                              \
+  do {                                                                                                                \
+    if (out_dt == kBF16) { if (p.width == 128) NXD_L2W(AKv, BKv, __nv_bfloat16, 128); else NXD_L2W(AKv, BKv, __nv_bfloat16, 256); } \
+    else { if (p.width == 128) NXD_L2W(AKv, BKv, float, 128); else NXD_L2W(AKv, BKv, float, 256); }                    \
   } while (0)
   if (AK && BK_) NXD_L2(true, true);
   else if (AK && !BK_) NXD_L2(true, false);
   else if (!AK && !BK_) NXD_L2(false, false);
   else NXD_L2(false, true);
 #undef NXD_L2
+#undef NXD_L2W
   if (p.tail.tiles) {
-    const int tiles_m = (M + g2::TILE_M - 1) / g2::TILE_M, tiles_n = (N + g2::TILE_N - 1) / g2::TILE_N;
-    const dim3 tg(g2::TILE_M / 8, p.tail.tiles);
-    if (out_dt == kBF16)
-      launch_dependent(g2::gemm_tail_kernel<__nv_bfloat16>, tg, 256, 0, st, (const float*)workspace, (__nv_bfloat16*)out, M, N, p.tiles - p.tail.tiles, tiles_m, tiles_n, p.tail.splits, accumulate);
-    else
-      launch_dependent(g2::gemm_tail_kernel<float>, tg, 256, 0, st, (const float*)workspace, (float*)out, M, N, p.tiles - p.tail.tiles, tiles_m, tiles_n, p.tail.splits, accumulate);
+    const int tiles_m = (M + g2::TILE_M - 1) / g2::TILE_M, tiles_n = (N + p.width - 1) / p.width;
+    const dim3 tg(g2::TILE_M * p.width / 2048, p.tail.tiles);
+    auto sum = [&](auto kernel, auto* o) {
+      launch_dependent(kernel, tg, 256, 0, st, (const float*)workspace, o, M, N, p.tiles - p.tail.tiles, tiles_m, tiles_n, p.tail.splits, (int)accumulate);
+    };
+    if (out_dt == kBF16) sum(p.width == 128 ? g2::gemm_tail_kernel<__nv_bfloat16, 128> : g2::gemm_tail_kernel<__nv_bfloat16, 256>, (__nv_bfloat16*)out);
+    else sum(p.width == 128 ? g2::gemm_tail_kernel<float, 128> : g2::gemm_tail_kernel<float, 256>, (float*)out);
     NXD_CUDA_CHECK(cudaGetLastError());
   }
 }

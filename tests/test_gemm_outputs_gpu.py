@@ -99,3 +99,23 @@ def test_output_views_of_any_alignment():
             # fp32 sums over 72 terms; stored and added to, each with one rounding to bfloat16 (2^-9)
             assert (out.double() - want).abs().max() <= (2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -18) * want.abs().max()
             assert flat[0] == 0 and flat[-1] == 0
+
+
+# more parts than pairs of SMs: the tail (48 tiles in 3 parts each) itself takes several rounds
+@pytest.mark.parametrize("M,N,K", [(704, 4096, 11008), (700, 4088, 11016)])
+@pytest.mark.parametrize("trans", [(False, True), (False, False)])
+def test_tail_of_many_parts(M, N, K, trans):
+    from neuronx_distributed_b200 import ops
+
+    e = ops._ext.ext()
+    assert e.gemm_2cta_workspace(M, N, K, False, False) > 0
+    g = torch.Generator(device="cuda").manual_seed(N)
+    a = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    b = torch.randn(*((N, K) if trans[1] else (K, N)), generator=g, device="cuda").bfloat16()
+    out = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    e.gemm_bf16_2cta(a, b, out, trans[0], trans[1], False)
+    want = a.double() @ (b.double().t() if trans[1] else b.double())
+    assert (out.double() - want).abs().max() <= 2.0 ** -8 * want.abs().max() + 2.0 ** -20 * K       # fp32 sums over K terms, one rounding
+    again = torch.empty_like(out)
+    e.gemm_bf16_2cta(a, b, again, trans[0], trans[1], False)
+    assert torch.equal(out, again)
