@@ -381,7 +381,11 @@ void decode_attention(const void* q, const void* k, const void* v, const long* p
   switch (G) {
     case 1: NXD_DEC(1); break;
     case 2: NXD_DEC(2); break;
+    case 3: NXD_DEC(3); break;
     case 4: NXD_DEC(4); break;
+    case 5: NXD_DEC(5); break;
+    case 6: NXD_DEC(6); break;
+    case 7: NXD_DEC(7); break;
     case 8: NXD_DEC(8); break;
     default: nxd_throw("decode_attention: unsupported GQA group size", __FILE__, __LINE__);
   }

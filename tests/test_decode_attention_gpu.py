@@ -68,3 +68,24 @@ def test_numbers_of_stretches(batch, kv_heads, group, rows):
     want = _reference(q, k, v, pos)
     got = ops.attention.decode_attention(q, k, v, pos).float()
     assert (got - want).abs().max() <= 2.0 ** -8 * want.abs().max()
+
+
+@pytest.mark.parametrize("group", [3, 5, 6, 7])
+@pytest.mark.parametrize("rows,positions", [(1, [0, 0]), (130, [63, 64]), (700, [300, 699]), (2500, [2499, 40])])
+def test_groups_of_other_sizes(group, rows, positions):
+    from neuronx_distributed_b200 import ops
+
+    assert ops.attention.decode_group_ok(*(torch.empty(2, 1, n, 128, dtype=torch.bfloat16, device="cuda") for n in (2 * group, 2, 2)))
+    test_edges(group, rows, positions)
+
+
+def test_rows_that_are_no_packets_go_the_general_way():
+    from neuronx_distributed_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(7)
+    k, v = (torch.randn(2, 200, 2, 132, generator=g, device="cuda").bfloat16()[..., 1:129] for _ in range(2))
+    q = torch.randn(2, 1, 12, 128, generator=g, device="cuda").bfloat16()
+    pos = torch.tensor([199, 60], device="cuda")
+    want = _reference(q, k, v, pos)
+    got = ops.attention.decode_attention(q, k, v, pos).float()
+    assert not ops.attention.decode_group_ok(q, k, v) and (got - want).abs().max() <= 2.0 ** -7 * want.abs().max()      # general way: bf16 probabilities too
