@@ -41,6 +41,18 @@ NXD_DEVICE void tcgen05_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
 NXD_DEVICE void prefetch_l2_tile(const CUtensorMap* map, int c0, int c1) {
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(c0), "r"(c1) : "memory");
 }
+// the four products of a k-block and the commit that frees its stage, from a warp that is together (one election; descriptors advance by 32 bytes)
+NXD_DEVICE void mma4_commit(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred p, q, t;\n\t.reg .b64 a, b;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "add.s64 a, %1, 2;\n\tadd.s64 b, %2, 2;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t"
+      "add.s64 a, %1, 4;\n\tadd.s64 b, %2, 4;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t"
+      "add.s64 a, %1, 6;\n\tadd.s64 b, %2, 6;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n\t}"
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(bar) : "memory");
+}
 NXD_DEVICE float4 ld_cluster_f4(uint32_t addr) {
   float4 v;
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
@@ -93,21 +105,16 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc(false, false, kSlab, TN);
-      int st = 0; uint32_t ph = 0;
-      for (int kb = kb0; kb < kb1; ++kb) {
-        mbar_wait(bar_full + 8 * st, ph);
-        tcgen05_fence_after();
-        const uint32_t sw = base + st * stage_bytes, sx = sw + kWBytes;
-#pragma unroll
-        for (int k = 0; k < BK / 16; ++k)
-          tcgen05_mma_f16(tmem, make_smem_desc(sw + k * 32, 16, 1024), make_smem_desc(sx + k * 32, 16, 1024), idesc, (kb > kb0 || k) ? 1u : 0u);
-        tcgen05_commit(bar_empty + 8 * st);
-        if (++st == stages) { st = 0; ph ^= 1; }
-      }
-      tcgen05_commit(bar_done);
+    const uint32_t idesc = make_idesc(false, false, kSlab, TN);
+    int st = 0; uint32_t ph = 0;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      mbar_wait(bar_full + 8 * st, ph);
+      tcgen05_fence_after();
+      const uint32_t sw = base + st * stage_bytes;
+      mma4_commit(tmem, make_smem_desc(sw, 16, 1024), make_smem_desc(sw + kWBytes, 16, 1024), idesc, kb > kb0 ? 1u : 0u, bar_empty + 8 * st);
+      if (++st == stages) { st = 0; ph ^= 1; }
     }
+    tcgen05_commit_e(bar_done);
     __syncwarp();
   }
   // ---- partial → shared memory as [token][128] fp32 over the ring (its last tile has been multiplied)
