@@ -99,6 +99,12 @@ NXD_DEVICE uint64_t add2(uint64_t a, uint64_t b) { uint64_t d; asm("add.rn.f32x2
 NXD_DEVICE uint64_t mul2(uint64_t a, uint64_t b) { uint64_t d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 NXD_DEVICE float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 
+NXD_DEVICE float silu_mul(float gate, float up) { return gate / (1.f + __expf(-gate)) * up; }
+// SwiGLU of two fp32 products as the kernels that store them first see them: rounded to bf16
+NXD_DEVICE float silu_mul_bf16(float gate, float up) {
+  return silu_mul(__bfloat162float(__float2bfloat16_rn(gate)), __bfloat162float(__float2bfloat16_rn(up)));
+}
+
 NXD_DEVICE float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

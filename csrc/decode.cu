@@ -396,14 +396,27 @@ void decode_attention(const void* q, const void* k, const void* v, const long* p
   NXD_CUDA_CHECK(cudaGetLastError());
 }
 
+// Rows of x for which the vector kernel is the faster one (the figures stand in gemv_bf16)
+static bool vector_rows(int M, int N, int K) {
+  const bool tiny = (long)N * K <= ((long)M * K < 4096 ? 8l << 20 : (long)M * K < 8192 ? 4l << 20 : 0);
+  return !((M >= 3 && !tiny) || (M == 2 && (long)N * K >= 28l << 20));
+}
+
+// y [M, I] = SwiGLU of x [M, K] · w [2 I, K]ᵀ for up to 8 rows; false: rows for the vector kernel, which is faster with a launch of SwiGLU behind it
+// than with a gate and an up row a warp (a token of 13B: 310.9 us, and 313.2 on the same scale)
+bool gemv_swiglu(const void* x, const void* w, void* y, int M, int I, int K, cudaStream_t st) {
+  if (vector_rows(M, 2 * I, K)) return false;
+  gemm_few_rows_swiglu(x, w, y, M, I, K, st);
+  return true;
+}
+
 void gemv_bf16(const void* x, const void* w, const void* residual, void* y, int M, int N, int K, cudaStream_t st) {
   // From three rows on (two where the weights are large) the vector kernel is bound by its multiply-adds and loads of x, not by
   // the weights: 27648 x 5120, 1 / 2 / 4 / 8 rows: 41 / 50 / 86 / 162 us against 45 / 46 / 46 / 46 on the tensor cores; 5120 x 5120,
   // 2 rows: 12.2 against 13.2.  Small weights with short rows are done before a ring is filled: 1024 x 1024, 3 / 4 rows 8.2 against
   // 10.2, 512 x 512, 8 rows 8.2 against 10.2, 5632 x 1024, 3 rows 10.2 against 12.3; but 64 x 4096, 4 rows 17 against 11, 32000 x 512,
   // 4 rows 21 against 13, 5632 x 1024, 8 rows 18 against 11.
-  const bool tiny = (long)N * K <= ((long)M * K < 4096 ? 8l << 20 : (long)M * K < 8192 ? 4l << 20 : 0);
-  if (((M >= 3 && !tiny) || (M == 2 && (long)N * K >= 28l << 20)) && N % 8 == 0 && K % 8 == 0 &&
+  if (!vector_rows(M, N, K) && N % 8 == 0 && K % 8 == 0 &&
       (((uintptr_t)x | (uintptr_t)w | (uintptr_t)y | (uintptr_t)residual) % 16) == 0)
     return gemm_few_rows(x, w, residual, y, M, N, K, 0, st);
   const int grid = (N + 7) / 8;

@@ -94,10 +94,7 @@ __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const T* gu, T* out, si
     pg.load(gu + r * 2 * I + c);
     pu.load(gu + r * 2 * I + I + c);
 #pragma unroll
-    for (int j = 0; j < N; ++j) {
-      const float g = pg.f(j);
-      po.set(j, g / (1.f + __expf(-g)) * pu.f(j));
-    }
+    for (int j = 0; j < N; ++j) po.set(j, silu_mul(pg.f(j), pu.f(j)));
     po.store(out + r * I + c);
   }
 }

@@ -235,6 +235,47 @@ NXD_DEVICE int epilogue_tile_tma(uint32_t tmem_acc, uint32_t stage_smem, const C
   return groups;
 }
 
+// The same for tiles whose first 128 columns are gates and last 128 ups: SwiGLU of the two, 128 columns from col0 on.
+NXD_DEVICE void epilogue_tile_swiglu(uint32_t tmem_acc, uint32_t stage_smem, const CUtensorMap* omap, int row0, int col0, int q, int lane, bool issuer,
+                                     uint32_t& slab_ctr) {
+  const int row = q * 32 + lane;
+#pragma unroll 1
+  for (int s = 0; s < 2; ++s) {
+    const uint32_t buf = stage_smem + (slab_ctr & 1u) * kEpiSlabBytes;
+    if (issuer) bulk_wait_read<1>();
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    const uint32_t rbase = buf + (uint32_t)row * 128u;
+    const uint32_t sw = (uint32_t)(row & 7);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t g[32], u[32];
+      tcgen05_ld_32x32(tmem_acc + s * 64 + h * 32, g);
+      tcgen05_ld_32x32(tmem_acc + 128 + s * 64 + h * 32, u);
+      tcgen05_wait_ld();
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint4 pk;
+        __nv_bfloat162* o = (__nv_bfloat162*)&pk;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int i = 8 * c + 2 * j;
+          o[j] = __floats2bfloat162_rn(silu_mul_bf16(__uint_as_float(g[i]), __uint_as_float(u[i])),
+                                       silu_mul_bf16(__uint_as_float(g[i + 1]), __uint_as_float(u[i + 1])));
+        }
+        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};"
+                     ::"r"(rbase + (((uint32_t)(h * 4 + c) ^ sw) << 4)), "r"(pk.x), "r"(pk.y), "r"(pk.z), "r"(pk.w) : "memory");
+      }
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    if (issuer) {
+      tma_store_2d(omap, buf, col0 + s * 64, row0);
+      bulk_commit();
+    }
+    ++slab_ctr;
+  }
+}
+
 NXD_DEVICE uint32_t ld_acquire_gpu(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");

@@ -41,6 +41,10 @@ struct Group {
 // sums.  80 tiles on 74 pairs took two tiles' time for 1.08 of work.
 struct Tail { int tiles, splits, kb_per; };
 
+// MODE 0: one product.  MODE 5: SwiGLU of the product with [gate; up] weights; a tile's 256 columns are 128 gates (the first CTA's half of B) and the
+// 128 ups that belong to them (the second's), its outputs 128 columns; N counts outputs.
+__host__ __device__ constexpr bool whole(int mode) { return mode == 0 || mode == 5; }
+
 // one unit of work of a pair: an output tile and its range of k-blocks; `part`: a split of a tail tile, number `mat`
 struct Unit { int m_blk, n_blk, mat, kb0, kb1; bool part; };
 
@@ -49,7 +53,7 @@ NXD_DEVICE Unit unit_of(int unit, int num_tiles, int tiles_m, int tiles_n, int n
   Unit u;
   u.mat = 0;
   u.part = false;
-  if constexpr (MODE == 0) {
+  if constexpr (whole(MODE)) {
     const int x = unit - (num_tiles - tail.tiles);
     if (tail.tiles > 0 && x >= 0) {                        // never together with split_k
       u.part = true;
@@ -74,7 +78,7 @@ NXD_DEVICE Unit unit_of(int unit, int num_tiles, int tiles_m, int tiles_n, int n
     }
   } else {
     const int ks = unit / num_tiles;
-    tile_coords(unit - ks * num_tiles, tiles_m, tiles_n, MODE == 0 ? raster_rows(tiles_m) : kExpertRows, u.m_blk, u.n_blk);
+    tile_coords(unit - ks * num_tiles, tiles_m, tiles_n, whole(MODE) ? raster_rows(tiles_m) : kExpertRows, u.m_blk, u.n_blk);
     u.kb0 = ks * kb_per;
     u.kb1 = min(num_kb, (ks + 1) * kb_per);
   }
@@ -110,7 +114,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   const uint32_t cta = cluster_ctarank();
   const bool leader = cta == 0;
   int tiles_m = (M + TILE_M - 1) / TILE_M;
-  const int tiles_n = (N + TN - 1) / TN;
+  constexpr int kCols = MODE == 5 ? TN / 2 : TN;             // outputs of a tile
+  const int tiles_n = (N + kCols - 1) / kCols;
   if constexpr (MODE == 3) { if (grp.used_blocks) tiles_m = min(tiles_m, *grp.used_blocks * (grp.block_rows / TILE_M)); }
   const int num_tiles = (MODE == 4 ? grp.groups : 1) * tiles_m * tiles_n;
   const int num_kb = (K + BK - 1) / BK;
@@ -137,7 +142,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   cluster_sync_all();               // barriers of both CTAs are initialised before any remote arrive
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if constexpr (MODE == 0) {
+  if constexpr (whole(MODE)) {
     pdl_trigger();                                           // behind the allocation (launch_dependent)
     pdl_wait();                                              // all before this has run beside the end of the kernel before
   }
@@ -149,7 +154,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       for (int unit = pair; unit < num_units; unit += num_pairs) {
         const Unit u = unit_of<MODE>(unit, num_tiles, tiles_m, tiles_n, num_kb, kb_per, grp, tail);
         const int m0 = u.m_blk * TILE_M + (int)cta * CTA_M;
-        const int n0 = u.n_blk * TN + (int)cta * S::kHalfN;
+        const int n0 = MODE == 5 ? u.n_blk * kCols + (int)cta * N : u.n_blk * TN + (int)cta * S::kHalfN;
         int b_off = 0;
         if constexpr (MODE == 3) b_off = grp.block_expert[u.m_blk * TILE_M / grp.block_rows] * grp.b_rows;
         for (int kb = u.kb0; kb < u.kb1; ++kb) {
@@ -211,12 +216,14 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       const Unit u = unit_of<MODE>(unit, num_tiles, tiles_m, tiles_n, num_kb, kb_per, grp, tail);
       mbar_wait(bar_tfull + 8 * as, aphase);
       tcgen05_fence_after();
-      const int n0 = u.n_blk * TN, row0 = u.m_blk * TILE_M + (int)cta * CTA_M;
+      const int n0 = u.n_blk * kCols, row0 = u.m_blk * TILE_M + (int)cta * CTA_M;
       const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + as * TN;
       const bool empty = MODE == 4 && u.kb0 == u.kb1;
-      if (MODE == 0 && u.part) {
+      if (whole(MODE) && u.part) {
         epilogue_tile_tma_f32<TN>(acc, smem_base + S::kEpi, &tma_part, (int)cta * CTA_M, u.mat, 0, TN, q, lane, issuer, slab_ctr,
                               false, false);
+      } else if constexpr (MODE == 5) {
+        epilogue_tile_swiglu(acc, smem_base + S::kEpi, &tma_out, row0, n0, q, lane, issuer, slab_ctr);
       } else if constexpr (sizeof(OutT) == 4) {
         epilogue_tile_tma_f32<TN>(acc, smem_base + S::kEpi, &tma_out, row0, u.mat, n0, N, q, lane, issuer, slab_ctr,
                               accumulate || split_k > 1, empty);
@@ -248,24 +255,33 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
 }
 
 // out tile (+)= sum of its splits' partials, in order: one thread per 8 columns of a row
-template <typename OutT, int TN>
+// GATE: tiles of 128 gates and their 128 ups; SwiGLU of the two sums, 8 of 128 columns a thread
+template <typename OutT, int TN, bool GATE = false>
 __global__ void __launch_bounds__(256) gemm_tail_kernel(const float* part, OutT* out, int M, int N, int first,
                                                         int tiles_m, int tiles_n, int splits, int accumulate) {
   pdl_trigger();
   pdl_wait();
-  constexpr int kPer = TN / 8;                             // threads of a row
+  constexpr int kCols = GATE ? TN / 2 : TN, kPer = kCols / 8;      // outputs of a tile, threads of a row
   const int t = blockIdx.y, row = blockIdx.x * (256 / kPer) + threadIdx.x / kPer, col = threadIdx.x % kPer * 8;
   int m_blk, n_blk;
   tile_coords(first + t, tiles_m, tiles_n, raster_rows(tiles_m), m_blk, n_blk);
-  const int gr = m_blk * TILE_M + row, gc = n_blk * TN + col;
+  const int gr = m_blk * TILE_M + row, gc = n_blk * kCols + col;
   if (gr >= M || gc >= N) return;                          // N is a multiple of 8
-  const float* src = part + ((size_t)t * splits * TILE_M + row) * TN + col;
-  float a[8] = {};
+  float a[8] = {}, b[GATE ? 8 : 1] = {};
+  auto sum = [&](float* v, int c) {
+    const float* src = part + ((size_t)t * splits * TILE_M + row) * TN + c;
 #pragma unroll 4
-  for (int s = 0; s < splits; ++s) {
-    const float4 x = *reinterpret_cast<const float4*>(src + (size_t)s * TILE_M * TN);
-    const float4 y = *reinterpret_cast<const float4*>(src + (size_t)s * TILE_M * TN + 4);
-    a[0] += x.x; a[1] += x.y; a[2] += x.z; a[3] += x.w; a[4] += y.x; a[5] += y.y; a[6] += y.z; a[7] += y.w;
+    for (int s = 0; s < splits; ++s) {
+      const float4 x = *reinterpret_cast<const float4*>(src + (size_t)s * TILE_M * TN);
+      const float4 y = *reinterpret_cast<const float4*>(src + (size_t)s * TILE_M * TN + 4);
+      v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w; v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
+    }
+  };
+  sum(a, col);
+  if constexpr (GATE) {
+    sum(b, kCols + col);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a[j] = silu_mul_bf16(a[j], b[j]);
   }
   OutT* dst = out + (size_t)gr * N + gc;
 #pragma unroll
@@ -790,7 +806,7 @@ static void launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensor
   NXD_ALLOW_SMEM(kern, smem);
   // A dependent: barriers, TMEM and maps of the next product are set up beside the end of this one (1 x 1000 tokens of 13B: 1152 us, 1130 with
   // products, their tails, norms, SwiGLU and rotation so).  Not the grouped ones: they read the blocks' experts first and gain nothing.
-  if (MODE == 0) {
+  if (g2::whole(MODE)) {
     launch_dependent(kern, grid, g2::kThreads, smem, st, ta, tb, to, tp, (OutT*)out, M, N, K, accumulate, split_k, grp, tail);
   } else {
     kern<<<grid, g2::kThreads, smem, st>>>(ta, tb, to, tp, (OutT*)out, M, N, K, accumulate, split_k, grp, tail);
@@ -810,12 +826,12 @@ static CUtensorMap out_map(const void* out, int out_dt, bool accumulate, bool ma
 // A k-block of a 256 x 256 tile takes 0.31 us and one of 256 x 128 0.23 (their operands, 32 and 24 KB a CTA, come at about 105 GB/s an SM), a
 // launch 5; a pass over fp32 memory: 6 bytes/ps.
 struct GemmPlan { int tiles, split, width; g2::Tail tail; };      // width: columns of a tile
-static GemmPlan gemm_plan(int M, int N, int K, int out_dt, bool accumulate, bool split_k) {
+static GemmPlan gemm_plan(int M, int N, int K, int out_dt, bool accumulate, bool split_k, bool narrow = true) {
   const int pairs = std::max(1, device_sm_count() / 2), num_kb = (K + g2::BK - 1) / g2::BK;      // (no device: one, for the asking)
   const int tiles_m = (M + g2::TILE_M - 1) / g2::TILE_M;
   GemmPlan p;
   double best = 1e30;
-  for (int width = 256; width >= 128; width /= 2) {
+  for (int width = 256; width >= (narrow ? 128 : 256); width /= 2) {
     const double kb_us = width == 256 ? 0.31 : 0.2325;
     const int tiles = tiles_m * ((N + width - 1) / width);
     // The tail: the tiles of the last, partial round in s parts each, which may be several rounds themselves; worth it where it saves more than
@@ -905,6 +921,27 @@ void gemm_bf16_2cta(const void* a, const void* b, void* out, int M, int N, int K
     else sum(p.width == 128 ? g2::gemm_tail_kernel<float, 128> : g2::gemm_tail_kernel<float, 256>, (float*)out);
     NXD_CUDA_CHECK(cudaGetLastError());
   }
+}
+
+// y [M, I] = SwiGLU of x [M, K] · w [2 I, K]ᵀ (gate rows first), I a multiple of 128: the products stay in tensor memory instead of going to memory
+// and through another kernel.  The same bits as the two kernels where the tiles are the same.
+size_t gemm_swiglu_2cta_workspace(int M, int I, int K) {
+  const GemmPlan p = gemm_plan(M, 2 * I, K, kBF16, false, false, false);
+  return (size_t)p.tail.tiles * p.tail.splits * g2::TILE_M * p.width * sizeof(float);
+}
+void gemm_swiglu_2cta(const void* x, const void* w, void* y, int M, int I, int K, float* workspace, cudaStream_t st) {
+  if (I % 128 || K % 8) nxd_throw("gemm_swiglu_2cta: I must be a multiple of 128, K of 8", __FILE__, __LINE__);
+  const CUtensorMap ta = make_tmap_bf16(x, M, K, g2::BK, g2::CTA_M), tb = make_tmap_bf16(w, 2l * I, K, g2::BK, g2::HALF_N);
+  const CUtensorMap to = make_tmap_bf16(y, M, I, g2::kEpiSlabCols, g2::CTA_M);
+  GemmPlan p = gemm_plan(M, 2 * I, K, kBF16, false, false, false);
+  if (!workspace) p.tail = g2::Tail{0, 1, 1};
+  const int pairs = device_sm_count() / 2, units = p.tiles + p.tail.tiles * (p.tail.splits - 1), grid = 2 * (units < pairs ? units : pairs);
+  const CUtensorMap tp = p.tail.tiles ? make_tmap_mats(workspace, true, (uint64_t)p.tail.tiles * p.tail.splits, g2::TILE_M, p.width, 32, g2::CTA_M) : ta;
+  launch2<true, true, __nv_bfloat16, 5>(ta, tb, to, tp, y, M, I, K, 0, 1, g2::Group{}, p.tail, grid, st);
+  if (p.tail.tiles)
+    launch_dependent(g2::gemm_tail_kernel<__nv_bfloat16, 256, true>, dim3(g2::TILE_M / 16, p.tail.tiles), 256, 0, st, (const float*)workspace, (__nv_bfloat16*)y,
+                     M, I, p.tiles - p.tail.tiles, (M + g2::TILE_M - 1) / g2::TILE_M, I / 128, p.tail.splits, 0);
+  NXD_CUDA_CHECK(cudaGetLastError());
 }
 
 // Grouped GEMMs of routed experts whose row blocks are multiples of 256 rows (see grouped_gemm_bf16 / grouped_wgrad_bf16).

@@ -41,6 +41,16 @@ NXD_DEVICE void tcgen05_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
 NXD_DEVICE void prefetch_l2_tile(const CUtensorMap* map, int c0, int c1) {
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(c0), "r"(c1) : "memory");
 }
+NXD_DEVICE float2 ld_cluster_f2(uint32_t addr) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+  return v;
+}
+NXD_DEVICE float2 ld_shared_f2(uint32_t addr) {
+  float2 v;
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+  return v;
+}
 // the four products of a k-block and the commit that frees its stage, from a warp that is together (one election; descriptors advance by 32 bytes)
 NXD_DEVICE void mma4_commit(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate, uint32_t bar) {
   asm volatile(
@@ -60,6 +70,8 @@ NXD_DEVICE float4 ld_cluster_f4(uint32_t addr) {
 }
 
 // grid: split blocks (one cluster) per slab.  TN: tokens padded to 16; stage = W tile + x tile [TN, 64].
+// GATE: W holds N gate rows and then N up rows, a slab 64 of each, and y [M, N] is SwiGLU of the two products (no residual).
+template <bool GATE>
 __global__ void __launch_bounds__(kThreads)
 gemm_few_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant__ CUtensorMap tma_x, const __nv_bfloat16* residual,
                 __nv_bfloat16* y, int M, int N, int K, int TN, int stages, int tmem_cols, int split) {
@@ -71,13 +83,17 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant
   const uint32_t bar_full = bars, bar_empty = bars + 8 * kMaxStages, bar_done = bars + 16 * kMaxStages, tmem_slot = bar_done + 8;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = split > 1 ? (int)cluster_ctarank() : 0;
-  const int n0 = (int)blockIdx.x / split * kSlab;
+  constexpr int kCols = GATE ? kSlab / 2 : kSlab;          // outputs of a slab
+  const int n0 = (int)blockIdx.x / split * kCols;
   const int num_kb = (K + BK - 1) / BK, per = (num_kb + split - 1) / split;
   const int kb0 = rank * per, kb1 = min(num_kb, kb0 + per);       // the host leaves no rank without a k-block
 
   if (threadIdx.x == 0) {
     prefetch_tmap(&tma_w); prefetch_tmap(&tma_x);
-    for (int kb = kb0; kb < min(kb1, kb0 + kAhead); ++kb) prefetch_l2_tile(&tma_w, kb * BK, n0);
+    for (int kb = kb0; kb < min(kb1, kb0 + kAhead); ++kb) {
+      prefetch_l2_tile(&tma_w, kb * BK, n0);
+      if constexpr (GATE) prefetch_l2_tile(&tma_w, kb * BK, N + n0);
+    }
     for (int i = 0; i < stages; ++i) { mbar_init(bar_full + 8 * i, 1); mbar_init(bar_empty + 8 * i, 1); }
     mbar_init(bar_done, 1);
     fence_barrier_init();
@@ -98,7 +114,8 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant
         mbar_wait(bar_empty + 8 * st, ph ^ 1);
         mbar_expect_tx(bar_full + 8 * st, stage_bytes);
         const uint32_t sw = base + st * stage_bytes;
-        tma_load_2d(sw, &tma_w, bar_full + 8 * st, kb * BK, n0);
+        tma_load_2d(sw, &tma_w, bar_full + 8 * st, kb * BK, n0);                   // box {64, rows of a slab}
+        if constexpr (GATE) tma_load_2d(sw + kWBytes / 2, &tma_w, bar_full + 8 * st, kb * BK, N + n0);
         tma_load_2d(sw + kWBytes, &tma_x, bar_full + 8 * st, kb * BK, 0);
         if (++st == stages) { st = 0; ph ^= 1; }
       }
@@ -131,7 +148,23 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant
   tcgen05_fence_before();
   if (split > 1) cluster_sync_all(); else __syncthreads();
   if (warp == 1) { tcgen05_fence_after(); tcgen05_dealloc(tmem, tmem_cols); }
-  // ---- rank r sums and writes tokens r*4 + warp, + 4*split, ...: 256 contiguous bytes per warp
+  // ---- rank r sums and writes tokens r*4 + warp, + 4*split, ...: 256 contiguous bytes per warp (GATE: 128)
+  if constexpr (GATE) {
+    const int n = n0 + lane * 2;
+    for (int t = rank * 4 + warp; t < M; t += 4 * split) {
+      const uint32_t at = base + (t * kSlab + lane * 2) * 4;
+      float2 g, u;
+      for (int s = 0; s < split; ++s) {
+        const uint32_t from = split > 1 ? mapa_shared(at, s) : at;
+        const float2 a = split > 1 ? ld_cluster_f2(from) : ld_shared_f2(from), b = split > 1 ? ld_cluster_f2(from + 256) : ld_shared_f2(from + 256);
+        g = s ? make_float2(g.x + a.x, g.y + a.y) : a;
+        u = s ? make_float2(u.x + b.x, u.y + b.y) : b;
+      }
+      if (n < N) *reinterpret_cast<__nv_bfloat162*>(y + (long)t * N + n) = __floats2bfloat162_rn(silu_mul_bf16(g.x, u.x), silu_mul_bf16(g.y, u.y));
+    }
+    if (split > 1) cluster_sync_all();
+    return;
+  }
   const int n = n0 + lane * 4;
   for (int t = rank * 4 + warp; t < M; t += 4 * split) {
     const uint32_t at = base + (t * kSlab + lane * 4) * 4;
@@ -163,11 +196,12 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant
 
 }  // namespace few
 
-// split = 0: by rule
-void gemm_few_rows(const void* x, const void* w, const void* residual, void* y, int M, int N, int K, int split, cudaStream_t st) {
+// N: outputs; `gate`: SwiGLU of 2 N products
+static void few_rows(const void* x, const void* w, const void* residual, void* y, int M, int N, int K, int split, bool gate, cudaStream_t st) {
   using namespace few;
+  const int kCols = gate ? kSlab / 2 : kSlab;
   if (M < 1 || M > 256 || N % 8 || K % 8) nxd_throw("gemm_few_rows: 1 to 256 rows, N and K multiples of 8", __FILE__, __LINE__);
-  const int TN = (M + 15) / 16 * 16, slabs = (N + kSlab - 1) / kSlab, num_kb = (K + BK - 1) / BK;
+  const int TN = (M + 15) / 16 * 16, slabs = (N + kCols - 1) / kCols, num_kb = (K + BK - 1) / BK;
   if (split == 0) {
     // up to 128 rows (two blocks per SM): until every SM has a block; above (one per SM): while they still fit at once.
     // 4096 x 11008 (32 slabs), 48 rows, split 1 / 2 / 4 / 8: 52 / 30 / 21.4 / 21.2 us; 256 rows: 69 / 45 / 31 / 58 (two rounds of blocks).
@@ -184,8 +218,9 @@ void gemm_few_rows(const void* x, const void* w, const void* residual, void* y, 
   const int smem = 1024 + kBarBytes + ring_bytes;
   int cols = 32;
   while (cols < TN) cols *= 2;
-  const CUtensorMap tw = make_tmap_bf16(w, N, K, BK, kSlab), tx = make_tmap_bf16(x, M, K, BK, TN);
-  NXD_ALLOW_SMEM(gemm_few_kernel, 226 * 1024);
+  const CUtensorMap tw = make_tmap_bf16(w, gate ? 2l * N : N, K, BK, kCols), tx = make_tmap_bf16(x, M, K, BK, TN);
+  if (gate) NXD_ALLOW_SMEM(gemm_few_kernel<true>, 226 * 1024);
+  else NXD_ALLOW_SMEM(gemm_few_kernel<false>, 226 * 1024);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(slabs * split); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute attr[2]{};
@@ -194,8 +229,16 @@ void gemm_few_rows(const void* x, const void* w, const void* residual, void* y, 
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr; cfg.numAttrs = 2;
-  NXD_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_few_kernel, tw, tx, (const __nv_bfloat16*)residual, (__nv_bfloat16*)y, M, N, K, TN, stages,
-                                    cols, split));
+  NXD_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gate ? gemm_few_kernel<true> : gemm_few_kernel<false>, tw, tx, (const __nv_bfloat16*)residual,
+                                    (__nv_bfloat16*)y, M, N, K, TN, stages, cols, split));
+}
+
+// split = 0: by rule
+void gemm_few_rows(const void* x, const void* w, const void* residual, void* y, int M, int N, int K, int split, cudaStream_t st) {
+  few_rows(x, w, residual, y, M, N, K, split, false, st);
+}
+void gemm_few_rows_swiglu(const void* x, const void* w, void* y, int M, int I, int K, cudaStream_t st) {
+  few_rows(x, w, nullptr, y, M, I, K, 0, true, st);
 }
 
 }  // namespace nxd

@@ -242,7 +242,8 @@ c10::optional<Tensor> linear(const Tensor& x, const Tensor& weight, bool few) {
     return c10::nullopt;
   const int64_t K = weight.size(1), N = weight.size(0), M = K ? x.numel() / K : 0;
   const bool grads = at::GradMode::is_enabled() && (x.requires_grad() || weight.requires_grad());
-  if (M < 1 || N % 8 || K % 8 || N < 8 || ((M > 8 || grads) && M % 8)) return c10::nullopt;
+  const bool rows = M % 8 == 0 || (!grads && (M <= 8 || (few && M <= 64)));      // others as ops/gemm.py matmul takes them
+  if (M < 1 || N % 8 || K % 8 || N < 8 || !rows) return c10::nullopt;
   return Linear::apply(x, weight, few);
 }
 

@@ -25,7 +25,7 @@ from .. import ops
 from ..modules.qkv_linear import GQAQKVColumnParallelLinear
 from ..modules.rms_norm import RMSNorm
 from ..parallel_layers import parallel_state as ps
-from ..parallel_layers.layers import ColumnParallelLinear, ParallelEmbedding, RowParallelLinear
+from ..parallel_layers.layers import ColumnParallelLinear, ParallelEmbedding, RowParallelLinear, column_swiglu
 from ..parallel_layers.loss_functions import fused_linear_cross_entropy, parallel_cross_entropy
 
 
@@ -101,7 +101,7 @@ class LlamaMLP(nn.Module):
         )
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        return self.down_proj(ops.act.swiglu(self.gate_up_proj(x)))
+        return self.down_proj(column_swiglu(self.gate_up_proj, x))
 
 
 def _unwatched(proj: nn.Module) -> bool:

@@ -15,6 +15,7 @@ from .. import ops
 from ..inference.kv_cache import KVCacheManager
 from ..utils.sampling import Sampler
 from ..modules.rms_norm import RMSNorm
+from ..parallel_layers.layers import column_swiglu
 from .llama import LlamaConfig, LlamaForCausalLM
 
 
@@ -183,7 +184,7 @@ class LlamaForInference(nn.Module):
             mlp = layer.mlp
             if hasattr(mlp, "gate_up_proj") and hasattr(mlp, "down_proj") and not prefill and x.shape[0] * x.shape[1] <= 8:
                 # dense decode MLP: the residual add rides in the down-projection's GEMV(+all-reduce) epilogue
-                hmid = ops.act.swiglu(mlp.gate_up_proj(layer.post_attention_layernorm(x)))
+                hmid = column_swiglu(mlp.gate_up_proj, layer.post_attention_layernorm(x))
                 x = _row_linear_plus_residual(mlp.down_proj, hmid, x)
                 continue
             if not prefill and x.shape[0] * x.shape[1] <= 8 and hasattr(mlp, "expert_mlps") and hasattr(mlp, "router"):

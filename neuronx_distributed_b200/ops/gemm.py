@@ -25,7 +25,7 @@ def fused_wgrad_enabled() -> bool:
     return _ext.env("NXD_DISABLE_FUSED_WGRAD") != "1" and _ext.env("NXD_DISABLE_TCGEN05_GEMM") != "1"
 
 
-def _eligible(a: torch.Tensor, b: torch.Tensor, M: int, N: int, K: int) -> bool:
+def _eligible(a: torch.Tensor, b: torch.Tensor, M: int, N: int, K: int, any_rows: bool = False) -> bool:
     if _ext.env("NXD_DISABLE_TCGEN05_GEMM") == "1":
         return False
     if not (a.is_cuda and b.is_cuda and a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16):
@@ -35,7 +35,7 @@ def _eligible(a: torch.Tensor, b: torch.Tensor, M: int, N: int, K: int) -> bool:
     if not _ext.use_cuda(a, b) or not hasattr(_ext.ext(), "gemm_bf16"):
         return False
     # TMA needs 16-byte aligned rows; kernel handles ragged M/N/K tails via TMA zero fill
-    return M >= 1 and N % 8 == 0 and K % 8 == 0 and M % 8 == 0
+    return M >= 1 and N % 8 == 0 and K % 8 == 0 and (any_rows or M % 8 == 0)
 
 
 def _few_rows(M: int, N: int, K: int) -> bool:
@@ -70,11 +70,14 @@ def matmul(a: torch.Tensor, b: torch.Tensor, trans_a: bool = False, trans_b: boo
         # decode-time GEMV: a bandwidth problem (every weight byte read once), not a tensor-core one — csrc/decode.cu
         _ext.count_launch()
         return _ext.ext().gemv(a, b, None)
-    if _eligible(a, b, M, N, K) and out_dtype in (torch.bfloat16, torch.float32):
+    few = out is None and not trans_a and trans_b and out_dtype == torch.bfloat16 and _few_rows(M, N, K)
+    # Rows that are no multiple of 8: cuBLAS, but for up to 64 rows of x·Wᵀ (9 / 33 / 49 rows of 11008 -> 4096: 17.7 / 19.3 / 20.3 us, 20.7 / 20.7 / 21.2;
+    # 17 of 2816 -> 1024: 6.1 and 8.4; above, 97 of 3584 -> 8192: 17.6 and 14.9)
+    if _eligible(a, b, M, N, K, few and M <= 64) and out_dtype in (torch.bfloat16, torch.float32):
         if out is not None and out.data_ptr() % 16:          # outputs leave through TMA or 16-byte stores: by way of a buffer
             res = matmul(a, b, trans_a, trans_b, out_dtype=torch.float32)
             return out.add_(res) if accumulate else out.copy_(res)
-        if out is None and not trans_a and trans_b and out_dtype == torch.bfloat16 and _few_rows(M, N, K):
+        if few:
             _ext.count_launch()
             return _ext.ext().gemm_few_rows(a, b)
         if out is None:
@@ -100,6 +103,22 @@ def matmul(a: torch.Tensor, b: torch.Tensor, trans_a: bool = False, trans_b: boo
             out.copy_(res)
         return out
     return res.to(out_dtype)
+
+
+def linear_swiglu(x: torch.Tensor, w: torch.Tensor) -> Optional[torch.Tensor]:
+    """SwiGLU of ``x[..., K] @ w[2 I, K]^T`` (gate rows first) in one kernel, where there is one for it and it is faster than two: the
+    few-row kernel up to 128 rows (48 rows of 4096 -> 2 x 11008: 36.9 us and 39.2, 9 of 1024 -> 2 x 2816: 5.8 and 7.3; above, where a block fills an
+    SM, 129 rows 59.0 and 55.7), the CTA pairs from 136 rows on unless the few-row kernel takes them (1000 rows of 5120 -> 2 x 13824: the
+    55 MB of products stay on the chip)."""
+    K, N = x.shape[-1], w.shape[0]
+    M = x.numel() // K if K else 0
+    few = _few_rows(M, N, K)
+    if w.dim() != 2 or (few and (M > 128 or (M > 64 and M % 8))):
+        return None
+    y = _ext.ext().linear_swiglu(x, w, few)
+    if y is not None:
+        _ext.count_launch()
+    return y
 
 
 def linear_nt(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:

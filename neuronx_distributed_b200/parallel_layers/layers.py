@@ -30,6 +30,7 @@ import torch.distributed as dist
 import torch.nn.functional as F
 from torch import nn
 from torch.nn import init
+from torch.nn.modules.module import _global_forward_hooks, _global_forward_pre_hooks
 from torch.nn.parameter import Parameter
 
 from ..utils.logger import get_logger
@@ -831,6 +832,21 @@ class ColumnParallelLinear(BaseParallelLinear):
         bkey = prefix.replace("weight", "bias")
         if self.bias is not None and bkey in model_state_dict:
             model_state_dict[bkey] = F.pad(model_state_dict[bkey], (0, self.pad_size))
+
+
+def column_swiglu(proj: nn.Module, x: torch.Tensor) -> torch.Tensor:
+    """``swiglu(proj(x))`` for a projection whose rows are gates and then ups.  Without gradients, on one rank and where nobody sees what the
+    projection returns (a hook, a wrapper, a forward of its own, a recorder), the product and SwiGLU are one kernel."""
+    from .. import ops
+
+    if (not torch.is_grad_enabled() and type(proj) is ColumnParallelLinear and "forward" not in proj.__dict__ and not proj._forward_hooks
+            and not proj._forward_pre_hooks and not _global_forward_hooks and not _global_forward_pre_hooks and proj.bias is None
+            and not proj.skip_bias_add and not proj.pad and _group_size(proj.tensor_parallel_group) == 1 and not torch.is_autocast_enabled()
+            and ops.gemm._USE_2CTA and ops._ext.env("NXD_DISABLE_TCGEN05_GEMM") != "1" and ops._ext.native(x, proj.weight) is not None):
+        y = ops.gemm.linear_swiglu(x, proj.weight)
+        if y is not None:
+            return y
+    return ops.act.swiglu(proj(x))
 
 
 class RowParallelLinear(BaseParallelLinear):

@@ -1,0 +1,107 @@
+"""Product with [gate; up] weights and SwiGLU in one kernel, against mathematics in 64 bits and against the two kernels."""
+import pytest
+import torch
+
+from neuronx_distributed_b200 import ops
+from neuronx_distributed_b200.ops.gemm import _few_rows
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(M, I, K):
+    g = torch.Generator(device="cuda").manual_seed(M * 7 + I)
+    x = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    w = torch.randn(2 * I, K, generator=g, device="cuda").mul_(K ** -0.5).bfloat16()
+    return x, w
+
+
+# rows for the vector kernel are left to it; few rows (tokens padded to 16, slabs of 64 + 64 rows of W, K split over clusters), CTA pairs (whole tiles, tails)
+@pytest.mark.parametrize("M,I,K,taken", [(1, 2816, 1024, False), (2, 192, 72, False), (2, 11008, 4096, True), (3, 192, 72, False), (4, 3584, 8192, True),
+                                         (8, 11008, 4096, True), (9, 64, 8, True), (16, 192, 1000, True), (48, 11008, 4096, True), (65, 2816, 1024, True),
+                                         (128, 2816, 1024, True), (176, 11008, 4096, True), (200, 2816, 4096, True), (136, 2816, 1024, True), (256, 2816, 1024, True),
+                                         (264, 128, 72, True), (1000, 13824, 5120, True), (520, 1408, 4096, True), (301, 2816, 1024, False), (264, 192, 72, False)])
+def test_values(M, I, K, taken):
+    x, w = _case(M, I, K)
+    y = ops._ext.ext().linear_swiglu(x, w, _few_rows(M, 2 * I, K))
+    assert (y is not None) == taken
+    if not taken:
+        return
+    gate, up = (x.double() @ w.double().t()).chunk(2, -1)
+    want = torch.nn.functional.silu(gate) * up
+    # gate, up and the result are each rounded to bf16 once; silu's slope is at most 1.1
+    assert float((y.double() - want).norm() / want.norm()) < 3.2 * 2 ** -9
+    if M <= 8 or _few_rows(M, 2 * I, K):                    # the same sums: the same bits as two kernels give
+        assert torch.equal(y, ops.act.swiglu(ops._ext.ext().gemv(x, w, None) if M <= 8 else ops._ext.ext().gemm_few_rows(x, w)))
+    assert torch.equal(y, ops._ext.ext().linear_swiglu(x, w, _few_rows(M, 2 * I, K)))
+
+
+def _mlp():
+    import torch.distributed as dist
+
+    from neuronx_distributed_b200.models.llama import LlamaConfig, LlamaMLP
+    from neuronx_distributed_b200.parallel_layers import parallel_state as ps
+
+    if not dist.is_initialized():
+        dist.init_process_group("gloo", store=dist.HashStore(), rank=0, world_size=1)
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_model_parallel(tensor_model_parallel_size=1)
+    return LlamaMLP(LlamaConfig(hidden_size=256, intermediate_size=384, dtype=torch.bfloat16, device=torch.device("cuda", 0)))
+
+
+def test_projections_that_somebody_watches_are_called():
+    mlp, x = _mlp(), torch.randn(16, 1, 256, device="cuda").bfloat16()
+    with torch.no_grad():
+        plain = mlp(x)
+        seen = []
+        handle = mlp.gate_up_proj.register_forward_hook(lambda m, i, o: seen.append(o.shape))
+        watched = mlp(x)
+        handle.remove()
+        handle = torch.nn.modules.module.register_module_forward_hook(lambda m, i, o: seen.append(type(m).__name__))
+        mlp(x)
+        handle.remove()
+    assert seen[0] == (16, 1, 768) and "ColumnParallelLinear" in seen and torch.equal(plain, watched)
+    assert mlp(x.requires_grad_()).requires_grad
+
+
+def test_captured_graph_and_two_streams():
+    x, w = _case(264, 1408, 1024)
+    e = ops._ext.ext()
+    want = e.linear_swiglu(x, w, False)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = e.linear_swiglu(x, w, False)
+    y.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    got = []
+    for i in range(8):
+        with torch.cuda.stream(streams[i % 2]):
+            got.append(e.linear_swiglu(x, w, False))
+    torch.cuda.synchronize()
+    assert all(torch.equal(t, want) for t in got)
+
+
+@pytest.mark.parametrize("M", [9, 33, 63, 65, 127])
+@pytest.mark.parametrize("grads", [False, True])
+def test_rows_of_any_number(M, grads):
+    """x Wᵀ of up to 64 rows runs on the few-row kernel whatever their number; more that are no multiple of 8 on the library's."""
+    from neuronx_distributed_b200.parallel_layers.layers import tp_linear
+    from neuronx_distributed_b200.parallel_layers import parallel_state as ps
+
+    _mlp()
+    x, w = _case(M, 192, 264)
+    x.requires_grad_(grads), w.requires_grad_(grads)
+    before = ops._ext.launches()
+    with torch.set_grad_enabled(grads):
+        y = tp_linear(x, w, None, "none", "none", group=ps.get_tensor_model_parallel_group())
+    assert (ops._ext.launches() > before) == (M <= 64)
+    want = x.double() @ w.double().t()
+    assert float((y.double() - want).norm() / want.norm()) < 2 ** -8
+    if grads:
+        go = torch.randn_like(y)
+        gx, gw = torch.autograd.grad(y, (x, w), go)
+        for a, b in ((gx, go.double() @ w.double()), (gw, go.double().t() @ x.double())):
+            assert float((a.double() - b).norm() / b.norm()) < 2 ** -8
