@@ -445,6 +445,55 @@ __global__ void __launch_bounds__(256) ce_bwd_kernel(const T* logits, const int6
   }
 }
 
+// The mean of a causal language model's losses around those two passes: what the labels say of each row (s, b) of [S, B] logits, the mean of the
+// rows that count, and the gradient that the mean gives each of them.  Seventeen elementwise launches and their nodes did this: 1960 us a step of
+// the two-layer model whose time is the host's, 1830 with these.
+__global__ void __launch_bounds__(256) lm_targets_kernel(const int64_t* labels, long sb, long ss, int64_t* target, float* mask, int S, int B, int shift) {
+  pdl_trigger();
+  pdl_wait();
+  const int r = blockIdx.x * 256 + threadIdx.x;
+  if (r >= S * B) return;
+  const int s = r / B + shift, b = r % B;
+  const int64_t t = s < S ? labels[b * sb + s * ss] : -100;
+  target[r] = t == -100 ? 0 : t;                // rows that do not count are taken along, as target 0 times 0
+  mask[r] = t == -100 ? 0.f : 1.f;
+}
+
+// one block: sum(loss * mask) / max(sum(mask), 1) and its divisor; the sum in 64 bits
+__global__ void __launch_bounds__(1024) lm_mean_kernel(const float* loss, const float* mask, float* mean, float* divisor, int rows) {
+  pdl_trigger();
+  pdl_wait();
+  double sum = 0.;
+  int count = 0;
+#pragma unroll 4
+  for (int r = threadIdx.x; r < rows; r += 1024) {
+    const float m = mask[r];
+    sum += (double)(loss[r] * m);
+    count += m != 0.f;
+  }
+  __shared__ double sums[32];
+  __shared__ int counts[32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    count += __shfl_xor_sync(0xffffffffu, count, o);
+  }
+  if (threadIdx.x % 32 == 0) { sums[threadIdx.x / 32] = sum; counts[threadIdx.x / 32] = count; }
+  __syncthreads();
+  if (threadIdx.x) return;
+  for (int w = 1; w < 32; ++w) { sum += sums[w]; count += counts[w]; }
+  const float n = (float)max(count, 1);
+  *mean = (float)sum / n;
+  *divisor = n;
+}
+
+__global__ void __launch_bounds__(256) lm_row_grads_kernel(const float* gout, const float* divisor, const float* mask, float* grads, int rows) {
+  pdl_trigger();
+  pdl_wait();
+  const int r = blockIdx.x * 256 + threadIdx.x;
+  if (r < rows) grads[r] = *gout / *divisor * mask[r];
+}
+
 // ---------------------------------------------------------------- launchers
 template <typename T> static int pick_threads(int H) {
   const int nvec = H / Pack16<T>::N;
@@ -582,6 +631,19 @@ void ce_loss(const void* logits, const int64_t* target, float* lse, float* loss,
     if ((long)V * sizeof(T) >= 128 << 10 || rows <= 2 * num_sms()) go(ce_loss_kernel<T, 512>, 512);
     else go(ce_loss_kernel<T, 256>, 256);
   });
+  NXD_CUDA_CHECK(cudaGetLastError());
+}
+
+void lm_targets(const int64_t* labels, long sb, long ss, int64_t* target, float* mask, int S, int B, bool shift, cudaStream_t st) {
+  launch_dependent(lm_targets_kernel, (S * B + 255) / 256, 256, 0, st, labels, sb, ss, target, mask, S, B, (int)shift);
+  NXD_CUDA_CHECK(cudaGetLastError());
+}
+void lm_mean(const float* loss, const float* mask, float* mean, float* divisor, int rows, cudaStream_t st) {
+  launch_dependent(lm_mean_kernel, 1, 1024, 0, st, loss, mask, mean, divisor, rows);
+  NXD_CUDA_CHECK(cudaGetLastError());
+}
+void lm_row_grads(const float* gout, const float* divisor, const float* mask, float* grads, int rows, cudaStream_t st) {
+  launch_dependent(lm_row_grads_kernel, (rows + 255) / 256, 256, 0, st, gout, divisor, mask, grads, rows);
   NXD_CUDA_CHECK(cudaGetLastError());
 }
 

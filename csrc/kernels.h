@@ -30,6 +30,9 @@ void prefill_rope_kv(const void* q, const void* k, const void* v, const long (*s
                      const float* cos_t, const float* sin_t, int B, int S, int H, int K, int D, int dt, cudaStream_t st);
 void ce_stats(const void* logits, const int64_t* target, float* stats, int rows, int V, int vocab_start, int dt,
               cudaStream_t st);
+void lm_targets(const int64_t* labels, long sb, long ss, int64_t* target, float* mask, int S, int B, bool shift, cudaStream_t st);
+void lm_mean(const float* loss, const float* mask, float* mean, float* divisor, int rows, cudaStream_t st);
+void lm_row_grads(const float* gout, const float* divisor, const float* mask, float* grads, int rows, cudaStream_t st);
 void ce_loss(const void* logits, const int64_t* target, float* lse, float* loss, int rows, int V, int dt, cudaStream_t st);
 void ce_backward(const void* logits, const int64_t* target, const float* lse, const float* gout, void* grad, int rows,
                  int V, int vocab_start, float smoothing, int vocab, int dt, cudaStream_t st);

@@ -4,6 +4,8 @@
 // functorch and forward-mode AD, which the callers ask about (ops/_ext.py native()).  A node in Python costs about 20 us forward and 40 us
 // backward (its context, the interpreter's lock in the engine's thread, a dozen calls), a small training step has 23 of them: 2750 us a step
 // with them, 1900 with these.
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/extension.h>
 
@@ -157,6 +159,37 @@ struct CrossEntropy : Function<CrossEntropy> {
   }
 };
 
+// Mean of the losses of a causal language model's positions whose label is not -100: logits [S, B, V] of a whole vocabulary, labels [B, S].
+// The labels are read in forward alone, so that their buffer may take the next batch at once.
+struct CausalLoss : Function<CausalLoss> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& logits, const Tensor& labels, bool shift) {
+    const Tensor logits2 = rows(logits).contiguous();
+    c10::cuda::CUDAGuard guard(logits.device());
+    const auto st = c10::cuda::getCurrentCUDAStream().stream();
+    const int64_t S = labels.size(1), B = labels.size(0), T = S * B;
+    const Tensor target = at::empty({T}, labels.options()), mask = at::empty({T}, logits.options().dtype(at::kFloat));
+    const Tensor mean = at::empty({}, mask.options()), divisor = at::empty({}, mask.options());
+    nxd::lm_targets(labels.data_ptr<int64_t>(), labels.stride(0), labels.stride(1), target.data_ptr<int64_t>(), mask.data_ptr<float>(), (int)S, (int)B,
+                    shift, st);
+    auto o = ce_loss(logits2, target);
+    nxd::lm_mean(o[0].data_ptr<float>(), mask.data_ptr<float>(), mean.data_ptr<float>(), divisor.data_ptr<float>(), (int)T, st);
+    count(3);
+    ctx->save_for_backward({logits2, target, o[1], mask, divisor});
+    ctx->saved_data["shape"] = logits.sizes();
+    return mean;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto s = ctx->get_saved_variables();
+    c10::cuda::CUDAGuard guard(s[0].device());
+    const Tensor gout = g[0].to(at::kFloat).contiguous(), grads = at::empty_like(s[3]);
+    nxd::lm_row_grads(gout.data_ptr<float>(), s[4].data_ptr<float>(), s[3].data_ptr<float>(), grads.data_ptr<float>(), (int)grads.numel(),
+                      c10::cuda::getCurrentCUDAStream().stream());
+    count(2);
+    const Tensor d = ce_backward(s[0], s[1], s[2], grads, 0, 0.0, s[0].size(1));
+    return {d.view(ctx->saved_data["shape"].toIntVector()), Tensor(), Tensor()};
+  }
+};
+
 // --------------------------------------------------------------------------------------------------------------- linear
 // y = x Wᵀ of one rank.  The weight's gradient goes into its fp32 buffer where the optimizer gave it one (wgrad in
 // parallel_layers/layers.py, which is called for whatever the kernels do not take as it is).
@@ -265,6 +298,7 @@ void bind_native_autograd(py::module_& m) {
     return FlashAttention::apply(q, k, v, causal, scale);
   });
   n.def("cross_entropy", [](const Tensor& logits, const Tensor& target) { return CrossEntropy::apply(logits, target); });
+  n.def("causal_loss", [](const Tensor& logits, const Tensor& labels, bool shift) { return CausalLoss::apply(logits, labels, shift); });
   n.def("linear", &linear);
   n.def("pairs", &pairs);
   n.def("launches", [] { return g_launches.load(); });

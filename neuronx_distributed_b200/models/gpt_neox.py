@@ -15,7 +15,7 @@ from .. import ops
 from ..parallel_layers import parallel_state as ps
 from ..parallel_layers.layer_norm import LayerNorm
 from ..parallel_layers.layers import ColumnParallelLinear, ParallelEmbedding, RowParallelLinear
-from ..parallel_layers.loss_functions import parallel_cross_entropy
+from ..parallel_layers.loss_functions import causal_lm_loss, parallel_cross_entropy
 
 
 @dataclass
@@ -152,6 +152,9 @@ class GPTNeoXForCausalLM(nn.Module):
         logits = self.embed_out(self.gpt_neox(input_ids))           # [S, B, V/tp]
         if labels is None:
             return None, logits
+        loss = causal_lm_loss(logits, labels)
+        if loss is not None:
+            return loss, None
         tgt = labels.transpose(0, 1)
         tgt = torch.cat([tgt[1:], torch.full_like(tgt[:1], -100)], dim=0)
         mask = tgt != -100

@@ -26,7 +26,7 @@ from ..modules.qkv_linear import GQAQKVColumnParallelLinear
 from ..modules.rms_norm import RMSNorm
 from ..parallel_layers import parallel_state as ps
 from ..parallel_layers.layers import ColumnParallelLinear, ParallelEmbedding, RowParallelLinear, column_swiglu
-from ..parallel_layers.loss_functions import fused_linear_cross_entropy, parallel_cross_entropy
+from ..parallel_layers.loss_functions import causal_lm_loss, fused_linear_cross_entropy, parallel_cross_entropy
 
 
 @dataclass
@@ -303,6 +303,11 @@ class LlamaForCausalLM(nn.Module):
         h = self.model(input_ids)
         if labels is None:
             return None, self.lm_head(h)  # [S, B, V/tp]
+        if not _FUSED_LMHEAD_CE:
+            logits = self.lm_head(h)  # [S, B, V/tp]
+            loss = causal_lm_loss(logits, labels, shift_labels)
+            if loss is not None:
+                return loss, None
         # next-token objective: position s predicts labels[s+1]
         tgt = labels.transpose(0, 1)  # [S, B]
         if shift_labels:
@@ -312,7 +317,6 @@ class LlamaForCausalLM(nn.Module):
             loss = fused_linear_cross_entropy(h, self.lm_head.weight, tgt, sequence_parallel=self.config.sequence_parallel_enabled,
                                               chunk_rows=_LMHEAD_CE_CHUNK)
             return loss, None
-        logits = self.lm_head(h)  # [S, B, V/tp]
         mask = tgt != -100
         safe_tgt = torch.where(mask, tgt, torch.zeros_like(tgt))
         per_tok = parallel_cross_entropy(logits, safe_tgt)

@@ -13,7 +13,7 @@ from torch import nn
 from ..modules.moe import MoE, ExpertMLPsV2, RoutedExpertsMLPOpsConfig, RouterTopK, load_balancing_loss_func
 from ..modules.rms_norm import RMSNorm
 from ..parallel_layers.layers import ColumnParallelLinear, ParallelEmbedding
-from ..parallel_layers.loss_functions import parallel_cross_entropy
+from ..parallel_layers.loss_functions import causal_lm_loss, parallel_cross_entropy
 from .llama import LlamaAttention, LlamaConfig
 
 
@@ -108,10 +108,12 @@ class MixtralForCausalLM(nn.Module):
         logits = self.lm_head(self.norm(x))
         if labels is None:
             return None, logits
-        tgt = labels.transpose(0, 1)
-        tgt = torch.cat([tgt[1:], torch.full_like(tgt[:1], -100)], dim=0)
-        mask = tgt != -100
-        per_tok = parallel_cross_entropy(logits, torch.where(mask, tgt, torch.zeros_like(tgt)))
-        loss = (per_tok * mask).sum() / mask.sum().clamp(min=1)
+        loss = causal_lm_loss(logits, labels)
+        if loss is None:
+            tgt = labels.transpose(0, 1)
+            tgt = torch.cat([tgt[1:], torch.full_like(tgt[:1], -100)], dim=0)
+            mask = tgt != -100
+            per_tok = parallel_cross_entropy(logits, torch.where(mask, tgt, torch.zeros_like(tgt)))
+            loss = (per_tok * mask).sum() / mask.sum().clamp(min=1)
         aux = load_balancing_loss_func(all_logits, self.config.num_local_experts, self.config.num_experts_per_tok)
         return loss + self.config.router_aux_loss_coef * aux.to(loss.dtype), None

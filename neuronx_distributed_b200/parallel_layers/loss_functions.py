@@ -99,6 +99,22 @@ def parallel_cross_entropy(vocab_parallel_logits, target, label_smoothing: float
     return _ParallelCrossEntropy.apply(vocab_parallel_logits, target, label_smoothing, process_group)
 
 
+def causal_lm_loss(logits, labels, shift_labels: bool = True) -> Optional[torch.Tensor]:
+    """Mean loss of the positions whose label is not -100, from ``logits`` ``[S, B, V]`` of one rank and ``labels`` ``[B, S]``, shift and mean
+    in the kernels' own launches; with ``shift_labels`` position ``s`` predicts ``labels[:, s + 1]``.  ``None`` for what the models do in
+    several operations: shards of a vocabulary, CPU tensors, recording, tracing, functorch and forward-mode AD."""
+    from ..ops import _ext
+
+    if not isinstance(logits, torch.Tensor) or not isinstance(labels, torch.Tensor) or not logits.is_cuda:
+        return None
+    n = _ext.native(logits, labels)
+    if (n is None or logits.dtype not in (torch.bfloat16, torch.float32, torch.float16) or labels.dtype != torch.int64 or logits.dim() != 3
+            or labels.dim() != 2 or labels.t().shape != logits.shape[:2] or logits.device != labels.device or not logits.numel()
+            or labels.numel() >= 2 ** 31 - 256 or dist.get_world_size(ps.get_tensor_model_parallel_group()) > 1):
+        return None
+    return n.causal_loss(logits, labels, shift_labels)
+
+
 class DistributedLogprob(torch.autograd.Function):
     """log p(target) from vocab-parallel logits (DPO/ORPO-style objectives; reference :131-204)."""
 
