@@ -703,14 +703,16 @@ Tensor gemm_few_rows(const Tensor& x, const Tensor& w, int64_t split) {
   return y;
 }
 
-// SwiGLU of x [..., K] · w [2 I, K]ᵀ (gate rows first) in one product; None where there is no kernel for it.  few: ops/gemm.py _few_rows
-static c10::optional<Tensor> linear_swiglu(const Tensor& x, const Tensor& w, bool few) {
+// SwiGLU of x [..., K] · w [2 I, K]ᵀ (gate rows first) in one product; None where there is no kernel for it.  few: ops/gemm.py _few_rows.
+// `keep`: takes the products, [..., 2 I] (CTA pairs only)
+c10::optional<Tensor> linear_swiglu(const Tensor& x, const Tensor& w, bool few, Tensor* keep) {
   if (!x.is_cuda() || x.device() != w.device() || x.scalar_type() != at::kBFloat16 || w.scalar_type() != at::kBFloat16 || x.dim() < 2 || w.dim() != 2 ||
       !x.is_contiguous() || !w.is_contiguous() || x.size(-1) != w.size(1) || ((uintptr_t)x.data_ptr() | (uintptr_t)w.data_ptr()) % 16 || w.size(0) % 128)
     return c10::nullopt;
   const int64_t K = w.size(1), I = w.size(0) / 2, M = K ? x.numel() / K : 0;
   if (M < 1 || I < 64 || K < 8 || K % 8 || M >= (1l << 31) / 256) return c10::nullopt;
   const bool pairs = M > 8 && !few;
+  if (keep && !pairs) return c10::nullopt;
   if (pairs && (M % 8 || I % 128 || M <= 128)) return c10::nullopt;
   c10::cuda::CUDAGuard g(x.device());
   auto shape = x.sizes().vec();
@@ -724,7 +726,11 @@ static c10::optional<Tensor> linear_swiglu(const Tensor& x, const Tensor& w, boo
     const size_t bytes = nxd::gemm_swiglu_2cta_workspace((int)M, (int)I, (int)K);
     Tensor ws;
     if (bytes) ws = at::empty({(int64_t)(bytes / 4)}, x.options().dtype(at::kFloat));
-    nxd::gemm_swiglu_2cta(x.data_ptr(), w.data_ptr(), y.data_ptr(), (int)M, (int)I, (int)K, bytes ? ws.data_ptr<float>() : nullptr, stream());
+    if (keep) {
+      shape.back() = 2 * I;
+      *keep = at::empty(shape, x.options());
+    }
+    nxd::gemm_swiglu_2cta(x.data_ptr(), w.data_ptr(), y.data_ptr(), keep ? keep->data_ptr() : nullptr, (int)M, (int)I, (int)K, bytes ? ws.data_ptr<float>() : nullptr, stream());
   }
   return y;
 }
@@ -1041,7 +1047,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_gather", &moe_gather);
   m.def("moe_combine", &moe_combine);
   m.def("moe_combine_grad", &moe_combine_grad);
-  m.def("linear_swiglu", &linear_swiglu);
+  m.def("linear_swiglu", [](const Tensor& x, const Tensor& w, bool few) { return linear_swiglu(x, w, few, nullptr); });
   m.def("moe_normalize", &moe_normalize);
   m.def("moe_normalize_grad", &moe_normalize_grad);
   m.def("row_argmax", &row_argmax);

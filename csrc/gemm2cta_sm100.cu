@@ -42,8 +42,9 @@ struct Group {
 struct Tail { int tiles, splits, kb_per; };
 
 // MODE 0: one product.  MODE 5: SwiGLU of the product with [gate; up] weights; a tile's 256 columns are 128 gates (the first CTA's half of B) and the
-// 128 ups that belong to them (the second's), its outputs 128 columns; N counts outputs.
-__host__ __device__ constexpr bool whole(int mode) { return mode == 0 || mode == 5; }
+// 128 ups that belong to them (the second's), its outputs 128 columns; N counts outputs.  MODE 6: the products are kept too (a backward pass needs them).
+__host__ __device__ constexpr bool gated(int mode) { return mode == 5 || mode == 6; }
+__host__ __device__ constexpr bool whole(int mode) { return mode == 0 || gated(mode); }
 
 // one unit of work of a pair: an output tile and its range of k-blocks; `part`: a split of a tail tile, number `mat`
 struct Unit { int m_blk, n_blk, mat, kb0, kb1; bool part; };
@@ -96,8 +97,8 @@ struct Shape {
 template <bool A_KMAJOR, bool B_KMAJOR, typename OutT, int MODE, int TN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                      const __grid_constant__ CUtensorMap tma_out, const __grid_constant__ CUtensorMap tma_part, OutT* out,
-                      int M, int N, int K, int accumulate, int split_k, const Group grp, const Tail tail) {
+                      const __grid_constant__ CUtensorMap tma_out, const __grid_constant__ CUtensorMap tma_part,
+                      const __grid_constant__ CUtensorMap tma_keep, OutT* out, int M, int N, int K, int accumulate, int split_k, const Group grp, const Tail tail) {
   // accumulate: 0 store, 1 add to what is there.  split_k > 1 (fp32 outputs): that many pairs share one output tile, each sums
   // a K range and adds its partial — for weight gradients whose output has too few tiles to fill the 74 pairs while
   // K = tokens is long.  fp32 outputs always leave through TMA (stored or added in memory), bf16 ones unless they accumulate.
@@ -114,7 +115,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   const uint32_t cta = cluster_ctarank();
   const bool leader = cta == 0;
   int tiles_m = (M + TILE_M - 1) / TILE_M;
-  constexpr int kCols = MODE == 5 ? TN / 2 : TN;             // outputs of a tile
+  constexpr int kCols = gated(MODE) ? TN / 2 : TN;             // outputs of a tile
   const int tiles_n = (N + kCols - 1) / kCols;
   if constexpr (MODE == 3) { if (grp.used_blocks) tiles_m = min(tiles_m, *grp.used_blocks * (grp.block_rows / TILE_M)); }
   const int num_tiles = (MODE == 4 ? grp.groups : 1) * tiles_m * tiles_n;
@@ -154,7 +155,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       for (int unit = pair; unit < num_units; unit += num_pairs) {
         const Unit u = unit_of<MODE>(unit, num_tiles, tiles_m, tiles_n, num_kb, kb_per, grp, tail);
         const int m0 = u.m_blk * TILE_M + (int)cta * CTA_M;
-        const int n0 = MODE == 5 ? u.n_blk * kCols + (int)cta * N : u.n_blk * TN + (int)cta * S::kHalfN;
+        const int n0 = gated(MODE) ? u.n_blk * kCols + (int)cta * N : u.n_blk * TN + (int)cta * S::kHalfN;
         int b_off = 0;
         if constexpr (MODE == 3) b_off = grp.block_expert[u.m_blk * TILE_M / grp.block_rows] * grp.b_rows;
         for (int kb = u.kb0; kb < u.kb1; ++kb) {
@@ -222,7 +223,11 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       if (whole(MODE) && u.part) {
         epilogue_tile_tma_f32<TN>(acc, smem_base + S::kEpi, &tma_part, (int)cta * CTA_M, u.mat, 0, TN, q, lane, issuer, slab_ctr,
                               false, false);
-      } else if constexpr (MODE == 5) {
+      } else if constexpr (gated(MODE)) {
+        if constexpr (MODE == 6) {
+          epilogue_tile_tma<false, TN / 2>(acc, smem_base + S::kEpi, &tma_keep, row0, n0, 2 * N, q, lane, issuer, slab_ctr);
+          epilogue_tile_tma<false, TN / 2>(acc + TN / 2, smem_base + S::kEpi, &tma_keep, row0, N + n0, 2 * N, q, lane, issuer, slab_ctr);
+        }
         epilogue_tile_swiglu(acc, smem_base + S::kEpi, &tma_out, row0, n0, q, lane, issuer, slab_ctr);
       } else if constexpr (sizeof(OutT) == 4) {
         epilogue_tile_tma_f32<TN>(acc, smem_base + S::kEpi, &tma_out, row0, u.mat, n0, N, q, lane, issuer, slab_ctr,
@@ -255,10 +260,10 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
 }
 
 // out tile (+)= sum of its splits' partials, in order: one thread per 8 columns of a row
-// GATE: tiles of 128 gates and their 128 ups; SwiGLU of the two sums, 8 of 128 columns a thread
+// GATE: tiles of 128 gates and their 128 ups; SwiGLU of the two sums, 8 of 128 columns a thread; `keep`, if any: the sums, [M, 2 N]
 template <typename OutT, int TN, bool GATE = false>
 __global__ void __launch_bounds__(256) gemm_tail_kernel(const float* part, OutT* out, int M, int N, int first,
-                                                        int tiles_m, int tiles_n, int splits, int accumulate) {
+                                                        int tiles_m, int tiles_n, int splits, int accumulate, OutT* keep) {
   pdl_trigger();
   pdl_wait();
   constexpr int kCols = GATE ? TN / 2 : TN, kPer = kCols / 8;      // outputs of a tile, threads of a row
@@ -280,6 +285,11 @@ __global__ void __launch_bounds__(256) gemm_tail_kernel(const float* part, OutT*
   sum(a, col);
   if constexpr (GATE) {
     sum(b, kCols + col);
+    if (keep) {
+      OutT* row_of = keep + (size_t)gr * 2 * N + gc;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) { row_of[j] = from_f32<OutT>(a[j]); row_of[N + j] = from_f32<OutT>(b[j]); }
+    }
 #pragma unroll
     for (int j = 0; j < 8; ++j) a[j] = silu_mul_bf16(a[j], b[j]);
   }
@@ -800,16 +810,16 @@ CUtensorMap make_tmap_mats(const void* ptr, bool f32, uint64_t mats, uint64_t ro
 
 template <bool AK, bool BK_, typename OutT, int MODE = 0, int TN = g2::TILE_N>
 static void launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& to, const CUtensorMap& tp, void* out, int M, int N, int K,
-                    int accumulate, int split_k, const g2::Group& grp, const g2::Tail& tail, int grid, cudaStream_t st) {
+                    int accumulate, int split_k, const g2::Group& grp, const g2::Tail& tail, int grid, cudaStream_t st, const CUtensorMap* keep = nullptr) {
   auto kern = g2::gemm_bf16_2cta_kernel<AK, BK_, OutT, MODE, TN>;
   constexpr int smem = g2::Shape<TN>::kShared;
   NXD_ALLOW_SMEM(kern, smem);
   // A dependent: barriers, TMEM and maps of the next product are set up beside the end of this one (1 x 1000 tokens of 13B: 1152 us, 1130 with
   // products, their tails, norms, SwiGLU and rotation so).  Not the grouped ones: they read the blocks' experts first and gain nothing.
   if (g2::whole(MODE)) {
-    launch_dependent(kern, grid, g2::kThreads, smem, st, ta, tb, to, tp, (OutT*)out, M, N, K, accumulate, split_k, grp, tail);
+    launch_dependent(kern, grid, g2::kThreads, smem, st, ta, tb, to, tp, keep ? *keep : tp, (OutT*)out, M, N, K, accumulate, split_k, grp, tail);
   } else {
-    kern<<<grid, g2::kThreads, smem, st>>>(ta, tb, to, tp, (OutT*)out, M, N, K, accumulate, split_k, grp, tail);
+    kern<<<grid, g2::kThreads, smem, st>>>(ta, tb, to, tp, tp, (OutT*)out, M, N, K, accumulate, split_k, grp, tail);
     NXD_CUDA_CHECK(cudaGetLastError());
   }
 }
@@ -915,7 +925,7 @@ void gemm_bf16_2cta(const void* a, const void* b, void* out, int M, int N, int K
     const int tiles_m = (M + g2::TILE_M - 1) / g2::TILE_M, tiles_n = (N + p.width - 1) / p.width;
     const dim3 tg(g2::TILE_M * p.width / 2048, p.tail.tiles);
     auto sum = [&](auto kernel, auto* o) {
-      launch_dependent(kernel, tg, 256, 0, st, (const float*)workspace, o, M, N, p.tiles - p.tail.tiles, tiles_m, tiles_n, p.tail.splits, (int)accumulate);
+      launch_dependent(kernel, tg, 256, 0, st, (const float*)workspace, o, M, N, p.tiles - p.tail.tiles, tiles_m, tiles_n, p.tail.splits, (int)accumulate, decltype(o)(nullptr));
     };
     if (out_dt == kBF16) sum(p.width == 128 ? g2::gemm_tail_kernel<__nv_bfloat16, 128> : g2::gemm_tail_kernel<__nv_bfloat16, 256>, (__nv_bfloat16*)out);
     else sum(p.width == 128 ? g2::gemm_tail_kernel<float, 128> : g2::gemm_tail_kernel<float, 256>, (float*)out);
@@ -924,12 +934,13 @@ void gemm_bf16_2cta(const void* a, const void* b, void* out, int M, int N, int K
 }
 
 // y [M, I] = SwiGLU of x [M, K] · w [2 I, K]ᵀ (gate rows first), I a multiple of 128: the products stay in tensor memory instead of going to memory
-// and through another kernel.  The same bits as the two kernels where the tiles are the same.
+// and through another kernel; with `keep` they go to [M, 2 I] as well, and what is saved is reading them again.  The same bits as the two kernels
+// where the tiles are the same.
 size_t gemm_swiglu_2cta_workspace(int M, int I, int K) {
   const GemmPlan p = gemm_plan(M, 2 * I, K, kBF16, false, false, false);
   return (size_t)p.tail.tiles * p.tail.splits * g2::TILE_M * p.width * sizeof(float);
 }
-void gemm_swiglu_2cta(const void* x, const void* w, void* y, int M, int I, int K, float* workspace, cudaStream_t st) {
+void gemm_swiglu_2cta(const void* x, const void* w, void* y, void* keep, int M, int I, int K, float* workspace, cudaStream_t st) {
   if (I % 128 || K % 8) nxd_throw("gemm_swiglu_2cta: I must be a multiple of 128, K of 8", __FILE__, __LINE__);
   const CUtensorMap ta = make_tmap_bf16(x, M, K, g2::BK, g2::CTA_M), tb = make_tmap_bf16(w, 2l * I, K, g2::BK, g2::HALF_N);
   const CUtensorMap to = make_tmap_bf16(y, M, I, g2::kEpiSlabCols, g2::CTA_M);
@@ -937,10 +948,15 @@ void gemm_swiglu_2cta(const void* x, const void* w, void* y, int M, int I, int K
   if (!workspace) p.tail = g2::Tail{0, 1, 1};
   const int pairs = device_sm_count() / 2, units = p.tiles + p.tail.tiles * (p.tail.splits - 1), grid = 2 * (units < pairs ? units : pairs);
   const CUtensorMap tp = p.tail.tiles ? make_tmap_mats(workspace, true, (uint64_t)p.tail.tiles * p.tail.splits, g2::TILE_M, p.width, 32, g2::CTA_M) : ta;
-  launch2<true, true, __nv_bfloat16, 5>(ta, tb, to, tp, y, M, I, K, 0, 1, g2::Group{}, p.tail, grid, st);
+  if (keep) {
+    const CUtensorMap tk = make_tmap_bf16(keep, M, 2l * I, g2::kEpiSlabCols, g2::CTA_M);
+    launch2<true, true, __nv_bfloat16, 6>(ta, tb, to, tp, y, M, I, K, 0, 1, g2::Group{}, p.tail, grid, st, &tk);
+  } else {
+    launch2<true, true, __nv_bfloat16, 5>(ta, tb, to, tp, y, M, I, K, 0, 1, g2::Group{}, p.tail, grid, st);
+  }
   if (p.tail.tiles)
     launch_dependent(g2::gemm_tail_kernel<__nv_bfloat16, 256, true>, dim3(g2::TILE_M / 16, p.tail.tiles), 256, 0, st, (const float*)workspace, (__nv_bfloat16*)y,
-                     M, I, p.tiles - p.tail.tiles, (M + g2::TILE_M - 1) / g2::TILE_M, I / 128, p.tail.splits, 0);
+                     M, I, p.tiles - p.tail.tiles, (M + g2::TILE_M - 1) / g2::TILE_M, I / 128, p.tail.splits, 0, (__nv_bfloat16*)keep);
   NXD_CUDA_CHECK(cudaGetLastError());
 }
 

@@ -251,20 +251,40 @@ struct Linear : Function<Linear> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     const auto s = ctx->get_saved_variables();
-    const Tensor &x = s[0], &weight = s[1];
-    Tensor go = rows(g[0].contiguous()), x2 = rows(x).contiguous();
+    auto o = gradients(rows(g[0].contiguous()), s[0], s[1], ctx->saved_data["x"].toBool());
+    return {o.first, o.second, Tensor()};
+  }
+  static std::pair<Tensor, Tensor> gradients(Tensor go, const Tensor& x, const Tensor& weight, bool of_x) {
+    Tensor x2 = rows(x).contiguous();
     if (!aligned(go)) go = go.clone();
     if (!aligned(x2)) x2 = x2.clone();
     Tensor gx, gw;
-    if (ctx->saved_data["x"].toBool()) {
+    if (of_x) {
       gx = at::empty({go.size(0), weight.size(1)}, go.options());
       product(go, weight, gx, false, false, false);
-      auto shape = g[0].sizes().vec();
-      shape.back() = weight.size(1);
-      gx = gx.view(shape);
+      gx = gx.view(x.sizes());
     }
     if (weight.requires_grad()) gw = weight_gradient(go, x2, weight);
-    return {gx, gw, Tensor()};
+    return {gx, gw};
+  }
+};
+
+// SwiGLU of x · [gate; up]ᵀ, the two nodes in one: the products are kept for the backward pass as they leave the tensor cores, and not read again for it
+struct LinearSwiGLU : Function<LinearSwiGLU> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight) {
+    Tensor gate_up;
+    const auto y = linear_swiglu(x, weight, false, &gate_up);
+    TORCH_CHECK(y.has_value(), "linear_swiglu: no kernel for these operands");
+    count();
+    ctx->save_for_backward({x, weight, gate_up});
+    ctx->saved_data["x"] = x.requires_grad();
+    return *y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto s = ctx->get_saved_variables();
+    count();
+    auto o = Linear::gradients(swiglu_bwd(rows(g[0]).contiguous(), rows(s[2]).contiguous()), s[0], s[1], ctx->saved_data["x"].toBool());
+    return {o.first, o.second};
   }
 };
 
@@ -300,6 +320,7 @@ void bind_native_autograd(py::module_& m) {
   n.def("cross_entropy", [](const Tensor& logits, const Tensor& target) { return CrossEntropy::apply(logits, target); });
   n.def("causal_loss", [](const Tensor& logits, const Tensor& labels, bool shift) { return CausalLoss::apply(logits, labels, shift); });
   n.def("linear", &linear);
+  n.def("linear_swiglu", [](const Tensor& x, const Tensor& w) { return LinearSwiGLU::apply(x, w); });
   n.def("pairs", &pairs);
   n.def("launches", [] { return g_launches.load(); });
   n.def("set_weight_gradient", [](py::object wgrad, py::object enabled) {      // kept for the life of the process

@@ -105,16 +105,22 @@ def matmul(a: torch.Tensor, b: torch.Tensor, trans_a: bool = False, trans_b: boo
     return res.to(out_dtype)
 
 
-def linear_swiglu(x: torch.Tensor, w: torch.Tensor) -> Optional[torch.Tensor]:
+def linear_swiglu(x: torch.Tensor, w: torch.Tensor, nodes=None) -> Optional[torch.Tensor]:
     """SwiGLU of ``x[..., K] @ w[2 I, K]^T`` (gate rows first) in one kernel, where there is one for it and it is faster than two: the
     few-row kernel up to 128 rows (48 rows of 4096 -> 2 x 11008: 36.9 us and 39.2, 9 of 1024 -> 2 x 2816: 5.8 and 7.3; above, where a block fills an
     SM, 129 rows 59.0 and 55.7), the CTA pairs from 136 rows on unless the few-row kernel takes them (1000 rows of 5120 -> 2 x 13824: the
-    55 MB of products stay on the chip)."""
+    55 MB of products stay on the chip).  With gradients (``nodes``: those of ``_ext.native``) the CTA pairs alone."""
     K, N = x.shape[-1], w.shape[0]
     M = x.numel() // K if K else 0
     few = _few_rows(M, N, K)
     if w.dim() != 2 or (few and (M > 128 or (M > 64 and M % 8))):
         return None
+    if nodes is not None:
+        if (few or x.dim() < 2 or M % 8 or M <= 128 or N % 256 or K % 8 or not x.is_cuda or x.device != w.device or x.shape[-1] != w.shape[1]
+                or not x.dtype == w.dtype == torch.bfloat16 or not x.is_contiguous() or not w.is_contiguous() or x.data_ptr() % 16 or w.data_ptr() % 16
+                or M >= 2 ** 23):
+            return None
+        return nodes.linear_swiglu(x, w)
     y = _ext.ext().linear_swiglu(x, w, few)
     if y is not None:
         _ext.count_launch()

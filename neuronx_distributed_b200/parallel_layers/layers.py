@@ -30,7 +30,7 @@ import torch.distributed as dist
 import torch.nn.functional as F
 from torch import nn
 from torch.nn import init
-from torch.nn.modules.module import _global_forward_hooks, _global_forward_pre_hooks
+from torch.nn.modules.module import _global_backward_hooks, _global_backward_pre_hooks, _global_forward_hooks, _global_forward_pre_hooks
 from torch.nn.parameter import Parameter
 
 from ..utils.logger import get_logger
@@ -592,8 +592,8 @@ class _TPLinear(torch.autograd.Function):
 _NATIVE_WGRAD = None
 
 
-def _native_linear(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Tensor]:
-    """``x @ Wᵀ`` of one rank as a node without Python in it, or None where the kernels do not take its products as they are."""
+def _native_products(x: torch.Tensor, weight: torch.Tensor):
+    """The nodes without Python in them (``ops._ext.native``) where the package's own products may run, else None."""
     from .. import ops
 
     global _NATIVE_WGRAD
@@ -603,6 +603,16 @@ def _native_linear(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Tens
     if _NATIVE_WGRAD is not n:
         n.set_weight_gradient(lambda *a: wgrad(*a), lambda: ops.gemm.fused_wgrad_enabled())
         _NATIVE_WGRAD = n
+    return n
+
+
+def _native_linear(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Tensor]:
+    """``x @ Wᵀ`` of one rank as a node without Python in it, or None where the kernels do not take its products as they are."""
+    from .. import ops
+
+    n = _native_products(x, weight)
+    if n is None:
+        return None
     N, K = weight.shape if weight.dim() == 2 else (0, 0)
     return n.linear(x, weight, K > 0 and ops.gemm._few_rows(x.numel() // K, N, K))
 
@@ -835,15 +845,20 @@ class ColumnParallelLinear(BaseParallelLinear):
 
 
 def column_swiglu(proj: nn.Module, x: torch.Tensor) -> torch.Tensor:
-    """``swiglu(proj(x))`` for a projection whose rows are gates and then ups.  Without gradients, on one rank and where nobody sees what the
-    projection returns (a hook, a wrapper, a forward of its own, a recorder), the product and SwiGLU are one kernel."""
+    """``swiglu(proj(x))`` for a projection whose rows are gates and then ups.  On one rank and where nobody sees what the projection returns
+    or is given back (a hook, a wrapper, a forward of its own, a recorder), the product and SwiGLU are one kernel."""
     from .. import ops
 
-    if (not torch.is_grad_enabled() and type(proj) is ColumnParallelLinear and "forward" not in proj.__dict__ and not proj._forward_hooks
-            and not proj._forward_pre_hooks and not _global_forward_hooks and not _global_forward_pre_hooks and proj.bias is None
-            and not proj.skip_bias_add and not proj.pad and _group_size(proj.tensor_parallel_group) == 1 and not torch.is_autocast_enabled()
-            and ops.gemm._USE_2CTA and ops._ext.env("NXD_DISABLE_TCGEN05_GEMM") != "1" and ops._ext.native(x, proj.weight) is not None):
-        y = ops.gemm.linear_swiglu(x, proj.weight)
+    if (type(proj) is ColumnParallelLinear and "forward" not in proj.__dict__ and not proj._forward_hooks and not proj._forward_pre_hooks
+            and not proj._backward_hooks and not proj._backward_pre_hooks and not _global_forward_hooks and not _global_forward_pre_hooks
+            and not _global_backward_hooks and not _global_backward_pre_hooks and proj.bias is None
+            and not proj.skip_bias_add and not proj.pad and _group_size(proj.tensor_parallel_group) == 1 and not torch.is_autocast_enabled()):
+        n = _native_products(x, proj.weight)
+        if n is not None:
+            grads = torch.is_grad_enabled() and (x.requires_grad or proj.weight.requires_grad)
+            y = ops.gemm.linear_swiglu(x, proj.weight, n if grads else None)
+        else:
+            y = None
         if y is not None:
             return y
     return ops.act.swiglu(proj(x))

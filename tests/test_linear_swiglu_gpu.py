@@ -63,6 +63,47 @@ def test_projections_that_somebody_watches_are_called():
     assert mlp(x.requires_grad_()).requires_grad
 
 
+# whole tiles, tails, a remainder of rows, several rows' dimensions; with and without a gradient of x, into the optimizer's buffer and as .grad
+@pytest.mark.parametrize("shape,I", [((136, 1024), 2816), ((132, 2, 4096), 1408), ((1000, 72), 128), ((2, 260, 1024), 1408)])
+@pytest.mark.parametrize("of_x,buffer", [(True, False), (False, False), (True, True)])
+def test_gradients(shape, I, of_x, buffer):
+    from neuronx_distributed_b200.parallel_layers.layers import ColumnParallelLinear, column_swiglu
+
+    _mlp()
+    K = shape[-1]
+    x, w = _case(x_rows := torch.Size(shape[:-1]).numel(), I, K)
+    x, go = x.view(shape), torch.randn(*shape[:-1], I, device="cuda").bfloat16()
+    proj = ColumnParallelLinear(K, 2 * I, bias=False, gather_output=False, dtype=torch.bfloat16, device=torch.device("cuda", 0))
+    proj.weight.data.copy_(w)
+
+    def run(fused):
+        proj.weight.grad = None
+        if buffer:
+            proj.weight.main_grad = torch.ones(2 * I, K, device="cuda")
+            proj.weight.main_grad_fresh = False
+        xi = x.clone().requires_grad_(of_x)
+        before = ops._ext.launches()
+        y = column_swiglu(proj, xi) if fused else ops.act.swiglu(proj(xi))
+        launched = ops._ext.launches() - before
+        y.backward(go)
+        return y.detach(), xi.grad, proj.weight.main_grad if buffer else proj.weight.grad, launched
+
+    one, two = run(True), run(False)
+    assert (one[3], two[3]) == (1, 2) and x_rows > 128
+    for a, b in zip(one[:3], two[:3]):
+        assert (a is None) == (b is None)
+        # the same products but for the order of a tail's sums, each rounded to bf16 on the way: 2^-9 of the gates and ups, silu's slopes at most 1.1
+        assert a is None or float((a.double() - b.double()).norm() / b.double().norm()) < 2 ** -7
+    gate, up = (x.double() @ w.double().t()).chunk(2, -1)
+    want = torch.nn.functional.silu(gate) * up
+    assert float((one[0].double() - want).norm() / want.norm()) < 3.2 * 2 ** -9
+    handles = [proj.register_full_backward_hook(lambda m, gi, go: None)]
+    before = ops._ext.launches()
+    column_swiglu(proj, x.clone().requires_grad_(of_x))
+    assert ops._ext.launches() - before == 2                 # a watched projection is called
+    handles[0].remove()
+
+
 def test_captured_graph_and_two_streams():
     x, w = _case(264, 1408, 1024)
     e = ops._ext.ext()
