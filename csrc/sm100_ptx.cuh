@@ -182,34 +182,14 @@ NXD_DEVICE void tcgen05_mma_f16_2cta(uint32_t tmem_d, uint64_t desc_a, uint64_t 
 
 
 // ---- elected issue: the whole (converged) MMA warp executes these; one elected lane runs the tcgen05 instruction.
-// Issuing from `if (lane == 0)` costs ~100 cycles per MMA (timed).  For the attention kernels (32-64-cycle UMMAs) that made the issuing thread the
-// bottleneck and the elected form fixed it.  For the big-tile GEMMs (128-cycle UMMAs) the elected form measured SLOWER
-// (8192^3: 1371 vs 1637 TFLOP/s — 32 lanes spinning on the mbarriers), so
-// the GEMM kernels keep single-lane issue; these helpers are kept for small-tile kernels.
-NXD_DEVICE void tcgen05_mma_f8_e(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "elect.sync _|q, 0xffffffff;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
+// Issuing from `if (lane == 0)` costs 100 to 130 cycles per MMA (timed), which is longer than a product of 128 columns lasts.  One election for a group
+// of products is the cheapest form: the macros and functions that issue a k-block's or a tile's products at once stand beside their kernels.
 NXD_DEVICE void tcgen05_commit_e(uint32_t bar) {
   asm volatile(
       "{\n\t.reg .pred q;\n\t"
       "elect.sync _|q, 0xffffffff;\n\t"
       "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
       ::"r"(bar) : "memory");
-}
-NXD_DEVICE void tcgen05_mma_f16_2cta_e(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "elect.sync _|q, 0xffffffff;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
 }
 NXD_DEVICE void tcgen05_commit_2cta_e(uint32_t bar, uint16_t cta_mask) {
   asm volatile(
