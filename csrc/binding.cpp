@@ -607,6 +607,22 @@ static Tensor grouped_gemm(const Tensor& a, const Tensor& w, const Tensor& block
                          (int)block_rows, nxd::kBF16, stream());
   return out;
 }
+// SwiGLU of the routed rows' products with [E, K, 2 I] weights; {y, products} or, without `keep`, {y}
+static std::vector<Tensor> grouped_swiglu(const Tensor& a, const Tensor& w, const Tensor& block_expert, int64_t block_rows, const Tensor& seg, bool keep) {
+  TORCH_CHECK(a.is_cuda() && a.scalar_type() == at::kBFloat16 && a.dim() == 2 && a.is_contiguous());
+  TORCH_CHECK(w.scalar_type() == at::kBFloat16 && w.dim() == 3 && w.is_contiguous() && w.device() == a.device());
+  TORCH_CHECK(block_expert.scalar_type() == at::kInt && block_expert.is_cuda());
+  const int M = a.size(0), K = a.size(1), E = w.size(0), I = w.size(2) / 2;
+  TORCH_CHECK(w.size(1) == K && w.size(2) % 256 == 0 && K % 64 == 0 && block_rows % 256 == 0 && block_expert.numel() * block_rows == M && M > 0);
+  TORCH_CHECK(seg.is_cuda() && seg.is_contiguous() && seg.scalar_type() == at::kInt && seg.numel() == E + 1);
+  c10::cuda::CUDAGuard guard(a.device());
+  std::vector<Tensor> out{at::empty({M, I}, a.options())};
+  if (keep) out.push_back(at::empty({M, 2 * I}, a.options()));
+  nxd::grouped_swiglu_2cta(a.data_ptr(), w.data_ptr(), out[0].data_ptr(), keep ? out[1].data_ptr() : nullptr, M, I, K, E, block_expert.data_ptr<int>(),
+                           seg.data_ptr<int>() + E, (int)block_rows, stream());
+  return out;
+}
+
 // dW[e] = x[rows of e]ᵀ · dy[rows of e]  → out [E, Mo, No] (bf16 or fp32), optionally accumulated.  slot_token (int32 [rows], optional): -1
 // for the rows behind an expert's last one, which are zero in x and dy
 static void grouped_wgrad(const Tensor& x, const Tensor& dy, Tensor out, const Tensor& seg_first_block, int64_t block_rows,
@@ -1047,6 +1063,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_gather", &moe_gather);
   m.def("moe_combine", &moe_combine);
   m.def("moe_combine_grad", &moe_combine_grad);
+  m.def("grouped_swiglu", &grouped_swiglu);
   m.def("linear_swiglu", [](const Tensor& x, const Tensor& w, bool few) { return linear_swiglu(x, w, few, nullptr); });
   m.def("moe_normalize", &moe_normalize);
   m.def("moe_normalize_grad", &moe_normalize_grad);

@@ -42,9 +42,11 @@ struct Group {
 struct Tail { int tiles, splits, kb_per; };
 
 // MODE 0: one product.  MODE 5: SwiGLU of the product with [gate; up] weights; a tile's 256 columns are 128 gates (the first CTA's half of B) and the
-// 128 ups that belong to them (the second's), its outputs 128 columns; N counts outputs.  MODE 6: the products are kept too (a backward pass needs them).
-__host__ __device__ constexpr bool gated(int mode) { return mode == 5 || mode == 6; }
-__host__ __device__ constexpr bool whole(int mode) { return mode == 0 || gated(mode); }
+// 128 ups that belong to them (the second's), its outputs 128 columns; N counts outputs.  MODE 6: the products are kept too (a backward
+// pass needs them).  MODE 7: routed experts with [gate up] weights, the products kept if `accumulate`.
+__host__ __device__ constexpr bool gated(int mode) { return mode >= 5 && mode <= 7; }
+__host__ __device__ constexpr bool experts(int mode) { return mode == 3 || mode == 7; }
+__host__ __device__ constexpr bool whole(int mode) { return mode == 0 || mode == 5 || mode == 6; }
 
 // one unit of work of a pair: an output tile and its range of k-blocks; `part`: a split of a tail tile, number `mat`
 struct Unit { int m_blk, n_blk, mat, kb0, kb1; bool part; };
@@ -117,7 +119,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   int tiles_m = (M + TILE_M - 1) / TILE_M;
   constexpr int kCols = gated(MODE) ? TN / 2 : TN;             // outputs of a tile
   const int tiles_n = (N + kCols - 1) / kCols;
-  if constexpr (MODE == 3) { if (grp.used_blocks) tiles_m = min(tiles_m, *grp.used_blocks * (grp.block_rows / TILE_M)); }
+  if constexpr (experts(MODE)) { if (grp.used_blocks) tiles_m = min(tiles_m, *grp.used_blocks * (grp.block_rows / TILE_M)); }
   const int num_tiles = (MODE == 4 ? grp.groups : 1) * tiles_m * tiles_n;
   const int num_kb = (K + BK - 1) / BK;
   const int kb_per = (num_kb + split_k - 1) / split_k;       // k-blocks per split (host guarantees no empty split)
@@ -157,7 +159,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
         const int m0 = u.m_blk * TILE_M + (int)cta * CTA_M;
         const int n0 = gated(MODE) ? u.n_blk * kCols + (int)cta * N : u.n_blk * TN + (int)cta * S::kHalfN;
         int b_off = 0;
-        if constexpr (MODE == 3) b_off = grp.block_expert[u.m_blk * TILE_M / grp.block_rows] * grp.b_rows;
+        if constexpr (experts(MODE)) b_off = grp.block_expert[u.m_blk * TILE_M / grp.block_rows] * grp.b_rows;
         for (int kb = u.kb0; kb < u.kb1; ++kb) {
           mbar_wait(bar_empty + 8 * stage, phase ^ 1);
           const uint32_t full = bar_full + 8 * stage;          // same offset in the leader's smem
@@ -224,7 +226,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
         epilogue_tile_tma_f32<TN>(acc, smem_base + S::kEpi, &tma_part, (int)cta * CTA_M, u.mat, 0, TN, q, lane, issuer, slab_ctr,
                               false, false);
       } else if constexpr (gated(MODE)) {
-        if constexpr (MODE == 6) {
+        if (MODE == 6 || (MODE == 7 && accumulate)) {
           epilogue_tile_tma<false, TN / 2>(acc, smem_base + S::kEpi, &tma_keep, row0, n0, 2 * N, q, lane, issuer, slab_ctr);
           epilogue_tile_tma<false, TN / 2>(acc + TN / 2, smem_base + S::kEpi, &tma_keep, row0, N + n0, 2 * N, q, lane, issuer, slab_ctr);
         }
@@ -819,7 +821,7 @@ static void launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensor
   if (g2::whole(MODE)) {
     launch_dependent(kern, grid, g2::kThreads, smem, st, ta, tb, to, tp, keep ? *keep : tp, (OutT*)out, M, N, K, accumulate, split_k, grp, tail);
   } else {
-    kern<<<grid, g2::kThreads, smem, st>>>(ta, tb, to, tp, tp, (OutT*)out, M, N, K, accumulate, split_k, grp, tail);
+    kern<<<grid, g2::kThreads, smem, st>>>(ta, tb, to, tp, keep ? *keep : tp, (OutT*)out, M, N, K, accumulate, split_k, grp, tail);
     NXD_CUDA_CHECK(cudaGetLastError());
   }
 }
@@ -976,6 +978,18 @@ void grouped_gemm_bf16_2cta(const void* a, const void* b, void* out, int M, int 
     if (out_dt == kBF16) launch2<true, false, __nv_bfloat16, 3>(ta, tb, to, to, out, M, N, K, 0, 1, grp, g2::Tail{0, 1, 1}, grid, st);
     else launch2<true, false, float, 3>(ta, tb, to, to, out, M, N, K, 0, 1, grp, g2::Tail{0, 1, 1}, grid, st);
   }
+}
+
+// y [M, I] = SwiGLU of the routed rows' products with their expert's [K, gate up] weights b [E, K, 2 I], I a multiple of 128; keep, if any: the products
+void grouped_swiglu_2cta(const void* a, const void* b, void* y, void* keep, int M, int I, int K, int E, const int* block_expert, const int* used_blocks,
+                         int block_rows, cudaStream_t st) {
+  if (I % 128 || K % 64 || block_rows % g2::TILE_M) nxd_throw("grouped_swiglu_2cta: I in 128s, K in 64s, blocks of 256 rows", __FILE__, __LINE__);
+  const CUtensorMap ta = make_tmap_bf16(a, M, K, g2::BK, g2::CTA_M), tb = make_tmap_bf16(b, (uint64_t)E * K, 2l * I, 64, g2::BK);
+  const CUtensorMap to = make_tmap_bf16(y, M, I, g2::kEpiSlabCols, g2::CTA_M);
+  const CUtensorMap tk = keep ? make_tmap_bf16(keep, M, 2l * I, g2::kEpiSlabCols, g2::CTA_M) : to;
+  const g2::Group grp{block_expert, nullptr, used_blocks, block_rows, K, E, nullptr};
+  const int tiles = ((M + g2::TILE_M - 1) / g2::TILE_M) * (I / 128), pairs = device_sm_count() / 2, grid = 2 * (tiles < pairs ? tiles : pairs);
+  launch2<true, false, __nv_bfloat16, 7>(ta, tb, to, to, y, M, I, K, keep != nullptr, 1, grp, g2::Tail{0, 1, 1}, grid, st, &tk);
 }
 
 void grouped_wgrad_bf16_2cta(const void* a, const void* b, void* out, int rows_total, int Mo, int No, int E, const int* seg_first_block,

@@ -111,6 +111,8 @@ void zero1_all_gather(const float* master, const int64_t* peer_bufs, long param_
 void gemm_few_rows_swiglu(const void* x, const void* w, void* y, int M, int I, int K, cudaStream_t st);
 bool gemv_swiglu(const void* x, const void* w, void* y, int M, int I, int K, cudaStream_t st);
 size_t gemm_swiglu_2cta_workspace(int M, int I, int K);
+void grouped_swiglu_2cta(const void* a, const void* b, void* y, void* keep, int M, int I, int K, int E, const int* block_expert, const int* used_blocks,
+                         int block_rows, cudaStream_t st);
 void gemm_swiglu_2cta(const void* x, const void* w, void* y, void* keep, int M, int I, int K, float* workspace, cudaStream_t st);
 void gemm_few_rows(const void* x, const void* w, const void* residual, void* y, int M, int N, int K, int split, cudaStream_t st);
 void gemm_fp8(const void* a, const void* b, void* out, int M, int N, int K, const float* scale_a, const float* scale_b,

@@ -129,8 +129,8 @@ def _grouped_swiglu(hidden: torch.Tensor, expert_affinities: torch.Tensor, exper
     T, k = expert_index.shape
     slots = mb.make_slots(expert_index, num_experts, get_num_blocks(T, k, num_experts, mb.BLOCK))
     x = mb.gather(hidden, slots)
-    h = ops.gemm.grouped_matmul(x, experts.gate_up_proj.weight, slots.block_expert, slots.seg, mb.BLOCK, skip_unused=True, slot_token=slots.token)
-    y = ops.gemm.grouped_matmul(ops.act.swiglu(h), experts.down_proj.weight, slots.block_expert, slots.seg, mb.BLOCK, skip_unused=True,
+    h = ops.gemm.grouped_swiglu(x, experts.gate_up_proj.weight, slots.block_expert, slots.seg, mb.BLOCK, slot_token=slots.token)
+    y = ops.gemm.grouped_matmul(h, experts.down_proj.weight, slots.block_expert, slots.seg, mb.BLOCK, skip_unused=True,
                                 slot_token=slots.token)
     return mb.combine(y, expert_affinities.float(), slots)
 

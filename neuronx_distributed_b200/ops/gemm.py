@@ -162,6 +162,10 @@ class _GroupedMatmul(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gy):
         x, w, b2e, seg, slot_token = ctx.saved_tensors
+        return *_GroupedMatmul.gradients(ctx, gy, x, w, b2e, seg, slot_token), None, None, None, None, None
+
+    @staticmethod
+    def gradients(ctx, gy, x, w, b2e, seg, slot_token):
         extra = () if slot_token is None else (slot_token,)
         gy = gy.contiguous()
         gx = gw = None
@@ -181,7 +185,28 @@ class _GroupedMatmul(torch.autograd.Function):
             else:
                 gw = torch.empty_like(w)
                 _ext.ext().grouped_wgrad(x.contiguous(), gy, gw, seg, ctx.block_size, False, *extra)
-        return gx, gw, None, None, None, None, None
+        return gx, gw
+
+
+class _GroupedSwiGLU(torch.autograd.Function):
+    """``_GroupedMatmul`` over the used blocks and SwiGLU in one kernel; the products are kept for the backward pass alone."""
+
+    @staticmethod
+    def forward(ctx, x, w, b2e, seg_first_block, block_size, slot_token, keep):
+        _ext.count_launch()
+        x = x.contiguous()
+        out = _ext.ext().grouped_swiglu(x, w.contiguous(), b2e, block_size, seg_first_block, keep)
+        ctx.block_size, ctx.skip_unused = block_size, True
+        if keep:
+            ctx.save_for_backward(x, w, b2e, seg_first_block, slot_token, out[1])
+        return out[0]
+
+    @staticmethod
+    def backward(ctx, gh):
+        *saved, h = ctx.saved_tensors
+        _ext.count_launch()
+        gy = _ext.ext().swiglu_bwd(gh.contiguous(), h)
+        return *_GroupedMatmul.gradients(ctx, gy, *saved), None, None, None, None, None
 
 
 def grouped_matmul(x: torch.Tensor, w: torch.Tensor, block_to_expert: torch.Tensor, seg_first_block: torch.Tensor,
@@ -192,3 +217,16 @@ def grouped_matmul(x: torch.Tensor, w: torch.Tensor, block_to_expert: torch.Tens
     if _grouped_ok(x, w, block_size):
         return _GroupedMatmul.apply(x, w, block_to_expert.int(), seg_first_block.int(), block_size, skip_unused, slot_token)
     return _grouped_ref(x, w, block_to_expert, block_size)
+
+
+def grouped_swiglu(x: torch.Tensor, w: torch.Tensor, block_to_expert: torch.Tensor, seg_first_block: torch.Tensor, block_size: int,
+                   slot_token: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """SwiGLU of ``grouped_matmul(..., skip_unused=True)``.  Whole tiles of gates and ups on plain CUDA tensors that nobody records or traces: one
+    kernel (8 experts, 4096 tokens of 2 choices, 4096 -> 2 x 3584, both ways, in turn: 1910 us and 2020; 1024 tokens 708 and 770)."""
+    from . import act
+
+    if (_grouped_ok(x, w, block_size) and block_size % 256 == 0 and w.shape[2] % 256 == 0 and x.shape[0] and x.device == w.device and x.dim() == 2
+            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and _ext.native(x, w) is not None):
+        keep = torch.is_grad_enabled() and (x.requires_grad or w.requires_grad)
+        return _GroupedSwiGLU.apply(x, w, block_to_expert.int(), seg_first_block.int(), block_size, slot_token, keep)
+    return act.swiglu(grouped_matmul(x, w, block_to_expert, seg_first_block, block_size, skip_unused=True, slot_token=slot_token))

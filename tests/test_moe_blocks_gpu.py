@@ -63,6 +63,31 @@ def test_experts(T, E, H, I, choice):
             assert not got[3][e].any() and not got[4][e].any()
 
 
+@pytest.mark.parametrize("T,E,H,I", [(40, 4, 64, 128), (700, 8, 320, 256), (1500, 3, 1024, 1408)])
+@pytest.mark.parametrize("grads", [False, True])
+def test_gated_products_are_those_of_two_kernels(T, E, H, I, grads):
+    """The same tiles and sums, SwiGLU of the same rounded products: the same bits, in the rows of blocks with tokens, both ways."""
+    from neuronx_distributed_b200 import ops
+
+    mb = ops.moe_blocks
+    g = torch.Generator(device="cuda").manual_seed(T)
+    idx = torch.stack([torch.randperm(E, generator=g, device="cuda")[:2] for _ in range(T)])
+    slots = mb.make_slots(idx, E, (2 * T + mb.BLOCK - 1) // mb.BLOCK + E)
+    hidden = torch.randn(T, H, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(E, H, 2 * I, generator=g, device="cuda") * H ** -0.5).bfloat16().requires_grad_(grads)
+    x = mb.gather(hidden, slots).detach().requires_grad_(grads)
+    before = ops._ext.launches()
+    one = ops.gemm.grouped_swiglu(x, w, slots.block_expert, slots.seg, mb.BLOCK, slots.token)
+    assert ops._ext.launches() - before == 1
+    two = ops.act.swiglu(ops.gemm.grouped_matmul(x, w, slots.block_expert, slots.seg, mb.BLOCK, skip_unused=True, slot_token=slots.token))
+    used = int(slots.seg[-1]) * mb.BLOCK
+    assert torch.equal(one[:used], two[:used]) and one.requires_grad == grads
+    if grads:
+        go = torch.randn_like(one) * (slots.token >= 0).unsqueeze(1)
+        a, b = (torch.autograd.grad(y, (x, w), go) for y in (one, two))
+        assert torch.equal(a[0][:used], b[0][:used]) and torch.equal(a[1], b[1])
+
+
 @pytest.mark.parametrize("n,E,block", [(1, 1, 128), (1023, 5, 256), (1025, 256, 128), (70000, 33, 256)])
 def test_slots(n, E, block):
     from neuronx_distributed_b200 import ops
