@@ -225,6 +225,13 @@ static void multi_tensor_sq_norm(const std::vector<Tensor>& ts, Tensor out) {
   c10::cuda::CUDAGuard g(ts[0].device());
   nxd::multi_tensor_sq_norm(refs(ts), dt_code(ts[0]), out.data_ptr<float>(), stream());
 }
+static std::vector<Tensor> clip_coefficient(const Tensor& sq, double max_norm) {
+  TORCH_CHECK(sq.is_cuda() && sq.scalar_type() == at::kFloat && sq.numel() == 1);
+  c10::cuda::CUDAGuard g(sq.device());
+  std::vector<Tensor> o{at::empty_like(sq), at::empty_like(sq)};
+  nxd::clip_coefficient(sq.data_ptr<float>(), (float)max_norm, o[0].data_ptr<float>(), o[1].data_ptr<float>(), stream());
+  return o;
+}
 // buffer (fp32) = grad (bf16 / fp16), or += it
 static void grad_to_buffer(const Tensor& grad, Tensor buffer, bool add) {
   CHECK_IN(grad); CHECK_IN(buffer);
@@ -1033,6 +1040,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("ce_loss", &ce_loss);
   m.def("ce_backward", &ce_backward);
   m.def("multi_tensor_sq_norm", &multi_tensor_sq_norm);
+  m.def("clip_coefficient", &clip_coefficient);
   m.def("grad_to_buffer", &grad_to_buffer);
   m.def("multi_tensor_scale", &multi_tensor_scale);
   m.def("fused_adamw", &fused_adamw);

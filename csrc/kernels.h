@@ -39,6 +39,7 @@ void ce_backward(const void* logits, const int64_t* target, const float* lse, co
 
 // ---- optim.cu
 struct TensorRef { void* ptr; long numel; };
+void clip_coefficient(const float* sq, float max_norm, float* norm, float* coeff, cudaStream_t st);
 void multi_tensor_sq_norm(const std::vector<TensorRef>& ts, int dt, float* out, cudaStream_t st);
 void grad_to_buffer(const void* grad, int dt, float* buffer, long n, bool add, cudaStream_t st);
 void multi_tensor_scale(const std::vector<TensorRef>& ts, int dt, const float* scale, cudaStream_t st);

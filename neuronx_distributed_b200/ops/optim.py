@@ -36,6 +36,16 @@ def multi_tensor_sq_norm(tensors: Sequence[torch.Tensor]) -> torch.Tensor:
     return total
 
 
+def clip_coefficient(sq: torch.Tensor, max_norm):
+    """``(norm, coefficient)`` of a squared gradient norm: what clipping to ``max_norm`` multiplies the gradients by, at most 1."""
+    if (isinstance(max_norm, (int, float)) and sq.dtype == torch.float32 and sq.dim() == 0 and _ext.use_cuda(sq)
+            and not (torch.is_grad_enabled() and sq.requires_grad)):
+        _ext.count_launch()
+        return _ext.ext().clip_coefficient(sq, max_norm)
+    norm = sq.sqrt()
+    return norm, torch.clamp(max_norm / (norm + 1e-6), max=1.0)
+
+
 def multi_tensor_scale_(tensors: Sequence[torch.Tensor], scale: Union[float, torch.Tensor]) -> None:
     """In-place ``t *= scale`` for every tensor; ``scale`` may be a device scalar."""
     tensors = [t for t in tensors if t.numel() > 0]

@@ -394,12 +394,14 @@ class Zero1Optimizer(torch.optim.Optimizer):
                     continue
                 piece = fg.grad_shard[s0 : s0 + n]
                 (sharded if getattr(slot.param, "tensor_model_parallel", False) else dup).append(piece)
+        if tp == 1:                                # every weight is one: one launch
+            sharded, dup = sharded + dup, []
         total = ops.optim.multi_tensor_sq_norm(sharded).to(dev) if sharded else torch.zeros((), device=dev)
         if dup:
             total = total + ops.optim.multi_tensor_sq_norm(dup).to(dev) / tp
         return total.float()
 
-    def _global_grad_norm(self) -> torch.Tensor:
+    def _global_sq_norm(self) -> torch.Tensor:
         sq = self._shard_sq_norm()
         if self.world > 1:
             comm.all_reduce(sq, group=self.pg)
@@ -408,7 +410,7 @@ class Zero1Optimizer(torch.optim.Optimizer):
                 comm.all_reduce(sq, group=ps.get_tensor_model_parallel_group())
             if ps.get_pipeline_model_parallel_size() > 1:
                 comm.all_reduce(sq, group=ps.get_pipeline_model_parallel_group())
-        return sq.sqrt()
+        return sq
 
     @property
     def grad_norm(self) -> Optional[torch.Tensor]:
@@ -422,8 +424,7 @@ class Zero1Optimizer(torch.optim.Optimizer):
         self._reduce_scatter_grads()
         coeff = None
         if self.grad_clipping:
-            self._grad_norm = self._global_grad_norm()
-            coeff = torch.clamp(self.max_norm / (self._grad_norm + 1e-6), max=1.0)
+            self._grad_norm, coeff = ops.optim.clip_coefficient(self._global_sq_norm(), self.max_norm)
         for fg in self.flat_groups:
             fg.base_param.grad = fg.grad_shard if fg.grad_shard.dtype == fg.base_param.dtype else fg.grad_shard.to(fg.base_param.dtype)
         self._sync_hparams()
@@ -593,8 +594,7 @@ class NeuronEPZero1Optimizer(torch.optim.Optimizer):
                 comm.all_reduce(sq, group=ps.get_tensor_model_parallel_group())
             if ps.get_pipeline_model_parallel_size() > 1:
                 comm.all_reduce(sq, group=ps.get_pipeline_model_parallel_group())
-            self._grad_norm = sq.sqrt()
-            coeff = torch.clamp(self.max_norm / (self._grad_norm + 1e-6), max=1.0)
+            self._grad_norm, coeff = ops.optim.clip_coefficient(sq, self.max_norm)
         for o in self._opts:
             for fg in o.flat_groups:
                 fg.base_param.grad = fg.grad_shard.to(fg.base_param.dtype)
