@@ -316,7 +316,7 @@ static py::tuple moe_block_metadata(const Tensor& expert_index, int64_t num_expe
 }
 
 // out [V, H] bf16 or fp32 += rows of gy [T, H] bf16 at ids [T] int64 (with zero_first: = )
-static void embedding_grad(const Tensor& ids, const Tensor& gy, Tensor out, bool zero_first) {
+void embedding_grad(const Tensor& ids, const Tensor& gy, Tensor out, bool zero_first) {
   CHECK_IN(ids); CHECK_IN(gy); CHECK_IN(out);
   TORCH_CHECK(ids.scalar_type() == at::kLong && gy.scalar_type() == at::kBFloat16 && (out.scalar_type() == at::kFloat || out.scalar_type() == at::kBFloat16) &&
               gy.dim() == 2 && out.dim() == 2 && gy.size(0) == ids.numel() && gy.size(1) == out.size(1) && gy.size(1) % 8 == 0);

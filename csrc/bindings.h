@@ -23,6 +23,7 @@ std::vector<Tensor> flash_attn_bwd(const Tensor& go, const Tensor& q, const Tens
 void gemm_bf16(const Tensor& a, const Tensor& b, Tensor out, bool trans_a, bool trans_b, bool accumulate);
 void gemm_bf16_2cta(const Tensor& a, const Tensor& b, Tensor out, bool trans_a, bool trans_b, bool accumulate);
 Tensor gemm_few_rows(const Tensor& x, const Tensor& w, int64_t split);
+void embedding_grad(const Tensor& ids, const Tensor& gy, Tensor out, bool zero_first);
 c10::optional<Tensor> linear_swiglu(const Tensor& x, const Tensor& w, bool few, Tensor* keep);
 Tensor gemv(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& residual);
 

@@ -1,5 +1,5 @@
-// Autograd nodes of the training path without Python in them: norms, SwiGLU, rotation of a fused projection, attention, vocabulary loss and
-// the linear layer of one rank.  Each does what the torch.autograd.Function of the same name in ops/ or parallel_layers/layers.py does
+// Autograd nodes of the training path without Python in them: token table, norms, SwiGLU, rotation of a fused projection, attention, vocabulary
+// loss and the linear layer of one rank.  Each does what the torch.autograd.Function of the same name in ops/ or parallel_layers/layers.py does
 // (the same kernels on the same tensors, the same tensors saved); those stay for CPU tensors, tensor subclasses, recording, tracing,
 // functorch and forward-mode AD, which the callers ask about (ops/_ext.py native()).  A node in Python costs about 20 us forward and 40 us
 // backward (its context, the interpreter's lock in the engine's thread, a dozen calls), a small training step has 23 of them: 2750 us a step
@@ -156,6 +156,27 @@ struct CrossEntropy : Function<CrossEntropy> {
     const Tensor d = ce_backward(s[0].contiguous(), s[1].contiguous().to(at::kLong), s[2], g[0].reshape({-1}).to(at::kFloat).contiguous(), 0, 0.0,
                                  s[0].size(1));
     return {d.view(ctx->saved_data["shape"].toIntVector()), Tensor()};
+  }
+};
+
+// Rows of a token table; the gradient (csrc/embedding_grad.cu) goes through autograd like the lookup's own, and only the ids are kept.
+struct TableLookup : Function<TableLookup> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& ids, const Tensor& weight) {
+    ctx->save_for_backward({ids});
+    ctx->saved_data["rows"] = weight.size(0);
+    return at::embedding(weight, ids);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const Tensor ids = ctx->get_saved_variables()[0];
+    const int64_t n = ctx->saved_data["rows"].toInt();
+    if (at::GradMode::is_enabled() || g[0].scalar_type() != at::kBFloat16)      // create_graph: the gradient is differentiated again
+      return {Tensor(), at::embedding_dense_backward(g[0], ids, n, -1, false)};
+    Tensor gy = rows(g[0]).contiguous();
+    if (!aligned(gy)) gy = gy.clone();
+    count(3);
+    const Tensor out = at::empty({n, gy.size(1)}, gy.options());
+    embedding_grad(ids.reshape({-1}).contiguous(), gy, out, true);
+    return {Tensor(), out};
   }
 };
 
@@ -319,6 +340,7 @@ void bind_native_autograd(py::module_& m) {
   });
   n.def("cross_entropy", [](const Tensor& logits, const Tensor& target) { return CrossEntropy::apply(logits, target); });
   n.def("causal_loss", [](const Tensor& logits, const Tensor& labels, bool shift) { return CausalLoss::apply(logits, labels, shift); });
+  n.def("table_lookup", [](const Tensor& ids, const Tensor& weight) { return TableLookup::apply(ids, weight); });
   n.def("linear", &linear);
   n.def("linear_swiglu", [](const Tensor& x, const Tensor& w) { return LinearSwiGLU::apply(x, w); });
   n.def("pairs", &pairs);

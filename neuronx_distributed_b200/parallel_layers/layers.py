@@ -363,7 +363,10 @@ class ParallelEmbedding(BaseParallelLayer):
                 and self.weight.requires_grad and torch.is_grad_enabled() and getattr(self.weight, "main_grad", None) is not None):
             ids = ids.long()
             if _own_table_gradient_ok(ids, self.weight):
-                return _TableLookup.apply(ids, self.weight)
+                from .. import ops
+
+                n = ops._ext.native(ids, self.weight)
+                return _TableLookup.apply(ids, self.weight) if n is None else n.table_lookup(ids, self.weight)
         return F.embedding(
             ids.long(), self.weight, self.padding_idx, self.max_norm, self.norm_type, self.scale_grad_by_freq, self.sparse
         )
@@ -405,6 +408,11 @@ class ParallelEmbedding(BaseParallelLayer):
             return mappings.reduce_scatter_to_sequence_parallel_region(
                 out.transpose(0, 1).contiguous(), 0, self.tensor_model_parallel_group
             )
+        if tp == 1 and isinstance(out, torch.Tensor):
+            from .. import ops
+
+            if ops._ext.native(out) is not None:
+                return out                                  # nothing to add up, and nobody records that
         return mappings.reduce_from_tensor_model_parallel_region(out, self.tensor_model_parallel_group)
 
     def _use_embedding_rs(self, input_: torch.Tensor) -> bool:

@@ -108,3 +108,18 @@ def test_tokens_outside_the_table_add_nothing():
     ops._ext.ext().embedding_grad(ids, gy, out, False)
     ok = (ids >= 0) & (ids < 6)
     _close(out, 1 + _sums(ids[ok], gy[ok], 6), 70)
+
+
+@pytest.mark.parametrize("shape", [(1,), (3, 257), (2, 4, 33)])
+def test_lookups_with_and_without_python_in_their_node(shape):
+    from neuronx_distributed_b200.parallel_layers.layers import _TableLookup
+
+    g = torch.Generator(device="cuda").manual_seed(len(shape))
+    w = torch.randn(500, 72, generator=g, device="cuda").bfloat16().requires_grad_()
+    ids = torch.randint(0, 500, shape, generator=g, device="cuda")
+    go = torch.randn(*shape, 72, generator=g, device="cuda").bfloat16()
+    out = []
+    for lookup in (_TableLookup.apply, ops._ext.ext().native.table_lookup):
+        y = lookup(ids, w)
+        out.append((y, *torch.autograd.grad(y, w, go.transpose(0, -1).contiguous().transpose(0, -1))))
+    assert all(torch.equal(a, b) for a, b in zip(*out)) and torch.equal(out[0][0], w[ids])
