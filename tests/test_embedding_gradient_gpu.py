@@ -112,6 +112,7 @@ def test_tokens_outside_the_table_add_nothing():
 
 @pytest.mark.parametrize("shape", [(1,), (3, 257), (2, 4, 33)])
 def test_lookups_with_and_without_python_in_their_node(shape):
+    from neuronx_distributed_b200 import ops
     from neuronx_distributed_b200.parallel_layers.layers import _TableLookup
 
     g = torch.Generator(device="cuda").manual_seed(len(shape))
