@@ -76,16 +76,21 @@ class _Combine(torch.autograd.Function):
 class _Normalize(torch.autograd.Function):
     @staticmethod
     def forward(ctx, aff, idx):
-        aff = aff.contiguous()
         ctx.save_for_backward(aff, idx)
         _ext.count_launch()
-        return _ext.ext().moe_normalize(aff, idx)
+        return _ext.ext().moe_normalize(aff.contiguous(), idx)
 
     @staticmethod
     def backward(ctx, g):
         aff, idx = ctx.saved_tensors
+        if torch.is_grad_enabled():                         # create_graph: the gradient is differentiated again
+            mask = torch.zeros_like(aff).scatter_(1, idx, 1.0)
+            a = aff * mask
+            total = a.sum(-1, keepdim=True)
+            s = total.clamp(min=1e-9)
+            return (g / s - (g * a / s / s).sum(-1, keepdim=True) * (total >= 1e-9)) * mask, None
         _ext.count_launch()
-        return _ext.ext().moe_normalize_grad(g.contiguous(), aff, idx), None
+        return _ext.ext().moe_normalize_grad(g.contiguous(), aff.contiguous(), idx), None
 
 
 def normalize_ok(aff: torch.Tensor, expert_index: torch.Tensor) -> bool:

@@ -176,3 +176,25 @@ def test_weight_gradients_without_padding(counts, accumulate):
     ops._ext.ext().grouped_wgrad(x, dy, out[0], s.seg, block, accumulate)
     ops._ext.ext().grouped_wgrad(x, dy, out[1], s.seg, block, accumulate, s.token)
     assert torch.equal(out[0], out[1]) and torch.isfinite(out[1]).all()
+
+
+@pytest.mark.parametrize("strided", [False, True])
+def test_normalized_affinities_are_differentiated_twice(strided):
+    from neuronx_distributed_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(5)
+    T, E = 90, 12
+    leaf = torch.rand((E, T) if strided else (T, E), generator=g, device="cuda").requires_grad_()
+    idx = torch.randint(0, E, (T, 3), generator=g, device="cuda")
+    go = torch.randn(T, E, generator=g, device="cuda")
+    results = []
+    for kernel in (True, False):
+        aff = leaf.double() if not kernel else leaf
+        aff = aff.t() if strided else aff
+        assert not kernel or ops.moe_blocks.normalize_ok(aff, idx)
+        m = aff * torch.zeros_like(aff).scatter_(1, idx, 1.0)
+        w = ops.moe_blocks.normalize(aff, idx) if kernel else m / m.sum(-1, keepdim=True).clamp(min=1e-9)
+        (first,) = torch.autograd.grad((w.square() * go).sum(), leaf, create_graph=True)
+        results.append([first, *torch.autograd.grad(first.square().sum(), leaf)])
+    for a, b in zip(*results):                # sums of up to three products and quotients in 32 bits, twice
+        assert (a.double() - b).norm() <= 1e-5 * b.norm()
