@@ -424,14 +424,32 @@ static Tensor decode_rope_kv(const Tensor& q, const Tensor& k, const Tensor& v, 
 
 // ---- decode ---------------------------------------------------------------------------------------
 // q [B,1,H,128]; k/v cache [B,L,Hkv,128] (any b/s/h strides, head_dim contiguous); positions [B] int64 (attend to ≤ pos)
+// Rows of 128 at addresses that are multiples of `bytes` = `step` elements; strides of dimensions of one don't matter
+static bool rows_at(const Tensor& t, int64_t step, uintptr_t bytes) {
+  bool ok = t.stride(3) == 1 && (uintptr_t)t.data_ptr() % bytes == 0;
+  for (int d = 0; d < 3; ++d) ok = ok && (t.size(d) == 1 || t.stride(d) % step == 0);
+  return ok;
+}
+// Whether single-token attention goes to decode_attn_kernel: one to eight query heads per cache head, cache rows of whole 16-byte packets and queries
+// of 4-byte words, as it copies and reads them.  Shapes that don't belong together go to it as well, to be refused.  No launch, any device
+static bool decode_views_ok(const Tensor& q, const Tensor& k, const Tensor& v) {
+  if (q.dim() != 4 || k.dim() != 4 || v.dim() != 4 || k.size(2) < 1 || k.stride(3) != 1 || v.stride(3) != 1) return false;
+  const int64_t group = q.size(2) / k.size(2);
+  if (q.size(2) % k.size(2) || group < 1 || group > 8) return false;
+  if (q.size(1) != 1) return true;
+  if (v.sizes() != k.sizes() || v.scalar_type() != k.scalar_type()) return (group & (group - 1)) == 0;
+  return rows_at(k, 8, 16) && rows_at(v, 8, 16) && (!q.is_contiguous() || rows_at(q, 2, 4));      // other queries are copied first
+}
+static void check_decode(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& positions) {
+  TORCH_CHECK(q.is_cuda() && q.scalar_type() == at::kBFloat16 && q.dim() == 4 && q.size(1) == 1 && q.size(3) == 128);
+  TORCH_CHECK(k.scalar_type() == at::kBFloat16 && k.dim() == 4 && k.size(3) == 128 && v.scalar_type() == at::kBFloat16 && v.sizes() == k.sizes());
+  TORCH_CHECK(k.device() == q.device() && v.device() == q.device() && k.size(0) == q.size(0) && k.size(2) > 0 && q.size(2) % k.size(2) == 0);
+  TORCH_CHECK(rows_at(k, 8, 16) && rows_at(v, 8, 16) && rows_at(q, 2, 4), "decode_attention: cache rows are whole 16-byte packets, queries 4-byte words");
+  TORCH_CHECK(positions.scalar_type() == at::kLong && positions.device() == q.device() && positions.is_contiguous() && positions.numel() == q.size(0));
+}
 static Tensor decode_attention(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& positions, double scale) {
-  TORCH_CHECK(q.is_cuda() && q.scalar_type() == at::kBFloat16 && q.dim() == 4 && q.size(1) == 1 && q.size(3) == 128 && q.stride(3) == 1);
-  TORCH_CHECK(k.scalar_type() == at::kBFloat16 && k.dim() == 4 && k.size(3) == 128 && k.stride(3) == 1 && v.stride(3) == 1 &&
-              v.sizes() == k.sizes());
-  TORCH_CHECK(positions.scalar_type() == at::kLong && positions.is_cuda() && positions.is_contiguous() && positions.numel() == q.size(0));
+  check_decode(q, k, v, positions);
   const int B = q.size(0), H = q.size(2), L = k.size(1), Hkv = k.size(2);
-  TORCH_CHECK(H % Hkv == 0 && k.size(0) == B);
-  TORCH_CHECK(q.stride(2) % 8 == 0 && k.stride(1) % 8 == 0 && k.stride(2) % 8 == 0 && v.stride(1) % 8 == 0 && v.stride(2) % 8 == 0);
   c10::cuda::CUDAGuard guard(q.device());
   const int splits = nxd::decode_splits(B * Hkv, L);
   Tensor out = at::empty({B, 1, H, 128}, q.options());
@@ -448,13 +466,8 @@ static Tensor decode_attention(const Tensor& q, const Tensor& k, const Tensor& v
 // >= L: nothing / everything of this shard is visible).
 static std::vector<Tensor> decode_attention_partial(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& positions,
                                                     double scale) {
-  TORCH_CHECK(q.is_cuda() && q.scalar_type() == at::kBFloat16 && q.dim() == 4 && q.size(1) == 1 && q.size(3) == 128 && q.stride(3) == 1);
-  TORCH_CHECK(k.scalar_type() == at::kBFloat16 && k.dim() == 4 && k.size(3) == 128 && k.stride(3) == 1 && v.stride(3) == 1 &&
-              v.sizes() == k.sizes());
-  TORCH_CHECK(positions.scalar_type() == at::kLong && positions.is_cuda() && positions.is_contiguous() && positions.numel() == q.size(0));
+  check_decode(q, k, v, positions);
   const int B = q.size(0), H = q.size(2), L = k.size(1), Hkv = k.size(2);
-  TORCH_CHECK(H % Hkv == 0 && k.size(0) == B);
-  TORCH_CHECK(q.stride(2) % 8 == 0 && k.stride(1) % 8 == 0 && k.stride(2) % 8 == 0 && v.stride(1) % 8 == 0 && v.stride(2) % 8 == 0);
   c10::cuda::CUDAGuard guard(q.device());
   const int splits = nxd::decode_splits(B * Hkv, L);
   Tensor fin_o = at::empty({B, H, 128}, q.options().dtype(at::kFloat));
@@ -1051,6 +1064,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_bf16_2cta", &gemm_bf16_2cta);
   m.def("oneshot_allreduce", &oneshot_allreduce);
   m.def("decode_attention", &decode_attention);
+  m.def("decode_views_ok", &decode_views_ok);
   m.def("decode_attention_partial", &decode_attention_partial);
   m.def("nvls_embedding_gather", &nvls_embedding_gather);
   m.def("nvls_publish", &nvls_publish);

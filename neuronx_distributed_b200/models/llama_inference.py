@@ -322,7 +322,7 @@ def _decode_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, positio
     Hkv, L = k.shape[2], k.shape[1]
     e = ops._ext.ext() if q.is_cuda else None
     if (e is not None and hasattr(e, "decode_attention") and D == 128 and q.dtype == torch.bfloat16 and k.dtype == torch.bfloat16
-            and k.stride(3) == 1 and v.stride(3) == 1 and ops.attention.decode_group_ok(q, k, v)):
+            and ops.attention.decode_group_ok(q, k, v)):
         # flash-decoding kernel (csrc/decode.cu): split over the cache length, GQA group shares each K/V read
         ops._ext.count_launch(2)
         return e.decode_attention(q.contiguous(), k, v, positions.to(torch.long).contiguous(), 1.0 / math.sqrt(D))

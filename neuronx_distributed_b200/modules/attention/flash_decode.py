@@ -43,12 +43,12 @@ def _local_partial(q_all: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
 
     CUDA / bf16 / head_dim 128: the split-KV decode kernel (``csrc/decode.cu`` ``decode_attn_kernel`` + the partial combine):
     K/V are read once per KV head for the whole GQA group.  Otherwise fp32 torch math."""
-    from ...ops import _ext
+    from ...ops import _ext, attention
 
     B, _, H, D = q_all.shape
     l_local, Hkv = k_cache.shape[1], k_cache.shape[2]
     if (_ext.use_cuda(q_all, k_cache, v_cache) and q_all.dtype == torch.bfloat16 and k_cache.dtype == torch.bfloat16 and D == 128
-            and H % Hkv == 0 and (H // Hkv) in (1, 2, 4, 8) and hasattr(_ext.ext(), "decode_attention_partial")):
+            and hasattr(_ext.ext(), "decode_attention_partial") and attention.decode_group_ok(q_all, k_cache, v_cache)):
         _ext.count_launch(2)
         o, ml = _ext.ext().decode_attention_partial(q_all.contiguous(), k_cache, v_cache, local_pos.to(torch.long).contiguous(),
                                                     float(scale))

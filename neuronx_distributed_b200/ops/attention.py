@@ -128,13 +128,9 @@ def flash_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: b
 
 
 def decode_group_ok(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bool:
-    """Up to eight query heads per key/value head are what the single-token kernels share a cache row among.  Groups of 3, 5, 6 and 7 take caches
-    whose rows are whole 16-byte packets; others go the general way, as all of them once did."""
-    H, Hkv = q.shape[2], k.shape[2]
-    if H // Hkv in (1, 2, 4, 8):
-        return True
-    return (H % Hkv == 0 and H // Hkv <= 8 and v.dtype == k.dtype and v.shape == k.shape
-            and all(t.data_ptr() % 16 == 0 and all(t.stride(d) % 8 == 0 for d in range(3)) for t in (k, v)))
+    """Up to eight query heads per key/value head are what the single-token kernels share a cache row among.  They take caches whose rows are
+    whole 16-byte packets; others go the general way."""
+    return _ext._load().decode_views_ok(q, k, v)
 
 
 def decode_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, positions: torch.Tensor,
@@ -147,7 +143,7 @@ def decode_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
     e = _ext.ext() if q.is_cuda else None
     if (e is not None and hasattr(e, "decode_attention") and D == 128 and q.dtype == torch.bfloat16 and k_cache.dtype == torch.bfloat16
-            and k_cache.stride(3) == 1 and v_cache.stride(3) == 1 and decode_group_ok(q, k_cache, v_cache)):
+            and decode_group_ok(q, k_cache, v_cache)):
         _ext.count_launch(2)
         return e.decode_attention(q.contiguous(), k_cache, v_cache, positions.to(torch.long).contiguous(), float(scale))
     qt, kt, vt = q.transpose(1, 2), k_cache.transpose(1, 2), v_cache.transpose(1, 2)

@@ -89,3 +89,41 @@ def test_rows_that_are_no_packets_go_the_general_way():
     want = _reference(q, k, v, pos)
     got = ops.attention.decode_attention(q, k, v, pos).float()
     assert not ops.attention.decode_group_ok(q, k, v) and (got - want).abs().max() <= 2.0 ** -7 * want.abs().max()      # general way: bf16 probabilities too
+
+
+@pytest.mark.parametrize("group", [1, 2, 4, 8])
+def test_such_rows_of_every_group(group):
+    from neuronx_distributed_b200 import ops
+    from neuronx_distributed_b200.models import llama_inference
+    from neuronx_distributed_b200.modules.attention.flash_decode import _local_partial
+
+    g = torch.Generator(device="cuda").manual_seed(group)
+    q = torch.randn(2, 1, 2 * group, 128, generator=g, device="cuda").bfloat16()
+    pos = torch.tensor([89, 60], device="cuda")
+    rows = torch.randn(2, 2, 90, 2, 136, generator=g, device="cuda").bfloat16()
+    for k, v in (rows[..., 4:132].unbind(), (rows[0, ..., :128], rows[1, ..., 1:129])):
+        assert not ops.attention.decode_group_ok(q, k, v)
+        want = _reference(q, k, v, pos)
+        o, _, l = _local_partial(q, k, v, pos, 128 ** -0.5)
+        for got in (ops.attention.decode_attention(q, k, v, pos), llama_inference._decode_attention(q, k, v, pos), (o / l[..., None]).unsqueeze(1)):
+            assert (got.float() - want).abs().max() <= 2.0 ** -7 * want.abs().max()
+
+
+@pytest.mark.parametrize("group", [3, 5, 6, 7])
+def test_parts_of_groups_of_other_sizes(group):
+    """A shard of a cache, as distributed decoding calls it: un-normalised output, row maximum and row sum."""
+    from neuronx_distributed_b200 import ops
+    from neuronx_distributed_b200.modules.attention.flash_decode import _local_partial
+
+    g = torch.Generator(device="cuda").manual_seed(group)
+    k, v = (torch.randn(2, 300, 2, 128, generator=g, device="cuda").bfloat16() for _ in range(2))
+    q = torch.randn(2, 1, 2 * group, 128, generator=g, device="cuda").bfloat16()
+    pos = torch.tensor([400, 70], device="cuda")
+    before = ops._ext.launches()
+    o, m, l = _local_partial(q, k, v, pos, 128 ** -0.5)
+    assert ops._ext.launches() - before == 2
+    want = _reference(q, k, v, pos)[:, 0]
+    assert (o / l[..., None] - want).abs().max() <= 2.0 ** -8 * want.abs().max()
+    s = torch.einsum("bhd,blhd->bhl", q[:, 0].float(), k.float().repeat_interleave(group, 2)) * 128 ** -0.5
+    s[1, :, 71:] = -math.inf
+    torch.testing.assert_close(m, s.amax(-1), rtol=1e-5, atol=1e-5)
