@@ -313,6 +313,7 @@ def _window_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, positio
         inside = (rel >= 0) & (rel < W)
         tm = tree_mask.to(q.device)[:, rel.clamp(0, W - 1)].permute(1, 0, 2)                   # [B, W, L]
         mask = ((rel < 0)[:, None, :] | (inside[:, None, :] & tm))[:, None]
+    qt, kt, vt = (ops.attention.packets(t) for t in (qt, kt, vt))
     return torch.nn.functional.scaled_dot_product_attention(qt, kt, vt, attn_mask=mask).transpose(1, 2)
 
 
@@ -331,5 +332,6 @@ def _decode_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, positio
     if H != Hkv:
         kt, vt = kt.repeat_interleave(H // Hkv, 1), vt.repeat_interleave(H // Hkv, 1)
     mask = (torch.arange(L, device=q.device)[None, :] <= positions[:, None])[:, None, None, :]
+    qt, kt, vt = (ops.attention.packets(t) for t in (qt, kt, vt))
     o = torch.nn.functional.scaled_dot_product_attention(qt, kt, vt, attn_mask=mask)
     return o.transpose(1, 2)

@@ -16,13 +16,28 @@ import torch.nn.functional as F
 from . import _ext
 
 
+def whole_packets(t: torch.Tensor) -> bool:
+    """Every row (last dimension) begins at a multiple of 16 bytes."""
+    size = t.element_size()
+    return (t.data_ptr() % 16 == 0 and t.stride(-1) == 1
+            and all(n == 1 or st * size % 16 == 0 for n, st in zip(t.shape[:-1], t.stride()[:-1])))
+
+
+def packets(t: torch.Tensor) -> torch.Tensor:
+    """What PyTorch's attention kernels can load: they read rows in 16-byte packets from wherever a view begins, which on others is a misaligned
+    access.  Those are copied.  (Rows that are strided or no whole packets by themselves do not go to those kernels, or are padded there.)"""
+    if not t.is_cuda or t.stride(-1) != 1 or t.shape[-1] * t.element_size() % 16 or whole_packets(t):
+        return t
+    return t.clone(memory_format=torch.contiguous_format)
+
+
 def _sdpa(q, k, v, causal: bool, scale: Optional[float]):
     hq, hkv = q.shape[2], k.shape[2]
     qt, kt, vt = q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2)
     if hq != hkv:
         kt = kt.repeat_interleave(hq // hkv, dim=1)
         vt = vt.repeat_interleave(hq // hkv, dim=1)
-    o = F.scaled_dot_product_attention(qt, kt, vt, is_causal=causal, scale=scale)
+    o = F.scaled_dot_product_attention(packets(qt), packets(kt), packets(vt), is_causal=causal, scale=scale)
     return o.transpose(1, 2)
 
 
@@ -150,4 +165,4 @@ def decode_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
     if H != Hkv:
         kt, vt = kt.repeat_interleave(H // Hkv, 1), vt.repeat_interleave(H // Hkv, 1)
     mask = (torch.arange(L, device=q.device)[None, :] <= positions[:, None])[:, None, None, :]
-    return torch.nn.functional.scaled_dot_product_attention(qt, kt, vt, attn_mask=mask, scale=scale).transpose(1, 2)
+    return F.scaled_dot_product_attention(packets(qt), packets(kt), packets(vt), attn_mask=mask, scale=scale).transpose(1, 2)

@@ -67,3 +67,22 @@ def test_groups_of_more_than_eight_heads_go_the_general_way():
     if ops._ext._load() is None:
         pytest.skip("extension not built")
     assert not ops.attention.decode_group_ok(torch.zeros(2, 1, 18, 128, dtype=torch.bfloat16), *_caches())
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+def test_views_of_whole_packets(dtype):
+    """What the library's attention gets as it is: rows at multiples of 16 bytes; strides of dimensions of one don't count."""
+    import torch
+
+    from neuronx_distributed_b200 import ops
+
+    ok, per = ops.attention.whole_packets, 16 // getattr(torch, dtype).itemsize
+    t = torch.zeros(2 * 3 * 5 * 144 + 16, dtype=getattr(torch, dtype))
+    assert t.data_ptr() % 16 == 0
+
+    def view(shape=(2, 3, 5, 128), strides=(3 * 5 * 144, 5 * 144, 144, 1), offset=0):
+        return t.as_strided(shape, strides, offset)
+
+    assert ok(view()) and ok(view(offset=per)) and ok(view().transpose(1, 2)) and ok(view((1, 3, 1, 128), (3, 144, 7, 1)))
+    assert not ok(view(offset=1)) and not ok(view(offset=per // 2)) and not ok(view(strides=(3 * 5 * 144, 5 * 144, 128 + per // 2, 1)))
+    assert not ok(view(strides=(3 * 5 * 144 - 1, 5 * 144, 144, 1))) and not ok(view().transpose(2, 3))
