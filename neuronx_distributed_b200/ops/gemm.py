@@ -188,25 +188,18 @@ class _GroupedMatmul(torch.autograd.Function):
         return gx, gw
 
 
-class _GroupedSwiGLU(torch.autograd.Function):
-    """``_GroupedMatmul`` over the used blocks and SwiGLU in one kernel; the products are kept for the backward pass alone."""
+class _GroupedProducts(torch.autograd.Function):
+    """``_GroupedMatmul`` over the used blocks, its ``products`` ([] around them: they are no input) computed already."""
 
     @staticmethod
-    def forward(ctx, x, w, b2e, seg_first_block, block_size, slot_token, keep):
-        _ext.count_launch()
-        x = x.contiguous()
-        out = _ext.ext().grouped_swiglu(x, w.contiguous(), b2e, block_size, seg_first_block, keep)
+    def forward(ctx, x, w, b2e, seg_first_block, block_size, slot_token, products):
         ctx.block_size, ctx.skip_unused = block_size, True
-        if keep:
-            ctx.save_for_backward(x, w, b2e, seg_first_block, slot_token, out[1])
-        return out[0]
+        ctx.save_for_backward(x, w, b2e, seg_first_block, slot_token)
+        return products[0]
 
     @staticmethod
-    def backward(ctx, gh):
-        *saved, h = ctx.saved_tensors
-        _ext.count_launch()
-        gy = _ext.ext().swiglu_bwd(gh.contiguous(), h)
-        return *_GroupedMatmul.gradients(ctx, gy, *saved), None, None, None, None, None
+    def backward(ctx, gy):
+        return *_GroupedMatmul.gradients(ctx, gy, *ctx.saved_tensors), None, None, None, None, None
 
 
 def grouped_matmul(x: torch.Tensor, w: torch.Tensor, block_to_expert: torch.Tensor, seg_first_block: torch.Tensor,
@@ -227,6 +220,13 @@ def grouped_swiglu(x: torch.Tensor, w: torch.Tensor, block_to_expert: torch.Tens
 
     if (_grouped_ok(x, w, block_size) and block_size % 256 == 0 and w.shape[2] % 256 == 0 and x.shape[0] and x.device == w.device and x.dim() == 2
             and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and _ext.native(x, w) is not None):
-        keep = torch.is_grad_enabled() and (x.requires_grad or w.requires_grad)
-        return _GroupedSwiGLU.apply(x, w, block_to_expert.int(), seg_first_block.int(), block_size, slot_token, keep)
+        keep, b2e, seg = torch.is_grad_enabled() and (x.requires_grad or w.requires_grad), block_to_expert.int(), seg_first_block.int()
+        _ext.count_launch()
+        x = x.contiguous()
+        with torch.no_grad():
+            out = _ext.ext().grouped_swiglu(x, w.contiguous(), b2e, block_size, seg, keep)
+        if not keep:
+            return out[0]
+        # two nodes: the products are given back before the gradients of rows and weights need memory
+        return _ext.native(x, w).swiglu_of(_GroupedProducts.apply(x, w, b2e, seg, block_size, slot_token, out[1:]), out[0])
     return act.swiglu(grouped_matmul(x, w, block_to_expert, seg_first_block, block_size, skip_unused=True, slot_token=slot_token))

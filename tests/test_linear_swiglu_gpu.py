@@ -146,3 +146,41 @@ def test_rows_of_any_number(M, grads):
         gx, gw = torch.autograd.grad(y, (x, w), go)
         for a, b in ((gx, go.double() @ w.double()), (gw, go.double().t() @ x.double())):
             assert float((a.double() - b).norm() / b.norm()) < 2 ** -8
+
+
+def _peak_of_backward(forward, args):
+    """Bytes above what is held before the backward pass."""
+    y = forward()
+    go = torch.ones_like(y)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    held = torch.cuda.memory_allocated()
+    torch.autograd.grad(y, args, go)
+    return torch.cuda.max_memory_allocated() - held
+
+
+def test_products_are_given_back_before_the_gradients_are_computed():
+    """The backward pass needs no more memory than that of the two nodes: gradients of 2 I columns, of x and of W without the products."""
+    from neuronx_distributed_b200.parallel_layers.layers import ColumnParallelLinear, column_swiglu
+
+    _mlp()
+    M, I, K = 2048, 2816, 1024
+    x, w = _case(M, I, K)
+    proj = ColumnParallelLinear(K, 2 * I, bias=False, gather_output=False, dtype=torch.bfloat16, device=torch.device("cuda", 0))
+    proj.weight.data.copy_(w)
+    x.requires_grad_()
+    one, two = (_peak_of_backward(f, (x, proj.weight)) for f in (lambda: column_swiglu(proj, x), lambda: ops.act.swiglu(proj(x))))
+    assert one <= two + 2 ** 16 and one < 2 * (M * 2 * I + M * K + 2 * I * K)
+
+
+def test_products_of_experts_are_given_back_before_the_gradients_are_computed():
+    mb = ops.moe_blocks
+    T, E, H, I = 2048, 4, 512, 1408
+    idx = torch.stack([torch.randperm(E, device="cuda")[:2] for _ in range(T)])
+    slots = mb.make_slots(idx, E, (2 * T + mb.BLOCK - 1) // mb.BLOCK + E)
+    x = mb.gather(torch.randn(T, H, device="cuda").bfloat16(), slots).detach().requires_grad_()
+    w = (torch.randn(E, H, 2 * I, device="cuda") * H ** -0.5).bfloat16().requires_grad_()
+    a = (x, w, slots.block_expert, slots.seg, mb.BLOCK)
+    one, two = (_peak_of_backward(f, (x, w)) for f in (
+        lambda: ops.gemm.grouped_swiglu(*a, slots.token), lambda: ops.act.swiglu(ops.gemm.grouped_matmul(*a, skip_unused=True, slot_token=slots.token))))
+    assert one <= two + 2 ** 16
