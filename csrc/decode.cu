@@ -367,9 +367,11 @@ void decode_attention(const void* q, const void* k, const void* v, const long* p
   dim3 grid(Hkv, B, splits);
   const float sl2 = scale * 1.4426950408889634f;
   const bool whole = splits == 1 && fin_o == nullptr;
-  // Launches that three blocks per SM take at once are a few round trips to memory long, and need them deeper rather than more of them
-  // at a time; so do blocks that copy long stretches for a single head and have little else to do (8 x 8192 rows, 32 heads: 111.0 us and 112.3).
-  const bool few = (long)Hkv * B * splits <= 3l * device_sm_count() || (G == 1 && L / splits >= 2000);
+  // Launches that three blocks per SM take at once are a few round trips to memory long, and need them deeper rather than more of them at a time.
+  // Single heads' blocks copy the most and compute the least: in launches of 896 to 1280 of them, caches in memory, two stages took 0.89 to 1.02 of
+  // the time of three (16 x 2048 rows, 8 heads: 20.7 us and 23.2; 16 x 4096, 40 heads: 144.6 and 148.2; 8 x 8192, 32 heads: 118.4 and 118.1;
+  // 3 x 16384, 32 heads: 103.2 and 100.9), by no length of theirs in particular.
+  const bool few = (long)Hkv * B * splits <= 3l * device_sm_count();
 #define NXD_DEC_STAGES(Gv, Sv)                                                                                       \
   do {                                                                                                               \
     NXD_ALLOW_SMEM((decode_attn_kernel<Gv, Sv>), dec_smem_bytes(Sv));                                                  \

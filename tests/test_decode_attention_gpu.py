@@ -58,7 +58,7 @@ def test_partial_results_merge_to_the_whole():
 @pytest.mark.parametrize("batch,kv_heads,group,rows", [(1, 1, 4, 4096), (1, 1, 8, 4097), (1, 1, 1, 8193), (1, 1, 2, 20000), (1, 40, 1, 2048), (4, 8, 4, 7000),
                                                       (16, 8, 8, 4096), (3, 37, 2, 511)])
 def test_numbers_of_stretches(batch, kv_heads, group, rows):
-    """Merges of 2 to 64 stretches (16 of them at once), launches of more and of fewer than two blocks per SM."""
+    """Merges of 2 to 64 stretches (16 of them at once), launches of more and of fewer than three blocks per SM."""
     from neuronx_distributed_b200 import ops
 
     g = torch.Generator(device="cuda").manual_seed(rows)
@@ -127,3 +127,27 @@ def test_parts_of_groups_of_other_sizes(group):
     s = torch.einsum("bhd,blhd->bhl", q[:, 0].float(), k.float().repeat_interleave(group, 2)) * 128 ** -0.5
     s[1, :, 71:] = -math.inf
     torch.testing.assert_close(m, s.amax(-1), rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("batch,kv_heads,group,rows", [(16, 8, 1, 2000), (16, 8, 2, 2000), (16, 8, 3, 1999), (16, 8, 5, 2001), (16, 8, 6, 2000), (16, 8, 7, 1900),
+                                                      (8, 32, 1, 4096), (8, 32, 1, 8192)])
+def test_launches_of_more_than_three_blocks_per_sm(batch, kv_heads, group, rows):
+    """Two stages a warp: sequences of no row, of one, of a tile more or less, of every row, and of lengths in between."""
+    from neuronx_distributed_b200 import ops
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert batch * kv_heads * min((6 * sms + batch * kv_heads - 1) // (batch * kv_heads), (rows + 255) // 256) > 3 * sms
+    g = torch.Generator(device="cuda").manual_seed(rows + group)
+    k, v = (torch.randn(batch, rows, kv_heads, 128, generator=g, device="cuda").bfloat16() for _ in range(2))
+    q = torch.randn(batch, 1, kv_heads * group, 128, generator=g, device="cuda").bfloat16() * 2
+    pos = torch.randint(0, rows, (batch,), generator=g, device="cuda")
+    pos[:7] = torch.tensor([-1, 0, 63, 64, rows - 1, rows + 5, rows // 2])
+    want = _reference(q, k, v, pos)
+    for b, p in enumerate(pos.tolist()):
+        k[b, p + 1:], v[b, p + 1:] = math.nan, math.nan                            # rows behind the position are never used
+    got = ops.attention.decode_attention(q, k, v, pos).float()
+    for b in range(batch):                                                         # one rounding to bfloat16 over fp32 sums
+        assert (got[b] - want[b]).abs().max() <= 2.0 ** -8 * want[b].abs().max()
+    o, ml = ops._ext.ext().decode_attention_partial(q, k, v, pos, 128 ** -0.5)
+    o = torch.where(ml[..., 1:] > 0, o / ml[..., 1:], 0)
+    assert (o - want[:, 0]).abs().max() <= 2.0 ** -8 * want.abs().max()
