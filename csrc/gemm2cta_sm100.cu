@@ -835,8 +835,14 @@ static CUtensorMap out_map(const void* out, int out_dt, bool accumulate, bool ma
 }
 
 // How a product is shared out: tiles of 256 or 128 columns; split-K of every tile (fp32 outputs), or of the last round's tiles alone, or neither.
-// A k-block of a 256 x 256 tile takes 0.31 us and one of 256 x 128 0.23 (their operands, 32 and 24 KB a CTA, come at about 105 GB/s an SM), a
-// launch 5; a pass over fp32 memory: 6 bytes/ps.
+// In us, for the estimates: a k-block of a 256 x 256 tile and of one of 256 x 128 (their operands, 32 and 24 KB a CTA, come at about 105 GB/s an
+// SM); the launch that sums a tail; a MB of a tail's fp32 parts and of a pass over fp32 outputs.
+constexpr double kWideUs = 0.31, kNarrowUs = 0.2325, kTailUs = 2.0, kPartUs = 1 / 7.0, kPassUs = 1 / 6.0;
+// A tail's parts fill at most this many rounds of pairs, 58 MB of fp32 on 148 SMs: what a product may take beside its output.  In one, two, three
+// and any number of rounds, us: 2048 x 4096 x 22016 308 / 310 / 292 / 292 (57 MB), 2048 x 4096 x 32000 464 / 468 / 426 / 429 (57), 512 x 5120 x 27648
+// 163 / 141 / 137 / 137 (52), 704 x 4096 x 22016 159 / 117 / 116 / 116 (38), 1000 x 4096 x 32064 216 in all.  Without it 134 MB for
+// 1000 x 4096 x 128256.
+constexpr int kTailRounds = 3;
 struct GemmPlan { int tiles, split, width; g2::Tail tail; };      // width: columns of a tile
 static GemmPlan gemm_plan(int M, int N, int K, int out_dt, bool accumulate, bool split_k, bool narrow = true) {
   const int pairs = std::max(1, device_sm_count() / 2), num_kb = (K + g2::BK - 1) / g2::BK;      // (no device: one, for the asking)
@@ -844,10 +850,10 @@ static GemmPlan gemm_plan(int M, int N, int K, int out_dt, bool accumulate, bool
   GemmPlan p;
   double best = 1e30;
   for (int width = 256; width >= (narrow ? 128 : 256); width /= 2) {
-    const double kb_us = width == 256 ? 0.31 : 0.2325;
+    const double kb_us = width == 256 ? kWideUs : kNarrowUs;
     const int tiles = tiles_m * ((N + width - 1) / width);
     // The tail: the tiles of the last, partial round in s parts each, which may be several rounds themselves; worth it where it saves more than
-    // the launch that sums (2 us) and its traffic.  Chosen so and before (256 columns, s pairs a tile in one round), us: 512 x 5120 x 13824 in 3
+    // the launch that sums and its traffic.  Chosen so and before (256 columns, s pairs a tile in one round), us: 512 x 5120 x 13824 in 3
     // parts 64 and 74; 704 x 4096 x 11008 in 3 parts 56 and 62; 304 x 4096 x 4096 in 128 columns 19.6 and 21.2, 304 x 1024 x 2816 in 128 columns
     // and 4 parts 10.6 and 15.8, 1000 x 1024 x 1024 in 128 columns 8.2 and 10.0; 1000 x 5120 x 13824 (80 tiles) 101 in 5 parts, 147 without.  66
     // such products of 200 to 1504 rows: none slower than before by more than its noise but one (200 x 4096 x 11008, 37 and 34), a twelfth of a per
@@ -857,8 +863,9 @@ static GemmPlan gemm_plan(int M, int N, int K, int out_dt, bool accumulate, bool
     for (int s = 1; s <= (last > 0 ? 16 : 1); ++s) {
       const int per = (num_kb + s - 1) / s;
       if (s > 1 && (num_kb / s < 4 || per * (s - 1) >= num_kb)) continue;      // short parts, or an empty one
+      if (s > 1 && last * s * width > kTailRounds * pairs * g2::TILE_N) break;
       const int rounds = (last * s + pairs - 1) / pairs;
-      double cost = ((tiles / pairs) * num_kb + rounds * per) * kb_us + (s > 1 ? 2.0 + 2.0 * last * s * width * 0.001024 / 7.0 : 0.);
+      double cost = ((tiles / pairs) * num_kb + rounds * per) * kb_us + (s > 1 ? kTailUs + 2.0 * last * s * width * 0.001024 * kPartUs : 0.);
       if (s > 1) cost /= 0.97;                             // a tie stays whole
       if (cost < best) {
         best = cost;
@@ -874,12 +881,12 @@ static GemmPlan gemm_plan(int M, int N, int K, int out_dt, bool accumulate, bool
   // tiles are a tail, whose partials are summed in order, so that the same inputs give the same bits.
   if (out_dt == kF32 && M >= g2::TILE_M && split_k) {
     const int tiles = tiles_m * ((N + g2::TILE_N - 1) / g2::TILE_N);
-    const double pass_us = (double)M * N * 4 / 6e6;
+    const double pass_us = (double)M * N * 4e-6 * kPassUs;
     for (int s2 = 2; s2 <= 8; ++s2) {
       if (num_kb / s2 < 16) break;
       const int per = (num_kb + s2 - 1) / s2;
       if (per * (s2 - 1) >= num_kb) continue;                       // would leave an empty split
-      const double cost = (double)((tiles * s2 + pairs - 1) / pairs) * per * 0.31 + (s2 - 1) * pass_us + (accumulate ? 0. : pass_us);
+      const double cost = (double)((tiles * s2 + pairs - 1) / pairs) * per * kWideUs + (s2 - 1) * pass_us + (accumulate ? 0. : pass_us);
       if (cost < best) {
         best = cost;
         p.tiles = tiles; p.split = s2; p.width = g2::TILE_N;
@@ -890,7 +897,7 @@ static GemmPlan gemm_plan(int M, int N, int K, int out_dt, bool accumulate, bool
   return p;
 }
 
-// bytes of fp32 workspace that gemm_bf16_2cta takes for these sizes (0: none)
+// bytes of fp32 workspace that gemm_bf16_2cta takes for these sizes (0: none; at most kTailRounds * 256 KB for each pair of SMs)
 size_t gemm_2cta_workspace(int M, int N, int K, int out_dt, bool accumulate, bool split_k) {
   const GemmPlan p = gemm_plan(M, N, K, out_dt, accumulate, split_k);
   return (size_t)p.tail.tiles * p.tail.splits * g2::TILE_M * p.width * sizeof(float);

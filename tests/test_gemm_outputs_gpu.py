@@ -119,3 +119,25 @@ def test_tail_of_many_parts(M, N, K, trans):
     again = torch.empty_like(out)
     e.gemm_bf16_2cta(a, b, again, trans[0], trans[1], False)
     assert torch.equal(out, again)
+
+
+def test_parts_of_a_tail_are_bounded():
+    """The fp32 workspace of a product is at most three parts of 256 KB for each pair of SMs, however long K is; one beyond that is shared out
+    otherwise and is right."""
+    import random
+
+    from neuronx_distributed_b200 import ops
+
+    e, rng = ops._ext.ext(), random.Random(3)
+    bound = 3 * (torch.cuda.get_device_properties(0).multi_processor_count // 2) * 256 * 256 * 4
+    sizes = [(1000, 4096, 128256), (2048, 4096, 22016), (3584, 1024, 28672), (3000, 4096, 32000)]
+    sizes += [(8 * rng.randint(16, 1024), 128 * rng.randint(1, 256), 64 * rng.randint(4, 4096)) for _ in range(2000)]
+    taken = [e.gemm_2cta_workspace(*size, f32, add) for size in sizes for f32, add in ((False, False), (True, False), (True, True))]
+    assert max(taken) <= bound and sum(t > 0 for t in taken) > len(sizes) // 4
+    M, N, K = 504, 5120, 65536                             # 40 tiles: 7 parts of each would be 73 MB
+    a, b = (torch.randn(n, K, device="cuda").bfloat16() for n in (M, N))
+    out = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    e.gemm_bf16_2cta(a, b, out, False, True, False)
+    want = a.double() @ b.double().t()
+    # one rounding to bfloat16 of sums of K products in 32 bits
+    assert (out.double() - want).abs().max() <= 2.0 ** -8 * want.abs().max() + 2.0 ** -20 * K
