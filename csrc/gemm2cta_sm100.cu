@@ -286,11 +286,15 @@ __global__ void __launch_bounds__(256) gemm_tail_kernel(const float* part, OutT*
   };
   sum(a, col);
   if constexpr (GATE) {
+    static_assert(sizeof(OutT) == 2);
     sum(b, kCols + col);
     if (keep) {
-      OutT* row_of = keep + (size_t)gr * 2 * N + gc;
+      Pack16<OutT> gate, up;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) { row_of[j] = from_f32<OutT>(a[j]); row_of[N + j] = from_f32<OutT>(b[j]); }
+      for (int j = 0; j < 8; ++j) { gate.set(j, a[j]); up.set(j, b[j]); }
+      OutT* row_of = keep + (size_t)gr * 2 * N + gc;
+      gate.store(row_of);
+      up.store(row_of + N);
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) a[j] = silu_mul_bf16(a[j], b[j]);
