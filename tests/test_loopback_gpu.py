@@ -1,8 +1,7 @@
-"""Single-GPU loopback: TWO processes on cuda:0 run the cross-rank kernels against each other (the driver's 1-GPU `pytest -m gpu`
-then exercises the flag / epoch protocols of the fused TP kernels, the NVLS-layout collectives and the symmetric-memory
-exchange instead of skipping them).  No multicast mapping exists between two contexts of one device, so the NVLS kernels run
-their unicast fallback (same protocol, peer pointers instead of the multicast address); the references are plain fp32 matmuls
-computed locally — every rank can rebuild all ranks' inputs from the seeds, no library collective is involved."""
+"""The cross-rank kernels against each other without a library collective: the flag / epoch protocols of the fused TP kernels, the
+NVLS-layout collectives and the symmetric-memory exchange, two processes on a GPU each.  The references are plain fp32 matmuls
+computed locally — every rank can rebuild all ranks' inputs from the seeds.  On one GPU they are skipped: kernels that wait on one another
+have to run at the same time (``test_symm_protocol_cpu.py`` and ``test_misc_cpu.py`` cover the protocols without a GPU)."""
 import pytest
 import torch
 
@@ -27,7 +26,7 @@ def _symm_and_collectives(rank, world):
 
     g = dist.group.WORLD
     ws = symm.get_vmm_workspace(g, "loopback_probe", 8 << 20)
-    assert not ws.has_multicast and len(ws.ptr_list) == world and ws.ptr_list[rank] == ws.local_ptr
+    assert len(ws.ptr_list) == world and ws.ptr_list[rank] == ws.local_ptr
     for it in range(3):                                   # epochs / parity halves
         xs = [_inputs(r, (1 << 16,), 10 + it) for r in range(world)]
         ref = sum(x.float() for x in xs)
@@ -62,7 +61,7 @@ def _fused_tp(rank, world):
 
     _fused_impl._NVLS_MODE = "force"
     ws = _fused_impl.workspace(dist.group.WORLD)
-    assert ws.nvls_enabled() and not ws.nv.has_multicast
+    assert ws.nvls_enabled()
     for wire in ("bf16", "fp32"):
         os.environ["NXD_TP_WIRE"] = wire
         for it, (ms, N, K) in enumerate([(256, 512, 256), (512, 1000, 512), (256, 512, 256)]):

@@ -355,7 +355,7 @@ def _embedding_gather_loopback(rank, world):
 
 
 def test_embedding_gather_over_peer_memory_loopback():
-    """``embedding_rs``: two processes on cuda:0 publish their vocabulary shards and pull rows from each other."""
+    """``embedding_rs``: two processes publish their vocabulary shards and pull rows from each other."""
     import sys
 
     sys.path.insert(0, os.path.join(ROOT, "tests"))
@@ -389,7 +389,7 @@ def _all_to_all_loopback(rank, world):
 
 
 def test_all_to_all_over_peer_memory_loopback():
-    """EP dispatch / combine without NCCL: publish + pull kernels between two processes on cuda:0."""
+    """EP dispatch / combine without NCCL: publish + pull kernels between two processes."""
     import sys
 
     sys.path.insert(0, os.path.join(ROOT, "tests"))
