@@ -67,13 +67,6 @@ NXD_DEVICE void mma_ts4(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint
                ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate), "n"(B1), "n"(2 * B1), "n"(3 * B1), "n"(A2), "n"(A2 + 8)
                : "memory");
 }
-NXD_DEVICE void tcgen05_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-                 "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-               : "r"(taddr)
-               : "memory");
-}
 NXD_DEVICE void tcgen05_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
@@ -972,9 +965,9 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
 }
 
 // −δ·scale and −lse·log2e per (b, h, s), and zeros for the row's dQ accumulator (rows up to S_pad).  16 lanes per row, 16 bytes per
-// lane; heads fastest, as o and dO lie in memory.  The main kernel's blocks take their places and load K and V beside this one, and the
-// conversion of dQ starts on the SMs that run out of it: whole backward, 1 x 2048 x 32 heads, 146 us with launches one after the other,
-// 140 so, 136 with one row per half warp instead of four in flight; 1 x 1000 x 32: 61 and 53; 1 x 70 x 32: 21.6 and 14.5.
+// lane; heads fastest, as o and dO lie in memory.  The main kernel's blocks take their places and load K, V, Q and dO beside this one, and the
+// conversion of dQ starts on the SMs that run out of it: whole backward with a main kernel of 116 us, 1 x 2048 x 32 heads, 146 us with launches
+// one after the other, 140 so, 136 with one row per half warp instead of four in flight; 1 x 1000 x 32: 61 and 53; 1 x 70 x 32: 21.6 and 14.5.
 __global__ void __launch_bounds__(256) fa_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ go,
                                    const float* __restrict__ lse, const float* __restrict__ dlse, float* __restrict__ stats,
                                    float* __restrict__ dq_acc, long stats_stride, int B, int S,
@@ -1154,7 +1147,7 @@ void flash_attn_bwd(const void* go, const void* q, const void* k, const void* v,
   if (det) NXD_CUDA_CHECK(cudaMemsetAsync(turnstile, 0, (size_t)B * H * flash_attn_bwd_query_tiles(S_q) * sizeof(unsigned), st));
   {
     const long rows = (long)B * H * S_pad;
-    // an ordinary launch: the main kernel loads K and V before it waits for this one, so they have to be there when this one starts
+    // an ordinary launch: the main kernel loads K, V, Q and dO before it waits for this one, so they have to be there when this one starts
     fa_bwd_prep_kernel<<<(unsigned)((rows + 15) / 16), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)go, lse, dlse, stats,
                                                                      dq_acc, p.stats_stride, B, S_q, H, S_pad, os[0], os[1], os[2], gs[0],
                                                                      gs[1], gs[2], scale);

@@ -7,7 +7,9 @@
 //   warp 0      TMA producer   : cp.async.bulk.tensor → 128B-swizzled smem ring (4 stages × 48 KB)
 //   warp 1      MMA issuer     : one thread issues tcgen05.mma (M=128, N=256, K=16) into a
 //                                double-buffered 128×256 fp32 accumulator in TMEM (2×256 columns);
-//                                tcgen05.commit releases smem stages / publishes accumulators
+//                                tcgen05.commit releases smem stages / publishes accumulators.  A product of 256 columns lasts
+//                                as long as one thread takes to issue it (about 130 cycles); one election for a k-block, as the CTA
+//                                pairs have it (gemm2cta.cuh), has not been tried here, nor in the tensor-parallel and block-scaled kernels
 //   warps 2-5   epilogue       : tcgen05.ld (32 lanes × 32 columns per warp) → convert → global stores
 //
 // Operand majors are template parameters so forward (A K-major, B K-major), dgrad (B MN-major) and wgrad
@@ -24,7 +26,7 @@
 //           red.release.sys; after its last tile every CTA turns into a reducer that acquires the 8
 //           counters of a row-block, sums the partials in fp32 and writes the bf16 result.
 //   Payload regions are double-buffered by call parity and flags are monotonic, so consecutive calls need
-//   no barrier ("symmetric memory protocol").
+//   no barrier.
 #include <cuda.h>
 
 #include "common.cuh"

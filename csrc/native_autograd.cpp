@@ -2,8 +2,8 @@
 // loss and the linear layer of one rank.  Each does what the torch.autograd.Function of the same name in ops/ or parallel_layers/layers.py does
 // (the same kernels on the same tensors, the same tensors saved); those stay for CPU tensors, tensor subclasses, recording, tracing,
 // functorch and forward-mode AD, which the callers ask about (ops/_ext.py native()).  A node in Python costs about 20 us forward and 40 us
-// backward (its context, the interpreter's lock in the engine's thread, a dozen calls), a small training step has 23 of them: 2750 us a step
-// with them, 1900 with these.
+// backward (its context, the interpreter's lock in the engine's thread, a dozen calls), a small training step had 23 of them: 2750 us a step
+// with them, 1900 with the first of these.
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>

@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(256) gemv_allreduce_kernel(const __nv_bfloat16
   finish_call(state, epoch);
 }
 
-// ---- vocab-parallel embedding lookup for a sequence-parallel consumer (SURVEY §7.4 `embedding_rs`) -------------------------
+// ---- vocab-parallel embedding lookup for a sequence-parallel consumer (`embedding_rs`) -------------------------
 // The reference looks every token up in the local vocab shard (zero rows for foreign ids), producing the full [S, B, H]
 // partial, and reduce-scatters it (layers.py:334-378): S·B·H elements written, masked and pushed through a collective although
 // every output row has exactly ONE non-zero contributor.  With NVSwitch peer memory the lookup itself can be remote:

@@ -14,7 +14,7 @@
 //   vmm_bind         bind the local memory, map the multicast VA                          → ok / error string
 //   vmm_ptrs         unicast pointer table + multicast base (0 if unavailable)
 // Driver entry points are resolved with cudaGetDriverEntryPoint so the extension does not link libcuda (the build box
-// has no driver).  No reference counterpart: the reference's collectives are XLA ops (SURVEY §5.8).
+// has no driver).  No reference counterpart: the reference's collectives are XLA ops.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <errno.h>

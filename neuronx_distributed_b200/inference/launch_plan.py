@@ -53,7 +53,7 @@ _EXT_PURE = frozenset({"rmsnorm_fwd", "rmsnorm_bwd", "add_rmsnorm_fwd", "add_rms
                        "rope_qkv_fwd", "rope_qkv_bwd",
                        "ce_stats", "ce_loss", "ce_backward", "decode_attention", "decode_attention_partial", "gemv", "gemm_few_rows", "gemv_mx",
                        "gemm_mxfp8", "moe_block_tkg", "moe_block_metadata", "moe_slots", "moe_gather", "moe_combine",
-                       "moe_combine_grad", "moe_normalize", "moe_normalize_grad", "row_argmax", "row_topk", "flash_attn_fwd",
+                       "moe_combine_grad", "row_argmax", "row_topk", "flash_attn_fwd",
                        "flash_attn_bwd", "flash_attn_bwd_parts", "moe_block_tkg_supported", "row_topk_supported", "grouped_gemm"})
 # … and the ones that write exactly these positional arguments (everything else they take is read-only)
 _EXT_WRITES = {"gemm_bf16": (2,), "gemm_bf16_2cta": (2,), "gemm_fp8": (2,), "grouped_wgrad": (2,), "decode_rope_kv": (6, 7),
