@@ -10,7 +10,7 @@ meta-path finder that fabricates those packages:
   (dim-0 sharded optimizer state + fp32 master weights + reduce-scatter / all-gather);
 * everything else resolves to inert placeholders so that ``import neuronx_distributed`` succeeds.
 
-This is the "reference's own NCCL(+cuBLAS) build" of BASELINE.md: the reference's code runs unchanged, its XLA
+This is the "reference's own NCCL(+cuBLAS) build": the reference's code runs unchanged, its XLA
 collectives land on NCCL and its matmuls on cuBLAS.
 """
 from __future__ import annotations

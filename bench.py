@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Headline benchmark: Llama-2-7B training tokens/s on N GPUs of one node with TP=N (BASELINE.json).
+"""Headline benchmark: Llama-2-7B training tokens/s on N GPUs of one node with TP=N.
 
     python bench.py --gpus 1 --steps 5 --warmup 3
     python -m torch.distributed.run --nnodes=1 --nproc-per-node N --master-addr 127.0.0.1 --master-port P \
@@ -25,7 +25,7 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 # published number closest to the metric: Llama-2-7B gate 6.90 seq/s at seq 8192 on 32 NeuronCores
-# (BASELINE.md; test/integration/llama2_7B/test_long_seqlen.py:95-97) = 56,525 tokens/s
+# (test/integration/llama2_7B/test_long_seqlen.py:95-97) = 56,525 tokens/s
 PUBLISHED_TOKENS_PER_S = 6.90 * 8192
 
 
@@ -37,8 +37,8 @@ def parse():
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--mode", default="train", choices=["train", "decode", "pp", "naguzen", "pinirax", "pulenex", "noresun", "kulisun",
                                                         "kekelix"],
-                    help="train (default, the headline: Llama-2-7B training tokens/s) | decode (BASELINE config 5: Llama-2-13B "
-                         "inference latency, batch 1, seq 2048) | pp (BASELINE config 4: GPT-NeoX-20B TP x PP=2 1F1B training) | "
+                    help="train (default, the headline: Llama-2-7B training tokens/s) | decode (Llama-2-13B "
+                         "inference latency, batch 1, seq 2048) | pp (GPT-NeoX-20B TP x PP=2 1F1B training) | "
                          "naguzen (serving throughput and per-kernel rooflines of the Naguzen design beside Llama at equal size) | "
                          "pinirax (the same for the Pinirax design beside Naguzen at equal size) | "
                          "pulenex (the same for the Pulenex design beside Naguzen and Pinirax at equal size) | "
@@ -56,7 +56,7 @@ def parse():
                          "that reports the exposed TP-collective time per step")
     ap.add_argument("--tp", type=int, default=0, help="tensor-parallel degree (default: gpus / dp)")
     ap.add_argument("--dp", type=int, default=1, help="data-parallel degree: ZeRO-1 shards the optimizer over it and its gradient "
-                                                      "reduce-scatter kernel runs in the step (BASELINE config 3: --gpus 8 --tp 4 --dp 2)")
+                                                      "reduce-scatter kernel runs in the step (e.g. --gpus 8 --tp 4 --dp 2)")
     ap.add_argument("--micro-batch", type=int, default=0,
                     help="sequences per forward/backward (0 = auto: 2 up to 2 GPUs, 4 beyond — fewer fp32 wgrad read-modify-write "
                          "passes and TP collectives off their latency floor; 4 does not fit in 180 GB at TP=1); same value in both arms")
@@ -127,7 +127,7 @@ def run_reference(args):
 
 
 def _tp_comm_info(tp: int, backend: str) -> dict:
-    """What crosses NVLink on the TP hot path, stated in the JSON line (wire precision must be in `config`)."""
+    """What crosses NVLink on the TP hot path, stated in the JSON line (its wire precision among it)."""
     if tp == 1:
         return {"tp_collectives": "none (tp=1)", "wire_dtype": "n/a"}
     if backend != "fused":
@@ -334,7 +334,7 @@ def main():
         e2e = {"value": tokens_per_step * args.steps / float(tt.item()), "unit": "tokens/s",
                "h2d_bytes_per_step": h2d // args.steps, "d2h_bytes_per_step": d2h // args.steps}
 
-    # ---- exposed tensor-parallel communication (BASELINE metric): same step with the TP collectives replaced by local copies of
+    # ---- exposed tensor-parallel communication: same step with the TP collectives replaced by local copies of
     #      the same shape ("nocomm" backend, numerically meaningless) → exposed = t(step) − t(nocomm step).  Runs last because it
     #      trashes the weights; any failure only drops this key.
     comm_report = None

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Llama inference sample + latency benchmark (BASELINE config 5: Llama-2-13B, TP=8, batch 1, seq 2048) — counterpart of the
+"""Llama inference sample + latency benchmark (Llama-2-13B, TP=8, batch 1, seq 2048) — counterpart of the
 reference's ``examples/inference/run_llama.py`` / ``runner.py`` (trace → load → generate → benchmark → report).
 
   torchrun --nproc-per-node 8 examples/inference/run_llama.py --model 13b --tp_degree 8 --batch_size 1 \

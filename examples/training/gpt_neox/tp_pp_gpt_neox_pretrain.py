@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""GPT-NeoX pre-training, TP × PP 1F1B (BASELINE config 4: NeoX-20B, TP=4 × PP=2 on 8 GPUs) — counterpart of the reference's
+"""GPT-NeoX pre-training, TP × PP 1F1B (NeoX-20B, TP=4 × PP=2 on 8 GPUs) — counterpart of the reference's
 ``examples/training/tp_dp_gpt_neox_hf_pretrain``.
 
   torchrun --nproc-per-node 8 examples/training/gpt_neox/tp_pp_gpt_neox_pretrain.py --model 20b --tensor_parallel_size 4 \

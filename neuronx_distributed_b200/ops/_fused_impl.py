@@ -12,7 +12,7 @@ Row + sequence-parallel     (``out_mode="scatter"``):
 Design choice vs the reference: the gathered activation is kept (one D2D copy out of the symmetric
 buffer) instead of being re-all-gathered in backward (reference layers_utils.py:82-87) — HBM is
 plentiful on B200 and NVLink is the scarce resource on these paths.  Wire dtype is bf16 with fp32
-accumulation at the owner (the reference reduces fp32 on the wire, layers.py:1031-1045); see DESIGN.md.
+accumulation at the owner (the reference reduces fp32 on the wire, layers.py:1031-1045).
 
 Protocol state (epochs, cumulative counters) lives in :class:`TPWorkspace`, one per process group.
 """
@@ -309,7 +309,7 @@ _LOGGED = set()
 
 
 def _log_once(key: str, msg: str) -> None:
-    """One warning per (reason) — a fused→library fallback must never be silent (VERDICT r1 weak #3)."""
+    """One warning per (reason) — a fused→library fallback must never be silent."""
     if key in _LOGGED:
         return
     _LOGGED.add(key)

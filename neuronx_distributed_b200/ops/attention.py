@@ -1,6 +1,5 @@
 """Causal self-attention (flash style).  Kernel: ``csrc/attention_sm100.cu`` (tcgen05 QK^T / PV with
-TMEM accumulators, online softmax) when built; otherwise the PyTorch SDPA library call, which is
-flagged as a *library* path in DESIGN.md.  Reference call sites: ``kernels/flash_attn.py:162-212``
+TMEM accumulators, online softmax) when built; otherwise the PyTorch SDPA library call.  Reference call sites: ``kernels/flash_attn.py:162-212``
 (``nki_flash_attn_func``), ``modeling_llama_nxd.py:468-475``.
 
 Layout: q ``[B, S, Hq, D]``, k/v ``[B, S, Hkv, D]`` → out ``[B, S, Hq, D]``.

@@ -7,7 +7,7 @@ directly (P2P ld/st over NVSwitch).  Handles travel over the gloo control group.
 
 A :class:`SymmWorkspace` is created lazily per (process group, purpose) and reused; kernels use
 monotonically increasing epochs with double-buffered payload so no extra barrier is needed
-between consecutive calls (see DESIGN.md §symmetric memory protocol).
+between consecutive calls.
 """
 from __future__ import annotations
 

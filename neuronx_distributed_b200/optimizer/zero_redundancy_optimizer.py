@@ -1,8 +1,7 @@
 """ZeRO-1: optimizer state and fp32 master weights sharded over the data-parallel group.
 
 Role parity with reference ``optimizer/zero_redundancy_optimizer.py`` (``NeuronZero1Optimizer``
-:30, ``NeuronEPZero1Optimizer`` :163) whose base class lives in torch_xla (external, K13 in
-SURVEY §2.9) — this is a from-scratch implementation designed for B200:
+:30, ``NeuronEPZero1Optimizer`` :163) whose base class lives in torch_xla (external) — this is a from-scratch implementation designed for B200:
 
 * **Flat contiguous buffers.**  Per (param-group, dtype) the model parameters are re-pointed
   into one flat ``param_flat`` buffer and gradients accumulate into one flat fp32 (or bf16)

@@ -15,8 +15,7 @@ B200 design notes
 * Weight init is TP-degree independent: build the full fp32 master weight from the default
   RNG, cast, keep this rank's (strided) slice.
 * Row-parallel reductions honour ``reduce_dtype`` (fp32 default, as the reference) on the
-  library path; the fused path accumulates in fp32 and moves bf16 on the wire (documented in
-  DESIGN.md).
+  library path; the fused path accumulates in fp32 and moves bf16 on the wire.
 """
 from __future__ import annotations
 

@@ -171,7 +171,7 @@ def from_parallel_logits_to_logprobs(vocab_parallel_logits, target, inference: b
 
 
 # ---------------------------------------------------------------------------------------------------------------------
-# lm_head + cross entropy without materialising the logits (SURVEY §7.4 ``lmhead_ce_fused``)
+# lm_head + cross entropy without materialising the logits (``lmhead_ce_fused``)
 # ---------------------------------------------------------------------------------------------------------------------
 class _FusedLinearCrossEntropy(torch.autograd.Function):
     """``mean_over_unmasked( CE( gather(h) @ Wᵀ , target) )`` in row chunks: per chunk the vocab-parallel logits

@@ -1,4 +1,4 @@
-"""Profiling / debugging helpers (SURVEY §5.1, §5.2).
+"""Profiling / debugging helpers.
 
 * ``nvtx_range(name)`` — NVTX range when ``NXD_NVTX=1`` (no-op otherwise): pipeline tasks, decoder layers and optimizer phases
   are bracketed so Nsight timelines show the schedule.  The reference's only timeline is a host-clock Chrome trace that is

@@ -1,5 +1,5 @@
 """Run a function on N local processes (gloo on CPU / nccl on GPUs) — the analogue of the
-reference's ``NXD_CPU_MODE=1 torchrun --nproc-per-node=N`` integration tier (SURVEY §4)."""
+reference's ``NXD_CPU_MODE=1 torchrun --nproc-per-node=N`` integration tier."""
 from __future__ import annotations
 
 import os

@@ -1,6 +1,6 @@
 """Unit tests of the model-building components that the bigger model tests only touch indirectly: GQA-QKV with KV replication,
 input-channel parallel conv, pad_model, RNG tracker, grad norm / clip, DistributedLogprob, the extra routers, shared experts,
-token shuffling (SURVEY §2.3 / §2.6)."""
+token shuffling."""
 
 import pytest
 import torch

@@ -1,4 +1,4 @@
-"""every public name of the reference must be importable from the same place here."""
+"""Every public name of the reference must be importable from the same place here."""
 import importlib
 
 import pytest

@@ -1,5 +1,5 @@
 """Column/Row/Embedding/CE fwd+bwd parity vs single-device torch modules on 2 gloo ranks
-(BASELINE config #1; role of reference test/integration/parallel_layers/test_layers.py)."""
+(role of reference test/integration/parallel_layers/test_layers.py)."""
 import pytest
 import torch
 import torch.nn.functional as F

@@ -1,4 +1,4 @@
-"""BASELINE config 5 through ``bench.py --mode decode``: Llama-2-13B inference latency at TP = N, batch 1, sequence 2048
+"""``bench.py --mode decode``: Llama-2-13B inference latency at TP = N, batch 1, sequence 2048
 (prompt 1024 + 1024 generated tokens), random-init weights, synthetic prompt.
 
 Metric (reference ``examples/inference/modules/benchmark.py:9-73``, ``runner.py:521-602``): latency percentiles of the full

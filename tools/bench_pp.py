@@ -1,8 +1,8 @@
-"""BASELINE config 4 through ``bench.py --mode pp``: GPT-NeoX-20B pre-training step with tensor parallel x pipeline parallel
+"""``bench.py --mode pp``: GPT-NeoX-20B pre-training step with tensor parallel x pipeline parallel
 (NxDPPModel, 1F1B schedule, NCCL p2p between stages, fused TP kernels inside each stage), bf16, ZeRO-1 (fp32 master + fp32
 gradient accumulation), synthetic tokens, random-init weights built directly on the device (meta-device init).
 
-    torchrun --nproc-per-node 8 bench.py --mode pp --gpus 8            # TP=4 x PP=2 (the BASELINE shape)
+    torchrun --nproc-per-node 8 bench.py --mode pp --gpus 8            # TP=4 x PP=2 (the headline shape)
     torchrun --nproc-per-node 4 bench.py --mode pp --gpus 4            # TP=2 x PP=2
 
 value = tokens/s of the whole job (device-timed with CUDA events, max over ranks).  The pipeline bubble is measured, not

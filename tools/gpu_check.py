@@ -1,8 +1,8 @@
-"""On-GPU numerics + timing smoke for every hand-written kernel (run under gpurun).
+"""On-GPU numerics + timing smoke for every hand-written kernel (needs a B200).
 
 usage: python tools/gpu_check.py [elementwise|gemm|gemm_perf|all]
 Each check prints one line `CHECK name PASS/FAIL max_err=…`; results are also appended to
-gpurun_out/gpu_check.jsonl.  Comparison target is always a plain PyTorch fp32 reference."""
+gpu_check.jsonl (in `NXD_OUT`, else the working folder).  Comparison target is always a plain PyTorch fp32 reference."""
 import json
 import os
 import sys
@@ -12,8 +12,7 @@ import torch
 sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 from neuronx_distributed_b200 import ops  # noqa: E402
 
-OUT = os.path.join(os.environ.get("GRAFT_REPO_ROOT", "."), "gpurun_out")
-os.makedirs(OUT, exist_ok=True)
+OUT = os.environ.get("NXD_OUT", ".")
 dev = torch.device("cuda")
 RESULTS = []
 

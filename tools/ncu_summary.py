@@ -1,5 +1,5 @@
 """Condense an .ncu-rep (captured with --set full) into a committed text summary: per kernel the headline metrics of the raw page.
-usage: python tools/ncu_summary.py gpurun_out/x.ncu-rep > profiles/x_ncu_summary.txt"""
+usage: python tools/ncu_summary.py x.ncu-rep > profiles/x_ncu_summary.txt"""
 import csv
 import io
 import subprocess
