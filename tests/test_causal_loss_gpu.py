@@ -85,3 +85,17 @@ def test_not_taken_and_captured():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(got, want)
+
+
+def test_recorded_gradients_and_recomputation():
+    from torch.utils.checkpoint import checkpoint
+
+    from neuronx_distributed_b200.parallel_layers.loss_functions import causal_lm_loss
+
+    _setup()
+    x, labels = torch.randn(70, 3, 520, device="cuda").bfloat16().requires_grad_(), torch.randint(0, 520, (3, 70), device="cuda")
+    want, = torch.autograd.grad(causal_lm_loss(x, labels), x)
+    for loss in (causal_lm_loss(x, labels), checkpoint(causal_lm_loss, x, labels, use_reentrant=False)):
+        got, = torch.autograd.grad(loss, x, create_graph=True)
+        again, = torch.autograd.grad(loss, x)
+        assert torch.equal(got, want) and torch.equal(again, want)

@@ -124,3 +124,19 @@ def test_lookups_with_and_without_python_in_their_node(shape):
         y = lookup(ids, w)
         out.append((y, *torch.autograd.grad(y, w, go.transpose(0, -1).contiguous().transpose(0, -1))))
     assert all(torch.equal(a, b) for a, b in zip(*out)) and torch.equal(out[0][0], w[ids])
+
+
+def test_its_gradient_is_differentiated_again():
+    """The gradient of the table is linear in the upstream one: with create_graph it keeps its graph, in both nodes."""
+    from neuronx_distributed_b200 import ops
+    from neuronx_distributed_b200.parallel_layers.layers import _TableLookup
+
+    g = torch.Generator(device="cuda").manual_seed(9)
+    w = torch.randn(40, 64, generator=g, device="cuda").bfloat16().requires_grad_()
+    ids = torch.randint(0, 40, (3, 50), generator=g, device="cuda")
+    go = torch.randn(3, 50, 64, generator=g, device="cuda").bfloat16().requires_grad_()
+    second = []
+    for lookup in (_TableLookup.apply, ops._ext.ext().native.table_lookup, lambda i, t: torch.nn.functional.embedding(i, t)):
+        (gw,) = torch.autograd.grad(lookup(ids, w), w, go, create_graph=True)
+        second.append(torch.autograd.grad(gw.float().square().sum(), go)[0])
+    assert torch.equal(second[0], second[2]) and torch.equal(second[1], second[2]) and second[2].any()

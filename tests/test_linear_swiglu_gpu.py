@@ -184,3 +184,55 @@ def test_products_of_experts_are_given_back_before_the_gradients_are_computed():
     one, two = (_peak_of_backward(f, (x, w)) for f in (
         lambda: ops.gemm.grouped_swiglu(*a, slots.token), lambda: ops.act.swiglu(ops.gemm.grouped_matmul(*a, skip_unused=True, slot_token=slots.token))))
     assert one <= two + 2 ** 16
+
+
+# numbers of rows that are no multiple of 8 (and few or many of them): the two kernels or the library's, by the same rules as a plain projection
+@pytest.mark.parametrize("M", [65, 97, 301, 777, 1001])
+@pytest.mark.parametrize("grads", [False, True])
+def test_rows_that_the_one_kernel_leaves(M, grads):
+    mlp = _mlp()
+    x, w = _case(M, 384, 256)
+    mlp.gate_up_proj.weight.data.copy_(w)
+    x, weights = x.view(M, 1, 256).requires_grad_(grads), (mlp.gate_up_proj.weight, mlp.down_proj.weight)
+    with torch.set_grad_enabled(grads):
+        y = mlp(x)
+    ref = [t.detach().double().requires_grad_() for t in (x, *weights)]
+    gate, up = (ref[0] @ ref[1].t()).chunk(2, -1)
+    want = torch.nn.functional.silu(gate) * up @ ref[2].t()
+    # gate, up, their SwiGLU and the result are each rounded to bf16 once; silu's slope is at most 1.1
+    assert float((y.detach().double() - want).norm() / want.norm()) < 4.2 * 2 ** -9
+    if grads:
+        go = torch.randn_like(y)
+        for a, b in zip(torch.autograd.grad(y, (x, *weights), go), torch.autograd.grad(want, ref, go.double())):
+            assert float((a.double() - b).norm() / b.norm()) < 2 ** -6        # two more products, each of rounded factors
+
+
+@pytest.mark.parametrize("how", ["create", "checkpoint", "hooks"])
+def test_its_nodes_as_programs_use_them(how):
+    """Recorded gradients, recomputation and hooks on what is saved: the results of a plain backward pass, and the same tensors saved."""
+    from torch.utils.checkpoint import checkpoint
+
+    from neuronx_distributed_b200.parallel_layers.layers import ColumnParallelLinear, column_swiglu
+
+    _mlp()
+    M, I, K = 264, 1408, 1024
+    x, w = _case(M, I, K)
+    proj = ColumnParallelLinear(K, 2 * I, bias=False, gather_output=False, dtype=torch.bfloat16, device=torch.device("cuda", 0))
+    proj.weight.data.copy_(w)
+    go = torch.randn(M, I, device="cuda").bfloat16()
+    x.requires_grad_()
+    want = torch.autograd.grad(column_swiglu(proj, x), (x, proj.weight), go)
+    packed, before = [], ops._ext.launches()
+    if how == "checkpoint":
+        y = checkpoint(column_swiglu, proj, x, use_reentrant=False)
+    elif how == "hooks":
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(tuple(t.shape)) or t.cpu(), lambda t: t.cuda()):
+            y = column_swiglu(proj, x)
+        assert sorted(packed) == sorted([(M, K), (2 * I, K), (M, 2 * I)])
+    else:
+        y = column_swiglu(proj, x)
+    assert ops._ext.launches() - before == 1
+    got = torch.autograd.grad(y, (x, proj.weight), go, retain_graph=True, create_graph=how == "create")
+    again = torch.autograd.grad(y, (x, proj.weight), go)
+    for a, b, c in zip(want, got, again):
+        assert torch.equal(a, b) and torch.equal(a, c)
