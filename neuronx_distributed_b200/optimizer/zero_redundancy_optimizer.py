@@ -393,7 +393,7 @@ class Zero1Optimizer(torch.optim.Optimizer):
                     continue
                 piece = fg.grad_shard[s0 : s0 + n]
                 (sharded if getattr(slot.param, "tensor_model_parallel", False) else dup).append(piece)
-        if tp == 1:                                # every weight is one: one launch
+        if tp == 1 and all(fg.device == dev for fg in self.flat_groups):      # every weight is one: one launch
             sharded, dup = sharded + dup, []
         total = ops.optim.multi_tensor_sq_norm(sharded).to(dev) if sharded else torch.zeros((), device=dev)
         if dup:
